@@ -100,7 +100,7 @@ struct s14_ctx {
         uint32_t wait_limit = 1u << 22;  // polls of about a microsecond: a few seconds
     } ep;
     float *glue = nullptr;    // [kGlueTokens, 25] dot products and mean squares of the hyper-connection calls
-    uint16_t *glue16 = nullptr;  // [4, 8192] BF16 vectors between the steps of the executor calls
+    uint16_t *glue16 = nullptr;  // [8192] a BF16 vector between the steps of an executor call
     UmmaScratch umma{nullptr, nullptr, nullptr};  // scratch of the tcgen05 layer kernel
     bool use_umma = true;                // S14_TENSOR_PATH=off in the environment turns it off
     const UmmaScratch *umma_scratch() const { return use_umma ? &umma : nullptr; }
@@ -134,7 +134,7 @@ extern "C" int32_t s14_ctx_create(int32_t device, s14_ctx **out) {
     CUDA_OK(cudaMalloc(&ctx->select, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->dev_table, sizeof(JobTable)));
     CUDA_OK(cudaMalloc(&ctx->glue, sizeof(float) * kGlueTokens * 25));
-    CUDA_OK(cudaMalloc(&ctx->glue16, sizeof(uint16_t) * 4 * 8192));
+    CUDA_OK(cudaMalloc(&ctx->glue16, sizeof(uint16_t) * 8192));
     CUDA_OK(cudaMalloc(&ctx->x_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->y_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->status, sizeof(uint32_t)));
@@ -2205,17 +2205,22 @@ static void check_streams(const char *what, uint32_t n_tokens, uint32_t hc, uint
     if (dtype != S14_STREAM_F32 && dtype != S14_STREAM_BF16) throw ContractError(std::string(what) + ": unknown stream type");
 }
 
+static void check_hc(const char *what, const s14_ctx *ctx, const s14_hc_params *p, const void *x) {
+    if (!ctx || !p || !x) throw ContractError(std::string(what) + ": NULL argument");
+    check_streams(what, p->n_tokens, p->hc, p->hidden, p->dtype);
+    if (!p->hc_fn || !p->hc_scale || !p->hc_base) throw ContractError(std::string(what) + ": hc_fn, hc_scale or hc_base is NULL");
+    if (!std::isfinite(p->norm_eps) || p->norm_eps <= 0.0f || !std::isfinite(p->hc_eps) || p->hc_eps <= 0.0f)
+        throw ContractError(std::string(what) + ": norm_eps and hc_eps must be finite and positive");
+}
+
 static int32_t hc_reduce_call(s14_ctx *ctx, void *stream, const s14_hc_params *p, bool head, const void *x, void *reduced,
                               float *post, float *comb, float *pre, const char *what) {
     S14_TRY
-    if (!ctx || !p || !x || !reduced) throw ContractError(std::string(what) + ": NULL argument");
-    check_streams(what, p->n_tokens, p->hc, p->hidden, p->dtype);
-    if (!p->hc_fn || !p->hc_scale || !p->hc_base) throw ContractError(std::string(what) + ": hc_fn, hc_scale or hc_base is NULL");
+    check_hc(what, ctx, p, x);
+    if (!reduced) throw ContractError(std::string(what) + ": NULL argument");
     if (!head && (!post || !comb)) throw ContractError(std::string(what) + ": post or comb is NULL");
     if (head && !pre) throw ContractError(std::string(what) + ": pre is NULL");
     if (!head && p->sinkhorn_iters == 0) throw ContractError(std::string(what) + ": at least one Sinkhorn round");
-    if (!std::isfinite(p->norm_eps) || p->norm_eps <= 0.0f || !std::isfinite(p->hc_eps) || p->hc_eps <= 0.0f)
-        throw ContractError(std::string(what) + ": norm_eps and hc_eps must be finite and positive");
     CUDA_OK(cudaSetDevice(ctx->device));
     cudaError_t err;
     ctx->launches += launch_hc_pre(stream_of(ctx, stream), p->dtype == S14_STREAM_BF16, head, p->n_tokens, p->hidden, x, p->hc_fn,
@@ -2328,15 +2333,13 @@ extern "C" int32_t s14_exec_hc_head_norm_full_logits(s14_ctx *ctx, void *stream,
         throw ContractError("s14_exec_hc_head_norm_full_logits: one token, BF16 state");
     if (n_rows == 0) throw ContractError("s14_exec_hc_head_norm_full_logits: no vocabulary rows");
     if (head->hidden > kMaxDim) throw ContractError("s14_exec_hc_head_norm_full_logits: hidden above 4096");
-    uint16_t *reduced = ctx->glue16 + 8192, *normed = ctx->glue16 + 2 * 8192;
-    float *pre = ctx->glue + (size_t)kGlueTokens * 24 + 512;
-    int32_t rc = hc_reduce_call(ctx, stream, head, true, state_bf16, reduced, nullptr, nullptr, pre, "s14_exec_hc_head_norm_full_logits");
-    if (rc != S14_OK) return rc;
+    check_hc("s14_exec_hc_head_norm_full_logits", ctx, head, state_bf16);
+    CUDA_OK(cudaSetDevice(ctx->device));
     cudaStream_t st = stream_of(ctx, stream);
-    CUDA_OK(launch_rms_norm(st, true, 1, head->hidden, reduced, norm_weight, head->norm_eps, normed));
-    CUDA_OK(launch_bf16_to_f32(st, normed, ctx->x_stage, head->hidden));
+    CUDA_OK(launch_head_prep(st, state_bf16, head->hc_fn, head->hc_scale, head->hc_base, norm_weight, head->hidden, head->norm_eps,
+                             head->hc_eps, ctx->x_stage));
     CUDA_OK(launch_head_logits(st, ctx->sm_count, ctx->x_stage, 1, head_weight_bf16, n_rows, head->hidden, logits_out, n_rows));
-    ctx->launches += 3;
+    ctx->launches += 2;
     return S14_OK;
     S14_CATCH
 }

@@ -2,6 +2,8 @@
 #ifndef S14_DEVICE_CUH
 #define S14_DEVICE_CUH
 
+#include <algorithm>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -120,6 +122,30 @@ __device__ __forceinline__ PageView page_view(const uint8_t *page, uint32_t kind
     v.s2 = v.s3 + sb;
     (void)kind;
     return v;
+}
+
+// A launch as a programmatic dependent of what precedes it in the stream, optionally in clusters of
+// `cluster` CTAs (0: none).  The kernels launched so wait with cudaGridDependencySynchronize() before they
+// touch anything an earlier kernel writes; in front of it they read only what no kernel of this library
+// writes (weights, pages, tables).  A kernel that does not trigger early (any kernel of the caller) is
+// complete before such a launch starts.
+template <class Kernel, class... Args>
+inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace s14

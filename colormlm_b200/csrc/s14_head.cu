@@ -1,0 +1,453 @@
+// The LM head of a decode step or a verify block: full logits of 1..8 tokens over a BF16 matrix, the greedy
+// token, and the steps before it (the head's hyper-connection reduce and RMSNorm) as one launch.
+// Reference: fast16/research/polaris_meridian_v1/local_s14_primitives/final_head.py:43-191,
+// scheduler/s14_runner/src/runner.rs:485-508.
+#include <cooperative_groups.h>
+
+#include "s14_device.cuh"
+
+namespace s14 {
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+// ---- logits -------------------------------------------------------------------------------------
+//
+// logits[t, v] = sum_k x[t, k] * W[v, k], W BF16, 1 GB per call at 129280 x 4096: the weight stream bounds it
+// (1.06 GB / 6.55 TB/s = 162 us), so what a weight element costs on the SM has to stay below 1.5 clocks per
+// 12 elements.  A register kernel does not manage that for eight tokens: it reads 32 bytes of x per weight
+// element through the L1 and converts a partial sum to double per 4 products (16 conversions per clock and
+// SM), 1118 us.  Here x is split once per CTA into three BF16 parts (x = h + m + l exactly: 6, 8 and 8
+// significant bits, each remainder's sign being worth one more) kept in shared memory, and a warp takes
+// sixteen rows of W as the A operand of mma.m16n8k16, the eight tokens' parts as B: every product is exact in
+// F32.  The sums of sixteen products with h (14-bit products: few of their bits fall off the F32 sum) go to
+// double every 16 elements of K; m and l, 2^-6 and 2^-15 of h, are summed in F32 over 128 elements and then
+// added (blocks of K that do not depend on the number of tokens).  Measured error (N(0,1) x N(0,0.02), K = 4096):
+// 3.9e-8 RMS, the register kernel's 4-product chains 6.0e-8.
+// A lane loads 16 bytes (eight k) of each of its two rows: words 0, 1 are its k slots of a first MMA, words 2, 3
+// of a second one, and x is read from shared memory in the same order, so K is only permuted.  Two warps share
+// sixteen rows (the halves of K): 8080 row tiles over 148 x 8 pairs leave the last round 97 % full.  Eight
+// 16-byte loads per lane are in flight (64 KB per SM), across row tiles; they need room in the L1, which shared
+// memory takes away (with eight tokens' 198 KB of parts resident: 290 us).  So K is walked in `phases` of at
+// most 50 KB of parts, the CTA's row tiles once per phase, their sums waiting in shared memory in between.
+constexpr uint32_t kHeadThreads = 512, kHeadPairs = kHeadThreads / 64u, kHeadDepth = 4;
+constexpr uint32_t kHeadPad = 64;   // a token's row of parts: the lanes of two tokens then use all banks once
+constexpr uint32_t kHeadTiles = 56; // row tiles of a CTA whose sums wait between phases (1 KB each)
+constexpr size_t kHeadPartBytes = 50u * 1024u;
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The BF16 parts of v: 6 significant bits, then 8, then the 8 that are left (nearest each time, so a remainder
+// is at most half a unit of the part before).  Infinities and NaNs go into the first alone.
+__device__ __forceinline__ void head_parts(float v, uint32_t (&p)[3]) {
+    uint32_t h = (__float_as_uint(v) + 0x00020000u) & 0xfffc0000u;
+    if ((h & 0x7f800000u) == 0x7f800000u && isfinite(v)) h = __float_as_uint(v) & 0xfffc0000u;  // would round to infinity
+    if (!isfinite(v)) {
+        const __nv_bfloat16 b = __float2bfloat16_rn(v);
+        p[0] = *reinterpret_cast<const uint16_t *>(&b);
+        p[1] = p[2] = 0u;
+        return;
+    }
+    const float r = __fsub_rn(v, __uint_as_float(h));  // exact
+    const __nv_bfloat16 m = __float2bfloat16_rn(r), l = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m)));
+    p[0] = h >> 16;
+    p[1] = *reinterpret_cast<const uint16_t *>(&m);
+    p[2] = *reinterpret_cast<const uint16_t *>(&l);
+}
+
+__global__ void __launch_bounds__(kHeadThreads, 1)
+k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
+           uint32_t out_stride, uint32_t n_tokens, uint32_t phases) {
+    extern __shared__ __align__(16) uint8_t s_parts[];      // [3][n_tokens][pitch], then the tiles' sums [tile][4][32]
+    __shared__ double s_half[kHeadPairs][2][4][32];          // the second warp's half of K, by tile parity
+    cudaTriggerProgrammaticLaunchCompletion();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, pair = warp >> 1, half = warp & 1u;
+    const uint32_t g = lane >> 2, q = lane & 3u;
+    const uint32_t span = hidden / phases;                   // of K per phase
+    const uint32_t pitch = span * 2u + kHeadPad, part_bytes = n_tokens * pitch;
+    const uint32_t steps = span >> 6;                        // of 32 k, of this warp's half: a multiple of four
+    const uint32_t n_tiles = (n_rows + 15u) >> 4, grid = gridDim.x;
+    double *const s_sum = reinterpret_cast<double *>(s_parts + 3u * part_bytes);
+    // the CTA's tiles: blockIdx.x + i * grid, i < n_mine; at most kHeadTiles at a time, dealt to the pairs in turn
+    const uint32_t n_mine = n_tiles > blockIdx.x ? (n_tiles - blockIdx.x + grid - 1u) / grid : 0u;
+    const uint32_t batch = phases > 1u ? kHeadTiles : n_mine;
+
+    // the weights do not depend on the kernel before this one: their first loads are in flight while x is split
+    const uint16_t *p0, *p1;
+    auto rows_of = [&](uint32_t i, uint32_t phase) {
+        const uint32_t t = blockIdx.x + i * grid, r0 = min(t * 16u + g, n_rows - 1u), r1 = min(t * 16u + g + 8u, n_rows - 1u);
+        const uint32_t k0 = phase * span + half * (span >> 1) + q * 8u;
+        p0 = w + (size_t)r0 * hidden + k0;
+        p1 = w + (size_t)r1 * hidden + k0;
+    };
+    uint4 a0[kHeadDepth], a1[kHeadDepth];
+    auto fetch = [&](uint32_t i, uint32_t k) {
+        a0[i] = ldg_stream(reinterpret_cast<const uint4 *>(p0 + (k + i) * 32u));
+        a1[i] = ldg_stream(reinterpret_cast<const uint4 *>(p1 + (k + i) * 32u));
+    };
+    if (pair < n_mine) {
+        rows_of(pair, 0u);
+#pragma unroll
+        for (uint32_t i = 0; i < kHeadDepth; ++i) fetch(i, 0u);
+    }
+    cudaGridDependencySynchronize();
+    const uint8_t *const sb = s_parts + (g < n_tokens ? g : 0u) * pitch + half * span + q * 16u;
+    const bool has_b = g < n_tokens;
+    uint32_t parity = 0;
+#pragma unroll 1
+    for (uint32_t base = 0; base < n_mine; base += batch) {
+        const uint32_t end = min(base + batch, n_mine);
+#pragma unroll 1
+        for (uint32_t phase = 0; phase < phases; ++phase) {
+            __syncthreads();  // the parts of the phase before are not read any more
+            for (uint32_t i = tid; i < n_tokens * (span >> 1); i += kHeadThreads) {
+                const uint32_t t = i / (span >> 1), k2 = i - t * (span >> 1);
+                const float2 v = __ldg(reinterpret_cast<const float2 *>(x + (size_t)t * hidden + phase * span) + k2);
+                uint32_t px[3], py[3];
+                head_parts(v.x, px);
+                head_parts(v.y, py);
+#pragma unroll
+                for (uint32_t part = 0; part < 3; ++part)
+                    *reinterpret_cast<uint32_t *>(s_parts + part * part_bytes + t * pitch + k2 * 4u) = px[part] | (py[part] << 16);
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (uint32_t i = base + pair; i < end; i += kHeadPairs, parity ^= 1u) {
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                // what this pair reads after this tile: its next tile, of this phase or the next, or of the next batch
+                uint32_t next = i + kHeadPairs, next_phase = phase;
+                if (next >= end) {
+                    next = base + pair;
+                    if (++next_phase == phases) next_phase = 0u, next = end + pair;
+                }
+                const bool more = next < n_mine;
+#pragma unroll 1
+                for (uint32_t s0 = 0; s0 < steps; s0 += kHeadDepth) {
+                    const bool last = s0 + kHeadDepth == steps;
+                    if (last && more) rows_of(next, next_phase);
+                    const uint32_t k_next = last ? 0u : s0 + kHeadDepth;
+                    float low[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (uint32_t j = 0; j < kHeadDepth; ++j) {
+                        float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                        uint4 b[3];
+#pragma unroll
+                        for (uint32_t part = 0; part < 3; ++part) {
+                            b[part] = make_uint4(0u, 0u, 0u, 0u);
+                            if (has_b) b[part] = *reinterpret_cast<const uint4 *>(sb + part * part_bytes + (s0 + j) * 64u);
+                        }
+                        mma_bf16(c[0], a0[j].x, a1[j].x, a0[j].y, a1[j].y, b[0].x, b[0].y);
+                        mma_bf16(c[1], a0[j].z, a1[j].z, a0[j].w, a1[j].w, b[0].z, b[0].w);
+#pragma unroll
+                        for (int part = 2; part >= 1; --part) {
+                            mma_bf16(low, a0[j].x, a1[j].x, a0[j].y, a1[j].y, b[part].x, b[part].y);
+                            mma_bf16(low, a0[j].z, a1[j].z, a0[j].w, a1[j].w, b[part].z, b[part].w);
+                        }
+                        if (!last || more) fetch(j, k_next);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            acc[e] += (double)c[0][e];
+                            acc[e] += (double)c[1][e];
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[e] += (double)low[e];
+                }
+                if (half == 1u) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s_half[pair][parity][e][lane] = acc[e];
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(1u + pair) : "memory");
+                if (half == 0u) {
+                    double *const sum = s_sum + (size_t)(i - base) * 128u + lane;   // (this lane's own words)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        acc[e] += s_half[pair][parity][e][lane];
+                        if (phase > 0u) acc[e] += sum[e * 32];
+                        if (phase + 1u < phases) {
+                            sum[e * 32] = acc[e];
+                        } else {
+                            // lane holds rows g, g + 8 of the tile and tokens 2 q, 2 q + 1
+                            const uint32_t row = (blockIdx.x + i * grid) * 16u + g + (e >> 1) * 8u, t = 2u * q + (e & 1);
+                            if (row < n_rows && t < n_tokens) out[(size_t)t * out_stride + row] = (float)acc[e];
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Any hidden size that is a multiple of 8: a warp per row; 8 products in F32, carried in F64.
+template <int NT>
+__global__ void __launch_bounds__(256)
+k_head_logits(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
+              uint32_t out_stride) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t v = warp; v < n_rows; v += n_warps) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(w + (size_t)v * hidden);
+        double acc[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = 0.0;
+        for (uint32_t p = lane; p < (hidden >> 3); p += 32u) {
+            const uint4 q = ldg_stream(row + p);
+            const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
+            float wf[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                wf[i * 2] = __uint_as_float(wd[i] << 16);
+                wf[i * 2 + 1] = __uint_as_float(wd[i] & 0xffff0000u);
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8));
+                const float4 xb = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8 + 4));
+                float2 part = make_float2(0.f, 0.f);
+                part = __ffma2_rn(make_float2(wf[0], wf[1]), make_float2(xa.x, xa.y), part);
+                part = __ffma2_rn(make_float2(wf[2], wf[3]), make_float2(xa.z, xa.w), part);
+                part = __ffma2_rn(make_float2(wf[4], wf[5]), make_float2(xb.x, xb.y), part);
+                part = __ffma2_rn(make_float2(wf[6], wf[7]), make_float2(xb.z, xb.w), part);
+                acc[t] += (double)part.x + (double)part.y;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const double s = warp_sum(acc[t]);
+            if (lane == 0) out[(size_t)t * out_stride + v] = (float)s;
+        }
+    }
+}
+
+// ---- greedy token -------------------------------------------------------------------------------
+//
+// Largest logit, lowest id on ties, -1 if there is a NaN.  One CTA reads 517 KB at the rate one SM takes in
+// (13.9 us for 129 280 logits); a cluster of eight shares the reading and hands its candidates over in shared
+// memory, so the call still needs no scratch that calls on several streams would share.  A candidate is
+// (logit as an ordered integer, ~id): the largest one wins; all ones: a NaN.
+constexpr uint32_t kArgmaxCluster = 8, kArgmaxThreads = 512;
+
+__device__ __forceinline__ unsigned long long argmax_key(float v, uint32_t i) {
+    if (v != v) return ~0ull;
+    const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));  // -0 and +0 are equal
+    return ((unsigned long long)((b & 0x80000000u) ? ~b : (b | 0x80000000u)) << 32) | (0xffffffffu - i);
+}
+
+__global__ void __launch_bounds__(kArgmaxThreads)
+k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__restrict__ result) {
+    __shared__ unsigned long long s_warp[kArgmaxThreads / 32], s_cta[kArgmaxCluster];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
+    cudaGridDependencySynchronize();
+    const uint32_t n = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
+    unsigned long long best = 0ull;
+    auto take = [&](float v, uint32_t i) {
+        const unsigned long long k = argmax_key(v, i);
+        best = k > best ? k : best;
+    };
+    if ((reinterpret_cast<uintptr_t>(logits) & 15u) == 0u) {
+        const uint32_t n4 = vocab >> 2;
+#pragma unroll 4
+        for (uint32_t i = rank * kArgmaxThreads + tid; i < n4; i += n * kArgmaxThreads) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(logits) + i);
+            take(v.x, 4u * i), take(v.y, 4u * i + 1u), take(v.z, 4u * i + 2u), take(v.w, 4u * i + 3u);
+        }
+        if (rank == 0u && tid < (vocab & 3u)) take(logits[n4 * 4u + tid], n4 * 4u + tid);
+    } else {
+        for (uint32_t i = rank * kArgmaxThreads + tid; i < vocab; i += n * kArgmaxThreads) take(__ldcg(logits + i), i);
+    }
+    auto warp_max = [](unsigned long long k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, k, o);
+            k = other > k ? other : k;
+        }
+        return k;
+    };
+    best = warp_max(best);
+    if ((tid & 31u) == 0u) s_warp[tid >> 5] = best;
+    __syncthreads();
+    if (tid < 32u) {
+        best = warp_max(tid < kArgmaxThreads / 32u ? s_warp[tid] : 0ull);
+        if (tid == 0u) *cluster.map_shared_rank(&s_cta[rank], 0) = best;
+    }
+    cluster.sync();
+    if (rank == 0u && tid == 0u) {
+        for (uint32_t r = 0; r < n; ++r) best = s_cta[r] > best ? s_cta[r] : best;
+        *result = best == ~0ull ? -1ll : (int64_t)(0xffffffffu - (uint32_t)best);
+    }
+}
+
+// ---- the steps before the logits ----------------------------------------------------------------
+//
+// final_head.py:43-110: hyper-connection reduce of the four BF16 streams, RMSNorm, and the BF16 values as F32
+// (the logits kernel's input), one launch of one cluster instead of four: the 64 KB of a token's state and
+// matrix are split over eight SMs, the sums cross in shared memory.  The arithmetic is that of the operators
+// s14_cmd_hc_head_reduce and s14_cmd_rms_norm: long sums in double, the rest F32 in the expressions' order,
+// the reduced and the normalised vector rounded to BF16.
+constexpr uint32_t kPrepCluster = 8, kPrepThreads = 256;
+
+__device__ __forceinline__ float bf16_of(const uint16_t *p) { return __uint_as_float((uint32_t)__ldg(p) << 16); }
+
+__global__ void __launch_bounds__(kPrepThreads)
+k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, const float *__restrict__ scale,
+            const float *__restrict__ base, const float *__restrict__ norm_weight, uint32_t hidden, float norm_eps, float hc_eps,
+            float *__restrict__ x_out) {
+    __shared__ double s_red[kPrepThreads / 32][5];
+    __shared__ double s_sums[kPrepCluster][5];   // four dot products and the sum of squares of every CTA's share
+    __shared__ double s_ss[kPrepCluster];
+    __shared__ float s_pre[4];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
+    cudaGridDependencySynchronize();
+    const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t n = 4u * hidden, share = n / kPrepCluster;   // a multiple of 128
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (uint32_t i = tid * 4u; i < share; i += kPrepThreads * 4u) {
+        const uint32_t k = rank * share + i;
+        const uint2 b = __ldg(reinterpret_cast<const uint2 *>(state + k));
+        const float xs[4] = {__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xffff0000u), __uint_as_float(b.y << 16),
+                             __uint_as_float(b.y & 0xffff0000u)};
+        float4 f[4];
+#pragma unroll
+        for (uint32_t m = 0; m < 4; ++m) f[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)m * n + k));
+#pragma unroll
+        for (uint32_t m = 0; m < 4; ++m) {
+            v[m] += (double)xs[0] * (double)f[m].x;
+            v[m] += (double)xs[1] * (double)f[m].y;
+            v[m] += (double)xs[2] * (double)f[m].z;
+            v[m] += (double)xs[3] * (double)f[m].w;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) v[4] += (double)xs[e] * (double)xs[e];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 5; ++j) {
+        v[j] = warp_sum(v[j]);
+        if (lane == 0u) s_red[warp][j] = v[j];
+    }
+    __syncthreads();
+    if (tid < 5u) {
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t wi = 0; wi < kPrepThreads / 32u; ++wi) s += s_red[wi][tid];
+#pragma unroll
+        for (uint32_t r = 0; r < kPrepCluster; ++r) *cluster.map_shared_rank(&s_sums[rank][tid], r) = s;
+    }
+    cluster.sync();
+    if (tid < 4u) {
+        double dot = 0.0, ss = 0.0;
+#pragma unroll
+        for (uint32_t r = 0; r < kPrepCluster; ++r) dot += s_sums[r][tid], ss += s_sums[r][4];
+        const float rs = (float)(1.0 / sqrt((double)__fadd_rn((float)(ss / (double)n), norm_eps)));
+        const float mix = __fmul_rn((float)dot, rs);
+        s_pre[tid] = __fadd_rn((float)(1.0 / (1.0 + exp(-(double)__fadd_rn(__fmul_rn(mix, scale[0]), base[tid])))), hc_eps);
+    }
+    __syncthreads();
+    // this CTA's eighth of the hidden vector, at most four elements a thread (hidden <= 8192)
+    const uint32_t part = hidden / kPrepCluster;
+    float red[4];
+    double ss = 0.0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t e = tid + i * kPrepThreads, d = rank * part + e;
+        red[i] = 0.0f;
+        if (e < part) {
+            float acc = __fmul_rn(s_pre[0], bf16_of(state + d));
+#pragma unroll
+            for (uint32_t h = 1; h < 4; ++h) acc = __fadd_rn(acc, __fmul_rn(s_pre[h], bf16_of(state + (size_t)h * hidden + d)));
+            red[i] = __bfloat162float(__float2bfloat16_rn(acc));
+            ss += (double)red[i] * (double)red[i];
+        }
+    }
+    ss = warp_sum(ss);
+    __syncthreads();
+    if (lane == 0u) s_red[warp][0] = ss;
+    __syncthreads();
+    if (tid == 0u) {
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t wi = 0; wi < kPrepThreads / 32u; ++wi) s += s_red[wi][0];
+#pragma unroll
+        for (uint32_t r = 0; r < kPrepCluster; ++r) *cluster.map_shared_rank(&s_ss[rank], r) = s;
+    }
+    cluster.sync();
+    double all = 0.0;
+#pragma unroll
+    for (uint32_t r = 0; r < kPrepCluster; ++r) all += s_ss[r];
+    const float rs = (float)(1.0 / sqrt((double)__fadd_rn((float)(all / (double)hidden), norm_eps)));
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t e = tid + i * kPrepThreads, d = rank * part + e;
+        if (e < part) x_out[d] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__ldg(norm_weight + d), __fmul_rn(red[i], rs))));
+    }
+}
+
+// The largest dynamic shared memory k_head_mma may ask for on the current device (0: could not be set).
+size_t head_smem_limit() {
+    static size_t limit[64] = {};
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (!limit[dev]) {
+        cudaFuncAttributes fa;
+        int optin = 0;
+        if (cudaFuncGetAttributes(&fa, k_head_mma) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+            return 0;
+        const size_t most = (size_t)optin - fa.sharedSizeBytes;
+        if (cudaFuncSetAttribute(k_head_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
+        limit[dev] = most;
+    }
+    return limit[dev];
+}
+
+}  // namespace
+
+cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, uint32_t n_tokens, const uint16_t *w, uint32_t n_rows,
+                               uint32_t hidden, float *out, uint32_t out_stride) {
+    // the tensor-core kernel: phases of K in whole groups of steps per half row, as few as keep the parts small;
+    // sizes that have none take the register kernel
+    for (uint32_t phases = 1; phases <= 8u; phases *= 2u) {
+        const size_t parts = 3u * (size_t)n_tokens * (hidden / phases * 2u + kHeadPad);
+        const size_t smem = parts + (phases > 1u ? kHeadTiles * 1024u : 0u);
+        if (hidden % (256u * phases) != 0u || smem > head_smem_limit()) continue;
+        if (parts > kHeadPartBytes && hidden % (512u * phases) == 0u && phases < 8u) continue;
+        const uint32_t tiles = (n_rows + 15u) / 16u;
+        const uint32_t ctas = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
+        return launch_pdl(k_head_mma, dim3(ctas), dim3(kHeadThreads), smem, st, 0u, x, w, out, n_rows, hidden, out_stride, n_tokens,
+                          phases);
+    }
+    const uint32_t blocks = std::min((n_rows + 7u) / 8u, (uint32_t)sm_count * 8u);
+    switch (n_tokens) {
+    case 1: k_head_logits<1><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 2: k_head_logits<2><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 3: k_head_logits<3><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 4: k_head_logits<4><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 5: k_head_logits<5><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 6: k_head_logits<6><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    case 7: k_head_logits<7><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    default: k_head_logits<8><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_greedy_argmax(cudaStream_t st, const float *logits, uint32_t vocab, int64_t *result) {
+    return launch_pdl(k_greedy_argmax, dim3(kArgmaxCluster), dim3(kArgmaxThreads), 0, st, kArgmaxCluster, logits, vocab, result);
+}
+
+cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float *fn, const float *scale, const float *base,
+                             const float *norm_weight, uint32_t hidden, float norm_eps, float hc_eps, float *x_out) {
+    return launch_pdl(k_head_prep, dim3(kPrepCluster), dim3(kPrepThreads), 0, st, kPrepCluster, state, fn, scale, base, norm_weight,
+                      hidden, norm_eps, hc_eps, x_out);
+}
+
+}  // namespace s14

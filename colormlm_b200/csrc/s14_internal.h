@@ -162,6 +162,10 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
                                uint32_t out_stride);
 cudaError_t launch_greedy_argmax(cudaStream_t st, const float *logits, uint32_t vocab,
                                  int64_t *result);
+// The head's reduce of a BF16 state, RMSNorm, and the BF16 result as F32 values (x_out [hidden]); hidden a multiple of
+// 256 up to 8192.
+cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float *fn, const float *scale, const float *base,
+                             const float *norm_weight, uint32_t hidden, float norm_eps, float hc_eps, float *x_out);
 
 // ---- a block of tokens through one layer, grouped by expert (s14_moe_block.cu) ----
 constexpr uint32_t kBlockNt = 12;  // most tokens of one chunk (two MMAs of N = 96: sixteen digit rows per token)

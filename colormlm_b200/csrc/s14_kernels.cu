@@ -825,131 +825,6 @@ k_router(const float *__restrict__ x, const uint16_t *__restrict__ wr, const flo
     if (threadIdx.x == 0) *counter = 0u;  // ready for the next launch
 }
 
-// --------------------------------------------------------------- LM head ----
-
-// logits[t, v] = sum_k x[t,k] * bf16(W[v,k]); warp per vocabulary row; 8 products
-// in F32, carried in F64.
-template <int NT>
-__global__ void __launch_bounds__(256)
-k_head_logits(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out,
-              uint32_t n_rows, uint32_t hidden, uint32_t out_stride) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t v = warp; v < n_rows; v += n_warps) {
-        const uint4 *row = reinterpret_cast<const uint4 *>(w + (size_t)v * hidden);
-        double acc[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = 0.0;
-        // four 16-byte loads of the row in flight per lane (the row is read once, from HBM); the sums
-        // are taken in the order of the chunks, as before
-        for (uint32_t p0 = lane; p0 < (hidden >> 3); p0 += 128u) {
-            uint4 q4[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                q4[u] = (p0 + 32u * u < (hidden >> 3)) ? ldg_stream(row + p0 + 32u * u) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t p = p0 + 32u * u;
-                if (p >= (hidden >> 3)) break;
-                const uint32_t wd[4] = {q4[u].x, q4[u].y, q4[u].z, q4[u].w};
-                float wf[8];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    wf[i * 2] = __uint_as_float(wd[i] << 16);
-                    wf[i * 2 + 1] = __uint_as_float(wd[i] & 0xffff0000u);
-                }
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8));
-                    const float4 xb = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8 + 4));
-                    float2 part = make_float2(0.f, 0.f);
-                    part = __ffma2_rn(make_float2(wf[0], wf[1]), make_float2(xa.x, xa.y), part);
-                    part = __ffma2_rn(make_float2(wf[2], wf[3]), make_float2(xa.z, xa.w), part);
-                    part = __ffma2_rn(make_float2(wf[4], wf[5]), make_float2(xb.x, xb.y), part);
-                    part = __ffma2_rn(make_float2(wf[6], wf[7]), make_float2(xb.z, xb.w), part);
-                    acc[t] += (double)part.x + (double)part.y;
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            const double s = warp_sum(acc[t]);
-            if (lane == 0) out[(size_t)t * out_stride + v] = (float)s;
-        }
-    }
-}
-
-// greedy argmax, lowest id wins ties, NaN -> -1; single block.
-__global__ void __launch_bounds__(1024)
-k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__restrict__ result) {
-    __shared__ float sv[32];
-    __shared__ uint32_t si[32];
-    __shared__ int snan;
-    if (threadIdx.x == 0) snan = 0;
-    __syncthreads();
-    float best = -INFINITY;
-    uint32_t best_i = 0xffffffffu;
-    bool nan = false;
-    // four logits per load where the array allows it (a thread meets its indices in ascending order, so
-    // "first largest" stays "lowest index" within a thread)
-    const bool vec = (vocab & 3u) == 0u && (reinterpret_cast<uintptr_t>(logits) & 15u) == 0u;
-    if (vec) {
-        for (uint32_t i = threadIdx.x * 4u; i < vocab; i += blockDim.x * 4u) {
-            const float4 q = *reinterpret_cast<const float4 *>(logits + i);
-            const float vs[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                const float v = vs[k];
-                nan |= (v != v);
-                if (best_i == 0xffffffffu || v > best) {
-                    best = v;
-                    best_i = i + k;
-                }
-            }
-        }
-    } else {
-        for (uint32_t i = threadIdx.x; i < vocab; i += blockDim.x) {
-            const float v = logits[i];
-            nan |= (v != v);
-            if (best_i == 0xffffffffu || v > best) {
-                best = v;
-                best_i = i;
-            }
-        }
-    }
-    if (nan) snan = 1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const uint32_t oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-        if (oi != 0xffffffffu && (best_i == 0xffffffffu || ob > best || (ob == best && oi < best_i))) {
-            best = ob;
-            best_i = oi;
-        }
-    }
-    if ((threadIdx.x & 31u) == 0) {
-        sv[threadIdx.x >> 5] = best;
-        si[threadIdx.x >> 5] = best_i;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        best = sv[threadIdx.x];
-        best_i = si[threadIdx.x];
-        if (threadIdx.x >= (blockDim.x >> 5)) best_i = 0xffffffffu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const uint32_t oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-            if (oi != 0xffffffffu && (best_i == 0xffffffffu || ob > best || (ob == best && oi < best_i))) {
-                best = ob;
-                best_i = oi;
-            }
-        }
-        if (threadIdx.x == 0) *result = snan ? -1 : (int64_t)best_i;
-    }
-}
-
 // ------------------------------------------------------------- launchers ----
 
 static inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
@@ -1422,29 +1297,6 @@ cudaError_t launch_stack_step(cudaStream_t st, const float *x, const float *y, f
 cudaError_t launch_mix_slots(cudaStream_t st, const float *slots, const float *weights, uint32_t n_routed,
                              int has_shared, float *y, uint32_t hidden) {
     k_mix_slots<<<ceil_div(hidden, 256), 256, 0, st>>>(slots, weights, n_routed, has_shared, y, hidden);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, uint32_t n_tokens,
-                               const uint16_t *w, uint32_t n_rows, uint32_t hidden, float *out,
-                               uint32_t out_stride) {
-    const uint32_t blocks = min(ceil_div(n_rows, 8), (uint32_t)sm_count * 8u);
-    switch (n_tokens) {
-    case 1: k_head_logits<1><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 2: k_head_logits<2><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 3: k_head_logits<3><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 4: k_head_logits<4><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 5: k_head_logits<5><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 6: k_head_logits<6><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    case 7: k_head_logits<7><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    default: k_head_logits<8><<<blocks, 256, 0, st>>>(x, w, out, n_rows, hidden, out_stride); break;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_greedy_argmax(cudaStream_t st, const float *logits, uint32_t vocab,
-                                 int64_t *result) {
-    k_greedy_argmax<<<1, 1024, 0, st>>>(logits, vocab, result);
     return cudaGetLastError();
 }
 

@@ -1260,7 +1260,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
 }
 
 template <class Kernel, class... Args>
-cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, Args... args) {
+cudaError_t launch_layer(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -1360,10 +1360,10 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     // launches; the kernel's own dependency calls are then no-ops.
     const bool pdl = ex.world <= 1u && y != nullptr;
     if (trace)
-        return launch_pdl(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
+        return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
                           counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
                           residual ? 1u : 0u);
-    return launch_pdl(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
+    return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
                       counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
                       residual ? 1u : 0u);
 }

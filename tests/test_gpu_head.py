@@ -1,0 +1,92 @@
+"""The LM head's kernels at the edges of their tiles (GPU): logits against a float64 product, the greedy token
+against numpy, the fused steps before the logits against the operators they are made of."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from colormlm_b200.s14 import S14Context
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("cuda_lib")]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    c = S14Context(0)
+    yield c
+    c.close()
+
+
+# rows: less than a tile, tiles with a remainder, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in
+# phases); hidden: one group of steps, several phases, a size the tensor-core kernel leaves to the other one (264)
+@pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (2, 17, 1280), (3, 2385, 4096), (5, 33, 264),
+                                                (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096)])
+def test_logits_at_the_edges_of_the_tiles(ctx, tokens, rows, hidden):
+    g = torch.Generator(device="cuda").manual_seed(tokens * rows + hidden)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g)
+    w = torch.empty(rows, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g)
+    out = torch.full((tokens, rows + 3), 7.0, device="cuda")
+    ctx.cmd_head_logits(x, w.view(torch.int16), out, n_rows=rows)
+    for r0 in range(0, rows, 16384):
+        wd = w[r0:r0 + 16384].double()
+        ref, mag = x.double() @ wd.T, x.double().abs() @ wd.T.abs()
+        # exact products; a sum of sixteen loses at most three units of 2^-23 of its terms' magnitudes on its way into
+        # double, the result one of 2^-24
+        assert bool(((out[:, r0:min(r0 + 16384, rows)].double() - ref).abs() <= 4 * 2.0 ** -23 * mag).all())
+    assert bool((out[:, rows:] == 7.0).all())
+
+
+def test_logits_of_infinite_and_largest_values(ctx):
+    x = torch.zeros(2, 512, device="cuda")
+    x[0, 5], x[1, 300] = float("inf"), 3.4028e38
+    w = torch.ones(40, 512, dtype=torch.bfloat16, device="cuda") * 0.5
+    out = torch.empty(2, 40, device="cuda")
+    ctx.cmd_head_logits(x, w.view(torch.int16), out)
+    assert bool((out[0] == float("inf")).all())
+    assert bool((out[1] == x[1, 300] * 0.5).all())
+
+
+@pytest.mark.parametrize("vocab,offset", [(1, 0), (3, 0), (2047, 1), (4096, 0), (16385, 0), (129280, 0), (129281, 3)])
+def test_greedy_token(ctx, vocab, offset):
+    g = np.random.default_rng(vocab)
+    full = torch.empty(vocab + offset, device="cuda")
+    res = torch.empty(1, dtype=torch.int64, device="cuda")
+
+    def token(v):
+        full[offset:] = torch.from_numpy(v).cuda()
+        ctx.cmd_greedy_argmax(full[offset:], res)
+        return int(res.item())
+
+    v = g.standard_normal(vocab).astype(np.float32)
+    assert token(v) == int(v.argmax())
+    hits = np.unique(g.integers(0, vocab, 3))  # the lowest id of the largest value, wherever the others lie
+    v[hits] = 9.0
+    assert token(v) == int(hits[0])
+    v = -np.abs(v) * 0.0
+    v[vocab - 1] = 0.0  # -0 and +0 are equal
+    assert token(v) == 0
+    assert token(np.full(vocab, -np.inf, np.float32)) == 0
+    v[vocab // 2] = np.nan
+    assert token(v) == -1
+
+
+@pytest.mark.parametrize("hidden", [256, 1024, 2304, 4096])
+def test_full_logits_equal_their_operators(ctx, hidden):
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    state = torch.randn(1, 4, hidden, device="cuda", generator=g).to(torch.bfloat16)
+    fn, base = torch.randn(4, 4 * hidden, device="cuda", generator=g) * 0.02, torch.rand(4, device="cuda", generator=g) - 0.5
+    scale, norm = torch.rand(1, device="cuda", generator=g), torch.rand(hidden, device="cuda", generator=g) + 0.5
+    w = (torch.randn(100, hidden, device="cuda", generator=g) * 0.02).to(torch.bfloat16).view(torch.int16)
+    out, want = torch.empty(100, device="cuda"), torch.empty(100, device="cuda")
+    red, pre = torch.empty(1, hidden, dtype=torch.bfloat16, device="cuda"), torch.empty(1, 4, device="cuda")
+    normed = torch.empty_like(red)
+    ctx.exec_hc_head_norm_full_logits(state, fn, scale, base, norm, w, out)
+    ctx.cmd_hc_head_reduce(state, fn, scale, base, red, pre)
+    ctx.cmd_rms_norm(red, norm, normed)
+    ctx.cmd_head_logits(normed.float(), w, want)
+    # the double sums run in another order: a coefficient may round the other way, which moves an element of the
+    # reduced vector by at most one BF16 unit (2^-8 relative) and so a logit by 2^-8 |x| |w|
+    mag = normed.float().abs()[0] @ w.view(torch.bfloat16).float().abs().T
+    assert bool(((out - want).abs() <= 2.0 ** -8 * mag).all())
