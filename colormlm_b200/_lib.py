@@ -20,7 +20,7 @@ MAX_BLOCK_TOKENS = 8
 PAGE_MXFP4, PAGE_FP8 = 0, 1
 ACCUM_PAIRWISE, ACCUM_REFERENCE = 0, 1
 LAYER_PATH_TENSOR, LAYER_PATH_TENSOR_PER_TOKEN, LAYER_PATH_TENSOR_STACK, LAYER_PATH_F32, LAYER_PATH_REFERENCE = 1, 2, 3, 4, 5
-LAYER_PATH_ROUTER_KERNEL = 0x100
+LAYER_PATH_ROUTER_KERNEL, LAYER_PATH_FP8_SHARED_KERNEL = 0x100, 0x200
 LAYER_PATH_TENSOR_BLOCK = 6
 STREAM_F32, STREAM_BF16 = 0, 1
 EP_SHARED_BY_TOKEN = 0xFFFFFFFF

@@ -100,7 +100,6 @@ struct s14_ctx {
         uint32_t wait_limit = 1u << 22;  // polls of about a microsecond: a few seconds
     } ep;
     float *glue = nullptr;    // [kGlueTokens, 25] dot products and mean squares of the hyper-connection calls
-    uint16_t *glue16 = nullptr;  // [8192] a BF16 vector between the steps of an executor call
     UmmaScratch umma{nullptr, nullptr, nullptr};  // scratch of the tcgen05 layer kernel
     bool use_umma = true;                // S14_TENSOR_PATH=off in the environment turns it off
     const UmmaScratch *umma_scratch() const { return use_umma ? &umma : nullptr; }
@@ -134,7 +133,6 @@ extern "C" int32_t s14_ctx_create(int32_t device, s14_ctx **out) {
     CUDA_OK(cudaMalloc(&ctx->select, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->dev_table, sizeof(JobTable)));
     CUDA_OK(cudaMalloc(&ctx->glue, sizeof(float) * kGlueTokens * 25));
-    CUDA_OK(cudaMalloc(&ctx->glue16, sizeof(uint16_t) * 8192));
     CUDA_OK(cudaMalloc(&ctx->x_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->y_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->status, sizeof(uint32_t)));
@@ -174,7 +172,6 @@ extern "C" int32_t s14_ctx_destroy(s14_ctx *ctx) {
     cudaFree(ctx->scores);
     cudaFree(ctx->select);
     cudaFree(ctx->glue);
-    cudaFree(ctx->glue16);
     cudaFree(ctx->dev_table);
     cudaFree(ctx->x_stage);
     cudaFree(ctx->y_stage);
@@ -610,8 +607,8 @@ static void build_job_table(const s14_moe_layer_desc &desc, JobTable &tab) {
     tab.token_job_begin[desc.n_tokens] = pos;
 }
 
-static int32_t enqueue_layer(s14_ctx *ctx, cudaStream_t st, const s14_moe_layer_desc &desc,
-                             const float *x, float *y) {
+static int32_t enqueue_layer(s14_ctx *ctx, cudaStream_t st, const s14_moe_layer_desc &desc, const float *x, float *y,
+                             const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr) {
     S14_TRY
     JobTable tab;
     build_job_table(desc, tab);
@@ -622,7 +619,8 @@ static int32_t enqueue_layer(s14_ctx *ctx, cudaStream_t st, const s14_moe_layer_
     for (uint32_t j = 0; j < tab.n_jobs; ++j) all_mxfp4 = all_mxfp4 && tab.jobs[j].kind == S14_PAGE_MXFP4;
     const int launched = launch_moe_layer(st, ctx->mode, ctx->sm_count, nullptr, tab, tab.n_tokens,
                                           tab.n_jobs, desc.hidden, desc.inter, x, ctx->h, ctx->d, y,
-                                          &err, nullptr, all_mxfp4, ctx->counters, ctx->umma_scratch());
+                                          &err, nullptr, all_mxfp4, ctx->counters, ctx->umma_scratch(), nullptr, nullptr, x_bf16,
+                                          x_stage);
     ctx->last_path = last_layer_path();
     ctx->launches += launched;
     if (err != cudaSuccess) return cuda_fail(err, "S14 MoE layer launch");
@@ -975,8 +973,26 @@ extern "C" int32_t s14_cmd_stack_decode(s14_ctx *ctx, void *stream, s14_stack *s
         if (err != cudaSuccess) return cuda_fail(err, "S14 stack launch");
         return S14_OK;
     }
-    // the layers one by one: router and layer kernels into ybuf, then the step to the next token
     const float *cur = x;
+    if (has_shared && c.shared_kind == S14_PAGE_FP8 && umma_router_ok(ctx->sm_count, c.n_experts) &&
+        fp8_shared_layer_ok(ctx->sm_count, ctx->mode, ctx->umma_scratch(), c.top_k, c.hidden, c.inter)) {
+        // FP8 shared experts: three launches per layer, the layer kernel hands the next token over itself
+        for (uint32_t l = 0; l < c.n_layers; ++l) {
+            FusedRouter fr = stack_router(ctx, stack, l);
+            fr.shared_page = nullptr;
+            fr.y_out = stack->layers[l].y_out;
+            float *next = (l + 1 == c.n_layers) ? h_out : stack->hbuf + (size_t)((l + 1) & 1u) * c.hidden;
+            cudaError_t err;
+            ctx->launches += launch_layer_fp8_shared(st, ctx->sm_count, unused, &fr, stack->layers[l].shared_page, cur, nullptr, nullptr,
+                                                     ctx->h, ctx->d, next, ctx->counters, ctx->umma_scratch(), c.hidden, c.inter,
+                                                     c.residual != 0, &err);
+            ctx->last_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
+            if (err != cudaSuccess) return cuda_fail(err, "S14 stack layer launch");
+            cur = next;
+        }
+        return S14_OK;
+    }
+    // the layers one by one: router and layer kernels into ybuf, then the step to the next token
     for (uint32_t l = 0; l < c.n_layers; ++l) {
         const FusedRouter fr = stack_router(ctx, stack, l);
         cudaError_t err;
@@ -2303,7 +2319,6 @@ extern "C" int32_t s14_exec_routed_and_shared_moe_then_hc_post(s14_ctx *ctx, voi
         throw ContractError("s14_exec_routed_and_shared_moe_then_hc_post: hidden and intermediate must be 1024, 2048 or 4096");
     CUDA_OK(cudaSetDevice(ctx->device));
     cudaStream_t st = stream_of(ctx, stream);
-    CUDA_OK(launch_bf16_to_f32(st, d->ffn_input_bf16, ctx->x_stage, d->hidden));
     s14_moe_layer_desc ld = {};
     ld.hidden = d->hidden;
     ld.inter = d->inter;
@@ -2311,12 +2326,11 @@ extern "C" int32_t s14_exec_routed_and_shared_moe_then_hc_post(s14_ctx *ctx, voi
     ld.shared_kind = d->shared_kind;
     ld.shared_page = d->shared_page;
     ld.routes = d->route;
-    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->y_stage);
+    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->y_stage, d->ffn_input_bf16, ctx->x_stage);
     if (rc != S14_OK) return rc;
-    uint16_t *branch = d->moe_branch_out_bf16 ? d->moe_branch_out_bf16 : ctx->glue16;
-    CUDA_OK(launch_f32_to_bf16(st, ctx->y_stage, branch, d->hidden));
-    CUDA_OK(launch_hc_post(st, true, 1, d->hidden, branch, d->residual_bf16, d->post, d->comb, d->state_out_bf16));
-    ctx->launches += 3;
+    CUDA_OK(launch_branch_post(st, d->hidden, ctx->y_stage, d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb,
+                               d->state_out_bf16));
+    ctx->launches += 1;
     return S14_OK;
     S14_CATCH
 }

@@ -233,9 +233,33 @@ __global__ void __launch_bounds__(256) k_bf16_to_f32(const uint16_t *__restrict_
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i < n) out[i] = __uint_as_float((uint32_t)__ldg(in + i) << 16);
 }
-__global__ void __launch_bounds__(256) k_f32_to_bf16(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out, uint32_t n) {
-    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
-    if (i < n) out[i] = __float2bfloat16_rn(__ldg(in + i));
+// The end of the executor's expert step: the branch rounded to BF16 (left in branch_out if the caller wants it)
+// and expanded into the four streams as k_hc_post does.  One token.
+__global__ void __launch_bounds__(256)
+k_branch_post(const float *__restrict__ y, uint16_t *__restrict__ branch_out, const void *__restrict__ residual,
+              const float *__restrict__ post, const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
+    const uint32_t d = blockIdx.x * 256u + threadIdx.x;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (d >= hidden) return;
+    float r[kHc], c[kHc * kHc], p[kHc];
+#pragma unroll
+    for (uint32_t h = 0; h < kHc; ++h) {
+        r[h] = stream_ld<true>(residual, (size_t)h * hidden + d);
+        p[h] = __ldg(post + h);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldg(comb + i);
+    const __nv_bfloat16 b16 = __float2bfloat16_rn(__ldcg(y + d));
+    if (branch_out) branch_out[d] = *reinterpret_cast<const uint16_t *>(&b16);
+    const float b = __bfloat162float(b16);
+#pragma unroll
+    for (uint32_t o = 0; o < kHc; ++o) {
+        float s = __fmul_rn(c[o], r[0]);
+#pragma unroll
+        for (uint32_t h = 1; h < kHc; ++h) s = __fadd_rn(s, __fmul_rn(c[h * kHc + o], r[h]));
+        stream_st<true>(merged, (size_t)o * hidden + d, __fadd_rn(__fmul_rn(p[o], b), s));
+    }
 }
 
 }  // namespace
@@ -244,9 +268,10 @@ cudaError_t launch_bf16_to_f32(cudaStream_t st, const uint16_t *in, float *out, 
     k_bf16_to_f32<<<(n + 255u) / 256u, 256, 0, st>>>(in, out, n);
     return cudaGetLastError();
 }
-cudaError_t launch_f32_to_bf16(cudaStream_t st, const float *in, uint16_t *out, uint32_t n) {
-    k_f32_to_bf16<<<(n + 255u) / 256u, 256, 0, st>>>(in, reinterpret_cast<__nv_bfloat16 *>(out), n);
-    return cudaGetLastError();
+cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y, uint16_t *branch_out, const void *residual,
+                               const float *post, const float *comb, void *merged) {
+    return launch_pdl(k_branch_post, dim3((hidden + 255u) / 256u), dim3(256), 0, st, 0u, y, branch_out, residual, post, comb, hidden,
+                      merged);
 }
 
 // dots: [n_tokens, 24] scratch, mean_sq: [n_tokens] scratch.  Returns the number of kernels launched.

@@ -84,6 +84,7 @@ struct FusedRouter {
     uint32_t shared_kind;
     uint32_t ep_rank, ep_world, shared_owner;
     uint32_t has_shared;               // every layer has a shared expert (a stack's layers say where)
+    float *y_out;                      // a single layer: its output before the residual [hidden], or NULL
 };
 
 // What one layer of a decode stack brings of its own (device memory, constant during a step): the
@@ -119,7 +120,22 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                      uint32_t hidden, uint32_t inter, const float *x, float *h, float *d, float *y,
                      cudaError_t *err, const KernelMarks *km = nullptr, bool all_mxfp4 = false,
                      unsigned int *counters = nullptr, const struct UmmaScratch *umma = nullptr,
-                     const FusedRouter *router = nullptr, const EpExchange *ep = nullptr);
+                     const FusedRouter *router = nullptr, const EpExchange *ep = nullptr,
+                     const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr);
+// (x_bf16, x_stage: the token as BF16; its F32 values are written to x_stage, which is x)
+// Whether a one-token layer with an FP8 shared page runs it by kernels of its own in front of the tensor-core layer
+// kernel, which runs the routed experts and adds the shared expert's output last.
+bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const struct UmmaScratch *umma, uint32_t n_routed, uint32_t hidden, uint32_t inter);
+// That layer (three launches): the routed experts' jobs, or a router without the shared expert.  h: [inter], d:
+// [kMaxJobs, hidden] scratch.  With `residual` y = x + moe(x).
+int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
+                            const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
+                            unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, bool residual,
+                            cudaError_t *err);
+// One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or x_bf16 with its F32 values left in x_out;
+// h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096.
+cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,
+                              float *h, float *d, uint32_t hidden, uint32_t inter);
 // Scratch of the tcgen05 layer kernel (s14_moe_umma.cu): per job the digit tile of its hidden
 // values and the tile's block exponents (umma_scratch_bytes), and the device status word a
 // timed-out wait sets.
@@ -140,13 +156,15 @@ bool umma_router_ok(int sm_count, uint32_t n_experts);
 __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT,
                                              uint32_t KU, uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early);
 // Both phases and the mix in one launch (y == nullptr: the expert outputs go to d, the caller mixes).
-// With a router the kernel computes the routes itself and the job tables are not read.
+// With a router the kernel computes the routes itself and the job tables are not read.  add_last [hidden]: a
+// vector that an earlier launch left, added to the mix after the jobs (a shared expert that is not one of them).
 cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable *dev, const JobTable &param,
                                   const float *x, float *d, float *y, uint8_t *tiles, unsigned int *counters,
                                   uint32_t *status, uint32_t hidden, uint32_t inter,
                                   const FusedRouter *router = nullptr, const EpExchange *ep = nullptr,
                                   unsigned long long *trace = nullptr, const StackLayer *stack = nullptr,
-                                  uint32_t n_layers = 1, float *hbuf = nullptr, bool residual = false);
+                                  uint32_t n_layers = 1, float *hbuf = nullptr, bool residual = false,
+                                  const float *add_last = nullptr);
 int launch_router(cudaStream_t st, const s14_router_desc &r, float *scores, float *select,
                   JobTable *table_out, const uint8_t *const *page_table, const uint8_t *shared_page,
                   uint32_t shared_kind, unsigned int *counter, cudaError_t *err,
@@ -235,7 +253,9 @@ cudaError_t launch_rms_norm(cudaStream_t st, bool bf16, uint32_t n_tokens, uint3
                             void *out);
 cudaError_t launch_router_hash(cudaStream_t st, const s14_router_desc &r, const int64_t *tid2eid);
 cudaError_t launch_bf16_to_f32(cudaStream_t st, const uint16_t *in, float *out, uint32_t n);
-cudaError_t launch_f32_to_bf16(cudaStream_t st, const float *in, uint16_t *out, uint32_t n);
+// branch = BF16 of y (to branch_out, or NULL), merged = post * branch + comb . residual: one token of BF16 streams.
+cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y, uint16_t *branch_out, const void *residual,
+                               const float *post, const float *comb, void *merged);
 
 }  // namespace s14
 

@@ -953,10 +953,49 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                      const JobTable &param_table, uint32_t n_tokens, uint32_t n_jobs_max,
                      uint32_t hidden, uint32_t inter, const float *x, float *h, float *d, float *y,
                      cudaError_t *err, const KernelMarks *km, bool all_mxfp4, unsigned int *counters,
-                     const UmmaScratch *umma, const FusedRouter *router, const EpExchange *ep) {
+                     const UmmaScratch *umma, const FusedRouter *router, const EpExchange *ep, const uint16_t *x_bf16,
+                     float *x_stage) {
     int launches = 0;
     *err = cudaSuccess;
     t_last_layer_path = 0;
+    if (n_tokens == 1u && y && !ep && !km && counters && (router ? router->ep_world <= 1u : !dev_table)) {
+        // the checkpoint's page kinds: routed MXFP4 experts and an FP8 shared expert
+        JobTable routed = {};
+        const uint8_t *shared = nullptr;
+        uint32_t n_routed = 0;
+        FusedRouter rt = {};
+        if (router) {
+            rt = *router;
+            if (rt.shared_page && rt.shared_kind == S14_PAGE_FP8) shared = rt.shared_page;
+            rt.shared_page = nullptr;
+            n_routed = umma_router_ok(sm_count, rt.n_experts) ? rt.top_k : 0u;
+        } else {
+            routed.n_tokens = 1;
+            for (uint32_t i = param_table.token_job_begin[0]; i < param_table.token_job_begin[1]; ++i) {
+                Job jb = param_table.jobs[param_table.token_jobs[i]];
+                if (jb.is_shared && jb.kind == S14_PAGE_FP8) {
+                    shared = jb.page;
+                    continue;
+                }
+                jb.out_index = n_routed;
+                routed.jobs[n_routed] = jb;
+                routed.token_jobs[n_routed] = (uint8_t)n_routed;
+                ++n_routed;
+            }
+            routed.n_jobs = routed.token_job_begin[1] = n_routed;
+        }
+        if (shared && fp8_shared_layer_ok(sm_count, mode, umma, n_routed, hidden, inter)) {
+            launches = launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
+                                               counters, umma, hidden, inter, false, err);
+            t_last_layer_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
+            return launches;
+        }
+    }
+    if (x_bf16) {
+        *err = launch_bf16_to_f32(st, x_bf16, x_stage, hidden * n_tokens);
+        if (*err != cudaSuccess) return launches;
+        ++launches;
+    }
     const bool tensor_path = mode != S14_ACCUM_REFERENCE && all_mxfp4 && counters && umma &&
                              umma_layer_ok(sm_count, n_tokens, n_jobs_max, hidden, inter);
     if (ep && ep->world > 1u && !(tensor_path && router && umma_router_ok(sm_count, router->n_experts))) {
@@ -1076,6 +1115,23 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
     launches += 1;
     *err = cudaGetLastError();
     return launches;
+}
+
+bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const UmmaScratch *umma, uint32_t n_routed, uint32_t hidden, uint32_t inter) {
+    return mode != S14_ACCUM_REFERENCE && umma && umma_layer_ok(sm_count, 1u, n_routed, hidden, inter) &&
+           (hidden == 1024u || hidden == 2048u || hidden == 4096u) && (inter == 1024u || inter == 2048u || inter == 4096u);
+}
+
+int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
+                            const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
+                            unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, bool residual,
+                            cudaError_t *err) {
+    float *shared_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
+    *err = launch_fp8_expert(st, sm_count, x, x_bf16, x_stage, shared_page, h, shared_out, hidden, inter);
+    if (*err != cudaSuccess) return 0;
+    *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, y, umma->tiles, counters, umma->status, hidden, inter, router,
+                                 nullptr, umma->trace, nullptr, 1, nullptr, residual, shared_out);
+    return 3;
 }
 
 int launch_router(cudaStream_t st, const s14_router_desc &r, float *scores, float *select,

@@ -176,7 +176,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                  unsigned int *counters, uint32_t *__restrict__ status, uint32_t hidden, uint32_t inter,
                  uint32_t ring, unsigned long long *trace, const __grid_constant__ FusedRouter rt,
                  const __grid_constant__ EpExchange ep, const StackLayer *__restrict__ stack, uint32_t n_layers,
-                 float *hbuf, uint32_t residual) {
+                 float *hbuf, uint32_t residual, const float *add_last) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kBars];
     __shared__ __align__(16) uint8_t sE[kExpMax];        // block exponents of the token's digits
@@ -301,6 +301,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
         else if (lane == 3u) v = (unsigned long long)rt.shared_page;
         else if (lane == 4u) v = (unsigned long long)rt.ids_out;
         else if (lane == 5u) v = (unsigned long long)rt.weights_out;
+        else if (lane == 6u) v = (unsigned long long)rt.y_out;
         reinterpret_cast<unsigned long long *>(&s_layer[0])[lane] = v;
     }
     if (warp == 1u) {
@@ -1031,6 +1032,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                                     if (residual)
                                         x_in = l == 0u ? __ldcg(x + n)
                                                        : __uint_as_float((uint32_t)ld_relaxed_gpu(x_words + (size_t)par * kMaxHidden + n));
+                                    const float last = add_last ? __ldcg(add_last + n) : 0.0f;
                                     uint32_t vals[kJobsMax];
                                     uint32_t tries = 0;
                                     bool got = true;
@@ -1064,6 +1066,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                                                 acc = (s_mix_slot[par][jj] >> 31) ? __fadd_rn(acc, dv) : __fadd_rn(acc, __fmul_rn(s_mix_w[par][jj], dv));
                                             }
                                         }
+                                        if (add_last) acc = __fadd_rn(acc, last);
                                         const float out = residual ? __fadd_rn(x_in, acc) : acc;
                                         if (l + 1u == L) y[n] = out;
                                         else st_relaxed_gpu(x_words + (size_t)(par ^ 1u) * kMaxHidden + n, ((unsigned long long)(want + 1u) << 32) | __float_as_uint(out));
@@ -1343,7 +1346,7 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
                                   const float *x, float *d, float *y, uint8_t *tiles, unsigned int *counters,
                                   uint32_t *status, uint32_t hidden, uint32_t inter, const FusedRouter *router,
                                   const EpExchange *ep, unsigned long long *trace, const StackLayer *stack,
-                                  uint32_t n_layers, float *hbuf, bool residual) {
+                                  uint32_t n_layers, float *hbuf, bool residual, const float *add_last) {
     const uint32_t ring = ring_slots(hidden, inter, dynamic_limit());
     if (ring < 2u) return cudaErrorInvalidConfiguration;
     FusedRouter rt = {};
@@ -1352,6 +1355,7 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     EpExchange ex = {};
     if (ep) ex = *ep;
     if (ex.world > 1u && !router) return cudaErrorInvalidValue;  // the mix needs every route's weight
+    if (add_last && (stack || ex.world > 1u || !y)) return cudaErrorInvalidValue;
     if (stack && (!router || n_layers == 0u || n_layers > kMaxLayers || (n_layers > 1u && !hbuf) || ex.world > 1u || rt.ep_world > 1u))
         return cudaErrorInvalidValue;  // a stack routes its own layers on one GPU
     const size_t smem = (size_t)ring * kSlot + umma_fixed_smem(hidden, inter);
@@ -1362,10 +1366,10 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     if (trace)
         return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
                           counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                          residual ? 1u : 0u);
+                          residual ? 1u : 0u, add_last);
     return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
                       counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                      residual ? 1u : 0u);
+                      residual ? 1u : 0u, add_last);
 }
 
 }  // namespace s14

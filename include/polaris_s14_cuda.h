@@ -102,7 +102,8 @@ S14_API uint64_t s14_ctx_launch_count(const s14_ctx *ctx);
 /* Which implementation the context's last MoE layer or stack call ran (the library chooses by
  * accumulation mode, page kinds, token count and sizes; no counterpart in the reference):
  * exactly one of the first five values, ORed with ROUTER_KERNEL if the routes came from a kernel
- * launch of their own instead of being picked inside the layer kernel.  0: no such call yet. */
+ * launch of their own instead of being picked inside the layer kernel, and with FP8_SHARED_KERNEL if the shared
+ * expert ran in kernels of its own.  0: no such call yet. */
 #define S14_LAYER_PATH_TENSOR 1u           /* tcgen05 layer kernel, one launch per layer-token */
 #define S14_LAYER_PATH_TENSOR_PER_TOKEN 2u /* a block of tokens: one launch of it per token */
 #define S14_LAYER_PATH_TENSOR_STACK 3u     /* a whole stack of layers in one launch of it */
@@ -110,6 +111,7 @@ S14_API uint64_t s14_ctx_launch_count(const s14_ctx *ctx);
 #define S14_LAYER_PATH_REFERENCE 5u        /* reference-order kernels */
 #define S14_LAYER_PATH_TENSOR_BLOCK 6u     /* grouped tcgen05 kernels: every expert page streamed once per block */
 #define S14_LAYER_PATH_ROUTER_KERNEL 0x100u
+#define S14_LAYER_PATH_FP8_SHARED_KERNEL 0x200u /* with TENSOR: an FP8 shared expert by two launches in front of it */
 S14_API uint32_t s14_ctx_last_layer_path(const s14_ctx *ctx);
 
 /* Per-kernel timing of s14_cmd_routed_moe_layer for profiling runs: while enabled,

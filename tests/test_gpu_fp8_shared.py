@@ -1,0 +1,88 @@
+"""Layers with the checkpoint's page kinds - routed MXFP4 experts, FP8 shared expert - on the path that runs the
+shared expert by kernels of its own in front of the tensor-core layer kernel (GPU), against the CPU oracle."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from colormlm_b200 import _lib as L
+from colormlm_b200 import synth
+from colormlm_b200.s14 import DecodeStack, S14Context, TokenRoute
+
+from .test_gpu_parity import assert_pairwise_close, dev, dev_page, make_layer
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("cuda_lib")]
+PATH = L.LAYER_PATH_TENSOR | L.LAYER_PATH_FP8_SHARED_KERNEL
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    c = S14Context(0)
+    yield c
+    c.close()
+
+
+# every width of a lane's share of a row; one route and six
+@pytest.mark.parametrize("hidden,inter,routed", [(1024, 4096, 6), (2048, 2048, 1), (4096, 1024, 6)])
+def test_layer_and_executor_step_with_an_fp8_shared_expert(ctx, oracle, hidden, inter, routed):
+    g, pages, shared = make_layer(71 + hidden + routed, hidden, inter, routed, L.PAGE_FP8)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter, L.PAGE_FP8)
+    w = np.asarray([0.4, 0.3, 0.25, 0.2, 0.2, 0.15][:routed], np.float32)
+    route = TokenRoute(list(range(routed)), w, [p.data_ptr() for p in pages_dev])
+    x16 = dev(synth.activations(g, 1, hidden)[0]).to(torch.bfloat16)
+    x = x16.float()
+    want = oracle.moe_layer_acc64(x.cpu().numpy(), pages, w, shared, L.PAGE_FP8, hidden, inter)
+    y = torch.empty(1, hidden, device="cuda")
+    for _ in range(2):
+        ctx.cmd_moe_layer(x[None], y, [route], shared_dev.data_ptr(), L.PAGE_FP8, hidden, inter)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and ctx.last_layer_path == PATH
+        assert_pairwise_close(oracle, y.cpu().numpy()[0], want)
+    residual = dev(synth.hc_streams(g, 1, hidden)[0]).to(torch.bfloat16)
+    post, comb = dev(g.uniform(0.2, 1.8, 4).astype(np.float32)), dev(g.uniform(0.05, 0.6, (4, 4)).astype(np.float32))
+    state, branch = torch.empty_like(residual), torch.empty_like(x16)
+    ctx.exec_routed_and_shared_moe_then_hc_post(x16, residual, post, comb, route, shared_dev.data_ptr(), L.PAGE_FP8, inter, state, branch)
+    assert ctx.last_layer_path == PATH
+    merged = torch.empty_like(residual)
+    ctx.cmd_hc_post(branch[None], residual[None], post[None], comb[None], merged[None])
+    torch.cuda.synchronize()
+    assert torch.equal(branch, y[0].to(torch.bfloat16)) and torch.equal(state, merged)
+
+
+@pytest.mark.parametrize("residual", [True, False])
+def test_stack_with_fp8_shared_experts(ctx, oracle, residual):
+    hidden, inter, n_experts, n_layers = 1024, 1024, 24, 3
+    host, layers, keep = [], [], []
+    for l in range(n_layers):
+        g, pages, shared = make_layer(900 + l, hidden, inter, n_experts, L.PAGE_FP8)
+        wr, bias = synth.router_weight_bf16(g, n_experts, hidden), synth.router_bias(g, n_experts)
+        host.append((pages, shared, wr, bias))
+        pd, sd = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter, L.PAGE_FP8)
+        keep.append((pd, sd))
+        layers.append({"wr": dev(wr.view(np.int16)), "bias": dev(bias), "shared": sd.data_ptr(),
+                       "table": torch.tensor([p.data_ptr() for p in pd], dtype=torch.int64, device="cuda"),
+                       "ids": torch.empty(6, dtype=torch.int32, device="cuda"),
+                       "weights": torch.empty(6, device="cuda"), "y": torch.empty(hidden, device="cuda")})
+    stack = DecodeStack(ctx, layers, inter=inter, shared_kind=L.PAGE_FP8, residual=residual)
+    x = synth.activations(synth.rng(5), 1, hidden)[0] * np.float32(0.25)
+    h = dev(x)
+    try:
+        before = ctx.launch_count
+        stack.cmd_decode(h, h)  # in place
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and ctx.launch_count - before == 3 * n_layers and ctx.last_layer_path == PATH
+        cur = x
+        for (pages, shared, wr, bias), ly in zip(host, layers):
+            rid, rw, _, _ = oracle.router(cur, wr, bias, 0, 6, 1.0)
+            assert np.array_equal(ly["ids"].cpu().numpy(), rid)
+            want = oracle.moe_layer_acc64(cur, [pages[i] for i in rid], rw, shared, L.PAGE_FP8, hidden, inter)
+            # the FP8 rows add the sixteen products of a piece in F32 (two chains of eight: at most nine roundings of
+            # 2^-24 of the terms' magnitudes, 3e-7 RMS of the output), which is what the bound of the F32 paths allows
+            assert_pairwise_close(oracle, ly["y"].cpu().numpy(), want)
+            got = ly["y"].cpu().numpy()
+            cur = (cur + got).astype(np.float32) if residual else got
+        assert np.array_equal(h.cpu().numpy(), cur)
+    finally:
+        stack.close()
