@@ -99,7 +99,7 @@ struct s14_ctx {
         bool connected = false;
         uint32_t wait_limit = 1u << 22;  // polls of about a microsecond: a few seconds
     } ep;
-    float *glue = nullptr;    // [kGlueTokens, 25] dot products and mean squares of the hyper-connection calls
+    double *glue = nullptr;   // partial dot products of the hyper-connection calls (hc_scratch_bytes)
     UmmaScratch umma{nullptr, nullptr, nullptr};  // scratch of the tcgen05 layer kernel
     bool use_umma = true;                // S14_TENSOR_PATH=off in the environment turns it off
     const UmmaScratch *umma_scratch() const { return use_umma ? &umma : nullptr; }
@@ -132,7 +132,7 @@ extern "C" int32_t s14_ctx_create(int32_t device, s14_ctx **out) {
     CUDA_OK(cudaMalloc(&ctx->scores, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->select, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->dev_table, sizeof(JobTable)));
-    CUDA_OK(cudaMalloc(&ctx->glue, sizeof(float) * kGlueTokens * 25));
+    CUDA_OK(cudaMalloc(&ctx->glue, hc_scratch_bytes(kGlueTokens)));
     CUDA_OK(cudaMalloc(&ctx->x_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->y_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->status, sizeof(uint32_t)));
@@ -2240,8 +2240,8 @@ static int32_t hc_reduce_call(s14_ctx *ctx, void *stream, const s14_hc_params *p
     CUDA_OK(cudaSetDevice(ctx->device));
     cudaError_t err;
     ctx->launches += launch_hc_pre(stream_of(ctx, stream), p->dtype == S14_STREAM_BF16, head, p->n_tokens, p->hidden, x, p->hc_fn,
-                                   p->hc_scale, p->hc_base, p->norm_eps, p->sinkhorn_iters, p->hc_eps, ctx->glue,
-                                   ctx->glue + (size_t)kGlueTokens * 24, reduced, post, comb, pre, &err);
+                                   p->hc_scale, p->hc_base, p->norm_eps, p->sinkhorn_iters, p->hc_eps, ctx->glue, reduced,
+                                   post, comb, pre, &err);
     if (err != cudaSuccess) return cuda_fail(err, what);
     return S14_OK;
     S14_CATCH

@@ -11,21 +11,26 @@
 // arithmetic of the CPU restatement the tests compare with.
 // A token's state is hc = 4 streams of `hidden` values, F32 or BF16 (the reference's state is BF16
 // [1, 1, 4, 4096]); results are rounded to the streams' type where the Python code casts back.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "s14_device.cuh"
 
 namespace s14 {
 
+namespace cg = cooperative_groups;
+
 namespace {
 
 constexpr uint32_t kHc = 4;
 constexpr uint32_t kMixMax = (2 + kHc) * kHc;
 
+// What an earlier kernel wrote is read from the L2: these kernels may be resident before that kernel ends, and
+// an SM's L1 may still hold the line's earlier contents.
 template <bool kBf16>
 __device__ __forceinline__ float stream_ld(const void *p, size_t i) {
-    if constexpr (kBf16) return __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p) + i) << 16);
-    else return __ldg(reinterpret_cast<const float *>(p) + i);
+    if constexpr (kBf16) return __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const uint16_t *>(p) + i) << 16);
+    else return __ldcg(reinterpret_cast<const float *>(p) + i);
 }
 template <bool kBf16>
 __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
@@ -33,58 +38,50 @@ __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
     else reinterpret_cast<float *>(p)[i] = v;
 }
 
-// sum of v over the CTA's 256 threads (every thread gets it); red: 8 doubles of shared memory
-__device__ __forceinline__ double block_sum_256(double v, double *red) {
-    v = warp_sum(v);
-    __syncthreads();
-    if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
+// Eight stream values from one (BF16) or two (F32) 16-byte loads, and back; one by one where a caller's buffer is not
+// aligned to 16 bytes (`vec`, the same for all threads of a launch).
+template <bool kBf16>
+__device__ __forceinline__ void stream_ld8(const void *p, size_t i, float (&v)[8], bool vec) {
+    if (!vec) {
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += red[w];
-    return s;
+        for (int k = 0; k < 8; ++k) v[k] = stream_ld<kBf16>(p, i + k);
+        return;
+    }
+    if constexpr (kBf16) {
+        const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(p) + i));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[2 * k] = __uint_as_float(w[k] << 16), v[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+    } else {
+        const float4 a = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i));
+        const float4 b = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i) + 1);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    }
+}
+template <bool kBf16>
+__device__ __forceinline__ void stream_st8(void *p, size_t i, const float (&v)[8], bool vec) {
+    if (!vec) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) stream_st<kBf16>(p, i + k, v[k]);
+        return;
+    }
+    if constexpr (kBf16) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+            w[k] = *reinterpret_cast<const uint32_t *>(&b);
+        }
+        *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p) + i) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+        float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p) + i);
+        o[0] = make_float4(v[0], v[1], v[2], v[3]);
+        o[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
 }
 
 __device__ __forceinline__ float sigmoid_f32(float v) { return (float)(1.0 / (1.0 + exp(-(double)v))); }
-
-// CTA (m, t): the dot product of token t's flattened streams with row m of fn, in double, rounded to
-// F32; CTA (0, t) also writes the mean of the squares.  256 threads.
-template <bool kBf16>
-__global__ void __launch_bounds__(256)
-k_hc_mixes(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, float *__restrict__ dots,
-           float *__restrict__ mean_sq, uint32_t n_mix) {
-    __shared__ double red[8];
-    const uint32_t m = blockIdx.x, t = blockIdx.y;
-    const float4 *row = reinterpret_cast<const float4 *>(fn + (size_t)m * n);
-    double acc = 0.0, ss = 0.0;
-    // four elements per thread and step, four steps' loads in flight (n is a multiple of 1024)
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < (n >> 2); i += 256u) {
-        float v[4];
-        if constexpr (kBf16) {
-            const uint2 q = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(x) + (size_t)t * n) + i);
-            v[0] = __uint_as_float(q.x << 16), v[1] = __uint_as_float(q.x & 0xffff0000u);
-            v[2] = __uint_as_float(q.y << 16), v[3] = __uint_as_float(q.y & 0xffff0000u);
-        } else {
-            const float4 q = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + (size_t)t * n) + i);
-            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-        }
-        const float4 w = __ldg(row + i);
-        const float wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const double d = (double)v[k];
-            acc += d * (double)wv[k];
-            ss += d * d;
-        }
-    }
-    const double dot = block_sum_256(acc, red);
-    if (m == 0u) {
-        const double s2 = block_sum_256(ss, red);
-        if (threadIdx.x == 0) mean_sq[t] = (float)(s2 / (double)n);
-    }
-    if (threadIdx.x == 0) dots[(size_t)t * n_mix + m] = (float)dot;
-}
+__device__ __forceinline__ float rsqrt_of(float mean_sq, float eps) { return (float)(1.0 / sqrt((double)__fadd_rn(mean_sq, eps))); }
 
 // hc.py:19-84 by one warp: 24 logits -> pre [4], post [4], comb [4][4], F32 in the reference's order.  Lane
 // l < 16 owns comb[l / 4][l % 4]; a row's or column's four values are fetched with shuffles and added in
@@ -117,86 +114,298 @@ __device__ __forceinline__ void split_sinkhorn_warp(const float *mixes, const fl
     comb = c;
 }
 
-// One CTA per token: the coefficients from the dots (one warp), then reduced[d] = sum_h pre[h] x[h][d].
-// kHead: the head's reduce (final_head.py:43-81): hc logits, pre = sigmoid(mix * scale + base) + eps only.
+// reduced[d] = sum_h pre[h] x[h][d] for eight consecutive d.
+template <bool kBf16>
+__device__ __forceinline__ void reduce_streams8(const void *x, size_t x0, uint32_t hidden, uint32_t d, const float (&pre)[kHc],
+                                                float (&acc)[8], bool vec) {
+    float v[kHc][8];
+#pragma unroll
+    for (uint32_t h = 0; h < kHc; ++h) stream_ld8<kBf16>(x, x0 + (size_t)h * hidden + d, v[h], vec);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        acc[k] = __fmul_rn(pre[0], v[0][k]);
+#pragma unroll
+        for (uint32_t h = 1; h < kHc; ++h) acc[k] = __fadd_rn(acc[k], __fmul_rn(pre[h], v[h][k]));
+    }
+}
+
+// hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
+// only) of few tokens: one cluster of sixteen CTAs per token.  The call is all latency: 1.5 MB of fn per token,
+// then a serial chain of 20 Sinkhorn rounds.  Every CTA takes a sixteenth of the flattened streams against all
+// rows of fn (98 KB, asked for before the wait for the state, all loads in flight together), the partial sums
+// cross in shared memory, every CTA makes the coefficients itself and reduces its sixteenth of the hidden
+// vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
+constexpr uint32_t kPreCluster = 16, kPreThreads = 512;
 template <bool kBf16, bool kHead>
-__global__ void __launch_bounds__(256)
-k_hc_reduce(const void *__restrict__ x, const float *__restrict__ dots, const float *__restrict__ mean_sq,
-            const float *__restrict__ scale, const float *__restrict__ base, uint32_t hidden, float norm_eps, uint32_t iters,
-            float hc_eps, void *__restrict__ reduced, float *__restrict__ post_out, float *__restrict__ comb_out,
-            float *__restrict__ pre_out) {
-    __shared__ float s_pre[kHc], s_mix[kMixMax];
-    const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u;
-    constexpr uint32_t n_mix = kHead ? kHc : kMixMax;
-    if (threadIdx.x < 32u) {
-        const float rs = (float)(1.0 / sqrt((double)__fadd_rn(mean_sq[t], norm_eps)));
-        if (lane < n_mix) s_mix[lane] = __fmul_rn(dots[(size_t)t * n_mix + lane], rs);
-        __syncwarp();
-        float pre;
-        if constexpr (kHead) {
-            const uint32_t h = lane & 3u;
-            pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[h], scale[0]), base[h])), hc_eps);
+__global__ void __launch_bounds__(kPreThreads)
+k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *__restrict__ scale, const float *__restrict__ base,
+         uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced, float *__restrict__ post_out,
+         float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec) {
+    constexpr uint32_t n_mix = kHead ? kHc : kMixMax, kRows = n_mix / 2u;   // rows per half of the CTA
+    __shared__ double s_warp[kPreThreads / 32][kRows + 1];
+    __shared__ double s_part[kPreCluster][n_mix + 1];                      // [n_mix]: the sum of squares
+    __shared__ float s_mix[n_mix], s_pre[kHc];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), t = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t n = kHc * hidden, share = n / kPreCluster, k0 = rank * share;   // a multiple of 64
+    const uint32_t half = tid >> 8, c = tid & 255u;                          // half of the rows, column of four elements
+    double acc[kRows], ss = 0.0;
+#pragma unroll
+    for (uint32_t m = 0; m < kRows; ++m) acc[m] = 0.0;
+    float4 f[kRows];
+    auto fetch = [&](uint32_t i) {
+#pragma unroll
+        for (uint32_t m = 0; m < kRows; ++m) f[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)(half * kRows + m) * n + k0 + i));
+    };
+    if (c * 4u < share) fetch(c * 4u);
+    cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
+    cudaGridDependencySynchronize();
+    for (uint32_t i = c * 4u; i < share; i += 1024u) {
+        float v[4];
+        if constexpr (kBf16) {
+            const uint2 q = __ldcg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(x) + (size_t)t * n + k0 + i));
+            v[0] = __uint_as_float(q.x << 16), v[1] = __uint_as_float(q.x & 0xffff0000u);
+            v[2] = __uint_as_float(q.y << 16), v[3] = __uint_as_float(q.y & 0xffff0000u);
         } else {
-            float post, comb;
-            split_sinkhorn_warp(s_mix, scale, base, iters, hc_eps, lane, pre, post, comb);
-            if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
-            if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
+            const float4 q = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + (size_t)t * n + k0 + i));
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
         }
+        if (i != c * 4u) fetch(i);
+        const double d0 = v[0], d1 = v[1], d2 = v[2], d3 = v[3];
+#pragma unroll
+        for (uint32_t m = 0; m < kRows; ++m) acc[m] += (d0 * (double)f[m].x + d1 * (double)f[m].y) + (d2 * (double)f[m].z + d3 * (double)f[m].w);
+        if (half == 0u) ss += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+    }
+#pragma unroll
+    for (uint32_t m = 0; m < kRows; ++m) {
+        acc[m] = warp_sum(acc[m]);
+        if (lane == 0u) s_warp[warp][m] = acc[m];
+    }
+    ss = warp_sum(ss);
+    if (lane == 0u) s_warp[warp][kRows] = ss;
+    __syncthreads();
+    if (tid <= n_mix) {
+        const uint32_t w0 = tid < n_mix ? (tid / kRows) * 8u : 0u, m = tid < n_mix ? tid % kRows : kRows;
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t w = 0; w < 8u; ++w) s += s_warp[w0 + w][m];
+#pragma unroll
+        for (uint32_t r = 0; r < kPreCluster; ++r) *cluster.map_shared_rank(&s_part[rank][tid], r) = s;
+    }
+    cluster.sync();
+    if (warp == 0u) {
+        double s = 0.0;
+        if (lane <= n_mix) {
+#pragma unroll
+            for (uint32_t r = 0; r < kPreCluster; ++r) s += s_part[r][lane];
+        }
+        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, n_mix) / (double)n), norm_eps);
+        if (lane < n_mix) s_mix[lane] = __fmul_rn((float)s, rs);
+        __syncwarp();
+        // pre first: the other warps reduce the streams while this one of the first CTA goes on to post and comb
         if (lane < kHc) {
+            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], scale[0]), base[lane])), hc_eps);
             s_pre[lane] = pre;
-            if (pre_out) pre_out[(size_t)t * kHc + lane] = pre;
+            if (pre_out && rank == 0u) pre_out[(size_t)t * kHc + lane] = pre;
         }
     }
     __syncthreads();
-    const size_t x0 = (size_t)t * kHc * hidden;
-    for (uint32_t d = threadIdx.x; d < hidden; d += 256u) {
-        float acc = __fmul_rn(s_pre[0], stream_ld<kBf16>(x, x0 + d));
-#pragma unroll
-        for (uint32_t h = 1; h < kHc; ++h) acc = __fadd_rn(acc, __fmul_rn(s_pre[h], stream_ld<kBf16>(x, x0 + (size_t)h * hidden + d)));
-        stream_st<kBf16>(reduced, (size_t)t * hidden + d, acc);
+    const uint32_t part = hidden / kPreCluster;   // a multiple of 16
+    if (!kHead && rank == 0u && warp == 0u) {
+        float pre, post, comb;
+        split_sinkhorn_warp(s_mix, scale, base, iters, hc_eps, lane, pre, post, comb);
+        if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
+        if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
+    }
+    const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
+    // the last threads, so that the warp with the Sinkhorn rounds has none of it
+    for (uint32_t i = (kPreThreads - 1u - tid) * 8u; i < part; i += kPreThreads * 8u) {
+        float v[8];
+        reduce_streams8<kBf16>(x, (size_t)t * n, hidden, rank * part + i, pre, v, vec != 0u);
+        stream_st8<kBf16>(reduced, (size_t)t * hidden + rank * part + i, v, vec != 0u);
     }
 }
 
-// hc.py:127-148: merged[t][o][d] = post[o] * branch[d] + sum_h comb[h][o] * residual[h][d].
+// The dot products of many tokens with the rows of fn, and the sums of squares, on mma.m8n8k4.f64: a CTA takes
+// sixteen tokens and a slice of K, each of its eight warps a part of the slice.  A vector kernel with a CTA per
+// (row, token) read every token 24 times and every row once per token and converted all of it to double each
+// time (70 us for 370 tokens of 4096); here a row's element serves sixteen tokens and a token's 24 rows (12 us:
+// the FP64 pipe's 64 products per clock and SM bound it at 8).  K is permuted inside steps of sixteen: lane q of
+// a quad takes four consecutive elements as its slots of four MMAs.  Writes partial sums [slice][token][25] in double.
+constexpr uint32_t kDotTokens = 16;
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
+k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, uint32_t n_tokens, double *__restrict__ partial) {
+    __shared__ double s_acc[8][kDotTokens][kMixMax + 1];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
+    const uint32_t t0 = blockIdx.x * kDotTokens, len = n / (gridDim.y * 8u);   // a multiple of 16
+    const uint32_t k0 = (blockIdx.y * 8u + warp) * len + q * 4u;
+    const uint32_t ta = min(t0 + g, n_tokens - 1u), tb = min(t0 + g + 8u, n_tokens - 1u);
+    double c[2][3][2] = {}, ss[2] = {0.0, 0.0};
+    auto load4 = [&](uint32_t t, uint32_t k, float (&v)[4]) {
+        if constexpr (kBf16) {
+            const uint2 w = __ldcg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(x) + (size_t)t * n + k));
+            v[0] = __uint_as_float(w.x << 16), v[1] = __uint_as_float(w.x & 0xffff0000u);
+            v[2] = __uint_as_float(w.y << 16), v[3] = __uint_as_float(w.y & 0xffff0000u);
+        } else {
+            const float4 w = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + (size_t)t * n + k));
+            v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
+        }
+    };
+#pragma unroll 2
+    for (uint32_t k = k0; k < k0 + len; k += 16u) {
+        float va[4], vb[4];
+        load4(ta, k, va);
+        load4(tb, k, vb);
+        float4 w[3];
+#pragma unroll
+        for (uint32_t m = 0; m < 3; ++m) w[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)(m * 8u + g) * n + k));
+#pragma unroll
+        for (uint32_t s = 0; s < 4; ++s) {
+            const double a = va[s], b = vb[s];
+            ss[0] += a * a;
+            ss[1] += b * b;
+#pragma unroll
+            for (uint32_t m = 0; m < 3; ++m) {
+                const double f = s == 0u ? w[m].x : (s == 1u ? w[m].y : (s == 2u ? w[m].z : w[m].w));
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                             : "+d"(c[0][m][0]), "+d"(c[0][m][1])
+                             : "d"(a), "d"(f));
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                             : "+d"(c[1][m][0]), "+d"(c[1][m][1])
+                             : "d"(b), "d"(f));
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+#pragma unroll
+        for (uint32_t m = 0; m < 3; ++m)
+#pragma unroll
+            for (uint32_t e = 0; e < 2; ++e) s_acc[warp][h * 8u + g][m * 8u + 2u * q + e] = c[h][m][e];
+        ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 1);
+        ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 2);
+        if (q == 0u) s_acc[warp][h * 8u + g][kMixMax] = ss[h];
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < kDotTokens * (kMixMax + 1u); i += 256u) {
+        const uint32_t t = i / (kMixMax + 1u), m = i - t * (kMixMax + 1u);
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) s += s_acc[w][t][m];
+        if (t0 + t < n_tokens) partial[((size_t)blockIdx.y * n_tokens + t0 + t) * (kMixMax + 1u) + m] = s;
+    }
+}
+
+// One CTA per token: the coefficients from the partial sums (one warp), then the reduced vector.
+template <bool kBf16>
+__global__ void __launch_bounds__(256)
+k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint32_t slices, const float *__restrict__ scale,
+            const float *__restrict__ base, uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced,
+            float *__restrict__ post_out, float *__restrict__ comb_out, uint32_t vec) {
+    __shared__ float s_pre[kHc], s_mix[kMixMax];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (warp == 0u) {
+        double s = 0.0;
+        if (lane <= kMixMax)
+            for (uint32_t p = 0; p < slices; ++p) s += __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMixMax + 1u) + lane);
+        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMixMax) / (double)(kHc * hidden)), norm_eps);
+        if (lane < kMixMax) s_mix[lane] = __fmul_rn((float)s, rs);
+        __syncwarp();
+        if (lane < kHc) s_pre[lane] = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], scale[0]), base[lane])), hc_eps);
+    }
+    __syncthreads();
+    if (warp == 0u) {  // the other warps reduce the streams meanwhile
+        float pre, post, comb;
+        split_sinkhorn_warp(s_mix, scale, base, iters, hc_eps, lane, pre, post, comb);
+        if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
+        if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
+        return;
+    }
+    const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
+    for (uint32_t d = (threadIdx.x - 32u) * 8u; d < hidden; d += 224u * 8u) {
+        float v[8];
+        reduce_streams8<kBf16>(x, (size_t)t * kHc * hidden, hidden, d, pre, v, vec != 0u);
+        stream_st8<kBf16>(reduced, (size_t)t * hidden + d, v, vec != 0u);
+    }
+}
+
+// hc.py:127-148: merged[t][o][d] = post[o] * branch[d] + sum_h comb[h][o] * residual[h][d]; eight d per thread.
+template <bool kBf16>
+__global__ void __launch_bounds__(128)
 k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, const float *__restrict__ post,
-          const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
-    const uint32_t d = blockIdx.x * 256u + threadIdx.x, t = blockIdx.y;
+          const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged, uint32_t vec) {
+    const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * 8u, t = blockIdx.y;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (d >= hidden) return;
-    float r[kHc], c[kHc * kHc], p[kHc];
+    float r[kHc][8], b[8], c[kHc * kHc], p[kHc];
 #pragma unroll
     for (uint32_t h = 0; h < kHc; ++h) {
-        r[h] = stream_ld<kBf16>(residual, ((size_t)t * kHc + h) * hidden + d);
-        p[h] = __ldg(post + (size_t)t * kHc + h);
+        stream_ld8<kBf16>(residual, ((size_t)t * kHc + h) * hidden + d, r[h], vec != 0u);
+        p[h] = __ldcg(post + (size_t)t * kHc + h);
     }
+    stream_ld8<kBf16>(branch, (size_t)t * hidden + d, b, vec != 0u);
 #pragma unroll
-    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldg(comb + (size_t)t * kHc * kHc + i);
-    const float b = stream_ld<kBf16>(branch, (size_t)t * hidden + d);
+    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldcg(comb + (size_t)t * kHc * kHc + i);
 #pragma unroll
     for (uint32_t o = 0; o < kHc; ++o) {
-        float s = __fmul_rn(c[o], r[0]);
+        float v[8];
 #pragma unroll
-        for (uint32_t h = 1; h < kHc; ++h) s = __fadd_rn(s, __fmul_rn(c[h * kHc + o], r[h]));
-        stream_st<kBf16>(merged, ((size_t)t * kHc + o) * hidden + d, __fadd_rn(__fmul_rn(p[o], b), s));
+        for (int k = 0; k < 8; ++k) {
+            float s = __fmul_rn(c[o], r[0][k]);
+#pragma unroll
+            for (uint32_t h = 1; h < kHc; ++h) s = __fadd_rn(s, __fmul_rn(c[h * kHc + o], r[h][k]));
+            v[k] = __fadd_rn(__fmul_rn(p[o], b[k]), s);
+        }
+        stream_st8<kBf16>(merged, ((size_t)t * kHc + o) * hidden + d, v, vec != 0u);
     }
 }
 
-// final_head.py:84-110: out = w * (x * rsqrt(mean(x^2) + eps)); one CTA per token.
+// final_head.py:84-110: out = w * (x * rsqrt(mean(x^2) + eps)); one CTA per token, the token in registers
+// (eight values per thread and step; hidden <= 8192: at most four steps), so it is read once.
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
-k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out) {
+k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out,
+           uint32_t vec) {
     __shared__ double red[8];
     const uint32_t t = blockIdx.x;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    float v[4][8];
     double ss = 0.0;
-    for (uint32_t i = threadIdx.x; i < hidden; i += 256u) {
-        const double v = (double)stream_ld<kBf16>(x, (size_t)t * hidden + i);
-        ss += v * v;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t d = (i * 256u + threadIdx.x) * 8u;
+        if (d < hidden) {
+            stream_ld8<kBf16>(x, (size_t)t * hidden + d, v[i], vec != 0u);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ss += (double)v[i][k] * (double)v[i][k];
+        }
     }
-    const float ms = (float)(block_sum_256(ss, red) / (double)hidden);
-    const float rs = (float)(1.0 / sqrt((double)__fadd_rn(ms, eps)));
-    for (uint32_t i = threadIdx.x; i < hidden; i += 256u)
-        stream_st<kBf16>(out, (size_t)t * hidden + i, __fmul_rn(__ldg(w + i), __fmul_rn(stream_ld<kBf16>(x, (size_t)t * hidden + i), rs)));
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += red[i];
+    const float rs = rsqrt_of((float)(ss / (double)hidden), eps);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t d = (i * 256u + threadIdx.x) * 8u;
+        if (d < hidden) {
+            float wv[8];
+            stream_ld8<false>(w, d, wv, vec != 0u);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) wv[k] = __fmul_rn(wv[k], __fmul_rn(v[i][k], rs));
+            stream_st8<kBf16>(out, (size_t)t * hidden + d, wv, vec != 0u);
+        }
+    }
 }
 
 // executor.py:638-668 for the hash-routed layers: the ids are the token's row of tid2eid, the weights the
@@ -246,10 +455,10 @@ k_branch_post(const float *__restrict__ y, uint16_t *__restrict__ branch_out, co
 #pragma unroll
     for (uint32_t h = 0; h < kHc; ++h) {
         r[h] = stream_ld<true>(residual, (size_t)h * hidden + d);
-        p[h] = __ldg(post + h);
+        p[h] = __ldcg(post + h);
     }
 #pragma unroll
-    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldg(comb + i);
+    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldcg(comb + i);
     const __nv_bfloat16 b16 = __float2bfloat16_rn(__ldcg(y + d));
     if (branch_out) branch_out[d] = *reinterpret_cast<const uint16_t *>(&b16);
     const float b = __bfloat162float(b16);
@@ -274,35 +483,82 @@ cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y,
                       merged);
 }
 
-// dots: [n_tokens, 24] scratch, mean_sq: [n_tokens] scratch.  Returns the number of kernels launched.
+size_t hc_scratch_bytes(uint32_t max_tokens) { return (size_t)(std::max(8u * max_tokens, 8192u)) * (kMixMax + 1u) * sizeof(double); }
+
+// Whether all the addresses are multiples of 16 (rows of 256 and more elements keep that).
+template <class... P>
+static uint32_t aligned16(P... p) {
+    return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0u ? 1u : 0u;
+}
+
+// A kernel in clusters of sixteen (beyond the portable eight): allowed once per kernel and device.
+template <class Kernel>
+static cudaError_t allow_wide_clusters(Kernel kernel, bool (&done)[64]) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+    if (!done[dev]) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        done[dev] = e == cudaSuccess;
+    }
+    return e;
+}
+
+template <bool kBf16, bool kHead>
+static cudaError_t launch_hc_pre_cluster(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
+                                         const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
+                                         void *reduced, float *post, float *comb, float *pre) {
+    static bool done[64] = {};
+    const cudaError_t e = allow_wide_clusters(k_hc_pre<kBf16, kHead>, done);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(k_hc_pre<kBf16, kHead>, dim3(kPreCluster, n_tokens), dim3(kPreThreads), 0, st, kPreCluster, x, fn, scale, base,
+                      hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced));
+}
+
+template <bool kBf16>
+static cudaError_t launch_hc_pre_many(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
+                                      const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
+                                      double *partial, void *reduced, float *post, float *comb) {
+    // slices of K: enough CTAs for the SMs, each warp's part whole steps of sixteen (n / 1024 is a whole number)
+    const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden;
+    uint32_t slices = 8u;
+    while (slices < 64u && groups * slices < 148u && (n / (slices * 2u * 8u)) % 16u == 0u) slices *= 2u;
+    const cudaError_t e = launch_pdl(k_hc_dots<kBf16>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(k_hc_reduce<kBf16>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,
+                      norm_eps, iters, hc_eps, reduced, post, comb, aligned16(x, reduced));
+}
+
+// scratch: hc_scratch_bytes of the most tokens.  Returns the number of kernels launched.
 int launch_hc_pre(cudaStream_t st, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
-                  const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, float *dots, float *mean_sq,
-                  void *reduced, float *post, float *comb, float *pre, cudaError_t *err) {
-    const uint32_t n_mix = head ? kHc : kMixMax, n = kHc * hidden;
-    const dim3 grid(n_mix, n_tokens);
-    if (bf16) k_hc_mixes<true><<<grid, 256, 0, st>>>(x, fn, n, dots, mean_sq, n_mix);
-    else k_hc_mixes<false><<<grid, 256, 0, st>>>(x, fn, n, dots, mean_sq, n_mix);
-    if (bf16 && head) k_hc_reduce<true, true><<<n_tokens, 256, 0, st>>>(x, dots, mean_sq, scale, base, hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-    else if (bf16) k_hc_reduce<true, false><<<n_tokens, 256, 0, st>>>(x, dots, mean_sq, scale, base, hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-    else if (head) k_hc_reduce<false, true><<<n_tokens, 256, 0, st>>>(x, dots, mean_sq, scale, base, hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-    else k_hc_reduce<false, false><<<n_tokens, 256, 0, st>>>(x, dots, mean_sq, scale, base, hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-    *err = cudaGetLastError();
+                  const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
+                  float *post, float *comb, float *pre, cudaError_t *err) {
+    // up to eight tokens the clusters fit the GPU side by side; the head's reduce (four rows) has no other form
+    if (head || n_tokens <= 8u) {
+        if (bf16 && head) *err = launch_hc_pre_cluster<true, true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+        else if (bf16) *err = launch_hc_pre_cluster<true, false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+        else if (head) *err = launch_hc_pre_cluster<false, true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+        else *err = launch_hc_pre_cluster<false, false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+        return 1;
+    }
+    *err = bf16 ? launch_hc_pre_many<true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced, post, comb)
+                : launch_hc_pre_many<false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced, post, comb);
     return 2;
 }
 
 cudaError_t launch_hc_post(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged) {
-    const dim3 grid((hidden + 255u) / 256u, n_tokens);
-    if (bf16) k_hc_post<true><<<grid, 256, 0, st>>>(branch, residual, post, comb, hidden, merged);
-    else k_hc_post<false><<<grid, 256, 0, st>>>(branch, residual, post, comb, hidden, merged);
-    return cudaGetLastError();
+    const dim3 grid((hidden + 1023u) / 1024u, n_tokens);
+    const uint32_t vec = aligned16(branch, residual, merged);
+    if (bf16) return launch_pdl(k_hc_post<true>, grid, dim3(128), 0, st, 0u, branch, residual, post, comb, hidden, merged, vec);
+    return launch_pdl(k_hc_post<false>, grid, dim3(128), 0, st, 0u, branch, residual, post, comb, hidden, merged, vec);
 }
 
 cudaError_t launch_rms_norm(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
                             void *out) {
-    if (bf16) k_rms_norm<true><<<n_tokens, 256, 0, st>>>(x, w, hidden, eps, out);
-    else k_rms_norm<false><<<n_tokens, 256, 0, st>>>(x, w, hidden, eps, out);
-    return cudaGetLastError();
+    const uint32_t vec = aligned16(x, w, out);
+    if (bf16) return launch_pdl(k_rms_norm<true>, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec);
+    return launch_pdl(k_rms_norm<false>, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec);
 }
 
 cudaError_t launch_router_hash(cudaStream_t st, const s14_router_desc &r, const int64_t *tid2eid) {

@@ -108,7 +108,7 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
             __syncthreads();  // the parts of the phase before are not read any more
             for (uint32_t i = tid; i < n_tokens * (span >> 1); i += kHeadThreads) {
                 const uint32_t t = i / (span >> 1), k2 = i - t * (span >> 1);
-                const float2 v = __ldg(reinterpret_cast<const float2 *>(x + (size_t)t * hidden + phase * span) + k2);
+                const float2 v = __ldcg(reinterpret_cast<const float2 *>(x + (size_t)t * hidden + phase * span) + k2);
                 uint32_t px[3], py[3];
                 head_parts(v.x, px);
                 head_parts(v.y, py);
@@ -260,7 +260,7 @@ k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__res
             const float4 v = __ldcg(reinterpret_cast<const float4 *>(logits) + i);
             take(v.x, 4u * i), take(v.y, 4u * i + 1u), take(v.z, 4u * i + 2u), take(v.w, 4u * i + 3u);
         }
-        if (rank == 0u && tid < (vocab & 3u)) take(logits[n4 * 4u + tid], n4 * 4u + tid);
+        if (rank == 0u && tid < (vocab & 3u)) take(__ldcg(logits + n4 * 4u + tid), n4 * 4u + tid);
     } else {
         for (uint32_t i = rank * kArgmaxThreads + tid; i < vocab; i += n * kArgmaxThreads) take(__ldcg(logits + i), i);
     }
@@ -295,7 +295,7 @@ k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__res
 // the reduced and the normalised vector rounded to BF16.
 constexpr uint32_t kPrepCluster = 8, kPrepThreads = 256;
 
-__device__ __forceinline__ float bf16_of(const uint16_t *p) { return __uint_as_float((uint32_t)__ldg(p) << 16); }
+__device__ __forceinline__ float bf16_of(const uint16_t *p) { return __uint_as_float((uint32_t)__ldcg(p) << 16); }
 
 __global__ void __launch_bounds__(kPrepThreads)
 k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, const float *__restrict__ scale,
@@ -314,7 +314,7 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (uint32_t i = tid * 4u; i < share; i += kPrepThreads * 4u) {
         const uint32_t k = rank * share + i;
-        const uint2 b = __ldg(reinterpret_cast<const uint2 *>(state + k));
+        const uint2 b = __ldcg(reinterpret_cast<const uint2 *>(state + k));
         const float xs[4] = {__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xffff0000u), __uint_as_float(b.y << 16),
                              __uint_as_float(b.y & 0xffff0000u)};
         float4 f[4];

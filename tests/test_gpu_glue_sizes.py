@@ -1,0 +1,78 @@
+"""The layer-glue operators where their kernels change form: the cluster kernel's last token count and the first of
+the matrix kernel, a group of sixteen tokens with a remainder, the smallest and the largest hidden size, buffers
+that are not aligned to 16 bytes (GPU, against the CPU oracle)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from colormlm_b200 import synth
+from colormlm_b200.s14 import S14Context
+
+from .test_gpu_glue import bits16, close_coeff, close_streams, dev, f32_of_bits
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("cuda_lib")]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    c = S14Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("n_tokens,hidden", [(1, 256), (8, 1280), (9, 256), (9, 8192), (16, 2048), (33, 768), (150, 1024)])
+def test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden):
+    g = synth.rng(77 + n_tokens + hidden)
+    fn, scale, base = synth.hc_params(g, hidden)
+    nw = g.uniform(0.5, 1.5, size=hidden).astype(np.float32)
+    x = dev(synth.hc_streams(g, n_tokens, hidden), bf16)
+    host = (lambda t: bits16(t)) if bf16 else (lambda t: t.cpu().numpy())
+    as_f32 = (lambda a: f32_of_bits(a)) if bf16 else (lambda a: a)
+    red, merged = torch.empty((n_tokens, hidden), dtype=x.dtype, device="cuda"), torch.empty_like(x)
+    post, comb = torch.empty((n_tokens, 4), device="cuda"), torch.empty((n_tokens, 4, 4), device="cuda")
+    normed = torch.empty_like(red)
+    ctx.cmd_hc_pre(x, dev(fn), dev(scale), dev(base), red, post, comb)
+    ctx.cmd_rms_norm(red, dev(nw), normed)
+    ctx.cmd_hc_post(normed, x, post, comb, merged)
+    torch.cuda.synchronize()
+    r_ref, p_ref, c_ref = oracle.hc_pre(host(x), fn, scale, base, dtype=int(bf16))
+    close_coeff(post.cpu().numpy(), p_ref)
+    close_coeff(comb.cpu().numpy(), c_ref)
+    close_streams(as_f32(host(red)), as_f32(r_ref), bf16)
+    close_streams(as_f32(host(normed)), as_f32(oracle.rms_norm(host(red), nw, dtype=int(bf16))), bf16)
+    m_ref = oracle.hc_post(host(normed), host(x), post.cpu().numpy(), comb.cpu().numpy(), dtype=int(bf16))
+    assert np.array_equal(as_f32(host(merged)), as_f32(m_ref))
+    # the head's reduce, one cluster per token for any number of tokens
+    hfn, hscale, hbase = synth.hc_params(g, hidden, head=True)
+    pre = torch.empty((n_tokens, 4), device="cuda")
+    ctx.cmd_hc_head_reduce(x, dev(hfn), dev(hscale), dev(hbase), red, pre)
+    h_ref, pre_ref = oracle.hc_head_reduce(host(x), hfn, hscale, hbase, dtype=int(bf16))
+    close_coeff(pre.cpu().numpy(), pre_ref)
+    close_streams(as_f32(host(red)), as_f32(h_ref), bf16)
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_buffers_that_are_not_16_byte_aligned(ctx, bf16):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    t, h, dt = 3, 512, torch.bfloat16 if bf16 else torch.float32
+    make = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dt)
+    branch, res, nw = make(t, h), make(t, 4, h), torch.rand(h, device="cuda", generator=g)
+    post, comb = torch.rand(t, 4, device="cuda", generator=g), torch.rand(t, 4, 4, device="cuda", generator=g)
+
+    def moved(a):
+        big = torch.empty(a.numel() + 1, dtype=a.dtype, device="cuda")
+        big[1:] = a.reshape(-1)
+        return big[1:].view(a.shape)
+
+    want_m, want_n = torch.empty_like(res), torch.empty_like(branch)
+    ctx.cmd_hc_post(branch, res, post, comb, want_m)
+    ctx.cmd_rms_norm(branch, nw, want_n)
+    got_m, got_n = moved(want_m), moved(want_n)
+    got_m.zero_(), got_n.zero_()
+    ctx.cmd_hc_post(moved(branch), moved(res), post, comb, got_m)
+    ctx.cmd_rms_norm(moved(branch), moved(nw), got_n)
+    assert torch.equal(got_m, want_m) and torch.equal(got_n, want_n)
