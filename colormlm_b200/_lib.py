@@ -296,6 +296,17 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def pycall():
+    """The CPython extension of the per-token calls (csrc/s14_pycall.cpp)."""
+    lib()
+    try:
+        from . import _s14call
+    except ImportError as e:
+        raise ImportError(f"colormlm_b200/_s14call.so cannot be loaded ({e}): build it with `python -m colormlm_b200.build`. "
+                          "There is no fallback implementation.") from e
+    return _s14call
+
+
 def check(status: int) -> None:
     if status != OK:
         raise S14Error(status, lib().s14_last_error().decode("utf-8", "replace"))

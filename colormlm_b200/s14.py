@@ -122,7 +122,8 @@ class S14Context:
     def __init__(self, device: int = 0):
         h = C.c_void_p()
         check(L.lib().s14_ctx_create(device, C.byref(h)))
-        self._h = h
+        self._h, self._hv = h, h.value
+        self._calls = L.pycall()
         self.device = device
         self.pipelines = S14NumericPipelines(self)
 
@@ -134,7 +135,7 @@ class S14Context:
         if self._h:
             L.lib().s14_ep_exchange_disconnect(self._h)
             check(L.lib().s14_ctx_destroy(self._h))
-            self._h = None
+            self._h = self._hv = None
 
     def __del__(self):
         try:
@@ -201,15 +202,10 @@ class S14Context:
                              shared_kind: int, inter: int, y, ids_out=None, weights_out=None, *,
                              score_fn: int = L.SCORE_SIGMOID, top_k: int = 6, route_scale: float = 1.0,
                              stream: Optional[int] = None) -> None:
-        d = L.RoutedLayerDesc()
-        d.router = _router_desc(x, wr_bf16, bias, ids_out, weights_out, score_fn, top_k, route_scale)
-        d.inter = inter
-        d.shared_kind = shared_kind
-        d.page_table = page_table.data_ptr()
-        d.shared_page = shared_page
-        d.y = y.data_ptr()
-        check(L.lib().s14_cmd_routed_moe_layer(
-            self._h, stream if stream is not None else _torch_stream(), C.byref(d)))
+        rc = self._calls.routed_layer(self._hv, stream, x, wr_bf16, bias, page_table, shared_page, shared_kind, inter, y, ids_out,
+                                      weights_out, score_fn, top_k, route_scale)
+        if rc:
+            check(rc)
 
     def cmd_routed_moe_experts_ep(self, x, wr_bf16, bias, page_table, shared_page: Optional[int],
                                   shared_kind: int, inter: int, slots_out, ids_out, weights_out, *,
@@ -346,25 +342,26 @@ class S14Context:
     def cmd_hc_pre(self, x, hc_fn, hc_scale, hc_base, reduced, post, comb, *, iters: int = 20, norm_eps: float = 1e-6,
                    hc_eps: float = 1e-6, stream: Optional[int] = None) -> None:
         """x [T, 4, hidden] (float32 or bfloat16) -> reduced [T, hidden], post [T, 4], comb [T, 4, 4]."""
-        p = _hc_params(x, hc_fn, hc_scale, hc_base, iters, norm_eps, hc_eps)
-        check(L.lib().s14_cmd_hc_pre(self._h, stream if stream is not None else _torch_stream(), C.byref(p), x.data_ptr(),
-                                     reduced.data_ptr(), post.data_ptr(), comb.data_ptr()))
+        rc = self._calls.hc_pre(self._hv, stream, x, hc_fn, hc_scale, hc_base, reduced, post, comb, iters, norm_eps, hc_eps)
+        if rc != 0:
+            _refused(rc, x)
 
     def cmd_hc_post(self, branch, residual, post, comb, merged, stream: Optional[int] = None) -> None:
         """merged [T, 4, hidden] = post * branch + sum_h comb[h] * residual[h]."""
-        check(L.lib().s14_cmd_hc_post(self._h, stream if stream is not None else _torch_stream(), residual.shape[0],
-                                      residual.shape[1], residual.shape[2], _stream_type(residual), branch.data_ptr(),
-                                      residual.data_ptr(), post.data_ptr(), comb.data_ptr(), merged.data_ptr()))
+        rc = self._calls.hc_post(self._hv, stream, branch, residual, post, comb, merged)
+        if rc != 0:
+            _refused(rc, residual)
 
     def cmd_rms_norm(self, x, weight, out, *, eps: float = 1e-6, stream: Optional[int] = None) -> None:
-        check(L.lib().s14_cmd_rms_norm(self._h, stream if stream is not None else _torch_stream(), x.shape[0], x.shape[1],
-                                       _stream_type(x), x.data_ptr(), weight.data_ptr(), eps, out.data_ptr()))
+        rc = self._calls.rms_norm(self._hv, stream, x, weight, eps, out)
+        if rc != 0:
+            _refused(rc, x)
 
     def cmd_hc_head_reduce(self, x, hc_fn, hc_scale, hc_base, reduced, pre, *, norm_eps: float = 1e-6, hc_eps: float = 1e-6,
                            stream: Optional[int] = None) -> None:
-        p = _hc_params(x, hc_fn, hc_scale, hc_base, 1, norm_eps, hc_eps)
-        check(L.lib().s14_cmd_hc_head_reduce(self._h, stream if stream is not None else _torch_stream(), C.byref(p),
-                                             x.data_ptr(), reduced.data_ptr(), pre.data_ptr()))
+        rc = self._calls.hc_head_reduce(self._hv, stream, x, hc_fn, hc_scale, hc_base, reduced, pre, norm_eps, hc_eps)
+        if rc != 0:
+            _refused(rc, x)
 
     def cmd_router_hash(self, x, wr_bf16, tid2eid_rows, ids_out, weights_out, *, score_fn: int = L.SCORE_SQRT_SOFTPLUS,
                         route_scale: float = 1.5, stream: Optional[int] = None) -> None:
@@ -378,39 +375,30 @@ class S14Context:
                                                 shared_page: Optional[int], shared_kind: int, inter: int, state_out,
                                                 moe_branch_out=None, stream: Optional[int] = None) -> None:
         """ffn_input bfloat16 [hidden], residual bfloat16 [4, hidden] -> state_out bfloat16 [4, hidden]."""
-        ld, keep = _layer_desc([route], shared_page, shared_kind, ffn_input.shape[-1], inter)
-        d = L.ExecMoeDesc()
-        d.hidden, d.inter, d.shared_kind = ffn_input.shape[-1], inter, shared_kind
-        d.route = C.cast(ld.routes, C.c_void_p)
-        d.shared_page = shared_page
-        d.ffn_input_bf16, d.residual_bf16 = ffn_input.data_ptr(), residual.data_ptr()
-        d.post, d.comb = post.data_ptr(), comb.data_ptr()
-        d.state_out_bf16 = state_out.data_ptr()
-        d.moe_branch_out_bf16 = moe_branch_out.data_ptr() if moe_branch_out is not None else None
-        check(L.lib().s14_exec_routed_and_shared_moe_then_hc_post(
-            self._h, stream if stream is not None else _torch_stream(), C.byref(d)))
-        del keep
+        rc = self._calls.exec_moe(self._hv, stream, ffn_input, residual, post, comb, route, shared_page, shared_kind, inter, state_out,
+                                  moe_branch_out)
+        if rc is None:
+            raise S14Error(L.ERR_CONTRACT, _ROUTE_ITEMS)
+        check(rc)
 
     def exec_hc_head_norm_full_logits(self, state, hc_fn, hc_scale, hc_base, norm_weight, head_weight_bf16, logits_out, *,
                                       norm_eps: float = 1e-6, hc_eps: float = 1e-6, stream: Optional[int] = None) -> None:
         """state bfloat16 [1, 4, hidden] -> logits_out float32 [rows of head_weight_bf16]."""
-        p = _hc_params(state, hc_fn, hc_scale, hc_base, 1, norm_eps, hc_eps)
-        check(L.lib().s14_exec_hc_head_norm_full_logits(
-            self._h, stream if stream is not None else _torch_stream(), C.byref(p), norm_weight.data_ptr(),
-            head_weight_bf16.data_ptr(), head_weight_bf16.shape[0], state.data_ptr(), logits_out.data_ptr()))
+        rc = self._calls.exec_head(self._hv, stream, state, hc_fn, hc_scale, hc_base, norm_weight, head_weight_bf16, logits_out,
+                                   norm_eps, hc_eps)
+        if rc != 0:
+            _refused(rc, state)
 
     def cmd_head_logits(self, x, weight_bf16, logits_out, *, n_rows: Optional[int] = None,
                         stream: Optional[int] = None) -> None:
-        n_tokens = 1 if x.dim() == 1 else x.shape[0]
-        rows = n_rows if n_rows is not None else weight_bf16.shape[0]
-        stride = logits_out.shape[-1]
-        check(L.lib().s14_cmd_head_logits(self._h, stream if stream is not None else _torch_stream(),
-                                          x.data_ptr(), n_tokens, weight_bf16.data_ptr(), rows,
-                                          weight_bf16.shape[1], logits_out.data_ptr(), stride))
+        rc = self._calls.head_logits(self._hv, stream, x, weight_bf16, logits_out, n_rows)
+        if rc:
+            check(rc)
 
     def cmd_greedy_argmax(self, logits, result, stream: Optional[int] = None) -> None:
-        check(L.lib().s14_cmd_greedy_argmax(self._h, stream if stream is not None else _torch_stream(),
-                                            logits.data_ptr(), logits.numel(), result.data_ptr()))
+        rc = self._calls.greedy_argmax(self._hv, stream, logits, result)
+        if rc:
+            check(rc)
 
 
 def _stream_type(t) -> int:
@@ -423,13 +411,14 @@ def _stream_type(t) -> int:
     raise S14Error(L.ERR_CONTRACT, "a token's streams are float32 or bfloat16 tensors")
 
 
-def _hc_params(x, hc_fn, hc_scale, hc_base, iters, norm_eps, hc_eps) -> "L.HcParams":
-    p = L.HcParams()
-    p.n_tokens, p.hc, p.hidden = x.shape[0], x.shape[1], x.shape[2]
-    p.dtype = _stream_type(x)
-    p.sinkhorn_iters, p.norm_eps, p.hc_eps = iters, norm_eps, hc_eps
-    p.hc_fn, p.hc_scale, p.hc_base = hc_fn.data_ptr(), hc_scale.data_ptr(), hc_base.data_ptr()
-    return p
+def _refused(status, streams) -> None:
+    """A call on a token's streams that did not run: None for streams of another type, else the status."""
+    if status is None:
+        _stream_type(streams)
+    check(status)
+
+
+_ROUTE_ITEMS = "a token route holds at most 6 matching ids/weights/pages"
 
 
 @dataclass
@@ -446,7 +435,7 @@ def _layer_desc(routes, shared_page, shared_kind, hidden, inter):
     for t, r in enumerate(routes):
         n = len(r.expert_ids)
         if n > L.EXPERTS_PER_TOKEN or len(r.weights) != n or len(r.pages) != n:
-            raise S14Error(L.ERR_CONTRACT, "a token route holds at most 6 matching ids/weights/pages")
+            raise S14Error(L.ERR_CONTRACT, _ROUTE_ITEMS)
         arr[t].n_routed = n
         for j in range(n):
             arr[t].expert_ids[j] = int(r.expert_ids[j])
@@ -486,12 +475,13 @@ class DecodeStack:
                 setattr(arr[i], field, t.data_ptr() if t is not None else None)
         h = C.c_void_p()
         check(L.lib().s14_stack_create(ctx._h, C.byref(cfg), arr, C.byref(h)))
-        self._h = h
+        self._h, self._hv = h, h.value
         self.hidden, self.n_layers = cfg.hidden, cfg.n_layers
 
     def cmd_decode(self, x, h_out, stream: Optional[int] = None) -> None:
-        check(L.lib().s14_cmd_stack_decode(self._ctx._h, stream if stream is not None else _torch_stream(), self._h,
-                                           x.data_ptr(), h_out.data_ptr()))
+        rc = self._ctx._calls.stack_decode(self._ctx._hv, stream, self._hv, x, h_out)
+        if rc:
+            check(rc)
 
     def decode_host(self, host_x: np.ndarray, host_h: np.ndarray) -> None:
         check(L.lib().s14_stack_decode_host(self._ctx._h, self._h, host_x.ctypes.data, host_h.ctypes.data))
@@ -504,7 +494,7 @@ class DecodeStack:
     def close(self) -> None:
         if self._h:
             L.lib().s14_stack_destroy(self._h)
-            self._h = None
+            self._h = self._hv = None
 
     def __del__(self):
         try:
@@ -522,7 +512,7 @@ class MoeBlock:
         self.hidden, self.inter, self.max_tokens = hidden, inter, max_tokens
         h = C.c_void_p()
         check(L.lib().s14_block_create(ctx.handle, hidden, inter, max_tokens, C.byref(h)))
-        self._h = h
+        self._h, self._hv = h, h.value
 
     def cmd_moe_block(self, x, y, routes: Sequence["TokenRoute"], shared_page: Optional[int],
                       stream: Optional[int] = None) -> None:
@@ -537,15 +527,10 @@ class MoeBlock:
                              weights_out=None, *, score_fn: int = L.SCORE_SIGMOID, top_k: int = 6,
                              route_scale: float = 1.0, stream: Optional[int] = None) -> None:
         """Router on the device: x, y device [n_tokens, hidden]; ids_out / weights_out [n_tokens, top_k]."""
-        d = L.RoutedLayerDesc()
-        d.router = _router_desc(x, wr_bf16, bias, ids_out, weights_out, score_fn, top_k, route_scale)
-        d.inter = self.inter
-        d.shared_kind = L.PAGE_MXFP4
-        d.page_table = page_table.data_ptr()
-        d.shared_page = shared_page
-        d.y = y.data_ptr()
-        check(L.lib().s14_cmd_routed_moe_block(self._ctx.handle, stream if stream is not None else _torch_stream(),
-                                               self._h, C.byref(d)))
+        rc = self._ctx._calls.routed_block(self._ctx._hv, stream, self._hv, x, wr_bf16, bias, page_table, shared_page, L.PAGE_MXFP4,
+                                           self.inter, y, ids_out, weights_out, score_fn, top_k, route_scale)
+        if rc:
+            check(rc)
 
     def cmd_routed_moe_block_experts_ep(self, x, wr_bf16, bias, page_table, shared_page: Optional[int], pairs_out, ids_out,
                                         weights_out, *, ep_rank: int, ep_world: int, shared_owner: int,
@@ -630,7 +615,7 @@ class MoeBlock:
             # follow the order of the header: disconnect everywhere, a host barrier, then destroy
             L.lib().s14_block_ep_disconnect(self._h)
             check(L.lib().s14_block_destroy(self._h))
-            self._h = None
+            self._h = self._hv = None
 
     def __del__(self):
         try:
@@ -680,6 +665,7 @@ class S14NumericPipelines:
 
     def __init__(self, ctx: S14Context):
         self._ctx = ctx
+        self._calls = ctx._calls
 
     def _h(self):
         return self._ctx.handle
@@ -720,23 +706,20 @@ class S14NumericPipelines:
                                               C.byref(d)))
         return d
 
-    def _stream(self, stream):
-        return stream if stream is not None else _torch_stream()
-
     def cmd_mxfp4_matvec(self, dispatch, stream=None) -> None:
-        check(L.lib().s14_cmd_mxfp4_matvec(self._h(), self._stream(stream), C.byref(dispatch)))
+        check(self._calls.mxfp4_matvec(self._ctx._hv, stream, dispatch))
 
     def cmd_fp8_matvec(self, dispatch, stream=None) -> None:
-        check(L.lib().s14_cmd_fp8_matvec(self._h(), self._stream(stream), C.byref(dispatch)))
+        check(self._calls.fp8_matvec(self._ctx._hv, stream, dispatch))
 
     def cmd_swiglu_limit(self, dispatch, stream=None) -> None:
-        check(L.lib().s14_cmd_swiglu_limit(self._h(), self._stream(stream), C.byref(dispatch)))
+        check(self._calls.swiglu_limit(self._ctx._hv, stream, dispatch))
 
     def cmd_route_mix(self, dispatch, stream=None) -> None:
-        check(L.lib().s14_cmd_route_mix(self._h(), self._stream(stream), C.byref(dispatch)))
+        check(self._calls.route_mix(self._ctx._hv, stream, dispatch))
 
     def cmd_moe_accumulate(self, dispatch, stream=None) -> None:
-        check(L.lib().s14_cmd_moe_accumulate(self._h(), self._stream(stream), C.byref(dispatch)))
+        check(self._calls.moe_accumulate(self._ctx._hv, stream, dispatch))
 
 
 def _key(layer: int, kind: int, slot: int) -> L.ExpertKey:
