@@ -49,9 +49,98 @@ __device__ __forceinline__ float dot16_e4m3(const uint4 &q, const float *__restr
 
 // ------------------------------------------------- primitive operators ------
 
-// y[n] = sum_k x[k] * e2m1(w[n,k]) * 2^(s[n,k/32]-127); warp per row.
+// y[n] = sum_k x[k] * e2m1(w[n,k]) * 2^(s[n,k/32]-127).  A matrix of the checkpoint's sizes is 4 MB: launch, first
+// byte and the x reads bound the call, not the bandwidth.  A warp owns NR rows at a time and splits K over its
+// lanes in 16-byte pieces (one scale block each), the pieces of its rows (four each per step) in flight together and
+// the first ones asked for before the wait for the kernel in front (weights do not depend on it).  x lies in
+// shared memory as [eighth of a piece][piece], so that a warp's lanes read consecutive 16 bytes; reading it
+// through the L1 with a 128-byte stride between lanes, one piece in flight, took 10.6 us for 2048 x 4096
+// (this kernel: 3.3).  Two rows per warp halve the x reads, which cost more than the weights (128 bytes for 16),
+// once there are two rows for every warp.
+constexpr uint32_t kMvThreads = 512, kMvBatch = 4, kMvMaxK = 32768;
+template <uint32_t NR>
+__global__ void __launch_bounds__(kMvThreads, 1)
+k_mxfp4_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w, const uint8_t *__restrict__ s,
+                        float *__restrict__ y, uint32_t n_rows, uint32_t k) {
+    extern __shared__ __align__(16) float sx[];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, groups = k >> 5;
+    const uint32_t n_warps = gridDim.x * (kMvThreads / 32u);
+    const uint32_t batches = (groups + 32u * kMvBatch - 1u) / (32u * kMvBatch);
+    uint4 q[NR][kMvBatch];
+    uint32_t sc[NR][kMvBatch];
+    // rows n, n + n_warps of the step (row, batch); pieces past a row's end and rows past the matrix count as zeros
+    auto fetch = [&](uint32_t n, uint32_t batch) {
+#pragma unroll
+        for (uint32_t r = 0; r < NR; ++r) {
+            const uint32_t row = n + r * n_warps;
+#pragma unroll
+            for (uint32_t j = 0; j < kMvBatch; ++j) {
+                const uint32_t p = (batch * kMvBatch + j) * 32u + lane;
+                const bool there = row < n_rows && p < groups;
+                q[r][j] = there ? ldg_stream(reinterpret_cast<const uint4 *>(w + (size_t)row * (k >> 1)) + p) : make_uint4(0u, 0u, 0u, 0u);
+                sc[r][j] = there ? __ldg(s + (size_t)row * groups + p) : 0u;
+            }
+        }
+    };
+    uint32_t n = warp * gridDim.x + blockIdx.x;  // the CTAs' numbers of rows differ by one at most
+    if (n < n_rows) fetch(n, 0u);
+    cudaGridDependencySynchronize();
+    for (uint32_t i = threadIdx.x; i < (k >> 2); i += kMvThreads)
+        reinterpret_cast<float4 *>(sx)[(i & 7u) * groups + (i >> 3)] = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+    __syncthreads();
+    while (n < n_rows) {
+        double acc[NR];
+#pragma unroll
+        for (uint32_t r = 0; r < NR; ++r) acc[r] = 0.0;
+        const uint32_t next = n + NR * n_warps;
+        for (uint32_t b = 0; b < batches; ++b) {
+            uint4 cur[NR][kMvBatch];
+            uint32_t cs[NR][kMvBatch];
+#pragma unroll
+            for (uint32_t r = 0; r < NR; ++r)
+#pragma unroll
+                for (uint32_t j = 0; j < kMvBatch; ++j) cur[r][j] = q[r][j], cs[r][j] = sc[r][j];
+            if (b + 1u < batches) fetch(n, b + 1u);
+            else if (next < n_rows) fetch(next, 0u);
+#pragma unroll
+            for (uint32_t j = 0; j < kMvBatch; ++j) {
+                const uint32_t p = (b * kMvBatch + j) * 32u + lane;
+                if (p >= groups) break;
+                float2 part[NR];
+#pragma unroll
+                for (uint32_t r = 0; r < NR; ++r) part[r] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) {
+                    const float4 xa = reinterpret_cast<const float4 *>(sx)[(2u * i) * groups + p];
+                    const float4 xb = reinterpret_cast<const float4 *>(sx)[(2u * i + 1u) * groups + p];
+#pragma unroll
+                    for (uint32_t r = 0; r < NR; ++r) {
+                        const uint4 &c = cur[r][j];
+                        uint32_t h0, h1, h2, h3;
+                        e2m1x8_to_h2x4(i == 0u ? c.x : (i == 1u ? c.y : (i == 2u ? c.z : c.w)), h0, h1, h2, h3);
+                        part[r] = __ffma2_rn(h2_to_f2(h0), make_float2(xa.x, xa.y), part[r]);
+                        part[r] = __ffma2_rn(h2_to_f2(h1), make_float2(xa.z, xa.w), part[r]);
+                        part[r] = __ffma2_rn(h2_to_f2(h2), make_float2(xb.x, xb.y), part[r]);
+                        part[r] = __ffma2_rn(h2_to_f2(h3), make_float2(xb.z, xb.w), part[r]);
+                    }
+                }
+#pragma unroll
+                for (uint32_t r = 0; r < NR; ++r) acc[r] += (double)(part[r].x + part[r].y) * ue8m0_to_f64(cs[r][j]);
+            }
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < NR; ++r) {
+            const double v = warp_sum(acc[r]);
+            if (lane == 0u && n + r * n_warps < n_rows) y[n + r * n_warps] = (float)v;
+        }
+        n = next;
+    }
+}
+
+// The same for rows longer than x fits shared memory: a warp per row, x through the L1.
 __global__ void __launch_bounds__(256)
-k_mxfp4_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w,
+k_mxfp4_matvec_long(const float *__restrict__ x, const uint8_t *__restrict__ w,
                         const uint8_t *__restrict__ s, float *__restrict__ y, uint32_t n_rows,
                         uint32_t k) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -281,25 +370,33 @@ k_fp8_matvec_reference(const float *__restrict__ x, const uint8_t *__restrict__ 
     y[(size_t)t * n_rows + n] = sum;
 }
 
+// The element-wise operators wait for the kernel in front of them inside the launch (launch_pdl) and read what it
+// wrote from the L2.
 // s14_swiglu_limit.comp:14-20
 __global__ void k_swiglu_limit(const float *__restrict__ gate, const float *__restrict__ up,
                                float *__restrict__ y, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = swiglu_limit_f32(gate[i], up[i]);
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (i < n) y[i] = swiglu_limit_f32(__ldcg(gate + i), __ldcg(up + i));
 }
 
 // s14_route_mix.comp:16-20
 __global__ void k_route_mix(const float *__restrict__ expert, float *__restrict__ routed, uint32_t n,
                             float weight) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) routed[i] = __fmul_rn(weight, expert[i]);
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (i < n) routed[i] = __fmul_rn(weight, __ldcg(expert + i));
 }
 
 // s14_moe_accumulate.comp:17-21
 __global__ void k_moe_accumulate(const float *__restrict__ expert, float *__restrict__ acc,
                                  uint32_t n, float weight) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) acc[i] = __fadd_rn(acc[i], __fmul_rn(weight, expert[i]));
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (i < n) acc[i] = __fadd_rn(__ldcg(acc + i), __fmul_rn(weight, __ldcg(expert + i)));
 }
 
 // ------------------------------------------------------- fused MoE layer ----
@@ -829,13 +926,37 @@ k_router(const float *__restrict__ x, const uint16_t *__restrict__ wr, const flo
 
 static inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
+// Shared memory for the longest x the row kernels hold, once per device.
+static cudaError_t matvec_smem_attribute() {
+    static bool done[64] = {};
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+    if (done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(k_mxfp4_matvec_pairwise<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMvMaxK * sizeof(float)));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_mxfp4_matvec_pairwise<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMvMaxK * sizeof(float)));
+    done[dev] = e == cudaSuccess;
+    return e;
+}
+
 cudaError_t launch_mxfp4_matvec(cudaStream_t st, uint32_t mode, int sm_count, const float *x,
                                 const uint8_t *w, const uint8_t *s, float *y, uint32_t n, uint32_t k) {
     if (mode == S14_ACCUM_REFERENCE) {
         k_mxfp4_matvec_reference<<<ceil_div(n, 128), 128, 0, st>>>(x, w, s, y, n, k);
     } else {
-        const uint32_t blocks = min(ceil_div(n, 8), (uint32_t)sm_count * 8u);
-        k_mxfp4_matvec_pairwise<<<blocks, 256, 0, st>>>(x, w, s, y, n, k);
+        if (k > kMvMaxK) {
+            k_mxfp4_matvec_long<<<min(ceil_div(n, 8), (uint32_t)sm_count * 8u), 256, 0, st>>>(x, w, s, y, n, k);
+            return cudaGetLastError();
+        }
+        // one CTA of sixteen warps per SM; two rows per warp when every warp has two
+        const cudaError_t e = matvec_smem_attribute();
+        if (e != cudaSuccess) return e;
+        const size_t smem = (size_t)k * sizeof(float);
+        const dim3 grid(min(n, (uint32_t)sm_count)), block(kMvThreads);
+        if (n >= 2u * (kMvThreads / 32u) * (uint32_t)sm_count)
+            return launch_pdl(k_mxfp4_matvec_pairwise<2>, grid, block, smem, st, 0u, x, w, s, y, n, k);
+        return launch_pdl(k_mxfp4_matvec_pairwise<1>, grid, block, smem, st, 0u, x, w, s, y, n, k);
     }
     return cudaGetLastError();
 }
@@ -913,20 +1034,17 @@ cudaError_t launch_fp8_matvec(cudaStream_t st, uint32_t mode, int sm_count, uint
 
 cudaError_t launch_swiglu_limit(cudaStream_t st, const float *gate, const float *up, float *y,
                                 uint32_t n) {
-    k_swiglu_limit<<<ceil_div(n, 256), 256, 0, st>>>(gate, up, y, n);
-    return cudaGetLastError();
+    return launch_pdl(k_swiglu_limit, dim3(ceil_div(n, 256)), dim3(256), 0, st, 0u, gate, up, y, n);
 }
 
 cudaError_t launch_route_mix(cudaStream_t st, const float *expert, float *routed, uint32_t n,
                              float weight) {
-    k_route_mix<<<ceil_div(n, 256), 256, 0, st>>>(expert, routed, n, weight);
-    return cudaGetLastError();
+    return launch_pdl(k_route_mix, dim3(ceil_div(n, 256)), dim3(256), 0, st, 0u, expert, routed, n, weight);
 }
 
 cudaError_t launch_moe_accumulate(cudaStream_t st, const float *expert, float *acc, uint32_t n,
                                   float weight) {
-    k_moe_accumulate<<<ceil_div(n, 256), 256, 0, st>>>(expert, acc, n, weight);
-    return cudaGetLastError();
+    return launch_pdl(k_moe_accumulate, dim3(ceil_div(n, 256)), dim3(256), 0, st, 0u, expert, acc, n, weight);
 }
 
 template <int KC>
