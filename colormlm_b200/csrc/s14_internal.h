@@ -186,7 +186,7 @@ cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float
                              const float *norm_weight, uint32_t hidden, float norm_eps, float hc_eps, float *x_out);
 
 // ---- a block of tokens through one layer, grouped by expert (s14_moe_block.cu) ----
-constexpr uint32_t kBlockNt = 12;  // most tokens of one chunk (two MMAs of N = 96: sixteen digit rows per token)
+constexpr uint32_t kBlockNt = 24;  // most tokens of one chunk (two MMAs of N = 96: eight digit rows per token at least)
 // Up to kBlockNt (token, route) pairs that share an expert page.  The chunks of one expert follow
 // one another: c0 is the first of them, nch their number.
 struct BlockChunk {

@@ -6,8 +6,8 @@
 //
 // The contraction is the one of the one-token layer kernel (s14_moe_umma.cu), widened along N:
 // tcgen05.mma kind::mxf4.block_scale with A = 128 weight rows x 64 K-elements of page bytes as they
-// are, and B = the sixteen balanced base-8 digit rows of EVERY token of a chunk (up to kBlockNt tokens
-// that share the expert: N = 16 * tokens).  Accumulator columns 16 t .. 16 t + 15 hold the digit
+// are, and B = the sixteen balanced base-8 digit rows of EVERY token of a chunk (up to twelve tokens
+// that share the expert: N = 16 * tokens; official arithmetic: eight rows each, up to twenty-four tokens).  Accumulator columns 16 t .. 16 t + 15 hold the digit
 // shares of token t's dot products; added in double and rounded once they give the double-accumulated
 // dot product rounded to F32, so every token's result is bit-identical to what the one-token kernel
 // and the double-accumulating CPU restatement give for that token alone.
@@ -15,7 +15,7 @@
 // Five or six launches per layer, all plain stream order (the routed calls run the router's two launches first):
 //   k_block_digits   x [T, hidden] -> digit tiles (2 KB per token and 256 elements) + block exponents
 //   k_block_group    routes [T, top_k] -> chunks (expert page, <= nt_cap tokens: 2 for small blocks, else 6 or
-//                    12); an item index decodes to (chunk, slice or row tile) from the chunk records
+//                    12; twice as many in the official arithmetic); an item index decodes to (chunk, slice or row tile) from the chunk records
 //   k_block_gemm<0>  up items (chunk, one or two slices of 64 intermediate elements): w1 | w3 units x the
 //                    chunk's token tiles; epilogue: limited SwiGLU, then either the digit tiles of the hidden
 //                    values per (token, route) pair (small blocks) or the hidden values themselves, whose
@@ -47,12 +47,15 @@ namespace s14 {
 
 namespace {
 
-constexpr uint32_t kNt = kBlockNt;          // most tokens of a chunk
-constexpr uint32_t kNtHalf = 6;             // tokens of one MMA: N = 96 accumulator columns
-constexpr uint32_t kAccCols = 16u * kNtHalf;
-static_assert(kNt == 2u * kNtHalf, "a wide chunk is two halves, one per issuing thread");
+// A chunk's B operand is made of groups of sixteen digit rows: one token each, or, in the official arithmetic,
+// whose values need eight digit rows, two tokens (rows 0-7 and 8-15).
+constexpr uint32_t kGrp = 12;               // most groups of a chunk
+constexpr uint32_t kGrpHalf = 6;            // groups of one MMA: N = 96 accumulator columns
+constexpr uint32_t kAccCols = 16u * kGrpHalf;
+static_assert(kGrp == 2u * kGrpHalf, "a wide chunk is two halves, one per issuing thread");
+static_assert(kBlockNt == 2u * kGrp, "a chunk record holds the tokens of the official arithmetic's chunks");
 constexpr uint32_t kStageA = kUnitStride;                  // a unit's codes, then its scales
-// a ring stage: a unit, then the token tiles (2 KB each) of the unit's K range for as many tokens as a chunk may hold
+// a ring stage: a unit, then the token tiles of the unit's K range (2 KB per group) for as many groups as a chunk may hold
 static_assert(kStageA % 1024u == 0u && 2048u % 1024u == 0u, "operand tiles keep the 1 KB alignment of the 128-byte swizzle");
 constexpr uint32_t kGThreads = 512;
 constexpr uint32_t kGRingMax = 12;
@@ -104,6 +107,10 @@ struct GemmArgs {
 
 // torch's .to(torch.bfloat16).float()
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+// two values rounded the same way: the first in the lower half of the word
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16;
+}
 
 // The nearest E4M3FN value (ties to even) of |v| <= 448: three mantissa bits; below 2^-6 multiples of 2^-9.
 __device__ __forceinline__ float e4m3fn_round(float v) {
@@ -123,15 +130,21 @@ __device__ __forceinline__ float e4m3fn_round(float v) {
 // (l42_real_reference/l42_reference.py:389-403): per 128 elements amax = max(|x|, 1e-4), scale =
 // 2^ceil(log2(amax / 448)) (F32 quotient, the logarithm taken in double and rounded to F32), x / scale
 // clipped to +-448, rounded to E4M3FN, times the scale.  The quantised values are F32 values with four
-// significant bits, which the digit rows hold exactly.
+// significant bits: within a scale block, whose largest magnitude is below 2^E, all are multiples of
+// 2^(E-18) (the smallest E4M3FN step is 2^-18 of the range's end), so the eight upper digit rows hold them and
+// the lower eight would be zero.  A tile then is 1 KB (eight rows) and two tokens share sixteen operand rows: half
+// the tile bytes and twice the tokens per pass over a page (official layer of 1000 tokens at 4096 x 2048:
+// 2458 -> 1894 us).
+template <bool kQuant>
 __global__ void __launch_bounds__(512)
-k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t quant) {
+k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps) {
+    constexpr uint32_t kRows = kQuant ? 8u : 16u;
     const uint32_t v = blockIdx.x, g = threadIdx.x;
     if (g >= (K >> 3)) return;  // whole warps leave: K is a multiple of 256
     const float4 p0 = __ldg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
     const float4 p1 = __ldg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
     float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-    if (quant) {
+    if constexpr (kQuant) {
         // a group of 128 elements is sixteen neighbouring threads
         float am = 0.0f;
 #pragma unroll
@@ -146,7 +159,7 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
         for (int i = 0; i < 8; ++i)
             xs[i] = __fmul_rn(e4m3fn_round(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f)), scale);
     }
-    digits_of8(xs, g, dig + (size_t)v * (K >> 8) * 2048u, exps + (size_t)v * (K >> 5));
+    digits_of8<(int)kRows>(xs, g, dig + (size_t)v * (K >> 8) * (kRows * 128u), exps + (size_t)v * (K >> 5));
 }
 
 // Groups the block's (token, route) pairs by expert.  Group 0 is the shared expert (every token, mix
@@ -256,11 +269,12 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 }
 
 // An item as the CTA's roles read it, decoded once per batch into shared memory.
+template <uint32_t kTok>
 struct ItemRec {
     unsigned long long page;
     uint32_t nt, r;            // pairs of the chunk; slice (up) or row tile (down)
-    uint32_t tok[kNt];
-    uint32_t pair[kNt];
+    uint32_t tok[kTok];
+    uint32_t pair[kTok];
 };
 // kMt: row tiles (slices of the up phase) per item.
 //   1 (small blocks): chunks of up to six tokens (the host uses two); the two issuing threads take the even and
@@ -278,11 +292,14 @@ __global__ void __launch_bounds__(kGThreads, 1)
 k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kGBars];
-    constexpr uint32_t kTok = kWide ? kNt : kNtHalf;   // most tokens of a chunk in this shape
-    constexpr uint32_t kBatch = kWide ? 96u : 48u;     // items decoded at a time (the records share the static shared memory with the ring)
-    __shared__ __align__(16) ItemRec s_rec[kBatch];
+    constexpr uint32_t kTpg = kMode == kModeOfficial ? 2u : 1u;   // tokens per group of sixteen digit rows
+    constexpr uint32_t kRows = 16u / kTpg, kTileB = kRows * 128u; // a token's digit rows, and the bytes of its tile
+    constexpr uint32_t kHalf = kGrpHalf * kTpg;                   // most tokens of one MMA
+    constexpr uint32_t kTok = kWide ? 2u * kHalf : kHalf;         // most tokens of a chunk in this shape
+    constexpr uint32_t kBatch = kWide && kTpg == 1u ? 96u : 48u;  // items decoded at a time (the records share the static shared memory with the ring)
+    __shared__ __align__(16) ItemRec<kTok> s_rec[kBatch];
     __shared__ float s_up[kTok][64];                          // an item's up projections (even tokens) and gates (odd tokens), handed across
-    __shared__ __align__(16) uint8_t s_hst[kTok][16 * 2 * 16]; // an up item's digit chunks per token: [row][block][16 bytes]
+    __shared__ __align__(16) uint8_t s_hst[!kDown && kMode == kModeFused ? kTok : 1u][16 * 2 * 16]; // an up item's digit chunks per token: [row][block][16 bytes]
     __shared__ uint32_t tmem_slot, s_units;
     __shared__ int abort_flag;
 
@@ -351,12 +368,12 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
             const uint32_t c0 = __ldg(&g->c0), nch = __ldg(&g->nch), j = q - c0 * R;
             const uint32_t r = j / nch;
             const BlockChunk *ch = a.chunks + c0 + (j - r * nch);
-            ItemRec rec;
+            ItemRec<kTok> rec;
             rec.page = __ldg(reinterpret_cast<const unsigned long long *>(&ch->page));
             rec.nt = __ldg(&ch->nt) | (nch > 1u ? 0x100u : 0u);
             rec.r = r;
 #pragma unroll
-            for (uint32_t t = 0; t < kNt; ++t) {
+            for (uint32_t t = 0; t < kTok; ++t) {
                 rec.tok[t] = __ldg(&ch->tok[t]);
                 rec.pair[t] = __ldg(&ch->pair[t]);
             }
@@ -379,7 +396,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                         break;
                     }
                     const uint32_t full = bar(kGBarFull + p_slot), dst = smem_u32(sRing) + p_slot * a.stage;
-                    mbar_arrive_expect(full, kMt * kStageA + (a.by_threads ? 0u : (s_rec[i].nt & 0xFFu) * 2048u));
+                    mbar_arrive_expect(full, kMt * kStageA + (a.by_threads ? 0u : (s_rec[i].nt & 0xFFu) * kTileB));
                     // an expert with one chunk is read once; with more, its later chunks want the units in the L2
 #pragma unroll
                     for (uint32_t mt = 0; mt < kMt; ++mt) {
@@ -402,9 +419,9 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i) {
                 const uint32_t nt = s_rec[i].nt & 0xFFu;
-                uint32_t vec[kNtHalf];   // (small blocks: chunks of up to six tokens)
+                uint32_t vec[kHalf];   // (small blocks: chunks of one MMA)
 #pragma unroll
-                for (uint32_t t = 0; t < kNtHalf; ++t) vec[t] = kDown ? s_rec[i].pair[t] : s_rec[i].tok[t];
+                for (uint32_t t = 0; t < kHalf; ++t) vec[t] = kDown ? s_rec[i].pair[t] : s_rec[i].tok[t];
 #pragma unroll 1
                 for (uint32_t u = 0; u < nu; ++u) {
                     if (p_round && !mbar_wait(bar(kGBarDone + p_slot), (p_round - 1u) & 1u, abortp)) {
@@ -413,8 +430,8 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                     }
                     const uint32_t full = bar(kGBarFull + p_slot), dst = smem_u32(sRing) + p_slot * a.stage + kMt * kStageA;
 #pragma unroll
-                    for (uint32_t t = 0; t < kNtHalf; ++t)
-                        if (t < nt) bulk_copy(dst + t * 2048u, a.dig + ((size_t)vec[t] * nu + u) * 2048u, 2048u, full);
+                    for (uint32_t t = 0; t < kHalf; ++t)
+                        if (t < nt) bulk_copy(dst + t * kTileB, a.dig + ((size_t)vec[t] * nu + u) * kTileB, kTileB, full);
                     if (++p_slot == ring) {
                         p_slot = 0;
                         ++p_round;
@@ -429,14 +446,15 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
             constexpr uint32_t kStep = kWide ? 1u : 2u;
             const uint64_t a_desc0 = smem_desc(smem_u32(sRing), 1, 64, 2);
             const uint64_t sf_desc0 = smem_desc(smem_u32(sRing) + kUnitBytes, 0, 8, 0);
-            const uint64_t b_desc0 = smem_desc(smem_u32(sRing) + kMt * kStageA + (kWide ? m * kNtHalf * 2048u : 0u), 1, 64, 2);
+            const uint64_t b_desc0 = smem_desc(smem_u32(sRing) + kMt * kStageA + (kWide ? m * kGrpHalf * 2048u : 0u), 1, 64, 2);
             const uint32_t sfa_t = tmem + kGColSfa + m * 16u, sfb_t = tmem + kGColSfb + m * 16u;
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
-                const uint32_t buf = gi & 1u, nt_all = s_rec[i].nt & 0xFFu;
-                const uint32_t nt_m = !kWide ? nt_all
-                                             : (m == 0u ? (nt_all < kNtHalf ? nt_all : kNtHalf) : (nt_all > kNtHalf ? nt_all - kNtHalf : 0u));
-                const uint32_t idesc = umma_idesc_mxf4(16u * (nt_m ? nt_m : 1u));
+                const uint32_t buf = gi & 1u, ng = ((s_rec[i].nt & 0xFFu) + kTpg - 1u) / kTpg;
+                // this thread's groups (the second half of a last, half-filled group is stale bytes with scales of one:
+                // accumulator columns that nobody reads)
+                const uint32_t ng_m = !kWide ? ng : (m == 0u ? (ng < kGrpHalf ? ng : kGrpHalf) : (ng > kGrpHalf ? ng - kGrpHalf : 0u));
+                const uint32_t idesc = umma_idesc_mxf4(16u * (ng_m ? ng_m : 1u));
                 // one row tile per item: the accumulators of item gi - 2 have been read; two: those of item gi - 1
                 if (kMt == 1u) {
                     if (gi >= 2u) ok = mbar_wait(bar(kGBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
@@ -459,7 +477,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                         m_slot -= ring;
                         ++m_round;
                     }
-                    if (nt_m) {
+                    if (ng_m) {
                         fence_async_smem();  // the token tiles came by the threads' own copies: the tensor cores read them
                         fence_after();
                         const uint64_t sfd = sf_desc0 + s * (a.stage >> 4), sbd = sfb_desc0 + ku * (1024u >> 4);
@@ -499,19 +517,26 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                 ok = epi_all(mbar_wait(bar(kGBarAccDone + buf), (gi >> 1) & 1u, abortp));
                 if (!ok) break;
                 fence_after();
-                float v[kMt][kTok];
-                // two loads of sixteen columns in flight per wait: the two issuing threads' accumulators of one token
-                // (even and odd stages), or, in wide chunks, two neighbouring tokens of the half that holds them
+                // the row's results; official arithmetic: BF16 values, two tokens to a register
+                constexpr bool kOff = kMode == kModeOfficial;
+                float v[kOff ? 1u : kMt][kOff ? 1u : kTok] = {};
+                uint32_t vb[kOff ? kMt : 1u][kOff ? kTok / 2u : 1u] = {};
+                auto value = [&](uint32_t mt, uint32_t t) -> float {
+                    if constexpr (kOff) return __uint_as_float((t & 1u) ? vb[mt][t >> 1] & 0xFFFF0000u : vb[mt][t >> 1] << 16);
+                    else return v[mt][t];
+                };
+                // two loads of sixteen columns in flight per wait: the two issuing threads' accumulators of one group
+                // (even and odd stages), or, in wide chunks, two neighbouring groups of the half that holds them
+                constexpr uint32_t kStep = (kWide ? 2u : 1u) * kTpg;
 #pragma unroll
                 for (uint32_t mt = 0; mt < kMt; ++mt) {
 #pragma unroll
-                    for (uint32_t t = 0; t < kTok; t += (kWide ? 2u : 1u)) {
-                        v[mt][t] = 0.0f;
-                        if (kWide) v[mt][t + (kWide ? 1u : 0u)] = 0.0f;
+                    for (uint32_t t = 0; t < kTok; t += kStep) {
                         if (t < nt) {  // uniform in the CTA
                             uint32_t r0[16], r1[16];
-                            const uint32_t col0 = kWide ? (mt * 2u + t / kNtHalf) * kAccCols + 16u * (t % kNtHalf)
-                                                        : ((kMt == 1u ? buf : mt) * 2u) * kAccCols + 16u * t;
+                            const uint32_t g = t / kTpg;
+                            const uint32_t col0 = kWide ? (mt * 2u + g / kGrpHalf) * kAccCols + 16u * (g % kGrpHalf)
+                                                        : ((kMt == 1u ? buf : mt) * 2u) * kAccCols + 16u * g;
                             const uint32_t col1 = kWide ? col0 + 16u : col0 + kAccCols;
                             tmem_ld16(lane_base + kGColAcc + col0, r0);
                             tmem_ld16(lane_base + kGColAcc + col1, r1);
@@ -524,9 +549,17 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                                 lo1 += (double)__uint_as_float(r1[8 + c]);
                                 hi1 += (double)__uint_as_float(r1[c]);
                             }
-                            if (kWide) {
+                            // (results beyond nt are not used)
+                            if constexpr (kTpg == 2u) {
+                                if constexpr (kWide) {
+                                    vb[mt][t >> 1] = bf16_pair((float)hi0, (float)lo0);
+                                    vb[mt][(t >> 1) + 1u] = bf16_pair((float)hi1, (float)lo1);
+                                } else {
+                                    vb[mt][t >> 1] = bf16_pair((float)(hi0 + hi1), (float)(lo0 + lo1));
+                                }
+                            } else if constexpr (kWide) {
                                 v[mt][t] = (float)(lo0 + hi0);
-                                v[mt][t + (kWide ? 1u : 0u)] = (float)(lo1 + hi1);  // unused beyond nt
+                                v[mt][t + 1u] = (float)(lo1 + hi1);
                             } else {
                                 v[mt][t] = (float)((lo0 + hi0) + (lo1 + hi1));
                             }
@@ -544,7 +577,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                         for (uint32_t t = 0; t < kTok; ++t) {
                             if (t < nt) {
                                 const size_t at = (size_t)pair[t] * a.hidden + idx * 128u + row;
-                                const float o = kMode == kModeOfficial ? bf16_round(v[mt][t]) : v[mt][t];   // official: a linear's result is BF16
+                                const float o = value(mt, t);   // (official: a linear's result is BF16)
                                 if (a.ep_world > 1u) {
 #pragma unroll 1
                                     for (uint32_t p = 0; p < a.ep_world; ++p) a.out_peer[p][at] = o;
@@ -566,15 +599,14 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                             // arithmetic (s14_first_real_token/executor.py:712-743): gate and up rounded to BF16,
                             // the limited SwiGLU in F32, times the route's weight (not for the shared expert),
                             // rounded to BF16; the next launch also quantises them per 128 elements.
-                            constexpr bool kOff = kMode == kModeOfficial;
 #pragma unroll
                             for (uint32_t t = 0; t < kTok; ++t)
-                                if (t < nt && (t & 1u) != par) s_up[t][el] = kOff ? bf16_round(v[mt][t]) : v[mt][t];
+                                if (t < nt && (t & 1u) != par) s_up[t][el] = value(mt, t);
                             epi_sync();
 #pragma unroll
                             for (uint32_t t = 0; t < kTok; ++t) {
                                 if (t < nt && (t & 1u) == par) {
-                                    const float other = s_up[t][el], mine = kOff ? bf16_round(v[mt][t]) : v[mt][t];
+                                    const float other = s_up[t][el], mine = value(mt, t);
                                     const float hv = par ? swiglu_limit_f32(other, mine) : swiglu_limit_f32(mine, other);
                                     const uint32_t pr = pair[t];
                                     float wh = hv;
@@ -640,13 +672,14 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
             }
         } else if (warp >= kGLayWarp0) {
             // ---- the scale codes of the chunk's digit rows, as the atoms tensor memory takes (row n of
-            // the operand = 16 * token + digit row: byte (n % 32) * 16 + (n / 32) * 4 + block % 4 of the atom
+            // the operand = 16 * group + digit row (two tokens' rows of eight in the official arithmetic): byte (n % 32) * 16 + (n / 32) * 4 + block % 4 of the atom
             // of four scale blocks); digit row j < 8 of a block with exponent E has the code
             // 127 + E - 23 + 3 j, row 8 + j the code 127 + E - 47 + 3 j; the exponents are stored as E + 100.
             // A thread fetches its words of the item before it waits for the buffer. ----
             const uint32_t lt = tid - kGLayWarp0 * 32u;
             const uint32_t atom = lt >> 7, r32 = (lt >> 2) & 31u, col = lt & 3u;
-            const uint32_t tl = 2u * col + (r32 >> 4), j = r32 & 15u;   // the row's token inside a half, its digit row
+            // the row's group and token inside a half, its digit row
+            const uint32_t gl = 2u * col + (r32 >> 4), tl = gl * kTpg + (r32 & 15u) / kRows, j = r32 & (kRows - 1u);
             const int shift = j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20;
             const uint32_t bias = 0x01010101u * (uint32_t)shift;
 #pragma unroll 1
@@ -657,15 +690,15 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                 // stage: sixteen bytes per copy and thread (cp.async: these bytes do not pass through the
                 // bulk-copy unit that brings the pages; measured 1.83 -> 1.65 ms for 370 tokens, but 151 -> 165 us
                 // for 8), the copies' completion counted on the stage's barrier ----
-                const uint32_t n16 = nt * 128u;   // sixteen-byte pieces of the chunk's tiles of one unit
+                const uint32_t n16 = nt * (kTileB / 16u);   // sixteen-byte pieces of the chunk's tiles of one unit
                 auto copy_tiles = [&](uint32_t u) -> bool {
                     if (p_round && !mbar_wait(bar(kGBarDone + p_slot), (p_round - 1u) & 1u, abortp)) return false;
                     const uint32_t dst0 = smem_u32(sRing) + p_slot * a.stage + kMt * kStageA;
 #pragma unroll 1
                     for (uint32_t c = lt; c < n16; c += kGLayThreads) {
-                        const uint32_t tt = c >> 7, off = (c & 127u) << 4;
-                        const uint8_t *src = a.dig + ((size_t)vecs[tt] * nu + u) * 2048u + off;
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + tt * 2048u + off), "l"(src) : "memory");
+                        const uint32_t tt = c / (kTileB / 16u), off = (c % (kTileB / 16u)) << 4;
+                        const uint8_t *src = a.dig + ((size_t)vecs[tt] * nu + u) * kTileB + off;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + tt * kTileB + off), "l"(src) : "memory");
                     }
                     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar(kGBarFull + p_slot)) : "memory");
                     if (++p_slot == ring) {
@@ -679,8 +712,8 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                 uint32_t ew[kWide ? 2 : 1][16];
 #pragma unroll
                 for (uint32_t h = 0; h < (kWide ? 2u : 1u); ++h) {
-                    const uint32_t t = h * kNtHalf + tl;
-                    const bool mine = tl < kNtHalf && t < nt;
+                    const uint32_t t = h * kHalf + tl;
+                    const bool mine = gl < kGrpHalf && t < nt;
                     const uint32_t vec = mine ? vecs[t] : 0u;
                     const uint32_t *e4 = reinterpret_cast<const uint32_t *>(a.exps + (size_t)vec * (K >> 5)) + atom;
 #pragma unroll
@@ -868,8 +901,8 @@ bool moe_block_ok(int sm_count, uint32_t hidden, uint32_t inter, uint32_t n_expe
         return false;
     if ((hidden & 511u) || (inter & 511u) || hidden < 512u || inter < 512u || hidden > 4096u || inter > 4096u) return false;
     return block_ring(block_dynamic_limit(0), kStageA + 2u * 2048u, true) >= 2u &&
-           block_ring(block_dynamic_limit(1), 2u * kStageA + kNtHalf * 2048u, true) >= 2u &&
-           block_ring(block_dynamic_limit(2), 2u * kStageA + kNt * 2048u, false) >= 2u;
+           block_ring(block_dynamic_limit(1), 2u * kStageA + kGrpHalf * 2048u, true) >= 2u &&
+           block_ring(block_dynamic_limit(2), 2u * kStageA + kGrp * 2048u, false) >= 2u;
 }
 
 size_t moe_block_max_chunks(uint32_t max_tokens) {
@@ -890,17 +923,20 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     uint32_t shape;
     *err = cudaErrorInvalidConfiguration;
     if (official && (ep || pairs_out || !w.hval)) return 0;   // the official arithmetic runs on one GPU
-    if (nt_cap == 0u) shape = n_tokens <= 12u ? 0u : ((uint64_t)n_tokens * top_k >= 3ull * n_experts ? 2u : 1u);
-    else shape = nt_cap <= 2u ? 0u : (nt_cap <= kNtHalf ? 1u : 2u);
-    nt_cap = shape == 0u ? (nt_cap ? nt_cap : 2u) : (shape == 1u ? kNtHalf : kNt);
+    const uint32_t tpg = official ? 2u : 1u;   // tokens per group of sixteen digit rows
+    if (nt_cap == 0u) shape = n_tokens <= 12u ? 0u : ((uint64_t)n_tokens * top_k >= (uint64_t)(3u * tpg) * n_experts ? 2u : 1u);
+    else shape = nt_cap <= 2u ? 0u : (nt_cap <= kGrpHalf ? 1u : 2u);
+    const uint32_t groups = shape == 0u ? (nt_cap ? nt_cap : 2u) : (shape == 1u ? kGrpHalf : kGrp);
+    nt_cap = groups * tpg;
     const uint32_t mt = shape == 0u ? 1u : 2u;
-    const uint32_t stage = mt * kStageA + nt_cap * 2048u;
+    const uint32_t stage = mt * kStageA + groups * 2048u;
     const uint32_t ring = block_ring(block_dynamic_limit(shape), stage, shape != 2u);
     *err = cudaErrorInvalidConfiguration;
     if (ring < 2u || n_tokens == 0u) return 0;
     const uint32_t S = inter >> 6, RT = hidden >> 7;
     const size_t smem = (size_t)ring * stage + 2u * kSfbBytes;
-    k_block_digits<<<n_tokens, 512, 0, st>>>(x, hidden, w.xdig, w.xexp, official ? 1u : 0u);
+    if (official) k_block_digits<true><<<n_tokens, 512, 0, st>>>(x, hidden, w.xdig, w.xexp);
+    else k_block_digits<false><<<n_tokens, 512, 0, st>>>(x, hidden, w.xdig, w.xexp);
     if (ep_world == 0u) ep_world = 1u;
     k_block_group<<<1, 1024, 0, st>>>(ids, pages, page_table, shared_page, n_tokens, top_k, n_experts, S / mt, RT / mt, nt_cap,
                                      w.chunks, w.counts, ep_rank, ep_world, (shared_by_token && ep_world > 1u) ? 1u : 0u);
@@ -909,7 +945,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
         *err = cudaMemsetAsync(pairs_out, 0, (size_t)n_tokens * kPairsPerToken * hidden * sizeof(float), st);
         if (*err != cudaSuccess) return 2;
     }
-    const uint32_t by_threads = nt_cap > 2u ? 1u : 0u;
+    const uint32_t by_threads = shape != 0u ? 1u : 0u;
     GemmArgs up = {w.chunks, w.counts + 1, w.xdig, w.xexp, nullptr, w.hdig, w.hexp, by_threads, hidden, inter, ring, stage};
     GemmArgs down = {w.chunks, w.counts + 2, w.hdig, w.hexp, pairs_out ? pairs_out : w.d, nullptr, nullptr, by_threads, hidden, inter, ring, stage};
     if (ep) {
@@ -940,7 +976,8 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
         if (official) k_block_gemm<false, MT, WIDE, kModeOfficial><<<sm_count, kGThreads, smem, st>>>(up, status);   \
         else if (values) k_block_gemm<false, MT, WIDE, kModeValues><<<sm_count, kGThreads, smem, st>>>(up, status);  \
         else k_block_gemm<false, MT, WIDE, kModeFused><<<sm_count, kGThreads, smem, st>>>(up, status);              \
-        if (values) k_block_digits<<<n_tokens * kPairsPerToken, 512, 0, st>>>(w.hval, inter, w.hdig, w.hexp, official ? 1u : 0u); \
+        if (official) k_block_digits<true><<<n_tokens * kPairsPerToken, 512, 0, st>>>(w.hval, inter, w.hdig, w.hexp);        \
+        else if (values) k_block_digits<false><<<n_tokens * kPairsPerToken, 512, 0, st>>>(w.hval, inter, w.hdig, w.hexp);    \
         if (official) k_block_gemm<true, MT, WIDE, kModeOfficial><<<sm_count, kGThreads, smem, st>>>(down, status);  \
         else k_block_gemm<true, MT, WIDE, kModeFused><<<sm_count, kGThreads, smem, st>>>(down, status);             \
     } while (0)

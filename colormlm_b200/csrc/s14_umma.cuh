@@ -201,7 +201,9 @@ __device__ __forceinline__ int block_exponent(float bm) {
 // elements: sixteen rows of 128 bytes, the 16-byte chunk of scale block kb at position
 // (kb % 8) ^ (row % 8)) and, for the first thread of a scale block, the block's exponent.  Thread g
 // owns one 32-bit word of every digit row; the four lanes of a scale block agree on its exponent,
-// so whole warps call this together.
+// so whole warps call this together.  kRows = 8: the upper 24 bits alone (1 KB tiles of eight rows), for
+// values that are integer multiples of 2^(E-23), whose lower digits are zero.
+template <int kRows = 16>
 __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uint8_t *sB, uint8_t *sE) {
     float bm = 0.0f;
 #pragma unroll
@@ -213,7 +215,7 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
     // Four elements at a time: their code bytes [element][hi digits 0-3, hi 4-7, lo 0-3, lo 4-7] are
     // transposed to [digit row][element] and squeezed to nibbles; the two halves of a row's word are
     // joined at the end.
-    uint32_t half[2][16];
+    uint32_t half[2][kRows];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t c[4][4];
@@ -222,10 +224,10 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
             int hi, lo;
             split_hi_lo(xs[h * 4 + i], up, hi, lo);
             digit_code_bytes(hi, c[i][0], c[i][1]);
-            digit_code_bytes(lo, c[i][2], c[i][3]);
+            if constexpr (kRows == 16) digit_code_bytes(lo, c[i][2], c[i][3]);
         }
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {  // four digit rows at a time
+        for (int q4 = 0; q4 < kRows / 4; ++q4) {  // four digit rows at a time
             uint32_t a[4];
             transpose4(c[0][q4], c[1][q4], c[2][q4], c[3][q4], a);
 #pragma unroll
@@ -233,13 +235,13 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
         }
     }
     // word of digit row j: the codes of elements 0..7 in nibbles 0..7
-    uint32_t words[16];
+    uint32_t words[kRows];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) words[j] = pack_pairs(half[0][j], half[1][j]);
+    for (int j = 0; j < kRows; ++j) words[j] = pack_pairs(half[0][j], half[1][j]);
     const uint32_t kb = g >> 2;
-    uint8_t *chunk = sB + (kb >> 3) * 2048u + (g & 3u) * 4u;
+    uint8_t *chunk = sB + (kb >> 3) * (kRows * 128u) + (g & 3u) * 4u;
 #pragma unroll
-    for (uint32_t j = 0; j < 16; ++j)
+    for (uint32_t j = 0; j < (uint32_t)kRows; ++j)
         *reinterpret_cast<uint32_t *>(chunk + j * 128u + (((kb & 7u) ^ (j & 7u)) << 4)) = words[j];
     if ((g & 3u) == 0u) sE[kb] = (uint8_t)(E + 100);  // the block's exponent, biased
 }

@@ -112,6 +112,38 @@ def test_official_routed_block_with_wide_chunks(ctx, oracle):
         blk.close()
 
 
+@pytest.mark.parametrize("n_tokens,n_experts", [(1, 7), (5, 7), (12, 7), (13, 40), (30, 40), (13, 7), (25, 7), (49, 8)])
+def test_official_chunks_of_every_fill(ctx, oracle, n_tokens, n_experts):
+    """Two tokens share sixteen operand rows: chunks of four (up to 12 tokens), twelve (few pairs per expert) and
+    twenty-four, with odd and half-filled ones among them (the shared expert has all tokens).  Bit-identical to
+    the oracle's official layer of every token."""
+    hidden, inter = 1024, 512
+    g, pages, shared = make_layer(2300 + n_tokens, hidden, inter, n_experts, L.PAGE_MXFP4)
+    x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(synth.activations(g, n_tokens, hidden)))
+    x[0, :32] = 0.0                 # an empty scale block
+    x[n_tokens - 1, 32:160] *= 2.0 ** -30   # far below the clamp of the quantiser's scale
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    table = torch.tensor([p.data_ptr() for p in pages_dev], dtype=torch.int64, device="cuda")
+    wr, bias = synth.router_weight_bf16(g, n_experts, hidden), synth.router_bias(g, n_experts)
+    ids = torch.empty((n_tokens, 6), dtype=torch.int32, device="cuda")
+    wts = torch.empty((n_tokens, 6), dtype=torch.float32, device="cuda")
+    dx = dev(x)
+    dy = torch.full_like(dx, float("nan"))
+    blk = MoeBlock(ctx, hidden, inter, n_tokens)
+    try:
+        blk.set_semantics(True)
+        blk.cmd_routed_moe_block(dx, dev(wr), dev(bias), table, shared_dev.data_ptr(), dy, ids, wts)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0
+        y = dy.cpu().numpy()
+        for t in range(n_tokens):
+            rid, w = [int(v) for v in ids[t].cpu().numpy()], wts[t].cpu().numpy()
+            ref = oracle.official_moe_layer(x[t], [pages[i] for i in rid], w, shared, 0, hidden, inter)
+            assert np.array_equal(y[t].view(np.uint32), ref.view(np.uint32)), t
+    finally:
+        blk.close()
+
+
 def test_official_block_runs_on_one_gpu_only(ctx):
     """The expert-parallel calls refuse an official block, and a block with an exchange refuses the switch."""
     blk = MoeBlock(ctx, 1024, 1024, 8)
