@@ -974,31 +974,17 @@ extern "C" int32_t s14_cmd_stack_decode(s14_ctx *ctx, void *stream, s14_stack *s
         return S14_OK;
     }
     const float *cur = x;
-    if (has_shared && c.shared_kind == S14_PAGE_FP8 && umma_router_ok(ctx->sm_count, c.n_experts) &&
-        fp8_shared_layer_ok(ctx->sm_count, ctx->mode, ctx->umma_scratch(), c.top_k, c.hidden, c.inter)) {
-        // FP8 shared experts: three launches per layer, the layer kernel hands the next token over itself
-        for (uint32_t l = 0; l < c.n_layers; ++l) {
-            FusedRouter fr = stack_router(ctx, stack, l);
-            fr.shared_page = nullptr;
-            fr.y_out = stack->layers[l].y_out;
-            float *next = (l + 1 == c.n_layers) ? h_out : stack->hbuf + (size_t)((l + 1) & 1u) * c.hidden;
-            cudaError_t err;
-            ctx->launches += launch_layer_fp8_shared(st, ctx->sm_count, unused, &fr, stack->layers[l].shared_page, cur, nullptr, nullptr,
-                                                     ctx->h, ctx->d, next, ctx->counters, ctx->umma_scratch(), c.hidden, c.inter,
-                                                     c.residual != 0, &err);
-            ctx->last_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
-            if (err != cudaSuccess) return cuda_fail(err, "S14 stack layer launch");
-            cur = next;
-        }
-        return S14_OK;
-    }
-    // the layers one by one: router and layer kernels into ybuf, then the step to the next token
+    // the layers one by one: router and layer kernels into ybuf, then the step to the next token.  With FP8 shared
+    // experts every expert stays on the F32 register kernels: the tensor-core kernel's sums differ from theirs by
+    // 4e-7 of a layer's output, which the chain of layers amplifies (to 8e-5 after a few), and a decode step's
+    // results are to stay what they are.
+    const bool fp8_shared = has_shared && c.shared_kind == S14_PAGE_FP8;
     for (uint32_t l = 0; l < c.n_layers; ++l) {
         const FusedRouter fr = stack_router(ctx, stack, l);
         cudaError_t err;
         ctx->launches += launch_moe_layer(st, ctx->mode, ctx->sm_count, ctx->dev_table, unused, 1, n_jobs, c.hidden, c.inter,
                                           cur, ctx->h, ctx->d, stack->ybuf, &err, nullptr,
-                                          !has_shared || c.shared_kind == S14_PAGE_MXFP4, ctx->counters, ctx->umma_scratch(), &fr);
+                                          !fp8_shared, ctx->counters, fp8_shared ? nullptr : ctx->umma_scratch(), &fr);
         ctx->last_path = last_layer_path();
         if (err != cudaSuccess) return cuda_fail(err, "S14 stack layer launch");
         float *next = (l + 1 == c.n_layers) ? h_out : stack->hbuf + (size_t)((l + 1) & 1u) * c.hidden;

@@ -84,7 +84,6 @@ struct FusedRouter {
     uint32_t shared_kind;
     uint32_t ep_rank, ep_world, shared_owner;
     uint32_t has_shared;               // every layer has a shared expert (a stack's layers say where)
-    float *y_out;                      // a single layer: its output before the residual [hidden], or NULL
 };
 
 // What one layer of a decode stack brings of its own (device memory, constant during a step): the
@@ -127,11 +126,10 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
 // kernel, which runs the routed experts and adds the shared expert's output last.
 bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const struct UmmaScratch *umma, uint32_t n_routed, uint32_t hidden, uint32_t inter);
 // That layer (three launches): the routed experts' jobs, or a router without the shared expert.  h: [inter], d:
-// [kMaxJobs, hidden] scratch.  With `residual` y = x + moe(x).
+// [kMaxJobs, hidden] scratch.
 int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
                             const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
-                            unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, bool residual,
-                            cudaError_t *err);
+                            unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err);
 // One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or x_bf16 with its F32 values left in x_out;
 // h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096.
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,

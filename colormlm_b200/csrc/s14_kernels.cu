@@ -1104,7 +1104,7 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
         }
         if (shared && fp8_shared_layer_ok(sm_count, mode, umma, n_routed, hidden, inter)) {
             launches = launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
-                                               counters, umma, hidden, inter, false, err);
+                                               counters, umma, hidden, inter, err);
             t_last_layer_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
             return launches;
         }
@@ -1242,13 +1242,12 @@ bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const UmmaScratch *umma, u
 
 int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
                             const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
-                            unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, bool residual,
-                            cudaError_t *err) {
+                            unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err) {
     float *shared_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
     *err = launch_fp8_expert(st, sm_count, x, x_bf16, x_stage, shared_page, h, shared_out, hidden, inter);
     if (*err != cudaSuccess) return 0;
     *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, y, umma->tiles, counters, umma->status, hidden, inter, router,
-                                 nullptr, umma->trace, nullptr, 1, nullptr, residual, shared_out);
+                                 nullptr, umma->trace, nullptr, 1, nullptr, false, shared_out);
     return 3;
 }
 

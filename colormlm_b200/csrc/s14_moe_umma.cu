@@ -301,7 +301,6 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
         else if (lane == 3u) v = (unsigned long long)rt.shared_page;
         else if (lane == 4u) v = (unsigned long long)rt.ids_out;
         else if (lane == 5u) v = (unsigned long long)rt.weights_out;
-        else if (lane == 6u) v = (unsigned long long)rt.y_out;
         reinterpret_cast<unsigned long long *>(&s_layer[0])[lane] = v;
     }
     if (warp == 1u) {

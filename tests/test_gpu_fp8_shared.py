@@ -53,6 +53,8 @@ def test_layer_and_executor_step_with_an_fp8_shared_expert(ctx, oracle, hidden, 
 
 @pytest.mark.parametrize("residual", [True, False])
 def test_stack_with_fp8_shared_experts(ctx, oracle, residual):
+    """A chain of layers stays on the F32 register kernels, whose sums it is to reproduce: a layer's difference of
+    4e-7 grows along the chain."""
     hidden, inter, n_experts, n_layers = 1024, 1024, 24, 3
     host, layers, keep = [], [], []
     for l in range(n_layers):
@@ -69,17 +71,14 @@ def test_stack_with_fp8_shared_experts(ctx, oracle, residual):
     x = synth.activations(synth.rng(5), 1, hidden)[0] * np.float32(0.25)
     h = dev(x)
     try:
-        before = ctx.launch_count
         stack.cmd_decode(h, h)  # in place
         torch.cuda.synchronize()
-        assert ctx.device_status() == 0 and ctx.launch_count - before == 3 * n_layers and ctx.last_layer_path == PATH
+        assert ctx.device_status() == 0 and ctx.last_layer_path == L.LAYER_PATH_F32 | L.LAYER_PATH_ROUTER_KERNEL
         cur = x
         for (pages, shared, wr, bias), ly in zip(host, layers):
             rid, rw, _, _ = oracle.router(cur, wr, bias, 0, 6, 1.0)
             assert np.array_equal(ly["ids"].cpu().numpy(), rid)
             want = oracle.moe_layer_acc64(cur, [pages[i] for i in rid], rw, shared, L.PAGE_FP8, hidden, inter)
-            # the FP8 rows add the sixteen products of a piece in F32 (two chains of eight: at most nine roundings of
-            # 2^-24 of the terms' magnitudes, 3e-7 RMS of the output), which is what the bound of the F32 paths allows
             assert_pairwise_close(oracle, ly["y"].cpu().numpy(), want)
             got = ly["y"].cpu().numpy()
             cur = (cur + got).astype(np.float32) if residual else got
