@@ -1277,148 +1277,99 @@ k_stack_step(const float *__restrict__ x, const float *__restrict__ y, float *ou
 }
 
 // ---- the router for many tokens ----
-// Scores: a CTA holds the BF16 rows of eight experts in shared memory and walks a tile of 32 tokens,
-// one warp per token at a time: logit in double (every product f32 x bf16 is exact in double), score
-// and score + bias in F32 -- the arithmetic of k_router.
-constexpr uint32_t kRbTokens = 32;
-template <uint32_t kRbExperts, uint32_t kRbPerWarp>
-__global__ void __launch_bounds__(256)
-k_router_scores_batch(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
-                      float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
-                      uint32_t n_tokens, uint32_t score_fn) {
-    extern __shared__ __align__(16) uint16_t s_w[];  // [kRbExperts][hidden]
-    const uint32_t e0 = blockIdx.x * kRbExperts, t0 = blockIdx.y * kRbTokens;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t pieces = hidden >> 3;  // 16-byte pieces (8 weights) per row
-    for (uint32_t i = threadIdx.x; i < kRbExperts * pieces; i += blockDim.x) {
-        const uint32_t e = i / pieces, p = i - e * pieces;
-        uint4 q = make_uint4(0u, 0u, 0u, 0u);
-        if (e0 + e < n_experts) q = __ldg(reinterpret_cast<const uint4 *>(wr + (size_t)(e0 + e) * hidden) + p);
-        reinterpret_cast<uint4 *>(s_w)[i] = q;
-    }
-    __syncthreads();
-    // A warp takes kRbPerWarp tokens at a time, a weight's conversion to double serving all of them.  (Measured for
-    // 370 tokens x 256 experts with eight experts per CTA: 165 us with one token per warp, 159 with four - the FP64
-    // FMAs of the vector pipe bound it, not the conversions -, which is why large blocks take k_router_scores_dmma;
-    // small blocks run this kernel with two experts per CTA and one token per warp.)
-    for (uint32_t tb = t0 + warp * kRbPerWarp; tb < t0 + kRbTokens && tb < n_tokens; tb += 8u * kRbPerWarp) {
-        double acc[kRbPerWarp][kRbExperts];
+// Scores on the FP64 matrix pipe: a CTA takes 8 * kMt tokens x 8 * kNt experts, its warps the K range in equal parts
+// (their sums meet in shared memory, in warp order).  mma.m8n8k4.f64 wants one element of A (8 tokens x 4 k) and of B
+// (4 k x 8 experts) per lane and step; which k an element stands for is free as long as A and B agree, so a lane
+// takes eight neighbouring elements of its row (32 bytes of x, 16 of the weights) and feeds them to eight steps:
+// operands go from the L2 to registers, four lanes share a cache line, nothing is staged.  Every f32 and bf16 value is
+// exact in double, so is every product, and the sums are double: score and score + bias are those of k_router.
+//
+// A token's row is read once per 8 * kNt experts and a weight row once per 8 * kMt tokens; both come from the L2.
+// 16 x 16 tiles for large blocks (wider ones leave too few CTAs, narrower ones read x more often); a smaller grid than two CTAs
+// per SM takes 16 x 8, up to eight tokens 8 x 8 with the K range over sixteen warps.  Measured, x 256 experts x 4096:
+// 8 tokens 15 -> 8.3 us, 370 84 -> 40, 1000 166 -> 83 (before: operands staged in shared memory as doubles by 32 x 16
+// tiles with all of K in one warp; up to 32 tokens on the vector pipe); 45 tokens x 192 experts x 2048: 32 -> 10.
+template <uint32_t kMt, uint32_t kNt, uint32_t kWarps>
+__global__ void __launch_bounds__(kWarps * 32u)
+k_router_scores(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
+                float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
+                uint32_t n_tokens, uint32_t score_fn) {
+    __shared__ double s_c[kWarps][kMt * kNt][64];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, row = lane >> 2, col = lane & 3u;
+    const uint32_t e0 = blockIdx.x * (8u * kNt), t0 = blockIdx.y * (8u * kMt);
+    const uint32_t part = hidden / kWarps, first = warp * part + col * 8u;   // a whole number of steps of 32 elements
+    const float *xr[kMt];
+    const uint16_t *wp[kNt];
+    // (a token or expert past the end reads the last one again; its scores are not written)
 #pragma unroll
-        for (uint32_t j = 0; j < kRbPerWarp; ++j)
+    for (uint32_t m = 0; m < kMt; ++m) xr[m] = x + (size_t)min(t0 + m * 8u + row, n_tokens - 1u) * hidden + first;
 #pragma unroll
-            for (uint32_t e = 0; e < kRbExperts; ++e) acc[j][e] = 0.0;
-        for (uint32_t p = lane; p < pieces; p += 32u) {
-            double xv[kRbPerWarp][8];
+    for (uint32_t n = 0; n < kNt; ++n) wp[n] = wr + (size_t)min(e0 + n * 8u + row, n_experts - 1u) * hidden + first;
+    double c[kMt][kNt][2];
 #pragma unroll
-            for (uint32_t j = 0; j < kRbPerWarp; ++j) {
-                // (a token past the block's end reads the last token again; its result is not written)
-                const float *xt = x + (size_t)min(tb + j, n_tokens - 1u) * hidden;
-                const float4 xa = __ldg(reinterpret_cast<const float4 *>(xt + p * 8u));
-                const float4 xb = __ldg(reinterpret_cast<const float4 *>(xt + p * 8u + 4u));
-                xv[j][0] = xa.x, xv[j][1] = xa.y, xv[j][2] = xa.z, xv[j][3] = xa.w;
-                xv[j][4] = xb.x, xv[j][5] = xb.y, xv[j][6] = xb.z, xv[j][7] = xb.w;
-            }
+    for (uint32_t m = 0; m < kMt; ++m)
 #pragma unroll
-            for (uint32_t e = 0; e < kRbExperts; ++e) {
-                const uint4 q = reinterpret_cast<const uint4 *>(s_w + (size_t)e * hidden)[p];
-                const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
-                double w[8];
+        for (uint32_t n = 0; n < kNt; ++n) c[m][n][0] = c[m][n][1] = 0.0;
+    float4 xa[kMt], xb[kMt];
+    uint4 q[kNt];
+    auto load = [&](uint32_t k) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    w[i * 2] = (double)__uint_as_float(wd[i] << 16);
-                    w[i * 2 + 1] = (double)__uint_as_float(wd[i] & 0xffff0000u);
-                }
+        for (uint32_t n = 0; n < kNt; ++n) q[n] = __ldg(reinterpret_cast<const uint4 *>(wp[n] + k));
 #pragma unroll
-                for (uint32_t j = 0; j < kRbPerWarp; ++j) {
-                    double a0 = 0.0, a1 = 0.0;
+        for (uint32_t m = 0; m < kMt; ++m) {
+            xa[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k));
+            xb[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k) + 1);
+        }
+    };
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    load(0);
+#pragma unroll 1
+    for (uint32_t k = 0; k < part; k += 32u) {
+        float a[kMt][8];
+        uint32_t b[kNt][4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        a0 += xv[j][i * 2] * w[i * 2];
-                        a1 += xv[j][i * 2 + 1] * w[i * 2 + 1];
-                    }
-                    acc[j][e] += a0 + a1;
-                }
-            }
+        for (uint32_t m = 0; m < kMt; ++m) {
+            a[m][0] = xa[m].x, a[m][1] = xa[m].y, a[m][2] = xa[m].z, a[m][3] = xa[m].w;
+            a[m][4] = xb[m].x, a[m][5] = xb[m].y, a[m][6] = xb[m].z, a[m][7] = xb[m].w;
         }
 #pragma unroll
-        for (uint32_t j = 0; j < kRbPerWarp; ++j) {
+        for (uint32_t n = 0; n < kNt; ++n) b[n][0] = q[n].x, b[n][1] = q[n].y, b[n][2] = q[n].z, b[n][3] = q[n].w;
+        if (k + 32u < part) load(k + 32u);
 #pragma unroll
-            for (uint32_t e = 0; e < kRbExperts; ++e) {
-                const double sum = warp_sum(acc[j][e]);
-                if (lane == 0 && e0 + e < n_experts && tb + j < n_tokens) {
-                    const float sc = router_score_f32(sum, score_fn);
-                    scores[(size_t)(tb + j) * n_experts + e0 + e] = sc;
-                    select[(size_t)(tb + j) * n_experts + e0 + e] = __fadd_rn(sc, bias ? bias[e0 + e] : 0.0f);
-                }
-            }
-        }
-    }
-}
-
-// The same scores on the FP64 tensor path (B200 runs FP64 FMAs of the vector pipe at a sixteenth of
-// the FP32 rate, and a block of hundreds of tokens needs 0.4 G of them): a CTA takes 32 tokens x 16
-// experts, stages 256 elements of K at a time in shared memory as doubles (every f32 and bf16 value is
-// exact in double, every product of the two exact, the accumulation in double as before, in another order),
-// and its eight warps run mma.m8n8k4.f64 on 8 tokens x 8 experts each.
-constexpr uint32_t kRdTokens = 32, kRdExperts = 16, kRdK = 256, kRdPitch = kRdK + 4;  // pitch: rows 32 bytes apart mod 128
-__global__ void __launch_bounds__(256)
-k_router_scores_dmma(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
-                     float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
-                     uint32_t n_tokens, uint32_t score_fn) {
-    extern __shared__ __align__(16) double s_d[];
-    double *sx = s_d;                           // [kRdTokens][kRdPitch]
-    double *sw = s_d + kRdTokens * kRdPitch;    // [kRdExperts][kRdPitch]
-    const uint32_t e0 = blockIdx.x * kRdExperts, t0 = blockIdx.y * kRdTokens;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t tg = warp & 3u, eg = warp >> 2;
-    double c0 = 0.0, c1 = 0.0;
-    for (uint32_t k0 = 0; k0 < hidden; k0 += kRdK) {
-        __syncthreads();
+        for (uint32_t i = 0; i < 8; ++i) {
+            double av[kMt], bv[kNt];
 #pragma unroll
-        for (uint32_t i = 0; i < kRdTokens * kRdK / 4u / 256u; ++i) {
-            const uint32_t idx = tid + 256u * i, t = idx / (kRdK / 4u), f4 = idx % (kRdK / 4u);
-            // (a token past the block's end reads the last token again; its scores are not written)
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(x + (size_t)min(t0 + t, n_tokens - 1u) * hidden + k0) + f4);
-            double *d = sx + t * kRdPitch + f4 * 4u;
-            *reinterpret_cast<double2 *>(d) = make_double2((double)v.x, (double)v.y);
-            *reinterpret_cast<double2 *>(d + 2) = make_double2((double)v.z, (double)v.w);
-        }
+            for (uint32_t m = 0; m < kMt; ++m) av[m] = (double)a[m][i];
 #pragma unroll
-        for (uint32_t i = 0; i < kRdExperts * kRdK / 8u / 256u; ++i) {
-            const uint32_t idx = tid + 256u * i, e = idx / (kRdK / 8u), p8 = idx % (kRdK / 8u);
-            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(wr + (size_t)min(e0 + e, n_experts - 1u) * hidden + k0) + p8);
-            const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
-            double *d = sw + e * kRdPitch + p8 * 8u;
+            for (uint32_t n = 0; n < kNt; ++n)
+                bv[n] = (double)__uint_as_float((i & 1u) ? b[n][i >> 1] & 0xffff0000u : b[n][i >> 1] << 16);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<double2 *>(d + 2 * j) =
-                    make_double2((double)__uint_as_float(wd[j] << 16), (double)__uint_as_float(wd[j] & 0xffff0000u));
-        }
-        __syncthreads();
-        // A (8 tokens x 4 k, row major): lane holds (row lane / 4, column lane % 4); B (4 k x 8 experts, column
-        // major): lane holds (row lane % 4, column lane / 4), i.e. the expert's row at the same k
-        const double *pa = sx + (tg * 8u + (lane >> 2)) * kRdPitch + (lane & 3u);
-        const double *pb = sw + (eg * 8u + (lane >> 2)) * kRdPitch + (lane & 3u);
-#pragma unroll 8
-        for (uint32_t k = 0; k < kRdK; k += 4u) {
-            const double a = pa[k], b = pb[k];
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                         : "+d"(c0), "+d"(c1)
-                         : "d"(a), "d"(b));
+            for (uint32_t m = 0; m < kMt; ++m)
+#pragma unroll
+                for (uint32_t n = 0; n < kNt; ++n)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                                 : "+d"(c[m][n][0]), "+d"(c[m][n][1])
+                                 : "d"(av[m]), "d"(bv[n]));
         }
     }
     // C (8 x 8): lane holds row lane / 4, columns 2 (lane % 4) and 2 (lane % 4) + 1
-    const uint32_t t = t0 + tg * 8u + (lane >> 2), e = e0 + eg * 8u + (lane & 3u) * 2u;
-    if (t < n_tokens) {
-        if (e < n_experts) {
-            const float sc = router_score_f32(c0, score_fn);
+#pragma unroll
+    for (uint32_t m = 0; m < kMt; ++m)
+#pragma unroll
+        for (uint32_t n = 0; n < kNt; ++n)
+            *reinterpret_cast<double2 *>(&s_c[warp][m * kNt + n][row * 8u + col * 2u]) = make_double2(c[m][n][0], c[m][n][1]);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kMt * kNt * 64u; i += kWarps * 32u) {
+        const uint32_t tile = i >> 6, at = i & 63u;
+        double sum = s_c[0][tile][at];
+#pragma unroll
+        for (uint32_t w = 1; w < kWarps; ++w) sum += s_c[w][tile][at];
+        const uint32_t t = t0 + (tile / kNt) * 8u + (at >> 3), e = e0 + (tile % kNt) * 8u + (at & 7u);
+        if (t < n_tokens && e < n_experts) {
+            const float sc = router_score_f32(sum, score_fn);
             scores[(size_t)t * n_experts + e] = sc;
             select[(size_t)t * n_experts + e] = __fadd_rn(sc, bias ? bias[e] : 0.0f);
-        }
-        if (e + 1u < n_experts) {
-            const float sc = router_score_f32(c1, score_fn);
-            scores[(size_t)t * n_experts + e + 1u] = sc;
-            select[(size_t)t * n_experts + e + 1u] = __fadd_rn(sc, bias ? bias[e + 1u] : 0.0f);
         }
     }
 }
@@ -1428,36 +1379,26 @@ __global__ void __launch_bounds__(256)
 k_router_select_batch(const float *__restrict__ scores, const float *__restrict__ select, uint32_t n_experts, uint32_t n_tokens,
                       uint32_t top_k, float route_scale, int32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
     const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    cudaTriggerProgrammaticLaunchCompletion();
     if (t >= n_tokens) return;
+    cudaGridDependencySynchronize();
     router_select(scores + (size_t)t * n_experts, select + (size_t)t * n_experts, n_experts, top_k, route_scale,
                   ids_out + (size_t)t * top_k, weights_out + (size_t)t * top_k, nullptr, nullptr, nullptr, 0, threadIdx.x & 31u, 0,
                   1, 0);
 }
 
 int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, cudaError_t *err) {
-    // few tokens: two experts per CTA on the vector pipe, so that the grid covers the SMs; many: the FP64 tensor path
-    static bool attr_set[64] = {};
-    int dev = 0;
-    *err = cudaGetDevice(&dev);
+    auto run = [&](auto kernel, uint32_t mt, uint32_t nt, uint32_t warps) {
+        return launch_pdl(kernel, dim3(ceil_div(r.n_experts, 8u * nt), ceil_div(r.n_tokens, 8u * mt)), dim3(warps * 32u), 0, st, 0u, r.x,
+                          r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
+    };
+    if (r.hidden % 512u) *err = cudaErrorInvalidValue;   // (a block object's hidden size)
+    else if (r.n_tokens <= 8u) *err = run(k_router_scores<1, 1, 16>, 1, 1, 16);
+    else if (ceil_div(r.n_tokens, 16u) * ceil_div(r.n_experts, 16u) < 296u) *err = run(k_router_scores<2, 1, 8>, 2, 1, 8);
+    else *err = run(k_router_scores<2, 2, 8>, 2, 2, 8);
     if (*err != cudaSuccess) return 0;
-    const size_t smem_d = (size_t)(kRdTokens + kRdExperts) * kRdPitch * sizeof(double);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        *err = cudaFuncSetAttribute(k_router_scores_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_d);
-        if (*err != cudaSuccess) return 0;
-        attr_set[dev] = true;
-    }
-    if (r.n_tokens <= kRbTokens) {
-        const dim3 grid(ceil_div(r.n_experts, 2u), ceil_div(r.n_tokens, kRbTokens));
-        k_router_scores_batch<2, 1><<<grid, 256, (size_t)2u * r.hidden * sizeof(uint16_t), st>>>(
-            r.x, r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
-    } else {
-        const dim3 grid(ceil_div(r.n_experts, kRdExperts), ceil_div(r.n_tokens, kRdTokens));
-        k_router_scores_dmma<<<grid, 256, smem_d, st>>>(r.x, r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden,
-                                                       r.n_tokens, r.score_fn);
-    }
-    k_router_select_batch<<<ceil_div(r.n_tokens, 8), 256, 0, st>>>(scores, select, r.n_experts, r.n_tokens, r.top_k,
-                                                                  r.route_scale, r.ids_out, r.weights_out);
-    *err = cudaGetLastError();
+    *err = launch_pdl(k_router_select_batch, dim3(ceil_div(r.n_tokens, 8)), dim3(256), 0, st, 0u, (const float *)scores,
+                      (const float *)select, r.n_experts, r.n_tokens, r.top_k, r.route_scale, r.ids_out, r.weights_out);
     return 2;
 }
 
