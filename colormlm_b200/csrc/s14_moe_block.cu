@@ -139,10 +139,11 @@ template <bool kQuant>
 __global__ void __launch_bounds__(512)
 k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps) {
     constexpr uint32_t kRows = kQuant ? 8u : 16u;
-    const uint32_t v = blockIdx.x, g = threadIdx.x;
-    if (g >= (K >> 3)) return;  // whole warps leave: K is a multiple of 256
-    const float4 p0 = __ldg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
-    const float4 p1 = __ldg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
+    const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
+    const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
     float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
     if constexpr (kQuant) {
         // a group of 128 elements is sixteen neighbouring threads
@@ -179,6 +180,8 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     __shared__ unsigned long long gpage[kG];
     __shared__ uint32_t bad;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, G = n_experts + 1u, n = T * top_k;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (tid < kG) {
         cnt[tid] = 0u;
         fill[tid] = 0u;
@@ -188,7 +191,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     if (tid == 0) bad = 0u;
     __syncthreads();
     for (uint32_t i = tid; i < n; i += blockDim.x) {
-        const int32_t e = __ldg(ids + i);
+        const int32_t e = __ldcg(ids + i);
         if (e >= (int32_t)n_experts) bad = 1u;
         else if (e >= 0 && (uint32_t)e % ep_world == ep_rank) atomicAdd(&cnt[1 + e], 1u);  // expert parallel: the experts this rank owns
     }
@@ -232,7 +235,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     __syncthreads();
     if (bad) return;
     for (uint32_t i = tid; i < n; i += blockDim.x) {
-        const int32_t e = __ldg(ids + i);
+        const int32_t e = __ldcg(ids + i);
         if (e < 0 || (uint32_t)e % ep_world != ep_rank) continue;
         const uint32_t g = 1u + (uint32_t)e, t = i / top_k, m = i - t * top_k;
         const uint32_t k = atomicAdd(&fill[g], 1u);
@@ -340,6 +343,9 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
     __syncthreads();
     fence_after();
     const uint32_t tmem = tmem_slot;
+    // barriers and tensor memory are ready; from here on the launch reads what the ones before it leave
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const uint32_t n_items = __ldcg(a.n_items);
     // The CTA's items are q = cta, cta + grid, ...  The chunks of one expert follow one another and so
     // do their items, a row tile's chunks side by side (so that CTAs that run at the same time share
@@ -365,17 +371,17 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
         for (uint32_t i = tid; i < nb; i += kGThreads) {
             const uint32_t q = cta + (base + i) * grid;
             const BlockChunk *g = a.chunks + q / R;
-            const uint32_t c0 = __ldg(&g->c0), nch = __ldg(&g->nch), j = q - c0 * R;
+            const uint32_t c0 = __ldcg(&g->c0), nch = __ldcg(&g->nch), j = q - c0 * R;
             const uint32_t r = j / nch;
             const BlockChunk *ch = a.chunks + c0 + (j - r * nch);
             ItemRec<kTok> rec;
-            rec.page = __ldg(reinterpret_cast<const unsigned long long *>(&ch->page));
-            rec.nt = __ldg(&ch->nt) | (nch > 1u ? 0x100u : 0u);
+            rec.page = __ldcg(reinterpret_cast<const unsigned long long *>(&ch->page));
+            rec.nt = __ldcg(&ch->nt) | (nch > 1u ? 0x100u : 0u);
             rec.r = r;
 #pragma unroll
             for (uint32_t t = 0; t < kTok; ++t) {
-                rec.tok[t] = __ldg(&ch->tok[t]);
-                rec.pair[t] = __ldg(&ch->pair[t]);
+                rec.tok[t] = __ldcg(&ch->tok[t]);
+                rec.pair[t] = __ldcg(&ch->pair[t]);
             }
             s_rec[i] = rec;
         }
@@ -612,7 +618,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                                     float wh = hv;
                                     if constexpr (kOff) {
                                         const uint32_t tok = pr / kPairsPerToken, pos = pr - tok * kPairsPerToken;
-                                        if (pos < S14_EXPERTS_PER_TOKEN) wh = __fmul_rn(hv, __ldg(a.weights + tok * a.top_k + pos));
+                                        if (pos < S14_EXPERTS_PER_TOKEN) wh = __fmul_rn(hv, __ldcg(a.weights + tok * a.top_k + pos));
                                         wh = bf16_round(wh);
                                     }
                                     a.hval[(size_t)pr * a.inter + idx * 64u + el] = wh;
@@ -805,13 +811,17 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
 
 // y[t, n]: the ordered mix of token t (examples/s14_vulkan_numeric.rs:936-946): acc = 0; acc += w * d
 // over the routes in order; acc += d of the shared expert.  With `residual` the layer's input is added
-// (y = x + acc, what a layer of a stack hands to the next); y may be x.
+// (y = x + acc, what a layer of a stack hands to the next); y may be x.  Four outputs
+// per thread, the seven rows' loads in flight together (one value per thread,
+// row after row: 64 us for 1000 tokens of 4096, now 28).
 __global__ void __launch_bounds__(256)
 k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const float *__restrict__ weights,
             uint32_t top_k, int has_shared, float *y, uint32_t hidden, const uint32_t *__restrict__ counts,
             const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_world, uint32_t ep_call,
-            uint32_t wait_limit, uint32_t *status, uint32_t official) {
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
+            uint32_t wait_limit, uint32_t *status, uint32_t official, uint32_t vec) {
+    const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * 4u, t = blockIdx.y;   // hidden is a multiple of four
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (flags) {
         // expert parallel, exchange inside the kernels: every rank's rows of this call are in this rank's buffer
         // when its flag carries the call's number (bounded wait: about a microsecond per poll)
@@ -839,16 +849,47 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
     }
     if (n >= hidden || __ldcg(counts + 3)) return;
     const float *dt = d + (size_t)t * kPairsPerToken * hidden + n;
-    float acc = 0.0f;
+    // (a caller's buffers may lie on any 4-byte boundary)
+    auto load4 = [&](const float *p) {
+        return vec ? __ldcg(reinterpret_cast<const float4 *>(p)) : make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+    };
     // official arithmetic: the route's weight went into the expert's hidden values; the BF16 outputs are added
     // in F32 and the sum is rounded to BF16 (moe_branch, s14_first_real_token/executor.py:716-735)
-    for (uint32_t m = 0; m < top_k; ++m)
-        if (__ldg(ids + t * top_k + m) >= 0)
-            acc = __fadd_rn(acc, official ? __ldcg(dt + (size_t)m * hidden)
-                                          : __fmul_rn(__ldg(weights + t * top_k + m), __ldcg(dt + (size_t)m * hidden)));
-    if (has_shared) acc = __fadd_rn(acc, __ldcg(dt + (size_t)S14_EXPERTS_PER_TOKEN * hidden));
-    if (official) acc = bf16_round(acc);
-    y[(size_t)t * hidden + n] = residual ? __fadd_rn(x[(size_t)t * hidden + n], acc) : acc;
+    float4 row[S14_EXPERTS_PER_TOKEN + 1];
+    float w[S14_EXPERTS_PER_TOKEN];
+    bool there[S14_EXPERTS_PER_TOKEN];
+#pragma unroll
+    for (uint32_t m = 0; m < S14_EXPERTS_PER_TOKEN; ++m) {
+        there[m] = m < top_k && __ldcg(ids + t * top_k + m) >= 0;
+        w[m] = there[m] ? __ldcg(weights + t * top_k + m) : 0.0f;
+        row[m] = there[m] ? load4(dt + (size_t)m * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    constexpr uint32_t kSh = S14_EXPERTS_PER_TOKEN;
+    row[kSh] = has_shared ? load4(dt + (size_t)kSh * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 in = residual ? load4(x + (size_t)t * hidden + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    auto mix = [&](float float4::*c) {
+        float acc = 0.0f;
+#pragma unroll
+        for (uint32_t m = 0; m < S14_EXPERTS_PER_TOKEN; ++m)
+            if (there[m]) acc = __fadd_rn(acc, official ? row[m].*c : __fmul_rn(w[m], row[m].*c));
+        if (has_shared) acc = __fadd_rn(acc, row[kSh].*c);
+        if (official) acc = bf16_round(acc);
+        return residual ? __fadd_rn(in.*c, acc) : acc;
+    };
+    const float4 out = make_float4(mix(&float4::x), mix(&float4::y), mix(&float4::z), mix(&float4::w));
+    float *yt = y + (size_t)t * hidden + n;
+    if (vec) *reinterpret_cast<float4 *>(yt) = out;
+    else yt[0] = out.x, yt[1] = out.y, yt[2] = out.z, yt[3] = out.w;
+}
+
+cudaError_t launch_mix(cudaStream_t st, const float *pairs, const int32_t *ids, const float *weights, uint32_t n_tokens, uint32_t top_k,
+                       bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts, bool residual,
+                       const BlockEp *ep, uint32_t *status, bool official) {
+    const uintptr_t where = (uintptr_t)pairs | (uintptr_t)y | (residual ? (uintptr_t)x : 0u);
+    return launch_pdl(k_block_mix, dim3((hidden + 1023u) / 1024u, n_tokens), dim3(256), 0, st, 0u, pairs, ids, weights, top_k,
+                      has_shared ? 1 : 0, y, hidden, counts, x, residual ? 1u : 0u,
+                      (const unsigned long long *)(ep ? ep->flags : nullptr), ep ? ep->world : 1u, ep ? ep->call : 0u,
+                      ep ? ep->wait_limit : 0u, status, official ? 1u : 0u, (where & 15u) ? 0u : 1u);
 }
 
 constexpr int kMaxDevices = 64;
@@ -935,11 +976,19 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     if (ring < 2u || n_tokens == 0u) return 0;
     const uint32_t S = inter >> 6, RT = hidden >> 7;
     const size_t smem = (size_t)ring * stage + 2u * kSfbBytes;
-    if (official) k_block_digits<true><<<n_tokens, 512, 0, st>>>(x, hidden, w.xdig, w.xexp);
-    else k_block_digits<false><<<n_tokens, 512, 0, st>>>(x, hidden, w.xdig, w.xexp);
+    // The launches are programmatic dependents of one another: a kernel's blocks, barriers and tensor memory are
+    // set up while the one before runs out, and every kernel waits for it before it reads or writes anything.
+    auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps) {
+        if (*err != cudaSuccess) return;
+        *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps);
+    };
+    *err = cudaSuccess;
+    digits(x, n_tokens, hidden, w.xdig, w.xexp);
     if (ep_world == 0u) ep_world = 1u;
-    k_block_group<<<1, 1024, 0, st>>>(ids, pages, page_table, shared_page, n_tokens, top_k, n_experts, S / mt, RT / mt, nt_cap,
-                                     w.chunks, w.counts, ep_rank, ep_world, (shared_by_token && ep_world > 1u) ? 1u : 0u);
+    if (*err == cudaSuccess)
+        *err = launch_pdl(k_block_group, dim3(1), dim3(1024), 0, st, 0u, ids, pages, page_table, shared_page, n_tokens, top_k, n_experts,
+                          S / mt, RT / mt, nt_cap, w.chunks, w.counts, ep_rank, ep_world, (shared_by_token && ep_world > 1u) ? 1u : 0u);
+    if (*err != cudaSuccess) return 1;
     if (pairs_out && !ep) {
         // expert parallel: the pairs of the experts this rank owns; the others stay zero for the sum over the ranks
         *err = cudaMemsetAsync(pairs_out, 0, (size_t)n_tokens * kPairsPerToken * hidden * sizeof(float), st);
@@ -971,38 +1020,32 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
         up.top_k = top_k;
         ++launches;
     }
-#define S14_BLOCK_UP(MT, WIDE)                                                                                  \
-    do {                                                                                                        \
-        if (official) k_block_gemm<false, MT, WIDE, kModeOfficial><<<sm_count, kGThreads, smem, st>>>(up, status);   \
-        else if (values) k_block_gemm<false, MT, WIDE, kModeValues><<<sm_count, kGThreads, smem, st>>>(up, status);  \
-        else k_block_gemm<false, MT, WIDE, kModeFused><<<sm_count, kGThreads, smem, st>>>(up, status);              \
-        if (official) k_block_digits<true><<<n_tokens * kPairsPerToken, 512, 0, st>>>(w.hval, inter, w.hdig, w.hexp);        \
-        else if (values) k_block_digits<false><<<n_tokens * kPairsPerToken, 512, 0, st>>>(w.hval, inter, w.hdig, w.hexp);    \
-        if (official) k_block_gemm<true, MT, WIDE, kModeOfficial><<<sm_count, kGThreads, smem, st>>>(down, status);  \
-        else k_block_gemm<true, MT, WIDE, kModeFused><<<sm_count, kGThreads, smem, st>>>(down, status);             \
+    auto gemm = [&](auto kernel, const GemmArgs &args) {
+        if (*err == cudaSuccess) *err = launch_pdl(kernel, dim3(sm_count), dim3(kGThreads), smem, st, 0u, args, status);
+    };
+#define S14_BLOCK_UP(MT, WIDE)                                                                     \
+    do {                                                                                           \
+        if (official) gemm(k_block_gemm<false, MT, WIDE, kModeOfficial>, up);                      \
+        else if (values) gemm(k_block_gemm<false, MT, WIDE, kModeValues>, up);                     \
+        else gemm(k_block_gemm<false, MT, WIDE, kModeFused>, up);                                  \
+        if (values) digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp);              \
+        if (official) gemm(k_block_gemm<true, MT, WIDE, kModeOfficial>, down);                     \
+        else gemm(k_block_gemm<true, MT, WIDE, kModeFused>, down);                                 \
     } while (0)
     if (shape == 0u) S14_BLOCK_UP(1, false);
     else if (shape == 1u) S14_BLOCK_UP(2, false);
     else S14_BLOCK_UP(2, true);
 #undef S14_BLOCK_UP
-    if (pairs_out) {
-        *err = cudaGetLastError();
-        return launches;
-    }
-    k_block_mix<<<dim3((hidden + 255u) / 256u, n_tokens), 256, 0, st>>>(w.d, ids, weights, top_k, shared_page != nullptr, y, hidden,
-                                                                       w.counts, x, residual ? 1u : 0u, nullptr, 1u, 0u, 0u, status,
-                                                                       official ? 1u : 0u);
-    *err = cudaGetLastError();
+    if (pairs_out || *err != cudaSuccess) return launches;
+    *err = launch_mix(st, w.d, ids, weights, n_tokens, top_k, shared_page != nullptr, x, y, hidden, w.counts, residual, nullptr, status,
+                      official);
     return launches + 1;
 }
 
 cudaError_t launch_block_mix(cudaStream_t st, const float *pairs, const int32_t *ids, const float *weights, uint32_t n_tokens,
                              uint32_t top_k, bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts,
                              const BlockEp *ep, uint32_t *status) {
-    k_block_mix<<<dim3((hidden + 255u) / 256u, n_tokens), 256, 0, st>>>(pairs, ids, weights, top_k, has_shared, y, hidden, counts, x,
-                                                                       x ? 1u : 0u, ep ? ep->flags : nullptr, ep ? ep->world : 1u,
-                                                                       ep ? ep->call : 0u, ep ? ep->wait_limit : 0u, status, 0u);
-    return cudaGetLastError();
+    return launch_mix(st, pairs, ids, weights, n_tokens, top_k, has_shared, x, y, hidden, counts, x != nullptr, ep, status, false);
 }
 
 }  // namespace s14
