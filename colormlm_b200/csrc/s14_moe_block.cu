@@ -354,10 +354,11 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
     const uint32_t n_local = n_items > cta ? (n_items - cta + grid - 1u) / grid : 0u;
 
     const bool is_prod_a = tid == kGProdWarp * 32u, is_prod_b = tid == kGTileWarp * 32u && !a.by_threads;
-    const bool is_issuer = (warp == kGMmaWarp0 || warp == kGMmaWarp0 + 1u) && lane == 0;
+    const uint32_t warp_u = warp_uniform(warp);
+    const bool is_issuer = warp_u == kGMmaWarp0 || warp_u == kGMmaWarp0 + 1u;   // (whole warps)
     // what the roles carry from item to item
     uint32_t p_slot = 0, p_round = 0, p_units = 0;             // the copying threads: next stage
-    uint32_t m_slot = kWide ? 0u : warp - kGMmaWarp0, m_round = 0;   // the issuing threads: their next stage
+    uint32_t m_slot = kWide ? 0u : warp_u - kGMmaWarp0, m_round = 0;   // the issuing warps: their next stage
     uint32_t gi = 0;                                           // items so far
     bool ok = true;
     const unsigned long long once = l2_policy_evict_first();
@@ -448,68 +449,72 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
             // ---- MMA issue.  One row tile per item: thread m takes units m, m + 2, ... of every item (a ring slot
             // always belongs to the same thread: items have an even number of units and the ring an even number
             // of slots).  Two row tiles: thread m takes EVERY stage for its half of the chunk's tokens. ----
-            const uint32_t m = warp - kGMmaWarp0;
+            const uint32_t m = warp_u - kGMmaWarp0, tm = warp_uniform(tmem);
             constexpr uint32_t kStep = kWide ? 1u : 2u;
             const uint64_t a_desc0 = smem_desc(smem_u32(sRing), 1, 64, 2);
             const uint64_t sf_desc0 = smem_desc(smem_u32(sRing) + kUnitBytes, 0, 8, 0);
             const uint64_t b_desc0 = smem_desc(smem_u32(sRing) + kMt * kStageA + (kWide ? m * kGrpHalf * 2048u : 0u), 1, 64, 2);
-            const uint32_t sfa_t = tmem + kGColSfa + m * 16u, sfb_t = tmem + kGColSfb + m * 16u;
+            const uint32_t sfa_t = tm + kGColSfa + m * 16u, sfb_t = tm + kGColSfb + m * 16u;
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
-                const uint32_t buf = gi & 1u, ng = ((s_rec[i].nt & 0xFFu) + kTpg - 1u) / kTpg;
+                const uint32_t buf = gi & 1u, ng = (warp_uniform(s_rec[i].nt & 0xFFu) + kTpg - 1u) / kTpg;
                 // this thread's groups (the second half of a last, half-filled group is stale bytes with scales of one:
                 // accumulator columns that nobody reads)
                 const uint32_t ng_m = !kWide ? ng : (m == 0u ? (ng < kGrpHalf ? ng : kGrpHalf) : (ng > kGrpHalf ? ng - kGrpHalf : 0u));
                 const uint32_t idesc = umma_idesc_mxf4(16u * (ng_m ? ng_m : 1u));
                 // one row tile per item: the accumulators of item gi - 2 have been read; two: those of item gi - 1
                 if (kMt == 1u) {
-                    if (gi >= 2u) ok = mbar_wait(bar(kGBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
+                    if (gi >= 2u) ok = mbar_wait_warp(bar(kGBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
                 } else if (gi >= 1u) {
-                    ok = mbar_wait(bar(kGBarAccFree + ((gi - 1u) & 1u)), ((gi - 1u) >> 1) & 1u, abortp);
+                    ok = mbar_wait_warp(bar(kGBarAccFree + ((gi - 1u) & 1u)), ((gi - 1u) >> 1) & 1u, abortp);
                 }
-                ok = ok && mbar_wait(bar(kGBarSfb + buf), (gi >> 1) & 1u, abortp);
+                ok = ok && mbar_wait_warp(bar(kGBarSfb + buf), (gi >> 1) & 1u, abortp);
                 if (!ok) break;
                 fence_after();
-                const uint32_t acc = tmem + kGColAcc + ((kMt == 1u ? buf : 0u) * 2u + m) * kAccCols;   // row tile mt: + 2 * mt accumulators
+                const uint32_t acc = tm + kGColAcc + ((kMt == 1u ? buf : 0u) * 2u + m) * kAccCols;   // row tile mt: + 2 * mt accumulators
                 // the scale atoms of the item's digit rows: one buffer per item parity, or (wide chunks) per half
                 const uint64_t sfb_desc0 = smem_desc(smem_u32(sSfb) + (kWide ? m : buf) * kSfbBytes, 0, 8, 0);
 #pragma unroll 1
                 for (uint32_t ku = kWide ? 0u : m; ku < nu; ku += kStep) {
                     const uint32_t s = m_slot;
-                    ok = mbar_wait(bar(kGBarFull + s), m_round & 1u, abortp);
+                    ok = mbar_wait_warp(bar(kGBarFull + s), m_round & 1u, abortp);
                     if (!ok) break;
                     m_slot += kStep;
                     if (m_slot >= ring) {
                         m_slot -= ring;
                         ++m_round;
                     }
-                    if (ng_m) {
-                        fence_async_smem();  // the token tiles came by the threads' own copies: the tensor cores read them
-                        fence_after();
-                        const uint64_t sfd = sf_desc0 + s * (a.stage >> 4), sbd = sfb_desc0 + ku * (1024u >> 4);
+                    fence_async_smem();  // the token tiles came by the threads' own copies: the tensor cores read them
+                    fence_after();
+                    if (elect_one()) {
+                        if (ng_m) {
+                            const uint64_t sfd = sf_desc0 + s * (a.stage >> 4), sbd = sfb_desc0 + ku * (1024u >> 4);
 #pragma unroll
-                        for (uint32_t mt = 0; mt < kMt; ++mt) {
-                            tmem_copy_scales(sfa_t + mt * 8u, sfd + mt * (kStageA >> 4));
-                            tmem_copy_scales(sfa_t + mt * 8u + 4u, sfd + mt * (kStageA >> 4) + (kAtomBytes >> 4));
-                        }
-                        tmem_copy_scales(sfb_t, sbd);
-                        tmem_copy_scales(sfb_t + 4u, sbd + (kAtomBytes >> 4));
-                        const uint64_t ad = a_desc0 + s * (a.stage >> 4), bd = b_desc0 + s * (a.stage >> 4);
+                            for (uint32_t mt = 0; mt < kMt; ++mt) {
+                                tmem_copy_scales(sfa_t + mt * 8u, sfd + mt * (kStageA >> 4));
+                                tmem_copy_scales(sfa_t + mt * 8u + 4u, sfd + mt * (kStageA >> 4) + (kAtomBytes >> 4));
+                            }
+                            tmem_copy_scales(sfb_t, sbd);
+                            tmem_copy_scales(sfb_t + 4u, sbd + (kAtomBytes >> 4));
+                            const uint64_t ad = a_desc0 + s * (a.stage >> 4), bd = b_desc0 + s * (a.stage >> 4);
 #pragma unroll
-                        for (uint32_t mt = 0; mt < kMt; ++mt) {
+                            for (uint32_t mt = 0; mt < kMt; ++mt) {
 #pragma unroll
-                            for (uint32_t kk = 0; kk < 4; ++kk) {
-                                const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
-                                umma_mxf4(acc + mt * 2u * kAccCols, ad + mt * (kStageA >> 4) + kk * 2u, bd + kk * 2u,
-                                          idesc | (sfid << 29) | (sfid << 4), (sfa_t + mt * 8u + atom * 4u) | (sfid << 30),
-                                          (sfb_t + atom * 4u) | (sfid << 30), (ku >= kStep || kk) ? 1u : 0u);
+                                for (uint32_t kk = 0; kk < 4; ++kk) {
+                                    const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
+                                    umma_mxf4(acc + mt * 2u * kAccCols, ad + mt * (kStageA >> 4) + kk * 2u, bd + kk * 2u,
+                                              idesc | (sfid << 29) | (sfid << 4), (sfa_t + mt * 8u + atom * 4u) | (sfid << 30),
+                                              (sfb_t + atom * 4u) | (sfid << 30), (ku >= kStep || kk) ? 1u : 0u);
+                                }
                             }
                         }
+                        umma_commit(bar(kGBarDone + s));
                     }
-                    umma_commit(bar(kGBarDone + s));
+                    __syncwarp();
                 }
                 if (!ok) break;
-                umma_commit(bar(kGBarAccDone + buf));
+                if (elect_one()) umma_commit(bar(kGBarAccDone + buf));
+                __syncwarp();
             }
         } else if (warp < 4u) {
             // ---- epilogue: per token of the chunk the two accumulators' sixteen digit columns, added in
@@ -763,8 +768,9 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
     }
     if (is_issuer) {
         // nothing of this CTA's tensor work is in flight when the tensor memory is freed
-        umma_commit(bar(kGBarFin));
-        mbar_wait(bar(kGBarFin), 0, abortp);
+        if (elect_one()) umma_commit(bar(kGBarFin));
+        __syncwarp();
+        mbar_wait_warp(bar(kGBarFin), 0, abortp);
     }
     __syncwarp();
     if (is_prod_a) {

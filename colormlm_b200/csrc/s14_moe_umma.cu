@@ -454,7 +454,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     __syncwarp();
     {
         uint32_t gi0 = 0;                       // items of earlier layers
-        uint32_t m_slot = warp - kMmaWarp0, m_round = 0;  // issuing threads: position in the CTA's sequence of units
+        const uint32_t warp_u = warp_uniform(warp);
+        uint32_t m_slot = warp_u - kMmaWarp0, m_round = 0;  // issuing warps: position in the CTA's sequence of units
         uint32_t n_loaded = 0;                  // digit tiles of hidden values so far (issuing and tile threads)
         bool alive = true;
 #pragma unroll 1
@@ -800,7 +801,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             }
 
             // ---- roles.  Each waits (bounded) until the jobs and the CTA's items are there ----
-            const bool is_issuer = (warp == kMmaWarp0 || warp == kMmaWarp0 + 1u) && lane == 0;
+            const bool is_issuer = warp_u == kMmaWarp0 || warp_u == kMmaWarp0 + 1u;   // (whole warps)
             const bool role_thread = is_issuer || warp < kEpiThreads / 32u || warp >= kLoadWarp0;
             // Where the list is known from the start (`early`), only what needs the routes waits for
             // them: the tile threads (which pick them) here, the epilogue before its first item of a
@@ -814,46 +815,46 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             if (kTrace && tid == 0 && tr) tr[15] = n_items | (ring << 8) | (n_jobs << 16);
 
             if (is_issuer) {
-                // ---- MMA issue.  Issuing a tcgen05 operation costs the thread 70-90 cycles (measured), more
-                // than a 16 KB unit may take, so two threads issue: thread m takes units m, m + 2, ... of every
+                // ---- MMA issue, by two warps (one lane of each): warp m takes units m, m + 2, ... of every
                 // item (every item has an even number of units and the ring an even number of slots, so a slot
-                // always belongs to the same thread, which sees each phase of its barrier) and accumulates
+                // always belongs to the same warp, which sees each phase of its barrier) and accumulates
                 // into an accumulator of its own.  Items alternate between two accumulator buffers. ----
-                const uint32_t m = warp - kMmaWarp0;
+                const uint32_t m = warp_u - kMmaWarp0, tm = warp_uniform(tmem);
+                const uint32_t n_it = __all_sync(0xffffffffu, routes_ok) ? warp_uniform(n_items) : 0u;
                 const uint64_t a_desc0 = smem_desc(smem_u32(sRing), 1, 64, 2);
                 const uint64_t sf_desc0 = smem_desc(smem_u32(sRing) + kUnitBytes, 0, 8, 0);
                 const uint64_t bx_desc0 = smem_desc(smem_u32(sBx), 1, 64, 2);
-                const uint32_t sfa_t = tmem + kColSfa + m * 16u;  // a thread's copies and MMAs execute in issue order
-                bool ok = n_items == 0u || mbar_wait(bar(kBarXReady), par, abortp);
+                const uint32_t sfa_t = tm + kColSfa + m * 16u;  // a thread's copies and MMAs execute in issue order
+                bool ok = n_it == 0u || mbar_wait_warp(bar(kBarXReady), par, abortp);
                 uint32_t cur_job = 0xFFFFFFFFu, hb = 0;
 #pragma unroll 1
-                for (uint32_t i = 0; i < n_items && ok; ++i) {
+                for (uint32_t i = 0; i < n_it && ok; ++i) {
                     const uint32_t gi = gi0 + i;
-                    const uint32_t item = s_items[i], j = (item >> 8) & 0xFFu, buf = gi & 1u;
+                    const uint32_t item = warp_uniform(s_items[i]), j = (item >> 8) & 0xFFu, buf = gi & 1u;
                     const bool down = (item & kItemDown) != 0u;
                     const uint32_t nu = down ? KD : KU;
-                    if (gi >= 2u) ok = mbar_wait(bar(kBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
+                    if (gi >= 2u) ok = mbar_wait_warp(bar(kBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
                     uint64_t b_desc0 = bx_desc0;
-                    uint32_t sfb0 = tmem + kColSfbX;
+                    uint32_t sfb0 = tm + kColSfbX;
                     bool last_user = false;
                     if (down) {
                         if (j != cur_job) {
                             hb = n_loaded & 1u;
-                            ok = ok && mbar_wait(bar(kBarHReady + hb), (n_loaded >> 1) & 1u, abortp);
+                            ok = ok && mbar_wait_warp(bar(kBarHReady + hb), (n_loaded >> 1) & 1u, abortp);
                             cur_job = j;
                             ++n_loaded;
                         }
                         b_desc0 = smem_desc(smem_u32(sBh + hb * tile_bytes), 1, 64, 2);
-                        sfb0 = tmem + kColSfbH + hb * 128u;
-                        last_user = i + 1u >= n_items || ((s_items[i + 1u] >> 8) & 0xFFu) != j;
+                        sfb0 = tm + kColSfbH + hb * 128u;
+                        last_user = i + 1u >= n_it || ((warp_uniform(s_items[i + 1u]) >> 8) & 0xFFu) != j;
                     }
                     if (!ok) break;
                     fence_after();
-                    const uint32_t acc = tmem + kColAcc + (buf * 2u + m) * 16u;
+                    const uint32_t acc = tm + kColAcc + (buf * 2u + m) * 16u;
 #pragma unroll 1
                     for (uint32_t ku = m; ku < nu; ku += 2u) {
                         const uint32_t s = m_slot;
-                        ok = mbar_wait(bar(kBarFull + s), m_round & 1u, abortp);
+                        ok = mbar_wait_warp(bar(kBarFull + s), m_round & 1u, abortp);
                         if (!ok) break;
                         m_slot += 2u;
                         if (m_slot >= ring) {
@@ -862,23 +863,29 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                         }
                         if (ku == 0u) mark(16u + i * 4u);
                         fence_after();
-                        const uint64_t sfd = sf_desc0 + s * (kSlot >> 4);
-                        tmem_copy_scales(sfa_t, sfd);
-                        tmem_copy_scales(sfa_t + 4u, sfd + (kAtomBytes >> 4));
-                        const uint64_t ad = a_desc0 + s * (kSlot >> 4), bd = b_desc0 + ku * (2048u >> 4);
-                        const uint32_t sfb_t = sfb0 + ku * 8u;
+                        if (elect_one()) {
+                            const uint64_t sfd = sf_desc0 + s * (kSlot >> 4);
+                            tmem_copy_scales(sfa_t, sfd);
+                            tmem_copy_scales(sfa_t + 4u, sfd + (kAtomBytes >> 4));
+                            const uint64_t ad = a_desc0 + s * (kSlot >> 4), bd = b_desc0 + ku * (2048u >> 4);
+                            const uint32_t sfb_t = sfb0 + ku * 8u;
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) {
-                            const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
-                            umma_mxf4(acc, ad + kk * 2u, bd + kk * 2u, kIdesc | (sfid << 29) | (sfid << 4),
-                                      (sfa_t + atom * 4u) | (sfid << 30), (sfb_t + atom * 4u) | (sfid << 30),
-                                      (ku >= 2u || kk) ? 1u : 0u);
+                            for (uint32_t kk = 0; kk < 4; ++kk) {
+                                const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
+                                umma_mxf4(acc, ad + kk * 2u, bd + kk * 2u, kIdesc | (sfid << 29) | (sfid << 4),
+                                          (sfa_t + atom * 4u) | (sfid << 30), (sfb_t + atom * 4u) | (sfid << 30),
+                                          (ku >= 2u || kk) ? 1u : 0u);
+                            }
+                            umma_commit(bar(kBarDone + s));
                         }
-                        umma_commit(bar(kBarDone + s));
+                        __syncwarp();
                     }
                     if (!ok) break;
-                    umma_commit(bar(kBarAccDone + buf));
-                    if (down && last_user) umma_commit(bar(kBarHFree + hb));
+                    if (elect_one()) {
+                        umma_commit(bar(kBarAccDone + buf));
+                        if (down && last_user) umma_commit(bar(kBarHFree + hb));
+                    }
+                    __syncwarp();
                 }
             } else if (warp < kEpiThreads / 32u) {
                 // ---- epilogue: the item's two accumulators (sixteen digit columns each) are added in double
@@ -1168,10 +1175,12 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             if (warp == kProdWarp) __syncwarp();
             gi0 += n_items;
         }
-        if ((warp == kMmaWarp0 || warp == kMmaWarp0 + 1u) && lane == 0) {
+        if (warp_u == kMmaWarp0 || warp_u == kMmaWarp0 + 1u) {
             // nothing of this CTA's tensor work is in flight when the tensor memory is freed
-            umma_commit(bar(kBarFin));
-            mbar_wait(bar(kBarFin), 0, abortp);
+            __syncwarp();
+            if (elect_one()) umma_commit(bar(kBarFin));
+            __syncwarp();
+            mbar_wait_warp(bar(kBarFin), 0, abortp);
         }
     }
     if constexpr (kTrace) tr = trace_base();

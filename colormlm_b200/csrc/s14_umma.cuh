@@ -70,6 +70,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     return false;
 }
+// The same wait by a whole warp, which goes on (or gives up) together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+// One lane of a converged warp, always the same.  The issuing warps run their loops with all lanes on values that are
+// the same in all of them, and only the tcgen05 operations sit behind this: their descriptors and addresses can then
+// live in uniform registers, where a lane that runs the loop alone has to move every operand of every operation
+// (70-90 cycles of issue per operation).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0u;
+}
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 // Named barriers, plain and with a vote.  Every thread of the group executes them, whatever it has
 // seen, so a group never splits in front of a barrier; and every one starts by bringing the warp
 // back together, because a lane that has been polling or issuing on its own may still be behind its
