@@ -281,6 +281,9 @@ k_fp8_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w
 // warps takes eight rows, two warps per row (the halves of K), the tokens' activations are staged
 // once per CTA in shared memory, a 16-byte piece of weights is decoded once for all tokens, and the
 // two halves of a row are added through shared memory.  k a multiple of 32, 16-byte aligned operands.
+// A dependent launch: the first weights are asked for before the wait for the kernel in front, the next ones while a
+// piece is worked on (us a call in a queue of calls, before and after: 1024 x 4096 x 8 tokens 12.3 -> 9.8, 4700 x 640 x 8
+// 14.4 -> 11.4, 700 x 8192 x 5 14.4 -> 11.5; one token of 1024 x 4096 7.8 -> 3.1, half of it host time).
 constexpr uint32_t kFp8BlockRows = 8, kFp8BlockThreads = 512;
 template <int NT, bool F32_SCALE>
 __global__ void __launch_bounds__(kFp8BlockThreads)
@@ -294,10 +297,15 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
     // staged as [token][quarter of a piece][piece]: the lanes of a warp, which hold consecutive pieces,
     // then read consecutive 16 bytes (no bank conflicts)
     const uint32_t pieces = k >> 4, per = pieces >> 1;
+    const uint4 *wrow = reinterpret_cast<const uint4 *>(w + (size_t)n * k);
+    uint4 ahead = make_uint4(0u, 0u, 0u, 0u);
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (n < n_rows && lane < per) ahead = ldg_stream(wrow + half * per + lane);
+    cudaGridDependencySynchronize();
     for (uint32_t i = threadIdx.x; i < (NT * k) >> 2; i += kFp8BlockThreads) {
         const uint32_t t = i / (k >> 2), j = i % (k >> 2);
         reinterpret_cast<float4 *>(sx)[(size_t)t * (k >> 2) + (j & 3u) * pieces + (j >> 2)] =
-            __ldg(reinterpret_cast<const float4 *>(x) + i);
+            __ldcg(reinterpret_cast<const float4 *>(x) + i);
     }
     __syncthreads();
     const uint32_t k_groups = (k + 127u) >> 7;
@@ -305,10 +313,10 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc[t] = 0.0;
     if (n < n_rows) {
-        const uint4 *wrow = reinterpret_cast<const uint4 *>(w + (size_t)n * k);
         const size_t srow = (size_t)(n >> 7) * k_groups;
         for (uint32_t p = half * per + lane; p < (half + 1u) * per; p += 32u) {
-            const uint4 q = ldg_stream(wrow + p);
+            const uint4 q = ahead;
+            if (p + 32u < (half + 1u) * per) ahead = ldg_stream(wrow + p + 32u);
             const double sc = fp8_block_scale_f64<F32_SCALE>(scale, srow + (p >> 3));
             const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
             float2 wf[8];
@@ -982,7 +990,9 @@ static bool try_fp8_block(cudaStream_t st, int sm_count, const float *x, const u
     const size_t bytes = (size_t)NT * k * sizeof(float);
     if (n > (uint32_t)sm_count * 32u || (k & 31u) || ((uintptr_t)w & 15u) || ((uintptr_t)x & 15u)) return false;
     if (!fp8_block_smem_ok<NT, F32S>(bytes)) return false;
-    k_fp8_matvec_block<NT, F32S><<<(n + kFp8BlockRows - 1) / kFp8BlockRows, kFp8BlockThreads, bytes, st>>>(x, w, s, y, n, k);
+    // (a launch that is refused leaves its error to the caller's check, as the plain launches do)
+    (void)launch_pdl(k_fp8_matvec_block<NT, F32S>, dim3((n + kFp8BlockRows - 1) / kFp8BlockRows), dim3(kFp8BlockThreads), bytes, st, 0u, x,
+                     w, s, y, n, k);
     return true;
 }
 
