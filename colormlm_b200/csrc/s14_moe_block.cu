@@ -29,13 +29,16 @@
 //
 // Roles inside a GEMM CTA: all threads decode the CTA's items of a batch into shared-memory records; one
 // copying thread (the units of 17 KB page bytes of a ring stage: plain bulk copies, no multicast), two
-// MMA-issuing threads (even and odd stages of an item, accumulators of their own), four epilogue warps, eight
+// MMA-issuing warps (one lane of each; even and odd stages of an item, accumulators of their own), four epilogue warps, eight
 // warps that lay out the digit rows' scale codes of an item in shared memory (tcgen05.cp brings them to
 // tensor memory stage by stage, like the weights' scales) and then, for large blocks, fetch the chunk's token
 // tiles of every stage (cp.async, 16 bytes a thread; for small blocks a second copying thread brings them by
-// bulk copies).  What bounds the kernels is the number of bytes an SM takes in (45-50 GB/s per SM, whether
-// from memory or from the L2), so a large block takes TWO slices or row tiles per item: the token tiles of a
-// K range are fetched once for two units.  With the official expert arithmetic
+// bulk copies).  A large block takes TWO slices or row tiles per item: the token tiles of a K range are fetched once
+// for two units.  What bounds large blocks is the issue of the tcgen05 operations and the accumulator reads between two
+// items, not the copies (370 tokens, up kernel 612 us: 602 without the pages' copies, 594 without the tiles', 419
+// without the MMAs, 536 without the reads; the call 1076 -> 942-990 us since the issuing
+// loops are run by whole warps with one elected lane).
+// With the official expert arithmetic
 // (fast16/research/polaris_meridian_v1/s14_first_real_token/executor.py:712-743) the same contractions run on
 // quantised inputs: k_block_digits quantises per 128 elements to E4M3FN values (which the digit rows hold
 // exactly), the up epilogue works on BF16 gate and up and multiplies by the route weight, the down epilogue
@@ -284,10 +287,10 @@ struct ItemRec {
 //     the odd units of an item, each into an accumulator of its own, and items alternate between two
 //     accumulator buffers, so that an item's epilogue runs under the next item's MMAs.
 //   2 (larger blocks): the chunk's token tiles of a K range are fetched once for two units of page bytes (a
-//     stage holds both units, then the tiles): half the tile bytes, and what an SM takes in is what bounds
-//     these kernels.  Every issuing thread holds an accumulator per row tile and there is no second accumulator
+//     stage holds both units, then the tiles): half the tile bytes.
+//     Every issuing thread holds an accumulator per row tile and there is no second accumulator
 //     buffer (the next item's MMAs wait until the epilogue has read the accumulators, while the ring keeps filling).
-//     kWide (many tokens per expert): a chunk holds up to TWELVE tokens; issuing thread m takes the tokens
+//     kWide (many tokens per expert): a chunk holds up to TWELVE tokens (official arithmetic: 24); issuing warp m takes the tokens
 //     6 m .. 6 m + 5 (its own rows of the tile region, its own scale atoms, N = 96) for EVERY stage: fewer
 //     passes over an expert's page.  Otherwise chunks of six and even / odd stages as with one row tile.
 template <bool kDown, uint32_t kMt, bool kWide, uint32_t kMode>
