@@ -375,3 +375,32 @@ def test_block_rejects_what_it_cannot_run(ctx):
         assert torch.count_nonzero(y[:2]).item() == 0   # zero pages: every output is +0
     finally:
         blk.close()
+
+
+# tiles of the score kernel: up to 8 tokens, 16 x 8 (few tiles), 16 x 16 (at least 296 of them), each with remainders
+@pytest.mark.parametrize("n_tokens,n_experts", [(1, 6), (8, 21), (9, 7), (17, 65), (300, 250), (301, 256)])
+def test_routed_block_scores_at_the_tiles_edges(ctx, oracle, n_tokens, n_experts):
+    """Ids and weights bit-identical to the oracle's router; the mix into a y on a 4-byte boundary equal to the aligned one."""
+    hidden, inter = 512, 512
+    g, pages, shared = make_layer(3100 + n_tokens, hidden, inter, 8, L.PAGE_MXFP4)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    table = torch.tensor([pages_dev[e % 8].data_ptr() for e in range(n_experts)], dtype=torch.int64, device="cuda")
+    wr, bias = synth.router_weight_bf16(g, n_experts, hidden), synth.router_bias(g, n_experts)
+    x = synth.activations(g, n_tokens, hidden)
+    dx, dwr, dbias = dev(x), dev(wr.view(np.int16)), dev(bias)
+    ids = torch.empty((n_tokens, 6), dtype=torch.int32, device="cuda")
+    wts = torch.empty((n_tokens, 6), device="cuda")
+    y = torch.empty_like(dx)
+    odd = torch.empty(n_tokens * hidden + 1, device="cuda")[1:].view(n_tokens, hidden)
+    blk = MoeBlock(ctx, hidden, inter, n_tokens)
+    try:
+        for out in (y, odd):
+            blk.cmd_routed_moe_block(dx, dwr, dbias, table, shared_dev.data_ptr(), out, ids, wts)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and torch.equal(y, odd)
+        for t in range(n_tokens):
+            rid, rw, _, _ = oracle.router(x[t], wr, bias, 0, 6, 1.0)
+            assert np.array_equal(ids[t].cpu().numpy(), rid), t
+            assert np.array_equal(wts[t].cpu().numpy().view(np.uint32), rw.view(np.uint32)), t
+    finally:
+        blk.close()
