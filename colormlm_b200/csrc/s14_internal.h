@@ -131,7 +131,9 @@ int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &route
                             const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
                             unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err);
 // One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or x_bf16 with its F32 values left in x_out;
-// h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096.
+// h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary, x_bf16
+// (or NULL) on an 8-byte one.
+inline bool fp8_expert_takes(const uint16_t *x_bf16) { return (reinterpret_cast<uintptr_t>(x_bf16) & 7u) == 0u; }
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,
                               float *h, float *d, uint32_t hidden, uint32_t inter);
 // Scratch of the tcgen05 layer kernel (s14_moe_umma.cu): per job the digit tile of its hidden

@@ -1113,8 +1113,15 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
             routed.n_jobs = routed.token_job_begin[1] = n_routed;
         }
         if (shared && fp8_shared_layer_ok(sm_count, mode, umma, n_routed, hidden, inter)) {
-            launches = launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
-                                               counters, umma, hidden, inter, err);
+            // the expert's kernel reads a BF16 token in 8-byte pieces; a token on another boundary is converted first
+            if (!fp8_expert_takes(x_bf16)) {
+                *err = launch_bf16_to_f32(st, x_bf16, x_stage, hidden);
+                if (*err != cudaSuccess) return launches;
+                ++launches;
+                x_bf16 = nullptr;
+            }
+            launches += launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
+                                                counters, umma, hidden, inter, err);
             t_last_layer_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
             return launches;
         }

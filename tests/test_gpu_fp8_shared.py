@@ -51,6 +51,33 @@ def test_layer_and_executor_step_with_an_fp8_shared_expert(ctx, oracle, hidden, 
     assert torch.equal(branch, y[0].to(torch.bfloat16)) and torch.equal(state, merged)
 
 
+# elements past a 16-byte boundary: 2-, 4- and 8-byte ones; the state and the branch lie there too
+@pytest.mark.parametrize("offset", [1, 2, 4])
+@pytest.mark.parametrize("kind", [L.PAGE_FP8, L.PAGE_MXFP4])
+def test_executor_step_of_buffers_on_any_boundary(ctx, kind, offset):
+    hidden, inter, routed = 2048, 1024, 2
+    g, pages, shared = make_layer(5, hidden, inter, routed, kind)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter, kind)
+    route = TokenRoute(list(range(routed)), np.asarray([0.7, 0.4], np.float32), [p.data_ptr() for p in pages_dev])
+    x, residual = (dev(a).to(torch.bfloat16) for a in (synth.activations(g, 1, hidden)[0], synth.hc_streams(g, 1, hidden)[0]))
+    post, comb = dev(g.uniform(0.2, 1.8, 4).astype(np.float32)), dev(g.uniform(0.05, 0.6, (4, 4)).astype(np.float32))
+
+    def moved(a):
+        big = torch.empty(a.numel() + offset, dtype=a.dtype, device="cuda")
+        big[offset:] = a.reshape(-1)
+        return big[offset:].view(a.shape)
+
+    outs = []
+    for place in (lambda a: a, moved):
+        state, branch = place(torch.zeros_like(residual)), place(torch.zeros_like(x))
+        ctx.exec_routed_and_shared_moe_then_hc_post(place(x), place(residual), post, comb, route, shared_dev.data_ptr(), kind, inter,
+                                                    state, branch)
+        outs.append((state, branch))
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0 and torch.count_nonzero(outs[0][1]) > 0
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("residual", [True, False])
 def test_stack_with_fp8_shared_experts(ctx, oracle, residual):
     """A chain of layers stays on the F32 register kernels, whose sums it is to reproduce: a layer's difference of
