@@ -61,6 +61,27 @@ __device__ __forceinline__ void head_parts(float v, uint32_t (&p)[3]) {
     p[2] = *reinterpret_cast<const uint16_t *>(&l);
 }
 
+// One row's dot product by a whole warp as k_head_logits takes it, for the sums that the parts get wrong: an infinite
+// weight times a part that is zero is NaN, two parts of opposite sign make inf - inf of it, and a product near the
+// largest float overflows in two parts at once.  Out of line: its callers are never there with ordinary numbers, and
+// k_head_mma has no register to spare.
+__device__ __noinline__ float head_row_dot(const float *x, const uint16_t *w, uint32_t hidden) {
+    double acc = 0.0;
+#pragma unroll 1
+    for (uint32_t p = threadIdx.x & 31u; p < (hidden >> 3); p += 32u) {
+        const uint4 q = ldg_stream(reinterpret_cast<const uint4 *>(w) + p);
+        const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
+        float2 part = make_float2(0.f, 0.f);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const float2 xv = __ldcg(reinterpret_cast<const float2 *>(x + p * 8u) + i);
+            part = __ffma2_rn(make_float2(__uint_as_float(wd[i] << 16), __uint_as_float(wd[i] & 0xffff0000u)), xv, part);
+        }
+        acc += (double)part.x + (double)part.y;
+    }
+    return (float)warp_sum(acc);
+}
+
 __global__ void __launch_bounds__(kHeadThreads, 1)
 k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
            uint32_t out_stride, uint32_t n_tokens, uint32_t phases) {
@@ -175,7 +196,17 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
                         } else {
                             // lane holds rows g, g + 8 of the tile and tokens 2 q, 2 q + 1
                             const uint32_t row = (blockIdx.x + i * grid) * 16u + g + (e >> 1) * 8u, t = 2u * q + (e & 1);
-                            if (row < n_rows && t < n_tokens) out[(size_t)t * out_stride + row] = (float)acc[e];
+                            const bool mine = row < n_rows && t < n_tokens;
+                            if (mine) out[(size_t)t * out_stride + row] = (float)acc[e];
+                            // a sum that is not finite says little about the dot product (head_row_dot)
+                            uint32_t redo = __ballot_sync(0xffffffffu, mine && !isfinite(acc[e]));
+                            while (redo) {
+                                const uint32_t src = __ffs((int)redo) - 1, t_src = 2u * (src & 3u) + (e & 1);
+                                const uint32_t row_src = (blockIdx.x + i * grid) * 16u + (src >> 2) + (e >> 1) * 8u;
+                                const float v = head_row_dot(x + (size_t)t_src * hidden, w + (size_t)row_src * hidden, hidden);
+                                if (lane == src) out[(size_t)t * out_stride + row] = v;
+                                redo &= redo - 1u;
+                            }
                         }
                     }
                 }

@@ -48,6 +48,33 @@ def test_logits_of_infinite_and_largest_values(ctx):
     assert bool((out[1] == x[1, 300] * 0.5).all())
 
 
+# 264: the size that the register kernel takes alone; 4096 with eight tokens: several phases of K
+@pytest.mark.parametrize("tokens,hidden", [(1, 256), (1, 264), (3, 512), (8, 4096)])
+def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden):
+    """One infinite weight gives an infinite logit of its sign (x is finite and nowhere 0), both signs or a NaN give NaN,
+    and a product or sum beyond the largest float is infinite; the rows beside them are the ordinary ones."""
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    inf = float("inf")
+    x = (torch.rand(tokens, hidden, device="cuda", generator=g) + 0.5).to(torch.bfloat16).float()  # the last part is 0
+    x[-1] *= 1.0 + 2.0 ** -20                                                                       # ... or is not
+    w = torch.empty(70, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g)
+    out, plain = torch.empty(tokens, 70, device="cuda"), torch.empty(tokens, 70, device="cuda")
+    ctx.cmd_head_logits(x, w.view(torch.int16), plain)
+    w[3, 7], w[20, hidden - 1], w[33, 0], w[33, hidden // 2], w[41, 9], w[69, 8] = inf, -inf, inf, -inf, float("nan"), 3.3e38
+    w[50, ::2] = -2.0 ** 127
+    x[0, 8] = 3.0
+    ctx.cmd_head_logits(x, w.view(torch.int16), out)
+    assert bool((out[:, 3] == inf).all()) and bool((out[:, 20] == -inf).all()) and bool((out[:, 50] == -inf).all())
+    assert bool(out[:, [33, 41]].isnan().all()) and float(out[0, 69]) == inf
+    others = [r for r in range(70) if r not in (3, 20, 33, 41, 50, 69)]
+    assert torch.equal(out[1:, others], plain[1:, others]) and bool(out[:, others].isfinite().all())
+    # the greedy token is the row with the positive infinity (without the NaN rows)
+    out[:, [33, 41]] = 0.0
+    token = torch.empty(1, dtype=torch.int64, device="cuda")
+    ctx.cmd_greedy_argmax(out[0].contiguous(), token)
+    assert int(token) == 3
+
+
 @pytest.mark.parametrize("vocab,offset", [(1, 0), (3, 0), (2047, 1), (4096, 0), (16385, 0), (129280, 0), (129281, 3)])
 def test_greedy_token(ctx, vocab, offset):
     g = np.random.default_rng(vocab)
