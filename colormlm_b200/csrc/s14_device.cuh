@@ -58,11 +58,31 @@ __device__ __forceinline__ float ue8m0_to_f32(uint32_t code) {
     return __uint_as_float(code == 0u ? 0x00400000u : (code << 23));
 }
 
+// Weights that a kernel reads once.  ldg_stream takes the non-coherent path, which wants them unchanged from the
+// kernel's start to its end: for kernels that start when what precedes them is complete.  A kernel that waits for
+// it inside (launch_pdl) has ld_stream and, for what its warps share, ld_u8 and ld_f32.
 __device__ __forceinline__ uint4 ldg_stream(const uint4 *p) {
     uint4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_stream(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_u8(const uint8_t *p) {
+    uint32_t v;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_f32(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 
@@ -124,11 +144,24 @@ __device__ __forceinline__ PageView page_view(const uint8_t *page, uint32_t kind
     return v;
 }
 
+// The dependency calls of a kernel launched by launch_pdl: wait until what precedes the launch in the stream is complete
+// and its writes are visible, then let the launch behind be set up.  In this order a launch's set-up can overlap the
+// kernel directly in front of it alone: everything before that one is complete.
+__device__ __forceinline__ void dependency_wait() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+// A hint that the lines at p will be read: allowed in front of dependency_wait() even where an earlier kernel of the
+// stream still writes them, because it brings them to the L2, which that kernel's stores go through, and no value
+// to this kernel.
+__device__ __forceinline__ void l2_hint(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // A launch as a programmatic dependent of what precedes it in the stream, optionally in clusters of
-// `cluster` CTAs (0: none).  The kernels launched so wait with cudaGridDependencySynchronize() before they
-// touch anything an earlier kernel writes; in front of it they read only what no kernel of this library
-// writes (weights, pages, tables).  A kernel that does not trigger early (any kernel of the caller) is
-// complete before such a launch starts.
+// `cluster` CTAs (0: none).  The kernels launched so read nothing in front of dependency_wait(), weights and pages
+// included: a caller's kernel may write those too, and one that lets its own dependents start early is not even
+// complete when such a launch starts.  Behind it they use coherent loads that the compiler keeps in place (__ldcg,
+// ld_stream, ld_u8, ld_f32).  A non-coherent load (__ldg, or a plain one through a const __restrict__ pointer)
+// could return what the operand held before.
 template <class Kernel, class... Args>
 inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};

@@ -5,9 +5,9 @@
 //
 // A matvec of 25 MB: the weight stream bounds it (3.8 us at 6.55 TB/s), so every warp owns one row pair (one row
 // of w2 at a time), splits K over its lanes in 16-byte pieces and has all of a row's loads in flight at once
-// (115 KB per SM); the weights do not depend on earlier kernels, so they are asked for before the wait for the
-// token.  The vector lies in shared memory as [quarter of a piece][piece]: the lanes of a warp, which hold
-// consecutive pieces, read consecutive 16 bytes.  Sums as in the FP8 register kernels: F32 inside a piece, double
+// (115 KB per SM); the first ones are brought to the L2 before the wait for the token (the executor's step of 4096 x
+// 2048: 40.1 us, without that 42.2).  The vector lies in shared memory as [quarter of a piece][piece]: the lanes of a
+// warp, which hold consecutive pieces, read consecutive 16 bytes.  Sums as in the FP8 register kernels: F32 inside a piece, double
 // across pieces and lanes, one rounding.  Measured at 4096 x 2048 beside the register kernels that ran all
 // seven experts (35 + 25 us): these two launches and the layer kernel's six experts take 28 us together.
 #include "s14_device.cuh"
@@ -59,7 +59,12 @@ __device__ __forceinline__ void dot_piece(const uint4 *const (&q)[N], const floa
 template <uint32_t P>
 __device__ __forceinline__ void load_row(uint4 (&q)[P], const uint8_t *row, uint32_t lane) {
 #pragma unroll
-    for (uint32_t j = 0; j < P; ++j) q[j] = ldg_stream(reinterpret_cast<const uint4 *>(row) + j * 32u + lane);
+    for (uint32_t j = 0; j < P; ++j) q[j] = ld_stream(reinterpret_cast<const uint4 *>(row) + j * 32u + lane);
+}
+template <uint32_t P>
+__device__ __forceinline__ void hint_row(const uint8_t *row, uint32_t lane) {
+#pragma unroll
+    for (uint32_t j = 0; j < P; ++j) l2_hint(row + (j * 32u + lane) * 16u);
 }
 // scales: a row's codes, one per 128 elements (a piece's: piece / 8)
 template <uint32_t P>
@@ -71,7 +76,7 @@ __device__ __forceinline__ float dot_row(const uint4 (&qa)[P], const uint8_t *sc
         const uint4 *const q[1] = {&qa[j]};
         float dot[1];
         dot_piece<1>(q, sx, p, P * 32u, dot);
-        acc += (double)dot[0] * ue8m0_to_f64(__ldg(scales + (p >> 3)));
+        acc += (double)dot[0] * ue8m0_to_f64(ld_u8(scales + (p >> 3)));
     }
     return (float)warp_sum(acc);
 }
@@ -86,8 +91,8 @@ __device__ __forceinline__ void dot_rows(const uint4 (&qa)[P], const uint4 (&qb)
         const uint4 *const q[2] = {&qa[j], &qb[j]};
         float dot[2];
         dot_piece<2>(q, sx, p, P * 32u, dot);
-        a += (double)dot[0] * ue8m0_to_f64(__ldg(sa + (p >> 3)));
-        b += (double)dot[1] * ue8m0_to_f64(__ldg(sb + (p >> 3)));
+        a += (double)dot[0] * ue8m0_to_f64(ld_u8(sa + (p >> 3)));
+        b += (double)dot[1] * ue8m0_to_f64(ld_u8(sb + (p >> 3)));
     }
     va = (float)warp_sum(a);
     vb = (float)warp_sum(b);
@@ -100,16 +105,19 @@ k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16
                 const uint8_t *__restrict__ page, float *__restrict__ h, uint32_t inter) {
     constexpr uint32_t hidden = P * 512u;
     __shared__ __align__(16) float sx[hidden];
-    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, step = gridDim.x * kF8Warps;
     const PageView pv = page_view(page, S14_PAGE_FP8, hidden, inter);
     uint32_t row = warp * gridDim.x + blockIdx.x;  // the CTAs' numbers of rows differ by one at most
     uint4 q1[P], q3[P];
     if (row < inter) {
+        hint_row<P>(pv.w1 + (size_t)row * hidden, lane);
+        hint_row<P>(pv.w3 + (size_t)row * hidden, lane);
+    }
+    dependency_wait();
+    if (row < inter) {
         load_row<P>(q1, pv.w1 + (size_t)row * hidden, lane);
         load_row<P>(q3, pv.w3 + (size_t)row * hidden, lane);
     }
-    cudaGridDependencySynchronize();
     if (x_bf16) {
         stage_vector_bf16(sx, x_bf16, hidden);
         if (blockIdx.x == gridDim.x - 1u)
@@ -138,14 +146,15 @@ __global__ void __launch_bounds__(kF8Threads, 1)
 k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, float *__restrict__ d, uint32_t hidden) {
     constexpr uint32_t inter = P * 512u;
     __shared__ __align__(16) float sx[inter];
-    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, step = gridDim.x * kF8Warps;
     const PageView pv = page_view(page, S14_PAGE_FP8, hidden, inter);
     uint32_t row = warp * gridDim.x + blockIdx.x;
     uint4 qa[P], qb[P];  // this row and the warp's next one
+    if (row < hidden) hint_row<P>(pv.w2 + (size_t)row * inter, lane);
+    if (row + step < hidden) hint_row<P>(pv.w2 + (size_t)(row + step) * inter, lane);
+    dependency_wait();
     if (row < hidden) load_row<P>(qa, pv.w2 + (size_t)row * inter, lane);
     if (row + step < hidden) load_row<P>(qb, pv.w2 + (size_t)(row + step) * inter, lane);
-    cudaGridDependencySynchronize();
     stage_vector(sx, h, inter);
     __syncthreads();
 #pragma unroll 1

@@ -83,6 +83,14 @@ __device__ __forceinline__ void stream_st8(void *p, size_t i, const float (&v)[8
 __device__ __forceinline__ float sigmoid_f32(float v) { return (float)(1.0 / (1.0 + exp(-(double)v))); }
 __device__ __forceinline__ float rsqrt_of(float mean_sq, float eps) { return (float)(1.0 / sqrt((double)__fadd_rn(mean_sq, eps))); }
 
+// scale [3] (kHead: [1]) and base into shared memory by threads 0 .. 31, early in a kernel: read where they are used, they
+// would stand in the serial chain of the coefficients.
+template <bool kHead>
+__device__ __forceinline__ void load_coefficients(float *s_coef, const float *scale, const float *base, uint32_t tid) {
+    if (tid < (kHead ? 1u : 3u)) s_coef[tid] = __ldcg(scale + tid);
+    if (tid < (kHead ? kHc : kMixMax)) s_coef[3u + tid] = __ldcg(base + tid);
+}
+
 // hc.py:19-84 by one warp: 24 logits -> pre [4], post [4], comb [4][4], F32 in the reference's order.  Lane
 // l < 16 owns comb[l / 4][l % 4]; a row's or column's four values are fetched with shuffles and added in
 // index order, as the Python sums do; lanes 0-3 also make pre and post.  All 32 lanes call it.
@@ -132,7 +140,7 @@ __device__ __forceinline__ void reduce_streams8(const void *x, size_t x0, uint32
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
 // only) of few tokens: one cluster of sixteen CTAs per token.  The call is all latency: 1.5 MB of fn per token,
 // then a serial chain of 20 Sinkhorn rounds.  Every CTA takes a sixteenth of the flattened streams against all
-// rows of fn (98 KB, asked for before the wait for the state, all loads in flight together), the partial sums
+// rows of fn (98 KB, all loads in flight together), the partial sums
 // cross in shared memory, every CTA makes the coefficients itself and reduces its sixteenth of the hidden
 // vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
 constexpr uint32_t kPreCluster = 16, kPreThreads = 512;
@@ -144,8 +152,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     constexpr uint32_t n_mix = kHead ? kHc : kMixMax, kRows = n_mix / 2u;   // rows per half of the CTA
     __shared__ double s_warp[kPreThreads / 32][kRows + 1];
     __shared__ double s_part[kPreCluster][n_mix + 1];                      // [n_mix]: the sum of squares
-    __shared__ float s_mix[n_mix], s_pre[kHc];
-    cudaTriggerProgrammaticLaunchCompletion();
+    __shared__ float s_mix[n_mix], s_pre[kHc], s_coef[3 + n_mix];            // [3 + n_mix]: scale, base
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), t = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t n = kHc * hidden, share = n / kPreCluster, k0 = rank * share;   // a multiple of 64
@@ -156,11 +163,12 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     float4 f[kRows];
     auto fetch = [&](uint32_t i) {
 #pragma unroll
-        for (uint32_t m = 0; m < kRows; ++m) f[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)(half * kRows + m) * n + k0 + i));
+        for (uint32_t m = 0; m < kRows; ++m) f[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)(half * kRows + m) * n + k0 + i));
     };
-    if (c * 4u < share) fetch(c * 4u);
     cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
-    cudaGridDependencySynchronize();
+    dependency_wait();
+    if (c * 4u < share) fetch(c * 4u);
+    load_coefficients<kHead>(s_coef, scale, base, tid);
     for (uint32_t i = c * 4u; i < share; i += 1024u) {
         float v[4];
         if constexpr (kBf16) {
@@ -205,7 +213,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
         __syncwarp();
         // pre first: the other warps reduce the streams while this one of the first CTA goes on to post and comb
         if (lane < kHc) {
-            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], scale[0]), base[lane])), hc_eps);
+            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
             s_pre[lane] = pre;
             if (pre_out && rank == 0u) pre_out[(size_t)t * kHc + lane] = pre;
         }
@@ -214,7 +222,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     const uint32_t part = hidden / kPreCluster;   // a multiple of 16
     if (!kHead && rank == 0u && warp == 0u) {
         float pre, post, comb;
-        split_sinkhorn_warp(s_mix, scale, base, iters, hc_eps, lane, pre, post, comb);
+        split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
         if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
         if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
     }
@@ -238,8 +246,7 @@ template <bool kBf16>
 __global__ void __launch_bounds__(256)
 k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, uint32_t n_tokens, double *__restrict__ partial) {
     __shared__ double s_acc[8][kDotTokens][kMixMax + 1];
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
     const uint32_t t0 = blockIdx.x * kDotTokens, len = n / (gridDim.y * 8u);   // a multiple of 16
     const uint32_t k0 = (blockIdx.y * 8u + warp) * len + q * 4u;
@@ -262,7 +269,7 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
         load4(tb, k, vb);
         float4 w[3];
 #pragma unroll
-        for (uint32_t m = 0; m < 3; ++m) w[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)(m * 8u + g) * n + k));
+        for (uint32_t m = 0; m < 3; ++m) w[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)(m * 8u + g) * n + k));
 #pragma unroll
         for (uint32_t s = 0; s < 4; ++s) {
             const double a = va[s], b = vb[s];
@@ -306,23 +313,25 @@ __global__ void __launch_bounds__(256)
 k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint32_t slices, const float *__restrict__ scale,
             const float *__restrict__ base, uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced,
             float *__restrict__ post_out, float *__restrict__ comb_out, uint32_t vec) {
-    __shared__ float s_pre[kHc], s_mix[kMixMax];
+    __shared__ float s_pre[kHc], s_mix[kMixMax], s_coef[3 + kMixMax];
+    // (k_hc_dots in front of this launch has waited: the launch behind may be set up at once)
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (warp == 0u) {
+        load_coefficients<false>(s_coef, scale, base, lane);
         double s = 0.0;
         if (lane <= kMixMax)
             for (uint32_t p = 0; p < slices; ++p) s += __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMixMax + 1u) + lane);
         const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMixMax) / (double)(kHc * hidden)), norm_eps);
         if (lane < kMixMax) s_mix[lane] = __fmul_rn((float)s, rs);
         __syncwarp();
-        if (lane < kHc) s_pre[lane] = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], scale[0]), base[lane])), hc_eps);
+        if (lane < kHc) s_pre[lane] = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
     }
     __syncthreads();
     if (warp == 0u) {  // the other warps reduce the streams meanwhile
         float pre, post, comb;
-        split_sinkhorn_warp(s_mix, scale, base, iters, hc_eps, lane, pre, post, comb);
+        split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
         if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
         if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
         return;
@@ -341,8 +350,7 @@ __global__ void __launch_bounds__(128)
 k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, const float *__restrict__ post,
           const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged, uint32_t vec) {
     const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * 8u, t = blockIdx.y;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (d >= hidden) return;
     float r[kHc][8], b[8], c[kHc * kHc], p[kHc];
 #pragma unroll
@@ -375,8 +383,7 @@ k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hid
            uint32_t vec) {
     __shared__ double red[8];
     const uint32_t t = blockIdx.x;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     float v[4][8];
     double ss = 0.0;
 #pragma unroll
@@ -448,8 +455,7 @@ __global__ void __launch_bounds__(256)
 k_branch_post(const float *__restrict__ y, uint16_t *__restrict__ branch_out, const void *__restrict__ residual,
               const float *__restrict__ post, const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
     const uint32_t d = blockIdx.x * 256u + threadIdx.x;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (d >= hidden) return;
     float r[kHc], c[kHc * kHc], p[kHc];
 #pragma unroll

@@ -69,7 +69,7 @@ __device__ __noinline__ float head_row_dot(const float *x, const uint16_t *w, ui
     double acc = 0.0;
 #pragma unroll 1
     for (uint32_t p = threadIdx.x & 31u; p < (hidden >> 3); p += 32u) {
-        const uint4 q = ldg_stream(reinterpret_cast<const uint4 *>(w) + p);
+        const uint4 q = ld_stream(reinterpret_cast<const uint4 *>(w) + p);
         const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
         float2 part = make_float2(0.f, 0.f);
 #pragma unroll
@@ -87,7 +87,6 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
            uint32_t out_stride, uint32_t n_tokens, uint32_t phases) {
     extern __shared__ __align__(16) uint8_t s_parts[];      // [3][n_tokens][pitch], then the tiles' sums [tile][4][32]
     __shared__ double s_half[kHeadPairs][2][4][32];          // the second warp's half of K, by tile parity
-    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, pair = warp >> 1, half = warp & 1u;
     const uint32_t g = lane >> 2, q = lane & 3u;
     const uint32_t span = hidden / phases;                   // of K per phase
@@ -99,7 +98,6 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
     const uint32_t n_mine = n_tiles > blockIdx.x ? (n_tiles - blockIdx.x + grid - 1u) / grid : 0u;
     const uint32_t batch = phases > 1u ? kHeadTiles : n_mine;
 
-    // the weights do not depend on the kernel before this one: their first loads are in flight while x is split
     const uint16_t *p0, *p1;
     auto rows_of = [&](uint32_t i, uint32_t phase) {
         const uint32_t t = blockIdx.x + i * grid, r0 = min(t * 16u + g, n_rows - 1u), r1 = min(t * 16u + g + 8u, n_rows - 1u);
@@ -109,15 +107,15 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
     };
     uint4 a0[kHeadDepth], a1[kHeadDepth];
     auto fetch = [&](uint32_t i, uint32_t k) {
-        a0[i] = ldg_stream(reinterpret_cast<const uint4 *>(p0 + (k + i) * 32u));
-        a1[i] = ldg_stream(reinterpret_cast<const uint4 *>(p1 + (k + i) * 32u));
+        a0[i] = ld_stream(reinterpret_cast<const uint4 *>(p0 + (k + i) * 32u));
+        a1[i] = ld_stream(reinterpret_cast<const uint4 *>(p1 + (k + i) * 32u));
     };
-    if (pair < n_mine) {
+    dependency_wait();
+    if (pair < n_mine) {  // in flight while x is split
         rows_of(pair, 0u);
 #pragma unroll
         for (uint32_t i = 0; i < kHeadDepth; ++i) fetch(i, 0u);
     }
-    cudaGridDependencySynchronize();
     const uint8_t *const sb = s_parts + (g < n_tokens ? g : 0u) * pitch + half * span + q * 16u;
     const bool has_b = g < n_tokens;
     uint32_t parity = 0;
@@ -274,10 +272,9 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, uint32_t i) {
 __global__ void __launch_bounds__(kArgmaxThreads)
 k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__restrict__ result) {
     __shared__ unsigned long long s_warp[kArgmaxThreads / 32], s_cta[kArgmaxCluster];
-    cudaTriggerProgrammaticLaunchCompletion();
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
-    cudaGridDependencySynchronize();
+    dependency_wait();
     const uint32_t n = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
     unsigned long long best = 0ull;
     auto take = [&](float v, uint32_t i) {
@@ -336,12 +333,12 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
     __shared__ double s_sums[kPrepCluster][5];   // four dot products and the sum of squares of every CTA's share
     __shared__ double s_ss[kPrepCluster];
     __shared__ float s_pre[4];
-    cudaTriggerProgrammaticLaunchCompletion();
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
-    cudaGridDependencySynchronize();
+    dependency_wait();
     const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t n = 4u * hidden, share = n / kPrepCluster;   // a multiple of 128
+    const float scale0 = __ldcg(scale), base_h = tid < 4u ? __ldcg(base + tid) : 0.0f;  // (read here: a serial chain uses them)
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (uint32_t i = tid * 4u; i < share; i += kPrepThreads * 4u) {
         const uint32_t k = rank * share + i;
@@ -350,7 +347,7 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
                              __uint_as_float(b.y & 0xffff0000u)};
         float4 f[4];
 #pragma unroll
-        for (uint32_t m = 0; m < 4; ++m) f[m] = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)m * n + k));
+        for (uint32_t m = 0; m < 4; ++m) f[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)m * n + k));
 #pragma unroll
         for (uint32_t m = 0; m < 4; ++m) {
             v[m] += (double)xs[0] * (double)f[m].x;
@@ -381,7 +378,7 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
         for (uint32_t r = 0; r < kPrepCluster; ++r) dot += s_sums[r][tid], ss += s_sums[r][4];
         const float rs = (float)(1.0 / sqrt((double)__fadd_rn((float)(ss / (double)n), norm_eps)));
         const float mix = __fmul_rn((float)dot, rs);
-        s_pre[tid] = __fadd_rn((float)(1.0 / (1.0 + exp(-(double)__fadd_rn(__fmul_rn(mix, scale[0]), base[tid])))), hc_eps);
+        s_pre[tid] = __fadd_rn((float)(1.0 / (1.0 + exp(-(double)__fadd_rn(__fmul_rn(mix, scale0), base_h)))), hc_eps);
     }
     __syncthreads();
     // this CTA's eighth of the hidden vector, at most four elements a thread (hidden <= 8192)
@@ -419,7 +416,7 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) {
         const uint32_t e = tid + i * kPrepThreads, d = rank * part + e;
-        if (e < part) x_out[d] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__ldg(norm_weight + d), __fmul_rn(red[i], rs))));
+        if (e < part) x_out[d] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(__ldcg(norm_weight + d), __fmul_rn(red[i], rs))));
     }
 }
 

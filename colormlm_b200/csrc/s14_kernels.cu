@@ -52,7 +52,7 @@ __device__ __forceinline__ float dot16_e4m3(const uint4 &q, const float *__restr
 // y[n] = sum_k x[k] * e2m1(w[n,k]) * 2^(s[n,k/32]-127).  A matrix of the checkpoint's sizes is 4 MB: launch, first
 // byte and the x reads bound the call, not the bandwidth.  A warp owns NR rows at a time and splits K over its
 // lanes in 16-byte pieces (one scale block each), the pieces of its rows (four each per step) in flight together and
-// the first ones asked for before the wait for the kernel in front (weights do not depend on it).  x lies in
+// the first ones brought to the L2 before the wait for the kernel in front (l2_hint).  x lies in
 // shared memory as [eighth of a piece][piece], so that a warp's lanes read consecutive 16 bytes; reading it
 // through the L1 with a 128-byte stride between lanes, one piece in flight, took 10.6 us for 2048 x 4096
 // (this kernel: 3.3).  Two rows per warp halve the x reads, which cost more than the weights (128 bytes for 16),
@@ -63,7 +63,6 @@ __global__ void __launch_bounds__(kMvThreads, 1)
 k_mxfp4_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w, const uint8_t *__restrict__ s,
                         float *__restrict__ y, uint32_t n_rows, uint32_t k) {
     extern __shared__ __align__(16) float sx[];
-    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, groups = k >> 5;
     const uint32_t n_warps = gridDim.x * (kMvThreads / 32u);
     const uint32_t batches = (groups + 32u * kMvBatch - 1u) / (32u * kMvBatch);
@@ -78,14 +77,24 @@ k_mxfp4_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__
             for (uint32_t j = 0; j < kMvBatch; ++j) {
                 const uint32_t p = (batch * kMvBatch + j) * 32u + lane;
                 const bool there = row < n_rows && p < groups;
-                q[r][j] = there ? ldg_stream(reinterpret_cast<const uint4 *>(w + (size_t)row * (k >> 1)) + p) : make_uint4(0u, 0u, 0u, 0u);
-                sc[r][j] = there ? __ldg(s + (size_t)row * groups + p) : 0u;
+                q[r][j] = there ? ld_stream(reinterpret_cast<const uint4 *>(w + (size_t)row * (k >> 1)) + p) : make_uint4(0u, 0u, 0u, 0u);
+                sc[r][j] = there ? ld_u8(s + (size_t)row * groups + p) : 0u;
             }
         }
     };
     uint32_t n = warp * gridDim.x + blockIdx.x;  // the CTAs' numbers of rows differ by one at most
+#pragma unroll
+    for (uint32_t r = 0; r < NR; ++r)
+#pragma unroll
+        for (uint32_t j = 0; j < kMvBatch; ++j) {
+            const uint32_t row = n + r * n_warps, p = j * 32u + lane;
+            if (row < n_rows && p < groups) {
+                l2_hint(w + (size_t)row * (k >> 1) + p * 16u);
+                l2_hint(s + (size_t)row * groups + p);
+            }
+        }
+    dependency_wait();
     if (n < n_rows) fetch(n, 0u);
-    cudaGridDependencySynchronize();
     for (uint32_t i = threadIdx.x; i < (k >> 2); i += kMvThreads)
         reinterpret_cast<float4 *>(sx)[(i & 7u) * groups + (i >> 3)] = __ldcg(reinterpret_cast<const float4 *>(x) + i);
     __syncthreads();
@@ -208,8 +217,8 @@ __device__ __forceinline__ float e4m3_to_f32(uint32_t code) {
 
 template <bool F32_SCALE>
 __device__ __forceinline__ double fp8_block_scale_f64(const void *scale, size_t idx) {
-    if (F32_SCALE) return (double)__ldg(reinterpret_cast<const float *>(scale) + idx);
-    return ue8m0_to_f64(__ldg(reinterpret_cast<const uint8_t *>(scale) + idx));
+    if (F32_SCALE) return (double)ld_f32(reinterpret_cast<const float *>(scale) + idx);
+    return ue8m0_to_f64(ld_u8(reinterpret_cast<const uint8_t *>(scale) + idx));
 }
 
 template <bool F32_SCALE>
@@ -281,9 +290,9 @@ k_fp8_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w
 // warps takes eight rows, two warps per row (the halves of K), the tokens' activations are staged
 // once per CTA in shared memory, a 16-byte piece of weights is decoded once for all tokens, and the
 // two halves of a row are added through shared memory.  k a multiple of 32, 16-byte aligned operands.
-// A dependent launch: the first weights are asked for before the wait for the kernel in front, the next ones while a
-// piece is worked on (us a call in a queue of calls, before and after: 1024 x 4096 x 8 tokens 12.3 -> 9.8, 4700 x 640 x 8
-// 14.4 -> 11.4, 700 x 8192 x 5 14.4 -> 11.5; one token of 1024 x 4096 7.8 -> 3.1, half of it host time).
+// A dependent launch: the first weights are brought to the L2 before the wait for the kernel in front, the next ones are
+// asked for while a piece is worked on (us a call in a queue of calls, before and after: 1024 x 4096 x 8 tokens 12.3 ->
+// 9.8, 4700 x 640 x 8 14.4 -> 11.4, 700 x 8192 x 5 14.4 -> 11.5; one token of 1024 x 4096 7.8 -> 3.1, half of it host time).
 constexpr uint32_t kFp8BlockRows = 8, kFp8BlockThreads = 512;
 template <int NT, bool F32_SCALE>
 __global__ void __launch_bounds__(kFp8BlockThreads)
@@ -299,9 +308,9 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
     const uint32_t pieces = k >> 4, per = pieces >> 1;
     const uint4 *wrow = reinterpret_cast<const uint4 *>(w + (size_t)n * k);
     uint4 ahead = make_uint4(0u, 0u, 0u, 0u);
-    cudaTriggerProgrammaticLaunchCompletion();
-    if (n < n_rows && lane < per) ahead = ldg_stream(wrow + half * per + lane);
-    cudaGridDependencySynchronize();
+    if (n < n_rows && lane < per) l2_hint(wrow + half * per + lane);
+    dependency_wait();
+    if (n < n_rows && lane < per) ahead = ld_stream(wrow + half * per + lane);
     for (uint32_t i = threadIdx.x; i < (NT * k) >> 2; i += kFp8BlockThreads) {
         const uint32_t t = i / (k >> 2), j = i % (k >> 2);
         reinterpret_cast<float4 *>(sx)[(size_t)t * (k >> 2) + (j & 3u) * pieces + (j >> 2)] =
@@ -316,7 +325,7 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
         const size_t srow = (size_t)(n >> 7) * k_groups;
         for (uint32_t p = half * per + lane; p < (half + 1u) * per; p += 32u) {
             const uint4 q = ahead;
-            if (p + 32u < (half + 1u) * per) ahead = ldg_stream(wrow + p + 32u);
+            if (p + 32u < (half + 1u) * per) ahead = ld_stream(wrow + p + 32u);
             const double sc = fp8_block_scale_f64<F32_SCALE>(scale, srow + (p >> 3));
             const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
             float2 wf[8];
@@ -384,8 +393,7 @@ k_fp8_matvec_reference(const float *__restrict__ x, const uint8_t *__restrict__ 
 __global__ void k_swiglu_limit(const float *__restrict__ gate, const float *__restrict__ up,
                                float *__restrict__ y, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (i < n) y[i] = swiglu_limit_f32(__ldcg(gate + i), __ldcg(up + i));
 }
 
@@ -393,8 +401,7 @@ __global__ void k_swiglu_limit(const float *__restrict__ gate, const float *__re
 __global__ void k_route_mix(const float *__restrict__ expert, float *__restrict__ routed, uint32_t n,
                             float weight) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (i < n) routed[i] = __fmul_rn(weight, __ldcg(expert + i));
 }
 
@@ -402,8 +409,7 @@ __global__ void k_route_mix(const float *__restrict__ expert, float *__restrict_
 __global__ void k_moe_accumulate(const float *__restrict__ expert, float *__restrict__ acc,
                                  uint32_t n, float weight) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (i < n) acc[i] = __fadd_rn(__ldcg(acc + i), __fmul_rn(weight, __ldcg(expert + i)));
 }
 
@@ -1331,15 +1337,14 @@ k_router_scores(const float *__restrict__ x, const uint16_t *__restrict__ wr, co
     uint4 q[kNt];
     auto load = [&](uint32_t k) {
 #pragma unroll
-        for (uint32_t n = 0; n < kNt; ++n) q[n] = __ldg(reinterpret_cast<const uint4 *>(wp[n] + k));
+        for (uint32_t n = 0; n < kNt; ++n) q[n] = __ldcg(reinterpret_cast<const uint4 *>(wp[n] + k));
 #pragma unroll
         for (uint32_t m = 0; m < kMt; ++m) {
             xa[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k));
             xb[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k) + 1);
         }
     };
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     load(0);
 #pragma unroll 1
     for (uint32_t k = 0; k < part; k += 32u) {
@@ -1386,7 +1391,7 @@ k_router_scores(const float *__restrict__ x, const uint16_t *__restrict__ wr, co
         if (t < n_tokens && e < n_experts) {
             const float sc = router_score_f32(sum, score_fn);
             scores[(size_t)t * n_experts + e] = sc;
-            select[(size_t)t * n_experts + e] = __fadd_rn(sc, bias ? bias[e] : 0.0f);
+            select[(size_t)t * n_experts + e] = __fadd_rn(sc, bias ? __ldcg(bias + e) : 0.0f);
         }
     }
 }
@@ -1396,9 +1401,8 @@ __global__ void __launch_bounds__(256)
 k_router_select_batch(const float *__restrict__ scores, const float *__restrict__ select, uint32_t n_experts, uint32_t n_tokens,
                       uint32_t top_k, float route_scale, int32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
     const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    cudaTriggerProgrammaticLaunchCompletion();
+    dependency_wait();
     if (t >= n_tokens) return;
-    cudaGridDependencySynchronize();
     router_select(scores + (size_t)t * n_experts, select + (size_t)t * n_experts, n_experts, top_k, route_scale,
                   ids_out + (size_t)t * top_k, weights_out + (size_t)t * top_k, nullptr, nullptr, nullptr, 0, threadIdx.x & 31u, 0,
                   1, 0);

@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(512)
 k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps) {
     constexpr uint32_t kRows = kQuant ? 8u : 16u;
     const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
     const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
     float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
@@ -183,13 +182,12 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     __shared__ unsigned long long gpage[kG];
     __shared__ uint32_t bad;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, G = n_experts + 1u, n = T * top_k;
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (tid < kG) {
         cnt[tid] = 0u;
         fill[tid] = 0u;
         gpage[tid] = tid == 0u ? (unsigned long long)shared_page
-                               : ((page_table && tid < G) ? (unsigned long long)page_table[tid - 1u] : 0ull);
+                               : ((page_table && tid < G) ? __ldcg(reinterpret_cast<const unsigned long long *>(page_table + tid - 1u)) : 0ull);
     }
     if (tid == 0) bad = 0u;
     __syncthreads();
@@ -242,7 +240,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
         if (e < 0 || (uint32_t)e % ep_world != ep_rank) continue;
         const uint32_t g = 1u + (uint32_t)e, t = i / top_k, m = i - t * top_k;
         const uint32_t k = atomicAdd(&fill[g], 1u);
-        if (k == 0u && !page_table) gpage[g] = (unsigned long long)pages[i];
+        if (k == 0u && !page_table) gpage[g] = __ldcg(reinterpret_cast<const unsigned long long *>(pages + i));
         BlockChunk *ch = chunks + chunk0[g] + k / nt_cap;
         ch->tok[k % nt_cap] = t;
         ch->pair[k % nt_cap] = t * kPairsPerToken + m;
@@ -347,8 +345,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
     fence_after();
     const uint32_t tmem = tmem_slot;
     // barriers and tensor memory are ready; from here on the launch reads what the ones before it leave
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     const uint32_t n_items = __ldcg(a.n_items);
     // The CTA's items are q = cta, cta + grid, ...  The chunks of one expert follow one another and so
     // do their items, a row tile's chunks side by side (so that CTAs that run at the same time share
@@ -829,8 +826,7 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
             const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_world, uint32_t ep_call,
             uint32_t wait_limit, uint32_t *status, uint32_t official, uint32_t vec) {
     const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * 4u, t = blockIdx.y;   // hidden is a multiple of four
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    dependency_wait();
     if (flags) {
         // expert parallel, exchange inside the kernels: every rank's rows of this call are in this rank's buffer
         // when its flag carries the call's number (bounded wait: about a microsecond per poll)

@@ -85,6 +85,13 @@ typedef struct s14_moe_pages s14_moe_pages;
 
 S14_API const char *s14_last_error(void);
 
+/* Order on a stream: a call reads its operands, weights and pages included, when everything in front of it in the stream
+ * is complete, and what is behind it in the stream sees its results.  One exception: the one-token layer, stack and routed
+ * layer calls on MXFP4 pages ask for pages, router weights, biases and page tables while the kernel directly in front
+ * of them ends.  That matters only to a kernel of the caller that writes one of those AND lets its own programmatic
+ * dependents start before it has written it (cudaTriggerProgrammaticLaunchCompletion): put any other launch
+ * or an event wait between it and such a call. */
+
 /* ---- context: replaces VulkanContext::init + S14NumericPipelines::new/destroy
  *      (ssd_inference/src/device.rs:26-76, s14_vulkan.rs:195-205, 417-424) ------ */
 S14_API int32_t s14_ctx_create(int32_t device, s14_ctx **out);
