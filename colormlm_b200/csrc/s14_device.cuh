@@ -156,6 +156,13 @@ __device__ __forceinline__ void dependency_wait() {
 // to this kernel.
 __device__ __forceinline__ void l2_hint(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// The result of a launch.  A refused launch also stays behind as the thread's last error, where the next check of the
+// library, or of whoever shares the runtime with it, would find it and blame another call.
+inline cudaError_t launch_status(cudaError_t e) {
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
 // A launch as a programmatic dependent of what precedes it in the stream, optionally in clusters of
 // `cluster` CTAs (0: none).  The kernels launched so read nothing in front of dependency_wait(), weights and pages
 // included: a caller's kernel may write those too, and one that lets its own dependents start early is not even
@@ -178,7 +185,7 @@ inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem,
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cluster ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return launch_status(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 }  // namespace s14

@@ -988,35 +988,36 @@ static bool fp8_block_smem_ok(size_t bytes) {
     return configured[dev] == 1 && bytes <= 160u * 1024u;
 }
 
+// Whether the block kernel takes the call; *err: its launch's result.
 template <int NT, bool F32S>
 static bool try_fp8_block(cudaStream_t st, int sm_count, const float *x, const uint8_t *w, const void *s, float *y,
-                          uint32_t n, uint32_t k) {
+                          uint32_t n, uint32_t k, cudaError_t *err) {
     // few rows (a warp per row would leave most SMs with a handful of warps), k in whole scale
     // blocks, 16-byte aligned operands, the tokens' activations fit shared memory
     const size_t bytes = (size_t)NT * k * sizeof(float);
     if (n > (uint32_t)sm_count * 32u || (k & 31u) || ((uintptr_t)w & 15u) || ((uintptr_t)x & 15u)) return false;
     if (!fp8_block_smem_ok<NT, F32S>(bytes)) return false;
-    // (a launch that is refused leaves its error to the caller's check, as the plain launches do)
-    (void)launch_pdl(k_fp8_matvec_block<NT, F32S>, dim3((n + kFp8BlockRows - 1) / kFp8BlockRows), dim3(kFp8BlockThreads), bytes, st, 0u, x,
-                     w, s, y, n, k);
+    *err = launch_pdl(k_fp8_matvec_block<NT, F32S>, dim3((n + kFp8BlockRows - 1) / kFp8BlockRows), dim3(kFp8BlockThreads), bytes, st, 0u,
+                      x, w, s, y, n, k);
     return true;
 }
 
 template <bool F32S>
-static void launch_fp8_pairwise_nt(cudaStream_t st, int sm_count, uint32_t blocks, uint32_t nt, const float *x,
-                                   const uint8_t *w, const void *s, float *y, uint32_t n, uint32_t k) {
+static cudaError_t launch_fp8_pairwise_nt(cudaStream_t st, int sm_count, uint32_t blocks, uint32_t nt, const float *x,
+                                          const uint8_t *w, const void *s, float *y, uint32_t n, uint32_t k) {
     bool done = false;
+    cudaError_t err = cudaSuccess;
     switch (nt) {
-    case 1: done = try_fp8_block<1, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 2: done = try_fp8_block<2, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 3: done = try_fp8_block<3, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 4: done = try_fp8_block<4, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 5: done = try_fp8_block<5, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 6: done = try_fp8_block<6, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    case 7: done = try_fp8_block<7, F32S>(st, sm_count, x, w, s, y, n, k); break;
-    default: done = try_fp8_block<8, F32S>(st, sm_count, x, w, s, y, n, k); break;
+    case 1: done = try_fp8_block<1, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 2: done = try_fp8_block<2, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 3: done = try_fp8_block<3, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 4: done = try_fp8_block<4, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 5: done = try_fp8_block<5, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 6: done = try_fp8_block<6, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    case 7: done = try_fp8_block<7, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
+    default: done = try_fp8_block<8, F32S>(st, sm_count, x, w, s, y, n, k, &err); break;
     }
-    if (done) return;
+    if (done) return err;
     switch (nt) {
     case 1: k_fp8_matvec_pairwise<1, F32S><<<blocks, 256, 0, st>>>(x, w, s, y, n, k); break;
     case 2: k_fp8_matvec_pairwise<2, F32S><<<blocks, 256, 0, st>>>(x, w, s, y, n, k); break;
@@ -1027,6 +1028,7 @@ static void launch_fp8_pairwise_nt(cudaStream_t st, int sm_count, uint32_t block
     case 7: k_fp8_matvec_pairwise<7, F32S><<<blocks, 256, 0, st>>>(x, w, s, y, n, k); break;
     default: k_fp8_matvec_pairwise<8, F32S><<<blocks, 256, 0, st>>>(x, w, s, y, n, k); break;
     }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_fp8_matvec(cudaStream_t st, uint32_t mode, int sm_count, uint32_t scale_format,
@@ -1041,9 +1043,8 @@ cudaError_t launch_fp8_matvec(cudaStream_t st, uint32_t mode, int sm_count, uint
     } else {
         const uint32_t blocks = min(ceil_div(n, 8), (uint32_t)sm_count * 8u);
         if (scale_format == S14_SCALE_F32)
-            launch_fp8_pairwise_nt<true>(st, sm_count, blocks, n_tokens, x, w, s, y, n, k);
-        else
-            launch_fp8_pairwise_nt<false>(st, sm_count, blocks, n_tokens, x, w, s, y, n, k);
+            return launch_fp8_pairwise_nt<true>(st, sm_count, blocks, n_tokens, x, w, s, y, n, k);
+        return launch_fp8_pairwise_nt<false>(st, sm_count, blocks, n_tokens, x, w, s, y, n, k);
     }
     return cudaGetLastError();
 }

@@ -1282,7 +1282,7 @@ cudaError_t launch_layer(Kernel kernel, dim3 grid, dim3 block, size_t smem, cuda
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return launch_status(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 constexpr size_t kMaxSmem = 227u * 1024u;  // per CTA, static + dynamic
