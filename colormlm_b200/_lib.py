@@ -304,6 +304,7 @@ def pycall():
     except ImportError as e:
         raise ImportError(f"colormlm_b200/_s14call.so cannot be loaded ({e}): build it with `python -m colormlm_b200.build`. "
                           "There is no fallback implementation.") from e
+    _s14call.set_records(Mxfp4Dispatch, Fp8Dispatch, SwigluLimitDispatch, RouteMixDispatch, MoeAccumulateDispatch)
     return _s14call
 
 

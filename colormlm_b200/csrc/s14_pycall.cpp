@@ -328,17 +328,36 @@ PyObject *stack_decode(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     S14_DONE
 }
 
+// The Python classes of the bound operators' records, in the order of set_records' arguments: two of them have the
+// same size, so a record's bytes do not tell what it is.
+enum RecordKind { kMxfp4, kFp8, kSwiglu, kRouteMix, kAccumulate, kRecordKinds };
+PyTypeObject *record_types[kRecordKinds];
+
+PyObject *set_records(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    if (nargs != kRecordKinds) return PyErr_Format(PyExc_TypeError, "set_records: %d classes are needed", (int)kRecordKinds);
+    for (int i = 0; i < kRecordKinds; ++i)
+        if (!PyType_Check(a[i])) return PyErr_Format(PyExc_TypeError, "set_records: a class is needed");
+    for (int i = 0; i < kRecordKinds; ++i) {
+        PyTypeObject *old = record_types[i];
+        record_types[i] = (PyTypeObject *)Py_NewRef(a[i]);
+        Py_XDECREF(old);
+    }
+    Py_RETURN_NONE;
+}
+
 // (ctx, stream, dispatch): a bound operator's record, read through the buffer protocol
-template <class Dispatch, int32_t (*kCall)(s14_ctx *, void *, const Dispatch *)>
+template <RecordKind kKind, class Dispatch, int32_t (*kCall)(s14_ctx *, void *, const Dispatch *)>
 PyObject *bound(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     S14_ARGS("a bound operator", 3)
+    if (!record_types[kKind] || !PyObject_TypeCheck(a[2], record_types[kKind]))
+        return PyErr_Format(PyExc_TypeError, "the dispatch record is a %s, not one of this operator", Py_TYPE(a[2])->tp_name);
     s14_ctx *c = ctx_of(a[0]);
     void *st = stream_of(a[1]);
     Py_buffer v;
     if (PyObject_GetBuffer(a[2], &v, PyBUF_SIMPLE) != 0) return nullptr;
     if (v.len != (Py_ssize_t)sizeof(Dispatch)) {
         PyBuffer_Release(&v);
-        return PyErr_Format(PyExc_TypeError, "the dispatch record is of another operator");
+        return PyErr_Format(PyExc_TypeError, "the dispatch record is not laid out as the library's");
     }
     PyObject *r = unlocked([&] { return kCall(c, st, (const Dispatch *)v.buf); });
     PyBuffer_Release(&v);
@@ -348,6 +367,7 @@ PyObject *bound(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
 
 #define S14_FAST(name, fn) {name, (PyCFunction)(void (*)(void))(fn), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
+    S14_FAST("set_records", set_records),
     S14_FAST("hc_pre", hc_pre),
     S14_FAST("hc_post", hc_post),
     S14_FAST("hc_head_reduce", hc_head_reduce),
@@ -359,11 +379,11 @@ PyMethodDef methods[] = {
     S14_FAST("routed_layer", routed_layer),
     S14_FAST("routed_block", routed_block),
     S14_FAST("stack_decode", stack_decode),
-    S14_FAST("mxfp4_matvec", (bound<s14_mxfp4_dispatch, s14_cmd_mxfp4_matvec>)),
-    S14_FAST("fp8_matvec", (bound<s14_fp8_dispatch, s14_cmd_fp8_matvec>)),
-    S14_FAST("swiglu_limit", (bound<s14_swiglu_limit_dispatch, s14_cmd_swiglu_limit>)),
-    S14_FAST("route_mix", (bound<s14_route_mix_dispatch, s14_cmd_route_mix>)),
-    S14_FAST("moe_accumulate", (bound<s14_moe_accumulate_dispatch, s14_cmd_moe_accumulate>)),
+    S14_FAST("mxfp4_matvec", (bound<kMxfp4, s14_mxfp4_dispatch, s14_cmd_mxfp4_matvec>)),
+    S14_FAST("fp8_matvec", (bound<kFp8, s14_fp8_dispatch, s14_cmd_fp8_matvec>)),
+    S14_FAST("swiglu_limit", (bound<kSwiglu, s14_swiglu_limit_dispatch, s14_cmd_swiglu_limit>)),
+    S14_FAST("route_mix", (bound<kRouteMix, s14_route_mix_dispatch, s14_cmd_route_mix>)),
+    S14_FAST("moe_accumulate", (bound<kAccumulate, s14_moe_accumulate_dispatch, s14_cmd_moe_accumulate>)),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_s14call", "Per-token calls of the Python mirror over the C ABI.", -1, methods,
