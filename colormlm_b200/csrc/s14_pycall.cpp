@@ -14,11 +14,41 @@
 namespace {
 
 PyObject *n_data_ptr, *n_shape, *n_dtype, *n_numel, *n_expert_ids, *n_weights, *n_pages;  // interned names
-PyObject *t_float32, *t_bfloat16;         // torch's dtypes
-PyObject *f_device, *f_raw_stream;        // torch._C's lookups of the current device and its current stream
+PyObject *n_value, *n_as_parameter, *n_cuda_stream;
+PyTypeObject *t_void_p;                   // ctypes.c_void_p
+// What torch has to be asked, filled on the first call that needs it (a program that names its streams and uses host
+// buffers does without torch): its dtypes, and the lookups of the current device and its current stream.
+PyObject *t_float32, *t_bfloat16;
+PyObject *f_device, *f_raw_stream;        // two C functions; where torch lacks them, f_stream: torch.cuda.current_stream
+PyObject *f_stream;
 
 struct Failed {};   // a Python error is set
 struct Refused {};  // not a call the library could take: None is returned
+
+// What ctypes passes as a void pointer beside ints: its own c_void_p, and objects that name one as their parameter
+// (torch.cuda.Stream is one).
+void *foreign_pointer(PyObject *v, int depth = 0) {
+    PyObject *inner = nullptr;
+    if (PyObject_TypeCheck(v, t_void_p)) inner = PyObject_GetAttr(v, n_value);
+    else if (depth < 2 && PyObject_HasAttr(v, n_as_parameter)) inner = PyObject_GetAttr(v, n_as_parameter);
+    else PyErr_Format(PyExc_TypeError, "an address or handle is needed, not %s", Py_TYPE(v)->tp_name);
+    if (!inner) throw Failed{};
+    void *p = nullptr;
+    bool failed = false;
+    if (PyLong_Check(inner)) {
+        p = PyLong_AsVoidPtr(inner);
+        failed = PyErr_Occurred() != nullptr;
+    } else if (inner != Py_None) {
+        try {
+            p = foreign_pointer(inner, depth + 1);
+        } catch (const Failed &) {
+            failed = true;
+        }
+    }
+    Py_DECREF(inner);
+    if (failed) throw Failed{};
+    return p;
+}
 
 void *address(PyObject *tensor) {
     PyObject *args[1] = {tensor};
@@ -31,8 +61,9 @@ void *address(PyObject *tensor) {
 }
 void *address_or_null(PyObject *tensor) { return tensor == Py_None ? nullptr : address(tensor); }
 
-void *pointer(PyObject *v) {  // a device address or handle held as an int, or None
+void *pointer(PyObject *v) {  // a device address or handle held as an int, a ctypes.c_void_p, None, or what stands in for one
     if (v == Py_None) return nullptr;
+    if (!PyLong_Check(v)) return foreign_pointer(v);
     void *p = PyLong_AsVoidPtr(v);
     if (PyErr_Occurred()) throw Failed{};
     return p;
@@ -68,11 +99,39 @@ uint32_t token_count(PyObject *x) {
     return sizes(x, n, 1) == 1 ? 1u : n[0];
 }
 
+PyObject *attr_of(PyObject *o, const char *name) {
+    if (!o) throw Failed{};
+    PyObject *v = PyObject_GetAttrString(o, name);
+    Py_DECREF(o);
+    if (!v) throw Failed{};
+    return v;
+}
+PyObject *torch_attr(const char *name) { return attr_of(PyImport_ImportModule("torch"), name); }
+void ask_torch_types() {
+    PyObject *f = torch_attr("float32"), *b = torch_attr("bfloat16");
+    t_float32 = f, t_bfloat16 = b;
+}
+void ask_torch_streams() {
+    PyObject *init = attr_of(torch_attr("cuda"), "init");  // the raw lookups do not initialise torch
+    PyObject *done = PyObject_CallNoArgs(init);
+    Py_DECREF(init);
+    if (!done) throw Failed{};
+    Py_DECREF(done);
+    try {
+        PyObject *d = attr_of(torch_attr("_C"), "_cuda_getDevice"), *r = attr_of(torch_attr("_C"), "_cuda_getCurrentRawStream");
+        f_device = d, f_raw_stream = r;
+    } catch (const Failed &) {
+        PyErr_Clear();
+        f_stream = attr_of(torch_attr("cuda"), "current_stream");
+    }
+}
+
 // S14_STREAM_*; a tensor of another type ends the call with None, which the Python side reports
 uint32_t stream_type(PyObject *tensor) {
     PyObject *d = PyObject_GetAttr(tensor, n_dtype);
     if (!d) throw Failed{};
     Py_DECREF(d);  // torch keeps its dtypes
+    if (!t_bfloat16) ask_torch_types();
     if (d == t_bfloat16) return S14_STREAM_BF16;
     if (d == t_float32) return S14_STREAM_F32;
     throw Refused{};
@@ -82,10 +141,19 @@ uint32_t stream_type(PyObject *tensor) {
 // (cudaStreamLegacy), because the C ABI reads NULL as the context's own stream.
 void *stream_of(PyObject *stream) {
     if (stream != Py_None) return pointer(stream);
-    PyObject *dev = PyObject_CallNoArgs(f_device);
-    if (!dev) throw Failed{};
-    PyObject *raw = PyObject_CallOneArg(f_raw_stream, dev);
-    Py_DECREF(dev);
+    if (!f_raw_stream && !f_stream) ask_torch_streams();
+    PyObject *raw;
+    if (f_raw_stream) {
+        PyObject *dev = PyObject_CallNoArgs(f_device);
+        if (!dev) throw Failed{};
+        raw = PyObject_CallOneArg(f_raw_stream, dev);
+        Py_DECREF(dev);
+    } else {
+        PyObject *current = PyObject_CallNoArgs(f_stream);
+        if (!current) throw Failed{};
+        raw = PyObject_GetAttr(current, n_cuda_stream);
+        Py_DECREF(current);
+    }
     if (!raw) throw Failed{};
     void *p = PyLong_AsVoidPtr(raw);
     Py_DECREF(raw);
@@ -399,16 +467,15 @@ PyMODINIT_FUNC PyInit__s14call(void) {
     n_expert_ids = PyUnicode_InternFromString("expert_ids");
     n_weights = PyUnicode_InternFromString("weights");
     n_pages = PyUnicode_InternFromString("pages");
-    PyObject *torch = PyImport_ImportModule("torch");
-    if (!torch) return nullptr;
-    PyObject *core = PyObject_GetAttrString(torch, "_C");
-    if (!core) return nullptr;
-    t_float32 = PyObject_GetAttrString(torch, "float32");
-    t_bfloat16 = PyObject_GetAttrString(torch, "bfloat16");
-    f_device = PyObject_GetAttrString(core, "_cuda_getDevice");
-    f_raw_stream = PyObject_GetAttrString(core, "_cuda_getCurrentRawStream");
-    Py_DECREF(core);
-    Py_DECREF(torch);
-    if (!t_float32 || !t_bfloat16 || !f_device || !f_raw_stream) return nullptr;
+    n_value = PyUnicode_InternFromString("value");
+    n_as_parameter = PyUnicode_InternFromString("_as_parameter_");
+    n_cuda_stream = PyUnicode_InternFromString("cuda_stream");
+    PyObject *ctypes = PyImport_ImportModule("ctypes");
+    if (!ctypes) return nullptr;
+    PyObject *void_p = PyObject_GetAttrString(ctypes, "c_void_p");
+    Py_DECREF(ctypes);
+    if (!void_p) return nullptr;
+    if (!PyType_Check(void_p)) return PyErr_Format(PyExc_TypeError, "ctypes.c_void_p is not a class");
+    t_void_p = (PyTypeObject *)void_p;
     return PyModule_Create(&module);
 }

@@ -98,7 +98,9 @@ def _resolve_torch_stream():
     import torch
 
     torch.cuda.init()  # the raw lookups below do not initialise torch's CUDA state
-    device, raw = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+    device, raw = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device is None or raw is None:  # not part of torch's public interface
+        return lambda: torch.cuda.current_stream().cuda_stream or 1
 
     def lookup() -> int:
         return raw(device()) or 1

@@ -1,5 +1,7 @@
 """Operators behind a kernel of the caller that lets its dependents start early and writes their operands late, weights
 and pages included: the operator reads what that kernel leaves (GPU)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -106,3 +108,16 @@ def test_operands_written_late_by_a_kernel_that_lets_dependents_start(ctx, write
             torch.cuda.synchronize()
             assert torch.equal(y, want)
     assert ctx.device_status() == 0
+
+
+def test_streams_named_in_every_form(ctx):
+    x, w, want = torch.randn(3, 512, device="cuda"), torch.rand(512, device="cuda"), torch.empty(3, 512, device="cuda")
+    ctx.cmd_rms_norm(x, w, want)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for stream in (side, side.cuda_stream, ctypes.c_void_p(side.cuda_stream), None):
+        out = torch.zeros_like(want)
+        torch.cuda.synchronize()
+        ctx.cmd_rms_norm(x, w, out, stream=stream)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
