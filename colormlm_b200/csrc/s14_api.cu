@@ -2213,6 +2213,9 @@ static void check_hc(const char *what, const s14_ctx *ctx, const s14_hc_params *
     if (!p->hc_fn || !p->hc_scale || !p->hc_base) throw ContractError(std::string(what) + ": hc_fn, hc_scale or hc_base is NULL");
     if (!std::isfinite(p->norm_eps) || p->norm_eps <= 0.0f || !std::isfinite(p->hc_eps) || p->hc_eps <= 0.0f)
         throw ContractError(std::string(what) + ": norm_eps and hc_eps must be finite and positive");
+    // the dot products read four elements at a time
+    require_aligned(x, p->dtype == S14_STREAM_BF16 ? 8 : 16, "S14 token streams");
+    require_aligned(p->hc_fn, 16, "S14 hc_fn");
 }
 
 static int32_t hc_reduce_call(s14_ctx *ctx, void *stream, const s14_hc_params *p, bool head, const void *x, void *reduced,
@@ -2334,6 +2337,7 @@ extern "C" int32_t s14_exec_hc_head_norm_full_logits(s14_ctx *ctx, void *stream,
     if (n_rows == 0) throw ContractError("s14_exec_hc_head_norm_full_logits: no vocabulary rows");
     if (head->hidden > kMaxDim) throw ContractError("s14_exec_hc_head_norm_full_logits: hidden above 4096");
     check_hc("s14_exec_hc_head_norm_full_logits", ctx, head, state_bf16);
+    require_aligned(head_weight_bf16, 16, "S14 head weight");
     CUDA_OK(cudaSetDevice(ctx->device));
     cudaStream_t st = stream_of(ctx, stream);
     CUDA_OK(launch_head_prep(st, state_bf16, head->hc_fn, head->hc_scale, head->hc_base, norm_weight, head->hidden, head->norm_eps,

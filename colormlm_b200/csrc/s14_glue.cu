@@ -39,7 +39,9 @@ __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
 }
 
 // Eight stream values from one (BF16) or two (F32) 16-byte loads, and back; one by one where a caller's buffer is not
-// aligned to 16 bytes (`vec`, the same for all threads of a launch).
+// aligned to 16 bytes (`vec`, the same for all threads of a launch): all of hc_post and rms_norm, and hc_pre's reduced
+// vector.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the calls
+// refuse what is not aligned for that.
 template <bool kBf16>
 __device__ __forceinline__ void stream_ld8(const void *p, size_t i, float (&v)[8], bool vec) {
     if (!vec) {

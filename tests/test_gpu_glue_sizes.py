@@ -6,8 +6,9 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
+from colormlm_b200 import _lib as L
 from colormlm_b200 import synth
-from colormlm_b200.s14 import S14Context
+from colormlm_b200.s14 import S14Context, S14Error
 
 from .test_gpu_glue import bits16, close_coeff, close_streams, dev, f32_of_bits
 
@@ -76,3 +77,42 @@ def test_buffers_that_are_not_16_byte_aligned(ctx, bf16):
     ctx.cmd_hc_post(moved(branch), moved(res), post, comb, got_m)
     ctx.cmd_rms_norm(moved(branch), moved(nw), got_n)
     assert torch.equal(got_m, want_m) and torch.equal(got_n, want_n)
+
+
+def _offset(a, elements):
+    """A copy of a that lies `elements` past a 16-byte boundary."""
+    big = torch.empty(a.numel() + elements, dtype=a.dtype, device="cuda")
+    big[elements:] = a.reshape(-1)
+    return big[elements:].view(a.shape)
+
+
+@pytest.mark.parametrize("tokens", [1, 11])
+def test_reduce_of_streams_on_the_boundaries_it_takes(ctx, tokens):
+    """BF16 streams on an 8-byte boundary and results on any are taken; what the dot products cannot read is refused before
+    anything is launched."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    h = 512
+    x = torch.randn(tokens, 4, h, device="cuda", generator=g)
+    fn = torch.randn(24, 4 * h, device="cuda", generator=g) * 0.02
+    scale, base = torch.rand(3, device="cuda", generator=g), torch.rand(24, device="cuda", generator=g)
+    post, comb, pre = torch.empty(tokens, 4, device="cuda"), torch.empty(tokens, 4, 4, device="cuda"), torch.empty(tokens, 4, device="cuda")
+    b = x.to(torch.bfloat16)
+    red, moved = torch.empty(tokens, h, dtype=b.dtype, device="cuda"), _offset(torch.zeros(tokens, h, dtype=b.dtype, device="cuda"), 1)
+    ctx.cmd_hc_pre(b, fn, scale, base, red, post, comb)
+    ctx.cmd_hc_pre(_offset(b, 4), fn, _offset(scale, 1), _offset(base, 3), moved, _offset(post, 1), _offset(comb, 1))
+    assert torch.equal(red, moved)
+    launched = ctx.launch_count
+    for streams, matrix in ((_offset(b, 1), fn), (_offset(b, 2), fn), (_offset(x, 1), fn), (_offset(x, 2), fn), (x, _offset(fn, 1)),
+                            (b, _offset(fn, 2))):
+        out = torch.empty(tokens, h, dtype=streams.dtype, device="cuda")
+        for call in (lambda: ctx.cmd_hc_pre(streams, matrix, scale, base, out, post, comb),
+                     lambda: ctx.cmd_hc_head_reduce(streams, matrix, scale, base, out, pre)):
+            with pytest.raises(S14Error) as e:
+                call()
+            assert e.value.code == L.ERR_CONTRACT
+    w, norm, logits = torch.ones(20, h, dtype=torch.bfloat16, device="cuda").view(torch.int16), torch.ones(h, device="cuda"), torch.empty(20, device="cuda")
+    for state, matrix, head in ((_offset(b[:1], 1), fn, w), (b[:1], _offset(fn, 1), w), (b[:1], fn, _offset(w, 4))):
+        with pytest.raises(S14Error):
+            ctx.exec_hc_head_norm_full_logits(state, matrix, scale, base, norm, head, logits)
+    assert ctx.launch_count == launched
+    torch.cuda.synchronize()
