@@ -213,7 +213,9 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
     }
 }
 
-// Any hidden size that is a multiple of 8: a warp per row; 8 products in F32, carried in F64.
+// Any hidden size that is a multiple of 8: a warp per row; 8 products in F32, carried in F64.  Up to four tokens the
+// weight stream bounds it and four loads per lane pay (129280 x 4104, one token: 228 us, with one load 263; four tokens
+// 541 and 598); from five on the warps that the registers of four would cost do more (eight tokens 1138 and 1066).
 template <int NT>
 __global__ void __launch_bounds__(256)
 k_head_logits(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
@@ -221,30 +223,41 @@ k_head_logits(const float *__restrict__ x, const uint16_t *__restrict__ w, float
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    constexpr int kLoads = NT <= 4 ? 4 : 1;
     for (uint32_t v = warp; v < n_rows; v += n_warps) {
         const uint4 *row = reinterpret_cast<const uint4 *>(w + (size_t)v * hidden);
         double acc[NT];
 #pragma unroll
         for (int t = 0; t < NT; ++t) acc[t] = 0.0;
-        for (uint32_t p = lane; p < (hidden >> 3); p += 32u) {
-            const uint4 q = ldg_stream(row + p);
-            const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
-            float wf[8];
+        // 16-byte loads of the row in flight per lane (the row is read once, from HBM); the sums are taken in the order of
+        // the pieces
+        for (uint32_t p0 = lane; p0 < (hidden >> 3); p0 += 32u * kLoads) {
+            uint4 q4[kLoads];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                wf[i * 2] = __uint_as_float(wd[i] << 16);
-                wf[i * 2 + 1] = __uint_as_float(wd[i] & 0xffff0000u);
-            }
+            for (int u = 0; u < kLoads; ++u)
+                q4[u] = (p0 + 32u * u < (hidden >> 3)) ? ldg_stream(row + p0 + 32u * u) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8));
-                const float4 xb = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8 + 4));
-                float2 part = make_float2(0.f, 0.f);
-                part = __ffma2_rn(make_float2(wf[0], wf[1]), make_float2(xa.x, xa.y), part);
-                part = __ffma2_rn(make_float2(wf[2], wf[3]), make_float2(xa.z, xa.w), part);
-                part = __ffma2_rn(make_float2(wf[4], wf[5]), make_float2(xb.x, xb.y), part);
-                part = __ffma2_rn(make_float2(wf[6], wf[7]), make_float2(xb.z, xb.w), part);
-                acc[t] += (double)part.x + (double)part.y;
+            for (int u = 0; u < kLoads; ++u) {
+                const uint32_t p = p0 + 32u * u;
+                if (p >= (hidden >> 3)) break;
+                const uint32_t wd[4] = {q4[u].x, q4[u].y, q4[u].z, q4[u].w};
+                float wf[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    wf[i * 2] = __uint_as_float(wd[i] << 16);
+                    wf[i * 2 + 1] = __uint_as_float(wd[i] & 0xffff0000u);
+                }
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8));
+                    const float4 xb = __ldg(reinterpret_cast<const float4 *>(x + (size_t)t * hidden + p * 8 + 4));
+                    float2 part = make_float2(0.f, 0.f);
+                    part = __ffma2_rn(make_float2(wf[0], wf[1]), make_float2(xa.x, xa.y), part);
+                    part = __ffma2_rn(make_float2(wf[2], wf[3]), make_float2(xa.z, xa.w), part);
+                    part = __ffma2_rn(make_float2(wf[4], wf[5]), make_float2(xb.x, xb.y), part);
+                    part = __ffma2_rn(make_float2(wf[6], wf[7]), make_float2(xb.z, xb.w), part);
+                    acc[t] += (double)part.x + (double)part.y;
+                }
             }
         }
 #pragma unroll

@@ -20,9 +20,10 @@ def ctx():
 
 
 # rows: less than a tile, tiles with a remainder, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in
-# phases); hidden: one group of steps, several phases, a size the tensor-core kernel leaves to the other one (264)
-@pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (2, 17, 1280), (3, 2385, 4096), (5, 33, 264),
-                                                (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096)])
+# phases); hidden: one group of steps, several phases, sizes the tensor-core kernel leaves to the other one (264; 1048:
+# more than its four pieces per lane)
+@pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (2, 17, 1280), (3, 2385, 4096), (5, 33, 264), (3, 300, 1048),
+                                                (8, 300, 1048), (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096)])
 def test_logits_at_the_edges_of_the_tiles(ctx, tokens, rows, hidden):
     g = torch.Generator(device="cuda").manual_seed(tokens * rows + hidden)
     x = torch.randn(tokens, hidden, device="cuda", generator=g)
