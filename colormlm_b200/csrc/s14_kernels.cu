@@ -1093,7 +1093,7 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
     int launches = 0;
     *err = cudaSuccess;
     t_last_layer_path = 0;
-    if (n_tokens == 1u && y && !ep && !km && counters && (router ? router->ep_world <= 1u : !dev_table)) {
+    if (n_tokens == 1u && y && !ep && counters && (router ? router->ep_world <= 1u : !dev_table)) {
         // the checkpoint's page kinds: routed MXFP4 experts and an FP8 shared expert
         JobTable routed = {};
         const uint8_t *shared = nullptr;
@@ -1127,8 +1127,11 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                 ++launches;
                 x_bf16 = nullptr;
             }
+            if (km) cudaEventRecord(km->ev[0], st), cudaEventRecord(km->ev[1], st);
             launches += launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
                                                 counters, umma, hidden, inter, err);
+            if (km)  // as for the layer kernel alone (below): all of it is booked as the up phase
+                for (int i = 2; i < 5; ++i) cudaEventRecord(km->ev[i], st);
             t_last_layer_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
             return launches;
         }

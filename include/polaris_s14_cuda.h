@@ -125,7 +125,9 @@ S14_API uint32_t s14_ctx_last_layer_path(const s14_ctx *ctx);
  * every such call records CUDA events around its kernels, waits for the stream and
  * accumulates the durations (router, up phase, down phase, mix), the counterpart of
  * the reference's timestamp queries (examples/s14_vulkan_numeric.rs:1088-1101,
- * 1220-1260).  Not for timed throughput runs: the call becomes blocking. */
+ * 1220-1260).  The kernels are the ones that run without it; where one kernel runs several phases (the tensor-core
+ * layer kernel, with or without the two launches of an FP8 shared expert), all of its time is booked as the up
+ * phase.  Not for timed throughput runs: the call becomes blocking. */
 S14_API int32_t s14_ctx_set_kernel_timing(s14_ctx *ctx, int32_t enable);
 S14_API int32_t s14_ctx_kernel_times(s14_ctx *ctx, double ms_out[4], uint64_t *calls);
 

@@ -51,6 +51,32 @@ def test_layer_and_executor_step_with_an_fp8_shared_expert(ctx, oracle, hidden, 
     assert torch.equal(branch, y[0].to(torch.bfloat16)) and torch.equal(state, merged)
 
 
+def routed_layer(seed, hidden, inter, n_experts):
+    """A routed layer with an FP8 shared page: host pages and router, and what the calls take."""
+    g, pages, shared = make_layer(seed, hidden, inter, n_experts, L.PAGE_FP8)
+    wr, bias = synth.router_weight_bf16(g, n_experts, hidden), synth.router_bias(g, n_experts)
+    pd, sd = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter, L.PAGE_FP8)
+    table = torch.tensor([p.data_ptr() for p in pd], dtype=torch.int64, device="cuda")
+    x = synth.activations(g, 1, hidden)
+    return pages, shared, wr, bias, x, (pd, sd), (dev(wr.view(np.int16)), dev(bias), table, sd.data_ptr(), L.PAGE_FP8, inter)
+
+
+def test_kernel_timing_leaves_the_layer_on_its_path(ctx):
+    hidden, inter = 1024, 2048
+    _, _, _, _, x, keep, args = routed_layer(12, hidden, inter, 16)
+    dx, plain, timed = dev(x), torch.empty(1, hidden, device="cuda"), torch.empty(1, hidden, device="cuda")
+    ctx.cmd_routed_moe_layer(dx[0], *args, plain)
+    path = ctx.last_layer_path
+    ctx.set_kernel_timing(True)
+    try:
+        ctx.cmd_routed_moe_layer(dx[0], *args, timed)
+        times, calls = ctx.kernel_times()
+    finally:
+        ctx.set_kernel_timing(False)
+    assert path == PATH and ctx.last_layer_path == path and torch.equal(plain, timed)
+    assert calls == 1 and times["up"] > 0.0  # (one mark after all of the layer's kernels)
+
+
 # elements past a 16-byte boundary: 2-, 4- and 8-byte ones; the state and the branch lie there too
 @pytest.mark.parametrize("offset", [1, 2, 4])
 @pytest.mark.parametrize("kind", [L.PAGE_FP8, L.PAGE_MXFP4])
