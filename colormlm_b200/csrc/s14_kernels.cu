@@ -1093,25 +1093,27 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
     int launches = 0;
     *err = cudaSuccess;
     t_last_layer_path = 0;
-    if (n_tokens == 1u && y && !ep && counters && (router ? router->ep_world <= 1u : !dev_table)) {
-        // the checkpoint's page kinds: routed MXFP4 experts and an FP8 shared expert
+    // the checkpoint's page kinds: routed MXFP4 experts and an FP8 shared expert
+    const uint8_t *shared = nullptr;
+    if (n_tokens == 1u && y && !ep && counters) {
+        if (router && router->ep_world <= 1u && router->shared_kind == S14_PAGE_FP8) shared = router->shared_page;
+        if (!router && !dev_table)
+            for (uint32_t j = 0; j < param_table.n_jobs; ++j)
+                if (param_table.jobs[j].is_shared && param_table.jobs[j].kind == S14_PAGE_FP8) shared = param_table.jobs[j].page;
+    }
+    if (shared) {
         JobTable routed = {};
-        const uint8_t *shared = nullptr;
         uint32_t n_routed = 0;
         FusedRouter rt = {};
         if (router) {
             rt = *router;
-            if (rt.shared_page && rt.shared_kind == S14_PAGE_FP8) shared = rt.shared_page;
             rt.shared_page = nullptr;
             n_routed = umma_router_ok(sm_count, rt.n_experts) ? rt.top_k : 0u;
         } else {
             routed.n_tokens = 1;
             for (uint32_t i = param_table.token_job_begin[0]; i < param_table.token_job_begin[1]; ++i) {
                 Job jb = param_table.jobs[param_table.token_jobs[i]];
-                if (jb.is_shared && jb.kind == S14_PAGE_FP8) {
-                    shared = jb.page;
-                    continue;
-                }
+                if (jb.is_shared) continue;
                 jb.out_index = n_routed;
                 routed.jobs[n_routed] = jb;
                 routed.token_jobs[n_routed] = (uint8_t)n_routed;
@@ -1119,7 +1121,7 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
             }
             routed.n_jobs = routed.token_job_begin[1] = n_routed;
         }
-        if (shared && fp8_shared_layer_ok(sm_count, mode, umma, n_routed, hidden, inter)) {
+        if (fp8_shared_layer_ok(sm_count, mode, umma, n_routed, hidden, inter)) {
             // the expert's kernel reads a BF16 token in 8-byte pieces; a token on another boundary is converted first
             if (!fp8_expert_takes(x_bf16)) {
                 *err = launch_bf16_to_f32(st, x_bf16, x_stage, hidden);
