@@ -61,6 +61,31 @@ def routed_layer(seed, hidden, inter, n_experts):
     return pages, shared, wr, bias, x, (pd, sd), (dev(wr.view(np.int16)), dev(bias), table, sd.data_ptr(), L.PAGE_FP8, inter)
 
 
+# the router inside the layer kernel: fewer experts than SMs, and two experts' rows for some CTAs
+@pytest.mark.parametrize("hidden,inter,n_experts", [(1024, 2048, 7), (2048, 1024, 200), (4096, 2048, 24)])
+def test_routed_layer_with_an_fp8_shared_expert(ctx, oracle, hidden, inter, n_experts):
+    """The device call with and without outputs for the route, the call on host buffers and the bound one: the
+    oracle's route, its layer, and the same bits from each."""
+    pages, shared, wr, bias, x, keep, args = routed_layer(40 + n_experts, hidden, inter, n_experts)
+    ids, wts = torch.empty(6, dtype=torch.int32, device="cuda"), torch.empty(6, device="cuda")
+    y, again = torch.empty(1, hidden, device="cuda"), torch.empty(1, hidden, device="cuda")
+    for out, outs in ((y, (ids, wts)), (again, ())):
+        ctx.cmd_routed_moe_layer(dev(x)[0], *args, out, *outs)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and ctx.last_layer_path == PATH
+    rid, rw, _, _ = oracle.router(x[0], wr, bias, 0, 6, 1.0)
+    assert np.array_equal(ids.cpu().numpy(), rid) and np.array_equal(wts.cpu().numpy().view(np.uint32), rw.view(np.uint32))
+    want = oracle.moe_layer_acc64(x[0], [pages[i] for i in rid], rw, shared, L.PAGE_FP8, hidden, inter)
+    assert_pairwise_close(oracle, y.cpu().numpy()[0], want)
+    assert torch.equal(y, again)
+    bound = ctx.bind_routed_moe_layer_host(*args)
+    for call in (lambda *a: bound(x[0], *a), lambda out, i, w: ctx.routed_moe_layer_host(x[0], out, *args, i, w)):
+        host, host_ids, host_w = np.full(hidden, np.nan, np.float32), np.full(6, -1, np.int32), np.zeros(6, np.float32)
+        call(host, host_ids, host_w)
+        assert np.array_equal(host.view(np.uint32), y.cpu().numpy()[0].view(np.uint32))
+        assert np.array_equal(host_ids, rid) and np.array_equal(host_w.view(np.uint32), rw.view(np.uint32))
+
+
 def test_kernel_timing_leaves_the_layer_on_its_path(ctx):
     hidden, inter = 1024, 2048
     _, _, _, _, x, keep, args = routed_layer(12, hidden, inter, 16)
