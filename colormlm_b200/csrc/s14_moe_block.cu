@@ -426,9 +426,7 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i) {
                 const uint32_t nt = s_rec[i].nt & 0xFFu;
-                uint32_t vec[kHalf];   // (small blocks: chunks of one MMA)
-#pragma unroll
-                for (uint32_t t = 0; t < kHalf; ++t) vec[t] = kDown ? s_rec[i].pair[t] : s_rec[i].tok[t];
+                const uint32_t *vecs = kDown ? s_rec[i].pair : s_rec[i].tok;   // (small blocks: chunks of one MMA)
 #pragma unroll 1
                 for (uint32_t u = 0; u < nu; ++u) {
                     if (p_round && !mbar_wait(bar(kGBarDone + p_slot), (p_round - 1u) & 1u, abortp)) {
@@ -436,9 +434,11 @@ k_block_gemm(const __grid_constant__ GemmArgs a, uint32_t *status) {
                         break;
                     }
                     const uint32_t full = bar(kGBarFull + p_slot), dst = smem_u32(sRing) + p_slot * a.stage + kMt * kStageA;
-#pragma unroll
-                    for (uint32_t t = 0; t < kHalf; ++t)
-                        if (t < nt) bulk_copy(dst + t * kTileB, a.dig + ((size_t)vec[t] * nu + u) * kTileB, kTileB, full);
+                    // (a loop over the tokens there are: walking all that a chunk may hold, twelve predicated copies per
+                    // unit, this thread bound official blocks: 8 tokens of 128 experts 155 us, so 117; F32 119 and 114)
+#pragma unroll 1
+                    for (uint32_t t = 0; t < nt; ++t)
+                        bulk_copy(dst + t * kTileB, a.dig + ((size_t)vecs[t] * nu + u) * kTileB, kTileB, full);
                     if (++p_slot == ring) {
                         p_slot = 0;
                         ++p_round;
