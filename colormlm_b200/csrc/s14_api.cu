@@ -132,7 +132,7 @@ extern "C" int32_t s14_ctx_create(int32_t device, s14_ctx **out) {
     CUDA_OK(cudaMalloc(&ctx->scores, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->select, sizeof(float) * kMaxTokens * S14_N_ROUTED_EXPERTS));
     CUDA_OK(cudaMalloc(&ctx->dev_table, sizeof(JobTable)));
-    CUDA_OK(cudaMalloc(&ctx->glue, hc_scratch_bytes(kGlueTokens)));
+    CUDA_OK(cudaMalloc(&ctx->glue, hc_scratch_bytes(kGlueTokens, ctx->sm_count)));
     CUDA_OK(cudaMalloc(&ctx->x_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->y_stage, sizeof(float) * kMaxTokens * kMaxDim));
     CUDA_OK(cudaMalloc(&ctx->status, sizeof(uint32_t)));
@@ -2228,7 +2228,7 @@ static int32_t hc_reduce_call(s14_ctx *ctx, void *stream, const s14_hc_params *p
     if (!head && p->sinkhorn_iters == 0) throw ContractError(std::string(what) + ": at least one Sinkhorn round");
     CUDA_OK(cudaSetDevice(ctx->device));
     cudaError_t err;
-    ctx->launches += launch_hc_pre(stream_of(ctx, stream), p->dtype == S14_STREAM_BF16, head, p->n_tokens, p->hidden, x, p->hc_fn,
+    ctx->launches += launch_hc_pre(stream_of(ctx, stream), ctx->sm_count, p->dtype == S14_STREAM_BF16, head, p->n_tokens, p->hidden, x, p->hc_fn,
                                    p->hc_scale, p->hc_base, p->norm_eps, p->sinkhorn_iters, p->hc_eps, ctx->glue, reduced,
                                    post, comb, pre, &err);
     if (err != cudaSuccess) return cuda_fail(err, what);
@@ -2252,7 +2252,7 @@ extern "C" int32_t s14_cmd_hc_post(s14_ctx *ctx, void *stream, uint32_t n_tokens
     if (!ctx || !branch || !residual || !post || !comb || !merged) throw ContractError("s14_cmd_hc_post: NULL argument");
     check_streams("s14_cmd_hc_post", n_tokens, hc, hidden, dtype);
     CUDA_OK(cudaSetDevice(ctx->device));
-    const cudaError_t err = launch_hc_post(stream_of(ctx, stream), dtype == S14_STREAM_BF16, n_tokens, hidden, branch, residual, post,
+    const cudaError_t err = launch_hc_post(stream_of(ctx, stream), ctx->sm_count, dtype == S14_STREAM_BF16, n_tokens, hidden, branch, residual, post,
                                            comb, merged);
     ctx->launches += 1;
     if (err != cudaSuccess) return cuda_fail(err, "s14_cmd_hc_post");
@@ -2267,7 +2267,7 @@ extern "C" int32_t s14_cmd_rms_norm(s14_ctx *ctx, void *stream, uint32_t n_token
     check_streams("s14_cmd_rms_norm", n_tokens, 4, hidden, dtype);
     if (!std::isfinite(eps) || eps <= 0.0f) throw ContractError("s14_cmd_rms_norm: eps must be finite and positive");
     CUDA_OK(cudaSetDevice(ctx->device));
-    const cudaError_t err = launch_rms_norm(stream_of(ctx, stream), dtype == S14_STREAM_BF16, n_tokens, hidden, x, weight, eps, out);
+    const cudaError_t err = launch_rms_norm(stream_of(ctx, stream), ctx->sm_count, dtype == S14_STREAM_BF16, n_tokens, hidden, x, weight, eps, out);
     ctx->launches += 1;
     if (err != cudaSuccess) return cuda_fail(err, "s14_cmd_rms_norm");
     return S14_OK;

@@ -80,6 +80,11 @@ __device__ __forceinline__ uint32_t ld_u8(const uint8_t *p) {
     asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
+__device__ __forceinline__ float4 ld_f32x4(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float ld_f32(const float *p) {
     float v;
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));

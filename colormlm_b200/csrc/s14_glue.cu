@@ -11,6 +11,8 @@
 // arithmetic of the CPU restatement the tests compare with.
 // A token's state is hc = 4 streams of `hidden` values, F32 or BF16 (the reference's state is BF16
 // [1, 1, 4, 4096]); results are rounded to the streams' type where the Python code casts back.
+#include <type_traits>
+
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -38,47 +40,61 @@ __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
     else reinterpret_cast<float *>(p)[i] = v;
 }
 
-// Eight stream values from one (BF16) or two (F32) 16-byte loads, and back; one by one where a caller's buffer is not
-// aligned to 16 bytes (`vec`, the same for all threads of a launch): all of hc_post and rms_norm, and hc_pre's reduced
-// vector.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the calls
-// refuse what is not aligned for that.
-template <bool kBf16>
-__device__ __forceinline__ void stream_ld8(const void *p, size_t i, float (&v)[8], bool vec) {
+// N consecutive stream values, back and forth: eight BF16 or four F32 values are one 16-byte access, four BF16 values one of 8
+// bytes, eight F32 values two of 16 (which a warp's lanes make 32 bytes apart); one by one where a caller's buffer is
+// not aligned to 16 bytes (`vec`, the same for all threads of a launch): all of hc_post and rms_norm, and hc_pre's
+// reduced vector.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the
+// calls refuse what is not aligned for that.
+template <bool kBf16, int N>
+__device__ __forceinline__ void stream_ldn(const void *p, size_t i, float (&v)[N], bool vec) {
+    static_assert(N == 4 || N == 8, "values per thread");
     if (!vec) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = stream_ld<kBf16>(p, i + k);
+        for (int k = 0; k < N; ++k) v[k] = stream_ld<kBf16>(p, i + k);
         return;
     }
     if constexpr (kBf16) {
-        const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(p) + i));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        uint32_t w[N / 2];
+        const uint16_t *at = reinterpret_cast<const uint16_t *>(p) + i;
+        if constexpr (N == 8) {
+            const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(at));
+            w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+        } else {
+            const uint2 q = __ldcg(reinterpret_cast<const uint2 *>(at));
+            w[0] = q.x, w[1] = q.y;
+        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[2 * k] = __uint_as_float(w[k] << 16), v[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+        for (int k = 0; k < N / 2; ++k) v[2 * k] = __uint_as_float(w[k] << 16), v[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
     } else {
-        const float4 a = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i));
-        const float4 b = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i) + 1);
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        const float4 *at = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i);
+#pragma unroll
+        for (int k = 0; k < N / 4; ++k) {
+            const float4 a = __ldcg(at + k);
+            v[4 * k] = a.x, v[4 * k + 1] = a.y, v[4 * k + 2] = a.z, v[4 * k + 3] = a.w;
+        }
     }
 }
-template <bool kBf16>
-__device__ __forceinline__ void stream_st8(void *p, size_t i, const float (&v)[8], bool vec) {
+template <bool kBf16, int N>
+__device__ __forceinline__ void stream_stn(void *p, size_t i, const float (&v)[N], bool vec) {
     if (!vec) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) stream_st<kBf16>(p, i + k, v[k]);
+        for (int k = 0; k < N; ++k) stream_st<kBf16>(p, i + k, v[k]);
         return;
     }
     if constexpr (kBf16) {
-        uint32_t w[4];
+        uint32_t w[N / 2];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < N / 2; ++k) {
             const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
             w[k] = *reinterpret_cast<const uint32_t *>(&b);
         }
-        *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p) + i) = make_uint4(w[0], w[1], w[2], w[3]);
+        uint16_t *at = reinterpret_cast<uint16_t *>(p) + i;
+        if constexpr (N == 8) *reinterpret_cast<uint4 *>(at) = make_uint4(w[0], w[1], w[2], w[3]);
+        else *reinterpret_cast<uint2 *>(at) = make_uint2(w[0], w[1]);
     } else {
-        float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p) + i);
-        o[0] = make_float4(v[0], v[1], v[2], v[3]);
-        o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        float4 *at = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p) + i);
+#pragma unroll
+        for (int k = 0; k < N / 4; ++k) at[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     }
 }
 
@@ -124,15 +140,15 @@ __device__ __forceinline__ void split_sinkhorn_warp(const float *mixes, const fl
     comb = c;
 }
 
-// reduced[d] = sum_h pre[h] x[h][d] for eight consecutive d.
-template <bool kBf16>
-__device__ __forceinline__ void reduce_streams8(const void *x, size_t x0, uint32_t hidden, uint32_t d, const float (&pre)[kHc],
-                                                float (&acc)[8], bool vec) {
-    float v[kHc][8];
+// reduced[d] = sum_h pre[h] x[h][d] for N consecutive d.
+template <bool kBf16, int N>
+__device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_t hidden, uint32_t d, const float (&pre)[kHc],
+                                               float (&acc)[N], bool vec) {
+    float v[kHc][N];
 #pragma unroll
-    for (uint32_t h = 0; h < kHc; ++h) stream_ld8<kBf16>(x, x0 + (size_t)h * hidden + d, v[h], vec);
+    for (uint32_t h = 0; h < kHc; ++h) stream_ldn<kBf16, N>(x, x0 + (size_t)h * hidden + d, v[h], vec);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < N; ++k) {
         acc[k] = __fmul_rn(pre[0], v[0][k]);
 #pragma unroll
         for (uint32_t h = 1; h < kHc; ++h) acc[k] = __fadd_rn(acc[k], __fmul_rn(pre[h], v[h][k]));
@@ -140,24 +156,23 @@ __device__ __forceinline__ void reduce_streams8(const void *x, size_t x0, uint32
 }
 
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
-// only) of few tokens: one cluster of sixteen CTAs per token.  The call is all latency: 1.5 MB of fn per token,
-// then a serial chain of 20 Sinkhorn rounds.  Every CTA takes a sixteenth of the flattened streams against all
-// rows of fn (98 KB, all loads in flight together), the partial sums
-// cross in shared memory, every CTA makes the coefficients itself and reduces its sixteenth of the hidden
-// vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
-constexpr uint32_t kPreCluster = 16, kPreThreads = 512;
-template <bool kBf16, bool kHead>
+// only) of few tokens: one cluster of CTAs per token (sixteen, fewer for more tokens: launch_hc_pre).  The call is all
+// latency: 1.5 MB of fn per token, then a serial chain of 20 Sinkhorn rounds.  Every CTA takes its share of the
+// flattened streams against all rows of fn (98 KB, all loads in flight together), the partial sums cross in
+// shared memory, every CTA makes the coefficients itself and reduces its share of the hidden vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
+constexpr uint32_t kPreThreads = 512;
+template <bool kBf16, bool kHead, uint32_t kCluster>
 __global__ void __launch_bounds__(kPreThreads)
 k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *__restrict__ scale, const float *__restrict__ base,
          uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced, float *__restrict__ post_out,
          float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec) {
     constexpr uint32_t n_mix = kHead ? kHc : kMixMax, kRows = n_mix / 2u;   // rows per half of the CTA
     __shared__ double s_warp[kPreThreads / 32][kRows + 1];
-    __shared__ double s_part[kPreCluster][n_mix + 1];                      // [n_mix]: the sum of squares
+    __shared__ double s_part[kCluster][n_mix + 1];                      // [n_mix]: the sum of squares
     __shared__ float s_mix[n_mix], s_pre[kHc], s_coef[3 + n_mix];            // [3 + n_mix]: scale, base
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), t = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t n = kHc * hidden, share = n / kPreCluster, k0 = rank * share;   // a multiple of 64
+    const uint32_t n = kHc * hidden, share = n / kCluster, k0 = rank * share;   // a multiple of 64
     const uint32_t half = tid >> 8, c = tid & 255u;                          // half of the rows, column of four elements
     double acc[kRows], ss = 0.0;
 #pragma unroll
@@ -201,14 +216,14 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
 #pragma unroll
         for (uint32_t w = 0; w < 8u; ++w) s += s_warp[w0 + w][m];
 #pragma unroll
-        for (uint32_t r = 0; r < kPreCluster; ++r) *cluster.map_shared_rank(&s_part[rank][tid], r) = s;
+        for (uint32_t r = 0; r < kCluster; ++r) *cluster.map_shared_rank(&s_part[rank][tid], r) = s;
     }
     cluster.sync();
     if (warp == 0u) {
         double s = 0.0;
         if (lane <= n_mix) {
 #pragma unroll
-            for (uint32_t r = 0; r < kPreCluster; ++r) s += s_part[r][lane];
+            for (uint32_t r = 0; r < kCluster; ++r) s += s_part[r][lane];
         }
         const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, n_mix) / (double)n), norm_eps);
         if (lane < n_mix) s_mix[lane] = __fmul_rn((float)s, rs);
@@ -221,7 +236,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
         }
     }
     __syncthreads();
-    const uint32_t part = hidden / kPreCluster;   // a multiple of 16
+    const uint32_t part = hidden / kCluster;   // a multiple of 16
     if (!kHead && rank == 0u && warp == 0u) {
         float pre, post, comb;
         split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
@@ -232,8 +247,8 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     // the last threads, so that the warp with the Sinkhorn rounds has none of it
     for (uint32_t i = (kPreThreads - 1u - tid) * 8u; i < part; i += kPreThreads * 8u) {
         float v[8];
-        reduce_streams8<kBf16>(x, (size_t)t * n, hidden, rank * part + i, pre, v, vec != 0u);
-        stream_st8<kBf16>(reduced, (size_t)t * hidden + rank * part + i, v, vec != 0u);
+        reduce_streams<kBf16, 8>(x, (size_t)t * n, hidden, rank * part + i, pre, v, vec != 0u);
+        stream_stn<kBf16, 8>(reduced, (size_t)t * hidden + rank * part + i, v, vec != 0u);
     }
 }
 
@@ -244,16 +259,17 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
 // the FP64 pipe's 64 products per clock and SM bound it at 8).  K is permuted inside steps of sixteen: lane q of
 // a quad takes four consecutive elements as its slots of four MMAs.  Writes partial sums [slice][token][25] in double.
 constexpr uint32_t kDotTokens = 16;
-template <bool kBf16>
+template <bool kBf16, bool kHead>
 __global__ void __launch_bounds__(256)
 k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, uint32_t n_tokens, double *__restrict__ partial) {
-    __shared__ double s_acc[8][kDotTokens][kMixMax + 1];
+    constexpr uint32_t kMix = kHead ? kHc : kMixMax, kTiles = (kMix + 7u) / 8u;   // rows of fn, tiles of eight of them
+    __shared__ double s_acc[8][kDotTokens][kMix + 1];
     dependency_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
     const uint32_t t0 = blockIdx.x * kDotTokens, len = n / (gridDim.y * 8u);   // a multiple of 16
     const uint32_t k0 = (blockIdx.y * 8u + warp) * len + q * 4u;
     const uint32_t ta = min(t0 + g, n_tokens - 1u), tb = min(t0 + g + 8u, n_tokens - 1u);
-    double c[2][3][2] = {}, ss[2] = {0.0, 0.0};
+    double c[2][kTiles][2] = {}, ss[2] = {0.0, 0.0};
     auto load4 = [&](uint32_t t, uint32_t k, float (&v)[4]) {
         if constexpr (kBf16) {
             const uint2 w = __ldcg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(x) + (size_t)t * n + k));
@@ -269,16 +285,16 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
         float va[4], vb[4];
         load4(ta, k, va);
         load4(tb, k, vb);
-        float4 w[3];
+        float4 w[kTiles];   // (the head's four rows twice: columns 4..7 of its tile are not used)
 #pragma unroll
-        for (uint32_t m = 0; m < 3; ++m) w[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)(m * 8u + g) * n + k));
+        for (uint32_t m = 0; m < kTiles; ++m) w[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)((m * 8u + g) % kMix) * n + k));
 #pragma unroll
         for (uint32_t s = 0; s < 4; ++s) {
             const double a = va[s], b = vb[s];
             ss[0] += a * a;
             ss[1] += b * b;
 #pragma unroll
-            for (uint32_t m = 0; m < 3; ++m) {
+            for (uint32_t m = 0; m < kTiles; ++m) {
                 const double f = s == 0u ? w[m].x : (s == 1u ? w[m].y : (s == 2u ? w[m].z : w[m].w));
                 asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                              : "+d"(c[0][m][0]), "+d"(c[0][m][1])
@@ -292,46 +308,52 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
 #pragma unroll
     for (uint32_t h = 0; h < 2; ++h) {
 #pragma unroll
-        for (uint32_t m = 0; m < 3; ++m)
+        for (uint32_t m = 0; m < kTiles; ++m)
 #pragma unroll
-            for (uint32_t e = 0; e < 2; ++e) s_acc[warp][h * 8u + g][m * 8u + 2u * q + e] = c[h][m][e];
+            for (uint32_t e = 0; e < 2; ++e)
+                if (m * 8u + 2u * q + e < kMix) s_acc[warp][h * 8u + g][m * 8u + 2u * q + e] = c[h][m][e];
         ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 1);
         ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 2);
-        if (q == 0u) s_acc[warp][h * 8u + g][kMixMax] = ss[h];
+        if (q == 0u) s_acc[warp][h * 8u + g][kMix] = ss[h];
     }
     __syncthreads();
-    for (uint32_t i = tid; i < kDotTokens * (kMixMax + 1u); i += 256u) {
-        const uint32_t t = i / (kMixMax + 1u), m = i - t * (kMixMax + 1u);
+    for (uint32_t i = tid; i < kDotTokens * (kMix + 1u); i += 256u) {
+        const uint32_t t = i / (kMix + 1u), m = i - t * (kMix + 1u);
         double s = 0.0;
 #pragma unroll
         for (uint32_t w = 0; w < 8; ++w) s += s_acc[w][t][m];
-        if (t0 + t < n_tokens) partial[((size_t)blockIdx.y * n_tokens + t0 + t) * (kMixMax + 1u) + m] = s;
+        if (t0 + t < n_tokens) partial[((size_t)blockIdx.y * n_tokens + t0 + t) * (kMix + 1u) + m] = s;
     }
 }
 
 // One CTA per token: the coefficients from the partial sums (one warp), then the reduced vector.
-template <bool kBf16>
+template <bool kBf16, bool kHead, int N>
 __global__ void __launch_bounds__(256)
 k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint32_t slices, const float *__restrict__ scale,
             const float *__restrict__ base, uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced,
-            float *__restrict__ post_out, float *__restrict__ comb_out, uint32_t vec) {
-    __shared__ float s_pre[kHc], s_mix[kMixMax], s_coef[3 + kMixMax];
+            float *__restrict__ post_out, float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec) {
+    constexpr uint32_t kMix = kHead ? kHc : kMixMax;
+    __shared__ float s_pre[kHc], s_mix[kMix], s_coef[3 + kMix];
     // (k_hc_dots in front of this launch has waited: the launch behind may be set up at once)
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (warp == 0u) {
-        load_coefficients<false>(s_coef, scale, base, lane);
+        load_coefficients<kHead>(s_coef, scale, base, lane);
         double s = 0.0;
-        if (lane <= kMixMax)
-            for (uint32_t p = 0; p < slices; ++p) s += __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMixMax + 1u) + lane);
-        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMixMax) / (double)(kHc * hidden)), norm_eps);
-        if (lane < kMixMax) s_mix[lane] = __fmul_rn((float)s, rs);
+        if (lane <= kMix)
+            for (uint32_t p = 0; p < slices; ++p) s += __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMix + 1u) + lane);
+        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMix) / (double)(kHc * hidden)), norm_eps);
+        if (lane < kMix) s_mix[lane] = __fmul_rn((float)s, rs);
         __syncwarp();
-        if (lane < kHc) s_pre[lane] = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
+        if (lane < kHc) {
+            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
+            s_pre[lane] = pre;
+            if (kHead) pre_out[(size_t)t * kHc + lane] = pre;
+        }
     }
     __syncthreads();
-    if (warp == 0u) {  // the other warps reduce the streams meanwhile
+    if (!kHead && warp == 0u) {  // the other warps reduce the streams meanwhile
         float pre, post, comb;
         split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
         if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
@@ -339,62 +361,69 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
         return;
     }
     const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
-    for (uint32_t d = (threadIdx.x - 32u) * 8u; d < hidden; d += 224u * 8u) {
-        float v[8];
-        reduce_streams8<kBf16>(x, (size_t)t * kHc * hidden, hidden, d, pre, v, vec != 0u);
-        stream_st8<kBf16>(reduced, (size_t)t * hidden + d, v, vec != 0u);
+    constexpr uint32_t kFirst = kHead ? 0u : 32u;
+    for (uint32_t d = (threadIdx.x - kFirst) * N; d < hidden; d += (256u - kFirst) * N) {
+        float v[N];
+        reduce_streams<kBf16, N>(x, (size_t)t * kHc * hidden, hidden, d, pre, v, vec != 0u);
+        stream_stn<kBf16, N>(reduced, (size_t)t * hidden + d, v, vec != 0u);
     }
 }
 
-// hc.py:127-148: merged[t][o][d] = post[o] * branch[d] + sum_h comb[h][o] * residual[h][d]; eight d per thread.
-template <bool kBf16>
+// hc.py:127-148: merged[t][o][d] = post[o] * branch[d] + sum_h comb[h][o] * residual[h][d]; N d per thread.  A
+// token's twenty coefficients are the same for all its threads, so they are read through the L1; F32 values go four to a
+// thread, because the lanes' 16-byte accesses then meet in whole lines (4096, us, before these two and now: 150 tokens
+// F32 7.1 -> 3.3, 1024 28.2 -> 24.5; BF16 16 tokens 2.1 -> 1.7, 1024 10.6 -> 10.2).
+template <bool kBf16, int N>
 __global__ void __launch_bounds__(128)
 k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, const float *__restrict__ post,
           const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged, uint32_t vec) {
-    const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * 8u, t = blockIdx.y;
+    const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * N, t = blockIdx.y;
     dependency_wait();
     if (d >= hidden) return;
-    float r[kHc][8], b[8], c[kHc * kHc], p[kHc];
+    float r[kHc][N], b[N], c[kHc * kHc], p[kHc];
 #pragma unroll
     for (uint32_t h = 0; h < kHc; ++h) {
-        stream_ld8<kBf16>(residual, ((size_t)t * kHc + h) * hidden + d, r[h], vec != 0u);
-        p[h] = __ldcg(post + (size_t)t * kHc + h);
+        stream_ldn<kBf16, N>(residual, ((size_t)t * kHc + h) * hidden + d, r[h], vec != 0u);
+        p[h] = ld_f32(post + (size_t)t * kHc + h);
     }
-    stream_ld8<kBf16>(branch, (size_t)t * hidden + d, b, vec != 0u);
+    stream_ldn<kBf16, N>(branch, (size_t)t * hidden + d, b, vec != 0u);
 #pragma unroll
-    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldcg(comb + (size_t)t * kHc * kHc + i);
+    for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = ld_f32(comb + (size_t)t * kHc * kHc + i);
 #pragma unroll
     for (uint32_t o = 0; o < kHc; ++o) {
-        float v[8];
+        float v[N];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < N; ++k) {
             float s = __fmul_rn(c[o], r[0][k]);
 #pragma unroll
             for (uint32_t h = 1; h < kHc; ++h) s = __fadd_rn(s, __fmul_rn(c[h * kHc + o], r[h][k]));
             v[k] = __fadd_rn(__fmul_rn(p[o], b[k]), s);
         }
-        stream_st8<kBf16>(merged, ((size_t)t * kHc + o) * hidden + d, v, vec != 0u);
+        stream_stn<kBf16, N>(merged, ((size_t)t * kHc + o) * hidden + d, v, vec != 0u);
     }
 }
 
-// final_head.py:84-110: out = w * (x * rsqrt(mean(x^2) + eps)); one CTA per token, the token in registers
-// (eight values per thread and step; hidden <= 8192: at most four steps), so it is read once.
-template <bool kBf16>
-__global__ void __launch_bounds__(256)
+// final_head.py:84-110: out = w * (x * rsqrt(mean(x^2) + eps)); one CTA per token, N values per thread and step, kSteps
+// steps.  kHeld: the token stays in registers and is read once.  The weight is the same for all tokens and comes
+// through the L1.  All tokens read and written at once bound it, so the registers have to leave room for them: kBlocks
+// CTAs per SM (the launch's rule).
+template <bool kBf16, int N, int kSteps, int kBlocks, bool kHeld>
+__global__ void __launch_bounds__(256, kBlocks)
 k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out,
            uint32_t vec) {
     __shared__ double red[8];
     const uint32_t t = blockIdx.x;
     dependency_wait();
-    float v[4][8];
+    float v[kHeld ? kSteps : 1][N];
     double ss = 0.0;
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) {
-        const uint32_t d = (i * 256u + threadIdx.x) * 8u;
+    for (uint32_t i = 0; i < kSteps; ++i) {
+        const uint32_t d = (i * 256u + threadIdx.x) * N;
+        float(&vi)[N] = v[kHeld ? i : 0];
         if (d < hidden) {
-            stream_ld8<kBf16>(x, (size_t)t * hidden + d, v[i], vec != 0u);
+            stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec != 0u);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) ss += (double)v[i][k] * (double)v[i][k];
+            for (int k = 0; k < N; ++k) ss += (double)vi[k] * (double)vi[k];
         }
     }
     ss = warp_sum(ss);
@@ -405,14 +434,24 @@ k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hid
     for (int i = 0; i < 8; ++i) ss += red[i];
     const float rs = rsqrt_of((float)(ss / (double)hidden), eps);
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) {
-        const uint32_t d = (i * 256u + threadIdx.x) * 8u;
+    for (uint32_t i = 0; i < kSteps; ++i) {
+        const uint32_t d = (i * 256u + threadIdx.x) * N;
+        float(&vi)[N] = v[kHeld ? i : 0];
         if (d < hidden) {
-            float wv[8];
-            stream_ld8<false>(w, d, wv, vec != 0u);
+            if (!kHeld) stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec != 0u);
+            float wv[N];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) wv[k] = __fmul_rn(wv[k], __fmul_rn(v[i][k], rs));
-            stream_st8<kBf16>(out, (size_t)t * hidden + d, wv, vec != 0u);
+            for (int k = 0; k < N; k += 4) {
+                if (vec) {
+                    const float4 q = ld_f32x4(reinterpret_cast<const float4 *>(w + d + k));
+                    wv[k] = q.x, wv[k + 1] = q.y, wv[k + 2] = q.z, wv[k + 3] = q.w;
+                } else {
+                    wv[k] = ld_f32(w + d + k), wv[k + 1] = ld_f32(w + d + k + 1), wv[k + 2] = ld_f32(w + d + k + 2), wv[k + 3] = ld_f32(w + d + k + 3);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < N; ++k) wv[k] = __fmul_rn(wv[k], __fmul_rn(vi[k], rs));
+            stream_stn<kBf16, N>(out, (size_t)t * hidden + d, wv, vec != 0u);
         }
     }
 }
@@ -491,7 +530,11 @@ cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y,
                       merged);
 }
 
-size_t hc_scratch_bytes(uint32_t max_tokens) { return (size_t)(std::max(8u * max_tokens, 8192u)) * (kMixMax + 1u) * sizeof(double); }
+// (partial sums of launch_hc_pre_many: eight slices of K for any number of tokens, or fewer than 2 * sm_count groups of
+// sixteen tokens times slices)
+size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count) {
+    return (size_t)std::max(8u * max_tokens, 32u * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
+}
 
 // Whether all the addresses are multiples of 16 (rows of 256 and more elements keep that).
 template <class... P>
@@ -512,61 +555,114 @@ static cudaError_t allow_wide_clusters(Kernel kernel, bool (&done)[64]) {
     return e;
 }
 
-template <bool kBf16, bool kHead>
+template <bool kBf16, bool kHead, uint32_t kCluster>
 static cudaError_t launch_hc_pre_cluster(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                          const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
                                          void *reduced, float *post, float *comb, float *pre) {
     static bool done[64] = {};
-    const cudaError_t e = allow_wide_clusters(k_hc_pre<kBf16, kHead>, done);
+    const cudaError_t e = allow_wide_clusters(k_hc_pre<kBf16, kHead, kCluster>, done);
     if (e != cudaSuccess) return e;
-    return launch_pdl(k_hc_pre<kBf16, kHead>, dim3(kPreCluster, n_tokens), dim3(kPreThreads), 0, st, kPreCluster, x, fn, scale, base,
+    return launch_pdl(k_hc_pre<kBf16, kHead, kCluster>, dim3(kCluster, n_tokens), dim3(kPreThreads), 0, st, kCluster, x, fn, scale, base,
                       hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced));
 }
 
-template <bool kBf16>
-static cudaError_t launch_hc_pre_many(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
+template <bool kBf16, bool kHead>
+static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                       const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
-                                      double *partial, void *reduced, float *post, float *comb) {
+                                      double *partial, void *reduced, float *post, float *comb, float *pre) {
     // slices of K: enough CTAs for the SMs, each warp's part whole steps of sixteen (n / 1024 is a whole number)
     const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden;
     uint32_t slices = 8u;
-    while (slices < 64u && groups * slices < 148u && (n / (slices * 2u * 8u)) % 16u == 0u) slices *= 2u;
-    const cudaError_t e = launch_pdl(k_hc_dots<kBf16>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
+    while (slices < 64u && groups * slices < (uint32_t)sm_count && (n / (slices * 2u * 8u)) % 16u == 0u) slices *= 2u;
+    const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
-    return launch_pdl(k_hc_reduce<kBf16>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,
-                      norm_eps, iters, hc_eps, reduced, post, comb, aligned16(x, reduced));
+    return launch_pdl(k_hc_reduce<kBf16, kHead, kBf16 ? 8 : 4>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,
+                      norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced));
 }
 
 // scratch: hc_scratch_bytes of the most tokens.  Returns the number of kernels launched.
-int launch_hc_pre(cudaStream_t st, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
+int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                   const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
                   float *post, float *comb, float *pre, cudaError_t *err) {
-    // up to eight tokens the clusters fit the GPU side by side; the head's reduce (four rows) has no other form
-    if (head || n_tokens <= 8u) {
-        if (bf16 && head) *err = launch_hc_pre_cluster<true, true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-        else if (bf16) *err = launch_hc_pre_cluster<true, false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-        else if (head) *err = launch_hc_pre_cluster<false, true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-        else *err = launch_hc_pre_cluster<false, false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
-        return 1;
+    // one cluster per token while the clusters fit the GPU side by side, else two launches for all tokens
+    auto run = [&](auto is_bf16, auto is_head, auto size) {
+        constexpr bool kB = decltype(is_bf16)::value, kH = decltype(is_head)::value;
+        constexpr uint32_t kC = decltype(size)::value;
+        if constexpr (kC != 0u) {
+            *err = launch_hc_pre_cluster<kB, kH, kC>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+            return 1;
+        } else {
+            *err = launch_hc_pre_many<kB, kH>(st, sm_count, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced,
+                                              post, comb, pre);
+            return 2;
+        }
+    };
+    auto of_size = [&](auto is_head, auto size) { return bf16 ? run(std::true_type{}, is_head, size) : run(std::false_type{}, is_head, size); };
+    using U = uint32_t;
+    const uint32_t sms = (uint32_t)sm_count;
+    if (!head) {
+        // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together, or fourteen of eight (4096, us:
+        // seven tokens 8.6, eight 9.6, fourteen 9.8; clusters of sixteen 14.4 and 14.8; the two launches 11.2, 10.7, 11.4).
+        if (16u * n_tokens * 5u <= sms * 4u) return of_size(std::false_type{}, std::integral_constant<U, 16>{});
+        if (8u * n_tokens * 5u <= sms * 4u) return of_size(std::false_type{}, std::integral_constant<U, 8>{});
+        return of_size(std::false_type{}, std::integral_constant<U, 0>{});
     }
-    *err = bf16 ? launch_hc_pre_many<true>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced, post, comb)
-                : launch_hc_pre_many<false>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced, post, comb);
-    return 2;
+    // The head's four rows leave room for two CTAs, and smaller clusters pack closer: the largest whose CTAs come to at most
+    // one and a half per SM (4096, us: 8 tokens 4.1, 16 4.4, 32 5.2, 64 6.8; one cluster of sixteen for any number 4.1, 8.0,
+    // 12.3, 20.7, the two launches 8.9, 9.5, 9.8, 10.8 and from about 70 tokens on the least: 300 12.9, 1024 26.5).
+    const uint32_t room = sms + sms / 2u;
+    if (16u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 16>{});
+    if (8u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 8>{});
+    if (4u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 4>{});
+    if (2u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 2>{});
+    return of_size(std::true_type{}, std::integral_constant<U, 0>{});
 }
 
-cudaError_t launch_hc_post(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
+cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged) {
-    const dim3 grid((hidden + 1023u) / 1024u, n_tokens);
     const uint32_t vec = aligned16(branch, residual, merged);
-    if (bf16) return launch_pdl(k_hc_post<true>, grid, dim3(128), 0, st, 0u, branch, residual, post, comb, hidden, merged, vec);
-    return launch_pdl(k_hc_post<false>, grid, dim3(128), 0, st, 0u, branch, residual, post, comb, hidden, merged, vec);
+    // BF16: four values a thread (8-byte accesses) while their CTAs come to at most five per SM (one token of 4096 1.4 us, eight
+    // values 1.6; 64 tokens 1.9 and 2.0), above that eight (1024 tokens 10.2 us, four values 11.9)
+    const bool few = (uint64_t)n_tokens * hidden <= (uint64_t)sm_count * 5u * 512u;
+    auto run = [&](auto kernel, uint32_t per_thread) {
+        return launch_pdl(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, branch,
+                          residual, post, comb, hidden, merged, vec);
+    };
+    if (!bf16) return run(k_hc_post<false, 4>, 4);
+    return few ? run(k_hc_post<true, 4>, 4) : run(k_hc_post<true, 8>, 8);
 }
 
-cudaError_t launch_rms_norm(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
-                            void *out) {
-    const uint32_t vec = aligned16(x, w, out);
-    if (bf16) return launch_pdl(k_rms_norm<true>, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec);
-    return launch_pdl(k_rms_norm<false>, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec);
+// F32 tokens: eight values per thread while a token has an SM to itself (the fewest steps in series), else four, whose
+// 16-byte accesses meet in whole lines, with registers for as many CTAs per SM as there are tokens; above 4096 the
+// largest batches would spill and read the token twice.  us of 4096, one form for all / now: 16 tokens 2.7 / 2.6,
+// 300 5.2 / 3.6, 700 7.8 / 4.9, 1024 9.5 / 6.7; 8192 and 1024 tokens 16.4 / 12.0.  BF16 tokens are half the bytes, eight
+// values to a thread always: 4096 and 700 tokens 5.8 / 3.7.
+template <bool kBf16, int kSteps>
+static cudaError_t launch_rms_steps(cudaStream_t st, uint32_t sms, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
+                                    void *out, uint32_t vec) {
+    auto run = [&](auto kernel) { return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec); };
+    if (kBf16 || n_tokens <= sms) return run(k_rms_norm<kBf16, 8, kSteps, 1, true>);
+    if constexpr (!kBf16) {
+        constexpr int kFour = 2 * kSteps;   // steps of four values
+        if (kSteps == 1 && hidden <= 1024u) return run(k_rms_norm<false, 4, 1, 8, true>);
+        if (n_tokens <= 4u * sms) return run(k_rms_norm<false, 4, kFour, 1, true>);
+        if (n_tokens <= 6u * sms) return run(k_rms_norm<false, 4, kFour, 6, true>);
+        return run(k_rms_norm<false, 4, kFour, 8, (kFour < 8)>);
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w,
+                            float eps, void *out) {
+    const uint32_t vec = aligned16(x, w, out), sms = (uint32_t)sm_count;
+    auto run = [&](auto steps) {
+        constexpr int kS = decltype(steps)::value;
+        return bf16 ? launch_rms_steps<true, kS>(st, sms, n_tokens, hidden, x, w, eps, out, vec)
+                    : launch_rms_steps<false, kS>(st, sms, n_tokens, hidden, x, w, eps, out, vec);
+    };
+    if (hidden <= 2048u) return run(std::integral_constant<int, 1>{});
+    if (hidden <= 4096u) return run(std::integral_constant<int, 2>{});
+    return run(std::integral_constant<int, 4>{});
 }
 
 cudaError_t launch_router_hash(cudaStream_t st, const s14_router_desc &r, const int64_t *tid2eid) {

@@ -244,13 +244,13 @@ int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores
 
 // ---- the steps on either side of the MoE inside one layer (s14_glue.cu) ----
 // scratch: hc_scratch_bytes(the most tokens of a call).  Returns the number of kernels launched.
-size_t hc_scratch_bytes(uint32_t max_tokens);
-int launch_hc_pre(cudaStream_t st, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
+size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count);
+int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                   const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
                   float *post, float *comb, float *pre, cudaError_t *err);
-cudaError_t launch_hc_post(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
+cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged);
-cudaError_t launch_rms_norm(cudaStream_t st, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
+cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
                             void *out);
 cudaError_t launch_router_hash(cudaStream_t st, const s14_router_desc &r, const int64_t *tid2eid);
 cudaError_t launch_bf16_to_f32(cudaStream_t st, const uint16_t *in, float *out, uint32_t n);
