@@ -293,8 +293,12 @@ k_fp8_matvec_pairwise(const float *__restrict__ x, const uint8_t *__restrict__ w
 // A dependent launch: the first weights are brought to the L2 before the wait for the kernel in front, the next ones are
 // asked for while a piece is worked on (us a call in a queue of calls, before and after: 1024 x 4096 x 8 tokens 12.3 ->
 // 9.8, 4700 x 640 x 8 14.4 -> 11.4, 700 x 8192 x 5 14.4 -> 11.5; one token of 1024 x 4096 7.8 -> 3.1, half of it host time).
+// One token, more CTAs than SMs and long rows: a dependent launch's CTAs fill the slots that the launch in front leaves
+// and pile up on some SMs (2048 x 8192 one after the other: 9.7 us, an ordinary launch 7.2; 2048 x 4096 4.8 and 3.9;
+// short rows gain from it, 4096 x 1024 3.2 and 3.9), and with many CTAs per SM the piece ahead (kAhead) costs more
+// registers than it hides (4096 x 8192: 14.4 us, without 12.1).
 constexpr uint32_t kFp8BlockRows = 8, kFp8BlockThreads = 512;
-template <int NT, bool F32_SCALE>
+template <int NT, bool F32_SCALE, bool kAhead>
 __global__ void __launch_bounds__(kFp8BlockThreads)
 k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, const void *__restrict__ scale,
                    float *__restrict__ y, uint32_t n_rows, uint32_t k) {
@@ -310,7 +314,7 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
     uint4 ahead = make_uint4(0u, 0u, 0u, 0u);
     if (n < n_rows && lane < per) l2_hint(wrow + half * per + lane);
     dependency_wait();
-    if (n < n_rows && lane < per) ahead = ld_stream(wrow + half * per + lane);
+    if (kAhead && n < n_rows && lane < per) ahead = ld_stream(wrow + half * per + lane);
     for (uint32_t i = threadIdx.x; i < (NT * k) >> 2; i += kFp8BlockThreads) {
         const uint32_t t = i / (k >> 2), j = i % (k >> 2);
         reinterpret_cast<float4 *>(sx)[(size_t)t * (k >> 2) + (j & 3u) * pieces + (j >> 2)] =
@@ -324,8 +328,8 @@ k_fp8_matvec_block(const float *__restrict__ x, const uint8_t *__restrict__ w, c
     if (n < n_rows) {
         const size_t srow = (size_t)(n >> 7) * k_groups;
         for (uint32_t p = half * per + lane; p < (half + 1u) * per; p += 32u) {
-            const uint4 q = ahead;
-            if (p + 32u < (half + 1u) * per) ahead = ld_stream(wrow + p + 32u);
+            const uint4 q = kAhead ? ahead : ld_stream(wrow + p);
+            if (kAhead && p + 32u < (half + 1u) * per) ahead = ld_stream(wrow + p + 32u);
             const double sc = fp8_block_scale_f64<F32_SCALE>(scale, srow + (p >> 3));
             const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
             float2 wf[8];
@@ -976,13 +980,13 @@ cudaError_t launch_mxfp4_matvec(cudaStream_t st, uint32_t mode, int sm_count, co
 }
 
 // Largest dynamic shared memory k_fp8_matvec_block may ask for on the current device (0: not set).
-template <int NT, bool F32S>
+template <int NT, bool F32S, bool kAhead>
 static bool fp8_block_smem_ok(size_t bytes) {
     static int configured[64] = {};
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     if (!configured[dev]) {
-        configured[dev] = cudaFuncSetAttribute(k_fp8_matvec_block<NT, F32S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        configured[dev] = cudaFuncSetAttribute(k_fp8_matvec_block<NT, F32S, kAhead>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                160 * 1024) == cudaSuccess ? 1 : -1;
     }
     return configured[dev] == 1 && bytes <= 160u * 1024u;
@@ -996,9 +1000,19 @@ static bool try_fp8_block(cudaStream_t st, int sm_count, const float *x, const u
     // blocks, 16-byte aligned operands, the tokens' activations fit shared memory
     const size_t bytes = (size_t)NT * k * sizeof(float);
     if (n > (uint32_t)sm_count * 32u || (k & 31u) || ((uintptr_t)w & 15u) || ((uintptr_t)x & 15u)) return false;
-    if (!fp8_block_smem_ok<NT, F32S>(bytes)) return false;
-    *err = launch_pdl(k_fp8_matvec_block<NT, F32S>, dim3((n + kFp8BlockRows - 1) / kFp8BlockRows), dim3(kFp8BlockThreads), bytes, st, 0u,
-                      x, w, s, y, n, k);
+    const dim3 grid((n + kFp8BlockRows - 1) / kFp8BlockRows), block(kFp8BlockThreads);
+    if constexpr (NT == 1) {
+        if (grid.x > (uint32_t)sm_count && k >= 4096u) {
+            const bool ahead = grid.x <= 2u * (uint32_t)sm_count;
+            if (!(ahead ? fp8_block_smem_ok<NT, F32S, true>(bytes) : fp8_block_smem_ok<NT, F32S, false>(bytes))) return false;
+            if (ahead) k_fp8_matvec_block<NT, F32S, true><<<grid, block, bytes, st>>>(x, w, s, y, n, k);
+            else k_fp8_matvec_block<NT, F32S, false><<<grid, block, bytes, st>>>(x, w, s, y, n, k);
+            *err = cudaGetLastError();
+            return true;
+        }
+    }
+    if (!fp8_block_smem_ok<NT, F32S, true>(bytes)) return false;
+    *err = launch_pdl(k_fp8_matvec_block<NT, F32S, true>, grid, block, bytes, st, 0u, x, w, s, y, n, k);
     return true;
 }
 
