@@ -18,16 +18,18 @@ namespace {
 // (1.06 GB / 6.55 TB/s = 162 us), so what a weight element costs on the SM has to stay below 1.5 clocks per
 // 12 elements.  A register kernel does not manage that for eight tokens: it reads 32 bytes of x per weight
 // element through the L1 and converts a partial sum to double per 4 products (16 conversions per clock and
-// SM), 1118 us.  Here x is split once per CTA into three BF16 parts (x = h + m + l exactly: 6, 8 and 8
-// significant bits, each remainder's sign being worth one more) kept in shared memory, and a warp takes
+// SM), 1118 us.  Here x is split once per CTA into three BF16 parts (x = h + m + l: 6, 8 and 8
+// significant bits, each remainder's sign being worth one more; exact for |x| from 2^-110, below which m and l run out
+// of BF16's exponents, to where h may still be rounded up, 2^127) kept in shared memory, and a warp takes
 // sixteen rows of W as the A operand of mma.m16n8k16, the eight tokens' parts as B: every product is exact in
-// F32.  The sums of sixteen products with h (14-bit products: few of their bits fall off the F32 sum) go to
-// double every 16 elements of K; m and l, 2^-6 and 2^-15 of h, are summed in F32 over 128 elements and then
-// added (blocks of K that do not depend on the number of tokens).  Measured error (N(0,1) x N(0,0.02), K = 4096):
-// 3.9e-8 RMS, the register kernel's 4-product chains 6.0e-8.
+// F32.  The sums of sixteen products with h (few of their bits fall off the F32 sum) go to double every 16 elements of K;
+// m and l, 2^-6 (2^-3 for BF16 values) and 2^-15 of h, are summed in F32 over 128 elements and then added (blocks of K
+// that do not depend on the number of tokens).  Measured RMS error over the RMS result, N(0,1) x N(0,0.02), K = 4096
+// (2048 the same within 2 %), rounding the result alone 2.54e-8: F32 x 2.94e-8, the register kernel's 4-product chains
+// 4.75e-8; BF16 values 2.62e-8 and 2.65e-8 (with six bits in h 2.95e-8, four 2.68e-8).
 // A lane loads 16 bytes (eight k) of each of its two rows: words 0, 1 are its k slots of a first MMA, words 2, 3
 // of a second one, and x is read from shared memory in the same order, so K is only permuted.  Two warps share
-// sixteen rows (the halves of K): 8080 row tiles over 148 x 8 pairs leave the last round 97 % full.  Eight
+// sixteen rows (the halves of K): 8080 row tiles over 148 x 8 pairs are 6.8 rounds, the last one 82 % full.  Eight
 // 16-byte loads per lane are in flight (64 KB per SM), across row tiles; they need room in the L1, which shared
 // memory takes away (with eight tokens' 198 KB of parts resident: 290 us).  So K is walked in `phases` of at
 // most 50 KB of parts, the CTA's row tiles once per phase, their sums waiting in shared memory in between.
@@ -43,11 +45,15 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// The BF16 parts of v: 6 significant bits, then 8, then the 8 that are left (nearest each time, so a remainder
-// is at most half a unit of the part before).  Infinities and NaNs go into the first alone.
+// The BF16 parts of v: 6 significant bits, then 8, then the 8 that are left (nearest each time, so a remainder is at most
+// half a unit of the part before).  A BF16 value, which two parts hold in any case, gives the first one
+// three: the sums of its products lose less on their way into double.  Infinities and NaNs go into the first alone.
 __device__ __forceinline__ void head_parts(float v, uint32_t (&p)[3]) {
-    uint32_t h = (__float_as_uint(v) + 0x00020000u) & 0xfffc0000u;
-    if ((h & 0x7f800000u) == 0x7f800000u && isfinite(v)) h = __float_as_uint(v) & 0xfffc0000u;  // would round to infinity
+    const uint32_t u = __float_as_uint(v);
+    const bool bf16 = (u & 0xffffu) == 0u;
+    const uint32_t keep = bf16 ? 0xffe00000u : 0xfffc0000u;
+    uint32_t h = (u + (bf16 ? 0x00100000u : 0x00020000u)) & keep;
+    if ((h & 0x7f800000u) == 0x7f800000u && isfinite(v)) h = u & keep;  // would round to infinity
     if (!isfinite(v)) {
         const __nv_bfloat16 b = __float2bfloat16_rn(v);
         p[0] = *reinterpret_cast<const uint16_t *>(&b);
@@ -457,7 +463,10 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
                                uint32_t hidden, float *out, uint32_t out_stride) {
     // the tensor-core kernel: phases of K in whole groups of steps per half row, as few as keep the parts small;
     // sizes that have none take the register kernel
-    for (uint32_t phases = 1; phases <= 8u; phases *= 2u) {
+    // (and so do few rows: a tile of sixteen is one pair of warps that walks K, and most SMs have none or one.  us, tensor-core /
+    // register kernel: 1000 x 512 one token 2.8 / 1.8, 4000 x 4096 one token 19.7 / 8.1, 1000 x 2048 four tokens 8.5 / 4.9)
+    const bool few_rows = (uint64_t)n_rows * n_tokens <= 4096u && n_tokens <= 6u;
+    for (uint32_t phases = 1; phases <= 8u && !few_rows; phases *= 2u) {
         const size_t parts = 3u * (size_t)n_tokens * (hidden / phases * 2u + kHeadPad);
         const size_t smem = parts + (phases > 1u ? kHeadTiles * 1024u : 0u);
         if (hidden % (256u * phases) != 0u || smem > head_smem_limit()) continue;

@@ -19,11 +19,12 @@ def ctx():
     c.close()
 
 
-# rows: less than a tile, tiles with a remainder, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in
-# phases); hidden: one group of steps, several phases, sizes the tensor-core kernel leaves to the other one (264; 1048:
-# more than its four pieces per lane)
-@pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (2, 17, 1280), (3, 2385, 4096), (5, 33, 264), (3, 300, 1048),
-                                                (8, 300, 1048), (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096)])
+# rows: less than a tile (eight tokens; fewer take the register kernel), tiles with a remainder, the last of the register kernel
+# and the first of the other, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in phases); hidden: one group of
+# steps, several phases, sizes the tensor-core kernel leaves to the other one (264; 1048: more than its four pieces per lane)
+@pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (7, 17, 1280), (3, 2385, 4096), (5, 33, 264), (3, 300, 1048),
+                                                (8, 300, 1048), (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096),
+                                                (1, 4096, 512), (1, 4097, 768), (2, 2048, 256), (4, 1025, 1024), (6, 683, 256)])
 def test_logits_at_the_edges_of_the_tiles(ctx, tokens, rows, hidden):
     g = torch.Generator(device="cuda").manual_seed(tokens * rows + hidden)
     x = torch.randn(tokens, hidden, device="cuda", generator=g)
@@ -39,27 +40,45 @@ def test_logits_at_the_edges_of_the_tiles(ctx, tokens, rows, hidden):
     assert bool((out[:, rows:] == 7.0).all())
 
 
-def test_logits_of_infinite_and_largest_values(ctx):
+@pytest.mark.parametrize("rows", [40, 2100])
+def test_logits_of_infinite_and_largest_values(ctx, rows):
     x = torch.zeros(2, 512, device="cuda")
     x[0, 5], x[1, 300] = float("inf"), 3.4028e38
-    w = torch.ones(40, 512, dtype=torch.bfloat16, device="cuda") * 0.5
-    out = torch.empty(2, 40, device="cuda")
+    w = torch.ones(rows, 512, dtype=torch.bfloat16, device="cuda") * 0.5
+    out = torch.empty(2, rows, device="cuda")
     ctx.cmd_head_logits(x, w.view(torch.int16), out)
     assert bool((out[0] == float("inf")).all())
     assert bool((out[1] == x[1, 300] * 0.5).all())
 
 
-# 264: the size that the register kernel takes alone; 4096 with eight tokens: several phases of K
-@pytest.mark.parametrize("tokens,hidden", [(1, 256), (1, 264), (3, 512), (8, 4096)])
-def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden):
+@pytest.mark.parametrize("bf16", [False, True])
+def test_logits_are_as_close_as_sums_of_eight_products(ctx, bf16):
+    """What the sums add to the error of rounding the result, root mean square over that of the results: no more than sums of
+    eight products in F32 do, measured with the register kernel at N(0,1) x N(0,0.02) over 4096 (4.02e-8 for F32 x; 7.5e-9 for
+    BF16 values, whose products are exact)."""
+    g = torch.Generator(device="cuda").manual_seed(17)
+    x = torch.randn(8, 4096, device="cuda", generator=g)
+    x = x.to(torch.bfloat16).float() if bf16 else x
+    w = torch.empty(20000, 4096, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g)
+    for tokens in (1, 8):
+        out = torch.empty(tokens, 20000, device="cuda")
+        ctx.cmd_head_logits(x[:tokens], w.view(torch.int16), out)
+        ref = x[:tokens].double() @ w.double().T
+        added = (out.double() - ref).pow(2).mean() - (ref.float().double() - ref).pow(2).mean()
+        assert float((added.clamp(min=0) / ref.pow(2).mean()).sqrt()) <= (7.5e-9 if bf16 else 4.02e-8)
+
+
+# 264 and few rows times tokens: the register kernel; 4096 with eight tokens: several phases of K
+@pytest.mark.parametrize("tokens,hidden,rows", [(1, 256, 4100), (1, 264, 70), (1, 512, 70), (3, 512, 1400), (8, 4096, 70)])
+def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden, rows):
     """One infinite weight gives an infinite logit of its sign (x is finite and nowhere 0), both signs or a NaN give NaN,
     and a product or sum beyond the largest float is infinite; the rows beside them are the ordinary ones."""
     g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
     inf = float("inf")
     x = (torch.rand(tokens, hidden, device="cuda", generator=g) + 0.5).to(torch.bfloat16).float()  # the last part is 0
     x[-1] *= 1.0 + 2.0 ** -20                                                                       # ... or is not
-    w = torch.empty(70, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g)
-    out, plain = torch.empty(tokens, 70, device="cuda"), torch.empty(tokens, 70, device="cuda")
+    w = torch.empty(rows, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g)
+    out, plain = torch.empty(tokens, rows, device="cuda"), torch.empty(tokens, rows, device="cuda")
     ctx.cmd_head_logits(x, w.view(torch.int16), plain)
     w[3, 7], w[20, hidden - 1], w[33, 0], w[33, hidden // 2], w[41, 9], w[69, 8] = inf, -inf, inf, -inf, float("nan"), 3.3e38
     w[50, ::2] = -2.0 ** 127
@@ -67,7 +86,7 @@ def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden
     ctx.cmd_head_logits(x, w.view(torch.int16), out)
     assert bool((out[:, 3] == inf).all()) and bool((out[:, 20] == -inf).all()) and bool((out[:, 50] == -inf).all())
     assert bool(out[:, [33, 41]].isnan().all()) and float(out[0, 69]) == inf
-    others = [r for r in range(70) if r not in (3, 20, 33, 41, 50, 69)]
+    others = [r for r in range(rows) if r not in (3, 20, 33, 41, 50, 69)]
     assert torch.equal(out[1:, others], plain[1:, others]) and bool(out[:, others].isfinite().all())
     # the greedy token is the row with the positive infinity (without the NaN rows)
     out[:, [33, 41]] = 0.0
