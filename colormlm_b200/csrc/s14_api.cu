@@ -975,9 +975,9 @@ extern "C" int32_t s14_cmd_stack_decode(s14_ctx *ctx, void *stream, s14_stack *s
     }
     const float *cur = x;
     // the layers one by one: router and layer kernels into ybuf, then the step to the next token.  With FP8 shared
-    // experts every expert stays on the F32 register kernels: the tensor-core kernel's sums differ from theirs by
-    // 4e-7 of a layer's output, which the chain of layers amplifies (to 8e-5 after a few), and a decode step's
-    // results are to stay what they are.
+    // experts every expert stays on the F32 register kernels.  A layer called by itself runs its routed experts on the
+    // tensor cores, whose exact sums differ from these by 4e-7 of a layer's output; a chain of layers amplifies that (to
+    // 8e-5 after a few), more than a stack's results are allowed to move.
     const bool fp8_shared = has_shared && c.shared_kind == S14_PAGE_FP8;
     for (uint32_t l = 0; l < c.n_layers; ++l) {
         const FusedRouter fr = stack_router(ctx, stack, l);

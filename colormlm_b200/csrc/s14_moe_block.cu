@@ -36,7 +36,7 @@
 // bulk copies).  A large block takes TWO slices or row tiles per item: the token tiles of a K range are fetched once
 // for two units.  What bounds large blocks is the issue of the tcgen05 operations and the accumulator reads between two
 // items, not the copies (370 tokens, up kernel 612 us: 602 without the pages' copies, 594 without the tiles', 419
-// without the MMAs, 536 without the reads; the call 1076 -> 942-990 us since the issuing
+// without the MMAs, 536 without the reads; the call 1096 -> 987 us since the issuing
 // loops are run by whole warps with one elected lane).
 // With the official expert arithmetic
 // (fast16/research/polaris_meridian_v1/s14_first_real_token/executor.py:712-743) the same contractions run on

@@ -58,7 +58,9 @@ extern "C" {
  *                         row: the result is the reference's dot product with the accumulator
  *                         widened to double (what the reference's Python code computes with
  *                         accumulation_dtype=float64, local_s14_primitives/mxfp4.py:172-275).
- *                         One-token layers of MXFP4 pages run on the tensor cores (activations
+ *                         One-token layers of MXFP4 pages, and the routed experts of a layer
+ *                         called by itself whose shared page is FP8 (not those of a stack:
+ *                         the two agree to about 4e-7), run on the tensor cores (activations
  *                         as sixteen base-8 digit rows, tcgen05 block-scaled MMA, columns added
  *                         in double); everything else on F32 / F64 register kernels (a warp per
  *                         row, F32 inside a scale block, F64 across blocks and lanes).
