@@ -67,6 +67,33 @@ __device__ __forceinline__ void head_parts(float v, uint32_t (&p)[3]) {
     p[2] = *reinterpret_cast<const uint16_t *>(&l);
 }
 
+// Sixteen rows times the tokens over 128 elements of K, as one warp takes them: four steps of 32.  A row's logit is these
+// sums added in the order of K within each half of a phase, the halves added, the phases added: whichever
+// kernel and shard works the row out, the bits are the same.
+struct HeadBlock {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    float low[4] = {0.f, 0.f, 0.f, 0.f}, c[2][4];
+    __device__ __forceinline__ void step(const uint4 &a0, const uint4 &a1, const uint4 (&b)[3]) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[0][e] = c[1][e] = 0.f;
+        mma_bf16(c[0], a0.x, a1.x, a0.y, a1.y, b[0].x, b[0].y);
+        mma_bf16(c[1], a0.z, a1.z, a0.w, a1.w, b[0].z, b[0].w);
+#pragma unroll
+        for (int part = 2; part >= 1; --part) {
+            mma_bf16(low, a0.x, a1.x, a0.y, a1.y, b[part].x, b[part].y);
+            mma_bf16(low, a0.z, a1.z, a0.w, a1.w, b[part].z, b[part].w);
+        }
+    }
+    __device__ __forceinline__ void carry() {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            acc[e] += (double)c[0][e];
+            acc[e] += (double)c[1][e];
+        }
+    }
+    __device__ __forceinline__ double sum(int e) const { return acc[e] + (double)low[e]; }
+};
+
 // One row's dot product by a whole warp as k_head_logits takes it, for the sums that the parts get wrong: an infinite
 // weight times a part that is zero is NaN, two parts of opposite sign make inf - inf of it, and a product near the
 // largest float overflows in two parts at once.  Out of line: its callers are never there with ordinary numbers, and
@@ -157,32 +184,21 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
                     const bool last = s0 + kHeadDepth == steps;
                     if (last && more) rows_of(next, next_phase);
                     const uint32_t k_next = last ? 0u : s0 + kHeadDepth;
-                    float low[4] = {0.f, 0.f, 0.f, 0.f};
+                    HeadBlock blk;
 #pragma unroll
                     for (uint32_t j = 0; j < kHeadDepth; ++j) {
-                        float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
                         uint4 b[3];
 #pragma unroll
                         for (uint32_t part = 0; part < 3; ++part) {
                             b[part] = make_uint4(0u, 0u, 0u, 0u);
                             if (has_b) b[part] = *reinterpret_cast<const uint4 *>(sb + part * part_bytes + (s0 + j) * 64u);
                         }
-                        mma_bf16(c[0], a0[j].x, a1[j].x, a0[j].y, a1[j].y, b[0].x, b[0].y);
-                        mma_bf16(c[1], a0[j].z, a1[j].z, a0[j].w, a1[j].w, b[0].z, b[0].w);
-#pragma unroll
-                        for (int part = 2; part >= 1; --part) {
-                            mma_bf16(low, a0[j].x, a1[j].x, a0[j].y, a1[j].y, b[part].x, b[part].y);
-                            mma_bf16(low, a0[j].z, a1[j].z, a0[j].w, a1[j].w, b[part].z, b[part].w);
-                        }
+                        blk.step(a0[j], a1[j], b);
                         if (!last || more) fetch(j, k_next);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            acc[e] += (double)c[0][e];
-                            acc[e] += (double)c[1][e];
-                        }
+                        blk.carry();
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[e] += (double)low[e];
+                    for (int e = 0; e < 4; ++e) acc[e] += blk.sum(e);
                 }
                 if (half == 1u) {
 #pragma unroll
@@ -216,6 +232,112 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
                 }
             }
         }
+    }
+}
+
+// The same logits where there are fewer row tiles than the pairs of warps above: a CTA takes one tile, its warps the blocks
+// of 128 k in turn, their sums wait in shared memory and are added in k_head_mma's order (the same bits: a
+// vocabulary shard may be small where another is not).  There a pair walks all of K for its tile, here K is spread over
+// eight warps.  kShared (up to four tokens): x is split into its parts once per CTA; more tokens' parts do not fit beside a
+// second CTA, and every warp makes those of its blocks in the registers of the lanes that use them, which costs the
+// same for one token as for eight.  us, with the parts shared / in registers / by the register kernel below, which sums in
+// another order: 4000 x 4096 one token 12.6 / 20.2 / 9.0, eight - / 21.0 / 29.6; 1000 x 512 one token 2.5 / 3.4 / 1.8.
+constexpr uint32_t kFewThreads = 256;
+template <bool kShared>
+__global__ void __launch_bounds__(kFewThreads, 2)
+k_head_mma_few(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
+               uint32_t out_stride, uint32_t n_tokens, uint32_t phases) {
+    extern __shared__ __align__(16) uint8_t s_few[];         // [K / 128][4][32] sums of the blocks, then the parts [3][n_tokens][pitch]
+    double *const s_blk = reinterpret_cast<double *>(s_few);
+    uint8_t *const s_x = s_few + (size_t)hidden * 8u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
+    const uint32_t n_blk = hidden >> 7, row0 = blockIdx.x * 16u, pitch = hidden * 2u + kHeadPad;
+    const uint16_t *const p0 = w + (size_t)min(row0 + g, n_rows - 1u) * hidden + q * 8u;
+    const uint16_t *const p1 = w + (size_t)min(row0 + g + 8u, n_rows - 1u) * hidden + q * 8u;
+    const bool has_b = g < n_tokens;
+    const float *const xg = x + (size_t)(has_b ? g : 0u) * hidden + q * 8u;
+    uint4 a0[kHeadDepth], a1[kHeadDepth];
+    auto fetch = [&](uint32_t b) {
+#pragma unroll
+        for (uint32_t j = 0; j < kHeadDepth; ++j) {
+            a0[j] = ld_stream(reinterpret_cast<const uint4 *>(p0 + b * 128u + j * 32u));
+            a1[j] = ld_stream(reinterpret_cast<const uint4 *>(p1 + b * 128u + j * 32u));
+        }
+    };
+    dependency_wait();
+    if (warp < n_blk) fetch(warp);   // in flight while x is split
+    auto parts_of = [](const float4 &lo, const float4 &hi, uint4 (&bp)[3]) {
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        uint32_t wd[3][4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            uint32_t px[3], py[3];
+            head_parts(v[2 * i], px);
+            head_parts(v[2 * i + 1], py);
+#pragma unroll
+            for (uint32_t part = 0; part < 3; ++part) wd[part][i] = px[part] | (py[part] << 16);
+        }
+#pragma unroll
+        for (uint32_t part = 0; part < 3; ++part) bp[part] = make_uint4(wd[part][0], wd[part][1], wd[part][2], wd[part][3]);
+    };
+    if constexpr (kShared) {
+        for (uint32_t i = tid; i < n_tokens * (hidden >> 3); i += kFewThreads) {
+            const uint32_t t = i / (hidden >> 3), k8 = i - t * (hidden >> 3);
+            const float4 *at = reinterpret_cast<const float4 *>(x + (size_t)t * hidden) + 2u * k8;
+            uint4 bp[3];
+            parts_of(__ldcg(at), __ldcg(at + 1), bp);
+#pragma unroll
+            for (uint32_t part = 0; part < 3; ++part) *reinterpret_cast<uint4 *>(s_x + (part * n_tokens + t) * pitch + k8 * 16u) = bp[part];
+        }
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (uint32_t b = warp; b < n_blk; b += kFewThreads / 32u) {
+        if (b != warp) fetch(b);
+        HeadBlock blk;
+#pragma unroll
+        for (uint32_t j = 0; j < kHeadDepth; ++j) {
+            uint4 bp[3] = {};
+            if (has_b) {
+                if constexpr (kShared) {
+#pragma unroll
+                    for (uint32_t part = 0; part < 3; ++part)
+                        bp[part] = *reinterpret_cast<const uint4 *>(s_x + (part * n_tokens + g) * pitch + b * 256u + j * 64u + q * 16u);
+                } else {
+                    const float4 *at = reinterpret_cast<const float4 *>(xg + b * 128u + j * 32u);
+                    parts_of(__ldcg(at), __ldcg(at + 1), bp);
+                }
+            }
+            blk.step(a0[j], a1[j], bp);
+            blk.carry();
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s_blk[(b * 4u + e) * 32u + lane] = blk.sum(e);
+    }
+    __syncthreads();
+    if (tid >= 128u) return;
+    const uint32_t e = warp, per_phase = n_blk / phases;   // warp e: accumulator e of every lane
+    double sum = 0.0;
+#pragma unroll 1
+    for (uint32_t phase = 0; phase < phases; ++phase) {
+        double half[2];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            half[h] = 0.0;
+            for (uint32_t b = 0; b < per_phase / 2u; ++b) half[h] += s_blk[((phase * per_phase + h * (per_phase / 2u) + b) * 4u + e) * 32u + lane];
+        }
+        const double both = half[0] + half[1];
+        sum = phase ? both + sum : both;
+    }
+    const uint32_t row = row0 + g + (e >> 1) * 8u, t = 2u * q + (e & 1u);
+    const bool mine = row < n_rows && t < n_tokens;
+    if (mine) out[(size_t)t * out_stride + row] = (float)sum;
+    uint32_t redo = __ballot_sync(0xffffffffu, mine && !isfinite(sum));
+    while (redo) {
+        const uint32_t src = __ffs((int)redo) - 1, t_src = 2u * (src & 3u) + (e & 1u);
+        const float v = head_row_dot(x + (size_t)t_src * hidden, w + (size_t)(row0 + (src >> 2) + (e >> 1) * 8u) * hidden, hidden);
+        if (lane == src) out[(size_t)t * out_stride + row] = v;
+        redo &= redo - 1u;
     }
 }
 
@@ -439,19 +561,24 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
     }
 }
 
-// The largest dynamic shared memory k_head_mma may ask for on the current device (0: could not be set).
+// The largest dynamic shared memory all of the tensor-core kernels may ask for on the current device (0: could not be set).
 size_t head_smem_limit() {
     static size_t limit[64] = {};
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if (!limit[dev]) {
+        const void *const fns[] = {(const void *)k_head_mma, (const void *)k_head_mma_few<false>, (const void *)k_head_mma_few<true>};
         cudaFuncAttributes fa;
         int optin = 0;
-        if (cudaFuncGetAttributes(&fa, k_head_mma) != cudaSuccess ||
-            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-            return 0;
-        const size_t most = (size_t)optin - fa.sharedSizeBytes;
-        if (cudaFuncSetAttribute(k_head_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
+        size_t fixed = 0;
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+        for (const void *fn : fns) {
+            if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
+            fixed = std::max(fixed, fa.sharedSizeBytes);
+        }
+        const size_t most = (size_t)optin - fixed;
+        for (const void *fn : fns)
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
         limit[dev] = most;
     }
     return limit[dev];
@@ -463,15 +590,23 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
                                uint32_t hidden, float *out, uint32_t out_stride) {
     // the tensor-core kernel: phases of K in whole groups of steps per half row, as few as keep the parts small;
     // sizes that have none take the register kernel
-    // (and so do few rows: a tile of sixteen is one pair of warps that walks K, and most SMs have none or one.  us, tensor-core /
-    // register kernel: 1000 x 512 one token 2.8 / 1.8, 4000 x 4096 one token 19.7 / 8.1, 1000 x 2048 four tokens 8.5 / 4.9)
-    const bool few_rows = (uint64_t)n_rows * n_tokens <= 4096u && n_tokens <= 6u;
-    for (uint32_t phases = 1; phases <= 8u && !few_rows; phases *= 2u) {
+    // (which kernel a row is worked out by does not depend on how many rows or tokens a call has beyond what leaves its bits
+    // alone: a vocabulary may be dealt over ranks in shards of any size)
+    for (uint32_t phases = 1; phases <= 8u; phases *= 2u) {
         const size_t parts = 3u * (size_t)n_tokens * (hidden / phases * 2u + kHeadPad);
         const size_t smem = parts + (phases > 1u ? kHeadTiles * 1024u : 0u);
         if (hidden % (256u * phases) != 0u || smem > head_smem_limit()) continue;
         if (parts > kHeadPartBytes && hidden % (512u * phases) == 0u && phases < 8u) continue;
         const uint32_t tiles = (n_rows + 15u) / 16u;
+        // up to two tiles per SM: a CTA per tile
+        if (tiles <= 2u * (uint32_t)sm_count && (size_t)hidden * 8u + (n_tokens <= 4u ? parts * phases : 0u) <= head_smem_limit()) {
+            const size_t sums = (size_t)hidden * 8u, shared = 3u * (size_t)n_tokens * (hidden * 2u + kHeadPad);
+            if (n_tokens <= 4u)
+                return launch_pdl(k_head_mma_few<true>, dim3(tiles), dim3(kFewThreads), sums + shared, st, 0u, x, w, out, n_rows, hidden,
+                                  out_stride, n_tokens, phases);
+            return launch_pdl(k_head_mma_few<false>, dim3(tiles), dim3(kFewThreads), sums, st, 0u, x, w, out, n_rows, hidden, out_stride,
+                              n_tokens, phases);
+        }
         const uint32_t ctas = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
         return launch_pdl(k_head_mma, dim3(ctas), dim3(kHeadThreads), smem, st, 0u, x, w, out, n_rows, hidden, out_stride, n_tokens,
                           phases);

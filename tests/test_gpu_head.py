@@ -19,8 +19,7 @@ def ctx():
     c.close()
 
 
-# rows: less than a tile (eight tokens; fewer take the register kernel), tiles with a remainder, the last of the register kernel
-# and the first of the other, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in phases); hidden: one group of
+# rows: less than a tile, tiles with a remainder, few and many tiles, more tiles than the CTAs hold at a time (8 tokens of 4096 walk K in phases); hidden: one group of
 # steps, several phases, sizes the tensor-core kernel leaves to the other one (264; 1048: more than its four pieces per lane)
 @pytest.mark.parametrize("tokens,rows,hidden", [(1, 1, 256), (8, 15, 256), (7, 17, 1280), (3, 2385, 4096), (5, 33, 264), (3, 300, 1048),
                                                 (8, 300, 1048), (7, 1000, 7168), (8, 2369, 4096), (8, 132700, 1024), (8, 132700, 4096),
@@ -68,7 +67,7 @@ def test_logits_are_as_close_as_sums_of_eight_products(ctx, bf16):
         assert float((added.clamp(min=0) / ref.pow(2).mean()).sqrt()) <= (7.5e-9 if bf16 else 4.02e-8)
 
 
-# 264 and few rows times tokens: the register kernel; 4096 with eight tokens: several phases of K
+# 264: the register kernel; 4096 with eight tokens: several phases of K
 @pytest.mark.parametrize("tokens,hidden,rows", [(1, 256, 4100), (1, 264, 70), (1, 512, 70), (3, 512, 1400), (8, 4096, 70)])
 def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden, rows):
     """One infinite weight gives an infinite logit of its sign (x is finite and nowhere 0), both signs or a NaN give NaN,
@@ -93,6 +92,20 @@ def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden
     token = torch.empty(1, dtype=torch.int64, device="cuda")
     ctx.cmd_greedy_argmax(out[0].contiguous(), token)
     assert int(token) == 3
+
+
+# the kernel of few row tiles and the other one, in phases (8 tokens of 4096) and not, one block of K per half and many
+@pytest.mark.parametrize("tokens,hidden", [(1, 256), (3, 768), (1, 4096), (8, 4096), (2, 6144), (8, 7168)])
+def test_logits_of_a_vocabulary_shard_have_the_bits_of_the_whole(ctx, tokens, hidden):
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    x = torch.randn(tokens, hidden, device="cuda", generator=g)
+    w = torch.empty(9000, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g).view(torch.int16)
+    whole = torch.empty(tokens, 9000, device="cuda")
+    ctx.cmd_head_logits(x, w, whole)
+    for r0, r1 in ((0, 1), (5, 22), (100, 4836), (100, 4837), (8985, 9000)):
+        part = torch.empty(tokens, r1 - r0, device="cuda")
+        ctx.cmd_head_logits(x, w[r0:r1], part)
+        assert torch.equal(part, whole[:, r0:r1]), (r0, r1)
 
 
 @pytest.mark.parametrize("vocab,offset", [(1, 0), (3, 0), (2047, 1), (4096, 0), (16385, 0), (129280, 0), (129281, 3)])
