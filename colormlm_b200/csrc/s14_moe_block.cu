@@ -44,7 +44,7 @@
 // exactly), the up epilogue works on BF16 gate and up and multiplies by the route weight, the down epilogue
 // and the mix round to BF16.  Every wait is bounded; a wait that runs out raises the CTA's abort
 // flag, the status word is set, and the CTA waits for its copies in flight, frees its tensor memory and returns.
-#include "s14_umma.cuh"
+#include "s14_moe_block.cuh"
 
 namespace s14 {
 
@@ -57,9 +57,7 @@ constexpr uint32_t kGrpHalf = 6;            // groups of one MMA: N = 96 accumul
 constexpr uint32_t kAccCols = 16u * kGrpHalf;
 static_assert(kGrp == 2u * kGrpHalf, "a wide chunk is two halves, one per issuing thread");
 static_assert(kBlockNt == 2u * kGrp, "a chunk record holds the tokens of the official arithmetic's chunks");
-constexpr uint32_t kStageA = kUnitStride;                  // a unit's codes, then its scales
 // a ring stage: a unit, then the token tiles of the unit's K range (2 KB per group) for as many groups as a chunk may hold
-static_assert(kStageA % 1024u == 0u && 2048u % 1024u == 0u, "operand tiles keep the 1 KB alignment of the 128-byte swizzle");
 constexpr uint32_t kGThreads = 512;
 constexpr uint32_t kGRingMax = 12;
 constexpr uint32_t kSfbBytes = 16u * 1024u;                // an item's digit-row scale atoms: K / 256 units x 1 KB, K <= 4096
@@ -78,42 +76,6 @@ constexpr uint32_t kGBarAccFree = kGBarAccDone + 2;        // [2] ... have been 
 constexpr uint32_t kGBarSfb = kGBarAccFree + 2;            // [2] an item's digit-row scales are laid out
 constexpr uint32_t kGBarFin = kGBarSfb + 2;
 constexpr uint32_t kGBars = kGBarFin + 1;
-constexpr uint32_t kPairsPerToken = S14_EXPERTS_PER_TOKEN + 1;   // pair = token * 7 + position in the mix (6: shared)
-
-// What the up kernel's epilogue leaves (the down kernel: kModeOfficial rounds its rows to BF16, the others do not)
-constexpr uint32_t kModeFused = 0u;      // the digit rows of the hidden values, laid out by the epilogue itself (small blocks)
-constexpr uint32_t kModeOfficial = 1u;   // the official arithmetic's BF16 hidden values, times the route weight
-constexpr uint32_t kModeValues = 2u;     // the F32 hidden values; a digits launch follows (large blocks)
-
-struct GemmArgs {
-    const BlockChunk *chunks;
-    const uint32_t *n_items;    // device memory: written by the grouping kernel (chunks x slices or row tiles)
-    const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048]
-    const uint8_t *exps;        // their block exponents + 100, [vector][K / 32]
-    float *out;                 // down: the pairs' expert outputs [pair][hidden]
-    uint8_t *hdig, *hexp;       // up: digit tiles and exponents of the pairs' hidden values
-    uint32_t by_threads;        // the token tiles come by the tile threads' own copies (large blocks), else by bulk copies
-    uint32_t hidden, inter, ring, stage;   // stage: bytes of a ring stage (a unit and nt_cap token tiles)
-    // Expert parallel with the exchange inside the kernel: the pairs' outputs go into every rank's buffer
-    // (plain stores to peer memory), and the last CTA to finish tells every rank that this rank's rows of
-    // call `ep_call` are there (flags[rank] of the call's parity in every rank's buffer).
-    float *out_peer[kMaxEpWorld];
-    unsigned long long *flag_peer[kMaxEpWorld];
-    unsigned int *ep_counter;   // this GPU's arrival counter, zero at rest
-    uint32_t ep_world, ep_rank, ep_call;
-    // Up kernel, kModeOfficial / kModeValues: the pairs' hidden values [pair][inter] (official: weighted and
-    // BF16-valued) and, for the official arithmetic, the routes' weights [token][top_k]
-    float *hval;
-    const float *weights;
-    uint32_t top_k;
-};
-
-// torch's .to(torch.bfloat16).float()
-__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-// two values rounded the same way: the first in the lower half of the word
-__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16;
-}
 
 // The nearest E4M3FN value (ties to even) of |v| <= 448: three mantissa bits; below 2^-6 multiples of 2^-9.
 __device__ __forceinline__ float e4m3fn_round(float v) {
@@ -175,10 +137,10 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
 __global__ void __launch_bounds__(1024)
 k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict__ pages,
               const uint8_t *const *__restrict__ page_table, const uint8_t *shared_page, uint32_t T, uint32_t top_k,
-              uint32_t n_experts, uint32_t S, uint32_t RT, uint32_t nt_cap, BlockChunk *__restrict__ chunks,
+              uint32_t n_experts, uint32_t S, uint32_t RT, uint32_t nt_cap, uint32_t even, BlockChunk *__restrict__ chunks,
               uint32_t *__restrict__ counts, uint32_t ep_rank, uint32_t ep_world, uint32_t shared_by_token) {
     constexpr uint32_t kG = S14_N_ROUTED_EXPERTS + 1;
-    __shared__ uint32_t cnt[kG], fill[kG], chunk0[kG + 1];
+    __shared__ uint32_t cnt[kG], fill[kG], chunk0[kG + 1], size[kG];
     __shared__ unsigned long long gpage[kG];
     __shared__ uint32_t bad;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, G = n_experts + 1u, n = T * top_k;
@@ -219,8 +181,13 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
         for (uint32_t k = 0; k < kPer; ++k) {
             const uint32_t g = lane * kPer + k;
             if (g < G) {
+                const uint32_t n_ch = (cnt[g] + nt_cap - 1u) / nt_cap;
                 chunk0[g] = c;
-                c += (cnt[g] + nt_cap - 1u) / nt_cap;
+                c += n_ch;
+                // the chunks of an expert of like size, in whole multiples of `even`: what one of them costs goes with its size, and
+                // neighbouring items - an expert's chunks in turn - go to neighbouring CTAs (full chunks and a rest: 370 tokens 730
+                // us, so 705; 1000 official ones 1265 and 1165)
+                size[g] = n_ch ? ((cnt[g] + n_ch * even - 1u) / (n_ch * even)) * even : 1u;
             }
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
@@ -241,16 +208,16 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
         const uint32_t g = 1u + (uint32_t)e, t = i / top_k, m = i - t * top_k;
         const uint32_t k = atomicAdd(&fill[g], 1u);
         if (k == 0u && !page_table) gpage[g] = __ldcg(reinterpret_cast<const unsigned long long *>(pages + i));
-        BlockChunk *ch = chunks + chunk0[g] + k / nt_cap;
-        ch->tok[k % nt_cap] = t;
-        ch->pair[k % nt_cap] = t * kPairsPerToken + m;
+        BlockChunk *ch = chunks + chunk0[g] + k / size[g];
+        ch->tok[k % size[g]] = t;
+        ch->pair[k % size[g]] = t * kPairsPerToken + m;
     }
     if (shared_page) {
         for (uint32_t k = tid; sh_first + k * sh_step < T; k += blockDim.x) {
             const uint32_t t = sh_first + k * sh_step;
-            BlockChunk *ch = chunks + chunk0[0] + k / nt_cap;
-            ch->tok[k % nt_cap] = t;
-            ch->pair[k % nt_cap] = t * kPairsPerToken + S14_EXPERTS_PER_TOKEN;
+            BlockChunk *ch = chunks + chunk0[0] + k / size[0];
+            ch->tok[k % size[0]] = t;
+            ch->pair[k % size[0]] = t * kPairsPerToken + S14_EXPERTS_PER_TOKEN;
         }
     }
     __syncthreads();
@@ -266,7 +233,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
         const uint32_t g = lo, c0 = chunk0[g], nch = chunk0[g + 1u] - c0;
         BlockChunk *ch = chunks + c;
         ch->page = reinterpret_cast<const uint8_t *>(gpage[g]);
-        ch->nt = c + 1u < c0 + nch ? nt_cap : cnt[g] - (c - c0) * nt_cap;
+        ch->nt = c + 1u < c0 + nch ? size[g] : cnt[g] - (c - c0) * size[g];
         ch->c0 = c0;
         ch->nch = nch;
     }
@@ -992,7 +959,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     if (ep_world == 0u) ep_world = 1u;
     if (*err == cudaSuccess)
         *err = launch_pdl(k_block_group, dim3(1), dim3(1024), 0, st, 0u, ids, pages, page_table, shared_page, n_tokens, top_k, n_experts,
-                          S / mt, RT / mt, nt_cap, w.chunks, w.counts, ep_rank, ep_world, (shared_by_token && ep_world > 1u) ? 1u : 0u);
+                          S / mt, RT / mt, nt_cap, shape == 0u ? 1u : 2u * tpg, w.chunks, w.counts, ep_rank, ep_world, (shared_by_token && ep_world > 1u) ? 1u : 0u);
     if (*err != cudaSuccess) return 1;
     if (pairs_out && !ep) {
         // expert parallel: the pairs of the experts this rank owns; the others stay zero for the sum over the ranks
@@ -1028,19 +995,16 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     auto gemm = [&](auto kernel, const GemmArgs &args) {
         if (*err == cudaSuccess) *err = launch_pdl(kernel, dim3(sm_count), dim3(kGThreads), smem, st, 0u, args, status);
     };
-#define S14_BLOCK_UP(MT, WIDE)                                                                     \
-    do {                                                                                           \
-        if (official) gemm(k_block_gemm<false, MT, WIDE, kModeOfficial>, up);                      \
-        else if (values) gemm(k_block_gemm<false, MT, WIDE, kModeValues>, up);                     \
-        else gemm(k_block_gemm<false, MT, WIDE, kModeFused>, up);                                  \
-        if (values) digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp);              \
-        if (official) gemm(k_block_gemm<true, MT, WIDE, kModeOfficial>, down);                     \
-        else gemm(k_block_gemm<true, MT, WIDE, kModeFused>, down);                                 \
-    } while (0)
-    if (shape == 0u) S14_BLOCK_UP(1, false);
-    else if (shape == 1u) S14_BLOCK_UP(2, false);
-    else S14_BLOCK_UP(2, true);
-#undef S14_BLOCK_UP
+    auto pair_gemm = [&](bool is_down, const GemmArgs &args) {
+        if (*err == cudaSuccess) *err = launch_pair_gemm(st, sm_count, is_down, official, args, groups / 2u, status);
+    };
+    if (shape != 0u) pair_gemm(false, up);
+    else if (official) gemm(k_block_gemm<false, 1, false, kModeOfficial>, up);
+    else gemm(k_block_gemm<false, 1, false, kModeFused>, up);
+    if (values) digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp);
+    if (shape != 0u) pair_gemm(true, down);
+    else if (official) gemm(k_block_gemm<true, 1, false, kModeOfficial>, down);
+    else gemm(k_block_gemm<true, 1, false, kModeFused>, down);
     if (pairs_out || *err != cudaSuccess) return launches;
     *err = launch_mix(st, w.d, ids, weights, n_tokens, top_k, shared_page != nullptr, x, y, hidden, w.counts, residual, nullptr, status,
                       official);

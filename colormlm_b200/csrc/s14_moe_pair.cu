@@ -1,0 +1,626 @@
+// The contraction kernels of the grouped block path for blocks of more than twelve tokens: a PAIR of CTAs (a cluster of
+// two, the two SMs of a TPC) works on an item together, tcgen05.mma.cta_group::2.  What they compute is described in
+// s14_moe_block.cu; per item it is a chunk of up to twelve groups of sixteen digit rows (one token each, official
+// arithmetic: two) times 256 rows of an expert: two slices of the up projection or two row tiles of w2.
+//
+// Each CTA brings its own 128 rows of the page (a unit of 17 KB per step of 256 k) and HALF of the chunk's digit tiles; the
+// pair's tensor cores read both halves, so a step costs an SM 17 + 12 KB instead of 17 + 24, one MMA does N = 192
+// columns, and the accumulators of one row tile are all an SM holds: 192 columns, which leaves room for a second set.  So an
+// item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
+// (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
+// epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 506 / 294
+// us, now 427 / 204; 1000 tokens of the official arithmetic 1206 / 443, now 730 / 309.
+//
+// What bounds it.  A step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles, the issuing
+// warp's round 470, a step 600-700 on average.  A second warp that copies the codes ahead gets a probe to 389 cycles a
+// step, but adds a hand-off to every stage's way through the ring of seven (370 tokens 736 us instead of 704).  Sustained, the
+// 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.
+//
+// Roles in a CTA of 608 threads: warps 0-7 epilogue (two warpgroups, each with every lane of tensor memory, the even and
+// the odd groups of the chunk); warps 8-11 copy (the ring slots in turn, a lane per copy: a round of waiting, arming
+// and seven copies takes 0.3-0.5 us); warp 12 of the first CTA issues the pair's tensor operations, that of the second
+// passes on that its stage is complete; warps 13-18 lay out the scale codes of the digit rows of a stage.  A stage's barriers:
+// `full` in each CTA (unit, tiles, codes; in the first CTA also that the second's is complete), `done` in each (the commit
+// arrives at both).  Every wait is bounded; one that runs out raises the CTA's abort flag, the status word is set, the CTA
+// waits for its copies, and the pair meets at a cluster barrier before tensor memory is freed.
+#include "s14_moe_block.cuh"
+
+namespace s14 {
+
+namespace {
+
+constexpr uint32_t kPGroups = 12, kPCols = 16u * kPGroups;   // accumulator columns of a chunk
+constexpr uint32_t kPEpi = 256, kPProds = 4, kPProdWarp0 = kPEpi / 32u, kPMmaWarp = kPProdWarp0 + kPProds, kPCodeWarp0 = kPMmaWarp + 1u;
+constexpr uint32_t kPCodes = kPCols;                         // a thread per operand row
+constexpr uint32_t kPThreads = kPCodeWarp0 * 32u + kPCodes;
+constexpr uint32_t kPRingMax = 12;
+// tensor memory columns: two sets of accumulators, then the scale codes of four stages
+constexpr uint32_t kPColScale = 2u * kPCols, kPScaleSets = 4, kPScaleCols = 32;   // a set: unit codes [2][4], digit-row codes [2][8]
+static_assert(kPColScale + kPScaleSets * kPScaleCols <= 512u, "tensor memory map");
+// barriers
+constexpr uint32_t kPBarFull = 0, kPBarDone = kPRingMax;
+constexpr uint32_t kPBarAccDone = 2 * kPRingMax, kPBarAccFree = kPBarAccDone + 2, kPBarFin = kPBarAccFree + 2, kPBars = kPBarFin + 1;
+
+struct PairItem {
+    unsigned long long page;
+    uint32_t nt, r;             // pairs of the chunk (0x100: the expert has more chunks); pair of slices or row tiles
+};
+
+// ---- operations of a CTA pair ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the shared-memory address of the same variable in the first CTA of the pair
+__device__ __forceinline__ uint32_t first_cta(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// At another CTA's barrier.  Nothing that threads read is handed over with it - the tensor cores read either CTA's shared
+// memory behind that CTA's own proxy fence, and tensor memory is drained by its owner -, so it carries no wider fence: with
+// .release.cluster (and .acquire.cluster on the other side) a stage took a microsecond more.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
+        : "memory");
+}
+// every CTA's 512 bytes at the descriptor's place into its own tensor memory
+__device__ __forceinline__ void pair_copy_scales(uint32_t tmem, uint64_t desc) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
+}
+// arrives at the barrier of both CTAs when the tensor operations issued so far are complete
+__device__ __forceinline__ void pair_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+// M = 256: 128 rows in each CTA
+__device__ __forceinline__ constexpr uint32_t pair_idesc(uint32_t n) {
+    return (1u << 7) | (1u << 10) | ((n >> 3) << 17) | (1u << 23) | ((256u >> 4) << 24);
+}
+// The 128 threads of a warpgroup of the epilogue.
+__device__ __forceinline__ bool group_all(uint32_t id, bool ok) {
+    uint32_t r;
+    __syncwarp();
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.b32 p, %1, 0;\n"
+        "barrier.cta.red.and.pred q, %2, 128, p;\n"
+        "selp.b32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((uint32_t)ok), "r"(id)
+        : "memory");
+    return r != 0;
+}
+
+// The sum of a token's digit shares, rounded once: in F32 operations, two columns to an operation, because FP64 ones run at a
+// quarter of their rate while the tensor cores are busy (sixteen conversions and additions of 8 tokens x 128 rows: 4200
+// cycles, 1600 without the MMAs).  Added to s = 1.5 * 2^(e+5), where every share is below 2^(e+1), a share leaves what does not fit
+// 2^(e-18) exactly behind (t = s + v; v - (t - s)); those remainders likewise 20 bits below; what they leave is at most
+// 2^(e-39) and summed as it is.  The three parts are exact but for 2^-60 of the largest share - sums in double lose 2^-50 -
+// and are added with the rounding errors of their own sum.  Shares too large or too small for the constants go through double.
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+// columns 0-7 and 8-15 into three parts each
+__device__ __forceinline__ void digit_parts(const uint32_t (&r)[16], float2 sigma, float2 sigma2, float2 &p1, float2 &p2, float2 &p3) {
+    float2 s1 = sigma, s2 = sigma2;
+    p3 = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float2 v = make_float2(__uint_as_float(r[c]), __uint_as_float(r[8 + c]));
+        const float2 t1 = __fadd2_rn(s1, v);
+        const float2 v2 = minus2(v, minus2(t1, s1));
+        s1 = t1;
+        const float2 t2 = __fadd2_rn(s2, v2);
+        p3 = __fadd2_rn(p3, minus2(v2, minus2(t2, s2)));
+        s2 = t2;
+    }
+    p1 = minus2(s1, sigma);
+    p2 = minus2(s2, sigma2);
+}
+// a + b + c rounded once but for what is far below the last bit
+__device__ __forceinline__ float sum3(float a, float b, float c) {
+    const float t = __fadd_rn(b, c), tb = __fsub_rn(t, b), te = __fadd_rn(__fsub_rn(b, __fsub_rn(t, tb)), __fsub_rn(c, tb));
+    const float s = __fadd_rn(a, t), sa = __fsub_rn(s, a), se = __fadd_rn(__fsub_rn(a, __fsub_rn(s, sa)), __fsub_rn(t, sa));
+    return __fadd_rn(s, __fadd_rn(se, te));
+}
+// the exponent field of the largest of eight shares and whether the constants made of it are in range
+__device__ __forceinline__ uint32_t share_exponent(const uint32_t (&r)[16], int first) {
+    float m = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) m = fmaxf(m, fabsf(__uint_as_float(r[first + c])));
+    return __float_as_uint(m) & 0x7F800000u;   // (a NaN beside other shares is dropped here and makes the sum one)
+}
+__device__ __forceinline__ bool share_in_range(uint32_t ex) { return ex - (48u << 23) < (192u << 23); }   // 2^-79 .. 2^112
+__device__ __forceinline__ float2 share_sigmas(uint32_t ex) {
+    return make_float2(__uint_as_float(ex + (5u << 23) + 0x400000u), __uint_as_float(ex - (15u << 23) + 0x400000u));
+}
+__device__ __forceinline__ void digit_sums_f64(const uint32_t (&r)[16], double &first, double &second) {
+    first = second = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        first += (double)__uint_as_float(r[c]);
+        second += (double)__uint_as_float(r[8 + c]);
+    }
+}
+// all sixteen columns are one token's
+__device__ __forceinline__ float digit_sum(const uint32_t (&r)[16]) {
+    const uint32_t ex = max(share_exponent(r, 0), share_exponent(r, 8));
+    if (!share_in_range(ex)) {
+        double hi, lo;
+        digit_sums_f64(r, hi, lo);
+        return (float)(lo + hi);
+    }
+    const float2 sg = share_sigmas(ex);
+    float2 p1, p2, p3;
+    digit_parts(r, make_float2(sg.x, sg.x), make_float2(sg.y, sg.y), p1, p2, p3);
+    return sum3(__fadd_rn(p1.x, p1.y), __fadd_rn(p2.x, p2.y), __fadd_rn(p3.x, p3.y));   // (the first two additions are exact)
+}
+// columns 0-7 are one token's, 8-15 another's: their sums as BF16
+__device__ __forceinline__ uint32_t digit_sums_pair(const uint32_t (&r)[16]) {
+    const uint32_t e0 = share_exponent(r, 0), e1 = share_exponent(r, 8);
+    if (!share_in_range(e0) || !share_in_range(e1)) {
+        double a, b;
+        digit_sums_f64(r, a, b);
+        return bf16_pair((float)a, (float)b);
+    }
+    const float2 s0 = share_sigmas(e0), s1 = share_sigmas(e1);
+    float2 p1, p2, p3;
+    digit_parts(r, make_float2(s0.x, s1.x), make_float2(s0.y, s1.y), p1, p2, p3);
+    return bf16_pair(sum3(p1.x, p2.x, p3.x), sum3(p1.y, p2.y, p3.y));
+}
+
+template <bool kDown, bool kOff>
+__global__ void __launch_bounds__(kPThreads, 1)
+k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *status) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr uint32_t kTpg = kOff ? 2u : 1u;                     // tokens per group of sixteen digit rows
+    constexpr uint32_t kRows = 16u / kTpg, kTileB = kRows * 128u; // a token's digit rows, and the bytes of its tile
+    constexpr uint32_t kTok = kPGroups * kTpg;                    // most tokens of a chunk
+    constexpr uint32_t kMine = kPGroups / 2u;                     // groups of an epilogue thread
+    constexpr uint32_t kPBatch = kOff ? 56u : 96u;                // items decoded at a time (10 KB of static shared memory are left beside the ring)
+    __shared__ __align__(8) uint64_t bars[kPBars];
+    __shared__ __align__(16) PairItem s_rec[kPBatch];
+    __shared__ uint32_t s_pair[kPBatch][kTok];
+    __shared__ float s_x[2][kMine][64];                           // an item's gates and up projections, handed across (official: two BF16 each)
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+
+    const uint32_t tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31u;
+    const uint32_t rank = cluster_rank(), n_pairs = gridDim.x >> 1, me = blockIdx.x >> 1;
+    const uint32_t K = kDown ? a.inter : a.hidden;
+    const uint32_t nu = K >> 8;                                    // units of an item
+    const uint32_t ring = a.ring, stage = a.stage;
+    const uint32_t n_atoms = (half_cap * 32u + 127u) >> 7;         // scale atoms of a stage's digit rows, per 128 k
+    const uint32_t off_codes = kStageA + half_cap * 2048u;         // in a stage: the unit, the tiles, the digit rows' scale codes
+    const size_t page_off = kDown ? mxfp4_down_offset(a.hidden, a.inter) : 0u;
+    const uint32_t bar0 = smem_u32(bars), ring0 = smem_u32(smem);
+    auto bar = [&](uint32_t i) { return bar0 + i * 8u; };
+    volatile int *const abortp = &abort_flag;
+
+    if (tid < kPBars) {
+        uint32_t count = 1u;
+        // the copying thread, the codes' warps; the first CTA's: and the second CTA's stage
+        if (tid < kPRingMax) count = 1u + kPCodes / 32u + (rank == 0u ? 1u : 0u);
+        else if (tid >= kPBarAccFree && tid < kPBarAccFree + 2u) count = 2u * kPEpi / 32u;
+        mbar_init(bar(tid), count);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid == 0) abort_flag = 0;
+    if (warp == kPMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        fence_before();
+    }
+    __syncthreads();
+    cluster_barrier();   // the other CTA's barriers are there
+    fence_after();
+    const uint32_t tmem = tmem_slot;
+    dependency_wait();
+    const uint32_t n_items = __ldcg(a.n_items);
+    const uint32_t R = (kDown ? (a.hidden >> 7) : (a.inter >> 6)) / 2u;   // items per chunk
+    const uint32_t n_local = n_items > me ? (n_items - me + n_pairs - 1u) / n_pairs : 0u;
+
+    // what the roles carry from batch to batch
+    uint32_t slot = 0, round = 0, gi = 0, step = 0;
+    bool ok = true;
+    auto next_slot = [&]() {
+        if (++slot == ring) {
+            slot = 0;
+            ++round;
+        }
+    };
+    const unsigned long long once = l2_policy_evict_first();
+
+#pragma unroll 1
+    for (uint32_t base = 0; base < n_local; base += kPBatch) {
+        const uint32_t nb = n_local - base < kPBatch ? n_local - base : kPBatch;
+        // the batch's items into shared memory: the records, then the chunks' pairs, all loads in flight together
+        if (tid < nb) {
+            const uint32_t q = me + (base + tid) * n_pairs;
+            const BlockChunk *g = a.chunks + q / R;
+            const uint32_t c0 = __ldcg(&g->c0), nch = __ldcg(&g->nch), j = q - c0 * R;
+            const uint32_t r = j / nch, c = c0 + (j - r * nch);
+            s_rec[tid].page = __ldcg(reinterpret_cast<const unsigned long long *>(&a.chunks[c].page));
+            s_rec[tid].nt = __ldcg(&a.chunks[c].nt) | (nch > 1u ? 0x100u : 0u);
+            s_rec[tid].r = r;
+            s_pair[tid][0] = c;
+        }
+        __syncthreads();
+        {
+            constexpr uint32_t kLoads = (kPBatch * kTok + kPThreads - 1u) / kPThreads;
+            uint32_t p[kLoads];
+#pragma unroll
+            for (uint32_t k = 0; k < kLoads; ++k) {
+                const uint32_t i = (tid + k * kPThreads) / kTok, t = (tid + k * kPThreads) % kTok;
+                if (i < nb) p[k] = __ldcg(&a.chunks[s_pair[i][0]].pair[t]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t k = 0; k < kLoads; ++k) {
+                const uint32_t i = (tid + k * kPThreads) / kTok, t = (tid + k * kPThreads) % kTok;
+                if (i < nb) s_pair[i][t] = p[k];
+            }
+        }
+        __syncthreads();
+
+        if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds) {
+            // ---- a stage: the unit of this CTA's row tile, then the digit tiles of its half of the chunk ----
+#pragma unroll 1
+            for (uint32_t i = 0; i < nb && ok; ++i) {
+                const uint32_t multi = warp_uniform(s_rec[i].nt >> 8), nt = warp_uniform(s_rec[i].nt & 0xFFu);
+                const uint32_t half = (((nt + kTpg - 1u) / kTpg + 1u) >> 1) * kTpg, first = rank * half;   // this CTA's tokens
+                const uint32_t mine = nt > first ? min(nt - first, half) : 0u;
+                // a lane's copy of every stage: lane t < mine the tile of a token, the last lane the unit
+                const bool is_unit = lane == 31u;
+                const uint8_t *src = reinterpret_cast<const uint8_t *>(s_rec[i].page) + page_off +
+                                     (size_t)(s_rec[i].r * 2u + rank) * nu * kUnitStride;
+                if (lane < mine) {
+                    const uint32_t vec = kDown ? s_pair[i][first + lane] : s_pair[i][first + lane] / kPairsPerToken;
+                    src = a.dig + (size_t)vec * nu * kTileB;
+                }
+                const uint32_t bytes = is_unit ? kUnitStride : kTileB, to = ring0 + (is_unit ? 0u : kStageA + lane * kTileB);
+#pragma unroll 1
+                for (uint32_t u = 0; u < nu; ++u, src += bytes) {
+                    if ((slot & (kPProds - 1u)) == warp - kPProdWarp0) {
+                        ok = !round || mbar_wait_warp(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
+                        if (!ok) break;
+                        const uint32_t full = bar(kPBarFull + slot), dst = to + slot * stage;
+                        if (is_unit) {
+                            mbar_arrive_expect(full, kStageA + mine * kTileB);
+                            // an expert with one chunk is read once; with more, its later chunks want the units in the L2
+                            if (multi) bulk_copy(dst, src, kStageA, full);
+                            else bulk_copy_stream(dst, src, kStageA, full, once);
+                        } else if (lane < mine) {
+                            bulk_copy(dst, src, kTileB, full);   // (bytes that land before the barrier is armed are counted all the same)
+                        }
+                        __syncwarp();
+                    }
+                    next_slot();
+                }
+            }
+        } else if (warp == kPMmaWarp) {
+            if (rank == 0u) {
+                const uint32_t tm = warp_uniform(tmem);
+                const uint64_t a_desc0 = smem_desc(ring0, 1, 64, 2), b_desc0 = smem_desc(ring0 + kStageA, 1, 64, 2);
+                const uint64_t sa_desc0 = smem_desc(ring0 + kUnitBytes, 0, 8, 0), sb_desc0 = smem_desc(ring0 + off_codes, 0, 8, 0);
+#pragma unroll 1
+                for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
+                    const uint32_t buf = gi & 1u, nt = warp_uniform(s_rec[i].nt & 0xFFu);
+                    const uint32_t n = 32u * (((nt + kTpg - 1u) / kTpg + 1u) >> 1), idesc = pair_idesc(n);
+                    if (gi >= 2u) ok = mbar_wait_warp(bar(kPBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
+                    if (!ok) break;
+                    fence_after();
+                    const uint32_t acc = tm + buf * kPCols;
+                    const bool two = n > 128u;   // two scale atoms per 128 k
+#pragma unroll 1
+                    for (uint32_t ku = 0; ku < nu; ++ku) {
+                        ok = mbar_wait_warp(bar(kPBarFull + slot), round & 1u, abortp);
+                        if (!ok) break;
+                        fence_after();
+                        if (elect_one()) {
+                            const uint32_t at = slot * (stage >> 4), sfa = tm + kPColScale + (step & (kPScaleSets - 1u)) * kPScaleCols;
+                            const uint32_t sfb = sfa + 8u;
+                            pair_copy_scales(sfa, sa_desc0 + at);
+                            pair_copy_scales(sfa + 4u, sa_desc0 + at + (kAtomBytes >> 4));
+                            pair_copy_scales(sfb, sb_desc0 + at);
+                            pair_copy_scales(sfb + 8u, sb_desc0 + at + n_atoms * (kAtomBytes >> 4));
+                            if (two) {
+                                pair_copy_scales(sfb + 4u, sb_desc0 + at + (kAtomBytes >> 4));
+                                pair_copy_scales(sfb + 12u, sb_desc0 + at + (n_atoms + 1u) * (kAtomBytes >> 4));
+                            }
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; ++kk) {
+                                const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
+                                pair_mma(acc, a_desc0 + at + kk * 2u, b_desc0 + at + kk * 2u, idesc | (sfid << 29) | (sfid << 4),
+                                         (sfa + atom * 4u) | (sfid << 30), (sfb + atom * 8u) | (sfid << 30), (ku || kk) ? 1u : 0u);
+                            }
+                            pair_commit(bar(kPBarDone + slot));
+                        }
+                        __syncwarp();
+                        next_slot();
+                        ++step;
+                    }
+                    if (!ok) break;
+                    if (elect_one()) pair_commit(bar(kPBarAccDone + buf));
+                    __syncwarp();
+                }
+            } else {
+                // ---- the second CTA's stages are complete (every writer has made its bytes visible to the tensor cores) ----
+#pragma unroll 1
+                for (uint32_t i = 0; i < nb * nu && ok; ++i) {
+                    ok = mbar_wait_warp(bar(kPBarFull + slot), round & 1u, abortp);
+                    if (!ok) break;
+                    if (elect_one()) mbar_arrive_remote(first_cta(bar(kPBarFull + slot)));
+                    __syncwarp();
+                    next_slot();
+                }
+            }
+        } else if (warp < kPEpi / 32u) {
+            // ---- epilogue: a group's sixteen columns of digit shares, added exactly and rounded once ----
+            const uint32_t wg = warp >> 2, row = tid & 127u, el = row & 63u, par = row >> 6;
+            const uint32_t lane_base = tmem + (((warp & 3u) * 32u) << 16);
+            const uint32_t free0 = first_cta(bar(kPBarAccFree));
+#pragma unroll 1
+            for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
+                const uint32_t buf = gi & 1u, nt = s_rec[i].nt & 0xFFu, idx = s_rec[i].r * 2u + rank;   // slice or row tile
+                const uint32_t *pair = s_pair[i];
+                float wt[kOff && !kDown ? kMine : 1u];   // official: the route weights of the tokens this thread finishes
+                if constexpr (kOff && !kDown) {
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; ++m) {
+                        const uint32_t t = 2u * (2u * m + wg) + par;
+                        wt[m] = 1.0f;
+                        if (t < nt) {
+                            const uint32_t tok = pair[t] / kPairsPerToken, pos = pair[t] - tok * kPairsPerToken;
+                            if (pos < S14_EXPERTS_PER_TOKEN) wt[m] = __ldcg(a.weights + tok * a.top_k + pos);
+                        }
+                    }
+                }
+                ok = group_all(1u + wg, mbar_wait(bar(kPBarAccDone + buf), (gi >> 1) & 1u, abortp));
+                if (!ok) break;
+                fence_after();
+                // groups wg, wg + 2, ... of the chunk; official: two BF16 values to a register
+                float v[kOff ? 1u : kMine];
+                uint32_t vb[kOff ? kMine : 1u];
+#pragma unroll
+                for (uint32_t m = 0; m < kMine; m += 2u) {
+                    const uint32_t g = 2u * m + wg;
+                    if (g * kTpg < nt) {   // uniform in the warpgroup
+                        uint32_t r0[16], r1[16];
+                        tmem_ld16(lane_base + buf * kPCols + 16u * g, r0);
+                        tmem_ld16(lane_base + buf * kPCols + 16u * (g + 2u), r1);   // (not used beyond nt)
+                        tmem_ld_wait();
+                        if constexpr (kOff) {
+                            vb[m] = digit_sums_pair(r0);
+                            vb[m + 1u] = digit_sums_pair(r1);
+                        } else {
+                            v[m] = digit_sum(r0);
+                            v[m + 1u] = digit_sum(r1);
+                        }
+                    }
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(free0 + buf * 8u);
+                if constexpr (kDown) {
+                    // row idx * 128 + `row` of the pairs' expert outputs
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; ++m) {
+#pragma unroll
+                        for (uint32_t k = 0; k < kTpg; ++k) {
+                            const uint32_t t = (2u * m + wg) * kTpg + k;
+                            if (t < nt) {
+                                const size_t at = (size_t)pair[t] * a.hidden + idx * 128u + row;
+                                float o;
+                                if constexpr (kOff) o = __uint_as_float(k ? vb[m] & 0xFFFF0000u : vb[m] << 16);   // (a linear's result is BF16)
+                                else o = v[m];
+                                if (a.ep_world > 1u) {
+#pragma unroll 1
+                                    for (uint32_t p = 0; p < a.ep_world; ++p) a.out_peer[p][at] = o;
+                                } else {
+                                    a.out[at] = o;
+                                }
+                            }
+                        }
+                    }
+                } else {
+                    // threads 0-63 of the warpgroup hold the gates of the slice's elements, threads 64-127 their up
+                    // projections.  Each half finishes half of the tokens and hands the other the values it lacks.
+                    // Official arithmetic (s14_first_real_token/executor.py:712-743): gate and up rounded to BF16, the
+                    // limited SwiGLU in F32, times the route's weight (not for the shared expert), rounded to BF16.
+                    uint16_t *const s_h = reinterpret_cast<uint16_t *>(&s_x[wg][0][0]);   // [kMine][2][64]
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; ++m) {
+                        if constexpr (kOff) {
+                            if ((2u * m + wg) * 2u < nt) s_h[(m * 2u + par) * 64u + el] = (uint16_t)(par ? vb[m] & 0xFFFFu : vb[m] >> 16);
+                        } else {
+                            if (2u * m + wg < nt && (m & 1u) != par) s_x[wg][m][el] = v[m];
+                        }
+                    }
+                    group_all(1u + wg, true);
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; ++m) {
+                        const uint32_t t = kOff ? 2u * (2u * m + wg) + par : 2u * m + wg;
+                        if (t < nt && (kOff || (m & 1u) == par)) {
+                            float mine, other;
+                            if constexpr (kOff) {
+                                mine = __uint_as_float(par ? vb[m] & 0xFFFF0000u : vb[m] << 16);
+                                other = __uint_as_float((uint32_t)s_h[(m * 2u + (par ^ 1u)) * 64u + el] << 16);
+                            } else {
+                                mine = v[m];
+                                other = s_x[wg][m][el];
+                            }
+                            float hv = par ? swiglu_limit_f32(other, mine) : swiglu_limit_f32(mine, other);
+                            if constexpr (kOff) {
+                                const uint32_t pos = pair[t] % kPairsPerToken;
+                                if (pos < S14_EXPERTS_PER_TOKEN) hv = __fmul_rn(hv, wt[m]);
+                                hv = bf16_round(hv);
+                            }
+                            a.hval[(size_t)pair[t] * a.inter + idx * 64u + el] = hv;
+                        }
+                    }
+                }
+            }
+        } else if (warp >= kPCodeWarp0) {
+            // ---- the scale codes of ALL digit rows of the chunk (both CTAs' tensor cores multiply with every column) as the
+            // atoms tensor memory takes: row n of the operand = 16 * group + digit row, byte (n % 32) * 16 +
+            // (n / 32 % 4) * 4 + block % 4 of the atom of rows n / 128 and four scale blocks.  Digit row j < 8 of a block with
+            // exponent E has the code 127 + E - 23 + 3 j, row 8 + j the code 127 + E - 47 + 3 j; the exponents are stored as
+            // E + 100. ----
+            const uint32_t n = tid - kPCodeWarp0 * 32u;   // this thread's row
+            const uint32_t j = n & (kRows - 1u), n_tok = n / kRows;
+            const uint32_t bias = 0x01010101u * (uint32_t)(j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20);
+            const uint32_t code_at = off_codes + (n >> 7) * kAtomBytes + (n & 31u) * 16u + ((n >> 5) & 3u) * 4u;
+            const bool has_row = n < half_cap * 32u;
+            // the row's exponents in an item, or nullptr
+            auto exps_of = [&](uint32_t i) -> const uint4 * {
+                if (i >= nb || !has_row || n_tok >= (s_rec[i].nt & 0xFFu)) return nullptr;
+                const uint32_t vec = kDown ? s_pair[i][n_tok] : s_pair[i][n_tok] / kPairsPerToken;
+                return reinterpret_cast<const uint4 *>(a.exps + (size_t)vec * (K >> 5));
+            };
+            // two units' exponents per load, four loads in flight, each in registers of its own (a queue that moves them waits
+            // for the newest): the units in steps of eight, the last step of an item perhaps short
+            const uint4 *now = exps_of(0);
+            uint4 e[4];
+            auto fetch = [&](const uint4 *p, uint32_t u) { return p && u < nu ? __ldcg(p + (u >> 1)) : make_uint4(0u, 0u, 0u, 0u); };
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) e[k] = fetch(now, 2u * k);
+#pragma unroll 1
+            for (uint32_t i = 0; i < nb && ok; ++i) {
+                const uint4 *const then = exps_of(i + 1u);
+                const bool live = now != nullptr;
+#pragma unroll 1
+                for (uint32_t u0 = 0; u0 < nu && ok; u0 += 8u) {
+                    const bool more = u0 + 8u < nu;
+                    const uint4 *const from = more ? now : then;
+                    const uint32_t at_u = more ? u0 + 8u : 0u;
+#pragma unroll
+                    for (uint32_t k = 0; k < 8u; ++k) {
+                        if (u0 + k < nu && ok) {
+                            ok = !round || mbar_wait_warp(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
+                            if (ok) {
+                                if (has_row) {
+                                    uint8_t *const s = smem + slot * stage + code_at;
+                                    *reinterpret_cast<uint32_t *>(s) = live ? ((k & 1u) ? e[k >> 1].z : e[k >> 1].x) + bias : 0x7F7F7F7Fu;
+                                    *reinterpret_cast<uint32_t *>(s + n_atoms * kAtomBytes) =
+                                        live ? ((k & 1u) ? e[k >> 1].w : e[k >> 1].y) + bias : 0x7F7F7F7Fu;
+                                }
+                                fence_async_smem();   // tcgen05.cp reads them
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(bar(kPBarFull + slot));
+                                next_slot();
+                            }
+                        }
+                        if (k & 1u) e[k >> 1] = fetch(from, at_u + k - 1u);
+                    }
+                }
+                now = then;
+            }
+        }
+        __syncwarp();
+        __syncthreads();  // the records are rewritten; a role that gave up has raised the flag
+        if (abort_flag) break;
+    }
+    if (warp == kPMmaWarp && rank == 0u) {
+        // nothing of the pair's tensor work is in flight when the tensor memory is freed
+        if (elect_one()) pair_commit(bar(kPBarFin));
+        __syncwarp();
+    }
+    // ... which also arrives at the other CTA, behind the stages' arrivals
+    if (warp == kPMmaWarp) mbar_wait_warp(bar(kPBarFin), 0, abortp);
+    if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds && lane == 0) {
+        // copies in flight land in this CTA's shared memory, arrivals of the tensor operations at its barriers: wait for them
+#pragma unroll 1
+        for (uint32_t s = warp - kPProdWarp0; s < ring; s += kPProds) {
+            const uint32_t used = round + (s < slot ? 1u : 0u);   // rounds of this slot
+            uint32_t tries = 0;
+            if (used) {
+#pragma unroll 1
+                while (!mbar_try(bar((abort_flag ? kPBarFull : kPBarDone) + s), (used - 1u) & 1u) && ++tries < kSpin) {
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncwarp();
+    __syncthreads();
+    cluster_barrier();
+    if (warp == kPMmaWarp)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
+    if (tid == 0 && abort_flag) atomicExch(status, 0x5507u);
+    if constexpr (kDown && !kOff) {
+        if (a.ep_world > 1u) {
+            // every store of this CTA to the peers' buffers is ordered before the count; the last CTA of the
+            // grid publishes the call's number to every rank
+            if (warp < kPEpi / 32u) __threadfence_system();
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence_system();
+                if (atomicAdd(a.ep_counter, 1u) == gridDim.x - 1u) {
+                    *a.ep_counter = 0u;
+                    __threadfence_system();
+                    const unsigned long long word = abort_flag ? 0ull : (unsigned long long)a.ep_call;
+#pragma unroll 1
+                    for (uint32_t p = 0; p < a.ep_world; ++p)
+                        asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(a.flag_peer[p] + a.ep_rank), "l"(word) : "memory");
+                }
+            }
+        }
+    }
+}
+
+constexpr int kMaxDevices = 64;
+
+}  // namespace
+
+// The dynamic shared memory the pair kernels may ask for on the current device (set once per device).
+size_t pair_dynamic_limit() {
+    static size_t limit[kMaxDevices] = {};
+    int dev = -1, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    if (limit[dev]) return limit[dev];
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    const void *const fns[] = {(const void *)k_block_pair<false, false>, (const void *)k_block_pair<false, true>,
+                               (const void *)k_block_pair<true, false>, (const void *)k_block_pair<true, true>};
+    size_t fixed = 0;
+    cudaFuncAttributes fa;
+    for (const void *fn : fns) {
+        if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
+        fixed = std::max(fixed, fa.sharedSizeBytes);
+    }
+    fixed = (fixed + 1023u) & ~(size_t)1023u;   // the ring starts on a 1 KB boundary behind the static part
+    if ((size_t)optin <= fixed) return 0;
+    const size_t most = (size_t)optin - fixed;
+    for (const void *fn : fns)
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
+    limit[dev] = most;
+    return most;
+}
+
+cudaError_t launch_pair_gemm(cudaStream_t st, int sm_count, bool down, bool official, GemmArgs args, uint32_t half, uint32_t *status) {
+    args.stage = kStageA + half * 2048u + 2u * ((half * 32u + 127u) / 128u) * kAtomBytes;
+    args.ring = std::min<uint32_t>((uint32_t)(pair_dynamic_limit() / args.stage), kPRingMax);
+    if (args.ring < 2u || half == 0u || 2u * half > kPGroups) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)args.ring * args.stage;
+    const dim3 grid((uint32_t)sm_count & ~1u), block(kPThreads);
+    if (down)
+        return official ? launch_pdl(k_block_pair<true, true>, grid, block, smem, st, 2u, args, half, status)
+                        : launch_pdl(k_block_pair<true, false>, grid, block, smem, st, 2u, args, half, status);
+    return official ? launch_pdl(k_block_pair<false, true>, grid, block, smem, st, 2u, args, half, status)
+                    : launch_pdl(k_block_pair<false, false>, grid, block, smem, st, 2u, args, half, status);
+}
+
+}  // namespace s14
