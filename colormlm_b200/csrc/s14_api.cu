@@ -1863,7 +1863,7 @@ extern "C" int32_t s14_block_create(s14_ctx *ctx, uint32_t hidden, uint32_t inte
     CUDA_OK(cudaMalloc((void **)&blk->w.hdig, P * (inter >> 8) * 2048u));
     CUDA_OK(cudaMalloc((void **)&blk->w.hexp, P * (inter >> 5)));
     CUDA_OK(cudaMalloc((void **)&blk->w.d, P * hidden * sizeof(float)));
-    // the pairs' hidden values as F32 (large blocks and the official arithmetic); zero, so that the slot of a
+    // the pairs' hidden values as F32; zero, so that the slot of a
     // pair without a route always holds a finite value
     CUDA_OK(cudaMalloc((void **)&blk->w.hval, P * inter * sizeof(float)));
     CUDA_OK(cudaMemset(blk->w.hval, 0, P * inter * sizeof(float)));
@@ -1888,7 +1888,7 @@ static int32_t block_launch(s14_block *blk, cudaStream_t st, const float *x, flo
     s14_ctx *ctx = blk->ctx;
     cudaError_t err;
     ctx->launches += launch_moe_block(st, ctx->sm_count, blk->w, x, y, ids, weights, pages, page_table, shared_page, n_tokens,
-                                      top_k, n_experts, blk->hidden, blk->inter, ctx->status, &err, 0, blk->residual, 0, 1, nullptr,
+                                      top_k, n_experts, blk->hidden, blk->inter, ctx->status, &err, blk->residual, 0, 1, nullptr,
                                       nullptr, false, blk->official);
     ctx->last_path = S14_LAYER_PATH_TENSOR_BLOCK;
     if (err != cudaSuccess) return cuda_fail(err, "S14 MoE block launch");
@@ -2013,7 +2013,7 @@ extern "C" int32_t s14_cmd_routed_moe_block_experts_ep(s14_ctx *ctx, void *strea
     cudaError_t err;
     ctx->launches += launch_moe_block(st, ctx->sm_count, blk->w, rd.x, nullptr, rd.ids_out, rd.weights_out, nullptr, desc->page_table,
                                       (by_token || shared_owner == ep_rank) ? desc->shared_page : nullptr, rd.n_tokens, rd.top_k,
-                                      rd.n_experts, blk->hidden, blk->inter, ctx->status, &err, 0, false, ep_rank, ep_world, pairs_out,
+                                      rd.n_experts, blk->hidden, blk->inter, ctx->status, &err, false, ep_rank, ep_world, pairs_out,
                                       nullptr, by_token);
     ctx->last_path = S14_LAYER_PATH_TENSOR_BLOCK;
     if (err != cudaSuccess) return cuda_fail(err, "S14 MoE block launch");
@@ -2141,7 +2141,7 @@ extern "C" int32_t s14_cmd_routed_moe_block_ep(s14_ctx *ctx, void *stream, s14_b
     cudaError_t err;
     ctx->launches += launch_moe_block(st, ctx->sm_count, blk->w, rd.x, nullptr, rd.ids_out, rd.weights_out, nullptr, desc->page_table,
                                       (by_token || shared_owner == blk->ep.rank) ? desc->shared_page : nullptr, rd.n_tokens, rd.top_k,
-                                      rd.n_experts, blk->hidden, blk->inter, ctx->status, &err, 0, false, blk->ep.rank, blk->ep.world,
+                                      rd.n_experts, blk->hidden, blk->inter, ctx->status, &err, false, blk->ep.rank, blk->ep.world,
                                       ep.pairs_peer[blk->ep.rank], &ep, by_token);
     ctx->last_path = S14_LAYER_PATH_TENSOR_BLOCK;
     if (err != cudaSuccess) return cuda_fail(err, "S14 MoE block launch");

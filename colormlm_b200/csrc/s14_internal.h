@@ -185,8 +185,8 @@ cudaError_t launch_greedy_argmax(cudaStream_t st, const float *logits, uint32_t 
 cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float *fn, const float *scale, const float *base,
                              const float *norm_weight, uint32_t hidden, float norm_eps, float hc_eps, float *x_out);
 
-// ---- a block of tokens through one layer, grouped by expert (s14_moe_block.cu) ----
-constexpr uint32_t kBlockNt = 24;  // most tokens of one chunk (two MMAs of N = 96: eight digit rows per token at least)
+// ---- a block of tokens through one layer, grouped by expert (s14_moe_block.cu, s14_moe_pair.cu) ----
+constexpr uint32_t kBlockNt = 24;  // most tokens of one chunk (N = 192: eight digit rows per token at least)
 // Up to kBlockNt (token, route) pairs that share an expert page.  The chunks of one expert follow
 // one another: c0 is the first of them, nch their number.
 struct BlockChunk {
@@ -200,11 +200,11 @@ struct BlockChunk {
 // Device workspace of a block object, sized for max_tokens at creation.
 struct BlockWork {
     BlockChunk *chunks;
-    uint32_t *counts;          // [0] chunks, [1] up items, [2] down items, [3] an expert id was out of range
+    uint32_t *counts;          // [0] chunks, [1], [2] chunks x slices, row tiles (above twelve tokens pairs of them), [3] an expert id was out of range
     uint8_t *xdig, *xexp;      // the tokens' digit tiles and block exponents
     uint8_t *hdig, *hexp;      // the pairs' hidden values likewise
     float *d;                  // the pairs' expert outputs [pair, hidden]
-    float *hval;               // official arithmetic: the pairs' weighted hidden values [pair, inter] (NULL until asked for)
+    float *hval;               // the pairs' hidden values [pair, inter] (official arithmetic: BF16 values, times the route weight)
 };
 // Expert-parallel exchange of the block kernels over peer memory: every rank holds two pair buffers
 // [pairs, hidden] F32 (calls alternate between them) and, per buffer, one 8-byte word per rank: the number
@@ -228,7 +228,7 @@ size_t moe_block_max_chunks(uint32_t max_tokens);
 int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const float *x, float *y, const int32_t *ids,
                      const float *weights, const uint8_t *const *pages, const uint8_t *const *page_table,
                      const uint8_t *shared_page, uint32_t n_tokens, uint32_t top_k, uint32_t n_experts, uint32_t hidden,
-                     uint32_t inter, uint32_t *status, cudaError_t *err, uint32_t nt_cap = 0, bool residual = false,
+                     uint32_t inter, uint32_t *status, cudaError_t *err, bool residual = false,
                      uint32_t ep_rank = 0, uint32_t ep_world = 1, float *pairs_out = nullptr, const BlockEp *ep = nullptr,
                      bool shared_by_token = false, bool official = false);
 // With pairs_out (expert parallel: rank ep_rank of ep_world computes the experts e with e mod world == rank) the

@@ -1,5 +1,5 @@
-// What the two contraction kernels of the grouped block path share: s14_moe_block.cu (one CTA per item) and
-// s14_moe_pair.cu (a pair of CTAs per item).
+// What the files of the grouped block path share: s14_moe_block.cu (digits, grouping, mix, the launches) and
+// s14_moe_pair.cu (the contraction kernels).
 #ifndef S14_MOE_BLOCK_CUH
 #define S14_MOE_BLOCK_CUH
 
@@ -11,20 +11,16 @@ constexpr uint32_t kStageA = kUnitStride;                  // a unit's codes, th
 static_assert(kStageA % 1024u == 0u, "operand tiles keep the 1 KB alignment of the 128-byte swizzle");
 constexpr uint32_t kPairsPerToken = S14_EXPERTS_PER_TOKEN + 1;   // pair = token * 7 + position in the mix (6: shared)
 
-// What the up kernel's epilogue leaves (the down kernel: kModeOfficial rounds its rows to BF16, the others do not)
-constexpr uint32_t kModeFused = 0u;      // the digit rows of the hidden values, laid out by the epilogue itself (small blocks)
-constexpr uint32_t kModeOfficial = 1u;   // the official arithmetic's BF16 hidden values, times the route weight
-constexpr uint32_t kModeValues = 2u;     // the F32 hidden values; a digits launch follows (large blocks)
-
 struct GemmArgs {
     const BlockChunk *chunks;
-    const uint32_t *n_items;    // device memory: written by the grouping kernel (chunks x slices or row tiles)
-    const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048]
+    const uint32_t *n_chunks;   // device memory: written by the grouping kernel
+    const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048; official arithmetic: 1024]
     const uint8_t *exps;        // their block exponents + 100, [vector][K / 32]
+    float *hval;                // up: the pairs' hidden values [pair][inter] (official: BF16 values, times the route weight)
+    const float *weights;       // up, official arithmetic: the routes' weights [token][top_k]
     float *out;                 // down: the pairs' expert outputs [pair][hidden]
-    uint8_t *hdig, *hexp;       // up: digit tiles and exponents of the pairs' hidden values
-    uint32_t by_threads;        // the token tiles come by the tile threads' own copies (large blocks), else by bulk copies
-    uint32_t hidden, inter, ring, stage;   // stage: bytes of a ring stage (a unit and nt_cap token tiles)
+    uint32_t hidden, inter, top_k;
+    uint32_t ring, stage;       // stages, bytes of a stage (set by launch_pair_gemm)
     // Expert parallel with the exchange inside the kernel: the pairs' outputs go into every rank's buffer
     // (plain stores to peer memory), and the last CTA to finish tells every rank that this rank's rows of
     // call `ep_call` are there (flags[rank] of the call's parity in every rank's buffer).
@@ -32,11 +28,6 @@ struct GemmArgs {
     unsigned long long *flag_peer[kMaxEpWorld];
     unsigned int *ep_counter;   // this GPU's arrival counter, zero at rest
     uint32_t ep_world, ep_rank, ep_call;
-    // Up kernel, kModeOfficial / kModeValues: the pairs' hidden values [pair][inter] (official: weighted and
-    // BF16-valued) and, for the official arithmetic, the routes' weights [token][top_k]
-    float *hval;
-    const float *weights;
-    uint32_t top_k;
 };
 
 // The pair kernels (s14_moe_pair.cu): chunks of up to 2 * `half` groups of sixteen digit rows, two row tiles (slices) per item.

@@ -1,7 +1,7 @@
-// The contraction kernels of the grouped block path for blocks of more than twelve tokens: a PAIR of CTAs (a cluster of
-// two, the two SMs of a TPC) works on an item together, tcgen05.mma.cta_group::2.  What they compute is described in
-// s14_moe_block.cu; per item it is a chunk of up to twelve groups of sixteen digit rows (one token each, official
-// arithmetic: two) times 256 rows of an expert: two slices of the up projection or two row tiles of w2.
+// The contraction kernels of the grouped block path: a PAIR of CTAs (a cluster of two, the two SMs of a TPC) works on an
+// item together, tcgen05.mma.cta_group::2.  What they compute is described in s14_moe_block.cu; per item it is a chunk
+// of up to twelve groups of sixteen digit rows (one token each, official arithmetic: two) times 256 rows of an expert:
+// two slices of the up projection or two row tiles of w2.
 //
 // Each CTA brings its own 128 rows of the page (a unit of 17 KB per step of 256 k) and HALF of the chunk's digit tiles; the
 // pair's tensor cores read both halves, so a step costs an SM 17 + 12 KB instead of 17 + 24, one MMA does N = 192
@@ -9,7 +9,9 @@
 // item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
 // (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
 // epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 506 / 294
-// us, now 427 / 204; 1000 tokens of the official arithmetic 1206 / 443, now 730 / 309.
+// us, now 427 / 204; 1000 tokens of the official arithmetic 1206 / 443, now 730 / 309.  Small blocks, which took one row tile
+// and two tokens per SM with stages of 21 KB in a ring of eight and laid out the hidden values' digit rows in the up epilogue:
+// 8 tokens 117 us for the call, now 109.
 //
 // What bounds it.  A step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles, the issuing
 // warp's round 470, a step 600-700 on average.  A second warp that copies the codes ahead gets a probe to 389 cycles a
@@ -86,6 +88,23 @@ __device__ __forceinline__ void pair_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
                  "h"((uint16_t)3)
                  : "memory");
+}
+// Whether the phase is complete, without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.b32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// mbar_wait_warp with a test in front, 55 cycles where a try costs 83: most waits of a full pipeline are over when they begin.
+// (Not in the one-token layer kernel, whose waits are for the memory: a stack of 14 layers 348 us, with the test 360.)
+__device__ __forceinline__ bool stage_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, mbar_test(bar, parity) || mbar_wait(bar, parity, abort_flag));
 }
 // M = 256: 128 rows in each CTA
 __device__ __forceinline__ constexpr uint32_t pair_idesc(uint32_t n) {
@@ -229,8 +248,10 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
     fence_after();
     const uint32_t tmem = tmem_slot;
     dependency_wait();
-    const uint32_t n_items = __ldcg(a.n_items);
     const uint32_t R = (kDown ? (a.hidden >> 7) : (a.inter >> 6)) / 2u;   // items per chunk
+    // The pair's items are q = me, me + n_pairs, ...  The chunks of one expert follow one another and so do their items, a row
+    // tile's chunks side by side (so that pairs that run at the same time share the expert's units in the L2).
+    const uint32_t n_items = __ldcg(a.n_chunks) * R;
     const uint32_t n_local = n_items > me ? (n_items - me + n_pairs - 1u) / n_pairs : 0u;
 
     // what the roles carry from batch to batch
@@ -295,7 +316,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll 1
                 for (uint32_t u = 0; u < nu; ++u, src += bytes) {
                     if ((slot & (kPProds - 1u)) == warp - kPProdWarp0) {
-                        ok = !round || mbar_wait_warp(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
+                        ok = !round || stage_wait(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
                         if (!ok) break;
                         const uint32_t full = bar(kPBarFull + slot), dst = to + slot * stage;
                         if (is_unit) {
@@ -320,14 +341,14 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                 for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
                     const uint32_t buf = gi & 1u, nt = warp_uniform(s_rec[i].nt & 0xFFu);
                     const uint32_t n = 32u * (((nt + kTpg - 1u) / kTpg + 1u) >> 1), idesc = pair_idesc(n);
-                    if (gi >= 2u) ok = mbar_wait_warp(bar(kPBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
+                    if (gi >= 2u) ok = stage_wait(bar(kPBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
                     if (!ok) break;
                     fence_after();
                     const uint32_t acc = tm + buf * kPCols;
                     const bool two = n > 128u;   // two scale atoms per 128 k
 #pragma unroll 1
                     for (uint32_t ku = 0; ku < nu; ++ku) {
-                        ok = mbar_wait_warp(bar(kPBarFull + slot), round & 1u, abortp);
+                        ok = stage_wait(bar(kPBarFull + slot), round & 1u, abortp);
                         if (!ok) break;
                         fence_after();
                         if (elect_one()) {
@@ -361,7 +382,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                 // ---- the second CTA's stages are complete (every writer has made its bytes visible to the tensor cores) ----
 #pragma unroll 1
                 for (uint32_t i = 0; i < nb * nu && ok; ++i) {
-                    ok = mbar_wait_warp(bar(kPBarFull + slot), round & 1u, abortp);
+                    ok = stage_wait(bar(kPBarFull + slot), round & 1u, abortp);
                     if (!ok) break;
                     if (elect_one()) mbar_arrive_remote(first_cta(bar(kPBarFull + slot)));
                     __syncwarp();
@@ -510,7 +531,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll
                     for (uint32_t k = 0; k < 8u; ++k) {
                         if (u0 + k < nu && ok) {
-                            ok = !round || mbar_wait_warp(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
+                            ok = !round || stage_wait(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
                             if (ok) {
                                 if (has_row) {
                                     uint8_t *const s = smem + slot * stage + code_at;

@@ -47,18 +47,6 @@ __device__ __forceinline__ unsigned long long l2_policy_evict_first() {
 __device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
-// Whether the phase is complete, without waiting.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.b32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // One bounded hardware wait: returns when the phase completes or after about a microsecond.  (The limit as an immediate:
 // in a register it costs a warp 348 cycles on a phase that is complete, so 83.)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -73,10 +61,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: false when the phase did not complete in kSpin tries (each suspends the thread
-// for a microsecond at most, so about 0.1 s) or another role gave up.  The test in front costs a warp 55 cycles, a lane 42
-// (a try 83 and 69): most waits of a full pipeline are over when they begin.
+// for a microsecond at most, so about 0.1 s) or another role gave up.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_test(bar, parity)) return true;
 #pragma unroll 1
     for (uint32_t i = 0; i < kSpin; ++i) {
         if (mbar_try(bar, parity)) return true;

@@ -566,7 +566,8 @@ S14_API int32_t s14_block_ep_set_wait_limit(s14_block *blk, uint32_t polls);
 S14_API int32_t s14_block_ep_disconnect(s14_block *blk);
 S14_API int32_t s14_cmd_routed_moe_block_ep(s14_ctx *ctx, void *stream, s14_block *blk, const s14_routed_layer_desc *desc,
                                             uint32_t shared_owner, int32_t wait_and_mix);
-/* After the stream is synchronised: the last call's number of chunks, up items, down items, and 1 if
+/* After the stream is synchronised: the last call's number of chunks, that times the slices of the up projection, times the
+ * row tiles of the down projection (in calls of more than twelve tokens: times the pairs of them), and 1 if
  * an expert id was outside the table (the call then wrote no result). */
 S14_API int32_t s14_block_last_counts(s14_block *blk, uint32_t counts_out[4]);
 

@@ -128,6 +128,29 @@ def test_block_sweep_of_block_sizes_against_the_one_token_kernel(ctx):
         blk.close()
 
 
+@pytest.mark.parametrize("n_tokens", [3, 14])
+def test_block_of_values_outside_the_range_of_the_f32_sums(ctx, n_tokens):
+    """The digit shares are added in F32 with constants made of the largest one; shares below 2^-79 or from 2^113 on, and
+    those of a token of zeros, take the sum in double.  Every token equals its own one-token call."""
+    hidden, inter, n_experts = 1024, 1024, 8
+    g, pages, shared = make_layer(1850, hidden, inter, n_experts, L.PAGE_MXFP4)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    blk = MoeBlock(ctx, hidden, inter, 16)
+    ctx.set_accumulation(L.ACCUM_PAIRWISE)
+    try:
+        x = synth.activations(g, n_tokens, hidden)
+        x[0] *= np.float32(2.0 ** -78)
+        x[1] *= np.float32(2.0 ** 112)
+        x[2] = 0.0
+        routes = random_routes(g, n_tokens, n_experts)
+        y = run_block(ctx, blk, x, pages_dev, shared_dev, routes)
+        for t in range(n_tokens):
+            single = run_layer(ctx, x[t:t + 1], pages_dev, shared_dev, [routes[t]], L.PAGE_MXFP4, hidden, inter)[0]
+            assert np.array_equal(single.view(np.uint32), y[t].view(np.uint32)), t
+    finally:
+        blk.close()
+
+
 def test_block_of_the_largest_size(ctx):
     """1024 tokens (the most a block object takes) over 16 experts: every expert has hundreds of tokens, and with
     64 slices per chunk a CTA of the up kernel holds some 260 items, i.e. walks three batches of item records;
