@@ -424,10 +424,18 @@ k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__res
     };
     if ((reinterpret_cast<uintptr_t>(logits) & 15u) == 0u) {
         const uint32_t n4 = vocab >> 2;
-#pragma unroll 4
-        for (uint32_t i = rank * kArgmaxThreads + tid; i < n4; i += n * kArgmaxThreads) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(logits) + i);
-            take(v.x, 4u * i), take(v.y, 4u * i + 1u), take(v.z, 4u * i + 2u), take(v.w, 4u * i + 3u);
+        // eight loads in flight, the last round's too (a loop unrolled by four read what was left one after the other: 129 280
+        // logits are 7.9 loads a thread; eight calls behind the logits of eight tokens: 222 us for all, now 214)
+        constexpr uint32_t kLoads = 8;
+        for (uint32_t i0 = rank * kArgmaxThreads + tid; i0 < n4; i0 += kLoads * n * kArgmaxThreads) {
+            float4 v[kLoads];
+#pragma unroll
+            for (uint32_t k = 0; k < kLoads; ++k)
+                if (const uint32_t i = i0 + k * n * kArgmaxThreads; i < n4) v[k] = __ldcg(reinterpret_cast<const float4 *>(logits) + i);
+#pragma unroll
+            for (uint32_t k = 0; k < kLoads; ++k)
+                if (const uint32_t i = i0 + k * n * kArgmaxThreads; i < n4)
+                    take(v[k].x, 4u * i), take(v[k].y, 4u * i + 1u), take(v[k].z, 4u * i + 2u), take(v[k].w, 4u * i + 3u);
         }
         if (rank == 0u && tid < (vocab & 3u)) take(__ldcg(logits + n4 * 4u + tid), n4 * 4u + tid);
     } else {
