@@ -68,10 +68,12 @@ __device__ __forceinline__ float e4m3fn_round(float v) {
 // 2458 -> 1894 us).
 template <bool kQuant>
 __global__ void __launch_bounds__(512)
-k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps) {
+k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early) {
     constexpr uint32_t kRows = kQuant ? 8u : 16u;
     const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
-    dependency_wait();
+    // early: the launch in front neither writes x nor uses what is written here (it picks the routes), and whatever is in front
+    // of it is complete when this kernel starts; so the work runs beside it, and the wait for it comes last
+    if (!early) dependency_wait();
     const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
     const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
     float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
@@ -91,6 +93,7 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
             xs[i] = __fmul_rn(e4m3fn_round(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f)), scale);
     }
     digits_of8<(int)kRows>(xs, g, dig + (size_t)v * (K >> 8) * (kRows * 128u), exps + (size_t)v * (K >> 5));
+    if (early) dependency_wait();
 }
 
 // Groups the block's (token, route) pairs by expert.  Group 0 is the shared expert (every token, mix
@@ -119,10 +122,15 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     }
     if (tid == 0) bad = 0u;
     __syncthreads();
-    for (uint32_t i = tid; i < n; i += blockDim.x) {
-        const int32_t e = __ldcg(ids + i);
-        if (e >= (int32_t)n_experts) bad = 1u;
-        else if (e >= 0 && (uint32_t)e % ep_world == ep_rank) atomicAdd(&cnt[1 + e], 1u);  // expert parallel: the experts this rank owns
+    // the thread's pairs i = tid, tid + 1024, ...; an id that makes no pair here is -1
+    int32_t mine_id[S14_EXPERTS_PER_TOKEN];   // (up to 1024 tokens)
+#pragma unroll
+    for (uint32_t k = 0; k < S14_EXPERTS_PER_TOKEN; ++k) mine_id[k] = tid + k * 1024u < n ? __ldcg(ids + tid + k * 1024u) : -1;
+#pragma unroll
+    for (uint32_t k = 0; k < S14_EXPERTS_PER_TOKEN; ++k) {
+        if (mine_id[k] >= (int32_t)n_experts) bad = 1u;
+        if (mine_id[k] >= (int32_t)n_experts || mine_id[k] < 0 || (uint32_t)mine_id[k] % ep_world != ep_rank) mine_id[k] = -1;
+        else atomicAdd(&cnt[1 + mine_id[k]], 1u);  // expert parallel: the experts this rank owns
     }
     // the shared expert's members: every token; expert parallel with the shared page on every rank: the tokens
     // t with t mod world == rank (its work is a fifth of a large block's: on one rank it would bound the scaling)
@@ -173,10 +181,10 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     }
     __syncthreads();
     if (bad) return;
-    for (uint32_t i = tid; i < n; i += blockDim.x) {
-        const int32_t e = __ldcg(ids + i);
-        if (e < 0 || (uint32_t)e % ep_world != ep_rank) continue;
-        const uint32_t g = 1u + (uint32_t)e, t = i / top_k, m = i - t * top_k;
+#pragma unroll
+    for (uint32_t kk = 0; kk < S14_EXPERTS_PER_TOKEN; ++kk) {
+        if (mine_id[kk] < 0) continue;
+        const uint32_t i = tid + kk * 1024u, g = 1u + (uint32_t)mine_id[kk], t = i / top_k, m = i - t * top_k;
         const uint32_t k = atomicAdd(&fill[g], 1u);
         if (k == 0u && !page_table) gpage[g] = __ldcg(reinterpret_cast<const unsigned long long *>(pages + i));
         BlockChunk *ch = chunks + chunk0[g] + k / size[g];
@@ -260,9 +268,11 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
     bool there[S14_EXPERTS_PER_TOKEN];
 #pragma unroll
     for (uint32_t m = 0; m < S14_EXPERTS_PER_TOKEN; ++m) {
+        // (a position without a route has a row of its own all the same, with whatever is left in it: the row's load need not
+        // wait for the id)
         there[m] = m < top_k && __ldcg(ids + t * top_k + m) >= 0;
-        w[m] = there[m] ? __ldcg(weights + t * top_k + m) : 0.0f;
-        row[m] = there[m] ? load4(dt + (size_t)m * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w[m] = m < top_k ? __ldcg(weights + t * top_k + m) : 0.0f;
+        row[m] = m < top_k ? load4(dt + (size_t)m * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     constexpr uint32_t kSh = S14_EXPERTS_PER_TOKEN;
     row[kSh] = has_shared ? load4(dt + (size_t)kSh * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -322,12 +332,14 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     const uint32_t S = inter >> 6, RT = hidden >> 7, counted = small ? 1u : 2u;   // slices, row tiles; as `counts` reports them
     // The launches are programmatic dependents of one another: a kernel's blocks, barriers and tensor memory are
     // set up while the one before runs out, and every kernel waits for it before it reads or writes anything.
-    auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps) {
+    auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps, bool early) {
         if (*err != cudaSuccess) return;
-        *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps);
+        *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps,
+                          early ? 1u : 0u);
     };
     *err = cudaSuccess;
-    digits(x, n_tokens, hidden, w.xdig, w.xexp);
+    // (in front of it: the router's launch, or the copies of the host's routes)
+    digits(x, n_tokens, hidden, w.xdig, w.xexp, true);
     if (ep_world == 0u) ep_world = 1u;
     if (*err == cudaSuccess)
         *err = launch_pdl(k_block_group, dim3(1), dim3(1024), 0, st, 0u, ids, pages, page_table, shared_page, n_tokens, top_k, n_experts,
@@ -367,7 +379,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     // elements for the official arithmetic) lays out the rows of all pairs' slots (a slot without a route holds
     // zeros or an earlier call's values: finite numbers nobody reads the rows of).
     *err = launch_pair_gemm(st, sm_count, false, official, up, groups / 2u, status);
-    digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp);
+    digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp, false);
     if (*err == cudaSuccess) *err = launch_pair_gemm(st, sm_count, true, official, down, groups / 2u, status);
     const int launches = 5;
     if (pairs_out || *err != cudaSuccess) return launches;
