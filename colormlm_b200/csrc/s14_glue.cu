@@ -533,7 +533,8 @@ cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y,
 // (partial sums of launch_hc_pre_many: eight slices of K for any number of tokens, or fewer than 2 * sm_count groups of
 // sixteen tokens times slices)
 size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count) {
-    return (size_t)std::max(8u * max_tokens, 32u * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
+    // a row per slice and token: up to sixteen slices, or fewer than two CTAs of sixteen tokens per SM (launch_hc_pre_many)
+    return (size_t)std::max(16u * max_tokens, 32u * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
 }
 
 // Whether all the addresses are multiples of 16 (rows of 256 and more elements keep that).
@@ -573,7 +574,13 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
     // slices of K: enough CTAs for the SMs, each warp's part whole steps of sixteen (n / 1024 is a whole number)
     const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden;
     uint32_t slices = 8u;
-    while (slices < 64u && groups * slices < (uint32_t)sm_count && (n / (slices * 2u * 8u)) % 16u == 0u) slices *= 2u;
+    auto twice = [&]() { return (n / (slices * 2u * 8u)) % 16u == 0u; };
+    while (slices < 64u && groups * slices < (uint32_t)sm_count && twice()) slices *= 2u;
+    // ... sixteen instead of eight where the last round of CTAs would leave a fifth of the SMs idle.  370 tokens of 4096: 192 CTAs
+    // 24.6 us for both launches and 39.0 with the norm and the expand behind them, 384 CTAs 22.3 and 31.5; 700: 33.4 and 46.4, now
+    // 30.1 and 42.9; 370 F32 tokens 25.4 and 42.4, 24.6 and 36.0.  (150 tokens at 32 slices: 17.3 and 23.1, 15.3 and 23.6.)
+    const uint32_t sms = (uint32_t)sm_count, ctas = groups * slices;
+    if (slices == 8u && ctas * 5u < ((ctas + sms - 1u) / sms) * sms * 4u && twice()) slices *= 2u;
     const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
     return launch_pdl(k_hc_reduce<kBf16, kHead, kBf16 ? 8 : 4>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,
