@@ -161,11 +161,6 @@ __device__ __forceinline__ void dependency_wait() {
 // to this kernel.
 __device__ __forceinline__ void l2_hint(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Asks the L2 for bytes of this GPU's memory that a later copy will read (size a multiple of 16).
-__device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-
 // The result of a launch.  A refused launch also stays behind as the thread's last error, where the next check of the
 // library, or of whoever shares the runtime with it, would find it and blame another call.
 inline cudaError_t launch_status(cudaError_t e) {

@@ -98,23 +98,11 @@ __device__ __forceinline__ void dot_rows(const uint4 (&qa)[P], const uint4 (&qb)
     vb = (float)warp_sum(b);
 }
 
-// `units` units of every page from `offset` on into the L2, a unit per warp in turn.  The matvecs are two kernels of 17 and 8 MB
-// that use half of the memory's rate at most, the layer kernel behind them streams 80 MB between hand-offs: with
-// the up projections asked for under the first and the down projections under the second the executor's step takes 38.4 us,
-// without 39.2.
-__device__ __forceinline__ void fetch_next(const NextPages &next, size_t offset, uint32_t units) {
-    if ((threadIdx.x & 31u) != 0u) return;
-    for (uint32_t u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < next.n * units; u += gridDim.x * kF8Warps) {
-        const uint32_t e = u / units;
-        l2_prefetch(next.page[e] + offset + (size_t)(u - e * units) * kUnitStride, kUnitStride);
-    }
-}
-
 // h[i] = swiglu(w1[i] . x, w3[i] . x); x F32, or BF16 with its F32 values left in x_out for the layer kernel
 template <uint32_t P>
 __global__ void __launch_bounds__(kF8Threads, 1)
 k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16, float *__restrict__ x_out,
-                const uint8_t *__restrict__ page, float *__restrict__ h, uint32_t inter, const __grid_constant__ NextPages next) {
+                const uint8_t *__restrict__ page, float *__restrict__ h, uint32_t inter) {
     constexpr uint32_t hidden = P * 512u;
     __shared__ __align__(16) float sx[hidden];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, step = gridDim.x * kF8Warps;
@@ -137,7 +125,6 @@ k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16
     } else {
         stage_vector(sx, x, hidden);
     }
-    fetch_next(next, 0u, (uint32_t)mxfp4_up_units(hidden, inter));
     __syncthreads();
 #pragma unroll 1
     while (row < inter) {
@@ -156,8 +143,7 @@ k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16
 // d[n] = w2[n] . h
 template <uint32_t P>
 __global__ void __launch_bounds__(kF8Threads, 1)
-k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, float *__restrict__ d, uint32_t hidden,
-                  const __grid_constant__ NextPages next) {
+k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, float *__restrict__ d, uint32_t hidden) {
     constexpr uint32_t inter = P * 512u;
     __shared__ __align__(16) float sx[inter];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, step = gridDim.x * kF8Warps;
@@ -170,7 +156,6 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
     if (row < hidden) load_row<P>(qa, pv.w2 + (size_t)row * inter, lane);
     if (row + step < hidden) load_row<P>(qb, pv.w2 + (size_t)(row + step) * inter, lane);
     stage_vector(sx, h, inter);
-    fetch_next(next, mxfp4_down_offset(hidden, inter), (uint32_t)mxfp4_down_units(hidden, inter));
     __syncthreads();
 #pragma unroll 1
     while (row < hidden) {
@@ -186,19 +171,19 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
 }  // namespace
 
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,
-                              float *h, float *d, uint32_t hidden, uint32_t inter, const NextPages &next) {
+                              float *h, float *d, uint32_t hidden, uint32_t inter) {
     const dim3 grid(sm_count), block(kF8Threads);
     cudaError_t e;
     switch (hidden >> 9) {
-    case 2: e = launch_pdl(k_fp8_expert_up<2>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter, next); break;
-    case 4: e = launch_pdl(k_fp8_expert_up<4>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter, next); break;
-    default: e = launch_pdl(k_fp8_expert_up<8>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter, next); break;
+    case 2: e = launch_pdl(k_fp8_expert_up<2>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter); break;
+    case 4: e = launch_pdl(k_fp8_expert_up<4>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter); break;
+    default: e = launch_pdl(k_fp8_expert_up<8>, grid, block, 0, st, 0u, x, x_bf16, x_out, page, h, inter); break;
     }
     if (e != cudaSuccess) return e;
     switch (inter >> 9) {
-    case 2: return launch_pdl(k_fp8_expert_down<2>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden, next);
-    case 4: return launch_pdl(k_fp8_expert_down<4>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden, next);
-    default: return launch_pdl(k_fp8_expert_down<8>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden, next);
+    case 2: return launch_pdl(k_fp8_expert_down<2>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden);
+    case 4: return launch_pdl(k_fp8_expert_down<4>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden);
+    default: return launch_pdl(k_fp8_expert_down<8>, grid, block, 0, st, 0u, page, (const float *)h, d, hidden);
     }
 }
 

@@ -134,13 +134,8 @@ int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &route
 // h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary, x_bf16
 // (or NULL) on an 8-byte one.
 inline bool fp8_expert_takes(const uint16_t *x_bf16) { return (reinterpret_cast<uintptr_t>(x_bf16) & 7u) == 0u; }
-// `next`: MXFP4 pages of the same sizes that the launch behind reads; these kernels ask the L2 for them.
-struct NextPages {
-    const uint8_t *page[S14_EXPERTS_PER_TOKEN];
-    uint32_t n;
-};
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,
-                              float *h, float *d, uint32_t hidden, uint32_t inter, const NextPages &next);
+                              float *h, float *d, uint32_t hidden, uint32_t inter);
 // Scratch of the tcgen05 layer kernel (s14_moe_umma.cu): per job the digit tile of its hidden
 // values and the tile's block exponents (umma_scratch_bytes), and the device status word a
 // timed-out wait sets.

@@ -1287,10 +1287,7 @@ int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &route
                             const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
                             unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err) {
     float *shared_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
-    NextPages next = {};   // (with a router nobody knows them yet)
-    for (uint32_t j = 0; j < routed.n_jobs && next.n < S14_EXPERTS_PER_TOKEN; ++j)
-        if (routed.jobs[j].kind == S14_PAGE_MXFP4) next.page[next.n++] = routed.jobs[j].page;
-    *err = launch_fp8_expert(st, sm_count, x, x_bf16, x_stage, shared_page, h, shared_out, hidden, inter, next);
+    *err = launch_fp8_expert(st, sm_count, x, x_bf16, x_stage, shared_page, h, shared_out, hidden, inter);
     if (*err != cudaSuccess) return 0;
     *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, y, umma->tiles, counters, umma->status, hidden, inter, router,
                                  nullptr, umma->trace, nullptr, 1, nullptr, false, shared_out);

@@ -43,6 +43,10 @@ __device__ __forceinline__ unsigned long long l2_policy_evict_first() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
+// Asks the L2 for bytes of this GPU's memory that a later copy will read (size a multiple of 16).
+__device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // One bounded hardware wait: returns when the phase completes or after about a microsecond.  (The limit as an immediate:
 // in a register it costs a warp 348 cycles on a phase that is complete, so 83.)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
