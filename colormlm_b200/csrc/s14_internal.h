@@ -193,7 +193,6 @@ struct BlockChunk {
     const uint8_t *page;
     uint32_t nt;               // pairs in the chunk
     uint32_t c0, nch;
-    uint32_t tok[kBlockNt];    // the pairs' tokens (rows of x)
     uint32_t pair[kBlockNt];   // token * 7 + position in the mix (6: the shared expert)
     uint32_t pad;
 };

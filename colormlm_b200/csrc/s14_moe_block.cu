@@ -188,14 +188,12 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
         const uint32_t k = atomicAdd(&fill[g], 1u);
         if (k == 0u && !page_table) gpage[g] = __ldcg(reinterpret_cast<const unsigned long long *>(pages + i));
         BlockChunk *ch = chunks + chunk0[g] + k / size[g];
-        ch->tok[k % size[g]] = t;
         ch->pair[k % size[g]] = t * kPairsPerToken + m;
     }
     if (shared_page) {
         for (uint32_t k = tid; sh_first + k * sh_step < T; k += blockDim.x) {
             const uint32_t t = sh_first + k * sh_step;
             BlockChunk *ch = chunks + chunk0[0] + k / size[0];
-            ch->tok[k % size[0]] = t;
             ch->pair[k % size[0]] = t * kPairsPerToken + S14_EXPERTS_PER_TOKEN;
         }
     }
