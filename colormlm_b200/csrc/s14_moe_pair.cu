@@ -598,31 +598,31 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
         if (abort_flag) break;
     }
     if (warp == kPMmaWarp && rank == 0u) {
-        // nothing of the pair's tensor work is in flight when the tensor memory is freed
+        // All of the pair's tensor operations are complete before either CTA frees its tensor memory or leaves, also when a role
+        // has given up with stages queued: they read both CTAs' shared memory and write both CTAs' tensor memory.
         if (elect_one()) pair_commit(bar(kPBarFin));
         __syncwarp();
+        mbar_drain(bar(kPBarFin), 0);
     }
-    // ... which also arrives at the other CTA, behind the stages' arrivals
-    if (warp == kPMmaWarp) mbar_wait_warp(bar(kPBarFin), 0, abortp);
     if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds && lane == 0) {
         // copies in flight land in this CTA's shared memory, arrivals of the tensor operations at its barriers: wait for them
 #pragma unroll 1
         for (uint32_t s = warp - kPProdWarp0; s < ring; s += kPProds) {
             const uint32_t used = round + (s < slot ? 1u : 0u);   // rounds of this slot
-            uint32_t tries = 0;
-            if (used) {
-#pragma unroll 1
-                while (!mbar_try(bar((abort_flag ? kPBarFull : kPBarDone) + s), (used - 1u) & 1u) && ++tries < kSpin) {
-                }
-            }
+            if (used) mbar_drain(bar((abort_flag ? kPBarFull : kPBarDone) + s), (used - 1u) & 1u);
         }
     }
     fence_before();
     __syncwarp();
     __syncthreads();
     cluster_barrier();
-    if (warp == kPMmaWarp)
+    if (warp == kPMmaWarp) {
+        // the last commit also arrives in the second CTA, behind the stages' arrivals: none of them is on its way when that
+        // CTA leaves (behind the cluster barrier, because the first CTA may give up a wait's length after the second)
+        if (rank != 0u) mbar_drain(bar(kPBarFin), 0);
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
+    }
     if (tid == 0 && abort_flag) atomicExch(status, 0x5507u);
     if constexpr (kDown && !kOff) {
         if (a.ep_world > 1u) {

@@ -1176,11 +1176,11 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             gi0 += n_items;
         }
         if (warp_u == kMmaWarp0 || warp_u == kMmaWarp0 + 1u) {
-            // nothing of this CTA's tensor work is in flight when the tensor memory is freed
+            // nothing of this CTA's tensor work is in flight when the tensor memory is freed, also when a role has given up
             __syncwarp();
             if (elect_one()) umma_commit(bar(kBarFin));
             __syncwarp();
-            mbar_wait_warp(bar(kBarFin), 0, abortp);
+            mbar_drain(bar(kBarFin), 0);
         }
     }
     if constexpr (kTrace) tr = trace_base();
@@ -1193,10 +1193,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
 #pragma unroll 1
         for (uint32_t u = first; u < p_units; ++u) {
             const uint32_t s = u % ring, parity = (u / ring) & 1u;
-            uint32_t tries = 0;
-#pragma unroll 1
-            while (!mbar_try(bar(kBarFull + s), parity) && ++tries < kSpin) {
-            }
+            mbar_drain(bar(kBarFull + s), parity);
         }
     }
     fence_before();

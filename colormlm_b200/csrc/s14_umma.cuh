@@ -75,6 +75,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
+// Waits of a CTA that leaves, for what is still in flight into its memories: bounded as well, but they go on when a role has
+// given up, which is when there is most of it.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpin && !mbar_try(bar, parity); ++i) {
+    }
+}
 // One lane of a converged warp, always the same.  The issuing warps run their loops with all lanes on values that are
 // the same in all of them, and only the tcgen05 operations sit behind this: their descriptors and addresses can then
 // live in uniform registers, where a lane that runs the loop alone has to move every operand of every operation
