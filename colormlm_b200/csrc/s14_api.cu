@@ -1881,7 +1881,6 @@ extern "C" int32_t s14_block_create(s14_ctx *ctx, uint32_t hidden, uint32_t inte
     return S14_OK;
 }
 
-// After the stream is synchronised: counts[3] of the last call (an expert id outside the table).
 static int32_t block_launch(s14_block *blk, cudaStream_t st, const float *x, float *y, const int32_t *ids,
                             const float *weights, const uint8_t *const *pages, const uint8_t *const *page_table,
                             const uint8_t *shared_page, uint32_t n_tokens, uint32_t top_k, uint32_t n_experts) {
@@ -2189,8 +2188,8 @@ extern "C" int32_t s14_block_set_residual(s14_block *blk, int32_t residual) {
     return S14_OK;
 }
 
-// counts of the last call's grouping (after the stream is synchronised): chunks, up items, down
-// items, and 1 if an expert id was outside the table (the call then did nothing).
+// counts of the last call (after the stream is synchronised): chunks, that times slices, row tiles, and why the call
+// wrote no result (0: it did).
 extern "C" int32_t s14_block_last_counts(s14_block *blk, uint32_t counts_out[4]) {
     if (!blk || !counts_out) return fail(S14_ERR_CONTRACT, "s14_block_last_counts: NULL argument");
     CUDA_OK(cudaSetDevice(blk->device));

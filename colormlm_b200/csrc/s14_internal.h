@@ -196,10 +196,13 @@ struct BlockChunk {
     uint32_t pair[kBlockNt];   // token * 7 + position in the mix (6: the shared expert)
     uint32_t pad;
 };
+constexpr uint32_t kBlockBadId = 1;   // an expert id was out of range
+constexpr uint32_t kBlockGaveUp = 2;  // a wait inside a contraction kernel ran out
 // Device workspace of a block object, sized for max_tokens at creation.
 struct BlockWork {
     BlockChunk *chunks;
-    uint32_t *counts;          // [0] chunks, [1], [2] chunks x slices, row tiles (above twelve tokens pairs of them), [3] an expert id was out of range
+    uint32_t *counts;          // [0] chunks, [1], [2] chunks x slices, row tiles (above twelve tokens pairs of them), [3] why the call writes
+                               // no result: kBlockBadId, kBlockGaveUp (set anew by every call's grouping)
     uint8_t *xdig, *xexp;      // the tokens' digit tiles and block exponents
     uint8_t *hdig, *hexp;      // the pairs' hidden values likewise
     float *d;                  // the pairs' expert outputs [pair, hidden]
@@ -208,7 +211,8 @@ struct BlockWork {
 // Expert-parallel exchange of the block kernels over peer memory: every rank holds two pair buffers
 // [pairs, hidden] F32 (calls alternate between them) and, per buffer, one 8-byte word per rank: the number
 // of the last call whose rows that rank has written there.  The down kernel stores the rows of the experts it
-// owns into every rank's buffer (plain stores to peer memory) and its last CTA publishes the call's number;
+// owns into every rank's buffer (plain stores to peer memory) and its last CTA publishes the call's number (0 where any CTA of
+// the call's contraction kernels gave up: its rows are not there);
 // the mix waits (bounded) until every rank's word says this call.  A rank writes call s + 1 only after its own
 // mix of call s, which waited for every rank's rows of call s; so a rank that writes into a buffer for call
 // s + 2 knows that every rank has finished reading call s from it: two buffers are enough.

@@ -101,8 +101,8 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
 // shared expert's in token order, a routed expert's in the order its members arrive: every pair's
 // result depends on that pair alone, so the order changes no bit of the output).  ids: [T, top_k]
 // expert ids, negative = no route.  The page of a routed group is page_table[e], or, with per-route
-// pages, the page of one of its members.  counts: [0] chunks, [1] up items, [2] down items, [3] 1 if
-// an id was out of range (then no chunk is made).  One CTA of 1024 threads.
+// pages, the page of one of its members.  counts: [0] chunks, [1], [2] that times S, RT, [3] kBlockBadId if
+// an id was out of range (then no chunk is made), else 0.  One CTA of 1024 threads.
 __global__ void __launch_bounds__(1024)
 k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict__ pages,
               const uint8_t *const *__restrict__ page_table, const uint8_t *shared_page, uint32_t T, uint32_t top_k,
@@ -176,7 +176,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
             counts[0] = c_all;
             counts[1] = c_all * S;
             counts[2] = c_all * RT;
-            counts[3] = bad;
+            counts[3] = bad ? kBlockBadId : 0u;
         }
     }
     __syncthreads();
@@ -224,17 +224,21 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 __global__ void __launch_bounds__(256)
 k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const float *__restrict__ weights,
             uint32_t top_k, int has_shared, float *y, uint32_t hidden, const uint32_t *__restrict__ counts,
-            const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_world, uint32_t ep_call,
+            const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_rank, uint32_t ep_world, uint32_t ep_call,
             uint32_t wait_limit, uint32_t *status, uint32_t official, uint32_t vec) {
     const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * 4u, t = blockIdx.y;   // hidden is a multiple of four
     dependency_wait();
+    const uint32_t why = __ldcg(counts + 3);
     if (flags) {
         // expert parallel, exchange inside the kernels: every rank's rows of this call are in this rank's buffer
-        // when its flag carries the call's number (bounded wait: about a microsecond per poll)
+        // when its flag carries the call's number (bounded wait: about a microsecond per poll).  A rank that gave up has not
+        // published its own; it waits for the others all the same, because that is what tells it that they have read
+        // the buffer its next call but one writes.
         __shared__ int s_ok;
         if (threadIdx.x == 0) {
             int ok = 1;
             for (uint32_t p = 0; p < ep_world && ok; ++p) {
+                if (p == ep_rank && (why & kBlockGaveUp)) continue;
                 uint32_t tries = 0;
                 for (;;) {
                     unsigned long long v;
@@ -253,7 +257,7 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
         __syncthreads();
         if (!s_ok) return;
     }
-    if (n >= hidden || __ldcg(counts + 3)) return;
+    if (n >= hidden || why) return;
     const float *dt = d + (size_t)t * kPairsPerToken * hidden + n;
     // (a caller's buffers may lie on any 4-byte boundary)
     auto load4 = [&](const float *p) {
@@ -296,7 +300,7 @@ cudaError_t launch_mix(cudaStream_t st, const float *pairs, const int32_t *ids, 
     const uintptr_t where = (uintptr_t)pairs | (uintptr_t)y | (residual ? (uintptr_t)x : 0u);
     return launch_pdl(k_block_mix, dim3((hidden + 1023u) / 1024u, n_tokens), dim3(256), 0, st, 0u, pairs, ids, weights, top_k,
                       has_shared ? 1 : 0, y, hidden, counts, x, residual ? 1u : 0u,
-                      (const unsigned long long *)(ep ? ep->flags : nullptr), ep ? ep->world : 1u, ep ? ep->call : 0u,
+                      (const unsigned long long *)(ep ? ep->flags : nullptr), ep ? ep->rank : 0u, ep ? ep->world : 1u, ep ? ep->call : 0u,
                       ep ? ep->wait_limit : 0u, status, official ? 1u : 0u, (where & 15u) ? 0u : 1u);
 }
 
@@ -352,6 +356,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     GemmArgs up = {}, down = {};
     up.chunks = down.chunks = w.chunks;
     up.n_chunks = down.n_chunks = w.counts;
+    up.why = down.why = w.counts + 3;
     up.hidden = down.hidden = hidden;
     up.inter = down.inter = inter;
     up.dig = w.xdig;

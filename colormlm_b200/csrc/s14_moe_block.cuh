@@ -14,6 +14,7 @@ constexpr uint32_t kPairsPerToken = S14_EXPERTS_PER_TOKEN + 1;   // pair = token
 struct GemmArgs {
     const BlockChunk *chunks;
     const uint32_t *n_chunks;   // device memory: written by the grouping kernel
+    uint32_t *why;              // the call's counts[3]: kBlockGaveUp is added by a CTA that gives up
     const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048; official arithmetic: 1024]
     const uint8_t *exps;        // their block exponents + 100, [vector][K / 32]
     float *hval;                // up: the pairs' hidden values [pair][inter] (official: BF16 values, times the route weight)
@@ -23,7 +24,7 @@ struct GemmArgs {
     uint32_t ring, stage;       // stages, bytes of a stage (set by launch_pair_gemm)
     // Expert parallel with the exchange inside the kernel: the pairs' outputs go into every rank's buffer
     // (plain stores to peer memory), and the last CTA to finish tells every rank that this rank's rows of
-    // call `ep_call` are there (flags[rank] of the call's parity in every rank's buffer).
+    // call `ep_call` are there (flags[rank] of the call's parity in every rank's buffer), unless one of the call's CTAs gave up.
     float *out_peer[kMaxEpWorld];
     unsigned long long *flag_peer[kMaxEpWorld];
     unsigned int *ep_counter;   // this GPU's arrival counter, zero at rest

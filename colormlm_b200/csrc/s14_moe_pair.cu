@@ -623,11 +623,14 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
     }
-    if (tid == 0 && abort_flag) atomicExch(status, 0x5507u);
+    if (tid == 0 && abort_flag) {
+        atomicExch(status, 0x5507u);
+        atomicOr(a.why, kBlockGaveUp);
+    }
     if constexpr (kDown && !kOff) {
         if (a.ep_world > 1u) {
-            // every store of this CTA to the peers' buffers is ordered before the count; the last CTA of the
-            // grid publishes the call's number to every rank
+            // every store of this CTA to the peers' buffers, and that it gave up, is ordered before the count; the last CTA of
+            // the grid publishes the call's number to every rank, or 0 where a CTA of this kernel or of the up kernel gave up
             if (warp < kPEpi / 32u) __threadfence_system();
             __syncthreads();
             if (tid == 0) {
@@ -635,7 +638,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                 if (atomicAdd(a.ep_counter, 1u) == gridDim.x - 1u) {
                     *a.ep_counter = 0u;
                     __threadfence_system();
-                    const unsigned long long word = abort_flag ? 0ull : (unsigned long long)a.ep_call;
+                    const unsigned long long word = (atomicOr(a.why, 0u) & kBlockGaveUp) ? 0ull : (unsigned long long)a.ep_call;
 #pragma unroll 1
                     for (uint32_t p = 0; p < a.ep_world; ++p)
                         asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(a.flag_peer[p] + a.ep_rank), "l"(word) : "memory");

@@ -606,7 +606,8 @@ class MoeBlock:
         check(L.lib().s14_block_set_semantics(self._h, 1 if official else 0))
 
     def last_counts(self):
-        """(chunks, up items, down items, bad id flag) of the last call; synchronise the stream first."""
+        """Of the last call: chunks, that times slices and times row tiles (above twelve tokens: pairs of them), and why it wrote no
+        result (0: it did; 1: an expert id outside the table; 2: a wait inside a kernel ran out).  Synchronise the stream first."""
         out = (C.c_uint32 * 4)()
         check(L.lib().s14_block_last_counts(self._h, out))
         return tuple(int(v) for v in out)

@@ -552,7 +552,8 @@ S14_API int32_t s14_cmd_moe_block_mix(s14_ctx *ctx, void *stream, s14_block *blk
  * stores to peer memory over NVLink) and its last CTA publishes the call's number to every rank (one
  * 8-byte word per rank and buffer); the mix waits - bounded, about a microsecond per poll, default 2^22
  * polls; a wait that runs out sets the device status word 0x5508 and writes no y - until every rank's
- * word carries this call's number.  A rank writes call s + 1 only after its own mix of call s, which
+ * word carries this call's number.  A rank one of whose kernels gave up (status 0x5507 there) does not
+ * publish the call: it writes no y, and the others' waits run out.  A rank writes call s + 1 only after its own mix of call s, which
  * waited for every rank, so two buffers are enough.  Every rank issues the same sequence of calls; y
  * is bit-identical to the single-GPU block on every rank.
  *   create / connect / connect_local / disconnect: as s14_ep_exchange_* (connect_local: the ranks are
@@ -567,8 +568,8 @@ S14_API int32_t s14_block_ep_disconnect(s14_block *blk);
 S14_API int32_t s14_cmd_routed_moe_block_ep(s14_ctx *ctx, void *stream, s14_block *blk, const s14_routed_layer_desc *desc,
                                             uint32_t shared_owner, int32_t wait_and_mix);
 /* After the stream is synchronised: the last call's number of chunks, that times the slices of the up projection, times the
- * row tiles of the down projection (in calls of more than twelve tokens: times the pairs of them), and 1 if
- * an expert id was outside the table (the call then wrote no result). */
+ * row tiles of the down projection (in calls of more than twelve tokens: times the pairs of them), and why the call
+ * wrote no result: 0 it did, 1 an expert id was outside the table, 2 a wait inside a kernel ran out (status 0x5507). */
 S14_API int32_t s14_block_last_counts(s14_block *blk, uint32_t counts_out[4]);
 
 /* ---- the steps on either side of the MoE inside one layer ------------------------------------

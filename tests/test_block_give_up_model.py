@@ -44,3 +44,34 @@ def test_a_pair_that_gave_up_leaves_behind_its_tensor_work():
 def test_a_wait_that_ends_with_the_flag_would_leave_work_in_flight():
     rng = random.Random(7)
     assert not all(sound(leave(rng, drain=False)) for _ in range(20_000))
+
+
+# ---- publishing ----
+# A rank's call is two contraction kernels, every CTA of which may give up; a CTA that did has not stored its rows (down) or the
+# hidden values they are made of (up).  The CTAs of the second kernel count themselves in, in any order, and the last one publishes.
+
+
+def publish(rng, n_ctas, call, up_gave_up, down_gave_up, by_word, word):
+    """The number the last CTA publishes.  by_word: it reads the call's word, which every CTA that gave up has set before
+    it counted itself in; else its own flag."""
+    word = 0 if by_word else word           # the call's grouping sets it anew
+    if up_gave_up:
+        word = 1
+    order = rng.sample(range(n_ctas), n_ctas)
+    for cta in order:
+        word |= cta in down_gave_up
+    failed = word if by_word else order[-1] in down_gave_up
+    return (0 if failed else call), word
+
+
+@pytest.mark.parametrize("by_word", [True, False])
+def test_a_call_with_a_cta_that_gave_up_is_not_published(by_word):
+    rng = random.Random(11)
+    wrong, word, n = 0, 0, 8
+    for call in range(1, 2001):
+        up = {c for c in range(n) if rng.random() < 0.03}
+        down = {c for c in range(n) if rng.random() < 0.03}
+        # an up kernel that gave up leaves hidden values of an earlier call, which the down kernel works on
+        number, word = publish(rng, n, call, bool(up), down, by_word, word)
+        wrong += number != (0 if up or down else call)
+    assert (wrong == 0) == by_word
