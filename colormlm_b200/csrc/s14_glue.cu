@@ -530,8 +530,7 @@ cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y,
                       merged);
 }
 
-// (partial sums of launch_hc_pre_many: eight slices of K for any number of tokens, or fewer than 2 * sm_count groups of
-// sixteen tokens times slices)
+// The partial sums of launch_hc_pre_many.
 size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count) {
     // a row per slice and token: up to sixteen slices, or fewer than two CTAs of sixteen tokens per SM (launch_hc_pre_many)
     return (size_t)std::max(16u * max_tokens, 32u * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
@@ -576,11 +575,16 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
     uint32_t slices = 8u;
     auto twice = [&]() { return (n / (slices * 2u * 8u)) % 16u == 0u; };
     while (slices < 64u && groups * slices < (uint32_t)sm_count && twice()) slices *= 2u;
-    // ... sixteen instead of eight where the last round of CTAs would leave a fifth of the SMs idle.  370 tokens of 4096: 192 CTAs
-    // 24.6 us for both launches and 39.0 with the norm and the expand behind them, 384 CTAs 22.3 and 31.5; 700: 33.4 and 46.4, now
-    // 30.1 and 42.9; 370 F32 tokens 25.4 and 42.4, 24.6 and 36.0.  (150 tokens at 32 slices: 17.3 and 23.1, 15.3 and 23.6.)
-    const uint32_t sms = (uint32_t)sm_count, ctas = groups * slices;
-    if (slices == 8u && ctas * 5u < ((ctas + sms - 1u) / sms) * sms * 4u && twice()) slices *= 2u;
+    // ... sixteen instead of eight where the last round of CTAs would leave a fifth of the SMs idle and the rows are long enough:
+    // the second kernel adds up twice the slices, and with fewer rounds there is less to fill up.  us of both launches, eight
+    // and sixteen slices: 370 tokens of 4096 24.6 and 22.3 (with the norm and the expand behind them 36.0 and 31.5), 700 33.4
+    // and 30.1, F32 36.4 and 33.0; 420 of 1024 14.5 and 11.9; but 940 of 1024 21.2 and 22.3, 704 of 512 11.3 and 12.7.
+    // The head's four rows cost the first kernel little, so there the bound lies higher where two rounds become
+    // three (460 of 2048 9.7 and 12.1, of 4096 14.6 and 18.7, but with the norm behind it 30.7 and 22.8) and lower where three
+    // become five (704 of 1024 10.8 and 8.9, of 4096 27.7 and 19.0).  (150 tokens at 32 slices: 17.3 and 23.1, 15.3 and 23.6.)
+    const uint32_t sms = (uint32_t)sm_count, ctas = groups * slices, rounds = (ctas + sms - 1u) / sms;
+    const uint32_t least = !kHead ? (rounds <= 2u ? 1024u : 2048u) : (rounds <= 2u ? (kBf16 ? 4096u : 5120u) : (rounds == 3u ? 1024u : 2048u));
+    if (slices == 8u && hidden >= least && ctas * 5u < rounds * sms * 4u && twice()) slices *= 2u;
     const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
     return launch_pdl(k_hc_reduce<kBf16, kHead, kBf16 ? 8 : 4>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,

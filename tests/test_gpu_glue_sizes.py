@@ -27,7 +27,8 @@ def ctx():
 @pytest.mark.parametrize("bf16", [False, True])
 @pytest.mark.parametrize("n_tokens,hidden", [(1, 256), (7, 512), (8, 1280), (9, 256), (9, 8192), (13, 512), (14, 2048), (27, 256),
                                               (28, 768), (55, 256), (56, 1280), (111, 256), (112, 256), (150, 1024), (15, 512),
-                                              (149, 1024), (593, 256), (889, 512), (300, 512), (300, 768)])
+                                              (149, 1024), (593, 256), (889, 512), (300, 512), (300, 768), (300, 1024),
+                                              (600, 1024), (300, 5120), (889, 2048)])
 def test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden):
     g = synth.rng(77 + n_tokens + hidden)
     fn, scale, base = synth.hc_params(g, hidden)
@@ -49,8 +50,8 @@ def test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden):
     close_streams(as_f32(host(normed)), as_f32(oracle.rms_norm(host(red), nw, dtype=int(bf16))), bf16)
     m_ref = oracle.hc_post(host(normed), host(x), post.cpu().numpy(), comb.cpu().numpy(), dtype=int(bf16))
     assert np.array_equal(as_f32(host(merged)), as_f32(m_ref))
-    # hc_pre's clusters: sixteen CTAs up to 7 tokens, eight up to 14; sixteen slices of K at 300 x 512 and 889 x 512, eight where
-    # K has no sixteen (768); F32 norms change form at 149, 593 and 889 tokens
+    # hc_pre's clusters: sixteen CTAs up to 7 tokens, eight up to 14; sixteen slices of K at 300 x 1024 and 889 x 2048 (the head at
+    # 600 x 1024, 300 x 5120 and 889 x 2048), eight at 300 x 512 and 889 x 512 and where K has no sixteen (768); F32 norms change form at 149, 593 and 889 tokens
     # the head's reduce: clusters of sixteen CTAs per token (up to 13 tokens), eight (27), four (55), two (111), two launches
     hfn, hscale, hbase = synth.hc_params(g, hidden, head=True)
     pre = torch.empty((n_tokens, 4), device="cuda")
