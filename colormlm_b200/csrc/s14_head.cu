@@ -235,37 +235,45 @@ k_head_mma(const float *__restrict__ x, const uint16_t *__restrict__ w, float *_
     }
 }
 
-// The same logits where there are fewer row tiles than the pairs of warps above: a CTA takes one tile, its warps the blocks
-// of 128 k in turn, their sums wait in shared memory and are added in k_head_mma's order (the same bits: a
-// vocabulary shard may be small where another is not).  There a pair walks all of K for its tile, here K is spread over
-// eight warps.  kShared (up to four tokens): x is split into its parts once per CTA; more tokens' parts do not fit beside a
-// second CTA, and every warp makes those of its blocks in the registers of the lanes that use them, which costs the
-// same for one token as for eight.  us, with the parts shared / in registers / by the register kernel below, which sums in
-// another order: 4000 x 4096 one token 12.6 / 20.2 / 9.0, eight - / 21.0 / 29.6; 1000 x 512 one token 2.5 / 3.4 / 1.8.
-constexpr uint32_t kFewThreads = 256;
+// The same logits where there are at most two row tiles per SM: `wide` warps take one tile, the blocks of 128 k in turn, a
+// block's loads in flight while the one before is worked on; the blocks' sums wait in shared memory and are added in
+// k_head_mma's order (the same bits: a vocabulary shard may be small where another is not).  There a pair of warps walks all of
+// K for a tile.  Up to a tile per SM sixteen warps share one; above that eight do, in CTAs of one tile (two CTAs per SM) or of
+// two, which split x once for both.  kShared: x is split into its parts once per CTA; what does not fit in shared memory
+// beside room for the loads in the L1 is split by every warp in the registers of the lanes that use it, which costs the same
+// for one token as for eight.  What bounds it is the chain per block - loads, four dependent steps, the sums' way into double -
+// times the blocks of a warp: more loads ahead do not help (4000 x 4096 one token 10.8 with two blocks ahead, 10.6 with one),
+// more warps per tile do.  us, with eight warps to a tile always, no loads ahead and parts per CTA / now / by the register
+// kernel below, which sums in another order: 64 x 4096 one token 7.8 / 5.7 / 5.6, 1000 x 7168 one token 17.4 / 9.6 / 10.9,
+// four 38.8 / 18.3 / 16.2, 4000 x 4096 one token 11.9 / 10.5 / 8.8, four 24.2 / 13.3 / 23.6, eight 20.3 / 20.2 / 29.1.
+constexpr uint32_t kFewSmallParts = 2048;   // tokens x hidden up to which splitting x twice on an SM costs less than sharing it
+constexpr size_t kFewTwoBytes = 190u * 1024u, kFewOneBytes = 200u * 1024u;   // of shared memory: two tiles, one tile
 template <bool kShared>
-__global__ void __launch_bounds__(kFewThreads, 2)
+__global__ void __launch_bounds__(512, 1)
 k_head_mma_few(const float *__restrict__ x, const uint16_t *__restrict__ w, float *__restrict__ out, uint32_t n_rows, uint32_t hidden,
-               uint32_t out_stride, uint32_t n_tokens, uint32_t phases) {
-    extern __shared__ __align__(16) uint8_t s_few[];         // [K / 128][4][32] sums of the blocks, then the parts [3][n_tokens][pitch]
-    double *const s_blk = reinterpret_cast<double *>(s_few);
-    uint8_t *const s_x = s_few + (size_t)hidden * 8u;
+               uint32_t out_stride, uint32_t n_tokens, uint32_t phases, uint32_t wide) {
+    extern __shared__ __align__(16) uint8_t s_few[];   // [tile][K / 128][4][32] sums of the blocks, then the parts [3][n_tokens][pitch]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
-    const uint32_t n_blk = hidden >> 7, row0 = blockIdx.x * 16u, pitch = hidden * 2u + kHeadPad;
+    const uint32_t n_blk = hidden >> 7, per_half = n_blk / (2u * phases);
+    const uint32_t tiles = (blockDim.x >> 5) / wide, local = warp / wide, mine = warp - local * wide;   // `wide` warps to a tile
+    const uint32_t pitch = hidden * 2u + kHeadPad, row0 = (blockIdx.x * tiles + local) * 16u;
+    double *const s_sum = reinterpret_cast<double *>(s_few) + (size_t)local * n_blk * 128u;
+    uint8_t *const s_x = s_few + (size_t)tiles * n_blk * 1024u;
+    const bool has_b = g < n_tokens;
     const uint16_t *const p0 = w + (size_t)min(row0 + g, n_rows - 1u) * hidden + q * 8u;
     const uint16_t *const p1 = w + (size_t)min(row0 + g + 8u, n_rows - 1u) * hidden + q * 8u;
-    const bool has_b = g < n_tokens;
     const float *const xg = x + (size_t)(has_b ? g : 0u) * hidden + q * 8u;
     uint4 a0[kHeadDepth], a1[kHeadDepth];
-    auto fetch = [&](uint32_t b) {
-#pragma unroll
-        for (uint32_t j = 0; j < kHeadDepth; ++j) {
-            a0[j] = ld_stream(reinterpret_cast<const uint4 *>(p0 + b * 128u + j * 32u));
-            a1[j] = ld_stream(reinterpret_cast<const uint4 *>(p1 + b * 128u + j * 32u));
-        }
+    auto fetch = [&](uint32_t j, uint32_t b) {
+        a0[j] = ld_stream(reinterpret_cast<const uint4 *>(p0 + b * 128u + j * 32u));
+        a1[j] = ld_stream(reinterpret_cast<const uint4 *>(p1 + b * 128u + j * 32u));
     };
+    const uint32_t end = row0 < n_rows ? n_blk : 0u;   // (the last CTA may have a tile less)
     dependency_wait();
-    if (warp < n_blk) fetch(warp);   // in flight while x is split
+    if (mine < end) {   // in flight while x is split
+#pragma unroll
+        for (uint32_t j = 0; j < kHeadDepth; ++j) fetch(j, mine);
+    }
     auto parts_of = [](const float4 &lo, const float4 &hi, uint4 (&bp)[3]) {
         const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
         uint32_t wd[3][4];
@@ -281,7 +289,7 @@ k_head_mma_few(const float *__restrict__ x, const uint16_t *__restrict__ w, floa
         for (uint32_t part = 0; part < 3; ++part) bp[part] = make_uint4(wd[part][0], wd[part][1], wd[part][2], wd[part][3]);
     };
     if constexpr (kShared) {
-        for (uint32_t i = tid; i < n_tokens * (hidden >> 3); i += kFewThreads) {
+        for (uint32_t i = tid; i < n_tokens * (hidden >> 3); i += blockDim.x) {
             const uint32_t t = i / (hidden >> 3), k8 = i - t * (hidden >> 3);
             const float4 *at = reinterpret_cast<const float4 *>(x + (size_t)t * hidden) + 2u * k8;
             uint4 bp[3];
@@ -292,8 +300,8 @@ k_head_mma_few(const float *__restrict__ x, const uint16_t *__restrict__ w, floa
         __syncthreads();
     }
 #pragma unroll 1
-    for (uint32_t b = warp; b < n_blk; b += kFewThreads / 32u) {
-        if (b != warp) fetch(b);
+    for (uint32_t b = mine; b < end; b += wide) {
+        const bool more = b + wide < end;
         HeadBlock blk;
 #pragma unroll
         for (uint32_t j = 0; j < kHeadDepth; ++j) {
@@ -309,30 +317,32 @@ k_head_mma_few(const float *__restrict__ x, const uint16_t *__restrict__ w, floa
                 }
             }
             blk.step(a0[j], a1[j], bp);
+            if (more) fetch(j, b + wide);
             blk.carry();
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s_blk[(b * 4u + e) * 32u + lane] = blk.sum(e);
+        for (int e = 0; e < 4; ++e) s_sum[(b * 4u + e) * 32u + lane] = blk.sum(e);
     }
     __syncthreads();
-    if (tid >= 128u) return;
-    const uint32_t e = warp, per_phase = n_blk / phases;   // warp e: accumulator e of every lane
+    if (mine >= 4u || row0 >= n_rows) return;
+    const uint32_t e = mine;   // four warps of a tile: accumulator e of every lane
     double sum = 0.0;
 #pragma unroll 1
     for (uint32_t phase = 0; phase < phases; ++phase) {
-        double half[2];
-#pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) {
-            half[h] = 0.0;
-            for (uint32_t b = 0; b < per_phase / 2u; ++b) half[h] += s_blk[((phase * per_phase + h * (per_phase / 2u) + b) * 4u + e) * 32u + lane];
+        double half[2] = {0.0, 0.0};
+        const double *at = s_sum + ((size_t)phase * 2u * per_half * 4u + e) * 32u + lane;
+#pragma unroll 4
+        for (uint32_t p = 0; p < per_half; ++p) {
+            half[0] += at[p * 128u];
+            half[1] += at[(per_half + p) * 128u];
         }
         const double both = half[0] + half[1];
         sum = phase ? both + sum : both;
     }
     const uint32_t row = row0 + g + (e >> 1) * 8u, t = 2u * q + (e & 1u);
-    const bool mine = row < n_rows && t < n_tokens;
-    if (mine) out[(size_t)t * out_stride + row] = (float)sum;
-    uint32_t redo = __ballot_sync(0xffffffffu, mine && !isfinite(sum));
+    const bool ours = row < n_rows && t < n_tokens;
+    if (ours) out[(size_t)t * out_stride + row] = (float)sum;
+    uint32_t redo = __ballot_sync(0xffffffffu, ours && !isfinite(sum));
     while (redo) {
         const uint32_t src = __ffs((int)redo) - 1, t_src = 2u * (src & 3u) + (e & 1u);
         const float v = head_row_dot(x + (size_t)t_src * hidden, w + (size_t)(row0 + (src >> 2) + (e >> 1) * 8u) * hidden, hidden);
@@ -569,27 +579,30 @@ k_head_prep(const uint16_t *__restrict__ state, const float *__restrict__ fn, co
     }
 }
 
-// The largest dynamic shared memory all of the tensor-core kernels may ask for on the current device (0: could not be set).
-size_t head_smem_limit() {
-    static size_t limit[64] = {};
+// The largest dynamic shared memory a kernel may ask for on the current device (0: could not be set).
+size_t smem_limit_of(const void *fn, size_t (&limit)[64]) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if (!limit[dev]) {
-        const void *const fns[] = {(const void *)k_head_mma, (const void *)k_head_mma_few<false>, (const void *)k_head_mma_few<true>};
         cudaFuncAttributes fa;
         int optin = 0;
-        size_t fixed = 0;
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-        for (const void *fn : fns) {
-            if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
-            fixed = std::max(fixed, fa.sharedSizeBytes);
-        }
-        const size_t most = (size_t)optin - fixed;
-        for (const void *fn : fns)
-            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
+        if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+            return 0;
+        const size_t most = (size_t)optin - fa.sharedSizeBytes;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
         limit[dev] = most;
     }
     return limit[dev];
+}
+size_t head_smem_limit() {
+    static size_t limit[64] = {};
+    return smem_limit_of((const void *)k_head_mma, limit);
+}
+template <bool kShared>
+size_t few_smem_limit() {
+    static size_t limit[64] = {};
+    return smem_limit_of((const void *)k_head_mma_few<kShared>, limit);
 }
 
 }  // namespace
@@ -598,22 +611,31 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
                                uint32_t hidden, float *out, uint32_t out_stride) {
     // the tensor-core kernel: phases of K in whole groups of steps per half row, as few as keep the parts small;
     // sizes that have none take the register kernel
-    // (which kernel a row is worked out by does not depend on how many rows or tokens a call has beyond what leaves its bits
-    // alone: a vocabulary may be dealt over ranks in shards of any size)
+    // (a row's bits do not depend on how many rows a call has: a vocabulary may be dealt over ranks in shards of any size.
+    // They do depend on the number of tokens, which sets the phases and, for some hidden sizes, the kernel.)
     for (uint32_t phases = 1; phases <= 8u; phases *= 2u) {
         const size_t parts = 3u * (size_t)n_tokens * (hidden / phases * 2u + kHeadPad);
         const size_t smem = parts + (phases > 1u ? kHeadTiles * 1024u : 0u);
         if (hidden % (256u * phases) != 0u || smem > head_smem_limit()) continue;
         if (parts > kHeadPartBytes && hidden % (512u * phases) == 0u && phases < 8u) continue;
         const uint32_t tiles = (n_rows + 15u) / 16u;
-        // up to two tiles per SM: a CTA per tile
-        if (tiles <= 2u * (uint32_t)sm_count && (size_t)hidden * 8u + (n_tokens <= 4u ? parts * phases : 0u) <= head_smem_limit()) {
+        if (tiles <= 2u * (uint32_t)sm_count) {
             const size_t sums = (size_t)hidden * 8u, shared = 3u * (size_t)n_tokens * (hidden * 2u + kHeadPad);
-            if (n_tokens <= 4u)
-                return launch_pdl(k_head_mma_few<true>, dim3(tiles), dim3(kFewThreads), sums + shared, st, 0u, x, w, out, n_rows, hidden,
-                                  out_stride, n_tokens, phases);
-            return launch_pdl(k_head_mma_few<false>, dim3(tiles), dim3(kFewThreads), sums, st, 0u, x, w, out, n_rows, hidden, out_stride,
-                              n_tokens, phases);
+            const size_t most = few_smem_limit<true>();
+            auto few = [&](auto kernel, uint32_t warps, uint32_t wide, size_t bytes) {
+                const uint32_t per_cta = warps / wide;
+                return launch_pdl(kernel, dim3((tiles + per_cta - 1u) / per_cta), dim3(warps * 32u), bytes, st, 0u, x, w, out, n_rows, hidden,
+                                  out_stride, n_tokens, phases, wide);
+            };
+            const bool alone = tiles <= (uint32_t)sm_count;
+            // 4000 rows, us: 2048 x one token in CTAs of one tile 6.2, of two 6.7; 1024 x six 5.8 and 5.3; 4096 x five of two 14.5,
+            // split in registers 20.3; 7168 x two in two rounds of one tile 22.6, of two (198 KB) 27.1
+            if (!alone && n_tokens * hidden <= kFewSmallParts && sums + shared <= most) return few(k_head_mma_few<true>, 8u, 8u, sums + shared);
+            if (!alone && 2u * sums + shared <= std::min(kFewTwoBytes, most)) return few(k_head_mma_few<true>, 16u, 8u, 2u * sums + shared);
+            // (two rounds: 7168 x three 26.6, in registers 32.6; 4096 x six 21.3 and 20.3)
+            if ((alone || n_tokens <= 4u) && sums + shared <= std::min(kFewOneBytes, most))
+                return few(k_head_mma_few<true>, 16u, 16u, sums + shared);
+            if (sums <= few_smem_limit<false>()) return few(k_head_mma_few<false>, alone ? 16u : 8u, alone ? 16u : 8u, sums);
         }
         const uint32_t ctas = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
         return launch_pdl(k_head_mma, dim3(ctas), dim3(kHeadThreads), smem, st, 0u, x, w, out, n_rows, hidden, out_stride, n_tokens,

@@ -94,15 +94,16 @@ def test_logits_of_infinite_weights_and_overflowing_products(ctx, tokens, hidden
     assert int(token) == 3
 
 
-# the kernel of few row tiles and the other one, in phases (8 tokens of 4096) and not, one block of K per half and many
-@pytest.mark.parametrize("tokens,hidden", [(1, 256), (3, 768), (1, 4096), (8, 4096), (2, 6144), (8, 7168)])
+# the kernel of few row tiles and the other one, in phases (8 tokens of 4096) and not, one block of K per half and many; above a
+# tile per SM CTAs of one tile (up to 2048 tokens x hidden), of two, rounds of one (3 of 7168), parts in registers (8 tokens)
+@pytest.mark.parametrize("tokens,hidden", [(1, 256), (3, 768), (1, 2048), (1, 4096), (5, 1024), (4, 4096), (8, 4096), (2, 6144), (3, 7168), (8, 7168)])
 def test_logits_of_a_vocabulary_shard_have_the_bits_of_the_whole(ctx, tokens, hidden):
     g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
     x = torch.randn(tokens, hidden, device="cuda", generator=g)
     w = torch.empty(9000, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=g).view(torch.int16)
     whole = torch.empty(tokens, 9000, device="cuda")
     ctx.cmd_head_logits(x, w, whole)
-    for r0, r1 in ((0, 1), (5, 22), (100, 4836), (100, 4837), (8985, 9000)):
+    for r0, r1 in ((0, 1), (5, 22), (100, 2468), (100, 2470), (100, 4836), (100, 4837), (8985, 9000)):
         part = torch.empty(tokens, r1 - r0, device="cuda")
         ctx.cmd_head_logits(x, w[r0:r1], part)
         assert torch.equal(part, whole[:, r0:r1]), (r0, r1)
