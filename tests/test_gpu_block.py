@@ -10,6 +10,7 @@ torch = pytest.importorskip("torch")
 
 from colormlm_b200 import _lib as L
 from colormlm_b200 import synth
+from colormlm_b200.pages import ExpertPageLayout
 from colormlm_b200.s14 import MoeBlock, S14Context, S14Error, TokenRoute
 
 from .test_gpu_parity import dev, dev_page, make_layer, run_layer
@@ -128,25 +129,55 @@ def test_block_sweep_of_block_sizes_against_the_one_token_kernel(ctx):
         blk.close()
 
 
+def page_of_scales(g, hidden, inter, s1=(119, 123), s2=(119, 123)):
+    """An MXFP4 page of tensors whose w1 or w2 rows have one scale code each, drawn from the given range."""
+    lay = ExpertPageLayout(hidden, inter, L.PAGE_MXFP4)
+    rows = lambda n, k, r: np.repeat(g.integers(r[0], r[1] + 1, size=(n, 1), dtype=np.uint8), k // 32, axis=1)
+    return lay.pack(synth.mxfp4_codes(g, inter, hidden), synth.mxfp4_codes(g, inter, hidden), synth.mxfp4_codes(g, hidden, inter),
+                    rows(inter, hidden, s1), synth.mxfp4_scales(g, inter, hidden), rows(hidden, inter, s2))
+
+
+# Scale codes that put the digit shares of the gates, or of the outputs, on both sides of 2^-79 or of 2^113, with outputs that
+# show every one of them.  (In the official arithmetic small hidden values are quantised to zero, so there only the outputs can;
+# large gates saturate in both.)
+RANGES = {"gates_low": {"s1": (32, 42)}, "outputs_low": {"s2": (32, 42)}, "outputs_high": {"s2": (226, 233)}}
+
+
 @pytest.mark.parametrize("n_tokens", [3, 14])
-def test_block_of_values_outside_the_range_of_the_f32_sums(ctx, n_tokens):
+@pytest.mark.parametrize("where,official", [("gates_low", False), ("outputs_low", False), ("outputs_high", False),
+                                            ("outputs_low", True), ("outputs_high", True)])
+def test_block_of_values_outside_the_range_of_the_f32_sums(ctx, oracle, where, official, n_tokens):
     """The digit shares are added in F32 with constants made of the largest one; shares below 2^-79 or from 2^113 on, and
-    those of a token of zeros, take the sum in double.  Every token equals its own one-token call."""
+    those of a token of zeros, take the sum in double.  Every token has the oracle's bits, and the oracle's results are such
+    that a wrong sum shows: finite, different from zero, on both sides of the boundary, and moved by 2^-5 more input."""
     hidden, inter, n_experts = 1024, 1024, 8
-    g, pages, shared = make_layer(1850, hidden, inter, n_experts, L.PAGE_MXFP4)
+    g = synth.rng(1850)
+    pages = [page_of_scales(g, hidden, inter, **RANGES[where]) for _ in range(n_experts + 1)]
+    shared = pages.pop()
     pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    x = synth.activations(g, n_tokens, hidden)
+    if official:
+        x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(x))
+    x[2] = 0.0
+    routes = random_routes(g, n_tokens, n_experts)
+    layer = oracle.official_moe_layer if official else oracle.moe_layer_acc64
     blk = MoeBlock(ctx, hidden, inter, 16)
-    ctx.set_accumulation(L.ACCUM_PAIRWISE)
     try:
-        x = synth.activations(g, n_tokens, hidden)
-        x[0] *= np.float32(2.0 ** -78)
-        x[1] *= np.float32(2.0 ** 112)
-        x[2] = 0.0
-        routes = random_routes(g, n_tokens, n_experts)
+        blk.set_semantics(official)
         y = run_block(ctx, blk, x, pages_dev, shared_dev, routes)
         for t in range(n_tokens):
-            single = run_layer(ctx, x[t:t + 1], pages_dev, shared_dev, [routes[t]], L.PAGE_MXFP4, hidden, inter)[0]
-            assert np.array_equal(single.view(np.uint32), y[t].view(np.uint32)), t
+            ids, w = routes[t]
+            ref = layer(x[t], [pages[i] for i in ids], w, shared, 0, hidden, inter)
+            assert np.array_equal(y[t].view(np.uint32), ref.view(np.uint32)), t
+            if t == 2:
+                assert not ref.any()
+                continue
+            assert np.isfinite(ref).all() and np.count_nonzero(ref) > 0.99 * hidden
+            size = np.abs(ref[ref != 0])
+            low, high = (2.0 ** -79, 2.0 ** -79) if where.endswith("low") else (2.0 ** 112, 2.0 ** 113)
+            assert (size < low).sum() > 20 and (size > high).sum() > 20
+            moved = layer(x[t] * np.float32(1 + 2.0 ** -5), [pages[i] for i in ids], w, shared, 0, hidden, inter)
+            assert np.count_nonzero(moved != ref) > 0.9 * hidden
     finally:
         blk.close()
 
@@ -179,6 +210,40 @@ def test_block_of_the_largest_size(ctx):
         for t in (0, 1, 511, 777, 1023):
             single = run_layer(ctx, x[t:t + 1], pages_dev, shared_dev, [(ids_np[t].tolist(), w_np[t])], L.PAGE_MXFP4, hidden, inter)[0]
             assert np.array_equal(single.view(np.uint32), y[t].view(np.uint32)), t
+    finally:
+        blk.close()
+
+
+@pytest.mark.parametrize("official,inter,n_experts,batch", [(False, 512, 16, 96), (True, 2048, 256, 56)])
+def test_block_of_several_batches_of_item_records(ctx, oracle, official, inter, n_experts, batch):
+    """The contraction kernels decode their items in batches of `batch` records, and the roles carry their place in the ring,
+    the item and the step from batch to batch: 1000 tokens of 4096, with more down items per pair of CTAs than a batch has (in
+    the official arithmetic up items as well).  Several experts share a page; sampled tokens against the oracle."""
+    hidden, n_tokens, n_pages = 4096, 1000, 8
+    g, pages, shared = make_layer(1950 + inter, hidden, inter, n_pages, L.PAGE_MXFP4)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    table = torch.tensor([pages_dev[e % n_pages].data_ptr() for e in range(n_experts)], dtype=torch.int64, device="cuda")
+    wr, bias = dev(synth.router_weight_bf16(g, n_experts, hidden)), dev(synth.router_bias(g, n_experts))
+    x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(synth.activations(g, n_tokens, hidden)))
+    dx = dev(x)
+    dy = torch.full_like(dx, float("nan"))
+    ids = torch.empty((n_tokens, 6), dtype=torch.int32, device="cuda")
+    wts = torch.empty((n_tokens, 6), dtype=torch.float32, device="cuda")
+    blk = MoeBlock(ctx, hidden, inter, n_tokens)
+    layer = oracle.official_moe_layer if official else oracle.moe_layer_acc64
+    try:
+        blk.set_semantics(official)
+        blk.cmd_routed_moe_block(dx, wr, bias, table, shared_dev.data_ptr(), dy, ids, wts)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0
+        _, n_up, n_down, bad = blk.last_counts()
+        pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+        assert bad == 0 and n_down > batch * pairs and (n_up > batch * pairs or not official)
+        y, ids_np, w_np = dy.cpu().numpy(), ids.cpu().numpy(), wts.cpu().numpy()
+        assert not np.isnan(y).any()
+        for t in (0, 1, 498, 777, 999):
+            ref = layer(x[t], [pages[e % n_pages] for e in ids_np[t]], w_np[t], shared, 0, hidden, inter)
+            assert np.array_equal(y[t].view(np.uint32), ref.view(np.uint32)), t
     finally:
         blk.close()
 
@@ -400,8 +465,8 @@ def test_block_rejects_what_it_cannot_run(ctx):
         blk.close()
 
 
-# tiles of the score kernel: up to 8 tokens, 16 x 8 (few tiles), 16 x 16 (at least 296 of them), each with remainders
-@pytest.mark.parametrize("n_tokens,n_experts", [(1, 6), (8, 21), (9, 7), (17, 65), (300, 250), (301, 256)])
+# tiles of the score kernel: 8 x 8 (up to 64 tokens), 16 x 8 (few tiles), 16 x 16 (at least 296 of them), each with remainders
+@pytest.mark.parametrize("n_tokens,n_experts", [(1, 6), (8, 21), (9, 7), (17, 65), (64, 21), (65, 21), (100, 250), (300, 250), (301, 256)])
 def test_routed_block_scores_at_the_tiles_edges(ctx, oracle, n_tokens, n_experts):
     """Ids and weights bit-identical to the oracle's router; the mix into a y on a 4-byte boundary equal to the aligned one."""
     hidden, inter = 512, 512

@@ -9,7 +9,7 @@ torch = pytest.importorskip("torch")
 
 from colormlm_b200 import _lib as L
 from colormlm_b200 import synth
-from colormlm_b200.s14 import S14Context, S14MatvecShape, TokenRoute
+from colormlm_b200.s14 import MoeBlock, S14Context, S14MatvecShape, TokenRoute
 
 from .test_gpu_parity import dev, dev_page, make_layer
 
@@ -90,7 +90,31 @@ def _layer(ctx):
     return pages_dev + [shared_dev], (lambda: ctx.cmd_moe_layer(x, y, [route], shared_dev.data_ptr(), L.PAGE_FP8, h, i)), y
 
 
-@pytest.mark.parametrize("make", [_mxfp4, _fp8, _head, _site(1), _site(20), _layer], ids=["mxfp4", "fp8", "head", "site", "site20", "fp8_shared_layer"])
+def _block(tokens, official, routed):
+    """The block calls: their first digits launch reads x in front of its wait, behind the router's launches (or the copies of
+    the host's routes), which have waited."""
+    def make(ctx):
+        h, i, experts = 1024, 512, 8
+        g, pages, shared = make_layer(4, h, i, experts, L.PAGE_MXFP4)
+        pages_dev, shared_dev = [dev_page(p, h, i) for p in pages], dev_page(shared, h, i)
+        table = torch.tensor([p.data_ptr() for p in pages_dev], dtype=torch.int64, device="cuda")
+        x, y = dev(synth.activations(g, tokens, h)), torch.empty(tokens, h, device="cuda")
+        wr, bias = dev(synth.router_weight_bf16(g, experts, h).view(np.int16)), dev(synth.router_bias(g, experts))
+        blk = MoeBlock(ctx, h, i, tokens)
+        blk.set_semantics(official)
+        if routed:
+            return [x, wr, bias, pages_dev[0], shared_dev], (lambda keep=pages_dev: blk.cmd_routed_moe_block(x, wr, bias, table, shared_dev.data_ptr(), y)), y
+        routes = [TokenRoute([e, e + 2], np.asarray([0.7, 0.4], np.float32), [pages_dev[e].data_ptr(), pages_dev[e + 2].data_ptr()])
+                  for e in (t % 6 for t in range(tokens))]
+        return [x, pages_dev[0], shared_dev], (lambda keep=pages_dev: blk.cmd_moe_block(x, y, routes, shared_dev.data_ptr())), y
+
+    return make
+
+
+@pytest.mark.parametrize("make", [_mxfp4, _fp8, _head, _site(1), _site(20), _layer, _block(3, False, True), _block(20, False, True),
+                                  _block(3, True, True), _block(70, True, True), _block(5, False, False)],
+                         ids=["mxfp4", "fp8", "head", "site", "site20", "fp8_shared_layer", "block", "block20", "block_official",
+                              "block70_official", "block_host_routes"])
 def test_operands_written_late_by_a_kernel_that_lets_dependents_start(ctx, write_late, make):
     torch.manual_seed(1)
     operands, call, y = make(ctx)
