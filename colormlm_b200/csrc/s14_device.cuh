@@ -173,7 +173,8 @@ inline cudaError_t launch_status(cudaError_t e) {
 // included: a caller's kernel may write those too, and one that lets its own dependents start early is not even
 // complete when such a launch starts.  Behind it they use coherent loads that the compiler keeps in place (__ldcg,
 // ld_stream, ld_u8, ld_f32).  A non-coherent load (__ldg, or a plain one through a const __restrict__ pointer)
-// could return what the operand held before.
+// could return what the operand held before.  One kernel reads and writes in front of its wait: the first digits launch of a
+// block call (k_block_digits, early), behind k_router_select_batch, which triggers behind its own wait, or behind a copy.
 template <class Kernel, class... Args>
 inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};

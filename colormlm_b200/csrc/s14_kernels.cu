@@ -1329,7 +1329,7 @@ k_stack_step(const float *__restrict__ x, const float *__restrict__ y, float *ou
 //
 // A token's row is read once per 8 * kNt experts and a weight row once per 8 * kMt tokens; both come from the L2.
 // 16 x 16 tiles for large blocks (wider ones leave too few CTAs, narrower ones read x more often); a smaller grid than two CTAs
-// per SM takes 16 x 8, up to eight tokens 8 x 8 with the K range over sixteen warps.  Measured, x 256 experts x 4096:
+// per SM takes 16 x 8, up to 64 tokens 8 x 8 with the K range over sixteen warps.  Measured, x 256 experts x 4096:
 // 8 tokens 15 -> 8.3 us, 370 84 -> 40, 1000 166 -> 83 (before: operands staged in shared memory as doubles by 32 x 16
 // tiles with all of K in one warp; up to 32 tokens on the vector pipe); 45 tokens x 192 experts x 2048: 32 -> 10.
 template <uint32_t kMt, uint32_t kNt, uint32_t kWarps>
@@ -1421,7 +1421,7 @@ __global__ void __launch_bounds__(256)
 k_router_select_batch(const float *__restrict__ scores, const float *__restrict__ select, uint32_t n_experts, uint32_t n_tokens,
                       uint32_t top_k, float route_scale, int32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
     const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    dependency_wait();
+    dependency_wait();   // (triggers behind the wait: the digits launch behind reads x without waiting for this kernel)
     if (t >= n_tokens) return;
     router_select(scores + (size_t)t * n_experts, select + (size_t)t * n_experts, n_experts, top_k, route_scale,
                   ids_out + (size_t)t * top_k, weights_out + (size_t)t * top_k, nullptr, nullptr, nullptr, 0, threadIdx.x & 31u, 0,

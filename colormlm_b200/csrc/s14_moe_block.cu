@@ -9,8 +9,8 @@
 // are, and B = the sixteen balanced base-8 digit rows of EVERY token of a chunk (up to twelve tokens
 // that share the expert: N = 16 * tokens; official arithmetic: eight rows each, up to twenty-four tokens).
 // Accumulator columns 16 t .. 16 t + 15 hold the digit shares of token t's dot products; added without loss and
-// rounded once they give the double-accumulated dot product rounded to F32, so every token's result is bit-identical to what the one-token kernel
-// and the double-accumulating CPU restatement give for that token alone.
+// rounded once they give the dot product rounded to F32, so every token's result has the bits that the one-token kernel
+// and the double-accumulating CPU restatement give for that token alone, up to ties closer than a sum in double resolves.
 //
 // Six launches per layer, all plain stream order (the routed calls run the router's two launches first):
 //   k_block_digits   x [T, hidden] -> digit tiles (2 KB per token and 256 elements) + block exponents
@@ -41,6 +41,8 @@ namespace {
 constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens: most experts have one, and short stages make the ring deep
 constexpr uint32_t kGrpSparse = 6;   // fewer than three pairs (official arithmetic: six) per expert on average
 constexpr uint32_t kGrpDense = 12;
+// (Both bounds, and the one of twelve tokens, were found with one-CTA kernels that had other stages; on the pair kernel, whose
+// rings hold ten, nine and seven stages, the three sizes have not been compared with each other.)
 static_assert(kBlockNt == 2u * kGrpDense, "a chunk record holds the tokens of the official arithmetic's chunks");
 
 // The nearest E4M3FN value (ties to even) of |v| <= 448: three mantissa bits; below 2^-6 multiples of 2^-9.
@@ -72,7 +74,8 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
     constexpr uint32_t kRows = kQuant ? 8u : 16u;
     const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
     // early: the launch in front neither writes x nor uses what is written here (it picks the routes), and whatever is in front
-    // of it is complete when this kernel starts; so the work runs beside it, and the wait for it comes last
+    // of it is complete when this kernel starts, because it lets this one start behind its own wait (a launch that triggers in
+    // front of it would make this a race); so the work runs beside it, and the wait for it comes last
     if (!early) dependency_wait();
     const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
     const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
@@ -333,7 +336,8 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     const uint32_t groups = small ? kGrpSmall : ((uint64_t)n_tokens * top_k >= (uint64_t)(3u * tpg) * n_experts ? kGrpDense : kGrpSparse);
     const uint32_t S = inter >> 6, RT = hidden >> 7, counted = small ? 1u : 2u;   // slices, row tiles; as `counts` reports them
     // The launches are programmatic dependents of one another: a kernel's blocks, barriers and tensor memory are
-    // set up while the one before runs out, and every kernel waits for it before it reads or writes anything.
+    // set up while the one before runs out, and every kernel but the first digits launch (see there) waits for it before it
+    // reads or writes anything.
     auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps, bool early) {
         if (*err != cudaSuccess) return;
         *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps,

@@ -8,15 +8,19 @@
 // columns, and the accumulators of one row tile are all an SM holds: 192 columns, which leaves room for a second set.  So an
 // item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
 // (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
-// epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 506 / 294
-// us, now 427 / 204; 1000 tokens of the official arithmetic 1206 / 443, now 730 / 309.  Small blocks, which took one row tile
+// epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 507 / 294
+// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, now 577 / 311.  Small blocks, which took one row tile
 // and two tokens per SM with stages of 21 KB in a ring of eight and laid out the hidden values' digit rows in the up epilogue:
-// 8 tokens 117 us for the call, now 109.
+// 8 tokens 117 us for the call, now 109.  (Official blocks of two to eight tokens of smaller layers gained nothing: 4 tokens of
+// 2048 x 1536 49 us for the call, now 52.)
 //
-// What bounds it.  A step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles, the issuing
-// warp's round 470, a step 600-700 on average.  A second warp that copies the codes ahead gets a probe to 389 cycles a
+// What bounds it is not settled.  A step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles
+// (270 for the chunks 370 tokens have on average), the issuing warp's round 470 at most, but a step 700 on average at full
+// clock; the kernels take in 9 to 10.8 TB/s from the L2 meanwhile, and which of the intake and the hand-offs makes up the rest was
+// not measured.  A second warp that copies the codes ahead gets a probe to 389 cycles a
 // step, but adds a hand-off to every stage's way through the ring of seven (370 tokens 736 us instead of 704).  Sustained, the
-// 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.
+// 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.  A pair with more items
+// than a batch of records drains its pipeline between two batches (1000 official tokens: about 90 items, batches of 56).
 //
 // Roles in a CTA of 608 threads: warps 0-7 epilogue (two warpgroups, each with every lane of tensor memory, the even and
 // the odd groups of the chunk); warps 8-11 copy (the ring slots in turn, a lane per copy: a round of waiting, arming
@@ -24,7 +28,7 @@
 // passes on that its stage is complete; warps 13-18 lay out the scale codes of the digit rows of a stage.  A stage's barriers:
 // `full` in each CTA (unit, tiles, codes; in the first CTA also that the second's is complete), `done` in each (the commit
 // arrives at both).  Every wait is bounded; one that runs out raises the CTA's abort flag, the status word is set, the CTA
-// waits for its copies, and the pair meets at a cluster barrier before tensor memory is freed.
+// waits for its copies and the pair's tensor work, and the pair meets at a cluster barrier before tensor memory is freed.
 #include "s14_moe_block.cuh"
 
 namespace s14 {
@@ -64,9 +68,11 @@ __device__ __forceinline__ uint32_t first_cta(uint32_t addr) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
     return r;
 }
-// At another CTA's barrier.  Nothing that threads read is handed over with it - the tensor cores read either CTA's shared
-// memory behind that CTA's own proxy fence, and tensor memory is drained by its owner -, so it carries no wider fence: with
-// .release.cluster (and .acquire.cluster on the other side) a stage took a microsecond more.
+// At another CTA's barrier.  Nothing that threads read is handed over with it: the tensor cores read either CTA's shared
+// memory behind that CTA's own proxy fence, and tensor memory is drained by its owner.  So it carries no wider fence: with
+// .release.cluster (and .acquire.cluster on the other side) a stage took a microsecond more.  This relies on how the hardware
+// behaves; the memory model of PTX asks for cluster scope where scale codes that the second CTA's threads wrote are read by
+// operations the first one issued.  Every test compares bits.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
