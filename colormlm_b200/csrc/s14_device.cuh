@@ -175,23 +175,40 @@ inline cudaError_t launch_status(cudaError_t e) {
 // ld_stream, ld_u8, ld_f32).  A non-coherent load (__ldg, or a plain one through a const __restrict__ pointer)
 // could return what the operand held before.  One kernel reads and writes in front of its wait: the first digits launch of a
 // block call (k_block_digits, early), behind k_router_select_batch, which triggers behind its own wait, or behind a copy.
+//
+// `shared`: bytes of shared memory an SM needs for this kernel, 1 KB per CTA included (0: not said).  A dependent launch takes
+// over SMs from a kernel that is still running elsewhere, and without a word the SMs stay divided as that kernel has them:
+// behind one that fills shared memory the loads of the next find hardly any L1 to be in flight in.
 template <class Kernel, class... Args>
-inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args... args) {
+inline cudaError_t launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, size_t shared, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = cluster ? 2 : 1;
+    cfg.numAttrs = 1;
+    if (cluster) {
+        cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = cluster;
+        a.val.clusterDim.y = 1;
+        a.val.clusterDim.z = 1;
+    }
+    if (shared) {
+        constexpr size_t kMost = 228u * 1024u;   // of an SM
+        cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+        a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        a.val.sharedMemCarveout = (unsigned)std::min<size_t>(100u, (shared * 100u + kMost - 1u) / kMost);
+    }
     return launch_status(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+template <class Kernel, class... Args>
+inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, uint32_t cluster, Args... args) {
+    return launch_dependent(kernel, grid, block, smem, st, cluster, 0u, args...);
 }
 
 }  // namespace s14

@@ -623,9 +623,9 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
             const size_t sums = (size_t)hidden * 8u, shared = 3u * (size_t)n_tokens * (hidden * 2u + kHeadPad);
             const size_t most = few_smem_limit<true>();
             auto few = [&](auto kernel, uint32_t warps, uint32_t wide, size_t bytes) {
-                const uint32_t per_cta = warps / wide;
-                return launch_pdl(kernel, dim3((tiles + per_cta - 1u) / per_cta), dim3(warps * 32u), bytes, st, 0u, x, w, out, n_rows, hidden,
-                                  out_stride, n_tokens, phases, wide);
+                const uint32_t per_cta = warps / wide, resident = 16u / warps;
+                return launch_dependent(kernel, dim3((tiles + per_cta - 1u) / per_cta), dim3(warps * 32u), bytes, st, 0u, resident * (bytes + 1024u),
+                                        x, w, out, n_rows, hidden, out_stride, n_tokens, phases, wide);
             };
             const bool alone = tiles <= (uint32_t)sm_count;
             // 4000 rows, us: 2048 x one token in CTAs of one tile 6.2, of two 6.7; 1024 x six 5.8 and 5.3; 4096 x five of two 14.5,
@@ -638,8 +638,9 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
             if (sums <= few_smem_limit<false>()) return few(k_head_mma_few<false>, alone ? 16u : 8u, alone ? 16u : 8u, sums);
         }
         const uint32_t ctas = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
-        return launch_pdl(k_head_mma, dim3(ctas), dim3(kHeadThreads), smem, st, 0u, x, w, out, n_rows, hidden, out_stride, n_tokens,
-                          phases);
+        // (the division of the SM: 129280 x 4096 one token behind the layer kernel 296 us without it, 166 with it)
+        return launch_dependent(k_head_mma, dim3(ctas), dim3(kHeadThreads), smem, st, 0u, smem + sizeof(double) * kHeadPairs * 256u + 1024u, x, w,
+                                out, n_rows, hidden, out_stride, n_tokens, phases);
     }
     const uint32_t blocks = std::min((n_rows + 7u) / 8u, (uint32_t)sm_count * 8u);
     switch (n_tokens) {

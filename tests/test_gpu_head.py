@@ -5,7 +5,11 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from colormlm_b200.s14 import S14Context
+from colormlm_b200 import _lib as L
+from colormlm_b200 import synth
+from colormlm_b200.s14 import S14Context, TokenRoute
+
+from .test_gpu_parity import dev, dev_page, make_layer
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("cuda_lib")]
 
@@ -107,6 +111,39 @@ def test_logits_of_a_vocabulary_shard_have_the_bits_of_the_whole(ctx, tokens, hi
         part = torch.empty(tokens, r1 - r0, device="cuda")
         ctx.cmd_head_logits(x, w[r0:r1], part)
         assert torch.equal(part, whole[:, r0:r1]), (r0, r1)
+
+
+@pytest.mark.parametrize("rows", [4000, 40000])
+def test_logits_behind_a_kernel_that_fills_shared_memory(ctx, rows):
+    """The step of a decode loop: the layer kernel, then the logits as its dependent launch.  The 40000 rows' step took 1.36 times
+    as long as with a kernel in between, because the SMs kept the layer kernel's division and left the loads no L1."""
+    hidden, inter = 4096, 2048
+    g, pages, shared = make_layer(77, hidden, inter, 2, L.PAGE_MXFP4)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    route = TokenRoute([0, 1], np.asarray([0.6, 0.4], np.float32), [p.data_ptr() for p in pages_dev])
+    ctx.set_accumulation(L.ACCUM_PAIRWISE)
+    x, y = dev(synth.activations(g, 1, hidden)), torch.empty(1, hidden, device="cuda")
+    ws = [torch.empty(rows, hidden, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02).view(torch.int16) for _ in range(max(1, 80000 // rows))]
+    out, between = torch.empty(1, rows, device="cuda"), torch.zeros(1, device="cuda")
+
+    def run(apart):
+        times = []
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for w in ws * (80 // len(ws)):
+                ctx.cmd_moe_layer(x, y, [route], shared_dev.data_ptr(), L.PAGE_MXFP4, hidden, inter)
+                if apart:
+                    between.add_(1.0)
+                ctx.cmd_head_logits(y, w, out)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+
+    run(True)
+    assert ctx.last_layer_path & 0xFF == L.LAYER_PATH_TENSOR
+    assert run(False) < 1.15 * run(True)
 
 
 @pytest.mark.parametrize("vocab,offset", [(1, 0), (3, 0), (2047, 1), (4096, 0), (16385, 0), (129280, 0), (129281, 3)])
