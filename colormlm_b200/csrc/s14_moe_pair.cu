@@ -622,13 +622,11 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
     __syncwarp();
     __syncthreads();
     cluster_barrier();
-    if (warp == kPMmaWarp) {
-        // the last commit also arrives in the second CTA, behind the stages' arrivals: none of them is on its way when that
-        // CTA leaves (behind the cluster barrier, because the first CTA may give up a wait's length after the second)
-        if (rank != 0u) mbar_drain(bar(kPBarFin), 0);
-        __syncwarp();
+    // the last commit also arrives in the second CTA, behind the stages' arrivals: none of them is on its way when that
+    // CTA leaves (behind the cluster barrier, because the first CTA may give up a wait's length after the second)
+    if (rank != 0u && warp == kPCodeWarp0) mbar_drain(bar(kPBarFin), 0);
+    if (warp == kPMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
-    }
     if (tid == 0 && abort_flag) {
         atomicExch(status, 0x5507u);
         atomicOr(a.why, kBlockGaveUp);
