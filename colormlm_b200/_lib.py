@@ -185,6 +185,7 @@ SIGNATURES = {
     "s14_exec_routed_and_shared_moe_then_hc_post": (_I32, [_VP, _VP, _P(ExecMoeDesc)]),
     "s14_exec_hc_head_norm_full_logits": (_I32, [_VP, _VP, _P(HcParams), _VP, _VP, _U32, _VP, _VP]),
     "s14_layer_work_list": (_I32, [_U32, _U32, _U32, _U32, _U32, _U32, _VP, _U32, _VP]),
+    "s14_layer_pair_list": (_I32, [_U32, _U32, _U32, _U32, _U32, _U32, _VP, _U32, _VP]),
     "s14_mxfp4_expert_page_from_tensors": (_I32, [_U32, _U32, _VP, _VP]),
     "s14_mxfp4_expert_page_to_tensors": (_I32, [_U32, _U32, _VP, _VP]),
     "s14_validate_ue8m0_codes": (_I32, [_VP, _U64, _P(_U64)]),

@@ -639,6 +639,18 @@ extern "C" int32_t s14_layer_work_list(uint32_t cta, uint32_t n_ctas, uint32_t n
     return S14_OK;
 }
 
+extern "C" int32_t s14_layer_pair_list(uint32_t block, uint32_t n_ctas, uint32_t n_jobs, uint32_t n_early_jobs,
+                                       uint32_t hidden, uint32_t inter, uint32_t *items_out, uint32_t cap,
+                                       uint32_t *count) {
+    if (!count || (cap && !items_out)) return fail(S14_ERR_CONTRACT, "s14_layer_pair_list: NULL argument");
+    if (n_ctas == 0 || block >= n_ctas || (n_ctas & 1u) || (hidden & 511u) || (inter & 511u) || hidden == 0 || inter == 0)
+        return fail(S14_ERR_CONTRACT, "s14_layer_pair_list: block outside the grid, a grid without pairs, or sizes that are not multiples of 512");
+    const uint32_t early_items = std::min(n_early_jobs, n_jobs) * (inter >> 6);
+    *count = layer_pair_list(pair_cta(block, n_ctas, early_items), n_ctas, n_jobs, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8,
+                             items_out, cap, n_early_jobs);
+    return S14_OK;
+}
+
 extern "C" int32_t s14_cmd_moe_layer(s14_ctx *ctx, void *stream, const s14_moe_layer_desc *desc) {
     if (!ctx || !desc) return fail(S14_ERR_CONTRACT, "s14_cmd_moe_layer: NULL argument");
     return enqueue_layer(ctx, stream_of(ctx, stream), *desc, desc->x, desc->y);

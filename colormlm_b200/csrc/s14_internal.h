@@ -155,6 +155,10 @@ bool umma_router_ok(int sm_count, uint32_t n_experts);
 // The items CTA c of G runs, in order (see s14_moe_umma.cu); returns their number, writes at most cap.
 __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT,
                                              uint32_t KU, uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early);
+// ... and where CTAs run in pairs (s14_moe_umma.cu); the number that CTA `b` of the grid has in that deal
+__host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT,
+                                             uint32_t KU, uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early);
+__host__ __device__ uint32_t pair_cta(uint32_t b, uint32_t G, uint32_t F);
 // Both phases and the mix in one launch (y == nullptr: the expert outputs go to d, the caller mixes).
 // With a router the kernel computes the routes itself and the job tables are not read.  add_last [hidden]: a
 // vector that an earlier launch left, added to the mix after the jobs (a shared expert that is not one of them).

@@ -68,6 +68,8 @@ constexpr uint32_t kCntExit = 2;
 constexpr uint32_t kCntEnd = 4;
 constexpr uint32_t kRouterSlots = 2;                 // experts a CTA scores at most
 constexpr uint32_t kItemDown = 0x80000000u;
+constexpr uint32_t kItemHalf = 0x40000000u;        // an up item over half of K: the CTA pair shares it ...
+constexpr uint32_t kItemSecond = 0x20000000u;      // ... and this is the second half, whose sums go to the other CTA
 constexpr uint32_t kTraceWords = 96;   // time marks per CTA of a profiling run
 // The kernel's scratch in global memory, all of it stamped words but the launch count: a head (the
 // launch count, then the expert scores, [2 layer parities][256]), then per job a digit tile (a word
@@ -92,7 +94,8 @@ constexpr uint32_t kBarFin = kBarHFree + 2;           // both issuing threads ha
 constexpr uint32_t kBarRoutes = kBarFin + 1;          // the jobs and the CTA's items are in shared memory
 constexpr uint32_t kBarWr = kBarRoutes + 1;           // the layer's router rows of this CTA are in shared memory
 constexpr uint32_t kBarPages = kBarWr + 1;            // the picked experts' pages are in the job records (early lists)
-constexpr uint32_t kBars = kBarPages + 1;
+constexpr uint32_t kBarPart = kBarPages + 1;          // the other CTA's sums of a shared up item are in s_part
+constexpr uint32_t kBars = kBarPart + 1;
 constexpr uint32_t kRouteWarp = 15;                   // the warp that publishes the CTA's expert scores
 
 // Instruction descriptor: A and B E2M1 (format 1), both K-major, N = 16, UE8M0 scales, M = 128.
@@ -154,12 +157,67 @@ __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_
     return n;
 }
 
+// The deal where CTAs run in pairs (clusters of two).  Up items that do not go round evenly give some CTAs a whole item
+// more than the others (the benchmark's layer: 192 routed items over 148 CTAs, 44 of them with 32 units where the others have
+// 16), and the layer waits for those: an SM takes in 83 GB/s whatever the others do (eight units in flight), 3.4 us for the
+// second item.  A pair shares such an item along K: the CTA that the deal above gives it to takes the first half of its units
+// and finishes it, its partner the second half.  The two CTAs of a pair both hold early items or neither does (pair_cta), and
+// only the latter share, because an early item makes its CTA late (partners half the grid apart, some of them with early items:
+// no gain); so there may be at most as many shared items as such pairs, and half an item has to have an even number of units.
+// Otherwise the lists are those above.  The down items: the CTAs without a half first take what levels the units (of the jobs
+// that are finished first), the rest goes round all CTAs, those first (those last: 342 us).  14 layers of 4096 x 2048 in one
+// launch: 348.3 us, with shared items 338.5.
+//
+// CTA `b` of the grid as the deal numbers it: the first F / 2 pairs hold the F early items, two neighbouring numbers each; the
+// numbers of the other pairs lie half of those CTAs apart.
+__host__ __device__ uint32_t pair_cta(uint32_t b, uint32_t G, uint32_t F) {
+    if (F > G) F = 0u;   // (every CTA holds early items)
+    return b < F ? b : F + ((b - F) >> 1) + (b & 1u) * ((G - F) >> 1);
+}
+// CTA c's items as above, bit 30 set for a shared up item, bit 29 too for its second half.
+__host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU,
+                                             uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early) {
+    if (n_early > n_jobs) n_early = n_jobs;
+    const uint32_t U = n_jobs * S, D = n_jobs * RT, F = n_early * S;
+    const uint32_t a_full = G ? (U - F) / G : 0u, r = G ? (U - F) % G : 0u;
+    const uint32_t P = F > G ? 0u : (G - F) / 2u;   // pairs without early items
+    if ((G & 1u) || (F & 1u) || (KU & 3u) || r == 0u || r > P) return layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, cap, n_early);
+    uint32_t n = 0;
+    auto put = [&](uint32_t v) {
+        if (n < cap) items[n] = v;
+        ++n;
+    };
+    const uint32_t c_rot = (c + G - F) % G;
+    const bool first = c_rot < r, second = c_rot >= P && c_rot - P < r;
+    for (uint32_t q = c; q < U; q += G) {
+        const bool half = q >= F + a_full * G;   // of the last, incomplete round
+        put((half ? kItemHalf : 0u) | ((q / S) << 8) | (q % S));
+    }
+    if (second) {
+        const uint32_t q = F + a_full * G + (c_rot - P);
+        put(kItemHalf | kItemSecond | ((q / S) << 8) | (q % S));
+    }
+    // the CTAs without a half, `plain` numbers them; and every CTA's place when the rest goes round
+    const uint32_t n_plain = G - 2u * r, plain = c_rot < P ? c_rot - r : c_rot - 2u * r;
+    const uint32_t pos = second ? n_plain + r + c_rot - P : first ? n_plain + c_rot : plain;
+    auto put_down = [&](uint32_t p) { put(kItemDown | ((p / RT) << 8) | (p % RT)); };
+    uint32_t ahead = (KU / 2u + KD / 2u) / KD * n_plain;
+    const uint32_t ready = RT * (n_early + a_full * G / S);
+    if (ahead > ready) ahead = ready;
+    if (ahead > D) ahead = D;
+    if (!first && !second)
+        for (uint32_t p = plain; p < ahead; p += n_plain) put_down(p);
+    for (uint32_t p = ahead + pos; p < D; p += G) put_down(p);
+    return n;
+}
+
 namespace {
 
 // the one device copy of the deal (its divisions make it long; a CTA calls it once)
 __device__ __noinline__ uint32_t work_list_once(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU,
-                                                uint32_t KD, uint32_t *items, uint32_t n_early) {
-    const uint32_t n = layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
+                                                uint32_t KD, uint32_t *items, uint32_t n_early, uint32_t paired) {
+    const uint32_t n = paired ? layer_pair_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early)
+                              : layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
     return n < kMaxItems ? n : kMaxItems;
 }
 // Nothing on the kernel's paths may live in local memory: nearly all of the SM's L1 is carved out as
@@ -167,6 +225,23 @@ __device__ __noinline__ uint32_t work_list_once(uint32_t c, uint32_t G, uint32_t
 // an L2 round trip (measured: a 100-instruction block went from 0.25 to 3 microseconds).  Helpers are
 // inlined, arrays are indexed by unrolled loops, and only code that runs once per launch or layer
 // with little live state (the deal, the route records) is kept out of line.
+// And straight code that every warp meets once a layer is fetched again each time, about four cycles an instruction: the
+// counting loops of the selection and the copying thread's two steps are loops, not copies (14 layers 338 us, so 332.5).  That
+// is no rule for code whose operations overlap when it is unrolled (tensor-memory loads and their sums, the digits' halves, the
+// router's two rows: 1-2 us more as loops), and a chain of F32 operations in place of the FP64 ones of the SwiGLU and of
+// the digit sums, which pays in the block kernels, is longer here (339 and 343 us).
+
+// The two CTAs of a cluster.  The cluster barrier's halves, executed by every thread.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// v into the same variable of CTA `rank` of the cluster, counted in bytes on that CTA's barrier
+__device__ __forceinline__ void st_async_partner(uint32_t addr, double v, uint32_t bar, uint32_t rank) {
+    uint32_t a, b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar), "r"(rank));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a), "l"(__double_as_longlong(v)), "r"(b)
+                 : "memory");
+}
 
 // 512 threads = 16 warps, four per sub-partition of the SM: up to 128 registers per thread.
 template <bool kTrace>
@@ -176,12 +251,13 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                  unsigned int *counters, uint32_t *__restrict__ status, uint32_t hidden, uint32_t inter,
                  uint32_t ring, unsigned long long *trace, const __grid_constant__ FusedRouter rt,
                  const __grid_constant__ EpExchange ep, const StackLayer *__restrict__ stack, uint32_t n_layers,
-                 float *hbuf, uint32_t residual, const float *add_last) {
+                 float *hbuf, uint32_t residual, const float *add_last, uint32_t paired) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kBars];
     __shared__ __align__(16) uint8_t sE[kExpMax];        // block exponents of the token's digits
     __shared__ __align__(16) uint8_t sEh[2][kExpMax];    // ... of the digit tiles of hidden values
     __shared__ __align__(16) uint8_t s_hst[16 * 2 * 16]; // an up item's digit chunks: [row][block][16 bytes]
+    __shared__ __align__(8) double s_part[kEpiThreads];  // the partner's sums of a shared up item
     __shared__ float s_up[64];                           // an item's up projection, handed to the gate threads
     // per layer parity: the mix, in route order: weight (shared expert: 1) and row of the expert
     // outputs, bit 31 set for the shared expert; the layer's jobs, from the routes or the caller's table
@@ -191,6 +267,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     __shared__ uint32_t s_n_mix, s_n_jobs;
     __shared__ uint32_t s_items[kMaxItems];
     __shared__ uint32_t s_n_items;
+    __shared__ uint32_t s_part_armed, s_part_used;       // shared up items armed and finished so far, one per layer
     __shared__ unsigned long long s_page[S14_N_ROUTED_EXPERTS];  // the layer's page table, parked a layer ahead
     __shared__ float s_bias[S14_N_ROUTED_EXPERTS];       // the layer's bias, likewise
     __shared__ StackLayer s_layer[2];                    // the layer's own pointers, by layer parity
@@ -206,12 +283,20 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     __shared__ uint32_t s_abort_code;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t grid = gridDim.x, cta = blockIdx.x;
+    const uint32_t grid = gridDim.x;
     const uint32_t KU = hidden >> 8;   // units of an up item
     const uint32_t KD = inter >> 8;    // units of a down item
     const uint32_t RT = hidden >> 7;   // row tiles of w2
     const uint32_t S = inter >> 6;     // slices of an expert
     const uint32_t L = n_layers ? n_layers : 1u;
+    const bool routes_here = rt.weight != nullptr || stack != nullptr;
+    const bool table_param = !routes_here && dev_table == nullptr;
+    // the CTA's items are known at once unless the number of jobs depends on the routes (expert
+    // parallel: a rank keeps the experts it owns) or the table comes from an earlier kernel
+    const bool early = table_param || (routes_here && rt.ep_world <= 1u);
+    // the shared expert of a layer that picks its own routes: its up items run while the routes are picked
+    const uint32_t n_early_jobs = (early && routes_here && rt.has_shared) ? 1u : 0u;
+    const uint32_t cta = paired ? pair_cta(blockIdx.x, grid, n_early_jobs * S) : blockIdx.x;   // as the deal numbers it
     uint8_t *const sRing = smem;
     uint8_t *const sBx = smem + ring * kSlot;   // the token's digit tile, 2 KB per 256 K-elements
     uint8_t *const sBh = sBx + KU * 2048u;      // two digit tiles of hidden values
@@ -260,14 +345,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
 
     // Thread t < 512 owns elements 8t .. 8t+7 of the token (hidden <= 4096), for the digits and for
     // the router's dot products.
-    const bool routes_here = rt.weight != nullptr || stack != nullptr;
     const bool ep_on = ep.world > 1u;
-    const bool table_param = !routes_here && dev_table == nullptr;
-    // the CTA's items are known at once unless the number of jobs depends on the routes (expert
-    // parallel: a rank keeps the experts it owns) or the table comes from an earlier kernel
-    const bool early = table_param || (routes_here && rt.ep_world <= 1u);
-    // the shared expert of a layer that picks its own routes: its up items run while the routes are picked
-    const uint32_t n_early_jobs = (early && routes_here && rt.has_shared) ? 1u : 0u;
     const bool has_x = tid < (hidden >> 3);
     const bool is_producer = tid == kProdWarp * 32u;
     // The kernel is launched as a programmatic dependent of whatever precedes it in the stream: its
@@ -283,9 +361,10 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     if (tid < kBars) {
         uint32_t count = 1u;  // ring slots, routes
         if (tid >= kBarAccDone && tid < kBarAccDone + 2u) count = 2u;
-        else if (tid >= kBarAccFree && tid < kBarAccFree + 2u) count = kEpiThreads;
-        else if (tid == kBarXReady) count = 256u;
-        else if (tid >= kBarHReady && tid < kBarHReady + 2u) count = kLoadThreads;
+        // (one arrival per warp where whole warps arrive: 256 of them take a third of a microsecond)
+        else if (tid >= kBarAccFree && tid < kBarAccFree + 2u) count = kEpiThreads / 32u;
+        else if (tid == kBarXReady) count = 8u;
+        else if (tid >= kBarHReady && tid < kBarHReady + 2u) count = kLoadThreads / 32u;
         else if (tid >= kBarHFree && tid < kBarHFree + 2u) count = 2u;
         else if (tid == kBarFin) count = 2u;
         mbar_init(bar(tid), count);
@@ -313,6 +392,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             s_n_items = 0;
             s_n_jobs = 0;
             s_n_mix = 0;
+            s_part_armed = s_part_used = 0;
         }
         if (lane < 8u) s_prod[lane] = lane == 6u ? 1u : 0u;  // nothing issued yet, no wait has run out
         __syncwarp();
@@ -334,10 +414,11 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             nj = rt.top_k + (rt.has_shared ? 1u : 0u);
             if (lane == 0) s_n_jobs = nj;
         }
-        if (early && lane == 1u) s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, n_early_jobs);
+        if (early && lane == 1u) s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, n_early_jobs, paired);
     }
     __syncwarp();
     __syncthreads();
+    if (paired) cluster_arrive();  // this CTA's barriers are there
     if (tid == 0) mark(2);
     // a caller's table is complete now; otherwise the routes barrier opens when the routes are picked
     if (tid == 32u && table_param) mbar_arrive(bar(kBarRoutes));
@@ -401,9 +482,10 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             if (p_i >= n_it) break;
             const uint32_t item = s_items[p_i], j = (item >> 8) & 0xFFu, idx = item & 0xFFu;
             const bool down = (item & kItemDown) != 0u;
-            const uint32_t nu = down ? KD : KU;
+            const uint32_t nu = down ? KD : (item & kItemHalf) ? KU >> 1 : KU;
             const uint8_t *page = (!routes_known && !table_param) ? s_layer[par_l].shared_page : s_jobs[par_l][j].page;
-            const uint8_t *a = page + (down ? mxfp4_down_offset(hidden, inter) : 0u) + ((size_t)idx * nu + p_u) * kUnitStride;
+            const uint32_t from = (item & kItemSecond) ? nu : 0u;
+            const uint8_t *a = page + (down ? mxfp4_down_offset(hidden, inter) : 0u) + ((size_t)idx * (down ? KD : KU) + from + p_u) * kUnitStride;
 #pragma unroll 1
             for (; p_u < nu; ++p_u) {
                 if (head) {
@@ -481,6 +563,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 }
             }
             if (l == 0u) {
+                __syncwarp();
+                if (paired) cluster_wait();  // the partner's barriers are there, too
                 cudaGridDependencySynchronize();
                 if (tid == 0) {
                     s_ep_step = ep_on ? __ldcg(ep.step) : 0u;
@@ -625,7 +709,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             if (warp < 8u) {
                 store_digit_scales(tmem + kColSfbX, sE, hidden, warp & 3u, warp >> 2, 2u, lane);
                 fence_before();
-                mbar_arrive(bar(kBarXReady));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kBarXReady));
             }
             if (tid == 0) mark(6);
             if (routes_here && warp >= kLoadWarp0) {
@@ -656,7 +741,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     // Selection by counting, no serial rounds.  A key is (score + bias as an ordered integer,
                     // ~id): all keys differ, a larger key comes first.  Thread e counts the keys of its warp's
                     // 32 experts that beat its own; the experts of rank < top_k within a warp are the warp's
-                    // candidates (slot = warp * 8 + rank).  Then one thread per candidate slot counts the
+                    // candidates (slot = warp * 8 + rank).  Then four threads per candidate slot count the
                     // candidates that beat it: rank < top_k among the candidates = the route of that rank.
                     unsigned long long *s_cand = reinterpret_cast<unsigned long long *>(sBh);              // [64] keys, 0 = none
                     float *s_cand_score = reinterpret_cast<float *>(sBh + 512);                            // [64]
@@ -678,7 +763,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     {
                         uint32_t rank = 0;
                         const ulonglong2 *row = reinterpret_cast<const ulonglong2 *>(s_keys + wl * 32u);
-#pragma unroll
+#pragma unroll 4
                         for (uint32_t i = 0; i < 16; ++i) {
                             const ulonglong2 v = row[i];
                             rank += (v.x > key ? 1u : 0u) + (v.y > key ? 1u : 0u);
@@ -691,21 +776,25 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     }
                     if (lt == 0) mark(69);
                     load_sync();
-                    if (lt < 64u) {
-                        const unsigned long long mine = s_cand[lt];
+                    {
+                        // four threads per slot, each counts a quarter of the slots
+                        const uint32_t at = lt >> 2;
+                        const unsigned long long mine = s_cand[at];
                         uint32_t rank = 0;
-                        const ulonglong2 *row = reinterpret_cast<const ulonglong2 *>(s_cand);
-#pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) {
+                        const ulonglong2 *row = reinterpret_cast<const ulonglong2 *>(s_cand) + (lt & 3u) * 8u;
+#pragma unroll 4
+                        for (uint32_t i = 0; i < 8; ++i) {
                             const ulonglong2 v = row[i];
                             rank += (v.x > mine ? 1u : 0u) + (v.y > mine ? 1u : 0u);
                         }
-                        if (mine != 0ull && rank < rt.top_k) {
+                        rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+                        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+                        if ((lt & 3u) == 0u && mine != 0ull && rank < rt.top_k) {
                             s_pick_id[rank] = 0xffffffffu - (uint32_t)mine;
-                            s_pick_score[rank] = s_cand_score[lt];
-                            s_pick_page[rank] = s_cand_page[lt];
+                            s_pick_score[rank] = s_cand_score[at];
+                            s_pick_page[rank] = s_cand_page[at];
                             // (no expert parallelism: the job of route `rank` follows the shared expert's)
-                            if (early) s_jobs[par][n_early_jobs + rank].page = reinterpret_cast<const uint8_t *>(s_cand_page[lt]);
+                            if (early) s_jobs[par][n_early_jobs + rank].page = reinterpret_cast<const uint8_t *>(s_cand_page[at]);
                         }
                     }
                     load_sync();  // the picks are written; every candidate's page has been read
@@ -764,7 +853,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                         }
                         __syncwarp();
                         if (lane == 0 && !early)
-                            s_n_items = work_list_once(cta, grid, s_n_jobs, S, RT, KU, KD, s_items, 0u);
+                            s_n_items = work_list_once(cta, grid, s_n_jobs, S, RT, KU, KD, s_items, 0u, paired);
                         __syncwarp();
                     }
                 } else if (lt == 0) {
@@ -794,7 +883,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (lane == 0) {
                     s_n_jobs = nj;
                     s_n_mix = nm;
-                    s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, 0u);
+                    s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, 0u, paired);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(kBarRoutes));
@@ -832,10 +921,11 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     const uint32_t gi = gi0 + i;
                     const uint32_t item = warp_uniform(s_items[i]), j = (item >> 8) & 0xFFu, buf = gi & 1u;
                     const bool down = (item & kItemDown) != 0u;
-                    const uint32_t nu = down ? KD : KU;
+                    const uint32_t nu = down ? KD : (item & kItemHalf) ? KU >> 1 : KU;
                     if (gi >= 2u) ok = mbar_wait_warp(bar(kBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
-                    uint64_t b_desc0 = bx_desc0;
-                    uint32_t sfb0 = tm + kColSfbX;
+                    const uint32_t from = (item & kItemSecond) ? nu : 0u;   // units of K in front of this half
+                    uint64_t b_desc0 = bx_desc0 + from * (2048u >> 4);
+                    uint32_t sfb0 = tm + kColSfbX + from * 8u;
                     bool last_user = false;
                     if (down) {
                         if (j != cur_job) {
@@ -958,8 +1048,26 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                         sum += lo + hi;
                     }
                     fence_before();
-                    mbar_arrive(bar(kBarAccFree + buf));
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kBarAccFree + buf));
                     if (tid == 0) mark(52u + i);
+                    if (item & kItemHalf) {
+                        // An item that the pair shares: the second half's sums go into the first CTA's shared memory, each
+                        // store counted on its barrier.  One such item per CTA and layer; the next layer's token depends on
+                        // these sums, so they have been read when the partner's next ones arrive.
+                        if (item & kItemSecond) {
+                            st_async_partner(smem_u32(&s_part[row]), sum, bar(kBarPart), (blockIdx.x & 1u) ^ 1u);
+                            continue;
+                        }
+                        if (tid == 0) {
+                            mbar_arrive_expect(bar(kBarPart), kEpiThreads * (uint32_t)sizeof(double));
+                            s_part_armed = l + 1u;
+                        }
+                        ok = epi_all(mbar_wait(bar(kBarPart), par, abortp));
+                        if (!ok) break;
+                        if (tid == 0) s_part_used = l + 1u;
+                        sum += s_part[row];
+                    }
                     const float v = (float)sum;
                     if (!down) {
                         // lanes 0-63: gate of the slice's element `row`; lanes 64-127: its up projection
@@ -1151,11 +1259,10 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     ok = load_all(mine);
                     if (!ok) break;
                     if (lt == 0) mark(46u + i);
-                    if (warp < kLoadWarp0 + 4u) {
-                        store_digit_scales(tmem + kColSfbH + hb * 128u, sEh[hb], inter, warp & 3u, 0u, 1u, lane);
-                        fence_before();
-                    }
-                    mbar_arrive(bar(kBarHReady + hb));
+                    store_digit_scales(tmem + kColSfbH + hb * 128u, sEh[hb], inter, warp & 3u, (warp - kLoadWarp0) >> 2, 2u, lane);
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kBarHReady + hb));
                     if (lt == 0) mark(19u + i * 4u);
                     cur_job = j;
                     ++n_loaded;
@@ -1166,8 +1273,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 // shared expert (its address is known) is asked into the L2, where that layer's copies find
                 // it a layer-time later instead of taking HBM time from the routed experts' stream.
                 if (n_early_jobs && l + 1u < L) prefetch_shared(s_layer[par ^ 1u].shared_page);
-                produce(l, false);
-                if (l + 1u < L) produce(l + 1u, true);
+#pragma unroll 1
+                for (uint32_t k = 0; k < 2u && l + k < L; ++k) produce(l + k, k != 0u);
                 if (l + 1u == L) mark(12);
             }
             // the other lanes of its warp wait here (a warp barrier, no polling) until it has finished:
@@ -1199,6 +1306,14 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     fence_before();
     __syncwarp();  // the copying and the issuing threads rejoin their warps
     __syncthreads();
+    if (tid == 0 && abort_flag) {
+        // given up: the partner's sums of a shared item may be on their way
+        for (uint32_t i = 0; i < s_n_items; ++i) {
+            if ((s_items[i] & (kItemHalf | kItemSecond)) != kItemHalf) continue;
+            if (s_part_armed == s_part_used) mbar_arrive_expect(bar(kBarPart), kEpiThreads * (uint32_t)sizeof(double));
+            mbar_drain(bar(kBarPart), s_part_used & 1u);
+        }
+    }
     if (tid == 0) mark(13);
     if (warp == kMmaWarp0) {
         __syncwarp();
@@ -1243,6 +1358,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     }
     __syncwarp();
     __syncthreads();
+    if (paired) cluster_arrive();   // nothing of this CTA is on its way to its partner's shared memory
     // the last CTA to leave puts the counters back to zero for the next launch
     if (tid == 0) {
         if (abort_flag) atomicExch(status, s_abort_code);
@@ -1265,20 +1381,31 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (p != ep.rank) st_relaxed_sys(ep.slots[p] + credit + ep.rank, (unsigned long long)(s_ep_step + 1u));
         }
     }
+    __syncwarp();
+    if (paired) cluster_wait();   // a CTA stays until its partner writes nothing into it any more
 }
 
 template <class Kernel, class... Args>
-cudaError_t launch_layer(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, Args... args) {
+cudaError_t launch_layer(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, bool paired, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    if (pdl) {
+        cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+        a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        a.val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (paired) {
+        cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = 2;
+        a.val.clusterDim.y = 1;
+        a.val.clusterDim.z = 1;
+    }
     return launch_status(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
@@ -1302,6 +1429,31 @@ size_t dynamic_limit() {
     if (cudaFuncSetAttribute(k_moe_layer_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
     g_dynamic_limit[dev] = most;
     return most;
+}
+
+// Whether the grid runs as clusters of two, all of them resident at a time, because the CTAs wait for one another (asked once
+// per device, with the most shared memory a launch may have).
+bool pairs_resident(int sm_count) {
+    static int pairs[kMaxDevices] = {};   // 0: not asked yet, else one more than the clusters that fit
+    int dev = -1;
+    if ((sm_count & 1) || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    if (!pairs[dev]) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(sm_count);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = dynamic_limit();
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (launch_status(cudaOccupancyMaxActiveClusters(&n, k_moe_layer_umma<false>, &cfg)) != cudaSuccess) n = 0;
+        pairs[dev] = n + 1;
+    }
+    return 2 * (pairs[dev] - 1) >= sm_count;
 }
 
 // shared memory beside the ring: the token's digit tile, two tiles of hidden values, two router rows
@@ -1337,6 +1489,8 @@ bool umma_layer_ok(int sm_count, uint32_t n_tokens, uint32_t n_jobs_max, uint32_
     for (uint32_t c = 0; c < (uint32_t)sm_count; ++c)
         for (uint32_t n_early = 0; n_early < 2u; ++n_early)
             if (layer_work_list(c, (uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8, items, 0,
+                                n_early) > kMaxItems ||
+                layer_pair_list(c, (uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8, items, 0,
                                 n_early) > kMaxItems)
                 return false;
     return ring_slots(hidden, inter, dynamic_limit()) >= 2u;
@@ -1368,13 +1522,14 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     // paths (exchange inside the kernel, or expert outputs handed to a collective) are ordinary
     // launches; the kernel's own dependency calls are then no-ops.
     const bool pdl = ex.world <= 1u && y != nullptr;
+    const bool paired = pairs_resident(sm_count);
     if (trace)
-        return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
+        return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
                           counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                          residual ? 1u : 0u, add_last);
-    return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, dev, param, x, d, y, tiles,
+                          residual ? 1u : 0u, add_last, paired ? 1u : 0u);
+    return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
                       counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                      residual ? 1u : 0u, add_last);
+                      residual ? 1u : 0u, add_last, paired ? 1u : 0u);
 }
 
 }  // namespace s14
