@@ -608,7 +608,7 @@ static void build_job_table(const s14_moe_layer_desc &desc, JobTable &tab) {
 }
 
 static int32_t enqueue_layer(s14_ctx *ctx, cudaStream_t st, const s14_moe_layer_desc &desc, const float *x, float *y,
-                             const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr) {
+                             const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr, BranchPost *post = nullptr) {
     S14_TRY
     JobTable tab;
     build_job_table(desc, tab);
@@ -620,7 +620,7 @@ static int32_t enqueue_layer(s14_ctx *ctx, cudaStream_t st, const s14_moe_layer_
     const int launched = launch_moe_layer(st, ctx->mode, ctx->sm_count, nullptr, tab, tab.n_tokens,
                                           tab.n_jobs, desc.hidden, desc.inter, x, ctx->h, ctx->d, y,
                                           &err, nullptr, all_mxfp4, ctx->counters, ctx->umma_scratch(), nullptr, nullptr, x_bf16,
-                                          x_stage);
+                                          x_stage, post);
     ctx->last_path = last_layer_path();
     ctx->launches += launched;
     if (err != cudaSuccess) return cuda_fail(err, "S14 MoE layer launch");
@@ -2326,8 +2326,10 @@ extern "C" int32_t s14_exec_routed_and_shared_moe_then_hc_post(s14_ctx *ctx, voi
     ld.shared_kind = d->shared_kind;
     ld.shared_page = d->shared_page;
     ld.routes = d->route;
-    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->y_stage, d->ffn_input_bf16, ctx->x_stage);
+    BranchPost post = {d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb, d->state_out_bf16, false};
+    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->y_stage, d->ffn_input_bf16, ctx->x_stage, &post);
     if (rc != S14_OK) return rc;
+    if (post.done) return S14_OK;
     CUDA_OK(launch_branch_post(st, d->hidden, ctx->y_stage, d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb,
                                d->state_out_bf16));
     ctx->launches += 1;

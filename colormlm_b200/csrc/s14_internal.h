@@ -120,22 +120,32 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                      cudaError_t *err, const KernelMarks *km = nullptr, bool all_mxfp4 = false,
                      unsigned int *counters = nullptr, const struct UmmaScratch *umma = nullptr,
                      const FusedRouter *router = nullptr, const EpExchange *ep = nullptr,
-                     const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr);
-// (x_bf16, x_stage: the token as BF16; its F32 values are written to x_stage, which is x)
-// Whether a one-token layer with an FP8 shared page runs it by kernels of its own in front of the tensor-core layer
-// kernel, which runs the routed experts and adds the shared expert's output last.
+                     const uint16_t *x_bf16 = nullptr, float *x_stage = nullptr, struct BranchPost *post = nullptr);
+// (x_bf16, x_stage: the token as BF16; its F32 values may be written to x_stage, which is x)
+// What the executor's step does with a layer's output: rounded to BF16 (branch_out, or NULL), then hc_post over the
+// post-attention state.  A path that does it in its last launch, without writing y, sets `done`.
+struct BranchPost {
+    uint16_t *branch_out;
+    const void *residual;
+    const float *post, *comb;
+    void *merged;
+    bool done;
+};
+// Whether a one-token layer with an FP8 shared page runs it by kernels of its own behind the tensor-core layer
+// kernel, which runs the routed experts; the last one adds the shared expert's output to theirs.
 bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const struct UmmaScratch *umma, uint32_t n_routed, uint32_t hidden, uint32_t inter);
 // That layer (three launches): the routed experts' jobs, or a router without the shared expert.  h: [inter], d:
 // [kMaxJobs, hidden] scratch.
 int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
-                            const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
-                            unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err);
-// One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or x_bf16 with its F32 values left in x_out;
-// h [inter] scratch, d [hidden] the expert's output.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary, x_bf16
-// (or NULL) on an 8-byte one.
+                            const float *x, const uint16_t *x_bf16, float *h, float *d, float *y,
+                            unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err,
+                            BranchPost *post = nullptr);
+// One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or BF16 as x_bf16; h [inter] scratch; the expert's
+// output added to `routed` [hidden] goes to y, or through `post`.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary,
+// x_bf16 (or NULL) on an 8-byte one.
 inline bool fp8_expert_takes(const uint16_t *x_bf16) { return (reinterpret_cast<uintptr_t>(x_bf16) & 7u) == 0u; }
-cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, float *x_out, const uint8_t *page,
-                              float *h, float *d, uint32_t hidden, uint32_t inter);
+cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, const uint8_t *page,
+                              float *h, const float *routed, float *y, const BranchPost *post, uint32_t hidden, uint32_t inter);
 // Scratch of the tcgen05 layer kernel (s14_moe_umma.cu): per job the digit tile of its hidden
 // values and the tile's block exponents (umma_scratch_bytes), and the device status word a
 // timed-out wait sets.
@@ -160,15 +170,16 @@ __host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_
                                              uint32_t KU, uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early);
 __host__ __device__ uint32_t pair_cta(uint32_t b, uint32_t G, uint32_t F);
 // Both phases and the mix in one launch (y == nullptr: the expert outputs go to d, the caller mixes).
-// With a router the kernel computes the routes itself and the job tables are not read.  add_last [hidden]: a
-// vector that an earlier launch left, added to the mix after the jobs (a shared expert that is not one of them).
+// With a router the kernel computes the routes itself and the job tables are not read.  x_bf16: the token as BF16 values (x is
+// not read then), on an 8-byte boundary.  ahead: bytes that the launches behind will read, asked into the L2 when the kernel's own
+// copies are under way; on a 16-byte boundary.
 cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable *dev, const JobTable &param,
                                   const float *x, float *d, float *y, uint8_t *tiles, unsigned int *counters,
                                   uint32_t *status, uint32_t hidden, uint32_t inter,
                                   const FusedRouter *router = nullptr, const EpExchange *ep = nullptr,
                                   unsigned long long *trace = nullptr, const StackLayer *stack = nullptr,
                                   uint32_t n_layers = 1, float *hbuf = nullptr, bool residual = false,
-                                  const float *add_last = nullptr);
+                                  const uint16_t *x_bf16 = nullptr, const uint8_t *ahead = nullptr, size_t ahead_bytes = 0);
 int launch_router(cudaStream_t st, const s14_router_desc &r, float *scores, float *select,
                   JobTable *table_out, const uint8_t *const *page_table, const uint8_t *shared_page,
                   uint32_t shared_kind, unsigned int *counter, cudaError_t *err,

@@ -1103,7 +1103,7 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                      uint32_t hidden, uint32_t inter, const float *x, float *h, float *d, float *y,
                      cudaError_t *err, const KernelMarks *km, bool all_mxfp4, unsigned int *counters,
                      const UmmaScratch *umma, const FusedRouter *router, const EpExchange *ep, const uint16_t *x_bf16,
-                     float *x_stage) {
+                     float *x_stage, BranchPost *post) {
     int launches = 0;
     *err = cudaSuccess;
     t_last_layer_path = 0;
@@ -1144,8 +1144,8 @@ int launch_moe_layer(cudaStream_t st, uint32_t mode, int sm_count, const JobTabl
                 x_bf16 = nullptr;
             }
             if (km) cudaEventRecord(km->ev[0], st), cudaEventRecord(km->ev[1], st);
-            launches += launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, x_stage, h, d, y,
-                                                counters, umma, hidden, inter, err);
+            launches += launch_layer_fp8_shared(st, sm_count, routed, router ? &rt : nullptr, shared, x, x_bf16, h, d, y,
+                                                counters, umma, hidden, inter, err, post);
             if (km)  // as for the layer kernel alone (below): all of it is booked as the up phase
                 for (int i = 2; i < 5; ++i) cudaEventRecord(km->ev[i], st);
             t_last_layer_path = S14_LAYER_PATH_TENSOR | S14_LAYER_PATH_FP8_SHARED_KERNEL;
@@ -1284,13 +1284,17 @@ bool fp8_shared_layer_ok(int sm_count, uint32_t mode, const UmmaScratch *umma, u
 }
 
 int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &routed, const FusedRouter *router, const uint8_t *shared_page,
-                            const float *x, const uint16_t *x_bf16, float *x_stage, float *h, float *d, float *y,
-                            unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err) {
-    float *shared_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
-    *err = launch_fp8_expert(st, sm_count, x, x_bf16, x_stage, shared_page, h, shared_out, hidden, inter);
+                            const float *x, const uint16_t *x_bf16, float *h, float *d, float *y,
+                            unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err,
+                            BranchPost *post) {
+    // The layer kernel first: see s14_fp8_expert.cu.  y may be x: it is written last.
+    float *routed_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
+    const size_t page_bytes = 3u * ((size_t)hidden * inter + (size_t)(hidden >> 7) * (inter >> 7));
+    *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, routed_out, umma->tiles, counters, umma->status, hidden, inter, router,
+                                 nullptr, umma->trace, nullptr, 1, nullptr, false, x_bf16, shared_page, page_bytes);
     if (*err != cudaSuccess) return 0;
-    *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, y, umma->tiles, counters, umma->status, hidden, inter, router,
-                                 nullptr, umma->trace, nullptr, 1, nullptr, false, shared_out);
+    *err = launch_fp8_expert(st, sm_count, x, x_bf16, shared_page, h, routed_out, y, post, hidden, inter);
+    if (post && *err == cudaSuccess) post->done = true;
     return 3;
 }
 

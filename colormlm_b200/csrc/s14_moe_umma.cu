@@ -66,6 +66,7 @@ constexpr uint32_t kSpinGlobal = 1u << 20;  // polls (100 ns apart) of a counter
 // the context's counter array ([0] is the router kernel's); [1, kCntEnd) are zero between launches
 constexpr uint32_t kCntExit = 2;
 constexpr uint32_t kCntEnd = 4;
+constexpr uint32_t kAheadPiece = 16384;             // bytes of `ahead` per request
 constexpr uint32_t kRouterSlots = 2;                 // experts a CTA scores at most
 constexpr uint32_t kItemDown = 0x80000000u;
 constexpr uint32_t kItemHalf = 0x40000000u;        // an up item over half of K: the CTA pair shares it ...
@@ -251,7 +252,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                  unsigned int *counters, uint32_t *__restrict__ status, uint32_t hidden, uint32_t inter,
                  uint32_t ring, unsigned long long *trace, const __grid_constant__ FusedRouter rt,
                  const __grid_constant__ EpExchange ep, const StackLayer *__restrict__ stack, uint32_t n_layers,
-                 float *hbuf, uint32_t residual, const float *add_last, uint32_t paired) {
+                 float *hbuf, uint32_t residual, const uint16_t *x_bf16, const uint8_t *ahead, uint32_t ahead_bytes, uint32_t paired) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kBars];
     __shared__ __align__(16) uint8_t sE[kExpMax];        // block exponents of the token's digits
@@ -354,7 +355,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     // have written (the token, the counters, a device job table, the step count) is read only after
     // cudaGridDependencySynchronize() below.  In the same way the next launch may be set up from now
     // on.  Weights and page tables are constant during a step.
-    cudaTriggerProgrammaticLaunchCompletion();
+    // (`ahead`: see below)
+    if (ahead_bytes == 0u) cudaTriggerProgrammaticLaunchCompletion();
 
     // ---- set-up: the barriers by the first threads, the jobs and items that are known at launch
     // by warp 1 ----
@@ -520,6 +522,19 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
 #pragma unroll 1
         for (uint32_t u = cta; u < units; u += grid) l2_prefetch(page + (size_t)u * kUnitStride, kUnitStride);
     };
+    if (ahead_bytes != 0u) {
+        // A layer whose shared expert runs in the launches behind.  The first of them does not wait before it reads the token and
+        // the shared page: it may start when this kernel has waited, that is when everything in front of this one is complete.  And
+        // pages, tables and router rows are read behind the wait here, as by those launches; in front of it there is a hint.
+        if (is_producer && table_param && s_n_items) {
+            const uint32_t item = s_items[0];
+            const uint32_t nu = (item & kItemHalf) ? KU >> 1 : KU, from = (item & kItemSecond) ? nu : 0u;
+            l2_prefetch(s_jobs[0][(item >> 8) & 0xFFu].page + ((size_t)(item & 0xFFu) * KU + from) * kUnitStride, min(nu, ring) * kUnitStride);
+        }
+        __syncwarp();
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+    }
     if (is_producer) {
         if (n_early_jobs) prefetch_shared(s_layer[0].shared_page);  // the first layer's, before the token is there
         if (routes_here) {
@@ -558,8 +573,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (warp >= kLoadWarp0 && tid - kLoadWarp0 * 32u < rt.n_experts) {
                     const float *l_bias = stack ? stack[0].bias : rt.bias;
                     const uint8_t *const *l_table = stack ? stack[0].page_table : rt.page_table;
-                    s_page[tid - kLoadWarp0 * 32u] = __ldg(reinterpret_cast<const unsigned long long *>(l_table) + (tid - kLoadWarp0 * 32u));
-                    s_bias[tid - kLoadWarp0 * 32u] = l_bias ? __ldg(l_bias + (tid - kLoadWarp0 * 32u)) : 0.0f;
+                    s_page[tid - kLoadWarp0 * 32u] = __ldcg(reinterpret_cast<const unsigned long long *>(l_table) + (tid - kLoadWarp0 * 32u));
+                    s_bias[tid - kLoadWarp0 * 32u] = l_bias ? __ldcg(l_bias + (tid - kLoadWarp0 * 32u)) : 0.0f;
                 }
             }
             if (l == 0u) {
@@ -572,7 +587,16 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 }
             }
             if (l == 0u) {
-                if (has_x) {
+                if (has_x && x_bf16) {
+                    const uint2 b0 = __ldcg(reinterpret_cast<const uint2 *>(x_bf16) + 2u * tid);
+                    const uint2 b1 = __ldcg(reinterpret_cast<const uint2 *>(x_bf16) + 2u * tid + 1u);
+                    const uint32_t b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        xs[2 * i] = __uint_as_float(b[i] << 16);
+                        xs[2 * i + 1] = __uint_as_float(b[i] & 0xffff0000u);
+                    }
+                } else if (has_x) {
                     const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x) + 2u * tid);
                     const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x) + 2u * tid + 1u);
                     xs[0] = p0.x, xs[1] = p0.y, xs[2] = p0.z, xs[3] = p0.w;
@@ -1146,7 +1170,6 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                                     if (residual)
                                         x_in = l == 0u ? __ldcg(x + n)
                                                        : __uint_as_float((uint32_t)ld_relaxed_gpu(x_words + (size_t)par * kMaxHidden + n));
-                                    const float last = add_last ? __ldcg(add_last + n) : 0.0f;
                                     uint32_t vals[kJobsMax];
                                     uint32_t tries = 0;
                                     bool got = true;
@@ -1180,7 +1203,6 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                                                 acc = (s_mix_slot[par][jj] >> 31) ? __fadd_rn(acc, dv) : __fadd_rn(acc, __fmul_rn(s_mix_w[par][jj], dv));
                                             }
                                         }
-                                        if (add_last) acc = __fadd_rn(acc, last);
                                         const float out = residual ? __fadd_rn(x_in, acc) : acc;
                                         if (l + 1u == L) y[n] = out;
                                         else st_relaxed_gpu(x_words + (size_t)(par ^ 1u) * kMaxHidden + n, ((unsigned long long)(want + 1u) << 32) | __float_as_uint(out));
@@ -1275,7 +1297,14 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (n_early_jobs && l + 1u < L) prefetch_shared(s_layer[par ^ 1u].shared_page);
 #pragma unroll 1
                 for (uint32_t k = 0; k < 2u && l + k < L; ++k) produce(l + k, k != 0u);
-                if (l + 1u == L) mark(12);
+                if (l + 1u == L) {
+                    mark(12);
+                    // the kernel's own copies are under way and what is left is hand-offs: this CTA's share of what the launches
+                    // behind will read, into the L2
+#pragma unroll 1
+                    for (uint32_t u = cta * kAheadPiece; u < ahead_bytes; u += grid * kAheadPiece)
+                        l2_prefetch(ahead + u, min(kAheadPiece, ahead_bytes - u));
+                }
             }
             // the other lanes of its warp wait here (a warp barrier, no polling) until it has finished:
             // a lane that polls for the next layer's token would take the warp's issue slots from it
@@ -1505,7 +1534,8 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
                                   const float *x, float *d, float *y, uint8_t *tiles, unsigned int *counters,
                                   uint32_t *status, uint32_t hidden, uint32_t inter, const FusedRouter *router,
                                   const EpExchange *ep, unsigned long long *trace, const StackLayer *stack,
-                                  uint32_t n_layers, float *hbuf, bool residual, const float *add_last) {
+                                  uint32_t n_layers, float *hbuf, bool residual, const uint16_t *x_bf16, const uint8_t *ahead,
+                                  size_t ahead_bytes) {
     const uint32_t ring = ring_slots(hidden, inter, dynamic_limit());
     if (ring < 2u) return cudaErrorInvalidConfiguration;
     FusedRouter rt = {};
@@ -1514,7 +1544,6 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     EpExchange ex = {};
     if (ep) ex = *ep;
     if (ex.world > 1u && !router) return cudaErrorInvalidValue;  // the mix needs every route's weight
-    if (add_last && (stack || ex.world > 1u || !y)) return cudaErrorInvalidValue;
     if (stack && (!router || n_layers == 0u || n_layers > kMaxLayers || (n_layers > 1u && !hbuf) || ex.world > 1u || rt.ep_world > 1u))
         return cudaErrorInvalidValue;  // a stack routes its own layers on one GPU
     const size_t smem = (size_t)ring * kSlot + umma_fixed_smem(hidden, inter);
@@ -1526,10 +1555,10 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     if (trace)
         return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
                           counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                          residual ? 1u : 0u, add_last, paired ? 1u : 0u);
+                          residual ? 1u : 0u, x_bf16, ahead, (uint32_t)(ahead_bytes & ~(size_t)15u), paired ? 1u : 0u);
     return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
                       counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                      residual ? 1u : 0u, add_last, paired ? 1u : 0u);
+                      residual ? 1u : 0u, x_bf16, ahead, (uint32_t)(ahead_bytes & ~(size_t)15u), paired ? 1u : 0u);
 }
 
 }  // namespace s14

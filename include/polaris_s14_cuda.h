@@ -120,7 +120,7 @@ S14_API uint64_t s14_ctx_launch_count(const s14_ctx *ctx);
 #define S14_LAYER_PATH_REFERENCE 5u        /* reference-order kernels */
 #define S14_LAYER_PATH_TENSOR_BLOCK 6u     /* grouped tcgen05 kernels: every expert page streamed once per block */
 #define S14_LAYER_PATH_ROUTER_KERNEL 0x100u
-#define S14_LAYER_PATH_FP8_SHARED_KERNEL 0x200u /* with TENSOR: an FP8 shared expert by two launches in front of it */
+#define S14_LAYER_PATH_FP8_SHARED_KERNEL 0x200u /* with TENSOR: an FP8 shared expert by two launches behind it */
 S14_API uint32_t s14_ctx_last_layer_path(const s14_ctx *ctx);
 
 /* Per-kernel timing of s14_cmd_routed_moe_layer for profiling runs: while enabled,

@@ -163,3 +163,33 @@ def test_stack_with_fp8_shared_experts(ctx, oracle, residual):
         assert np.array_equal(h.cpu().numpy(), cur)
     finally:
         stack.close()
+
+
+@pytest.mark.parametrize("kind", [L.PAGE_FP8, L.PAGE_MXFP4])
+def test_calls_in_place_and_one_after_another(ctx, kind):
+    """The layer's y in place of x; the executor's state in place of the residual and its branch in place of the token; steps in a
+    row, each of which reads what the one before left."""
+    hidden, inter, routed = 2048, 2048, 3
+    g, pages, shared = make_layer(55, hidden, inter, routed, kind)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter, kind)
+    route = TokenRoute(list(range(routed)), np.asarray([0.3, 0.2, 0.1], np.float32), [p.data_ptr() for p in pages_dev])
+    x = dev(synth.activations(g, 1, hidden))
+    want, got = x.clone(), x.clone()
+    for _ in range(3):
+        y = torch.empty_like(want)
+        ctx.cmd_moe_layer(want * 0.01, y, [route], shared_dev.data_ptr(), kind, hidden, inter)
+        want = y
+        got *= 0.01
+        ctx.cmd_moe_layer(got, got, [route], shared_dev.data_ptr(), kind, hidden, inter)
+    assert torch.equal(got, want)
+    residual = dev(synth.hc_streams(g, 1, hidden)[0]).to(torch.bfloat16)
+    post, comb = dev(g.uniform(0.2, 1.8, 4).astype(np.float32)), dev(g.uniform(0.05, 0.6, (4, 4)).astype(np.float32))
+    t, s, t2, s2 = x[0].to(torch.bfloat16), residual, x[0].to(torch.bfloat16), residual.clone()
+    for _ in range(3):
+        branch, state = torch.empty_like(t), torch.empty_like(s)
+        ctx.exec_routed_and_shared_moe_then_hc_post(t, s, post, comb, route, shared_dev.data_ptr(), kind, inter, state, branch)
+        ctx.exec_routed_and_shared_moe_then_hc_post(t2, s2, post, comb, route, shared_dev.data_ptr(), kind, inter, s2, t2)
+        t, s = branch * 0.01, state
+        t2 *= 0.01
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0 and torch.equal(t, t2) and torch.equal(s, s2) and torch.isfinite(s.float()).all()

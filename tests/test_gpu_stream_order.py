@@ -90,6 +90,29 @@ def _layer(ctx):
     return pages_dev + [shared_dev], (lambda: ctx.cmd_moe_layer(x, y, [route], shared_dev.data_ptr(), L.PAGE_FP8, h, i)), y
 
 
+def _exec(ctx):
+    # (the shared expert's first launch reads the token and its page without a wait of its own)
+    h, i, routed = 1024, 2048, 2
+    g, pages, shared = make_layer(6, h, i, routed, L.PAGE_FP8)
+    pages_dev, shared_dev = [dev_page(p, h, i) for p in pages], dev_page(shared, h, i, L.PAGE_FP8)
+    route = TokenRoute(list(range(routed)), np.asarray([0.7, 0.4], np.float32), [p.data_ptr() for p in pages_dev])
+    x, residual = (dev(a).to(torch.bfloat16) for a in (synth.activations(g, 1, h)[0], synth.hc_streams(g, 1, h)[0]))
+    post, comb = torch.rand(4, device="cuda") + 0.2, torch.rand(4, 4, device="cuda")
+    state = torch.empty_like(residual)
+    return [x, residual, shared_dev, pages_dev[0], post, comb], (lambda keep=pages_dev: ctx.exec_routed_and_shared_moe_then_hc_post(
+        x, residual, post, comb, route, shared_dev.data_ptr(), L.PAGE_FP8, i, state, None)), state
+
+
+def _routed_layer(ctx):
+    h, i, experts = 1024, 1024, 9
+    g, pages, shared = make_layer(8, h, i, experts, L.PAGE_FP8)
+    pages_dev, shared_dev = [dev_page(p, h, i) for p in pages], dev_page(shared, h, i, L.PAGE_FP8)
+    table = torch.tensor([p.data_ptr() for p in pages_dev], dtype=torch.int64, device="cuda")
+    wr, bias = dev(synth.router_weight_bf16(g, experts, h).view(np.int16)), dev(synth.router_bias(g, experts))
+    x, y = dev(synth.activations(g, 1, h))[0], torch.empty(1, h, device="cuda")
+    return [x, wr, bias, shared_dev] + pages_dev, (lambda: ctx.cmd_routed_moe_layer(x, wr, bias, table, shared_dev.data_ptr(), L.PAGE_FP8, i, y)), y
+
+
 def _block(tokens, official, routed):
     """The block calls: their first digits launch reads x in front of its wait, behind the router's launches (or the copies of
     the host's routes), which have waited."""
@@ -111,9 +134,9 @@ def _block(tokens, official, routed):
     return make
 
 
-@pytest.mark.parametrize("make", [_mxfp4, _fp8, _head, _site(1), _site(20), _layer, _block(3, False, True), _block(20, False, True),
+@pytest.mark.parametrize("make", [_mxfp4, _fp8, _head, _site(1), _site(20), _layer, _exec, _routed_layer, _block(3, False, True), _block(20, False, True),
                                   _block(3, True, True), _block(70, True, True), _block(5, False, False)],
-                         ids=["mxfp4", "fp8", "head", "site", "site20", "fp8_shared_layer", "block", "block20", "block_official",
+                         ids=["mxfp4", "fp8", "head", "site", "site20", "fp8_shared_layer", "executor_step", "fp8_shared_routed_layer", "block", "block20", "block_official",
                               "block70_official", "block_host_routes"])
 def test_operands_written_late_by_a_kernel_that_lets_dependents_start(ctx, write_late, make):
     torch.manual_seed(1)
