@@ -188,3 +188,37 @@ def test_full_logits_equal_their_operators(ctx, hidden):
     # reduced vector by at most one BF16 unit (2^-8 relative) and so a logit by 2^-8 |x| |w|
     mag = normed.float().abs()[0] @ w.view(torch.bfloat16).float().abs().T
     assert bool(((out - want).abs() <= 2.0 ** -8 * mag).all())
+
+
+# one value; fewer than a warp's; a thread's loads of a round and one more; a whole round of the cluster and its neighbours
+@pytest.mark.parametrize("vocab", [1, 5, 2047, 2049, 32767, 131072, 131077])
+@pytest.mark.parametrize("offset", [0, 1])   # 16-byte loads, and not
+def test_greedy_token_at_the_edges_of_a_round(ctx, vocab, offset):
+    torch.manual_seed(vocab)
+    base = torch.randn(vocab + offset, device="cuda")
+    res = torch.empty(1, dtype=torch.int64, device="cuda")
+
+    def token(v):
+        full = base.clone()
+        full[offset:] = v
+        ctx.cmd_greedy_argmax(full[offset:], res)
+        return int(res.item())
+
+    v = base[offset:]
+    assert token(v) == int(v.cpu().argmax())
+    places = sorted({0, vocab // 3, vocab // 2, vocab - 1})
+    for p in places:
+        w = v.clone()
+        w[p] = 50.0
+        assert token(w) == p
+        w[places[-1]] = 50.0                      # the lowest of equal ones
+        assert token(w) == p
+        w[p] = float("inf")
+        assert token(w) == p
+        w[places[0]] = float("nan")
+        assert token(w) == -1
+    assert token(torch.full_like(v, -float("inf"))) == 0
+    w = torch.full_like(v, -1.0)
+    w[places[-1]] = 0.0
+    w[places[len(places) // 2]] = -0.0            # equal to +0
+    assert token(w) == places[len(places) // 2]
