@@ -42,8 +42,8 @@ __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
 
 // N consecutive stream values, back and forth: eight BF16 or four F32 values are one 16-byte access, four BF16 values one of 8
 // bytes, eight F32 values two of 16 (which a warp's lanes make 32 bytes apart); one by one where a caller's buffer is
-// not aligned to 16 bytes (`vec`, the same for all threads of a launch): all of hc_post and rms_norm, and hc_pre's
-// reduced vector.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the
+// not aligned to 16 bytes (`vec`): all of hc_post and rms_norm, and hc_pre's reduced vector.  Those kernels are compiled once for
+// each: with both forms in one kernel 370 tokens of 4096 took hc_post 7.6 us, now 6.2, and F32 norms 3.7, now 3.0.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the
 // calls refuse what is not aligned for that.
 template <bool kBf16, int N>
 __device__ __forceinline__ void stream_ldn(const void *p, size_t i, float (&v)[N], bool vec) {
@@ -140,6 +140,16 @@ __device__ __forceinline__ void split_sinkhorn_warp(const float *mixes, const fl
     comb = c;
 }
 
+// sum_h pre[h] v[h] in stream order
+template <int N>
+__device__ __forceinline__ void sum_streams(const float (&v)[kHc][N], const float (&pre)[kHc], float (&acc)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        acc[k] = __fmul_rn(pre[0], v[0][k]);
+#pragma unroll
+        for (uint32_t h = 1; h < kHc; ++h) acc[k] = __fadd_rn(acc[k], __fmul_rn(pre[h], v[h][k]));
+    }
+}
 // reduced[d] = sum_h pre[h] x[h][d] for N consecutive d.
 template <bool kBf16, int N>
 __device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_t hidden, uint32_t d, const float (&pre)[kHc],
@@ -147,12 +157,7 @@ __device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_
     float v[kHc][N];
 #pragma unroll
     for (uint32_t h = 0; h < kHc; ++h) stream_ldn<kBf16, N>(x, x0 + (size_t)h * hidden + d, v[h], vec);
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        acc[k] = __fmul_rn(pre[0], v[0][k]);
-#pragma unroll
-        for (uint32_t h = 1; h < kHc; ++h) acc[k] = __fadd_rn(acc[k], __fmul_rn(pre[h], v[h][k]));
-    }
+    sum_streams<N>(v, pre, acc);
 }
 
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
@@ -258,7 +263,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
 // time (70 us for 370 tokens of 4096); here a row's element serves sixteen tokens and a token's 24 rows (12 us:
 // the FP64 pipe's 64 products per clock and SM bound it at 8).  K is permuted inside steps of sixteen: lane q of
 // a quad takes four consecutive elements as its slots of four MMAs.  Writes partial sums [slice][token][25] in double.
-constexpr uint32_t kDotTokens = 16;
+constexpr uint32_t kDotTokens = 16, kHcSlices = 64;
 template <bool kBf16, bool kHead>
 __global__ void __launch_bounds__(256)
 k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, uint32_t n_tokens, double *__restrict__ partial) {
@@ -266,8 +271,9 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
     __shared__ double s_acc[8][kDotTokens][kMix + 1];
     dependency_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, q = lane & 3u;
-    const uint32_t t0 = blockIdx.x * kDotTokens, len = n / (gridDim.y * 8u);   // a multiple of 16
-    const uint32_t k0 = (blockIdx.y * 8u + warp) * len + q * 4u;
+    // steps of sixteen k, dealt to the warps of all slices as evenly as whole steps go
+    const uint32_t steps = n >> 4, parts = gridDim.y * 8u, me = blockIdx.y * 8u + warp;
+    const uint32_t t0 = blockIdx.x * kDotTokens, k0 = steps * me / parts * 16u + q * 4u, k1 = steps * (me + 1u) / parts * 16u + q * 4u;
     const uint32_t ta = min(t0 + g, n_tokens - 1u), tb = min(t0 + g + 8u, n_tokens - 1u);
     double c[2][kTiles][2] = {}, ss[2] = {0.0, 0.0};
     auto load4 = [&](uint32_t t, uint32_t k, float (&v)[4]) {
@@ -281,7 +287,7 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
         }
     };
 #pragma unroll 2
-    for (uint32_t k = k0; k < k0 + len; k += 16u) {
+    for (uint32_t k = k0; k < k1; k += 16u) {
         float va[4], vb[4];
         load4(ta, k, va);
         load4(tb, k, vb);
@@ -326,23 +332,50 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
     }
 }
 
-// One CTA per token: the coefficients from the partial sums (one warp), then the reduced vector.
-template <bool kBf16, bool kHead, int N>
+// One CTA per token: the coefficients from the partial sums (one warp), then the reduced vector.  All latency: the slices' sums
+// (added one after the other by one warp, four loads in flight, they were half of a call of 20 tokens: 10.5 us, now 8.1), the
+// coefficients, the streams.  kAhead: a thread reads its first N values of every stream in front of the wait for the sums (the rule
+// is the launch's).
+template <bool kBf16, bool kHead, int N, bool vec, bool kAhead>
 __global__ void __launch_bounds__(256)
 k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint32_t slices, const float *__restrict__ scale,
             const float *__restrict__ base, uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced,
-            float *__restrict__ post_out, float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec) {
+            float *__restrict__ post_out, float *__restrict__ comb_out, float *__restrict__ pre_out) {
     constexpr uint32_t kMix = kHead ? kHc : kMixMax;
+    __shared__ double s_sum[8][kMix + 1];
     __shared__ float s_pre[kHc], s_mix[kMix], s_coef[3 + kMix];
-    // (k_hc_dots in front of this launch has waited: the launch behind may be set up at once)
+    // k_hc_dots in front of this launch has waited, so everything in front of that kernel is complete: the launch behind may be
+    // set up at once, and the streams may be read in front of the wait for the sums.
     cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
     const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    constexpr uint32_t kFirst = kHead ? 0u : 32u;   // (the coefficients' warp has no part of the streams)
+    uint32_t d = (threadIdx.x - kFirst) * N;        // (that warp's is beyond them)
+    float v[kHc][N];
+    if (kAhead && d < hidden) {
+#pragma unroll
+        for (uint32_t h = 0; h < kHc; ++h) stream_ldn<kBf16, N>(x, ((size_t)t * kHc + h) * hidden + d, v[h], vec);
+    }
+    cudaGridDependencySynchronize();
+    // the slices' sums: a warp takes every eighth, at most eight of them, all loads in flight together
+    if (lane <= kMix) {
+        double u[8], s = 0.0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; ++k) {
+            const uint32_t p = warp + 8u * k;
+            u[k] = p < slices ? __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMix + 1u) + lane) : 0.0;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; ++k) s += u[k];
+        s_sum[warp][lane] = s;
+    }
+    if (warp == 0u) load_coefficients<kHead>(s_coef, scale, base, lane);
+    __syncthreads();
     if (warp == 0u) {
-        load_coefficients<kHead>(s_coef, scale, base, lane);
         double s = 0.0;
-        if (lane <= kMix)
-            for (uint32_t p = 0; p < slices; ++p) s += __ldcg(partial + ((size_t)p * gridDim.x + t) * (kMix + 1u) + lane);
+        if (lane <= kMix) {
+#pragma unroll
+            for (uint32_t w = 0; w < 8u; ++w) s += s_sum[w][lane];
+        }
         const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMix) / (double)(kHc * hidden)), norm_eps);
         if (lane < kMix) s_mix[lane] = __fmul_rn((float)s, rs);
         __syncwarp();
@@ -361,11 +394,18 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
         return;
     }
     const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
-    constexpr uint32_t kFirst = kHead ? 0u : 32u;
-    for (uint32_t d = (threadIdx.x - kFirst) * N; d < hidden; d += (256u - kFirst) * N) {
-        float v[N];
-        reduce_streams<kBf16, N>(x, (size_t)t * kHc * hidden, hidden, d, pre, v, vec != 0u);
-        stream_stn<kBf16, N>(reduced, (size_t)t * hidden + d, v, vec != 0u);
+    if constexpr (kAhead) {
+        if (d < hidden) {
+            float o[N];
+            sum_streams<N>(v, pre, o);
+            stream_stn<kBf16, N>(reduced, (size_t)t * hidden + d, o, vec);
+        }
+        d += (256u - kFirst) * N;
+    }
+    for (; d < hidden; d += (256u - kFirst) * N) {
+        float o[N];
+        reduce_streams<kBf16, N>(x, (size_t)t * kHc * hidden, hidden, d, pre, o, vec);
+        stream_stn<kBf16, N>(reduced, (size_t)t * hidden + d, o, vec);
     }
 }
 
@@ -373,20 +413,20 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
 // token's twenty coefficients are the same for all its threads, so they are read through the L1; F32 values go four to a
 // thread, because the lanes' 16-byte accesses then meet in whole lines (4096, us, before these two and now: 150 tokens
 // F32 7.1 -> 3.3, 1024 28.2 -> 24.5; BF16 16 tokens 2.1 -> 1.7, 1024 10.6 -> 10.2).
-template <bool kBf16, int N>
+template <bool kBf16, int N, bool vec>
 __global__ void __launch_bounds__(128)
 k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, const float *__restrict__ post,
-          const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged, uint32_t vec) {
+          const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
     const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * N, t = blockIdx.y;
     dependency_wait();
     if (d >= hidden) return;
     float r[kHc][N], b[N], c[kHc * kHc], p[kHc];
 #pragma unroll
     for (uint32_t h = 0; h < kHc; ++h) {
-        stream_ldn<kBf16, N>(residual, ((size_t)t * kHc + h) * hidden + d, r[h], vec != 0u);
+        stream_ldn<kBf16, N>(residual, ((size_t)t * kHc + h) * hidden + d, r[h], vec);
         p[h] = ld_f32(post + (size_t)t * kHc + h);
     }
-    stream_ldn<kBf16, N>(branch, (size_t)t * hidden + d, b, vec != 0u);
+    stream_ldn<kBf16, N>(branch, (size_t)t * hidden + d, b, vec);
 #pragma unroll
     for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = ld_f32(comb + (size_t)t * kHc * kHc + i);
 #pragma unroll
@@ -399,7 +439,7 @@ k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, co
             for (uint32_t h = 1; h < kHc; ++h) s = __fadd_rn(s, __fmul_rn(c[h * kHc + o], r[h][k]));
             v[k] = __fadd_rn(__fmul_rn(p[o], b[k]), s);
         }
-        stream_stn<kBf16, N>(merged, ((size_t)t * kHc + o) * hidden + d, v, vec != 0u);
+        stream_stn<kBf16, N>(merged, ((size_t)t * kHc + o) * hidden + d, v, vec);
     }
 }
 
@@ -407,10 +447,9 @@ k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, co
 // steps.  kHeld: the token stays in registers and is read once.  The weight is the same for all tokens and comes
 // through the L1.  All tokens read and written at once bound it, so the registers have to leave room for them: kBlocks
 // CTAs per SM (the launch's rule).
-template <bool kBf16, int N, int kSteps, int kBlocks, bool kHeld>
+template <bool kBf16, int N, int kSteps, int kBlocks, bool kHeld, bool vec>
 __global__ void __launch_bounds__(256, kBlocks)
-k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out,
-           uint32_t vec) {
+k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out) {
     __shared__ double red[8];
     const uint32_t t = blockIdx.x;
     dependency_wait();
@@ -421,7 +460,7 @@ k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hid
         const uint32_t d = (i * 256u + threadIdx.x) * N;
         float(&vi)[N] = v[kHeld ? i : 0];
         if (d < hidden) {
-            stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec != 0u);
+            stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec);
 #pragma unroll
             for (int k = 0; k < N; ++k) ss += (double)vi[k] * (double)vi[k];
         }
@@ -438,7 +477,7 @@ k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hid
         const uint32_t d = (i * 256u + threadIdx.x) * N;
         float(&vi)[N] = v[kHeld ? i : 0];
         if (d < hidden) {
-            if (!kHeld) stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec != 0u);
+            if (!kHeld) stream_ldn<kBf16, N>(x, (size_t)t * hidden + d, vi, vec);
             float wv[N];
 #pragma unroll
             for (int k = 0; k < N; k += 4) {
@@ -451,7 +490,7 @@ k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hid
             }
 #pragma unroll
             for (int k = 0; k < N; ++k) wv[k] = __fmul_rn(wv[k], __fmul_rn(vi[k], rs));
-            stream_stn<kBf16, N>(out, (size_t)t * hidden + d, wv, vec != 0u);
+            stream_stn<kBf16, N>(out, (size_t)t * hidden + d, wv, vec);
         }
     }
 }
@@ -532,8 +571,8 @@ cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y,
 
 // The partial sums of launch_hc_pre_many.
 size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count) {
-    // a row per slice and token: up to sixteen slices, or fewer than two CTAs of sixteen tokens per SM (launch_hc_pre_many)
-    return (size_t)std::max(16u * max_tokens, 32u * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
+    // a row per slice and token: slices times groups of sixteen tokens come to six CTAs per SM at most (launch_hc_pre_many)
+    return (size_t)std::max(std::max(max_tokens, kHcSlices * kDotTokens), 6u * kDotTokens * (uint32_t)sm_count) * (kMixMax + 1u) * sizeof(double);
 }
 
 // Whether all the addresses are multiples of 16 (rows of 256 and more elements keep that).
@@ -570,25 +609,26 @@ template <bool kBf16, bool kHead>
 static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                       const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
                                       double *partial, void *reduced, float *post, float *comb, float *pre) {
-    // slices of K: enough CTAs for the SMs, each warp's part whole steps of sixteen (n / 1024 is a whole number)
-    const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden;
-    uint32_t slices = 8u;
-    auto twice = [&]() { return (n / (slices * 2u * 8u)) % 16u == 0u; };
-    while (slices < 64u && groups * slices < (uint32_t)sm_count && twice()) slices *= 2u;
-    // ... sixteen instead of eight where the last round of CTAs would leave a fifth of the SMs idle and the rows are long enough:
-    // the second kernel adds up twice the slices, and with fewer rounds there is less to fill up.  us of both launches, eight
-    // and sixteen slices: 370 tokens of 4096 24.6 and 22.3 (with the norm and the expand behind them 36.0 and 31.5), 700 33.4
-    // and 30.1, F32 36.4 and 33.0; 420 of 1024 14.5 and 11.9; but 940 of 1024 21.2 and 22.3, 704 of 512 11.3 and 12.7.
-    // The head's four rows cost the first kernel little, so there the bound lies higher where two rounds become
-    // three (460 of 2048 9.7 and 12.1, of 4096 14.6 and 18.7, but with the norm behind it 30.7 and 22.8) and lower where three
-    // become five (704 of 1024 10.8 and 8.9, of 4096 27.7 and 19.0).  (150 tokens at 32 slices: 17.3 and 23.1, 15.3 and 23.6.)
-    const uint32_t sms = (uint32_t)sm_count, ctas = groups * slices, rounds = (ctas + sms - 1u) / sms;
-    const uint32_t least = !kHead ? (rounds <= 2u ? 1024u : 2048u) : (rounds <= 2u ? (kBf16 ? 4096u : 5120u) : (rounds == 3u ? 1024u : 2048u));
-    if (slices == 8u && hidden >= least && ctas * 5u < rounds * sms * 4u && twice()) slices *= 2u;
+    // Slices of K: as many as make the CTAs fit the SMs side by side, three to an SM by their registers (the head's, with four
+    // rows in place of 24, five, and a sixth that follows soon): one round, no tail.  At most 64, which the second kernel adds up,
+    // and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
+    // in one warp, and now: 20 tokens of 4096 10.5 and 8.1, 370 23.3 and 20.9, 700 34.1 and 30.9, 1000 45.8 and 40.3; 900 of
+    // 1024 20.6 and 16.0.  The head: 460 of 4096 18.7 and 11.5, 1000 30.1 and 23.3, 704 of 512 7.5 and 6.3.
+    const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden, sms = (uint32_t)sm_count;
+    const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, (kHead ? 6u : 3u) * sms / groups}));
     const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
-    return launch_pdl(k_hc_reduce<kBf16, kHead, kBf16 ? 8 : 4>, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden,
-                      norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced));
+    auto reduce = [&](auto kernel) {
+        return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, (const double *)partial, slices, scale, base, hidden, norm_eps, iters,
+                          hc_eps, reduced, post, comb, pre);
+    };
+    constexpr int kN = kBf16 ? 8 : 4;
+    if (!aligned16(x, reduced)) return reduce(k_hc_reduce<kBf16, kHead, kN, false, false>);
+    // The streams in front of the wait while all CTAs are resident with the registers that takes (64, F32 48: four and five to an
+    // SM).  us of the site, with and without: 370 tokens of 4096 30.6 and 32.3, 550 44.4 and 46.0, 650 46.7 and 43.3; F32 600 46.0 and 47.9,
+    // 1000 80.0 and 76.2.  (Twice the values: two CTAs to an SM, 370 tokens 34.5.)
+    const bool ahead = n_tokens <= (kBf16 ? 4u : 5u) * sms;
+    return ahead ? reduce(k_hc_reduce<kBf16, kHead, kN, true, true>) : reduce(k_hc_reduce<kBf16, kHead, kN, true, false>);
 }
 
 // scratch: hc_scratch_bytes of the most tokens.  Returns the number of kernels launched.
@@ -637,10 +677,11 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
     const bool few = (uint64_t)n_tokens * hidden <= (uint64_t)sm_count * 5u * 512u;
     auto run = [&](auto kernel, uint32_t per_thread) {
         return launch_pdl(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, branch,
-                          residual, post, comb, hidden, merged, vec);
+                          residual, post, comb, hidden, merged);
     };
-    if (!bf16) return run(k_hc_post<false, 4>, 4);
-    return few ? run(k_hc_post<true, 4>, 4) : run(k_hc_post<true, 8>, 8);
+    if (!bf16) return vec ? run(k_hc_post<false, 4, true>, 4) : run(k_hc_post<false, 4, false>, 4);
+    if (!vec) return few ? run(k_hc_post<true, 4, false>, 4) : run(k_hc_post<true, 8, false>, 8);
+    return few ? run(k_hc_post<true, 4, true>, 4) : run(k_hc_post<true, 8, true>, 8);
 }
 
 // F32 tokens: eight values per thread while a token has an SM to itself (the fewest steps in series), else four, whose
@@ -648,28 +689,31 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
 // largest batches would spill and read the token twice.  us of 4096, one form for all / now: 16 tokens 2.7 / 2.6,
 // 300 5.2 / 3.6, 700 7.8 / 4.9, 1024 9.5 / 6.7; 8192 and 1024 tokens 16.4 / 12.0.  BF16 tokens are half the bytes, eight
 // values to a thread always: 4096 and 700 tokens 5.8 / 3.7.
-template <bool kBf16, int kSteps>
+template <bool kBf16, int kSteps, bool kVec>
 static cudaError_t launch_rms_steps(cudaStream_t st, uint32_t sms, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
-                                    void *out, uint32_t vec) {
-    auto run = [&](auto kernel) { return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, vec); };
-    if (kBf16 || n_tokens <= sms) return run(k_rms_norm<kBf16, 8, kSteps, 1, true>);
+                                    void *out) {
+    auto run = [&](auto kernel) { return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out); };
+    if (kBf16 || n_tokens <= sms) return run(k_rms_norm<kBf16, 8, kSteps, 1, true, kVec>);
     if constexpr (!kBf16) {
         constexpr int kFour = 2 * kSteps;   // steps of four values
-        if (kSteps == 1 && hidden <= 1024u) return run(k_rms_norm<false, 4, 1, 8, true>);
-        if (n_tokens <= 4u * sms) return run(k_rms_norm<false, 4, kFour, 1, true>);
-        if (n_tokens <= 6u * sms) return run(k_rms_norm<false, 4, kFour, 6, true>);
-        return run(k_rms_norm<false, 4, kFour, 8, (kFour < 8)>);
+        if (kSteps == 1 && hidden <= 1024u) return run(k_rms_norm<false, 4, 1, 8, true, kVec>);
+        if (n_tokens <= 4u * sms) return run(k_rms_norm<false, 4, kFour, 1, true, kVec>);
+        if (n_tokens <= 6u * sms) return run(k_rms_norm<false, 4, kFour, 6, true, kVec>);
+        return run(k_rms_norm<false, 4, kFour, 8, (kFour < 8), kVec>);
     }
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w,
                             float eps, void *out) {
-    const uint32_t vec = aligned16(x, w, out), sms = (uint32_t)sm_count;
+    const uint32_t sms = (uint32_t)sm_count;
     auto run = [&](auto steps) {
         constexpr int kS = decltype(steps)::value;
-        return bf16 ? launch_rms_steps<true, kS>(st, sms, n_tokens, hidden, x, w, eps, out, vec)
-                    : launch_rms_steps<false, kS>(st, sms, n_tokens, hidden, x, w, eps, out, vec);
+        if (!aligned16(x, w, out))
+            return bf16 ? launch_rms_steps<true, kS, false>(st, sms, n_tokens, hidden, x, w, eps, out)
+                        : launch_rms_steps<false, kS, false>(st, sms, n_tokens, hidden, x, w, eps, out);
+        return bf16 ? launch_rms_steps<true, kS, true>(st, sms, n_tokens, hidden, x, w, eps, out)
+                    : launch_rms_steps<false, kS, true>(st, sms, n_tokens, hidden, x, w, eps, out);
     };
     if (hidden <= 2048u) return run(std::integral_constant<int, 1>{});
     if (hidden <= 4096u) return run(std::integral_constant<int, 2>{});

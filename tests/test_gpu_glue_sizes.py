@@ -121,3 +121,27 @@ def test_reduce_of_streams_on_the_boundaries_it_takes(ctx, tokens):
             ctx.exec_hc_head_norm_full_logits(state, matrix, scale, base, norm, head, logits)
     assert ctx.launch_count == launched
     torch.cuda.synchronize()
+
+
+# slices of K that are no whole number of steps each (37 of 128 steps at 190 x 512, 24 of 192 at 60 x 768), a step per warp (64 x 256),
+# one group of tokens and 64 slices (16 x 2048), one more token; the last token count whose streams are read in front of the wait on
+# 148 SMs and the one behind it (BF16 592, F32 740)
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("n_tokens,hidden", [(190, 512), (60, 768), (64, 256), (16, 2048), (17, 2304), (592, 512), (594, 512), (740, 512), (741, 256)])
+def test_sites_at_the_edges_of_slices(ctx, oracle, bf16, n_tokens, hidden):
+    test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden)
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_reduce_of_many_tokens_into_an_unaligned_result(ctx, bf16):
+    g = torch.Generator(device="cuda").manual_seed(9)
+    t, h, dt = 40, 768, torch.bfloat16 if bf16 else torch.float32
+    x = torch.randn(t, 4, h, device="cuda", generator=g).to(dt)
+    fn = torch.randn(24, 4 * h, device="cuda", generator=g) * 0.02
+    scale, base = torch.rand(3, device="cuda", generator=g), torch.rand(24, device="cuda", generator=g)
+    post, comb = torch.empty(t, 4, device="cuda"), torch.empty(t, 4, 4, device="cuda")
+    red, moved = torch.empty(t, h, dtype=dt, device="cuda"), _offset(torch.zeros(t, h, dtype=dt, device="cuda"), 1)
+    ctx.cmd_hc_pre(x, fn, scale, base, red, post, comb)
+    ctx.cmd_hc_pre(_offset(x, 4), fn, scale, base, moved, post, comb)
+    torch.cuda.synchronize()
+    assert torch.equal(red, moved)
