@@ -223,12 +223,14 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 // over the routes in order; acc += d of the shared expert.  With `residual` the layer's input is added
 // (y = x + acc, what a layer of a stack hands to the next); y may be x.  Four outputs
 // per thread, the seven rows' loads in flight together (one value per thread,
-// row after row: 64 us for 1000 tokens of 4096, now 28).
+// row after row: 64 us for 1000 tokens of 4096, now 28).  Compiled for aligned buffers and for others: with both forms in one
+// kernel the code that every warp fetches once was longer (a block of 45 tokens 148.1 us, so 147.6).
+template <bool vec>
 __global__ void __launch_bounds__(256)
 k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const float *__restrict__ weights,
             uint32_t top_k, int has_shared, float *y, uint32_t hidden, const uint32_t *__restrict__ counts,
             const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_rank, uint32_t ep_world, uint32_t ep_call,
-            uint32_t wait_limit, uint32_t *status, uint32_t official, uint32_t vec) {
+            uint32_t wait_limit, uint32_t *status, uint32_t official) {
     const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * 4u, t = blockIdx.y;   // hidden is a multiple of four
     dependency_wait();
     const uint32_t why = __ldcg(counts + 3);
@@ -301,10 +303,10 @@ cudaError_t launch_mix(cudaStream_t st, const float *pairs, const int32_t *ids, 
                        bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts, bool residual,
                        const BlockEp *ep, uint32_t *status, bool official) {
     const uintptr_t where = (uintptr_t)pairs | (uintptr_t)y | (residual ? (uintptr_t)x : 0u);
-    return launch_pdl(k_block_mix, dim3((hidden + 1023u) / 1024u, n_tokens), dim3(256), 0, st, 0u, pairs, ids, weights, top_k,
+    return launch_pdl((where & 15u) ? k_block_mix<false> : k_block_mix<true>, dim3((hidden + 1023u) / 1024u, n_tokens), dim3(256), 0, st, 0u, pairs, ids, weights, top_k,
                       has_shared ? 1 : 0, y, hidden, counts, x, residual ? 1u : 0u,
                       (const unsigned long long *)(ep ? ep->flags : nullptr), ep ? ep->rank : 0u, ep ? ep->world : 1u, ep ? ep->call : 0u,
-                      ep ? ep->wait_limit : 0u, status, official ? 1u : 0u, (where & 15u) ? 0u : 1u);
+                      ep ? ep->wait_limit : 0u, status, official ? 1u : 0u);
 }
 
 }  // namespace
