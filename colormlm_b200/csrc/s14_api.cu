@@ -646,8 +646,10 @@ extern "C" int32_t s14_layer_pair_list(uint32_t block, uint32_t n_ctas, uint32_t
     if (n_ctas == 0 || block >= n_ctas || (n_ctas & 1u) || (hidden & 511u) || (inter & 511u) || hidden == 0 || inter == 0)
         return fail(S14_ERR_CONTRACT, "s14_layer_pair_list: block outside the grid, a grid without pairs, or sizes that are not multiples of 512");
     const uint32_t early_items = std::min(n_early_jobs, n_jobs) * (inter >> 6);
-    *count = layer_pair_list(pair_cta(block, n_ctas, early_items), n_ctas, n_jobs, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8,
-                             items_out, cap, n_early_jobs);
+    const uint32_t cta = pair_cta(block, n_ctas, early_items), S = inter >> 6, RT = hidden >> 7, KU = hidden >> 8, KD = inter >> 8;
+    *count = layer_pairs_share(n_ctas, n_jobs, S, KU, n_early_jobs)
+                 ? layer_pair_list(cta, n_ctas, n_jobs, S, RT, KU, KD, items_out, cap, n_early_jobs)
+                 : layer_work_list(cta, n_ctas, n_jobs, S, RT, KU, KD, items_out, cap, n_early_jobs);
     return S14_OK;
 }
 

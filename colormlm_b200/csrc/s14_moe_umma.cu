@@ -167,7 +167,7 @@ __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_
 // no gain); so there may be at most as many shared items as such pairs, and half an item has to have an even number of units.
 // Otherwise the lists are those above.  The down items: the CTAs without a half first take what levels the units (of the jobs
 // that are finished first), the rest goes round all CTAs, those first (those last: 342 us).  14 layers of 4096 x 2048 in one
-// launch: 348.3 us, with shared items 338.5.
+// launch: 343.5 us, with shared items 331.5.
 //
 // CTA `b` of the grid as the deal numbers it: the first F / 2 pairs hold the F early items, two neighbouring numbers each; the
 // numbers of the other pairs lie half of those CTAs apart.
@@ -175,20 +175,24 @@ __host__ __device__ uint32_t pair_cta(uint32_t b, uint32_t G, uint32_t F) {
     if (F > G) F = 0u;   // (every CTA holds early items)
     return b < F ? b : F + ((b - F) >> 1) + (b & 1u) * ((G - F) >> 1);
 }
-// CTA c's items as above, bit 30 set for a shared up item, bit 29 too for its second half.
+__host__ __device__ bool layer_pairs_share(uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t KU, uint32_t n_early) {
+    if (n_early > n_jobs) n_early = n_jobs;
+    const uint32_t U = n_jobs * S, F = n_early * S, r = G ? (U - F) % G : 0u;
+    return !(G & 1u) && !(F & 1u) && !(KU & 3u) && r && F <= G && r <= (G - F) / 2u;
+}
+// CTA c's items as above, bit 30 set for a shared up item, bit 29 too for its second half (layer_pairs_share holds).
 __host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU,
                                              uint32_t KD, uint32_t *items, uint32_t cap, uint32_t n_early) {
     if (n_early > n_jobs) n_early = n_jobs;
     const uint32_t U = n_jobs * S, D = n_jobs * RT, F = n_early * S;
-    const uint32_t a_full = G ? (U - F) / G : 0u, r = G ? (U - F) % G : 0u;
-    const uint32_t P = F > G ? 0u : (G - F) / 2u;   // pairs without early items
-    if ((G & 1u) || (F & 1u) || (KU & 3u) || r == 0u || r > P) return layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, cap, n_early);
+    const uint32_t a_full = (U - F) / G, r = (U - F) - a_full * G;
+    const uint32_t P = (G - F) / 2u;   // pairs without early items
     uint32_t n = 0;
     auto put = [&](uint32_t v) {
         if (n < cap) items[n] = v;
         ++n;
     };
-    const uint32_t c_rot = (c + G - F) % G;
+    const uint32_t c_rot = c >= F ? c - F : c + G - F;
     const bool first = c_rot < r, second = c_rot >= P && c_rot - P < r;
     for (uint32_t q = c; q < U; q += G) {
         const bool half = q >= F + a_full * G;   // of the last, incomplete round
@@ -216,9 +220,13 @@ namespace {
 
 // the one device copy of the deal (its divisions make it long; a CTA calls it once)
 __device__ __noinline__ uint32_t work_list_once(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU,
-                                                uint32_t KD, uint32_t *items, uint32_t n_early, uint32_t paired) {
-    const uint32_t n = paired ? layer_pair_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early)
-                              : layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
+                                                uint32_t KD, uint32_t *items, uint32_t n_early) {
+    const uint32_t n = layer_work_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
+    return n < kMaxItems ? n : kMaxItems;
+}
+__device__ __noinline__ uint32_t pair_list_once(uint32_t c, uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU,
+                                                uint32_t KD, uint32_t *items, uint32_t n_early) {
+    const uint32_t n = layer_pair_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
     return n < kMaxItems ? n : kMaxItems;
 }
 // Nothing on the kernel's paths may live in local memory: nearly all of the SM's L1 is carved out as
@@ -227,8 +235,7 @@ __device__ __noinline__ uint32_t work_list_once(uint32_t c, uint32_t G, uint32_t
 // inlined, arrays are indexed by unrolled loops, and only code that runs once per launch or layer
 // with little live state (the deal, the route records) is kept out of line.
 // And straight code that every warp meets once a layer is fetched again each time, about four cycles an instruction: the
-// counting loops of the selection and the copying thread's two steps are loops, not copies (14 layers 338 us, so 332.5).  That
-// is no rule for code whose operations overlap when it is unrolled (tensor-memory loads and their sums, the digits' halves, the
+// counting loops of the selection are loops (14 layers of 2048 x 2048 269.3 us unrolled, so 264.2).  That is no rule for code whose operations overlap when it is unrolled (tensor-memory loads and their sums, the digits' halves, the
 // router's two rows: 1-2 us more as loops), and a chain of F32 operations in place of the FP64 ones of the SwiGLU and of
 // the digit sums, which pays in the block kernels, is longer here (339 and 343 us).
 
@@ -416,7 +423,9 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             nj = rt.top_k + (rt.has_shared ? 1u : 0u);
             if (lane == 0) s_n_jobs = nj;
         }
-        if (early && lane == 1u) s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, n_early_jobs, paired);
+        if (early && lane == 1u)
+            s_n_items = paired ? pair_list_once(cta, grid, nj, S, RT, KU, KD, s_items, n_early_jobs)
+                               : work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, n_early_jobs);
     }
     __syncwarp();
     __syncthreads();
@@ -877,7 +886,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                         }
                         __syncwarp();
                         if (lane == 0 && !early)
-                            s_n_items = work_list_once(cta, grid, s_n_jobs, S, RT, KU, KD, s_items, 0u, paired);
+                            s_n_items = work_list_once(cta, grid, s_n_jobs, S, RT, KU, KD, s_items, 0u);
                         __syncwarp();
                     }
                 } else if (lt == 0) {
@@ -907,7 +916,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (lane == 0) {
                     s_n_jobs = nj;
                     s_n_mix = nm;
-                    s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, 0u, paired);
+                    s_n_items = work_list_once(cta, grid, nj, S, RT, KU, KD, s_items, 0u);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(kBarRoutes));
@@ -1295,8 +1304,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 // shared expert (its address is known) is asked into the L2, where that layer's copies find
                 // it a layer-time later instead of taking HBM time from the routed experts' stream.
                 if (n_early_jobs && l + 1u < L) prefetch_shared(s_layer[par ^ 1u].shared_page);
-#pragma unroll 1
-                for (uint32_t k = 0; k < 2u && l + k < L; ++k) produce(l + k, k != 0u);
+                produce(l, false);
+                if (l + 1u < L) produce(l + 1u, true);
                 if (l + 1u == L) {
                     mark(12);
                     // the kernel's own copies are under way and what is left is hand-offs: this CTA's share of what the launches
@@ -1387,7 +1396,6 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     }
     __syncwarp();
     __syncthreads();
-    if (paired) cluster_arrive();   // nothing of this CTA is on its way to its partner's shared memory
     // the last CTA to leave puts the counters back to zero for the next launch
     if (tid == 0) {
         if (abort_flag) atomicExch(status, s_abort_code);
@@ -1410,8 +1418,13 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (p != ep.rank) st_relaxed_sys(ep.slots[p] + credit + ep.rank, (unsigned long long)(s_ep_step + 1u));
         }
     }
-    __syncwarp();
-    if (paired) cluster_wait();   // a CTA stays until its partner writes nothing into it any more
+    // A CTA that is done has received what its partner sends it.  One that has given up stays until its partner has, too, or is
+    // gone (threads that have exited are not waited for).
+    if (paired && abort_flag) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
 }
 
 template <class Kernel, class... Args>
@@ -1519,8 +1532,9 @@ bool umma_layer_ok(int sm_count, uint32_t n_tokens, uint32_t n_jobs_max, uint32_
         for (uint32_t n_early = 0; n_early < 2u; ++n_early)
             if (layer_work_list(c, (uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8, items, 0,
                                 n_early) > kMaxItems ||
-                layer_pair_list(c, (uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8, items, 0,
-                                n_early) > kMaxItems)
+                (layer_pairs_share((uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 8, n_early) &&
+                 layer_pair_list(c, (uint32_t)sm_count, n_jobs_max, inter >> 6, hidden >> 7, hidden >> 8, inter >> 8, items, 0,
+                                 n_early) > kMaxItems))
                 return false;
     return ring_slots(hidden, inter, dynamic_limit()) >= 2u;
 }
@@ -1551,7 +1565,13 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     // paths (exchange inside the kernel, or expert outputs handed to a collective) are ordinary
     // launches; the kernel's own dependency calls are then no-ops.
     const bool pdl = ex.world <= 1u && y != nullptr;
-    const bool paired = pairs_resident(sm_count);
+    // In pairs where items are shared and the launch gains by it: a launch in clusters takes 1.5 us more, and half an item of 16
+    // units saves 0.9 us a layer, of eight next to nothing.  us in pairs and not: 4096 x 2048, six given jobs of the executor's step
+    // 33.3 and 34.1, one routed layer 25.0 and 24.6, two 48.3 and 49.2; 2048 x 2048, the step 26.9 and 25.6, 14 layers 264 both.
+    const bool given = !router && !dev;   // the jobs are in `param`
+    const uint32_t n_early = router && rt.has_shared ? 1u : 0u, n_jobs = given ? param.n_jobs : rt.top_k + n_early;
+    const bool paired = hidden >= 4096u && !dev && ex.world <= 1u && rt.ep_world <= 1u && (given || n_layers > 1u) &&
+                        layer_pairs_share((uint32_t)sm_count, n_jobs, inter >> 6, hidden >> 8, n_early) && pairs_resident(sm_count);
     if (trace)
         return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
                           counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,

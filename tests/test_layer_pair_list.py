@@ -73,10 +73,10 @@ def ctx():
     c.close()
 
 
-# (with 148 CTAs) every up item shared, two units to a half; four shared of 448; 44 of 192; no shared expert
+# (with 148 CTAs; a launch is in pairs where hidden is 4096) every up item shared; 4 of 448; 44 of 192, no shared expert; 12 of 160
 @pytest.mark.gpu
-@pytest.mark.parametrize("hidden,inter,routed,shared", [(1024, 1024, 1, False), (2048, 4096, 6, True), (4096, 2048, 6, False),
-                                                        (1024, 2048, 4, True)])
+@pytest.mark.parametrize("hidden,inter,routed,shared", [(4096, 1024, 2, True), (4096, 4096, 6, True), (4096, 2048, 6, False),
+                                                        (4096, 2048, 4, True)])
 def test_layer_with_shared_items(cuda_lib, ctx, oracle, hidden, inter, routed, shared):
     from .test_gpu_parity import assert_pairwise_close, dev_page, make_layer, run_layer
 
@@ -92,14 +92,14 @@ def test_layer_with_shared_items(cuda_lib, ctx, oracle, hidden, inter, routed, s
 
 @pytest.mark.gpu
 def test_stack_with_shared_items_and_early_ones(cuda_lib, ctx, oracle):
-    """Three chained layers of 1024 x 2048: the shared expert's items run early, 44 of the 192 routed ones are shared, in
+    """Three chained layers of 4096 x 2048: the shared expert's items run early, 44 of the 192 routed ones are shared, in
     every layer (the barriers' phases)."""
     torch = pytest.importorskip("torch")
     from colormlm_b200.s14 import DecodeStack
 
     from .test_gpu_parity import assert_chain_close, dev, dev_page, make_layer, oracle_stack
 
-    hidden, inter, n_experts = 1024, 2048, 10
+    hidden, inter, n_experts = 4096, 2048, 7
     host, layers, keep = [], [], []
     for l in range(3):
         g, pages, shared = make_layer(9300 + l, hidden, inter, n_experts, L.PAGE_MXFP4)
