@@ -161,7 +161,7 @@ __device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_
 }
 
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
-// only) of few tokens: one cluster of CTAs per token (sixteen, fewer for more tokens: launch_hc_pre).  The call is all
+// only) of few tokens: one cluster of sixteen CTAs per token (the head fewer for more tokens: launch_hc_pre).  The call is all
 // latency: 1.5 MB of fn per token, then a serial chain of 20 Sinkhorn rounds.  Every CTA takes its share of the
 // flattened streams against all rows of fn (98 KB, all loads in flight together), the partial sums cross in
 // shared memory, every CTA makes the coefficients itself and reduces its share of the hidden vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
@@ -652,20 +652,19 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
     using U = uint32_t;
     const uint32_t sms = (uint32_t)sm_count;
     if (!head) {
-        // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together, or fourteen of eight (4096, us:
-        // seven tokens 8.6, eight 9.6, fourteen 9.8; clusters of sixteen 14.4 and 14.8; the two launches 11.2, 10.7, 11.4).
+        // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together (4096, us: one token 8.2, seven 8.4, the
+        // two launches 8.2 and 8.3, on the host one launch more; 7168 9.1 and 9.4, 9.5 and 9.7).  Fourteen clusters of eight took
+        // 9.7 for fourteen tokens, the two launches 8.3 (7168 11.3 and 9.7).
         if (16u * n_tokens * 5u <= sms * 4u) return of_size(std::false_type{}, std::integral_constant<U, 16>{});
-        if (8u * n_tokens * 5u <= sms * 4u) return of_size(std::false_type{}, std::integral_constant<U, 8>{});
         return of_size(std::false_type{}, std::integral_constant<U, 0>{});
     }
     // The head's four rows leave room for two CTAs, and smaller clusters pack closer: the largest whose CTAs come to at most
-    // one and a half per SM (4096, us: 8 tokens 4.1, 16 4.4, 32 5.2, 64 6.8; one cluster of sixteen for any number 4.1, 8.0,
-    // 12.3, 20.7, the two launches 8.9, 9.5, 9.8, 10.8 and from about 70 tokens on the least: 300 12.9, 1024 26.5).
+    // one and a half per SM (4096, us: 8 tokens 4.0, 20 4.5, 55 5.5, the two launches 4.7, 5.0, 6.7).  Clusters of two for up to 111
+    // tokens: 80 tokens 8.2, the two launches 6.8 (2048 5.6 and 5.1, 7168 12.0 and 7.6, 256 3.6 and 3.7).
     const uint32_t room = sms + sms / 2u;
     if (16u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 16>{});
     if (8u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 8>{});
     if (4u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 4>{});
-    if (2u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 2>{});
     return of_size(std::true_type{}, std::integral_constant<U, 0>{});
 }
 
