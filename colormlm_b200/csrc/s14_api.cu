@@ -1835,6 +1835,7 @@ extern "C" int32_t s14_block_destroy(s14_block *blk) {
     cudaFree(blk->w.chunks);
     cudaFree(blk->w.counts);
     cudaFree(blk->w.xdig);
+    cudaFree(blk->w.slots);
     cudaFree(blk->w.xexp);
     cudaFree(blk->w.hdig);
     cudaFree(blk->w.hexp);
@@ -1872,7 +1873,8 @@ extern "C" int32_t s14_block_create(s14_ctx *ctx, uint32_t hidden, uint32_t inte
     const size_t R = S14_EXPERTS_PER_TOKEN;
     CUDA_OK(cudaMalloc((void **)&blk->w.chunks, C * sizeof(BlockChunk)));
     CUDA_OK(cudaMalloc((void **)&blk->w.counts, 64));
-    CUDA_OK(cudaMalloc((void **)&blk->w.xdig, T * (hidden >> 8) * 2048u));
+    CUDA_OK(cudaMalloc((void **)&blk->w.xdig, T * (hidden >> 8) * kXDigBytes));
+    CUDA_OK(cudaMalloc((void **)&blk->w.slots, P));
     CUDA_OK(cudaMalloc((void **)&blk->w.xexp, T * (hidden >> 5)));
     CUDA_OK(cudaMalloc((void **)&blk->w.hdig, P * (inter >> 8) * 2048u));
     CUDA_OK(cudaMalloc((void **)&blk->w.hexp, P * (inter >> 5)));

@@ -203,7 +203,7 @@ cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float
                              const float *norm_weight, uint32_t hidden, float norm_eps, float hc_eps, float *x_out);
 
 // ---- a block of tokens through one layer, grouped by expert (s14_moe_block.cu, s14_moe_pair.cu) ----
-constexpr uint32_t kBlockNt = 24;  // most tokens of one chunk (N = 192: eight digit rows per token at least)
+constexpr uint32_t kBlockNt = 32;  // most tokens of one chunk (N = 192: six digit rows per token at least)
 // Up to kBlockNt (token, route) pairs that share an expert page.  The chunks of one expert follow
 // one another: c0 is the first of them, nch their number.
 struct BlockChunk {
@@ -215,12 +215,15 @@ struct BlockChunk {
 };
 constexpr uint32_t kBlockBadId = 1;   // an expert id was out of range
 constexpr uint32_t kBlockGaveUp = 2;  // a wait inside a contraction kernel ran out
+// Bytes of a token's digit tiles per 256 elements: sixteen rows of 128, or four forms of six rows (s14_moe_block.cu).
+constexpr uint32_t kXDigBytes = 4u * 6u * 128u;
 // Device workspace of a block object, sized for max_tokens at creation.
 struct BlockWork {
     BlockChunk *chunks;
     uint32_t *counts;          // [0] chunks, [1], [2] chunks x slices, row tiles (above twelve tokens pairs of them), [3] why the call writes
                                // no result: kBlockBadId, kBlockGaveUp (set anew by every call's grouping)
     uint8_t *xdig, *xexp;      // the tokens' digit tiles and block exponents
+    uint8_t *slots;            // official arithmetic: which of the four forms of a digit tile each pair's place in its chunk takes
     uint8_t *hdig, *hexp;      // the pairs' hidden values likewise
     float *d;                  // the pairs' expert outputs [pair, hidden]
     float *hval;               // the pairs' hidden values [pair, inter] (official arithmetic: BF16 values, times the route weight)

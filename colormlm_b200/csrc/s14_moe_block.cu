@@ -7,7 +7,7 @@
 // The contraction is the one of the one-token layer kernel (s14_moe_umma.cu), widened along N:
 // tcgen05.mma kind::mxf4.block_scale with A = 128 weight rows x 64 K-elements of page bytes as they
 // are, and B = the sixteen balanced base-8 digit rows of EVERY token of a chunk (up to twelve tokens
-// that share the expert: N = 16 * tokens; official arithmetic: eight rows each, up to twenty-four tokens).
+// that share the expert: N = 16 * tokens; official arithmetic: six rows each, up to thirty-two tokens).
 // Accumulator columns 16 t .. 16 t + 15 hold the digit shares of token t's dot products; added without loss and
 // rounded once they give the dot product rounded to F32, so every token's result has the bits that the one-token kernel
 // and the double-accumulating CPU restatement give for that token alone, up to ties closer than a sum in double resolves.
@@ -28,7 +28,8 @@
 // With the official expert arithmetic
 // (fast16/research/polaris_meridian_v1/s14_first_real_token/executor.py:712-743) the same contractions run on
 // quantised inputs: k_block_digits quantises per 128 elements to E4M3FN values (which the digit rows hold
-// exactly), the up epilogue works on BF16 gate and up and multiplies by the route weight, the down epilogue
+// exactly), the up epilogue leaves BF16 gate and up projections, the second k_block_digits makes the hidden values of them
+// (SwiGLU, times the route's weight, BF16), the down epilogue
 // and the mix round to BF16.
 #include "s14_moe_block.cuh"
 
@@ -36,14 +37,14 @@ namespace s14 {
 
 namespace {
 
-// A chunk's B operand is made of groups of sixteen digit rows: one token each, or, in the official arithmetic,
-// whose values need eight digit rows, two tokens (rows 0-7 and 8-15).  Most groups of a chunk:
+// A chunk's B operand is made of groups of sixteen digit rows: one token each; in the official arithmetic,
+// whose values need six digit rows, the tokens' rows follow one another.  Most groups of a chunk:
 constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens: most experts have one, and short stages make the ring deep
 constexpr uint32_t kGrpSparse = 6;   // fewer than three pairs (official arithmetic: six) per expert on average
 constexpr uint32_t kGrpDense = 12;
 // (Both bounds, and the one of twelve tokens, were found with one-CTA kernels that had other stages; on the pair kernel, whose
 // rings hold ten, nine and seven stages, the three sizes have not been compared with each other.)
-static_assert(kBlockNt == 2u * kGrpDense, "a chunk record holds the tokens of the official arithmetic's chunks");
+static_assert(kBlockNt == kGrpDense * 8u / 6u * 2u, "a chunk record holds the tokens of the official arithmetic's chunks");
 
 // The nearest E4M3FN value (ties to even) of |v| <= 448: three mantissa bits; below 2^-6 multiples of 2^-9.
 __device__ __forceinline__ float e4m3fn_round(float v) {
@@ -64,22 +65,47 @@ __device__ __forceinline__ float e4m3fn_round(float v) {
 // 2^ceil(log2(amax / 448)) (F32 quotient, the logarithm taken in double and rounded to F32), x / scale
 // clipped to +-448, rounded to E4M3FN, times the scale.  The quantised values are F32 values with four
 // significant bits: within a scale block, whose largest magnitude is below 2^E, all are multiples of
-// 2^(E-18) (the smallest E4M3FN step is 2^-18 of the range's end), so the eight upper digit rows hold them and
-// the lower eight would be zero.  A tile then is 1 KB (eight rows) and two tokens share sixteen operand rows: half
-// the tile bytes and twice the tokens per pass over a page (official layer of 1000 tokens at 4096 x 2048:
-// 2458 -> 1894 us).
+// 2^(E-18) (the smallest E4M3FN step is 2^-18 of the range's end), so six digit rows hold them (digit6_code_bytes) and a
+// chunk has room for 32 tokens where sixteen rows each leave room for twelve.  The rows of a chunk's tokens follow one another without
+// a gap, so a token's place in the 128-byte swizzle, which goes by the row modulo eight, depends on its place in its CTA's half of
+// the chunk (6 i mod 8: 0, 6, 4, 2 in turn).  A tile of 768 bytes therefore exists in four forms: all four of a token's (it is in
+// seven chunks), the one that its place takes of a pair's (`slots`, from k_block_group).  With eight rows, a tile of 1 KB, and 24 tokens to
+// a chunk 1000 tokens made 408 chunks, so 334.
+// With `slots` the vectors are the pairs' gate and up projections and the hidden values are made of them here, element by element over
+// the whole chip: in the up kernel's epilogue they stood in the way of the next item (see s14_moe_pair.cu).
 template <bool kQuant>
 __global__ void __launch_bounds__(512)
-k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early) {
-    constexpr uint32_t kRows = kQuant ? 8u : 16u;
+k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early,
+               const uint8_t *__restrict__ slots, const float *__restrict__ weights, uint32_t top_k) {
     const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
     // early: the launch in front neither writes x nor uses what is written here (it picks the routes), and whatever is in front
     // of it is complete when this kernel starts, because it lets this one start behind its own wait (a launch that triggers in
     // front of it would make this a race); so the work runs beside it, and the wait for it comes last
     if (!early) dependency_wait();
-    const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
-    const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
-    float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    float xs[8];
+    if (kQuant && slots) {
+        // the hidden values of pair v from its gates and up projections (s14_first_real_token/executor.py:712-743): the limited SwiGLU
+        // in F32, times the route's weight (not for the shared expert), rounded to BF16
+        const uint32_t tok = v / kPairsPerToken, pos = v - tok * kPairsPerToken;
+        const uint16_t *const row = reinterpret_cast<const uint16_t *>(x) + (size_t)v * 2u * K;
+        const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(row) + g), r = __ldcg(reinterpret_cast<const uint4 *>(row + K) + g);
+        const float wt = pos < top_k ? __ldcg(weights + tok * top_k + pos) : 1.0f;
+        const uint32_t gw[4] = {q.x, q.y, q.z, q.w}, uw[4] = {r.x, r.y, r.z, r.w};
+        bool sure[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            sure[i] = swiglu_quick(__uint_as_float((i & 1) ? gw[i >> 1] & 0xFFFF0000u : gw[i >> 1] << 16),
+                                   __uint_as_float((i & 1) ? uw[i >> 1] & 0xFFFF0000u : uw[i >> 1] << 16), wt, xs[i]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (!sure[i])
+                xs[i] = bf16_round(__fmul_rn(swiglu_once(__uint_as_float((i & 1) ? gw[i >> 1] & 0xFFFF0000u : gw[i >> 1] << 16),
+                                                         __uint_as_float((i & 1) ? uw[i >> 1] & 0xFFFF0000u : uw[i >> 1] << 16)), wt));
+    } else {
+        const float4 p0 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g);
+        const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
+        xs[0] = p0.x, xs[1] = p0.y, xs[2] = p0.z, xs[3] = p0.w, xs[4] = p1.x, xs[5] = p1.y, xs[6] = p1.z, xs[7] = p1.w;
+    }
     if constexpr (kQuant) {
         // a group of 128 elements is sixteen neighbouring threads
         float am = 0.0f;
@@ -88,14 +114,31 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
         am = fmaxf(am, 1e-4f);
-        int e = (int)ceilf((float)log2((double)__fdiv_rn(am, 448.0f)));
+        // (where the quotient is well above a power of two the logarithm's F32 value lies between the two integers)
+        const float quot = __fdiv_rn(am, 448.0f);
+        const uint32_t bits = __float_as_uint(quot);   // (normal: am is at least 1e-4)
+        int e = (int)(bits >> 23) - 126;
+        if ((bits & 0x7FFFFFu) < 128u) e = (int)ceilf((float)log2((double)quot));
         e = e < -126 ? -126 : (e > 126 ? 126 : e);
         const float scale = __uint_as_float((uint32_t)(127 + e) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             xs[i] = __fmul_rn(e4m3fn_round(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f)), scale);
     }
-    digits_of8<(int)kRows>(xs, g, dig + (size_t)v * (K >> 8) * (kRows * 128u), exps + (size_t)v * (K >> 5));
+    if constexpr (kQuant) {
+        uint32_t words[6];
+        digits6_of8(xs, g, words, exps + (size_t)v * (K >> 5));
+        const uint32_t kb = g >> 2, forms = slots ? 1u : 4u;
+        for (uint32_t i = 0; i < forms; ++i) {
+            const uint32_t form = slots ? __ldcg(slots + v) & 3u : i;
+            uint8_t *const chunk = dig + ((size_t)(v * forms + i) * (K >> 8) + (kb >> 3)) * 768u + (g & 3u) * 4u;
+#pragma unroll
+            for (uint32_t j = 0; j < 6; ++j)
+                *reinterpret_cast<uint32_t *>(chunk + j * 128u + (((kb & 7u) ^ ((6u * form + j) & 7u)) << 4)) = words[j];
+        }
+    } else {
+        digits_of8(xs, g, dig + (size_t)v * (K >> 8) * 2048u, exps + (size_t)v * (K >> 5));
+    }
     if (early) dependency_wait();
 }
 
@@ -110,7 +153,7 @@ __global__ void __launch_bounds__(1024)
 k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict__ pages,
               const uint8_t *const *__restrict__ page_table, const uint8_t *shared_page, uint32_t T, uint32_t top_k,
               uint32_t n_experts, uint32_t S, uint32_t RT, uint32_t nt_cap, uint32_t even, BlockChunk *__restrict__ chunks,
-              uint32_t *__restrict__ counts, uint32_t ep_rank, uint32_t ep_world, uint32_t shared_by_token) {
+              uint32_t *__restrict__ counts, uint32_t ep_rank, uint32_t ep_world, uint32_t shared_by_token, uint8_t *__restrict__ slots) {
     constexpr uint32_t kG = S14_N_ROUTED_EXPERTS + 1;
     __shared__ uint32_t cnt[kG], fill[kG], chunk0[kG + 1], size[kG];
     __shared__ unsigned long long gpage[kG];
@@ -184,20 +227,28 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
     }
     __syncthreads();
     if (bad) return;
+    // member k of group g: its chunk's record; official arithmetic: also the form its digit tile takes, which goes by the place in
+    // the half of the chunk that a CTA of the pair brings
+    auto place = [&](uint32_t g, uint32_t k, uint32_t pair) {
+        const uint32_t c = k / size[g], t = k - c * size[g];
+        chunks[chunk0[g] + c].pair[t] = pair;
+        if (slots) {
+            const uint32_t nt = min(size[g], cnt[g] - c * size[g]), half = (nt + 1u) >> 1;
+            slots[pair] = (uint8_t)((t < half ? t : t - half) & 3u);
+        }
+    };
 #pragma unroll
     for (uint32_t kk = 0; kk < S14_EXPERTS_PER_TOKEN; ++kk) {
         if (mine_id[kk] < 0) continue;
         const uint32_t i = tid + kk * 1024u, g = 1u + (uint32_t)mine_id[kk], t = i / top_k, m = i - t * top_k;
         const uint32_t k = atomicAdd(&fill[g], 1u);
         if (k == 0u && !page_table) gpage[g] = __ldcg(reinterpret_cast<const unsigned long long *>(pages + i));
-        BlockChunk *ch = chunks + chunk0[g] + k / size[g];
-        ch->pair[k % size[g]] = t * kPairsPerToken + m;
+        place(g, k, t * kPairsPerToken + m);
     }
     if (shared_page) {
         for (uint32_t k = tid; sh_first + k * sh_step < T; k += blockDim.x) {
             const uint32_t t = sh_first + k * sh_step;
-            BlockChunk *ch = chunks + chunk0[0] + k / size[0];
-            ch->pair[k % size[0]] = t * kPairsPerToken + S14_EXPERTS_PER_TOKEN;
+            place(0u, k, t * kPairsPerToken + S14_EXPERTS_PER_TOKEN);
         }
     }
     __syncthreads();
@@ -335,15 +386,17 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     if (n_tokens == 0u) return 0;
     const uint32_t tpg = official ? 2u : 1u;   // tokens per group of sixteen digit rows
     const bool small = n_tokens <= 12u;
+    // (a group is sixteen operand rows: one token, official arithmetic six rows a token; half of a chunk's groups are one CTA's)
     const uint32_t groups = small ? kGrpSmall : ((uint64_t)n_tokens * top_k >= (uint64_t)(3u * tpg) * n_experts ? kGrpDense : kGrpSparse);
     const uint32_t S = inter >> 6, RT = hidden >> 7, counted = small ? 1u : 2u;   // slices, row tiles; as `counts` reports them
+    const uint32_t cap = official ? groups * 8u / 6u * 2u : groups;   // tokens of a chunk: 4, 16, 32, or 2, 6, 12
     // The launches are programmatic dependents of one another: a kernel's blocks, barriers and tensor memory are
     // set up while the one before runs out, and every kernel but the first digits launch (see there) waits for it before it
     // reads or writes anything.
     auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps, bool early) {
         if (*err != cudaSuccess) return;
         *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps,
-                          early ? 1u : 0u);
+                          early ? 1u : 0u, early ? (const uint8_t *)nullptr : (const uint8_t *)w.slots, weights, top_k);
     };
     *err = cudaSuccess;
     // (in front of it: the router's launch, or the copies of the host's routes)
@@ -351,8 +404,8 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     if (ep_world == 0u) ep_world = 1u;
     if (*err == cudaSuccess)
         *err = launch_pdl(k_block_group, dim3(1), dim3(1024), 0, st, 0u, ids, pages, page_table, shared_page, n_tokens, top_k, n_experts,
-                          S / counted, RT / counted, groups * tpg, small ? 1u : 2u * tpg, w.chunks, w.counts, ep_rank, ep_world,
-                          (shared_by_token && ep_world > 1u) ? 1u : 0u);
+                          S / counted, RT / counted, cap, small ? 1u : 2u * tpg, w.chunks, w.counts, ep_rank, ep_world,
+                          (shared_by_token && ep_world > 1u) ? 1u : 0u, official ? w.slots : (uint8_t *)nullptr);
     if (*err != cudaSuccess) return 1;
     if (pairs_out && !ep) {
         // expert parallel: the pairs of the experts this rank owns; the others stay zero for the sum over the ranks
@@ -368,8 +421,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     up.dig = w.xdig;
     up.exps = w.xexp;
     up.hval = w.hval;
-    up.weights = weights;
-    up.top_k = top_k;
+    up.hval16 = reinterpret_cast<uint16_t *>(w.hval);   // (as many bytes)
     down.dig = w.hdig;
     down.exps = w.hexp;
     down.out = pairs_out ? pairs_out : w.d;

@@ -1,6 +1,6 @@
 // The contraction kernels of the grouped block path: a PAIR of CTAs (a cluster of two, the two SMs of a TPC) works on an
 // item together, tcgen05.mma.cta_group::2.  What they compute is described in s14_moe_block.cu; per item it is a chunk
-// of up to twelve groups of sixteen digit rows (one token each, official arithmetic: two) times 256 rows of an expert:
+// of up to twelve tokens of sixteen digit rows (official arithmetic: 32 tokens of six) times 256 rows of an expert:
 // two slices of the up projection or two row tiles of w2.
 //
 // Each CTA brings its own 128 rows of the page (a unit of 17 KB per step of 256 k) and HALF of the chunk's digit tiles; the
@@ -9,21 +9,26 @@
 // item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
 // (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
 // epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 507 / 294
-// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, now 577 / 311.  Small blocks, which took one row tile
+// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, then 577 / 311, now 461 / 258 (see below).  Small blocks, which took one row tile
 // and two tokens per SM with stages of 21 KB in a ring of eight and laid out the hidden values' digit rows in the up epilogue:
 // 8 tokens 117 us for the call, now 109.  (Official blocks of two to eight tokens of smaller layers gained nothing: 4 tokens of
 // 2048 x 1536 49 us for the call, now 52.)
 //
-// What bounds it is not settled.  A step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles
-// (270 for the chunks 370 tokens have on average), the issuing warp's round 470 at most, but a step 700 on average at full
-// clock; the kernels take in 9 to 10.8 TB/s from the L2 meanwhile, and which of the intake and the hand-offs makes up the rest was
-// not measured.  A second warp that copies the codes ahead gets a probe to 389 cycles a
+// What bounds it: a step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles
+// (270 for the chunks 370 tokens have on average), the issuing warp's round 470 at most, but a step 560 on average at full
+// clock; the kernels take in 9 to 10.8 TB/s from the L2 meanwhile.  Beside them the epilogue.  Cycles of an item at full clock,
+// waiting for accumulators / adding their columns / the rest: 370 tokens up 4100 / 3000 / 1950, down 1100 / 3050 / 490; official ones,
+// with exact sums and the SwiGLU here, up 950 / 3900 / 5500, down 540 / 4150 / 1550: there the epilogue was what bounded both
+// kernels (1000 tokens 1036 us, without an epilogue 825, without three of four MMAs 1003, without the tiles' copies 1067), and fewer steps
+// (six digit rows for eight) alone gave nothing.  So BF16 sums are settled by plain additions and a bound where that is possible, four
+// pairs of tokens side by side, and the SwiGLU is k_block_digits' work: 1161 us power limited, now 992.  (The like for F32 sums, one part of the
+// three exact: 370 tokens nothing, 8 tokens 115 -> 120.)  A second warp that copies the codes ahead gets a probe to 389 cycles a
 // step, but adds a hand-off to every stage's way through the ring of seven (370 tokens 736 us instead of 704).  Sustained, the
 // 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.  A pair with more items
-// than a batch of records drains its pipeline between two batches (1000 official tokens: about 90 items, batches of 56).
+// than a batch of records drains its pipeline between two batches (1000 official tokens: 73 items, batches of 56).
 //
 // Roles in a CTA of 608 threads: warps 0-7 epilogue (two warpgroups, each with every lane of tensor memory, the even and
-// the odd groups of the chunk); warps 8-11 copy (the ring slots in turn, a lane per copy: a round of waiting, arming
+// the odd tokens of the chunk, or its halves); warps 8-11 copy (the ring slots in turn, a lane per copy: a round of waiting, arming
 // and seven copies takes 0.3-0.5 us); warp 12 of the first CTA issues the pair's tensor operations, that of the second
 // passes on that its stage is complete; warps 13-18 lay out the scale codes of the digit rows of a stage.  A stage's barriers:
 // `full` in each CTA (unit, tiles, codes; in the first CTA also that the second's is complete), `done` in each (the commit
@@ -138,13 +143,14 @@ __device__ __forceinline__ bool group_all(uint32_t id, bool ok) {
 // 2^(e-39) and summed as it is.  The three parts are exact but for 2^-60 of the largest share - sums in double lose 2^-50 -
 // and are added with the rounding errors of their own sum.  Shares too large or too small for the constants go through double.
 __device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-// columns 0-7 and 8-15 into three parts each
-__device__ __forceinline__ void digit_parts(const uint32_t (&r)[16], float2 sigma, float2 sigma2, float2 &p1, float2 &p2, float2 &p3) {
+// columns first .. first + N - 1 and the N behind them into three parts each
+template <int N, int M>
+__device__ __forceinline__ void digit_parts(const uint32_t (&r)[M], int first, float2 sigma, float2 sigma2, float2 &p1, float2 &p2, float2 &p3) {
     float2 s1 = sigma, s2 = sigma2;
     p3 = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float2 v = make_float2(__uint_as_float(r[c]), __uint_as_float(r[8 + c]));
+    for (int c = 0; c < N; ++c) {
+        const float2 v = make_float2(__uint_as_float(r[first + c]), __uint_as_float(r[first + N + c]));
         const float2 t1 = __fadd2_rn(s1, v);
         const float2 v2 = minus2(v, minus2(t1, s1));
         s1 = t1;
@@ -161,107 +167,91 @@ __device__ __forceinline__ float sum3(float a, float b, float c) {
     const float s = __fadd_rn(a, t), sa = __fsub_rn(s, a), se = __fadd_rn(__fsub_rn(a, __fsub_rn(s, sa)), __fsub_rn(t, sa));
     return __fadd_rn(s, __fadd_rn(se, te));
 }
-// the exponent field of the largest of eight shares and whether the constants made of it are in range
-__device__ __forceinline__ uint32_t share_exponent(const uint32_t (&r)[16], int first) {
+// the exponent field of the largest of N shares and whether the constants made of it are in range
+template <int N, int M>
+__device__ __forceinline__ uint32_t share_exponent(const uint32_t (&r)[M], int first) {
     float m = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) m = fmaxf(m, fabsf(__uint_as_float(r[first + c])));
+    for (int c = 0; c < N; ++c) m = fmaxf(m, fabsf(__uint_as_float(r[first + c])));
     return __float_as_uint(m) & 0x7F800000u;   // (a NaN beside other shares is dropped here and makes the sum one)
 }
 __device__ __forceinline__ bool share_in_range(uint32_t ex) { return ex - (48u << 23) < (192u << 23); }   // 2^-79 .. 2^112
 __device__ __forceinline__ float2 share_sigmas(uint32_t ex) {
     return make_float2(__uint_as_float(ex + (5u << 23) + 0x400000u), __uint_as_float(ex - (15u << 23) + 0x400000u));
 }
-__device__ __forceinline__ void digit_sums_f64(const uint32_t (&r)[16], double &first, double &second) {
-    first = second = 0.0;
+template <int N, int M>
+__device__ __forceinline__ void digit_sums_f64(const uint32_t (&r)[M], int first, double &a, double &b) {
+    a = b = 0.0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        first += (double)__uint_as_float(r[c]);
-        second += (double)__uint_as_float(r[8 + c]);
+    for (int c = 0; c < N; ++c) {
+        a += (double)__uint_as_float(r[first + c]);
+        b += (double)__uint_as_float(r[first + N + c]);
     }
 }
 // all sixteen columns are one token's
 __device__ __forceinline__ float digit_sum(const uint32_t (&r)[16]) {
-    const uint32_t ex = max(share_exponent(r, 0), share_exponent(r, 8));
+    const uint32_t ex = max(share_exponent<8>(r, 0), share_exponent<8>(r, 8));
     if (!share_in_range(ex)) {
         double hi, lo;
-        digit_sums_f64(r, hi, lo);
+        digit_sums_f64<8>(r, 0, hi, lo);
         return (float)(lo + hi);
     }
     const float2 sg = share_sigmas(ex);
     float2 p1, p2, p3;
-    digit_parts(r, make_float2(sg.x, sg.x), make_float2(sg.y, sg.y), p1, p2, p3);
+    digit_parts<8>(r, 0, make_float2(sg.x, sg.x), make_float2(sg.y, sg.y), p1, p2, p3);
     return sum3(__fadd_rn(p1.x, p1.y), __fadd_rn(p2.x, p2.y), __fadd_rn(p3.x, p3.y));   // (the first two additions are exact)
 }
-// columns 0-7 are one token's, 8-15 another's: their sums as BF16
-__device__ __forceinline__ uint32_t digit_sums_pair(const uint32_t (&r)[16]) {
-    const uint32_t e0 = share_exponent(r, 0), e1 = share_exponent(r, 8);
+// official arithmetic: six columns from `first` are one token's, the next six another's: their sums as BF16
+template <int M>
+__device__ __forceinline__ uint32_t digit_sums_pair(const uint32_t (&r)[M], int first) {
+    const uint32_t e0 = share_exponent<6>(r, first), e1 = share_exponent<6>(r, first + 6);
     if (!share_in_range(e0) || !share_in_range(e1)) {
         double a, b;
-        digit_sums_f64(r, a, b);
+        digit_sums_f64<6>(r, first, a, b);
         return bf16_pair((float)a, (float)b);
     }
     const float2 s0 = share_sigmas(e0), s1 = share_sigmas(e1);
     float2 p1, p2, p3;
-    digit_parts(r, make_float2(s0.x, s1.x), make_float2(s0.y, s1.y), p1, p2, p3);
+    digit_parts<6>(r, first, make_float2(s0.x, s1.x), make_float2(s0.y, s1.y), p1, p2, p3);
     return bf16_pair(sum3(p1.x, p2.x, p3.x), sum3(p1.y, p2.y, p3.y));
 }
 
-// The limited SwiGLU (swiglu_limit_f32: the same bits) in F32 operations, as FP64 ones are scarce here (see above).  The
-// exponential by Ziv's method: e^t = 2^n e^r with r = t - n ln 2 in two floats (Cody and Waite's reduction, ln 2 in three
-// parts of which n times the first is exact), e^r by its Taylor series to r^11 / 11!, the terms from r^6 on in F32 and the
-// others in pairs of floats; the pair is within 2^-41 of e^t (4e7 arguments against an 80-bit exponential), so where the
-// bounds 2^-38 to either side round to the same float, that is e^t correctly rounded.  The others, one in 10^4, and gates
-// whose e^-g is beyond 2^57 take the FP64 path.  1000 tokens of the official arithmetic: 1160 us with FP64, now
-// 1124 (power limited 1245 and 1187).
-__device__ __noinline__ float swiglu_f64(float gate, float up) { return swiglu_limit_f32(gate, up); }
-__device__ __forceinline__ float swiglu_pair(float gate, float up) {
-    const float g = fminf(gate, 10.0f), u = fminf(fmaxf(up, -10.0f), 10.0f), t = -g;
-    const float n = rintf(__fmul_rn(t, 1.44269502f));
-    const float r0 = __fmaf_rn(n, -0x1.62e4p-1f, t);   // exact
-    const float p = __fmul_rn(n, 0x1.7f7d1cp-20f), pe = __fmaf_rn(n, 0x1.7f7d1cp-20f, -p);
-    const float a = __fsub_rn(r0, p), bb = __fsub_rn(a, r0);
-    const float al = __fmaf_rn(n, -0x1.ef357ap-45f,
-                               __fsub_rn(__fadd_rn(__fsub_rn(r0, __fsub_rn(a, bb)), __fsub_rn(-p, bb)), pe));
-    const float rh = __fadd_rn(a, al), rl = __fsub_rn(al, __fsub_rn(rh, a));
-    float h = __fmaf_rn(rh, 2.50521084e-8f, 2.75573192e-7f);
-    h = __fmaf_rn(rh, h, 2.75573188e-6f);
-    h = __fmaf_rn(rh, h, 2.48015876e-5f);
-    h = __fmaf_rn(rh, h, 1.98412701e-4f);
-    h = __fmaf_rn(rh, h, 1.38888892e-3f);
-    float l = 0.0f;
-    // (h, l) = c + r (h, l), c = 1 / 5! ... 1 / 0!
-    auto horner = [&](float c, float c_low) {
-        const float ph = __fmul_rn(rh, h), pl = __fmaf_rn(rl, h, __fmaf_rn(rh, l, __fmaf_rn(rh, h, -ph)));
-        h = __fadd_rn(c, ph);
-        l = __fadd_rn(__fsub_rn(ph, __fsub_rn(h, c)), __fadd_rn(pl, c_low));
-    };
-    horner(0x1.111112p-7f, -0x1.dddddep-32f);
-    horner(0x1.555556p-5f, -0x1.555556p-30f);
-    horner(0x1.555556p-3f, -0x1.555556p-28f);
-    horner(0.5f, 0.0f);
-    horner(1.0f, 0.0f);
-    horner(1.0f, 0.0f);
-    const float s = __fadd_rn(h, l), sl = __fsub_rn(l, __fsub_rn(s, h)), err = __fmul_rn(s, 0x1p-38f);
-    const float e0 = __fadd_rn(s, __fadd_rn(sl, err)), e1 = __fadd_rn(s, __fsub_rn(sl, err));
-    if (!(t < 40.0f) || e0 != e1) return swiglu_f64(gate, up);
-    const float e = __fmul_rn(e0, __uint_as_float((uint32_t)((int)n + 127) << 23));
-    return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, e)), u);
+// The same by plain additions, the smallest digits first, where that settles the BF16 values: each of the five sums on the way is
+// rounded once, by at most 2^-24 of it, so where 2^-23 of their magnitudes' sum to either side (which leaves room for the
+// roundings here) rounds to the same BF16 value, that is the exact sum's, and its F32 rounding's.  False, and nothing in `out`, for the
+// others (one in some thousand; with a bound made of the largest share every other warp had one).
+template <int M>
+__device__ __forceinline__ bool digit_sums_quick(const uint32_t (&r)[M], int first, uint32_t &out) {
+    float2 s = make_float2(__uint_as_float(r[first]), __uint_as_float(r[first + 6]));
+    float ma = 0.0f, mb = 0.0f;
+#pragma unroll
+    for (int c = 1; c < 6; ++c) {
+        s = __fadd2_rn(s, make_float2(__uint_as_float(r[first + c]), __uint_as_float(r[first + 6 + c])));
+        ma = __fadd_rn(ma, fabsf(s.x));
+        mb = __fadd_rn(mb, fabsf(s.y));
+    }
+    const float2 lo = __ffma2_rn(make_float2(ma, mb), make_float2(-0x1p-23f, -0x1p-23f), s);
+    const float2 hi = __ffma2_rn(make_float2(ma, mb), make_float2(0x1p-23f, 0x1p-23f), s);
+    out = bf16_pair(lo.x, lo.y);
+    return out == bf16_pair(hi.x, hi.y);
 }
+
+// Operand rows of half a chunk of nt tokens, a multiple of sixteen: those of the first (nt + 1) / 2 tokens.
+template <uint32_t kRows>
+__device__ __forceinline__ uint32_t half_rows(uint32_t nt) { return (((nt + 1u) >> 1) * kRows + 15u) & ~15u; }
 
 template <bool kDown, bool kOff>
 __global__ void __launch_bounds__(kPThreads, 1)
 k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr uint32_t kTpg = kOff ? 2u : 1u;                     // tokens per group of sixteen digit rows
-    constexpr uint32_t kRows = 16u / kTpg, kTileB = kRows * 128u; // a token's digit rows, and the bytes of its tile
-    constexpr uint32_t kTok = kPGroups * kTpg;                    // most tokens of a chunk
-    constexpr uint32_t kMine = kPGroups / 2u;                     // groups of an epilogue thread
+    constexpr uint32_t kRows = kOff ? 6u : 16u, kTileB = kRows * 128u;   // a token's digit rows, and the bytes of its tile
+    constexpr uint32_t kTok = kPCols / 2u / kRows * 2u;           // most tokens of a chunk
+    constexpr uint32_t kMine = kOff ? kTok / 4u : kPGroups / 2u;  // tokens of an epilogue thread (official: pairs of them)
     constexpr uint32_t kPBatch = kOff ? 56u : 96u;                // items decoded at a time (10 KB of static shared memory are left beside the ring)
     __shared__ __align__(8) uint64_t bars[kPBars];
     __shared__ __align__(16) PairItem s_rec[kPBatch];
     __shared__ uint32_t s_pair[kPBatch][kTok];
-    __shared__ float s_x[2][kMine][64];                           // an item's gates and up projections, handed across (official: two BF16 each)
+    __shared__ float s_x[2][kOff ? 1u : kMine][64];               // an item's gates and up projections, handed across
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -350,14 +340,15 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i) {
                 const uint32_t multi = warp_uniform(s_rec[i].nt >> 8), nt = warp_uniform(s_rec[i].nt & 0xFFu);
-                const uint32_t half = (((nt + kTpg - 1u) / kTpg + 1u) >> 1) * kTpg, first = rank * half;   // this CTA's tokens
+                const uint32_t half = (nt + 1u) >> 1, first = rank * half;   // this CTA's tokens
                 const uint32_t mine = nt > first ? min(nt - first, half) : 0u;
                 // a lane's copy of every stage: lane t < mine the tile of a token, the last lane the unit
                 const bool is_unit = lane == 31u;
                 const uint8_t *src = reinterpret_cast<const uint8_t *>(s_rec[i].page) + page_off +
                                      (size_t)(s_rec[i].r * 2u + rank) * nu * kUnitStride;
                 if (lane < mine) {
-                    const uint32_t vec = kDown ? s_pair[i][first + lane] : s_pair[i][first + lane] / kPairsPerToken;
+                    uint32_t vec = kDown ? s_pair[i][first + lane] : s_pair[i][first + lane] / kPairsPerToken;
+                    if constexpr (kOff && !kDown) vec = vec * 4u + (lane & 3u);   // the form for this place
                     src = a.dig + (size_t)vec * nu * kTileB;
                 }
                 const uint32_t bytes = is_unit ? kUnitStride : kTileB, to = ring0 + (is_unit ? 0u : kStageA + lane * kTileB);
@@ -388,7 +379,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll 1
                 for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
                     const uint32_t buf = gi & 1u, nt = warp_uniform(s_rec[i].nt & 0xFFu);
-                    const uint32_t n = 32u * (((nt + kTpg - 1u) / kTpg + 1u) >> 1), idesc = pair_idesc(n);
+                    const uint32_t n = 2u * half_rows<kRows>(nt), idesc = pair_idesc(n);
                     if (gi >= 2u) ok = stage_wait(bar(kPBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
                     if (!ok) break;
                     fence_after();
@@ -446,36 +437,43 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
             for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
                 const uint32_t buf = gi & 1u, nt = s_rec[i].nt & 0xFFu, idx = s_rec[i].r * 2u + rank;   // slice or row tile
                 const uint32_t *pair = s_pair[i];
-                float wt[kOff && !kDown ? kMine : 1u];   // official: the route weights of the tokens this thread finishes
-                if constexpr (kOff && !kDown) {
-#pragma unroll
-                    for (uint32_t m = 0; m < kMine; ++m) {
-                        const uint32_t t = 2u * (2u * m + wg) + par;
-                        wt[m] = 1.0f;
-                        if (t < nt) {
-                            const uint32_t tok = pair[t] / kPairsPerToken, pos = pair[t] - tok * kPairsPerToken;
-                            if (pos < S14_EXPERTS_PER_TOKEN) wt[m] = __ldcg(a.weights + tok * a.top_k + pos);
-                        }
-                    }
-                }
+                // official: this warpgroup's half of the chunk, its first token and how many there are
+                const uint32_t t0 = wg * ((nt + 1u) >> 1), n_tok = nt > t0 ? min(nt - t0, (nt + 1u) >> 1) : 0u;
                 ok = group_all(1u + wg, mbar_wait(bar(kPBarAccDone + buf), (gi >> 1) & 1u, abortp));
                 if (!ok) break;
                 fence_after();
-                // groups wg, wg + 2, ... of the chunk; official: two BF16 values to a register
+                // tokens wg, wg + 2, ... of the chunk; official: those of its half, two BF16 values to a register
                 float v[kOff ? 1u : kMine];
-                uint32_t vb[kOff ? kMine : 1u];
+                uint32_t vb[kOff ? kMine : 1u] = {};
+                if constexpr (kOff) {
+                    // eight tokens' six columns each at a time
+                    const uint32_t at = lane_base + buf * kPCols + wg * half_rows<kRows>(nt);
 #pragma unroll
-                for (uint32_t m = 0; m < kMine; m += 2u) {
-                    const uint32_t g = 2u * m + wg;
-                    if (g * kTpg < nt) {   // uniform in the warpgroup
-                        uint32_t r0[16], r1[16];
-                        tmem_ld16(lane_base + buf * kPCols + 16u * g, r0);
-                        tmem_ld16(lane_base + buf * kPCols + 16u * (g + 2u), r1);   // (not used beyond nt)
-                        tmem_ld_wait();
-                        if constexpr (kOff) {
-                            vb[m] = digit_sums_pair(r0);
-                            vb[m + 1u] = digit_sums_pair(r1);
-                        } else {
+                    for (uint32_t m = 0; m < kMine; m += 4u) {
+                        if (2u * m < n_tok) {   // uniform in the warpgroup
+                            uint32_t r[48];     // (columns beyond the half's rows are not used)
+                            tmem_ld16(at + 12u * m, *reinterpret_cast<uint32_t(*)[16]>(r));
+                            tmem_ld16(at + 12u * m + 16u, *reinterpret_cast<uint32_t(*)[16]>(r + 16));
+                            tmem_ld16(at + 12u * m + 32u, *reinterpret_cast<uint32_t(*)[16]>(r + 32));
+                            tmem_ld_wait();
+                            // (without a branch between the four, so that their chains run side by side)
+                            bool sure[4];
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; ++k) sure[k] = digit_sums_quick(r, 12 * (int)k, vb[m + k]);
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; ++k)
+                                if (!sure[k] && 2u * (m + k) < n_tok) vb[m + k] = digit_sums_pair(r, 12 * (int)k);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; m += 2u) {
+                        const uint32_t g = 2u * m + wg;
+                        if (g < nt) {   // uniform in the warpgroup
+                            uint32_t r0[16], r1[16];
+                            tmem_ld16(lane_base + buf * kPCols + 16u * g, r0);
+                            tmem_ld16(lane_base + buf * kPCols + 16u * (g + 2u), r1);   // (not used beyond nt)
+                            tmem_ld_wait();
                             v[m] = digit_sum(r0);
                             v[m + 1u] = digit_sum(r1);
                         }
@@ -489,10 +487,10 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll
                     for (uint32_t m = 0; m < kMine; ++m) {
 #pragma unroll
-                        for (uint32_t k = 0; k < kTpg; ++k) {
-                            const uint32_t t = (2u * m + wg) * kTpg + k;
-                            if (t < nt) {
-                                const size_t at = (size_t)pair[t] * a.hidden + idx * 128u + row;
+                        for (uint32_t k = 0; k < (kOff ? 2u : 1u); ++k) {
+                            const uint32_t t = kOff ? 2u * m + k : 2u * m + wg;
+                            if (t < (kOff ? n_tok : nt)) {
+                                const size_t at = (size_t)pair[kOff ? t0 + t : t] * a.hidden + idx * 128u + row;
                                 float o;
                                 if constexpr (kOff) o = __uint_as_float(k ? vb[m] & 0xFFFF0000u : vb[m] << 16);   // (a linear's result is BF16)
                                 else o = v[m];
@@ -505,40 +503,29 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                             }
                         }
                     }
+                } else if constexpr (kOff) {
+                    // threads 0-63 of the warpgroup hold the gates of the slice's elements, threads 64-127 their up projections: BF16
+                    // values into the pair's two rows (the rest is element by element and k_block_digits')
+#pragma unroll
+                    for (uint32_t m = 0; m < kMine; ++m) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 2; ++k)
+                            if (2u * m + k < n_tok)
+                                a.hval16[((size_t)pair[t0 + 2u * m + k] * 2u + par) * a.inter + idx * 64u + el] = (uint16_t)(k ? vb[m] >> 16 : vb[m]);
+                    }
                 } else {
                     // threads 0-63 of the warpgroup hold the gates of the slice's elements, threads 64-127 their up
                     // projections.  Each half finishes half of the tokens and hands the other the values it lacks.
-                    // Official arithmetic (s14_first_real_token/executor.py:712-743): gate and up rounded to BF16, the
-                    // limited SwiGLU in F32, times the route's weight (not for the shared expert), rounded to BF16.
-                    uint16_t *const s_h = reinterpret_cast<uint16_t *>(&s_x[wg][0][0]);   // [kMine][2][64]
 #pragma unroll
-                    for (uint32_t m = 0; m < kMine; ++m) {
-                        if constexpr (kOff) {
-                            if ((2u * m + wg) * 2u < nt) s_h[(m * 2u + par) * 64u + el] = (uint16_t)(par ? vb[m] & 0xFFFFu : vb[m] >> 16);
-                        } else {
-                            if (2u * m + wg < nt && (m & 1u) != par) s_x[wg][m][el] = v[m];
-                        }
-                    }
+                    for (uint32_t m = 0; m < kMine; ++m)
+                        if (2u * m + wg < nt && (m & 1u) != par) s_x[wg][m][el] = v[m];
                     group_all(1u + wg, true);
 #pragma unroll
                     for (uint32_t m = 0; m < kMine; ++m) {
-                        const uint32_t t = kOff ? 2u * (2u * m + wg) + par : 2u * m + wg;
-                        if (t < nt && (kOff || (m & 1u) == par)) {
-                            float mine, other;
-                            if constexpr (kOff) {
-                                mine = __uint_as_float(par ? vb[m] & 0xFFFF0000u : vb[m] << 16);
-                                other = __uint_as_float((uint32_t)s_h[(m * 2u + (par ^ 1u)) * 64u + el] << 16);
-                            } else {
-                                mine = v[m];
-                                other = s_x[wg][m][el];
-                            }
-                            float hv = par ? swiglu_pair(other, mine) : swiglu_pair(mine, other);
-                            if constexpr (kOff) {
-                                const uint32_t pos = pair[t] % kPairsPerToken;
-                                if (pos < S14_EXPERTS_PER_TOKEN) hv = __fmul_rn(hv, wt[m]);
-                                hv = bf16_round(hv);
-                            }
-                            a.hval[(size_t)pair[t] * a.inter + idx * 64u + el] = hv;
+                        const uint32_t t = 2u * m + wg;
+                        if (t < nt && (m & 1u) == par) {
+                            const float mine = v[m], other = s_x[wg][m][el];
+                            a.hval[(size_t)pair[t] * a.inter + idx * 64u + el] = par ? swiglu_pair(other, mine) : swiglu_pair(mine, other);
                         }
                     }
                 }
@@ -550,19 +537,32 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
             // exponent E has the code 127 + E - 23 + 3 j, row 8 + j the code 127 + E - 47 + 3 j; the exponents are stored as
             // E + 100. ----
             const uint32_t n = tid - kPCodeWarp0 * 32u;   // this thread's row
-            const uint32_t j = n & (kRows - 1u), n_tok = n / kRows;
-            const uint32_t bias = 0x01010101u * (uint32_t)(j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20);
             const uint32_t code_at = off_codes + (n >> 7) * kAtomBytes + (n & 31u) * 16u + ((n >> 5) & 3u) * 4u;
             const bool has_row = n < half_cap * 32u;
-            // the row's exponents in an item, or nullptr
+            // the row's exponents in an item, or nullptr, and (official: where the second half's rows start differs from item to item)
+            // what is added to them
+            uint32_t bias = 0u, bias_then = 0u;
+            if constexpr (!kOff) {
+                const uint32_t j = n & 15u;
+                bias = bias_then = 0x01010101u * (uint32_t)(j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20);
+            }
             auto exps_of = [&](uint32_t i) -> const uint4 * {
-                if (i >= nb || !has_row || n_tok >= (s_rec[i].nt & 0xFFu)) return nullptr;
-                const uint32_t vec = kDown ? s_pair[i][n_tok] : s_pair[i][n_tok] / kPairsPerToken;
+                if (i >= nb || !has_row) return nullptr;
+                const uint32_t nt = s_rec[i].nt & 0xFFu;
+                uint32_t t = n / kRows;
+                if constexpr (kOff) {
+                    const uint32_t half = (nt + 1u) >> 1, hr = half_rows<kRows>(nt), m = n < hr ? n : n - hr, in = m / kRows;
+                    t = in < half ? (n < hr ? in : half + in) : nt;   // (rows between the halves belong to nobody)
+                    bias_then = 0x01010101u * (10u + 3u * (m - in * kRows));
+                }
+                if (t >= nt) return nullptr;
+                const uint32_t vec = kDown ? s_pair[i][t] : s_pair[i][t] / kPairsPerToken;
                 return reinterpret_cast<const uint4 *>(a.exps + (size_t)vec * (K >> 5));
             };
             // two units' exponents per load, four loads in flight, each in registers of its own (a queue that moves them waits
             // for the newest): the units in steps of eight, the last step of an item perhaps short
             const uint4 *now = exps_of(0);
+            bias = bias_then;
             uint4 e[4];
             auto fetch = [&](const uint4 *p, uint32_t u) { return p && u < nu ? __ldcg(p + (u >> 1)) : make_uint4(0u, 0u, 0u, 0u); };
 #pragma unroll
@@ -597,6 +597,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                     }
                 }
                 now = then;
+                bias = bias_then;
             }
         }
         __syncwarp();

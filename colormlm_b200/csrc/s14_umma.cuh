@@ -223,9 +223,7 @@ __device__ __forceinline__ int block_exponent(float bm) {
 // elements: sixteen rows of 128 bytes, the 16-byte chunk of scale block kb at position
 // (kb % 8) ^ (row % 8)) and, for the first thread of a scale block, the block's exponent.  Thread g
 // owns one 32-bit word of every digit row; the four lanes of a scale block agree on its exponent,
-// so whole warps call this together.  kRows = 8: the upper 24 bits alone (1 KB tiles of eight rows), for
-// values that are integer multiples of 2^(E-23), whose lower digits are zero.
-template <int kRows = 16>
+// so whole warps call this together.
 __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uint8_t *sB, uint8_t *sE) {
     float bm = 0.0f;
 #pragma unroll
@@ -237,7 +235,7 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
     // Four elements at a time: their code bytes [element][hi digits 0-3, hi 4-7, lo 0-3, lo 4-7] are
     // transposed to [digit row][element] and squeezed to nibbles; the two halves of a row's word are
     // joined at the end.
-    uint32_t half[2][kRows];
+    uint32_t half[2][16];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t c[4][4];
@@ -246,10 +244,10 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
             int hi, lo;
             split_hi_lo(xs[h * 4 + i], up, hi, lo);
             digit_code_bytes(hi, c[i][0], c[i][1]);
-            if constexpr (kRows == 16) digit_code_bytes(lo, c[i][2], c[i][3]);
+            digit_code_bytes(lo, c[i][2], c[i][3]);
         }
 #pragma unroll
-        for (int q4 = 0; q4 < kRows / 4; ++q4) {  // four digit rows at a time
+        for (int q4 = 0; q4 < 4; ++q4) {  // four digit rows at a time
             uint32_t a[4];
             transpose4(c[0][q4], c[1][q4], c[2][q4], c[3][q4], a);
 #pragma unroll
@@ -257,15 +255,62 @@ __device__ __forceinline__ void digits_of8(const float (&xs)[8], uint32_t g, uin
         }
     }
     // word of digit row j: the codes of elements 0..7 in nibbles 0..7
-    uint32_t words[kRows];
+    uint32_t words[16];
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) words[j] = pack_pairs(half[0][j], half[1][j]);
+    for (int j = 0; j < 16; ++j) words[j] = pack_pairs(half[0][j], half[1][j]);
     const uint32_t kb = g >> 2;
-    uint8_t *chunk = sB + (kb >> 3) * (kRows * 128u) + (g & 3u) * 4u;
+    uint8_t *chunk = sB + (kb >> 3) * 2048u + (g & 3u) * 4u;
 #pragma unroll
-    for (uint32_t j = 0; j < (uint32_t)kRows; ++j)
+    for (uint32_t j = 0; j < 16u; ++j)
         *reinterpret_cast<uint32_t *>(chunk + j * 128u + (((kb & 7u) ^ (j & 7u)) << 4)) = words[j];
     if ((g & 3u) == 0u) sE[kb] = (uint8_t)(E + 100);  // the block's exponent, biased
+}
+
+// Six digit rows for values that are E4M3FN numbers times a power of two (four significant bits, and multiples of 2^(E-18)
+// where the scale block's largest magnitude is below 2^E): v = 2^(E-17) * sum_j c_j 8^j with every c_j an E2M1 value.  Of the
+// integer q = v 2^(18-E) = sum_j d_j 8^j the lower digits are balanced (-4 .. 3), the top one is in [-8, 8]; E2M1 holds half of any
+// of 0, 1, 2, 3, 4, 6, 8, 12.  A top digit of 5 or 7 goes one further from zero and the digit below it, which is 0 or -4 there (q is a
+// multiple of 2^14 then), takes the 8 back: 0, +-4, +-8 or -12.  All 254 values at every E of theirs, and so
+// times any scale: checked one by one.
+// Row j's scale is 2^(E-17+3j).
+__device__ __forceinline__ void digit6_code_bytes(int q, uint32_t &c03, uint32_t &c45) {
+    const uint32_t qb = (uint32_t)(q + 280868);   // 4 (8^5 - 1) / 7 + 8 * 8^5
+    uint32_t x = (qb & 0x3Fu) | ((qb & 0xFC0u) << 2);
+    x = (x & 0x0707u) | ((x & 0x3838u) << 1);     // field j (digit + 4) in nibble j, j < 4
+    c03 = prmt(0x090A0B0Cu, 0x03020100u, x);
+    const uint32_t f = (qb >> 12) & 7u, top = qb >> 15;   // top digit + 8: 1 .. 16
+    uint32_t c4 = (0x32109ABCu >> (4u * f)) & 0xFu;
+    if (top == 13u || top == 15u) c4 = f ? 0xEu : 0xFu;
+    if (top == 1u || top == 3u) c4 = f ? 6u : 4u;
+    const uint32_t c5 = (uint32_t)(0x6655432109ABCDDEull >> (4u * (top - 1u))) & 0xFu;
+    c45 = c4 | (c5 << 8);
+}
+// The words of the six digit rows of elements 8g .. 8g+7 and, from the first thread of a scale block, its exponent.
+__device__ __forceinline__ void digits6_of8(const float (&xs)[8], uint32_t g, uint32_t (&words)[6], uint8_t *sE) {
+    float bm = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bm = fmaxf(bm, fabsf(xs[i]));
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
+    const int E = block_exponent(bm);
+    const float up = __uint_as_float((uint32_t)(145 - E) << 23);  // 2^(18-E)
+    uint32_t half[2][6];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t c[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) digit6_code_bytes(__float2int_rn(xs[h * 4 + i] * up), c[i][0], c[i][1]);
+        uint32_t a[4], b[4];
+        transpose4(c[0][0], c[1][0], c[2][0], c[3][0], a);
+        transpose4(c[0][1], c[1][1], c[2][1], c[3][1], b);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) half[h][k] = pair_nibbles(a[k]);
+        half[h][4] = pair_nibbles(b[0]);
+        half[h][5] = pair_nibbles(b[1]);
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) words[j] = pack_pairs(half[0][j], half[1][j]);
+    if ((g & 3u) == 0u) sE[g >> 2] = (uint8_t)(E + 100);
 }
 
 // The scale codes of the sixteen digit rows of a vector of K elements, written to tensor memory by

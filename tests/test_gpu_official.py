@@ -157,3 +157,28 @@ def test_official_block_runs_on_one_gpu_only(ctx):
             blk.set_semantics(True)
     finally:
         blk.close()
+
+
+# chunks of 32 tokens and what is left over, halves of odd sizes, rows of six beside the sixteen of an operand; tokens whose gates
+# are far beyond the limit on either side, and tiny ones
+@pytest.mark.parametrize("n_tokens,n_experts", [(13, 1), (17, 6), (31, 1), (33, 1), (47, 3), (64, 2), (65, 2), (131, 4)])
+@pytest.mark.parametrize("hidden,inter", [(512, 512), (1024, 1536)])
+def test_official_blocks_of_full_chunks(ctx, oracle, n_tokens, n_experts, hidden, inter):
+    g, pages, shared = make_layer(2300 + n_tokens, hidden, inter, n_experts, L.PAGE_MXFP4)
+    x = synth.activations(g, n_tokens, hidden)
+    x[::5] *= np.float32(60.0)
+    x[1::5] *= np.float32(1e-4)
+    x[2, 64:96] = 0.0
+    routes = [(ids, w[:len(ids)]) for ids, w in random_routes(g, n_tokens, n_experts, ragged=True)]
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    blk = MoeBlock(ctx, hidden, inter, n_tokens)
+    try:
+        blk.set_semantics(True)
+        y = run_block(ctx, blk, x, pages_dev, shared_dev, routes)
+        for t in range(n_tokens):
+            ids, w = routes[t]
+            ref = oracle.official_moe_layer(x[t], [pages[i] for i in ids], w, shared, 0, hidden, inter)
+            bad = np.nonzero(y[t].view(np.uint32) != ref.view(np.uint32))[0]
+            assert bad.size == 0, (t, bad.size, bad[:8], y[t][bad[:4]], ref[bad[:4]])
+    finally:
+        blk.close()
