@@ -46,17 +46,15 @@ constexpr uint32_t kGrpDense = 12;
 // rings hold ten, nine and seven stages, the three sizes have not been compared with each other.)
 static_assert(kBlockNt == kGrpDense * 8u / 6u * 2u, "a chunk record holds the tokens of the official arithmetic's chunks");
 
-// The nearest E4M3FN value (ties to even) of |v| <= 448: three mantissa bits; below 2^-6 multiples of 2^-9.
-__device__ __forceinline__ float e4m3fn_round(float v) {
-    const float a = fabsf(v);
-    float q;
-    if (a < 0.015625f) {
-        q = __fmul_rn(rintf(__fmul_rn(a, 512.0f)), 0.001953125f);
-    } else {
-        const int e = (int)(__float_as_uint(a) >> 23) - 127;   // floor(log2 a)
-        q = __fmul_rn(rintf(__fmul_rn(a, __uint_as_float((uint32_t)(130 - e) << 23))), __uint_as_float((uint32_t)(124 + e) << 23));
-    }
-    return copysignf(q, v);
+// The nearest E4M3FN values (ties to even) of two numbers of magnitude 448 at most, as F32 values: the conversion there and back.
+// (Rounded by shifts of the exponent, with a branch for the subnormals, the second digits launch of 1000 tokens at 4096 x 2048 took
+// 70 us and takes 56, the first 24 and 18.)
+__device__ __forceinline__ float2 e4m3fn_round2(float a, float b) {
+    uint16_t p;
+    uint32_t h;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(p) : "f"(b), "f"(a));   // (the second operand is the lower byte)
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"(p));
+    return __half22float2(*reinterpret_cast<const __half2 *>(&h));
 }
 
 // The digit tiles and block exponents of n vectors of K elements (one CTA per vector).  With `quant` the
@@ -122,8 +120,11 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
         e = e < -126 ? -126 : (e > 126 ? 126 : e);
         const float scale = __uint_as_float((uint32_t)(127 + e) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            xs[i] = __fmul_rn(e4m3fn_round(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f)), scale);
+        for (int i = 0; i < 8; i += 2) {
+            const float2 q = e4m3fn_round2(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f), fminf(fmaxf(__fmul_rn(xs[i + 1], inv), -448.0f), 448.0f));
+            xs[i] = __fmul_rn(q.x, scale);
+            xs[i + 1] = __fmul_rn(q.y, scale);
+        }
     }
     if constexpr (kQuant) {
         uint32_t words[6];
