@@ -273,17 +273,20 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 
 // y[t, n]: the ordered mix of token t (examples/s14_vulkan_numeric.rs:936-946): acc = 0; acc += w * d
 // over the routes in order; acc += d of the shared expert.  With `residual` the layer's input is added
-// (y = x + acc, what a layer of a stack hands to the next); y may be x.  Four outputs
-// per thread, the seven rows' loads in flight together (one value per thread,
+// (y = x + acc, what a layer of a stack hands to the next); y may be x.  16 bytes of each
+// row per thread, the seven rows' loads in flight together (one value per thread,
 // row after row: 64 us for 1000 tokens of 4096, now 28).  Compiled for aligned buffers and for others: with both forms in one
 // kernel the code that every warp fetches once was longer (a block of 45 tokens 148.1 us, so 147.6).
-template <bool vec>
-__global__ void __launch_bounds__(256)
+// The official arithmetic's rows are BF16 values and are stored as such: 115 MB written and read for 1000 tokens, stored as F32, now 57
+// (the call, with its down kernel, 973 us power limited, now 956).  CTAs of 128 threads: 256 took 0.3 us more for a block of 8 tokens.
+template <bool vec, bool kOff>
+__global__ void __launch_bounds__(128)
 k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const float *__restrict__ weights,
             uint32_t top_k, int has_shared, float *y, uint32_t hidden, const uint32_t *__restrict__ counts,
             const float *x, uint32_t residual, const unsigned long long *flags, uint32_t ep_rank, uint32_t ep_world, uint32_t ep_call,
-            uint32_t wait_limit, uint32_t *status, uint32_t official) {
-    const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * 4u, t = blockIdx.y;   // hidden is a multiple of four
+            uint32_t wait_limit, uint32_t *status) {
+    constexpr uint32_t kPer = kOff ? 8u : 4u;
+    const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * kPer, t = blockIdx.y;   // hidden is a multiple of eight
     dependency_wait();
     const uint32_t why = __ldcg(counts + 3);
     if (flags) {
@@ -315,14 +318,32 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
         if (!s_ok) return;
     }
     if (n >= hidden || why) return;
-    const float *dt = d + (size_t)t * kPairsPerToken * hidden + n;
+    const size_t at = (size_t)t * kPairsPerToken * hidden + n;
     // (a caller's buffers may lie on any 4-byte boundary)
-    auto load4 = [&](const float *p) {
-        return vec ? __ldcg(reinterpret_cast<const float4 *>(p)) : make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+    auto load = [&](const float *p, float(&r)[kPer]) {
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; i += 4u) {
+            if constexpr (vec) {
+                const float4 q = __ldcg(reinterpret_cast<const float4 *>(p + i));
+                r[i] = q.x, r[i + 1u] = q.y, r[i + 2u] = q.z, r[i + 3u] = q.w;
+            } else {
+                r[i] = __ldcg(p + i), r[i + 1u] = __ldcg(p + i + 1u), r[i + 2u] = __ldcg(p + i + 2u), r[i + 3u] = __ldcg(p + i + 3u);
+            }
+        }
+    };
+    auto load_row = [&](uint32_t m, float(&r)[kPer]) {
+        if constexpr (kOff) {
+            const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const uint16_t *>(d) + at + (size_t)m * hidden));
+            const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (uint32_t i = 0; i < kPer; ++i) r[i] = __uint_as_float((i & 1u) ? qw[(i >> 1) & 3u] & 0xFFFF0000u : qw[(i >> 1) & 3u] << 16);
+        } else {
+            load(d + at + (size_t)m * hidden, r);
+        }
     };
     // official arithmetic: the route's weight went into the expert's hidden values; the BF16 outputs are added
     // in F32 and the sum is rounded to BF16 (moe_branch, s14_first_real_token/executor.py:716-735)
-    float4 row[S14_EXPERTS_PER_TOKEN + 1];
+    float row[S14_EXPERTS_PER_TOKEN + 1][kPer] = {}, in[kPer] = {};
     float w[S14_EXPERTS_PER_TOKEN];
     bool there[S14_EXPERTS_PER_TOKEN];
 #pragma unroll
@@ -331,34 +352,41 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
         // wait for the id)
         there[m] = m < top_k && __ldcg(ids + t * top_k + m) >= 0;
         w[m] = m < top_k ? __ldcg(weights + t * top_k + m) : 0.0f;
-        row[m] = m < top_k ? load4(dt + (size_t)m * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m < top_k) load_row(m, row[m]);
     }
     constexpr uint32_t kSh = S14_EXPERTS_PER_TOKEN;
-    row[kSh] = has_shared ? load4(dt + (size_t)kSh * hidden) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 in = residual ? load4(x + (size_t)t * hidden + n) : make_float4(0.f, 0.f, 0.f, 0.f);
-    auto mix = [&](float float4::*c) {
+    if (has_shared) load_row(kSh, row[kSh]);
+    if (residual) load(x + (size_t)t * hidden + n, in);
+    float out[kPer];
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
         float acc = 0.0f;
 #pragma unroll
         for (uint32_t m = 0; m < S14_EXPERTS_PER_TOKEN; ++m)
-            if (there[m]) acc = __fadd_rn(acc, official ? row[m].*c : __fmul_rn(w[m], row[m].*c));
-        if (has_shared) acc = __fadd_rn(acc, row[kSh].*c);
-        if (official) acc = bf16_round(acc);
-        return residual ? __fadd_rn(in.*c, acc) : acc;
-    };
-    const float4 out = make_float4(mix(&float4::x), mix(&float4::y), mix(&float4::z), mix(&float4::w));
+            if (there[m]) acc = __fadd_rn(acc, kOff ? row[m][i] : __fmul_rn(w[m], row[m][i]));
+        if (has_shared) acc = __fadd_rn(acc, row[kSh][i]);
+        if (kOff) acc = bf16_round(acc);
+        out[i] = residual ? __fadd_rn(in[i], acc) : acc;
+    }
     float *yt = y + (size_t)t * hidden + n;
-    if (vec) *reinterpret_cast<float4 *>(yt) = out;
-    else yt[0] = out.x, yt[1] = out.y, yt[2] = out.z, yt[3] = out.w;
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; i += 4u) {
+        if constexpr (vec) *reinterpret_cast<float4 *>(yt + i) = make_float4(out[i], out[i + 1u], out[i + 2u], out[i + 3u]);
+        else yt[i] = out[i], yt[i + 1u] = out[i + 1u], yt[i + 2u] = out[i + 2u], yt[i + 3u] = out[i + 3u];
+    }
 }
 
 cudaError_t launch_mix(cudaStream_t st, const float *pairs, const int32_t *ids, const float *weights, uint32_t n_tokens, uint32_t top_k,
                        bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts, bool residual,
                        const BlockEp *ep, uint32_t *status, bool official) {
-    const uintptr_t where = (uintptr_t)pairs | (uintptr_t)y | (residual ? (uintptr_t)x : 0u);
-    return launch_pdl((where & 15u) ? k_block_mix<false> : k_block_mix<true>, dim3((hidden + 1023u) / 1024u, n_tokens), dim3(256), 0, st, 0u, pairs, ids, weights, top_k,
+    const uintptr_t where = (uintptr_t)pairs | (uintptr_t)y | (residual ? (uintptr_t)x : 0u);   // (official: `pairs` is the block's own)
+    const uint32_t per_cta = official ? 1024u : 512u;
+    const auto kernel = (where & 15u) ? (official ? k_block_mix<false, true> : k_block_mix<false, false>)
+                                      : (official ? k_block_mix<true, true> : k_block_mix<true, false>);
+    return launch_pdl(kernel, dim3((hidden + per_cta - 1u) / per_cta, n_tokens), dim3(128), 0, st, 0u, pairs, ids, weights, top_k,
                       has_shared ? 1 : 0, y, hidden, counts, x, residual ? 1u : 0u,
                       (const unsigned long long *)(ep ? ep->flags : nullptr), ep ? ep->rank : 0u, ep ? ep->world : 1u, ep ? ep->call : 0u,
-                      ep ? ep->wait_limit : 0u, status, official ? 1u : 0u);
+                      ep ? ep->wait_limit : 0u, status);
 }
 
 }  // namespace
@@ -426,6 +454,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     down.dig = w.hdig;
     down.exps = w.hexp;
     down.out = pairs_out ? pairs_out : w.d;
+    down.out16 = reinterpret_cast<uint16_t *>(w.d);     // (half of its bytes)
     if (ep) {
         // exchange inside the kernel: the owned pairs' rows into every rank's buffer of the call's parity
         for (uint32_t p = 0; p < ep->world; ++p) {

@@ -20,6 +20,7 @@ struct GemmArgs {
     float *hval;                // up: the pairs' hidden values [pair][inter]
     uint16_t *hval16;           // official: their gates and up projections as BF16 values [pair][2][inter]
     float *out;                 // down: the pairs' expert outputs [pair][hidden]
+    uint16_t *out16;            // official: the same as BF16 values
     uint32_t hidden, inter;
     uint32_t ring, stage;       // stages, bytes of a stage (set by launch_pair_gemm)
     // Expert parallel with the exchange inside the kernel: the pairs' outputs go into every rank's buffer

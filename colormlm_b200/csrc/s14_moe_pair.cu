@@ -491,14 +491,13 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                             const uint32_t t = kOff ? 2u * m + k : 2u * m + wg;
                             if (t < (kOff ? n_tok : nt)) {
                                 const size_t at = (size_t)pair[kOff ? t0 + t : t] * a.hidden + idx * 128u + row;
-                                float o;
-                                if constexpr (kOff) o = __uint_as_float(k ? vb[m] & 0xFFFF0000u : vb[m] << 16);   // (a linear's result is BF16)
-                                else o = v[m];
-                                if (a.ep_world > 1u) {
+                                if constexpr (kOff) {
+                                    a.out16[at] = (uint16_t)(k ? vb[m] >> 16 : vb[m]);   // (a linear's result is BF16)
+                                } else if (a.ep_world > 1u) {
 #pragma unroll 1
-                                    for (uint32_t p = 0; p < a.ep_world; ++p) a.out_peer[p][at] = o;
+                                    for (uint32_t p = 0; p < a.ep_world; ++p) a.out_peer[p][at] = v[m];
                                 } else {
-                                    a.out[at] = o;
+                                    a.out[at] = v[m];
                                 }
                             }
                         }

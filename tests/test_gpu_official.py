@@ -9,7 +9,7 @@ torch = pytest.importorskip("torch")
 
 from colormlm_b200 import _lib as L
 from colormlm_b200 import synth
-from colormlm_b200.s14 import MoeBlock, S14Context, S14Error
+from colormlm_b200.s14 import MoeBlock, S14Context, S14Error, TokenRoute
 
 from .test_gpu_block import random_routes, run_block
 from .test_gpu_parity import dev, dev_page, make_layer
@@ -180,5 +180,35 @@ def test_official_blocks_of_full_chunks(ctx, oracle, n_tokens, n_experts, hidden
             ref = oracle.official_moe_layer(x[t], [pages[i] for i in ids], w, shared, 0, hidden, inter)
             bad = np.nonzero(y[t].view(np.uint32) != ref.view(np.uint32))[0]
             assert bad.size == 0, (t, bad.size, bad[:8], y[t][bad[:4]], ref[bad[:4]])
+    finally:
+        blk.close()
+
+
+# the mix reads BF16 rows out of the buffer that holds F32 rows otherwise: after a call of the other arithmetic, with ragged routes (positions
+# without a route keep what is left there), last CTAs that are half empty, results on a 4-byte boundary and added to the input
+@pytest.mark.parametrize("hidden", [512, 1024, 1536, 4096])
+@pytest.mark.parametrize("n_tokens", [1, 9, 40])
+def test_official_mix_after_the_other_arithmetic(ctx, oracle, n_tokens, hidden):
+    inter, n_experts = 512, 9
+    g, pages, shared = make_layer(2700 + n_tokens, hidden, inter, n_experts, L.PAGE_MXFP4)
+    x = synth.activations(g, n_tokens, hidden)
+    routes = [(ids, w[:len(ids)]) for ids, w in random_routes(g, n_tokens, n_experts, ragged=True)]
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    tr = [TokenRoute(ids, w, [pages_dev[i].data_ptr() for i in ids]) for ids, w in routes]
+    dx = dev(x)
+    odd = torch.full((n_tokens * hidden + 1,), float("nan"), device="cuda")[1:].view(n_tokens, hidden)
+    blk = MoeBlock(ctx, hidden, inter, n_tokens)
+    try:
+        f32 = run_block(ctx, blk, x * np.float32(1e30), pages_dev, shared_dev, routes)   # (large values, infinities as BF16 halves)
+        blk.set_semantics(True)
+        y = run_block(ctx, blk, x, pages_dev, shared_dev, routes)
+        blk.set_residual(True)
+        blk.cmd_moe_block(dx, odd, tr, shared_dev.data_ptr())
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and not np.array_equal(f32, y)
+        for t, (ids, w) in enumerate(routes):
+            ref = oracle.official_moe_layer(x[t], [pages[i] for i in ids], w, shared, 0, hidden, inter)
+            assert np.array_equal(y[t].view(np.uint32), ref.view(np.uint32)), t
+            assert np.array_equal(odd[t].cpu().numpy().view(np.uint32), (x[t] + ref).view(np.uint32)), t
     finally:
         blk.close()
