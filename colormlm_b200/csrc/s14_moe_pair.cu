@@ -9,7 +9,7 @@
 // item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
 // (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
 // epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 507 / 294
-// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, then 577 / 311, now 461 / 258 (see below).  Small blocks, which took one row tile
+// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, then 577 / 311, now 424 / 227 (see below).  Small blocks, which took one row tile
 // and two tokens per SM with stages of 21 KB in a ring of eight and laid out the hidden values' digit rows in the up epilogue:
 // 8 tokens 117 us for the call, now 109.  (Official blocks of two to eight tokens of smaller layers gained nothing: 4 tokens of
 // 2048 x 1536 49 us for the call, now 52.)

@@ -17,20 +17,21 @@
 // and its scale atoms are two plain bulk copies (cp.async.bulk, no multicast) into one ring slot.
 //   up item   (job, slice of 64 intermediate elements): hidden / 256 units accumulate into one
 //             accumulator (lanes 0-63 the gate, 64-127 the up projection); the epilogue applies the
-//             limited SwiGLU, writes the 64 hidden values as digit rows into the job's digit tile in
-//             global memory (L2) and counts the slice on the job's counter.
-//   down item (job, tile of 128 output rows): waits (bounded) until the job's counter says that
-//             every slice is there, takes the job's digit tile into shared memory, and accumulates
+//             limited SwiGLU and writes the 64 hidden values as digit rows into the job's digit tile in
+//             global memory (L2), in words that carry the stamp of launch and layer.
+//   down item (job, tile of 128 output rows): waits (bounded) until every word of the job's digit tile
+//             carries the stamp, takes the tile into shared memory, and accumulates
 //             intermediate / 256 units into one accumulator: the finished rows of the expert's
-//             output.  The last item of a row tile to finish (a counter, no waiting) applies the
-//             ordered mix to that tile.
-// No output passes through partial sums of several CTAs, so the result does not depend on how
-// items are dealt.  Items are dealt to the CTAs (one per SM, all resident) in a fixed pattern that
+//             output.  The CTA that holds the last job's item of a row tile waits for the other jobs' rows and
+//             applies the ordered mix to that tile.
+// An up item may be shared along K by the two CTAs of a cluster (layer_pair_list); both halves' sums are exact enough to be
+// added in double before the one rounding, and nothing else passes through partial sums of several CTAs, so the
+// result does not depend on how items are dealt.  Items are dealt to the CTAs (one per SM, all resident) in a fixed pattern that
 // levels the number of units per CTA; a CTA runs its up items first, then its down items.
 //
 // Roles inside a CTA: one copying thread, two MMA-issuing threads (even and odd units of an item,
 // an accumulator each), four epilogue warps (tcgen05.ld, sums, SwiGLU, digits, mix), eight warps
-// that fetch digit tiles for the down items.  Every wait (mbarrier, counter, peer word) is bounded;
+// that fetch digit tiles for the down items.  Every wait (mbarrier, stamped word, peer word) is bounded;
 // a wait that runs out raises the CTA's abort flag, the status word is set, and the CTA waits for
 // its copies in flight, frees its tensor memory and returns.
 #include "s14_umma.cuh"
