@@ -100,7 +100,7 @@ struct s14_ctx {
         uint32_t wait_limit = 1u << 22;  // polls of about a microsecond: a few seconds
     } ep;
     double *glue = nullptr;   // partial dot products of the hyper-connection calls (hc_scratch_bytes)
-    UmmaScratch umma{nullptr, nullptr, nullptr};  // scratch of the tcgen05 layer kernel
+    UmmaScratch umma{nullptr, nullptr, nullptr, nullptr};  // scratch of the tcgen05 layer kernel
     bool use_umma = true;                // S14_TENSOR_PATH=off in the environment turns it off
     const UmmaScratch *umma_scratch() const { return use_umma ? &umma : nullptr; }
 };
@@ -150,6 +150,9 @@ extern "C" int32_t s14_ctx_create(int32_t device, s14_ctx **out) {
     CUDA_OK(cudaMalloc(&ctx->umma.tiles, umma_scratch_bytes()));
     CUDA_OK(cudaMemset(ctx->umma.tiles, 0, umma_scratch_bytes()));  // no word carries a stamp yet
     ctx->umma.status = ctx->status;
+    static_assert(kNoSum == 0xFFFFFFFFu, "set byte by byte");
+    CUDA_OK(cudaMalloc(&ctx->umma.handed, sizeof(float) * kMaxDim));
+    CUDA_OK(cudaMemset(ctx->umma.handed, 0xFF, sizeof(float) * kMaxDim));
     if (const char *path = getenv("S14_TENSOR_PATH")) ctx->use_umma = strcmp(path, "off") != 0;
     for (auto &e : ctx->marks.ev) CUDA_OK(cudaEventCreate(&e));
     *out = ctx.release();
@@ -180,6 +183,7 @@ extern "C" int32_t s14_ctx_destroy(s14_ctx *ctx) {
     cudaFree(ctx->ids_stage);
     cudaFree(ctx->weights_stage);
     cudaFree(ctx->umma.tiles);
+    cudaFree(ctx->umma.handed);
     cudaFree(ctx->umma.trace);
     s14_ep_exchange_destroy(ctx);
     cudaFreeHost(ctx->y_host);
@@ -2331,10 +2335,10 @@ extern "C" int32_t s14_exec_routed_and_shared_moe_then_hc_post(s14_ctx *ctx, voi
     ld.shared_page = d->shared_page;
     ld.routes = d->route;
     BranchPost post = {d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb, d->state_out_bf16, false};
-    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->y_stage, d->ffn_input_bf16, ctx->x_stage, &post);
+    const int32_t rc = enqueue_layer(ctx, st, ld, ctx->x_stage, ctx->umma.handed, d->ffn_input_bf16, ctx->x_stage, &post);
     if (rc != S14_OK) return rc;
     if (post.done) return S14_OK;
-    CUDA_OK(launch_branch_post(st, d->hidden, ctx->y_stage, d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb,
+    CUDA_OK(launch_branch_post(st, d->hidden, ctx->umma.handed, d->moe_branch_out_bf16, d->residual_bf16, d->post, d->comb,
                                d->state_out_bf16));
     ctx->launches += 1;
     return S14_OK;

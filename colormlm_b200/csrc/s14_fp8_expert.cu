@@ -130,11 +130,11 @@ k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16
     dependency_wait();
 }
 
-// v[n] = routed[n] + w2[n] . h: to y, or (kPost) the branch of the executor's step, rounded to BF16, and hc_post over the
+// v[n] = routed[n] + w2[n] . h (where the layer kernel has left a sum: kNoSum): to y, or (kPost) the branch of the executor's step, rounded to BF16, and hc_post over the
 // post-attention state, lane o the o-th stream (hc.py:127-148; the operations of k_branch_post, whose launch it saves)
 template <uint32_t P, bool kPost>
 __global__ void __launch_bounds__(kF8Threads, 1)
-k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, const float *__restrict__ routed, float *__restrict__ y,
+k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, float *routed, float *__restrict__ y,
                   const __grid_constant__ BranchPost post, uint32_t hidden) {
     constexpr uint32_t inter = P * 512u;
     __shared__ __align__(16) float sx[inter];
@@ -162,8 +162,10 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
             for (uint32_t i = 0; i < 4; ++i) r[i] = __ldcg(static_cast<const uint16_t *>(post.residual) + (size_t)i * hidden + row);
         }
         const float v = __fadd_rn(base, dot_row<P>(qa, pv.s2 + (size_t)(row >> 7) * (inter >> 7), sx, lane));
+        const bool there = __float_as_uint(base) != kNoSum;
+        if (lane == 0u) routed[row] = __uint_as_float(kNoSum);   // (every lane has its copy: dot_row's shuffles lie in between)
         if constexpr (kPost) {
-            if (lane < 4u) {
+            if (there && lane < 4u) {
                 const __nv_bfloat16 b16 = __float2bfloat16_rn(v);
                 if (lane == 0u && post.branch_out) post.branch_out[row] = __bfloat16_as_ushort(b16);
                 float s = __fmul_rn(c[0], __uint_as_float(r[0] << 16));
@@ -173,7 +175,7 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
                     __bfloat16_as_ushort(__float2bfloat16_rn(__fadd_rn(__fmul_rn(p, __bfloat162float(b16)), s)));
             }
         } else {
-            if (lane == 0u) y[row] = v;
+            if (there && lane == 0u) y[row] = v;
         }
         row += step;
 #pragma unroll
@@ -185,7 +187,7 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
 }  // namespace
 
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, const uint8_t *page,
-                              float *h, const float *routed, float *y, const BranchPost *post, uint32_t hidden, uint32_t inter) {
+                              float *h, float *routed, float *y, const BranchPost *post, uint32_t hidden, uint32_t inter) {
     const dim3 grid(sm_count), block(kF8Threads);
     cudaError_t e;
     switch (hidden >> 9) {

@@ -530,9 +530,9 @@ __global__ void __launch_bounds__(256) k_bf16_to_f32(const uint16_t *__restrict_
     if (i < n) out[i] = __uint_as_float((uint32_t)__ldg(in + i) << 16);
 }
 // The end of the executor's expert step: the branch rounded to BF16 (left in branch_out if the caller wants it)
-// and expanded into the four streams as k_hc_post does.  One token.
+// and expanded into the four streams as k_hc_post does.  One token.  y: the layer's sums, or kNoSum where it wrote none.
 __global__ void __launch_bounds__(256)
-k_branch_post(const float *__restrict__ y, uint16_t *__restrict__ branch_out, const void *__restrict__ residual,
+k_branch_post(float *__restrict__ y, uint16_t *__restrict__ branch_out, const void *__restrict__ residual,
               const float *__restrict__ post, const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
     const uint32_t d = blockIdx.x * 256u + threadIdx.x;
     dependency_wait();
@@ -545,7 +545,10 @@ k_branch_post(const float *__restrict__ y, uint16_t *__restrict__ branch_out, co
     }
 #pragma unroll
     for (uint32_t i = 0; i < kHc * kHc; ++i) c[i] = __ldcg(comb + i);
-    const __nv_bfloat16 b16 = __float2bfloat16_rn(__ldcg(y + d));
+    const float v = __ldcg(y + d);
+    y[d] = __uint_as_float(kNoSum);
+    if (__float_as_uint(v) == kNoSum) return;
+    const __nv_bfloat16 b16 = __float2bfloat16_rn(v);
     if (branch_out) branch_out[d] = *reinterpret_cast<const uint16_t *>(&b16);
     const float b = __bfloat162float(b16);
 #pragma unroll
@@ -563,7 +566,7 @@ cudaError_t launch_bf16_to_f32(cudaStream_t st, const uint16_t *in, float *out, 
     k_bf16_to_f32<<<(n + 255u) / 256u, 256, 0, st>>>(in, out, n);
     return cudaGetLastError();
 }
-cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y, uint16_t *branch_out, const void *residual,
+cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, float *y, uint16_t *branch_out, const void *residual,
                                const float *post, const float *comb, void *merged) {
     return launch_pdl(k_branch_post, dim3((hidden + 255u) / 256u), dim3(256), 0, st, 0u, y, branch_out, residual, post, comb, hidden,
                       merged);

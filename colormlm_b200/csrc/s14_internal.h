@@ -141,11 +141,11 @@ int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &route
                             unsigned int *counters, const struct UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err,
                             BranchPost *post = nullptr);
 // One token through one expert of an FP8 page (s14_fp8_expert.cu): x F32, or BF16 as x_bf16; h [inter] scratch; the expert's
-// output added to `routed` [hidden] goes to y, or through `post`.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary,
+// output added to `routed` [hidden] (kNoSum: see there) goes to y, or through `post`.  hidden and inter 1024, 2048 or 4096; x on a 16-byte boundary,
 // x_bf16 (or NULL) on an 8-byte one.
 inline bool fp8_expert_takes(const uint16_t *x_bf16) { return (reinterpret_cast<uintptr_t>(x_bf16) & 7u) == 0u; }
 cudaError_t launch_fp8_expert(cudaStream_t st, int sm_count, const float *x, const uint16_t *x_bf16, const uint8_t *page,
-                              float *h, const float *routed, float *y, const BranchPost *post, uint32_t hidden, uint32_t inter);
+                              float *h, float *routed, float *y, const BranchPost *post, uint32_t hidden, uint32_t inter);
 // Scratch of the tcgen05 layer kernel (s14_moe_umma.cu): per job the digit tile of its hidden
 // values and the tile's block exponents (umma_scratch_bytes), and the device status word a
 // timed-out wait sets.
@@ -153,7 +153,13 @@ struct UmmaScratch {
     uint8_t *tiles;
     uint32_t *status;
     unsigned long long *trace;  // per-CTA time marks of the last launch (profiling runs), or nullptr
+    float *handed;              // [4096]: see kNoSum
 };
+// A layer's sums that a launch behind it goes on with (an FP8 shared expert's, the end of the executor's step) lie in `handed`,
+// which holds this value wherever there is none: a NaN that no addition gives (CUDA's is 0x7fffffff).  The launch that takes a sum
+// puts it back.  So what a layer kernel that gave up did not write is not taken from the call before, and the launch behind
+// writes no result for it either.
+constexpr uint32_t kNoSum = 0xFFFFFFFFu;
 size_t umma_scratch_bytes();
 size_t umma_trace_bytes(int sm_count);
 uint32_t umma_trace_words();
@@ -278,7 +284,7 @@ cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n
 cudaError_t launch_router_hash(cudaStream_t st, const s14_router_desc &r, const int64_t *tid2eid);
 cudaError_t launch_bf16_to_f32(cudaStream_t st, const uint16_t *in, float *out, uint32_t n);
 // branch = BF16 of y (to branch_out, or NULL), merged = post * branch + comb . residual: one token of BF16 streams.
-cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, const float *y, uint16_t *branch_out, const void *residual,
+cudaError_t launch_branch_post(cudaStream_t st, uint32_t hidden, float *y, uint16_t *branch_out, const void *residual,
                                const float *post, const float *comb, void *merged);
 
 }  // namespace s14

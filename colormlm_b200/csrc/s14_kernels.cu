@@ -1290,12 +1290,11 @@ int launch_layer_fp8_shared(cudaStream_t st, int sm_count, const JobTable &route
                             unsigned int *counters, const UmmaScratch *umma, uint32_t hidden, uint32_t inter, cudaError_t *err,
                             BranchPost *post) {
     // The layer kernel first: see s14_fp8_expert.cu.  y may be x: it is written last.
-    float *routed_out = d + (size_t)(S14_EXPERTS_PER_TOKEN + 1) * hidden;  // behind the layer kernel's rows
     const size_t page_bytes = 3u * ((size_t)hidden * inter + (size_t)(hidden >> 7) * (inter >> 7));
-    *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, routed_out, umma->tiles, counters, umma->status, hidden, inter, router,
+    *err = launch_moe_layer_umma(st, sm_count, nullptr, routed, x, d, umma->handed, umma->tiles, counters, umma->status, hidden, inter, router,
                                  nullptr, umma->trace, nullptr, 1, nullptr, false, x_bf16, shared_page, page_bytes);
     if (*err != cudaSuccess) return 0;
-    *err = launch_fp8_expert(st, sm_count, x, x_bf16, shared_page, h, routed_out, y, post, hidden, inter);
+    *err = launch_fp8_expert(st, sm_count, x, x_bf16, shared_page, h, umma->handed, y, post, hidden, inter);
     if (post && *err == cudaSuccess) post->done = true;
     return 3;
 }

@@ -1,5 +1,5 @@
 """Layers with the checkpoint's page kinds - routed MXFP4 experts, FP8 shared expert - on the path that runs the
-shared expert by kernels of its own in front of the tensor-core layer kernel (GPU), against the CPU oracle."""
+shared expert by kernels of its own behind the tensor-core layer kernel (GPU), against the CPU oracle."""
 import numpy as np
 import pytest
 
