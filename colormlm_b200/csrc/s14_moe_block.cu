@@ -279,6 +279,10 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 // kernel the code that every warp fetches once was longer (a block of 45 tokens 148.1 us, so 147.6).
 // The official arithmetic's rows are BF16 values and are stored as such: 115 MB written and read for 1000 tokens, stored as F32, now 57
 // (the call, with its down kernel, 973 us power limited, now 956).  CTAs of 128 threads: 256 took 0.3 us more for a block of 8 tokens.
+// The launch behind may start when the CTAs here exit, not earlier: all of them are resident at once, and while they are, the
+// CTAs of the next block's router scores, which fill the FP64 pipe of an SM, find room on few SMs only, several on one.  Blocks one
+// after another, 4096 x 2048, 64 experts, us: 200 tokens 336, so 319, official 221 and 210; 2048 x 1024, 370 tokens 212 and 203;
+// 8 and 45 tokens the same.
 template <bool vec, bool kOff>
 __global__ void __launch_bounds__(128)
 k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const float *__restrict__ weights,
@@ -287,7 +291,7 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
             uint32_t wait_limit, uint32_t *status) {
     constexpr uint32_t kPer = kOff ? 8u : 4u;
     const uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) * kPer, t = blockIdx.y;   // hidden is a multiple of eight
-    dependency_wait();
+    cudaGridDependencySynchronize();
     const uint32_t why = __ldcg(counts + 3);
     if (flags) {
         // expert parallel, exchange inside the kernels: every rank's rows of this call are in this rank's buffer
