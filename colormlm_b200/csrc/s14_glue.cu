@@ -413,8 +413,8 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
 // token's twenty coefficients are the same for all its threads, so they are read through the L1; F32 values go four to a
 // thread, because the lanes' 16-byte accesses then meet in whole lines (4096, us, before these two and now: 150 tokens
 // F32 7.1 -> 3.3, 1024 28.2 -> 24.5; BF16 16 tokens 2.1 -> 1.7, 1024 10.6 -> 10.2).
-template <bool kBf16, int N, bool vec>
-__global__ void __launch_bounds__(128)
+template <bool kBf16, int N, bool vec, bool kTight = false>
+__global__ void __launch_bounds__(128, kTight ? 8 : 0)
 k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, const float *__restrict__ post,
           const float *__restrict__ comb, uint32_t hidden, void *__restrict__ merged) {
     const uint32_t d = (blockIdx.x * 128u + threadIdx.x) * N, t = blockIdx.y;
@@ -674,16 +674,22 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
 cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged) {
     const uint32_t vec = aligned16(branch, residual, merged);
-    // BF16: four values a thread (8-byte accesses) while their CTAs come to at most five per SM (one token of 4096 1.4 us, eight
-    // values 1.6; 64 tokens 1.9 and 2.0), above that eight (1024 tokens 10.2 us, four values 11.9)
-    const bool few = (uint64_t)n_tokens * hidden <= (uint64_t)sm_count * 5u * 512u;
+    // BF16: four values a thread (8-byte accesses) while their CTAs come to less than four per SM (one token of 4096 1.4 us, eight
+    // values 1.6; 64 tokens 1.9 and 2.0), from there on eight (148 tokens of 2048 2.04 us, four values 2.16; 185 2.22 and 2.44; 1024
+    // of 4096 9.6 and 11.9)
+    const bool few = (uint64_t)n_tokens * hidden < (uint64_t)sm_count * 4u * 512u;
     auto run = [&](auto kernel, uint32_t per_thread) {
         return launch_pdl(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, branch,
                           residual, post, comb, hidden, merged);
     };
     if (!bf16) return vec ? run(k_hc_post<false, 4, true>, 4) : run(k_hc_post<false, 4, false>, 4);
-    if (!vec) return few ? run(k_hc_post<true, 4, false>, 4) : run(k_hc_post<true, 8, false>, 8);
-    return few ? run(k_hc_post<true, 4, true>, 4) : run(k_hc_post<true, 8, true>, 8);
+    if (!vec) return few ? run(k_hc_post<true, 4, false>, 4) : run(k_hc_post<true, 8, false, true>, 8);
+    if (few) return run(k_hc_post<true, 4, true>, 4);
+    // Eight values a thread take 72 registers, seven CTAs to an SM.  In 64 there are eight, so a call of four per SM starts while the
+    // one in front of it runs out (148 tokens of 4096 3.2 us, so 2.45; values one by one 592 tokens of 1024 13.2 and 8.2); more CTAs are
+    // faster with 72 (148 tokens of 7168 3.25 and 3.55, 900 of 4096 8.3 and 8.5).
+    const bool tight = (uint64_t)((hidden + 1023u) / 1024u) * n_tokens <= 4u * (uint64_t)sm_count;
+    return tight ? run(k_hc_post<true, 8, true, true>, 8) : run(k_hc_post<true, 8, true>, 8);
 }
 
 // F32 tokens: eight values per thread while a token has an SM to itself (the fewest steps in series), else four, whose
