@@ -678,9 +678,14 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
     // values 1.6; 64 tokens 1.9 and 2.0), from there on eight (148 tokens of 2048 2.04 us, four values 2.16; 185 2.22 and 2.44; 1024
     // of 4096 9.6 and 11.9)
     const bool few = (uint64_t)n_tokens * hidden < (uint64_t)sm_count * 4u * 512u;
+    // Up to 32 tokens (two groups of k_hc_dots): the SMs divided as that kernel needs them, three CTAs of 26 KB.  Its CTAs, the next
+    // site's, are to start while this kernel runs, and once the two need more than the SMs they have to share some, which an SM divided
+    // otherwise makes them wait for.  Sites one after another, us: 10 tokens of 7168 17.7, so 14.4, 14 of 5120 15.7 and 13.1, 12 of 4096 12.9
+    // and 12.0, 32 of 4096 14.6 and 13.1; from 64 tokens of 5120 on it gains nothing (150 of 4096 18.1 and 18.5).
+    const size_t divided = n_tokens <= 2u * kDotTokens ? 80u << 10 : 0u;
     auto run = [&](auto kernel, uint32_t per_thread) {
-        return launch_pdl(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, branch,
-                          residual, post, comb, hidden, merged);
+        return launch_dependent(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, divided,
+                                branch, residual, post, comb, hidden, merged);
     };
     if (!bf16) return vec ? run(k_hc_post<false, 4, true>, 4) : run(k_hc_post<false, 4, false>, 4);
     if (!vec) return few ? run(k_hc_post<true, 4, false>, 4) : run(k_hc_post<true, 8, false, true>, 8);
