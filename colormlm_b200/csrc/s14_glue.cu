@@ -613,12 +613,12 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
                                       const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
                                       double *partial, void *reduced, float *post, float *comb, float *pre) {
     // Slices of K: as many as make the CTAs fit the SMs side by side, three to an SM by their registers (the head's, with four
-    // rows in place of 24, five, and a sixth that follows soon): one round, no tail.  At most 64, which the second kernel adds up,
-    // and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
+    // rows in place of 24, six of BF16 streams and five of F32 ones, which with six took a second round: 1024 tokens of 7168 54.3 us, so
+    // 48.9, 900 of 512 8.1 and 7.4): one round, no tail.  At most 64, which the second kernel adds up, and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
     // in one warp, and now: 20 tokens of 4096 10.5 and 8.1, 370 23.3 and 20.9, 700 34.1 and 30.9, 1000 45.8 and 40.3; 900 of
     // 1024 20.6 and 16.0.  The head: 460 of 4096 18.7 and 11.5, 1000 30.1 and 23.3, 704 of 512 7.5 and 6.3.
     const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden, sms = (uint32_t)sm_count;
-    const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, (kHead ? 6u : 3u) * sms / groups}));
+    const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, (!kHead ? 3u : kBf16 ? 6u : 5u) * sms / groups}));
     const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
     auto reduce = [&](auto kernel) {
@@ -662,12 +662,14 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
         return of_size(std::false_type{}, std::integral_constant<U, 0>{});
     }
     // The head's four rows leave room for two CTAs, and smaller clusters pack closer: the largest whose CTAs come to at most
-    // one and a half per SM (4096, us: 8 tokens 4.0, 20 4.5, 55 5.5, the two launches 4.7, 5.0, 6.7).  Clusters of two for up to 111
-    // tokens: 80 tokens 8.2, the two launches 6.8 (2048 5.6 and 5.1, 7168 12.0 and 7.6, 256 3.6 and 3.7).
+    // one and a half per SM (4096, us: 8 tokens 4.0, 20 4.5, 55 5.5, the two launches 4.7, 5.0, 6.7).  Clusters of two only of short
+    // rows: up to 1024, or 1792 while their CTAs have an SM each (us, F32 streams, 64 and 111 tokens, the two launches: 512 3.3 and 3.7, 3.8 and
+    // 4.6; 1024 4.0 and 4.4, 4.4 and 4.5; 1536 4.4 and 5.1, 4.9 and 5.0; 2048 5.0 and 5.9, 4.9 and 5.8; 4096, 80 tokens, 8.2 and 6.8).
     const uint32_t room = sms + sms / 2u;
     if (16u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 16>{});
     if (8u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 8>{});
     if (4u * n_tokens <= room) return of_size(std::true_type{}, std::integral_constant<U, 4>{});
+    if (2u * n_tokens <= (hidden <= 1024u ? room : hidden <= 1792u ? sms : 0u)) return of_size(std::true_type{}, std::integral_constant<U, 2>{});
     return of_size(std::true_type{}, std::integral_constant<U, 0>{});
 }
 

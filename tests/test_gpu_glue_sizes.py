@@ -50,9 +50,9 @@ def test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden):
     close_streams(as_f32(host(normed)), as_f32(oracle.rms_norm(host(red), nw, dtype=int(bf16))), bf16)
     m_ref = oracle.hc_post(host(normed), host(x), post.cpu().numpy(), comb.cpu().numpy(), dtype=int(bf16))
     assert np.array_equal(as_f32(host(merged)), as_f32(m_ref))
-    # hc_pre's clusters: sixteen CTAs up to 7 tokens, eight up to 14; sixteen slices of K at 300 x 1024 and 889 x 2048 (the head at
-    # 600 x 1024, 300 x 5120 and 889 x 2048), eight at 300 x 512 and 889 x 512 and where K has no sixteen (768); F32 norms change form at 149, 593 and 889 tokens
-    # the head's reduce: clusters of sixteen CTAs per token (up to 13 tokens), eight (27), four (55), two (111), two launches
+    # hc_pre's clusters: sixteen CTAs up to 7 tokens, then two launches whose slices of K go by the tokens; F32 norms change form at 149,
+    # 593 and 889 tokens; the head's reduce: clusters of sixteen CTAs per token (up to 13 tokens), eight (27), four (55), two
+    # (short rows, up to 111 or 74), two launches
     hfn, hscale, hbase = synth.hc_params(g, hidden, head=True)
     pre = torch.empty((n_tokens, 4), device="cuda")
     ctx.cmd_hc_head_reduce(x, dev(hfn), dev(hscale), dev(hbase), red, pre)
@@ -145,3 +145,13 @@ def test_reduce_of_many_tokens_into_an_unaligned_result(ctx, bf16):
     ctx.cmd_hc_pre(_offset(x, 4), fn, scale, base, moved, post, comb)
     torch.cuda.synchronize()
     assert torch.equal(red, moved)
+
+
+# the head's clusters of two of short rows (on 148 SMs up to 111 tokens of 1024, 74 of 1792) and the two launches behind them; five
+# slices of K to an SM (F32, 592 tokens of 2048); hc_post's division of the SMs (32 tokens), its values a thread (148 of 2048) and its registers
+# (148 of 4096)
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("n_tokens,hidden", [(111, 1024), (112, 1024), (74, 1792), (75, 1792), (74, 2048), (592, 2048), (32, 512), (33, 512),
+                                             (147, 2048), (148, 2048), (148, 4096), (149, 4096)])
+def test_sites_where_forms_change(ctx, oracle, bf16, n_tokens, hidden):
+    test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden)
