@@ -614,11 +614,12 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
                                       double *partial, void *reduced, float *post, float *comb, float *pre) {
     // Slices of K: as many as make the CTAs fit the SMs side by side, three to an SM by their registers (the head's, with four
     // rows in place of 24, six of BF16 streams and five of F32 ones, which with six took a second round: 1024 tokens of 7168 54.3 us, so
-    // 48.9, 900 of 512 8.1 and 7.4): one round, no tail.  At most 64, which the second kernel adds up, and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
+    // 48.9, 900 of 512 8.1 and 7.4; but 300 of 7168, whose warps have five steps then, 13.6 and with five slices 15.3): one round, no tail.  At most 64, which the second kernel adds up, and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
     // in one warp, and now: 20 tokens of 4096 10.5 and 8.1, 370 23.3 and 20.9, 700 34.1 and 30.9, 1000 45.8 and 40.3; 900 of
     // 1024 20.6 and 16.0.  The head: 460 of 4096 18.7 and 11.5, 1000 30.1 and 23.3, 704 of 512 7.5 and 6.3.
     const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden, sms = (uint32_t)sm_count;
-    const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, (!kHead ? 3u : kBf16 ? 6u : 5u) * sms / groups}));
+    const uint32_t per_sm = !kHead ? 3u : kBf16 || (hidden >= 4096u && groups * 6u <= sms) ? 6u : 5u;
+    const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, per_sm * sms / groups}));
     const cudaError_t e = launch_pdl(k_hc_dots<kBf16, kHead>, dim3(groups, slices), dim3(256), 0, st, 0u, x, fn, n, n_tokens, partial);
     if (e != cudaSuccess) return e;
     auto reduce = [&](auto kernel) {
@@ -678,8 +679,9 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
     const uint32_t vec = aligned16(branch, residual, merged);
     // BF16: four values a thread (8-byte accesses) while their CTAs come to less than four per SM (one token of 4096 1.4 us, eight
     // values 1.6; 64 tokens 1.9 and 2.0), from there on eight (148 tokens of 2048 2.04 us, four values 2.16; 185 2.22 and 2.44; 1024
-    // of 4096 9.6 and 11.9)
-    const bool few = (uint64_t)n_tokens * hidden < (uint64_t)sm_count * 4u * 512u;
+    // of 4096 9.6 and 11.9); values one by one up to five per SM (300 tokens of 1024 3.0 us, eight values 5.4)
+    const uint64_t elements = (uint64_t)n_tokens * hidden, per_sm = (uint64_t)sm_count * 512u;
+    const bool few = vec ? elements < 4u * per_sm : elements <= 5u * per_sm;
     // Up to 32 tokens (two groups of k_hc_dots): the SMs divided as that kernel needs them, three CTAs of 26 KB.  Its CTAs, the next
     // site's, are to start while this kernel runs, and once the two need more than the SMs they have to share some, which an SM divided
     // otherwise makes them wait for.  Sites one after another, us: 10 tokens of 7168 17.7, so 14.4, 14 of 5120 15.7 and 13.1, 12 of 4096 12.9
