@@ -43,8 +43,9 @@ __device__ __forceinline__ void stream_st(void *p, size_t i, float v) {
 // N consecutive stream values, back and forth: eight BF16 or four F32 values are one 16-byte access, four BF16 values one of 8
 // bytes, eight F32 values two of 16 (which a warp's lanes make 32 bytes apart); one by one where a caller's buffer is
 // not aligned to 16 bytes (`vec`): all of hc_post and rms_norm, and hc_pre's reduced vector.  Those kernels are compiled once for
-// each: with both forms in one kernel 370 tokens of 4096 took hc_post 7.6 us, now 6.2, and F32 norms 3.7, now 3.0.  The dot products of hc_pre and of the head always read four values of x and of hc_fn at a time; the
-// calls refuse what is not aligned for that.
+// each (with both forms in one kernel 370 tokens of 4096 took hc_post 7.6 us, now 6.2, and F32 norms 3.7, now 3.0), the norm also
+// for either, which some sizes are faster with (launch_rms_norm).  The dot products of hc_pre and of the head always read four
+// values of x and of hc_fn at a time; the calls refuse what is not aligned for that.
 template <bool kBf16, int N>
 __device__ __forceinline__ void stream_ldn(const void *p, size_t i, float (&v)[N], bool vec) {
     static_assert(N == 4 || N == 8, "values per thread");
@@ -446,11 +447,13 @@ k_hc_post(const void *__restrict__ branch, const void *__restrict__ residual, co
 // final_head.py:84-110: out = w * (x * rsqrt(mean(x^2) + eps)); one CTA per token, N values per thread and step, kSteps
 // steps.  kHeld: the token stays in registers and is read once.  The weight is the same for all tokens and comes
 // through the L1.  All tokens read and written at once bound it, so the registers have to leave room for them: kBlocks
-// CTAs per SM (the launch's rule).
-template <bool kBf16, int N, int kSteps, int kBlocks, bool kHeld, bool vec>
+// CTAs per SM (the launch's rule).  kVec: the buffers are aligned to 16 bytes, are not, or either (`aligned` says which).
+constexpr int kUnaligned = 0, kAligned = 1, kEither = 2;
+template <bool kBf16, int N, int kSteps, int kBlocks, bool kHeld, int kVec>
 __global__ void __launch_bounds__(256, kBlocks)
-k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out) {
+k_rms_norm(const void *__restrict__ x, const float *__restrict__ w, uint32_t hidden, float eps, void *__restrict__ out, uint32_t aligned) {
     __shared__ double red[8];
+    const bool vec = kVec == kEither ? aligned != 0u : kVec == kAligned;
     const uint32_t t = blockIdx.x;
     dependency_wait();
     float v[kHeld ? kSteps : 1][N];
@@ -706,10 +709,10 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
 // largest batches would spill and read the token twice.  us of 4096, one form for all / now: 16 tokens 2.7 / 2.6,
 // 300 5.2 / 3.6, 700 7.8 / 4.9, 1024 9.5 / 6.7; 8192 and 1024 tokens 16.4 / 12.0.  BF16 tokens are half the bytes, eight
 // values to a thread always: 4096 and 700 tokens 5.8 / 3.7.
-template <bool kBf16, int kSteps, bool kVec>
+template <bool kBf16, int kSteps, int kVec>
 static cudaError_t launch_rms_steps(cudaStream_t st, uint32_t sms, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,
-                                    void *out) {
-    auto run = [&](auto kernel) { return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out); };
+                                    void *out, uint32_t aligned) {
+    auto run = [&](auto kernel) { return launch_pdl(kernel, dim3(n_tokens), dim3(256), 0, st, 0u, x, w, hidden, eps, out, aligned); };
     if (kBf16 || n_tokens <= sms) return run(k_rms_norm<kBf16, 8, kSteps, 1, true, kVec>);
     if constexpr (!kBf16) {
         constexpr int kFour = 2 * kSteps;   // steps of four values
@@ -723,14 +726,23 @@ static cudaError_t launch_rms_steps(cudaStream_t st, uint32_t sms, uint32_t n_to
 
 cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w,
                             float eps, void *out) {
-    const uint32_t sms = (uint32_t)sm_count;
+    const uint32_t sms = (uint32_t)sm_count, aligned = aligned16(x, w, out);
+    // The form for either kind of buffer, where it is the faster one.  us of it and of the other: aligned, short rows of few tokens (F32
+    // 250 tokens of 1024 1.76 and 1.84, 8 of 2048 1.68 and 1.79; but BF16 592 of 1024 2.35 and 2.25, F32 150 of 2048 2.34 and 2.05, 4096
+    // 2.7 and 2.4); not aligned, many BF16 tokens (592 of 4096 10.4 and 10.9, 1024 of 1024 5.4 and 6.0; but 148 of 2048 2.65 and 2.40),
+    // many F32 ones of short rows (592 of 1024 2.65 and 2.85; but 148 2.26 and 2.22, 592 of 4096 7.5 and 7.1) and few of long ones (148
+    // of 7168 6.5 and 7.0; but 250 7.8 and 7.2).
+    const bool either = aligned ? n_tokens <= (hidden <= 1024u ? 3u * sms : hidden <= 2048u ? sms : 0u)
+                                : n_tokens > sms ? bf16 || hidden <= 1024u : !bf16 && hidden > 4096u;
     auto run = [&](auto steps) {
         constexpr int kS = decltype(steps)::value;
-        if (!aligned16(x, w, out))
-            return bf16 ? launch_rms_steps<true, kS, false>(st, sms, n_tokens, hidden, x, w, eps, out)
-                        : launch_rms_steps<false, kS, false>(st, sms, n_tokens, hidden, x, w, eps, out);
-        return bf16 ? launch_rms_steps<true, kS, true>(st, sms, n_tokens, hidden, x, w, eps, out)
-                    : launch_rms_steps<false, kS, true>(st, sms, n_tokens, hidden, x, w, eps, out);
+        auto form = [&](auto vec) {
+            constexpr int kV = decltype(vec)::value;
+            return bf16 ? launch_rms_steps<true, kS, kV>(st, sms, n_tokens, hidden, x, w, eps, out, aligned)
+                        : launch_rms_steps<false, kS, kV>(st, sms, n_tokens, hidden, x, w, eps, out, aligned);
+        };
+        if (either) return form(std::integral_constant<int, kEither>{});
+        return aligned ? form(std::integral_constant<int, kAligned>{}) : form(std::integral_constant<int, kUnaligned>{});
     };
     if (hidden <= 2048u) return run(std::integral_constant<int, 1>{});
     if (hidden <= 4096u) return run(std::integral_constant<int, 2>{});

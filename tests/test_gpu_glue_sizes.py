@@ -155,3 +155,29 @@ def test_reduce_of_many_tokens_into_an_unaligned_result(ctx, bf16):
                                              (147, 2048), (148, 2048), (148, 4096), (149, 4096)])
 def test_sites_where_forms_change(ctx, oracle, bf16, n_tokens, hidden):
     test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden)
+
+
+# what goes by the number of tokens on other boundaries too: hc_post's values a thread and registers, the norm's forms
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("t,h", [(148, 1024), (149, 1024), (147, 2048), (148, 2048), (149, 4096), (296, 1024), (297, 1024), (444, 1024),
+                                 (445, 1024)])
+def test_many_tokens_on_any_boundary(ctx, bf16, t, h):
+    g = torch.Generator(device="cuda").manual_seed(t + h)
+    dt = torch.bfloat16 if bf16 else torch.float32
+    make = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dt)
+    branch, res, nw = make(t, h), make(t, 4, h), torch.rand(h, device="cuda", generator=g)
+    post, comb = torch.rand(t, 4, device="cuda", generator=g), torch.rand(t, 4, 4, device="cuda", generator=g)
+    want_m, want_n = torch.empty_like(res), torch.empty_like(branch)
+    ctx.cmd_hc_post(branch, res, post, comb, want_m)
+    ctx.cmd_rms_norm(branch, nw, want_n)
+    b, r = branch.float(), res.float()
+    ref = nw * (b * torch.rsqrt(b.double().pow(2).mean(1, keepdim=True) + 1e-6).float())
+    # an F32 sum in another order and three roundings: some 1e-6 of the result; a BF16 value is rounded by 2^-9 of it
+    assert (want_n.float() - ref).abs().max() <= (2.0 ** -8 if bf16 else 2e-6) * ref.abs().max()
+    ref = post[:, :, None] * b[:, None, :] + torch.einsum("tio,tid->tod", comb, r)
+    assert (want_m.float() - ref).abs().max() <= (2.0 ** -8 if bf16 else 2e-6) * ref.abs().max()
+    for offset in (1, 2, 4):
+        got_m, got_n = _offset(torch.zeros_like(want_m), offset), _offset(torch.zeros_like(want_n), offset)
+        ctx.cmd_hc_post(_offset(branch, offset), _offset(res, offset), post, comb, got_m)
+        ctx.cmd_rms_norm(_offset(branch, offset), _offset(nw, offset), got_n)
+        assert torch.equal(got_m, want_m) and torch.equal(got_n, want_n)
