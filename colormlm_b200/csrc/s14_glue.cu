@@ -685,11 +685,12 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
     // of 4096 9.6 and 11.9); values one by one up to five per SM (300 tokens of 1024 3.0 us, eight values 5.4)
     const uint64_t elements = (uint64_t)n_tokens * hidden, per_sm = (uint64_t)sm_count * 512u;
     const bool few = vec ? elements < 4u * per_sm : elements <= 5u * per_sm;
-    // Up to 32 tokens (two groups of k_hc_dots): the SMs divided as that kernel needs them, three CTAs of 26 KB.  Its CTAs, the next
+    // 8 to 32 tokens (two groups of k_hc_dots): the SMs divided as that kernel needs them, three CTAs of 26 KB.  Its CTAs, the next
     // site's, are to start while this kernel runs, and once the two need more than the SMs they have to share some, which an SM divided
     // otherwise makes them wait for.  Sites one after another, us: 10 tokens of 7168 17.7, so 14.4, 14 of 5120 15.7 and 13.1, 12 of 4096 12.9
     // and 12.0, 32 of 4096 14.6 and 13.1; from 64 tokens of 5120 on it gains nothing (150 of 4096 18.1 and 18.5).
-    const size_t divided = n_tokens <= 2u * kDotTokens ? 80u << 10 : 0u;
+    // (Fewer tokens' hc_pre is one launch, and the division itself costs one token 0.1 us.)
+    const size_t divided = n_tokens >= 8u && n_tokens <= 2u * kDotTokens ? 80u << 10 : 0u;
     auto run = [&](auto kernel, uint32_t per_thread) {
         return launch_dependent(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, divided,
                                 branch, residual, post, comb, hidden, merged);
