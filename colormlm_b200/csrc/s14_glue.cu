@@ -638,6 +638,9 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
     return ahead ? reduce(k_hc_reduce<kBf16, kHead, kN, true, true>) : reduce(k_hc_reduce<kBf16, kHead, kN, true, false>);
 }
 
+// hc_pre by a cluster of CTAs per token, for as many tokens as leave a fifth of the SMs (launch_hc_pre has the figures).
+static bool hc_pre_in_clusters(uint32_t n_tokens, uint32_t sms) { return 16u * n_tokens * 5u <= sms * 4u; }
+
 // scratch: hc_scratch_bytes of the most tokens.  Returns the number of kernels launched.
 int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                   const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
@@ -662,7 +665,7 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
         // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together (4096, us: one token 8.2, seven 8.4, the
         // two launches 8.2 and 8.3, on the host one launch more; 7168 9.1 and 9.4, 9.5 and 9.7).  Fourteen clusters of eight took
         // 9.7 for fourteen tokens, the two launches 8.3 (7168 11.3 and 9.7).
-        if (16u * n_tokens * 5u <= sms * 4u) return of_size(std::false_type{}, std::integral_constant<U, 16>{});
+        if (hc_pre_in_clusters(n_tokens, sms)) return of_size(std::false_type{}, std::integral_constant<U, 16>{});
         return of_size(std::false_type{}, std::integral_constant<U, 0>{});
     }
     // The head's four rows leave room for two CTAs, and smaller clusters pack closer: the largest whose CTAs come to at most
@@ -690,7 +693,7 @@ cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_
     // otherwise makes them wait for.  Sites one after another, us: 10 tokens of 7168 17.7, so 14.4, 14 of 5120 15.7 and 13.1, 12 of 4096 12.9
     // and 12.0, 32 of 4096 14.6 and 13.1; from 64 tokens of 5120 on it gains nothing (150 of 4096 18.1 and 18.5).
     // (Fewer tokens' hc_pre is one launch, and the division itself costs one token 0.1 us.)
-    const size_t divided = n_tokens >= 8u && n_tokens <= 2u * kDotTokens ? 80u << 10 : 0u;
+    const size_t divided = !hc_pre_in_clusters(n_tokens, (uint32_t)sm_count) && n_tokens <= 2u * kDotTokens ? 80u << 10 : 0u;
     auto run = [&](auto kernel, uint32_t per_thread) {
         return launch_dependent(kernel, dim3((hidden + 128u * per_thread - 1u) / (128u * per_thread), n_tokens), dim3(128), 0, st, 0u, divided,
                                 branch, residual, post, comb, hidden, merged);
