@@ -252,15 +252,18 @@ __device__ __forceinline__ void st_async_partner(uint32_t addr, double v, uint32
                  : "memory");
 }
 
-// 512 threads = 16 warps, four per sub-partition of the SM: up to 128 registers per thread.
-template <bool kTrace>
+// 512 threads = 16 warps, four per sub-partition of the SM: up to 128 registers per thread.  kPlain: launches without pairs of CTAs
+// and without `ahead`, as what those need lengthens the way of every item (one routed layer of 1024 x 1024 14.2 us, so 13.8, of 4096 x
+// 2048 23.6 and 23.4; five layers of 1024 x 1024 67.8 and 66.3).
+template <bool kTrace, bool kPlain>
 __global__ void __launch_bounds__(kThreads, 1)
 k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__ JobTable param_table,
                  const float *__restrict__ x, float *d_out, float *__restrict__ y, uint8_t *tiles,
                  unsigned int *counters, uint32_t *__restrict__ status, uint32_t hidden, uint32_t inter,
                  uint32_t ring, unsigned long long *trace, const __grid_constant__ FusedRouter rt,
                  const __grid_constant__ EpExchange ep, const StackLayer *__restrict__ stack, uint32_t n_layers,
-                 float *hbuf, uint32_t residual, const uint16_t *x_bf16, const uint8_t *ahead, uint32_t ahead_bytes, uint32_t paired) {
+                 float *hbuf, uint32_t residual, const uint16_t *x_bf16, const uint8_t *ahead, uint32_t ahead_arg, uint32_t paired_arg) {
+    const uint32_t ahead_bytes = kPlain ? 0u : ahead_arg, paired = kPlain ? 0u : paired_arg;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kBars];
     __shared__ __align__(16) uint8_t sE[kExpMax];        // block exponents of the token's digits
@@ -494,9 +497,9 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             if (p_i >= n_it) break;
             const uint32_t item = s_items[p_i], j = (item >> 8) & 0xFFu, idx = item & 0xFFu;
             const bool down = (item & kItemDown) != 0u;
-            const uint32_t nu = down ? KD : (item & kItemHalf) ? KU >> 1 : KU;
+            const uint32_t nu = down ? KD : !kPlain && (item & kItemHalf) ? KU >> 1 : KU;
             const uint8_t *page = (!routes_known && !table_param) ? s_layer[par_l].shared_page : s_jobs[par_l][j].page;
-            const uint32_t from = (item & kItemSecond) ? nu : 0u;
+            const uint32_t from = !kPlain && (item & kItemSecond) ? nu : 0u;
             const uint8_t *a = page + (down ? mxfp4_down_offset(hidden, inter) : 0u) + ((size_t)idx * (down ? KD : KU) + from + p_u) * kUnitStride;
 #pragma unroll 1
             for (; p_u < nu; ++p_u) {
@@ -955,9 +958,9 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     const uint32_t gi = gi0 + i;
                     const uint32_t item = warp_uniform(s_items[i]), j = (item >> 8) & 0xFFu, buf = gi & 1u;
                     const bool down = (item & kItemDown) != 0u;
-                    const uint32_t nu = down ? KD : (item & kItemHalf) ? KU >> 1 : KU;
+                    const uint32_t nu = down ? KD : !kPlain && (item & kItemHalf) ? KU >> 1 : KU;
                     if (gi >= 2u) ok = mbar_wait_warp(bar(kBarAccFree + buf), ((gi - 2u) >> 1) & 1u, abortp);
-                    const uint32_t from = (item & kItemSecond) ? nu : 0u;   // units of K in front of this half
+                    const uint32_t from = !kPlain && (item & kItemSecond) ? nu : 0u;   // units of K in front of this half
                     uint64_t b_desc0 = bx_desc0 + from * (2048u >> 4);
                     uint32_t sfb0 = tm + kColSfbX + from * 8u;
                     bool last_user = false;
@@ -1085,7 +1088,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar(kBarAccFree + buf));
                     if (tid == 0) mark(52u + i);
-                    if (item & kItemHalf) {
+                    if (!kPlain && (item & kItemHalf)) {
                         // An item that the pair shares: the second half's sums go into the first CTA's shared memory, each
                         // store counted on its barrier.  One such item per CTA and layer; the next layer's token depends on
                         // these sums, so they have been read when the partner's next ones arrive.
@@ -1345,7 +1348,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     fence_before();
     __syncwarp();  // the copying and the issuing threads rejoin their warps
     __syncthreads();
-    if (tid == 0 && abort_flag) {
+    if (!kPlain && tid == 0 && abort_flag) {
         // given up: the partner's sums of a shared item may be on their way
         for (uint32_t i = 0; i < s_n_items; ++i) {
             if ((s_items[i] & (kItemHalf | kItemSecond)) != kItemHalf) continue;
@@ -1464,12 +1467,16 @@ size_t dynamic_limit() {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     if (g_dynamic_limit[dev]) return g_dynamic_limit[dev];
-    cudaFuncAttributes fa, fb;
-    if (cudaFuncGetAttributes(&fa, k_moe_layer_umma<false>) != cudaSuccess) return 0;
-    if (cudaFuncGetAttributes(&fb, k_moe_layer_umma<true>) != cudaSuccess) return 0;
-    const size_t most = kMaxSmem - (fa.sharedSizeBytes > fb.sharedSizeBytes ? fa.sharedSizeBytes : fb.sharedSizeBytes);
-    if (cudaFuncSetAttribute(k_moe_layer_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
-    if (cudaFuncSetAttribute(k_moe_layer_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
+    const auto kernels = {k_moe_layer_umma<false, false>, k_moe_layer_umma<false, true>, k_moe_layer_umma<true, false>, k_moe_layer_umma<true, true>};
+    size_t fixed = 0;
+    for (auto *kernel : kernels) {
+        cudaFuncAttributes a;
+        if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess) return 0;
+        fixed = std::max(fixed, a.sharedSizeBytes);
+    }
+    const size_t most = kMaxSmem - fixed;
+    for (auto *kernel : kernels)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) return 0;
     g_dynamic_limit[dev] = most;
     return most;
 }
@@ -1493,7 +1500,7 @@ bool pairs_resident(int sm_count) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (launch_status(cudaOccupancyMaxActiveClusters(&n, k_moe_layer_umma<false>, &cfg)) != cudaSuccess) n = 0;
+        if (launch_status(cudaOccupancyMaxActiveClusters(&n, k_moe_layer_umma<false, false>, &cfg)) != cudaSuccess) n = 0;
         pairs[dev] = n + 1;
     }
     return 2 * (pairs[dev] - 1) >= sm_count;
@@ -1573,13 +1580,12 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     const uint32_t n_early = router && rt.has_shared ? 1u : 0u, n_jobs = given ? param.n_jobs : rt.top_k + n_early;
     const bool paired = hidden >= 4096u && !dev && ex.world <= 1u && rt.ep_world <= 1u && (given || n_layers > 1u) &&
                         layer_pairs_share((uint32_t)sm_count, n_jobs, inter >> 6, hidden >> 8, n_early) && pairs_resident(sm_count);
-    if (trace)
-        return launch_layer(k_moe_layer_umma<true>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
-                          counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                          residual ? 1u : 0u, x_bf16, ahead, (uint32_t)(ahead_bytes & ~(size_t)15u), paired ? 1u : 0u);
-    return launch_layer(k_moe_layer_umma<false>, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles,
-                      counters, status, hidden, inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf,
-                      residual ? 1u : 0u, x_bf16, ahead, (uint32_t)(ahead_bytes & ~(size_t)15u), paired ? 1u : 0u);
+    const bool plain = !paired && ahead_bytes < 16u;
+    const auto kernel = trace ? (plain ? k_moe_layer_umma<true, true> : k_moe_layer_umma<true, false>)
+                              : (plain ? k_moe_layer_umma<false, true> : k_moe_layer_umma<false, false>);
+    return launch_layer(kernel, dim3(sm_count), dim3(kThreads), smem, st, pdl, paired, dev, param, x, d, y, tiles, counters, status, hidden,
+                        inter, ring, trace, rt, ex, stack, stack ? n_layers : 1u, hbuf, residual ? 1u : 0u, x_bf16, ahead,
+                        (uint32_t)(ahead_bytes & ~(size_t)15u), paired ? 1u : 0u);
 }
 
 }  // namespace s14
