@@ -167,8 +167,9 @@ __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_
 // only the latter share, because an early item makes its CTA late (partners half the grid apart, some of them with early items:
 // no gain); so there may be at most as many shared items as such pairs, and half an item has to have an even number of units.
 // Otherwise the lists are those above.  The down items: the CTAs without a half first take what levels the units (of the jobs
-// that are finished first), the rest goes round all CTAs, those first (those last: 342 us).  14 layers of 4096 x 2048 in one
-// launch: 343.5 us, with shared items 331.5.
+// that are finished first), the rest goes round all CTAs, those first (those last: 342 us) unless a down item is longer than half an
+// up item, when they have more than the others by then (4096 x 4096: two given jobs and a shared one 26.6 us, so 23.4; without pairs
+// 25.2).  14 layers of 4096 x 2048 in one launch: 343.5 us, with shared items 331.5.
 //
 // CTA `b` of the grid as the deal numbers it: the first F / 2 pairs hold the F early items, two neighbouring numbers each; the
 // numbers of the other pairs lie half of those CTAs apart.
@@ -203,14 +204,17 @@ __host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_
         const uint32_t q = F + a_full * G + (c_rot - P);
         put(kItemHalf | kItemSecond | ((q / S) << 8) | (q % S));
     }
-    // the CTAs without a half, `plain` numbers them; and every CTA's place when the rest goes round
+    // the CTAs without a half, `plain` numbers them
     const uint32_t n_plain = G - 2u * r, plain = c_rot < P ? c_rot - r : c_rot - 2u * r;
-    const uint32_t pos = second ? n_plain + r + c_rot - P : first ? n_plain + c_rot : plain;
     auto put_down = [&](uint32_t p) { put(kItemDown | ((p / RT) << 8) | (p % RT)); };
     uint32_t ahead = (KU / 2u + KD / 2u) / KD * n_plain;
     const uint32_t ready = RT * (n_early + a_full * G / S);
     if (ahead > ready) ahead = ready;
     if (ahead > D) ahead = D;
+    // every CTA's place when the rest goes round: first those with fewer units by now
+    const bool halves_first = ahead && ahead % n_plain == 0u && ahead / n_plain * KD > KU / 2u;
+    const uint32_t pos = halves_first ? (second ? r + c_rot - P : first ? c_rot : 2u * r + plain)
+                                      : (second ? n_plain + r + c_rot - P : first ? n_plain + c_rot : plain);
     if (!first && !second)
         for (uint32_t p = plain; p < ahead; p += n_plain) put_down(p);
     for (uint32_t p = ahead + pos; p < D; p += G) put_down(p);

@@ -54,6 +54,14 @@ def test_the_benchmark_layer_shares_what_does_not_go_round(cuda_lib):
     assert max(u + sum(8 for it in items if it & DOWN) for u, items in zip(units, lists)) <= 40
 
 
+def test_long_down_items_go_to_the_pairs_that_share(cuda_lib):
+    """Three given jobs of 4096 x 4096 on 148 CTAs: a down item is as long as a whole up item, and after one of them a CTA without
+    a half has 32 units where the others have 24, so the others come first when the rest goes round."""
+    lists = [pair_list(b, 148, 3, 0, 4096, 4096) for b in range(148)]
+    assert any(it & HALF for items in lists for it in items)
+    assert max(sum(8 if it & HALF else 16 for it in items) for items in lists) == 40
+
+
 def test_rejects_bad_arguments(cuda_lib):
     count = C.c_uint32(0)
     for args in ((148, 148, 7, 0, 4096, 2048), (0, 0, 7, 0, 4096, 2048), (0, 147, 7, 0, 4096, 2048), (0, 148, 7, 0, 4000, 2048)):
@@ -88,6 +96,13 @@ def test_layer_with_shared_items(cuda_lib, ctx, oracle, hidden, inter, routed, s
     for _ in range(2):
         y = run_layer(ctx, x, pages_dev, shared_dev, [(list(range(routed)), w)], L.PAGE_MXFP4, hidden, inter)[0]
         assert_pairwise_close(oracle, y, want)
+
+
+# long down items: the rest of them goes round the pairs that share first
+@pytest.mark.gpu
+@pytest.mark.parametrize("routed,shared", [(2, True), (3, False)])
+def test_layer_with_shared_items_and_long_down_items(cuda_lib, ctx, oracle, routed, shared):
+    test_layer_with_shared_items(cuda_lib, ctx, oracle, 4096, 4096, routed, shared)
 
 
 @pytest.mark.gpu
