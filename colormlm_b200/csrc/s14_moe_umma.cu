@@ -168,8 +168,8 @@ __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_
 // no gain); so there may be at most as many shared items as such pairs, and half an item has to have an even number of units.
 // Otherwise the lists are those above.  The down items: the CTAs without a half first take what levels the units (of the jobs
 // that are finished first), the rest goes round all CTAs, those first (those last: 342 us) unless a down item is longer than half an
-// up item, when they have more than the others by then (4096 x 4096: two given jobs and a shared one 26.6 us, so 23.4; without pairs
-// 25.2).  14 layers of 4096 x 2048 in one launch: 343.5 us, with shared items 331.5.
+// up item, when they have more than the others by then, and the others can take the rest (4096 x 4096: two given jobs and a shared one
+// 26.6 us, so 23.4; without pairs 25.2; seven jobs, whose rest is longer, 35.5 and 35.8).  14 layers of 4096 x 2048 in one launch: 343.5 us, with shared items 331.5.
 //
 // CTA `b` of the grid as the deal numbers it: the first F / 2 pairs hold the F early items, two neighbouring numbers each; the
 // numbers of the other pairs lie half of those CTAs apart.
@@ -212,7 +212,7 @@ __host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_
     if (ahead > ready) ahead = ready;
     if (ahead > D) ahead = D;
     // every CTA's place when the rest goes round: first those with fewer units by now
-    const bool halves_first = ahead && ahead % n_plain == 0u && ahead / n_plain * KD > KU / 2u;
+    const bool halves_first = ahead && ahead % n_plain == 0u && ahead / n_plain * KD > KU / 2u && D - ahead <= 2u * r;
     const uint32_t pos = halves_first ? (second ? r + c_rot - P : first ? c_rot : 2u * r + plain)
                                       : (second ? n_plain + r + c_rot - P : first ? n_plain + c_rot : plain);
     if (!first && !second)
