@@ -81,7 +81,9 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
     // front of it would make this a race); so the work runs beside it, and the wait for it comes last
     if (!early) dependency_wait();
     float xs[8];
+    uint32_t place = 0u;   // the form that the pair's digit tile takes
     if (kQuant && slots) {
+        place = __ldcg(slots + v) & 3u;
         // the hidden values of pair v from its gates and up projections (s14_first_real_token/executor.py:712-743): the limited SwiGLU
         // in F32, times the route's weight (not for the shared expert), rounded to BF16
         const uint32_t tok = v / kPairsPerToken, pos = v - tok * kPairsPerToken;
@@ -131,7 +133,7 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
         digits6_of8(xs, g, words, exps + (size_t)v * (K >> 5));
         const uint32_t kb = g >> 2, forms = slots ? 1u : 4u;
         for (uint32_t i = 0; i < forms; ++i) {
-            const uint32_t form = slots ? __ldcg(slots + v) & 3u : i;
+            const uint32_t form = slots ? place : i;
             uint8_t *const chunk = dig + ((size_t)(v * forms + i) * (K >> 8) + (kb >> 3)) * 768u + (g & 3u) * 4u;
 #pragma unroll
             for (uint32_t j = 0; j < 6; ++j)

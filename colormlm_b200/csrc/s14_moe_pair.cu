@@ -240,13 +240,16 @@ __device__ __forceinline__ bool digit_sums_quick(const uint32_t (&r)[M], int fir
 template <uint32_t kRows>
 __device__ __forceinline__ uint32_t half_rows(uint32_t nt) { return (((nt + 1u) >> 1) * kRows + 15u) & ~15u; }
 
-template <bool kDown, bool kOff>
+// kTok: most tokens of a chunk: twelve, in the official arithmetic 4, 16 or 32.  There the kernel is compiled for each: what 32
+// tokens need of code in the epilogue, which every launch fetches anew, and of loads for the items' records lay in the way of small blocks (us,
+// one form and three: 8 tokens of 512 x 512 28.4 and 23.2, of 2048 x 1024, 64 experts, 48.6 and 42.2; one token of 4096 x 2048 47.0 and 40.3).
+template <bool kDown, bool kOff, uint32_t kTok>
 __global__ void __launch_bounds__(kPThreads, 1)
 k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr uint32_t kRows = kOff ? 6u : 16u, kTileB = kRows * 128u;   // a token's digit rows, and the bytes of its tile
-    constexpr uint32_t kTok = kPCols / 2u / kRows * 2u;           // most tokens of a chunk
-    constexpr uint32_t kMine = kOff ? kTok / 4u : kPGroups / 2u;  // tokens of an epilogue thread (official: pairs of them)
+    static_assert(kTok <= kPCols / 2u / kRows * 2u, "the columns of an accumulator");
+    constexpr uint32_t kMine = kOff ? kTok / 4u : kTok / 2u;      // tokens of an epilogue thread (official: pairs of them)
     constexpr uint32_t kPBatch = kOff ? 56u : 96u;                // items decoded at a time (10 KB of static shared memory are left beside the ring)
     __shared__ __align__(8) uint64_t bars[kPBars];
     __shared__ __align__(16) PairItem s_rec[kPBatch];
@@ -445,7 +448,12 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                 // tokens wg, wg + 2, ... of the chunk; official: those of its half, two BF16 values to a register
                 float v[kOff ? 1u : kMine];
                 uint32_t vb[kOff ? kMine : 1u] = {};
-                if constexpr (kOff) {
+                if constexpr (kOff && kTok == 4u) {
+                    uint32_t r[16];   // two tokens' six columns each
+                    tmem_ld16(lane_base + buf * kPCols + wg * half_rows<kRows>(nt), r);
+                    tmem_ld_wait();
+                    if (!digit_sums_quick(r, 0, vb[0]) && n_tok) vb[0] = digit_sums_pair(r, 0);
+                } else if constexpr (kOff) {
                     // eight tokens' six columns each at a time
                     const uint32_t at = lane_base + buf * kPCols + wg * half_rows<kRows>(nt);
 #pragma unroll
@@ -663,8 +671,10 @@ size_t pair_dynamic_limit() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     if (limit[dev]) return limit[dev];
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-    const void *const fns[] = {(const void *)k_block_pair<false, false>, (const void *)k_block_pair<false, true>,
-                               (const void *)k_block_pair<true, false>, (const void *)k_block_pair<true, true>};
+    const void *const fns[] = {(const void *)k_block_pair<false, false, 12>, (const void *)k_block_pair<true, false, 12>,
+                               (const void *)k_block_pair<false, true, 4>,   (const void *)k_block_pair<true, true, 4>,
+                               (const void *)k_block_pair<false, true, 16>,  (const void *)k_block_pair<true, true, 16>,
+                               (const void *)k_block_pair<false, true, 32>,  (const void *)k_block_pair<true, true, 32>};
     size_t fixed = 0;
     cudaFuncAttributes fa;
     for (const void *fn : fns) {
@@ -686,11 +696,13 @@ cudaError_t launch_pair_gemm(cudaStream_t st, int sm_count, bool down, bool offi
     if (args.ring < 2u || half == 0u || 2u * half > kPGroups) return cudaErrorInvalidConfiguration;
     const size_t smem = (size_t)args.ring * args.stage;
     const dim3 grid((uint32_t)sm_count & ~1u), block(kPThreads);
-    if (down)
-        return official ? launch_pdl(k_block_pair<true, true>, grid, block, smem, st, 2u, args, half, status)
-                        : launch_pdl(k_block_pair<true, false>, grid, block, smem, st, 2u, args, half, status);
-    return official ? launch_pdl(k_block_pair<false, true>, grid, block, smem, st, 2u, args, half, status)
-                    : launch_pdl(k_block_pair<false, false>, grid, block, smem, st, 2u, args, half, status);
+    auto run = [&](auto up_kernel, auto down_kernel) {
+        return launch_pdl(down ? down_kernel : up_kernel, grid, block, smem, st, 2u, args, half, status);
+    };
+    if (!official) return run(k_block_pair<false, false, 12>, k_block_pair<true, false, 12>);
+    if (half == 1u) return run(k_block_pair<false, true, 4>, k_block_pair<true, true, 4>);
+    if (half <= 3u) return run(k_block_pair<false, true, 16>, k_block_pair<true, true, 16>);
+    return run(k_block_pair<false, true, 32>, k_block_pair<true, true, 32>);
 }
 
 }  // namespace s14
