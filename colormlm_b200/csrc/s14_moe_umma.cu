@@ -1314,13 +1314,15 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 if (n_early_jobs && l + 1u < L) prefetch_shared(s_layer[par ^ 1u].shared_page);
                 produce(l, false);
                 if (l + 1u < L) produce(l + 1u, true);
-                if (l + 1u == L) {
-                    mark(12);
+                if (l + 1u == L) mark(12);
+                if constexpr (!kPlain) {
                     // the kernel's own copies are under way and what is left is hand-offs: this CTA's share of what the launches
                     // behind will read, into the L2
+                    if (l + 1u == L) {
 #pragma unroll 1
-                    for (uint32_t u = cta * kAheadPiece; u < ahead_bytes; u += grid * kAheadPiece)
-                        l2_prefetch(ahead + u, min(kAheadPiece, ahead_bytes - u));
+                        for (uint32_t u = cta * kAheadPiece; u < ahead_bytes; u += grid * kAheadPiece)
+                            l2_prefetch(ahead + u, min(kAheadPiece, ahead_bytes - u));
+                    }
                 }
             }
             // the other lanes of its warp wait here (a warp barrier, no polling) until it has finished:
