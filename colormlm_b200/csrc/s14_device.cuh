@@ -211,6 +211,26 @@ inline cudaError_t launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem,
     return launch_dependent(kernel, grid, block, smem, st, cluster, 0u, args...);
 }
 
+// The CTAs of a cluster where fits(n) says whether clusters of n can run: the most of 16 and, beyond which a device or the part of it
+// that the process has may refuse them, the portable 8.
+template <class Fits>
+inline uint32_t cluster_that_fits(Fits fits) {
+    return fits(16u) ? 16u : 8u;
+}
+
+// A kernel in clusters of sixteen (beyond the portable eight): allowed once per kernel and device.
+template <class Kernel>
+inline cudaError_t allow_wide_clusters(Kernel kernel, bool (&done)[64]) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+    if (!done[dev]) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        done[dev] = e == cudaSuccess;
+    }
+    return e;
+}
+
 }  // namespace s14
 
 #endif

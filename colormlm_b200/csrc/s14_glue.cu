@@ -587,19 +587,6 @@ static uint32_t aligned16(P... p) {
     return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0u ? 1u : 0u;
 }
 
-// A kernel in clusters of sixteen (beyond the portable eight): allowed once per kernel and device.
-template <class Kernel>
-static cudaError_t allow_wide_clusters(Kernel kernel, bool (&done)[64]) {
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
-    if (!done[dev]) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        done[dev] = e == cudaSuccess;
-    }
-    return e;
-}
-
 template <bool kBf16, bool kHead, uint32_t kCluster>
 static cudaError_t launch_hc_pre_cluster(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                          const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,

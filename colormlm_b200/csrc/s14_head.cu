@@ -409,12 +409,12 @@ k_head_logits(const float *__restrict__ x, const uint16_t *__restrict__ w, float
 // ---- greedy token -------------------------------------------------------------------------------
 //
 // Largest logit, lowest id on ties, -1 if there is a NaN.  One CTA reads 517 KB at the rate one SM takes in
-// (13.9 us for 129 280 logits); a cluster of sixteen shares the reading and hands its candidates over in shared
+// (13.9 us for 129 280 logits); a cluster of sixteen, or eight where sixteen are refused, shares the reading and hands its candidates over in shared
 // memory, so the call still needs no scratch that calls on several streams would share.  A thread keeps its largest logit and
 // that one's id; warps reduce the logit as an ordered integer, then the id of those that have it, in two operations each.
 // Calls one after another, us: eight CTAs and 64-bit candidates through shuffles 3.18 (129 280 logits), 2.04 (8192); with these
 // reductions 2.39, 1.81; and sixteen CTAs 2.04, 1.69 (and 1.49 for 64 logits, where the eight took 1.85).
-constexpr uint32_t kArgmaxCluster = 16, kArgmaxThreads = 512;
+constexpr uint32_t kArgmaxMost = 16, kArgmaxThreads = 512;
 
 struct ArgmaxBest {
     uint32_t key, id;   // the logit as an ordered integer (all ones: a NaN was met), the lowest id that has it
@@ -426,7 +426,7 @@ __device__ __forceinline__ ArgmaxBest warp_best(ArgmaxBest b) {
 
 __global__ void __launch_bounds__(kArgmaxThreads)
 k_greedy_argmax(const float *__restrict__ logits, uint32_t vocab, int64_t *__restrict__ result) {
-    __shared__ uint2 s_warp[kArgmaxThreads / 32], s_cta[kArgmaxCluster];
+    __shared__ uint2 s_warp[kArgmaxThreads / 32], s_cta[kArgmaxMost];
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
     dependency_wait();
@@ -659,17 +659,29 @@ cudaError_t launch_head_logits(cudaStream_t st, int sm_count, const float *x, ui
 }
 
 cudaError_t launch_greedy_argmax(cudaStream_t st, const float *logits, uint32_t vocab, int64_t *result) {
-    // a cluster of sixteen, beyond the portable eight: allowed once per device
+    // asked once per device
     static bool allowed[64] = {};
+    static uint32_t size[64] = {};
     int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
-    if (!allowed[dev]) {
-        e = launch_status(cudaFuncSetAttribute(k_greedy_argmax, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        if (e != cudaSuccess) return e;
-        allowed[dev] = true;
-    }
-    return launch_pdl(k_greedy_argmax, dim3(kArgmaxCluster), dim3(kArgmaxThreads), 0, st, kArgmaxCluster, logits, vocab, result);
+    if (!size[dev])
+        size[dev] = cluster_that_fits([&](uint32_t n) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = n;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(n);
+            cfg.blockDim = dim3(kArgmaxThreads);
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int fit = 0;
+            return launch_status(allow_wide_clusters(k_greedy_argmax, allowed)) == cudaSuccess &&
+                   launch_status(cudaOccupancyMaxActiveClusters(&fit, k_greedy_argmax, &cfg)) == cudaSuccess && fit > 0;
+        });
+    return launch_pdl(k_greedy_argmax, dim3(size[dev]), dim3(kArgmaxThreads), 0, st, size[dev], logits, vocab, result);
 }
 
 cudaError_t launch_head_prep(cudaStream_t st, const uint16_t *state, const float *fn, const float *scale, const float *base,

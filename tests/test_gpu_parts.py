@@ -100,3 +100,17 @@ def test_end_of_the_executors_step_behind_a_layer_that_gave_up(part):
 
     for got, want in zip(run(given(sums, left)), run(sums.clone())):
         assert torch.equal(got[..., left], want[..., left]) and (got[..., ~left] == 7.0).all() and (want[..., ~left] != 7.0).any()
+
+
+def test_greedy_token_of_either_cluster(part):
+    """Clusters of sixteen, and the eight that every device takes where sixteen are refused: the same token."""
+    lib = part("GREEDY")
+    assert [lib.cluster_of(n) for n in (16, 15, 8, 0)] == [16, 8, 8, 8]
+    for vocab in (1, 5, 4095, 129280):
+        logits = torch.randint(-50, 50, (vocab + 1,), device="cuda").float()   # (many ties)
+        for x in (logits[:vocab], logits[1:]):
+            want, got = int((x == x.max()).nonzero()[0]), torch.empty(2, dtype=torch.int64, device="cuda")
+            for k, cluster in enumerate((8, 16)):
+                assert lib.greedy(cluster, ptr(x), vocab, ptr(got[k:])) == 0
+            torch.cuda.synchronize()
+            assert got.tolist() == [want, want]
