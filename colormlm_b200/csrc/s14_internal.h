@@ -177,6 +177,7 @@ __host__ __device__ uint32_t layer_pair_list(uint32_t c, uint32_t G, uint32_t n_
 __host__ __device__ uint32_t pair_cta(uint32_t b, uint32_t G, uint32_t F);
 // whether that deal shares items (otherwise the lists are layer_work_list's)
 __host__ __device__ bool layer_pairs_share(uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t KU, uint32_t n_early);
+uint32_t layer_items_bound(uint32_t G, uint32_t n_jobs, uint32_t S, uint32_t RT, uint32_t KU, uint32_t KD);
 // Both phases and the mix in one launch (y == nullptr: the expert outputs go to d, the caller mixes).
 // With a router the kernel computes the routes itself and the job tables are not read.  x_bf16: the token as BF16 values (x is
 // not read then), on an 8-byte boundary.  ahead: bytes that the launches behind will read, asked into the L2 when the kernel's own

@@ -91,3 +91,25 @@ def test_rejects_bad_arguments(cuda_lib):
     for args in ((148, 148, 7, 0, 4096, 2048), (0, 0, 7, 0, 4096, 2048), (0, 148, 7, 0, 4000, 2048), (0, 148, 7, 0, 4096, 0)):
         with pytest.raises(L.S14Error):
             L.check(L.lib().s14_layer_work_list(*args, None, 0, C.byref(count)))
+
+
+def items_bound(n_ctas, n_jobs, hidden, inter):
+    """layer_items_bound of s14_moe_umma.cu."""
+    up, down, ku, kd = n_jobs * (inter // 64), n_jobs * (hidden // 128), hidden // 256, inter // 256
+    return -(-up // n_ctas) + 1 + max(1, (ku // 2 + kd // 2) // kd) + -(-down // n_ctas)
+
+
+@pytest.mark.parametrize("n_ctas", [148, 132, 64, 24, 23])
+@pytest.mark.parametrize("hidden,inter", [(512, 512), (1024, 4096), (4096, 512), (4096, 1024), (4096, 2048), (4096, 3584), (4096, 4096)])
+def test_no_cta_has_more_items_than_the_bound(cuda_lib, n_ctas, hidden, inter):
+    """What the launch checks instead of making all CTAs' lists; from 23 CTAs on it is no more than a CTA can hold."""
+    for n_jobs in range(1, 8):
+        bound = items_bound(n_ctas, n_jobs, hidden, inter)
+        assert bound <= 32
+        for n_early in (0, 1):
+            for c in range(n_ctas):
+                assert work_list(c, n_ctas, n_jobs, hidden, inter, cap=0, n_early=n_early)[1] <= bound
+                if n_ctas % 2 == 0:
+                    count = C.c_uint32(0)
+                    L.check(L.lib().s14_layer_pair_list(c, n_ctas, n_jobs, n_early, hidden, inter, None, 0, C.byref(count)))
+                    assert count.value <= bound
