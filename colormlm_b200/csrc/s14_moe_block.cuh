@@ -93,14 +93,15 @@ __device__ __noinline__ float swiglu_once(float gate, float up) { return swiglu_
 // settle it.  __expf(-g) is within 2 + 1.173 |g| units of the last place (2^-23 of the value at most), __fdividef within two; with
 // the five roundings of the exact expressions and the four here that is less than 1.1e-6 + 1.45e-7 |g| of the result, so where that much
 // to either side rounds to the same BF16 value, that is the result.  False for the others (one in some hundred), gates below -80,
-// results near the ends of F32's range, zeros and NaNs.
+// results near the ends of F32's range, products that are so before the weight (they lose bits that a large weight brings
+// back), zeros and NaNs.
 __device__ __forceinline__ bool swiglu_quick(float gate, float up, float weight, float &out) {
     const float g = fminf(gate, 10.0f), u = fminf(fmaxf(up, -10.0f), 10.0f), ag = fabsf(g);
-    const float v = __fmul_rn(__fmul_rn(__fdividef(g, __fadd_rn(1.0f, __expf(-g))), u), weight);
+    const float p = __fmul_rn(__fdividef(g, __fadd_rn(1.0f, __expf(-g))), u), v = __fmul_rn(p, weight);
     const float d = __fmaf_rn(ag, 1.45e-7f, 1.1e-6f);
     const uint32_t both = bf16_pair(__fmaf_rn(v, -d, v), __fmaf_rn(v, d, v));
     out = __uint_as_float(both << 16);
-    return ag <= 80.0f && fabsf(v) > 0x1p-110f && fabsf(v) < 0x1p120f && (both >> 16) == (both & 0xFFFFu);
+    return ag <= 80.0f && fabsf(p) > 0x1p-110f && fabsf(v) > 0x1p-110f && fabsf(v) < 0x1p120f && (both >> 16) == (both & 0xFFFFu);
 }
 
 }  // namespace

@@ -23,4 +23,68 @@ extern "C" int greedy(uint32_t cluster, const float *logits, uint32_t vocab, int
     return (int)(e != cudaSuccess ? e : s14::launch_pdl(s14::k_greedy_argmax, dim3(cluster), dim3(s14::kArgmaxThreads), 0, cudaStreamPerThread,
                                                          cluster, logits, vocab, result));
 }
+#elif defined(PART_QUICK)
+#include "s14_moe_pair.cu"
+namespace s14 {
+namespace {
+// counts[0]: pairs the fast form settles, counts[1]: of them those that differ from the exact one
+__global__ void k_swiglu(const float *ups, uint32_t n_ups, const float *weights, uint32_t n_weights, unsigned long long *counts) {
+    const float gate = __uint_as_float((blockIdx.x * 256u + threadIdx.x) << 16);   // every BF16 value
+    unsigned long long sure = 0, wrong = 0;
+    for (uint32_t i = 0; i < n_ups; ++i) {
+        const float exact = swiglu_limit_f32(gate, ups[i]), pair = swiglu_pair(gate, ups[i]);
+        wrong += __float_as_uint(exact) != __float_as_uint(pair) && !(exact != exact && pair != pair);
+        for (uint32_t j = 0; j < n_weights; ++j) {
+            float quick;
+            if (!swiglu_quick(gate, ups[i], weights[j], quick)) continue;
+            ++sure;
+            wrong += __float_as_uint(quick) != __float_as_uint(bf16_round(__fmul_rn(exact, weights[j])));
+        }
+    }
+    atomicAdd(counts, sure);
+    atomicAdd(counts + 1, wrong);
+}
+__device__ uint32_t next(uint32_t &s) {
+    s = s * 1664525u + 1013904223u;
+    return (s >> 16 ^ s) * 2654435769u;
+}
+// Two tokens' six shares: random ones whose size grows by eight, some without the larger ones, many made so that the sum lies at a BF16 tie
+// or next to one.
+__global__ void k_sums(uint32_t rounds, unsigned long long *counts) {
+    uint32_t state = blockIdx.x * 256u + threadIdx.x + 12345u;
+    unsigned long long sure = 0, wrong = 0;
+    for (uint32_t n = 0; n < rounds; ++n) {
+        uint32_t r[16] = {};
+        for (uint32_t t = 0; t < 2; ++t) {
+            const uint32_t kind = next(state), top = kind & 3u ? 6u : 1u + (kind >> 2) % 6u;
+            double sum = 0.0;
+            for (uint32_t j = 0; j < top; ++j) {
+                const float v = ((int)(next(state) >> 8) - (1 << 23)) * exp2f((float)(3 * (int)j - 40));
+                r[6u * t + j] = __float_as_uint(v);
+                sum += v;
+            }
+            if (kind & 16u) {   // the first share moves the sum to the nearest tie, or a few steps off
+                const float b = __uint_as_float((__float_as_uint((float)sum) & 0xFFFF0000u) | 0x8000u);
+                const int steps = (int)(next(state) % 17u) - 8;
+                r[6u * t] = __float_as_uint((float)((double)b - (sum - (double)__uint_as_float(r[6u * t])) + steps * fabs((double)b) * 0x1p-24));
+            }
+        }
+        uint32_t quick;
+        if (!digit_sums_quick(r, 0, quick)) continue;
+        ++sure;
+        wrong += quick != digit_sums_pair(r, 0);
+    }
+    atomicAdd(counts, sure);
+    atomicAdd(counts + 1, wrong);
+}
+}  // namespace
+}  // namespace s14
+extern "C" int swiglu(const float *ups, uint32_t n_ups, const float *weights, uint32_t n_weights, unsigned long long *counts) {
+    s14::k_swiglu<<<256, 256, 0, cudaStreamPerThread>>>(ups, n_ups, weights, n_weights, counts);
+    return (int)cudaGetLastError();
+}
+extern "C" int sums(uint32_t rounds, unsigned long long *counts) {
+    s14::k_sums<<<1024, 256, 0, cudaStreamPerThread>>>(rounds, counts);
+    return (int)cudaGetLastError();
+}
 #endif

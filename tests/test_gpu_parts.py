@@ -114,3 +114,20 @@ def test_greedy_token_of_either_cluster(part):
                 assert lib.greedy(cluster, ptr(x), vocab, ptr(got[k:])) == 0
             torch.cuda.synchronize()
             assert got.tolist() == [want, want]
+
+
+def test_what_the_fast_forms_settle_is_exact(part):
+    """The official blocks' SwiGLU over every BF16 gate, and their sums of six digit shares, many of them at BF16 ties: where the fast
+    form says that it settles the value, it is the exact form's."""
+    lib = part("QUICK")
+    g = torch.Generator().manual_seed(1)
+    ups = torch.cat([torch.tensor([0.0, -0.0, 1.0, 9.9375, 10.0, 10.0625, -10.0, -12.0, 2.0 ** -120, -2.0 ** -60, 3e38]),
+                     torch.randn(40, generator=g) * 4.0]).to(torch.bfloat16).float().cuda()
+    weights = torch.cat([torch.tensor([1.0, 0.0, 1.5, 2.0 ** -100, 1e30]), torch.rand(11, generator=g)]).cuda()
+    counts = torch.zeros(4, dtype=torch.int64, device="cuda")
+    assert lib.swiglu(ptr(ups), len(ups), ptr(weights), len(weights), ptr(counts)) == 0
+    assert lib.sums(64, ptr(counts[2:])) == 0
+    torch.cuda.synchronize()
+    swiglu, swiglu_wrong, sums, sums_wrong = counts.tolist()
+    assert swiglu_wrong == 0 and sums_wrong == 0
+    assert swiglu > 0.2 * 65536 * len(ups) * len(weights) and sums > 0.3 * 64 * 1024 * 256
