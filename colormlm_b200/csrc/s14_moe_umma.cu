@@ -948,7 +948,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                 routes_known = true;
             }
             const uint32_t n_jobs = routes_ok ? s_n_jobs : 0u, n_items = routes_ok ? s_n_items : 0u;
-            if (kTrace && tid == 0 && tr) tr[15] = n_items | (ring << 8) | (n_jobs << 16);
+            if (kTrace && tid == 0 && tr) tr[15] = n_items | (ring << 8) | (n_jobs << 16) | (paired << 24);
 
             if (is_issuer) {
                 // ---- MMA issue, by two warps (one lane of each): warp m takes units m, m + 2, ... of every

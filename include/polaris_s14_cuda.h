@@ -145,7 +145,7 @@ S14_API int32_t s14_ctx_kernel_times(s14_ctx *ctx, double ms_out[4], uint64_t *c
  * shared memory, 19+4i tile ready (down items); 12 all copies issued, 13 items done, 14 exit;
  * 85/86 (warp 0) and 87/88 (warp 15): the NEXT layer's token: first word seen, all words taken; 89
  * every warp has its words;
- * word 15 = items | ring slots << 8 | jobs << 16.  A word that was not written is 0.  read copies
+ * word 15 = items | ring slots << 8 | jobs << 16 | 1 << 24 if the CTAs ran in pairs.  A word that was not written is 0.  read copies
  * the marks of the last launch ([n_ctas][words_per_cta]). */
 S14_API int32_t s14_ctx_set_layer_trace(s14_ctx *ctx, int32_t enable);
 S14_API int32_t s14_ctx_read_layer_trace(s14_ctx *ctx, uint64_t *out, uint32_t cap_words, uint32_t *n_ctas,

@@ -141,3 +141,41 @@ def test_stack_with_shared_items_and_early_ones(cuda_lib, ctx, oracle):
             assert_chain_close(oracle, h.cpu().numpy(), want_h, "final token")
     finally:
         stack.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("call,hidden,inter,routed,paired", [("layer", 4096, 1024, 2, True), ("layer", 4096, 4096, 2, True), ("layer", 4096, 2048, 6, False),
+                                                             ("layer", 2048, 2048, 6, False), ("routed", 4096, 2048, 6, False),
+                                                             ("stack", 4096, 2048, 6, True), ("stack", 2048, 2048, 6, False)])
+def test_which_launches_run_in_pairs(cuda_lib, ctx, call, hidden, inter, routed, paired):
+    """By the mark of a traced launch (on 148 SMs): without it the tests above would pass on the kernel without pairs."""
+    torch = pytest.importorskip("torch")
+    from colormlm_b200.s14 import DecodeStack
+
+    from .test_gpu_parity import dev, dev_page, make_layer, run_layer
+
+    if ctx.sm_count != 148:
+        pytest.skip("the deals are those of 148 SMs")
+    g, pages, shared = make_layer(55, hidden, inter, 7, L.PAGE_MXFP4)
+    x, w = synth.activations(g, 1, hidden), np.full(routed, 0.25, np.float32)
+    pd, sd = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    wr, table = dev(synth.router_weight_bf16(g, 7, hidden).view(np.int16)), torch.tensor([p.data_ptr() for p in pd], dtype=torch.int64, device="cuda")
+    ctx.set_layer_trace(True)
+    try:
+        if call == "layer":
+            run_layer(ctx, x, pd, sd, [(list(range(routed)), w)], L.PAGE_MXFP4, hidden, inter)
+        elif call == "routed":
+            ctx.cmd_routed_moe_layer(dev(x)[0], wr, None, table, sd.data_ptr(), L.PAGE_MXFP4, inter, torch.empty(1, hidden, device="cuda"))
+        else:
+            layer = {"wr": wr, "bias": None, "shared": sd.data_ptr(), "table": table, "ids": None, "weights": None, "y": None}
+            stack = DecodeStack(ctx, [layer, layer], inter=inter, residual=True)
+            h = dev(x)[0]
+            stack.cmd_decode(h * 0.25, h)
+            torch.cuda.synchronize()
+            stack.close()
+        torch.cuda.synchronize()
+        mark = ctx.read_layer_trace()[:, 15]
+    finally:
+        ctx.set_layer_trace(False)
+    assert ctx.device_status() == 0 and len(mark) == 148
+    assert set(int(m) >> 24 for m in mark if m) == {int(paired)} and (mark != 0).sum() > 100
