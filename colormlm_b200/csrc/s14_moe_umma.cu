@@ -293,7 +293,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
     __shared__ unsigned long long s_page[S14_N_ROUTED_EXPERTS];  // the layer's page table, parked a layer ahead
     __shared__ float s_bias[S14_N_ROUTED_EXPERTS];       // the layer's bias, likewise
     __shared__ StackLayer s_layer[2];                    // the layer's own pointers, by layer parity
-    __shared__ uint32_t s_prod[8];                       // the copying thread's position between its steps
+    __shared__ uint32_t s_prod[8];                       // the copying thread's position between its steps; [7]: layers whose router rows it has asked for
     __shared__ uint32_t s_ep_step, s_stamp0;
     __shared__ uint32_t s_pick_id[8];                    // the picked experts by rank, their scores and pages
     __shared__ float s_pick_score[8];
@@ -498,6 +498,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
                         const uint16_t *wrn = s_layer[par_l ^ 1u].router_weight;
                         const uint32_t rows = (cta < rt.n_experts ? 1u : 0u) + (cta + grid < rt.n_experts ? 1u : 0u);
                         mbar_arrive_expect(bar(kBarWr), rows * hidden * 2u);
+                        s_prod[7] = ll + 2u;
 #pragma unroll 1
                         for (uint32_t k = 0; k < rows; ++k)
                             bulk_copy(smem_u32(sWr) + k * hidden * 2u, wrn + (size_t)(cta + k * grid) * hidden, hidden * 2u, bar(kBarWr));
@@ -565,6 +566,7 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             const uint16_t *wr0 = s_layer[0].router_weight;
             const uint32_t rows = (cta < rt.n_experts ? 1u : 0u) + (cta + grid < rt.n_experts ? 1u : 0u);
             mbar_arrive_expect(bar(kBarWr), rows * hidden * 2u);
+            s_prod[7] = 1u;
 #pragma unroll 1
             for (uint32_t k = 0; k < rows; ++k)
                 bulk_copy(smem_u32(sWr) + k * hidden * 2u, wr0 + (size_t)(cta + k * grid) * hidden, hidden * 2u, bar(kBarWr));
@@ -1356,6 +1358,8 @@ k_moe_layer_umma(const JobTable *__restrict__ dev_table, const __grid_constant__
             const uint32_t s = u % ring, parity = (u / ring) & 1u;
             mbar_drain(bar(kBarFull + s), parity);
         }
+        // ... and the router rows asked for last, which nobody waits for when a role has given up
+        if (s_prod[7]) mbar_drain(bar(kBarWr), (s_prod[7] - 1u) & 1u);
     }
     fence_before();
     __syncwarp();  // the copying and the issuing threads rejoin their warps
