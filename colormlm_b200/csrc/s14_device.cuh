@@ -169,12 +169,18 @@ inline cudaError_t launch_status(cudaError_t e) {
 }
 
 // A launch as a programmatic dependent of what precedes it in the stream, optionally in clusters of
-// `cluster` CTAs (0: none).  The kernels launched so read nothing in front of dependency_wait(), weights and pages
+// `cluster` CTAs (0: none).  But for those below the kernels launched so read nothing in front of dependency_wait(), weights and pages
 // included: a caller's kernel may write those too, and one that lets its own dependents start early is not even
 // complete when such a launch starts.  Behind it they use coherent loads that the compiler keeps in place (__ldcg,
 // ld_stream, ld_u8, ld_f32).  A non-coherent load (__ldg, or a plain one through a const __restrict__ pointer)
-// could return what the operand held before.  One kernel reads and writes in front of its wait: the first digits launch of a
-// block call (k_block_digits, early), behind k_router_select_batch, which triggers behind its own wait, or behind a copy.
+// could return what the operand held before.
+//
+// Three kernels read in front of their wait what the launch directly in front of them does not write, and may only follow a launch that
+// triggers behind its own wait, because then everything in front of that one is complete when they start: the first digits launch of a
+// block call (k_block_digits, early: reads x, writes digits), behind k_router_select_batch or a copy; k_hc_reduce with kAhead (the streams),
+// behind k_hc_dots; k_fp8_expert_up (the token and its page; writes h), behind the layer kernel with a page `ahead`.  The layer kernel
+// without one copies pages, router rows and tables, which are constant during a step, in front of its wait.  k_hc_reduce, k_router and
+// the layer kernel without a page ahead trigger in front of their own wait: none of the three may follow one of these directly.
 //
 // `shared`: bytes of shared memory an SM needs for this kernel, 1 KB per CTA included (0: not said).  A dependent launch takes
 // over SMs from a kernel that is still running elsewhere, and without a word the SMs stay divided as that kernel has them:

@@ -9,7 +9,7 @@
 // launch needs nothing of that kernel, so it runs on the SMs that kernel has left.  The vector lies in shared memory as [quarter
 // of a piece][piece]: the lanes of a warp, which hold consecutive pieces, read consecutive 16 bytes.  Sums as in the FP8
 // register kernels: F32 inside a piece, double across pieces and lanes, one rounding.  Measured at 4096 x 2048, other pages every
-// time: the executor's step, which is the layer kernel's six experts and these two launches, takes 33.3 us.  With both launches and
+// time: the executor's step, which is the layer kernel's six experts and these two launches, takes 32.6 us.  With both launches and
 // their own stream from memory in front of the layer kernel and a launch for branch and expand behind it: 39.9; behind it but
 // waiting for it: 35.5; on the register kernels, which ran all seven experts, 77.2.
 #include "s14_device.cuh"
@@ -130,8 +130,9 @@ k_fp8_expert_up(const float *__restrict__ x, const uint16_t *__restrict__ x_bf16
     dependency_wait();
 }
 
-// v[n] = routed[n] + w2[n] . h (where the layer kernel has left a sum: kNoSum): to y, or (kPost) the branch of the executor's step, rounded to BF16, and hc_post over the
-// post-attention state, lane o the o-th stream (hc.py:127-148; the operations of k_branch_post, whose launch it saves)
+// v[n] = routed[n] + w2[n] . h (where the layer kernel has left a sum: kNoSum): to y, or (kPost) the branch of the executor's step,
+// rounded to BF16, and hc_post over the post-attention state, lane o the o-th stream (hc.py:127-148; the operations of
+// k_branch_post, whose launch it saves)
 template <uint32_t P, bool kPost>
 __global__ void __launch_bounds__(kF8Threads, 1)
 k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h, float *routed, float *__restrict__ y,
@@ -143,8 +144,8 @@ k_fp8_expert_down(const uint8_t *__restrict__ page, const float *__restrict__ h,
     uint32_t row = warp * gridDim.x + blockIdx.x;
     uint4 qa[P], qb[P];  // this row and the warp's next one
     // what a row's result is made of beside the dot product: its sum and the streams.  Asked for in front of the row's weights, as
-    // behind them it comes microseconds later (the store below keeps the compiler from moving it: the step of 1024 x 2048 then took
-    // 22.0 us instead of 19.5)
+    // behind them it comes microseconds later (the store of kNoSum keeps the compiler from moving it: the step of 1024 x 2048 then took
+    // 22.0 us instead of 19.4)
     struct Row {
         float base;
         uint32_t r[4];

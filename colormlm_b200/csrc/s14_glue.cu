@@ -165,7 +165,9 @@ __device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_
 // only) of few tokens: one cluster of sixteen CTAs per token (the head fewer for more tokens: launch_hc_pre).  The call is all
 // latency: 1.5 MB of fn per token, then a serial chain of 20 Sinkhorn rounds.  Every CTA takes its share of the
 // flattened streams against all rows of fn (98 KB, all loads in flight together), the partial sums cross in
-// shared memory, every CTA makes the coefficients itself and reduces its share of the hidden vector: no scratch, no second launch, no vote.  One token of 4096: 10.9 us in two launches before, 6 us now.
+// shared memory, every CTA makes the coefficients itself and reduces its share of the hidden vector: no scratch, no second
+// launch, no vote.  One token of 4096, calls one after another: 10.9 us in the two launches of then, 8.2 now (as the two launches of
+// today: launch_hc_pre).
 constexpr uint32_t kPreThreads = 512;
 template <bool kBf16, bool kHead, uint32_t kCluster>
 __global__ void __launch_bounds__(kPreThreads)
@@ -602,11 +604,13 @@ template <bool kBf16, bool kHead>
 static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                       const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
                                       double *partial, void *reduced, float *post, float *comb, float *pre) {
-    // Slices of K: as many as make the CTAs fit the SMs side by side, three to an SM by their registers (the head's, with four
-    // rows in place of 24, six of BF16 streams and five of F32 ones, which with six took a second round: 1024 tokens of 7168 54.3 us, so
-    // 48.9, 900 of 512 8.1 and 7.4; but 300 of 7168, whose warps have five steps then, 13.6 and with five slices 15.3): one round, no tail.  At most 64, which the second kernel adds up, and a step of sixteen k for every warp.  us of both launches with eight or sixteen slices and a second kernel that added them
-    // in one warp, and now: 20 tokens of 4096 10.5 and 8.1, 370 23.3 and 20.9, 700 34.1 and 30.9, 1000 45.8 and 40.3; 900 of
-    // 1024 20.6 and 16.0.  The head: 460 of 4096 18.7 and 11.5, 1000 30.1 and 23.3, 704 of 512 7.5 and 6.3.
+    // Slices of K: as many as make the CTAs fit the SMs side by side, three to an SM by their registers (the head's, with four rows
+    // in place of 24, six of BF16 streams and five of F32 ones, which with six took a second round: 1024 tokens of 7168 54.3 us, so
+    // 48.9, 900 of 512 8.1 and 7.4; but 300 of 7168, whose warps have five steps then, 13.6 and with five slices 15.3): one round,
+    // no tail.  At most 64, which the second kernel adds up, and a step of sixteen k for every warp.  us of both launches with
+    // eight or sixteen slices and a second kernel that added them in one warp, and now: 20 tokens of 4096 10.5 and 8.1, 370 23.3
+    // and 20.9, 700 34.1 and 30.9, 1000 45.8 and 40.3; 900 of 1024 20.6 and 16.0.  The head: 460 of 4096 18.7 and 11.5, 1000 30.1
+    // and 23.3, 704 of 512 7.5 and 6.3.
     const uint32_t groups = (n_tokens + kDotTokens - 1u) / kDotTokens, n = kHc * hidden, sms = (uint32_t)sm_count;
     const uint32_t per_sm = !kHead ? 3u : kBf16 || (hidden >= 4096u && groups * 6u <= sms) ? 6u : 5u;
     const uint32_t slices = std::max(1u, std::min({kHcSlices, hidden / 32u, per_sm * sms / groups}));

@@ -232,8 +232,9 @@ struct BlockWork {
     uint8_t *xdig, *xexp;      // the tokens' digit tiles and block exponents
     uint8_t *slots;            // official arithmetic: which of the four forms of a digit tile each pair's place in its chunk takes
     uint8_t *hdig, *hexp;      // the pairs' hidden values likewise
-    float *d;                  // the pairs' expert outputs [pair, hidden]
-    float *hval;               // the pairs' hidden values [pair, inter] (official arithmetic: BF16 values, times the route weight)
+    float *d;                  // the pairs' expert outputs [pair, hidden]; official arithmetic: BF16 values, in the first half
+    float *hval;               // the pairs' hidden values [pair, inter]; official arithmetic: their gates and up projections [pair, 2, inter]
+                               // as BF16 values.  (What a pair without a route has there may be the other kind's bits.)
 };
 // Expert-parallel exchange of the block kernels over peer memory: every rank holds two pair buffers
 // [pairs, hidden] F32 (calls alternate between them) and, per buffer, one 8-byte word per rank: the number

@@ -473,8 +473,8 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
         down.ep_call = ep->call;
     }
     // The up kernel leaves the pairs' hidden values, and a second digits launch (which also quantises them per 128
-    // elements for the official arithmetic) lays out the rows of all pairs' slots (a slot without a route holds
-    // zeros or an earlier call's values: finite numbers nobody reads the rows of).
+    // elements for the official arithmetic) lays out the rows of all pairs' slots (a slot without a route holds what an
+    // earlier call left, perhaps in the other arithmetic, so any bits: its rows are copied into no chunk, and the mix skips it).
     *err = launch_pair_gemm(st, sm_count, false, official, up, groups / 2u, status);
     digits(w.hval, n_tokens * kPairsPerToken, inter, w.hdig, w.hexp, false);
     if (*err == cudaSuccess) *err = launch_pair_gemm(st, sm_count, true, official, down, groups / 2u, status);

@@ -15,7 +15,8 @@ struct GemmArgs {
     const BlockChunk *chunks;
     const uint32_t *n_chunks;   // device memory: written by the grouping kernel
     uint32_t *why;              // the call's counts[3]: kBlockGaveUp is added by a CTA that gives up
-    const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048]; official arithmetic: 768, the tokens' in four forms [token][4][K / 256][768]
+    const uint8_t *dig;         // digit tiles of the B vectors [vector][K / 256][2048]; official arithmetic: 768, the tokens'
+                                // in four forms [token][4][K / 256][768]
     const uint8_t *exps;        // their block exponents + 100, [vector][K / 32]
     float *hval;                // up: the pairs' hidden values [pair][inter]
     uint16_t *hval16;           // official: their gates and up projections as BF16 values [pair][2][inter]
@@ -45,13 +46,13 @@ __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) | (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16;
 }
 
-// The limited SwiGLU (swiglu_limit_f32: the same bits) in F32 operations, as FP64 ones are scarce here (see above).  The
+// The limited SwiGLU (swiglu_limit_f32: the same bits) in F32 operations: the F32 blocks' up epilogue, where FP64 ones run at a quarter of
+// their rate beside the MMAs, and what swiglu_quick does not settle.  The
 // exponential by Ziv's method: e^t = 2^n e^r with r = t - n ln 2 in two floats (Cody and Waite's reduction, ln 2 in three
 // parts of which n times the first is exact), e^r by its Taylor series to r^11 / 11!, the terms from r^6 on in F32 and the
 // others in pairs of floats; the pair is within 2^-41 of e^t (4e7 arguments against an 80-bit exponential), so where the
 // bounds 2^-38 to either side round to the same float, that is e^t correctly rounded.  The others, one in 10^4, and gates
-// whose e^-g is beyond 2^57 take the FP64 path.  1000 tokens of the official arithmetic: 1160 us with FP64, now
-// 1124 (power limited 1245 and 1187).
+// whose e^-g is beyond 2^57 take the FP64 path.  (1000 official tokens, when their epilogue had it: 1160 us with FP64, 1124 so.)
 __device__ __noinline__ float swiglu_f64(float gate, float up) { return swiglu_limit_f32(gate, up); }
 __device__ __forceinline__ float swiglu_pair(float gate, float up) {
     const float g = fminf(gate, 10.0f), u = fminf(fmaxf(up, -10.0f), 10.0f), t = -g;

@@ -169,7 +169,8 @@ __host__ __device__ uint32_t layer_work_list(uint32_t c, uint32_t G, uint32_t n_
 // Otherwise the lists are those above.  The down items: the CTAs without a half first take what levels the units (of the jobs
 // that are finished first), the rest goes round all CTAs, those first (those last: 342 us) unless a down item is longer than half an
 // up item, when they have more than the others by then, and the others can take the rest (4096 x 4096: two given jobs and a shared one
-// 26.6 us, so 23.4; without pairs 25.2; seven jobs, whose rest is longer, 35.5 and 35.8).  14 layers of 4096 x 2048 in one launch: 343.5 us, with shared items 331.5.
+// 26.6 us, so 23.4; without pairs 25.2; seven jobs, whose rest is longer, 35.5 and 35.8).  14 layers of 4096 x 2048 in one launch:
+// 343.5 us, with shared items 331.5.
 //
 // CTA `b` of the grid as the deal numbers it: the first F / 2 pairs hold the F early items, two neighbouring numbers each; the
 // numbers of the other pairs lie half of those CTAs apart.
@@ -240,15 +241,15 @@ __device__ __noinline__ uint32_t pair_list_once(uint32_t c, uint32_t G, uint32_t
     const uint32_t n = layer_pair_list(c, G, n_jobs, S, RT, KU, KD, items, kMaxItems, n_early);
     return n < kMaxItems ? n : kMaxItems;
 }
-// Nothing on the kernel's paths may live in local memory: nearly all of the SM's L1 is carved out as
-// shared memory, so the 544 threads' stack frames would miss it and every local access would cost
-// an L2 round trip (measured: a 100-instruction block went from 0.25 to 3 microseconds).  Helpers are
-// inlined, arrays are indexed by unrolled loops, and only code that runs once per launch or layer
-// with little live state (the deal, the route records) is kept out of line.
-// And straight code that every warp meets once a layer is fetched again each time, about four cycles an instruction: the
-// counting loops of the selection are loops (14 layers of 2048 x 2048 269.3 us unrolled, so 264.2).  That is no rule for code whose operations overlap when it is unrolled (tensor-memory loads and their sums, the digits' halves, the
-// router's two rows: 1-2 us more as loops), and a chain of F32 operations in place of the FP64 ones of the SwiGLU and of
-// the digit sums, which pays in the block kernels, is longer here (339 and 343 us).
+// Nothing on the kernel's paths may live in local memory: nearly all of the SM's L1 is carved out as shared memory, so the 512
+// threads' stack frames would miss it and every local access would cost an L2 round trip (measured: a 100-instruction block went
+// from 0.25 to 3 microseconds).  Helpers are inlined, arrays are indexed by unrolled loops, and only code that runs once per launch
+// or layer with little live state (the deal, the route records) is kept out of line.  And straight code that every warp meets once
+// a layer is fetched again each time, about four cycles an instruction: the counting loops of the selection are loops (14 layers of
+// 2048 x 2048 269.3 us unrolled, so 264.2; a single layer is 0.15-0.25 us faster with them unrolled, of 1024 x 1024 13.6 and
+// 13.8).  That is no rule for code whose operations overlap when it is unrolled (tensor-memory loads and their sums, the digits'
+// halves, the router's two rows: 1-2 us more as loops), and a chain of F32 operations in place of the FP64 ones of the SwiGLU and
+// of the digit sums, which pays in the block kernels, is longer here (339 and 343 us).
 
 // The two CTAs of a cluster.  The cluster barrier's halves, executed by every thread.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -1591,9 +1592,12 @@ cudaError_t launch_moe_layer_umma(cudaStream_t st, int sm_count, const JobTable 
     // paths (exchange inside the kernel, or expert outputs handed to a collective) are ordinary
     // launches; the kernel's own dependency calls are then no-ops.
     const bool pdl = ex.world <= 1u && y != nullptr;
-    // In pairs where items are shared and the launch gains by it: a launch in clusters takes 1.5 us more, and half an item of 16
-    // units saves 0.9 us a layer, of eight next to nothing.  us in pairs and not: 4096 x 2048, six given jobs of the executor's step
-    // 33.3 and 34.1, one routed layer 25.0 and 24.6, two 48.3 and 49.2; 2048 x 2048, the step 26.9 and 25.6, 14 layers 264 both.
+    // In pairs where items are shared and the launch gains by it (the calls take hidden sizes of 1024, 2048 and 4096): a launch in
+    // clusters takes 1.5 us more, and half an item of 16 units saves 0.9 us a layer, of eight next to nothing.  us in pairs and
+    // not: 4096 x 2048, six given jobs of the executor's step 33.3 and 34.1, one routed layer 25.0 and 24.6, two 48.3 and 49.2;
+    // 4096 x 1024, five layers 95 and 98, given jobs by number, with a shared one: one routed 12.7 and 14.6, three 14.9 and 15.7;
+    // 4096 x 4096, two routed 23.4 and 25.2, four 29.7 and 31.8, six 35.5 and 38.0; 2048 x 2048, the step 26.9 and 25.6, 14 layers
+    // 264 both.
     const bool given = !router && !dev;   // the jobs are in `param`
     const uint32_t n_early = router && rt.has_shared ? 1u : 0u, n_jobs = given ? param.n_jobs : rt.top_k + n_early;
     const bool paired = hidden >= 4096u && !dev && ex.world <= 1u && rt.ep_world <= 1u && (given || n_layers > 1u) &&

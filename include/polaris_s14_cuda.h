@@ -322,9 +322,10 @@ S14_API int32_t s14_cmd_moe_layer(s14_ctx *ctx, void *stream, const s14_moe_laye
 S14_API int32_t s14_layer_work_list(uint32_t cta, uint32_t n_ctas, uint32_t n_jobs, uint32_t n_early_jobs,
                                     uint32_t hidden, uint32_t inter, uint32_t *items_out, uint32_t cap,
                                     uint32_t *count);
-/* The same for CTA `block` of a grid whose CTAs run in pairs (block, block ^ 1), which is how the kernel is launched where
- * that gains time (hidden from 4096, several layers or given jobs, nothing expert parallel) and every pair fits on the device at a time.  An up item that would go to one CTA of a pair alone may be shared along K: bit 30,
- * and bit 29 in the list of the CTA that takes the second half. */
+/* The same for CTA `block` of a grid whose CTAs run in pairs (block, block ^ 1), for tests and for reading profiles like the
+ * list above: what a launch in pairs of these sizes would deal.  The kernel is launched so where that gains time (hidden 4096, several
+ * layers or given jobs, nothing expert parallel) and every pair fits on the device at a time.  An up item that would go to one CTA
+ * of a pair alone may be shared along K: bit 30, and bit 29 in the list of the CTA that takes the second half. */
 S14_API int32_t s14_layer_pair_list(uint32_t block, uint32_t n_ctas, uint32_t n_jobs, uint32_t n_early_jobs,
                                     uint32_t hidden, uint32_t inter, uint32_t *items_out, uint32_t cap,
                                     uint32_t *count);
