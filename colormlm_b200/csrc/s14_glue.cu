@@ -674,11 +674,11 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
 cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged) {
     const uint32_t vec = aligned16(branch, residual, merged);
-    // BF16: four values a thread (8-byte accesses) while their CTAs come to less than four per SM (one token of 4096 1.4 us, eight
-    // values 1.6; 64 tokens 1.9 and 2.0), from there on eight (148 tokens of 2048 2.04 us, four values 2.16; 185 2.22 and 2.44; 1024
-    // of 4096 9.6 and 11.9); values one by one up to five per SM (300 tokens of 1024 3.0 us, eight values 5.4)
-    const uint64_t elements = (uint64_t)n_tokens * hidden, per_sm = (uint64_t)sm_count * 512u;
-    const bool few = vec ? elements < 4u * per_sm : elements <= 5u * per_sm;
+    // BF16: four values a thread (8-byte accesses) while their CTAs come to at most five per SM (one token of 4096 1.4 us, eight
+    // values 1.6; 64 tokens 1.9 and 2.0), above that eight (1024 tokens 9.6 us, four values 11.9).  With four and five CTAs per SM
+    // calls one after another are faster with eight (148 tokens of 2048 2.04 us and 2.16), whole sites with four (370 of 1024
+    // 14.8 us and 15.3, 150 of 2048 14.7 and 15.1), and values one by one much so (300 of 1024 3.0 us and 5.4).
+    const bool few = (uint64_t)n_tokens * hidden <= (uint64_t)sm_count * 5u * 512u;
     // 8 to 32 tokens (two groups of k_hc_dots): the SMs divided as that kernel needs them, three CTAs of 26 KB.  Its CTAs, the next
     // site's, are to start while this kernel runs, and once the two need more than the SMs they have to share some, which an SM divided
     // otherwise makes them wait for.  Sites one after another, us: 10 tokens of 7168 17.7, so 14.4, 14 of 5120 15.7 and 13.1, 12 of 4096 12.9

@@ -148,18 +148,18 @@ def test_reduce_of_many_tokens_into_an_unaligned_result(ctx, bf16):
 
 
 # the head's clusters of two of short rows (on 148 SMs up to 111 tokens of 1024, 74 of 1792) and the two launches behind them; five
-# slices of K to an SM (F32, 592 tokens of 2048); hc_post's division of the SMs (32 tokens), its values a thread (148 of 2048) and its registers
+# slices of K to an SM (F32, 592 tokens of 2048); hc_post's division of the SMs (32 tokens), its values a thread (186 of 2048) and its registers
 # (148 of 4096)
 @pytest.mark.parametrize("bf16", [False, True])
 @pytest.mark.parametrize("n_tokens,hidden", [(111, 1024), (112, 1024), (74, 1792), (75, 1792), (74, 2048), (592, 2048), (32, 512), (33, 512),
-                                             (147, 2048), (148, 2048), (148, 4096), (149, 4096)])
+                                             (185, 2048), (186, 2048), (148, 4096), (149, 4096)])
 def test_sites_where_forms_change(ctx, oracle, bf16, n_tokens, hidden):
     test_sites_of_all_forms(ctx, oracle, bf16, n_tokens, hidden)
 
 
 # what goes by the number of tokens on other boundaries too: hc_post's values a thread and registers, the norm's forms
 @pytest.mark.parametrize("bf16", [False, True])
-@pytest.mark.parametrize("t,h", [(148, 1024), (149, 1024), (147, 2048), (148, 2048), (149, 4096), (296, 1024), (297, 1024), (444, 1024),
+@pytest.mark.parametrize("t,h", [(148, 1024), (149, 1024), (185, 2048), (186, 2048), (149, 4096), (296, 1024), (297, 1024), (444, 1024),
                                  (445, 1024)])
 def test_many_tokens_on_any_boundary(ctx, bf16, t, h):
     g = torch.Generator(device="cuda").manual_seed(t + h)
