@@ -43,7 +43,7 @@ constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens: most expe
 constexpr uint32_t kGrpSparse = 6;   // fewer than three pairs (official arithmetic: six) per expert on average
 constexpr uint32_t kGrpDense = 12;
 // (Both bounds, and the one of twelve tokens, were found with one-CTA kernels that had other stages; on the pair kernel, whose
-// rings hold ten, nine and seven stages, the three sizes have not been compared with each other.)
+// rings hold eight, eight and seven stages, the three sizes have not been compared with each other.)
 static_assert(kBlockNt == kGrpDense * 8u / 6u * 2u, "a chunk record holds the tokens of the official arithmetic's chunks");
 
 // The nearest E4M3FN values (ties to even) of two numbers of magnitude 448 at most, as F32 values: the conversion there and back.
@@ -401,7 +401,7 @@ bool moe_block_ok(int sm_count, uint32_t hidden, uint32_t inter, uint32_t n_expe
     if (sm_count <= 0 || n_experts == 0u || n_experts > S14_N_ROUTED_EXPERTS || top_k == 0u || top_k > S14_EXPERTS_PER_TOKEN)
         return false;
     if ((hidden & 511u) || (inter & 511u) || hidden < 512u || inter < 512u || hidden > 4096u || inter > 4096u) return false;
-    return pair_dynamic_limit() >= 4u * (kStageA + kGrpDense / 2u * 2048u + 4u * kAtomBytes);
+    return pair_dynamic_limit() >= 6u * (kStageA + kGrpDense / 2u * 2048u);
 }
 
 size_t moe_block_max_chunks(uint32_t max_tokens) {

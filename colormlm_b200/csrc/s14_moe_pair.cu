@@ -14,25 +14,29 @@
 // 8 tokens 117 us for the call, now 109.  (Official blocks of two to eight tokens of smaller layers gained nothing: 4 tokens of
 // 2048 x 1536 49 us for the call, now 52.)
 //
-// What bounds it: a step is four MMAs and six copies of scale codes: the MMAs of a full chunk take 384 cycles
-// (270 for the chunks 370 tokens have on average), the issuing warp's round 470 at most, but a step 560 on average at full
-// clock; the kernels take in 9 to 10.8 TB/s from the L2 meanwhile.  Beside them the epilogue.  Cycles of an item at full clock,
-// waiting for accumulators / adding their columns / the rest: 370 tokens up 4100 / 3000 / 1950, down 1100 / 3050 / 490; official ones,
+// What bounds it: a step is four MMAs and two copies of the unit's scale codes.  The MMAs of a full chunk take 384 cycles (270 for the
+// chunks 370 tokens have on average), a step takes 520 at full clock: an SM takes in some 50 bytes a clock then, 26 KB a step, and rings of
+// six stages and of seven are as fast, so it is the stream from the L2 that the rest waits for.  With the digit rows' codes laid out in
+// shared memory and copied too (six copies in the issuing warp's round, which looked at a stage only when it wanted it) a step took 600:
+// 370 tokens 675 us, so 635, 1000 official ones 820 and 806 (bursts; 785 and 725, 960 and 920 power limited).  Codes written by their warps
+// for one stage at a time, the unit's among them, took 900 a step: a wait costs 100 cycles, over or not.
+// Beside the steps the epilogue.  Cycles of an item at full clock,
+// waiting for accumulators / adding their columns / the rest: 370 tokens up 3450 / 2950 / 1900, down 900 / 3050 / 380; official ones,
 // with exact sums and the SwiGLU here, up 950 / 3900 / 5500, down 540 / 4150 / 1550: there the epilogue was what bounded both
 // kernels (1000 tokens 1036 us, without an epilogue 825, without three of four MMAs 1003, without the tiles' copies 1067), and fewer steps
 // (six digit rows for eight) alone gave nothing.  So BF16 sums are settled by plain additions and a bound where that is possible, four
 // pairs of tokens side by side, and the SwiGLU is k_block_digits' work: 1161 us power limited, now 992.  (The like for F32 sums, one part of the
-// three exact: 370 tokens nothing, 8 tokens 115 -> 120.)  A second warp that copies the codes ahead gets a probe to 389 cycles a
-// step, but adds a hand-off to every stage's way through the ring of seven (370 tokens 736 us instead of 704).  Sustained, the
+// three exact: 370 tokens nothing, 8 tokens 115 -> 120.)  Sustained, the
 // 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.  A pair with more items
 // than a batch of records drains its pipeline between two batches (1000 official tokens: 73 items, batches of 56).
 //
-// Roles in a CTA of 608 threads: warps 0-7 epilogue (two warpgroups, each with every lane of tensor memory, the even and
+// Roles in a CTA of 544 threads: warps 0-7 epilogue (two warpgroups, each with every lane of tensor memory, the even and
 // the odd tokens of the chunk, or its halves); warps 8-11 copy (the ring slots in turn, a lane per copy: a round of waiting, arming
-// and seven copies takes 0.3-0.5 us); warp 12 of the first CTA issues the pair's tensor operations, that of the second
-// passes on that its stage is complete; warps 13-18 lay out the scale codes of the digit rows of a stage.  A stage's barriers:
-// `full` in each CTA (unit, tiles, codes; in the first CTA also that the second's is complete), `done` in each (the commit
-// arrives at both).  Every wait is bounded; one that runs out raises the CTA's abort flag, the status word is set, the CTA
+// and seven copies takes 0.3-0.5 us); warps 12-15, one per quadrant of tensor memory, write the scale codes of the digit rows there, two
+// stages at a time and up to six ahead; warp 16 of the first CTA issues the pair's tensor operations, that of the second
+// passes on that its stage is there.  A stage's barriers: `full` in each CTA (unit and tiles; in the first CTA also that the second's
+// are there), `done` in each (the commit arrives at both); `rows` in the first CTA says that both CTAs' codes of a pair of stages are
+// written.  Every wait is bounded; one that runs out raises the CTA's abort flag, the status word is set, the CTA
 // waits for its copies and the pair's tensor work, and the pair meets at a cluster barrier before tensor memory is freed.
 #include "s14_moe_block.cuh"
 
@@ -41,16 +45,20 @@ namespace s14 {
 namespace {
 
 constexpr uint32_t kPGroups = 12, kPCols = 16u * kPGroups;   // accumulator columns of a chunk
-constexpr uint32_t kPEpi = 256, kPProds = 4, kPProdWarp0 = kPEpi / 32u, kPMmaWarp = kPProdWarp0 + kPProds, kPCodeWarp0 = kPMmaWarp + 1u;
-constexpr uint32_t kPCodes = kPCols;                         // a thread per operand row
-constexpr uint32_t kPThreads = kPCodeWarp0 * 32u + kPCodes;
-constexpr uint32_t kPRingMax = 12;
-// tensor memory columns: two sets of accumulators, then the scale codes of four stages
-constexpr uint32_t kPColScale = 2u * kPCols, kPScaleSets = 4, kPScaleCols = 32;   // a set: unit codes [2][4], digit-row codes [2][8]
-static_assert(kPColScale + kPScaleSets * kPScaleCols <= 512u, "tensor memory map");
+constexpr uint32_t kPEpi = 256, kPProds = 4, kPProdWarp0 = kPEpi / 32u, kPCodes = 4, kPCodeWarp0 = kPProdWarp0 + kPProds;
+constexpr uint32_t kPMmaWarp = kPCodeWarp0 + kPCodes, kPThreads = (kPMmaWarp + 1u) * 32u;
+static_assert(kPCodeWarp0 % 4u == 0u, "a warp reaches the lanes of tensor memory that its number modulo four says");
+// Most stages of the ring: with more of them small blocks ask the memory for more than it has, and some SMs get less than others (8 tokens,
+// 4096 x 2048, rings of 6 / 7 / 8 / 9 / 11: 110.4 / 109.6 / 109.4 / 110.0 / 115 us, 45 tokens of 2048 x 1536 122.1 / 121.3 / 121.2 / 123.0).
+constexpr uint32_t kPRingMax = 8;
+// tensor memory columns: two sets of accumulators, the digit rows' scale codes of six stages, the units' of four
+constexpr uint32_t kPRowSets = 3, kPRowCols = 32;    // a set: two stages, [2][2][8]
+constexpr uint32_t kPUnitSets = 4, kPUnitCols = 8;   // [2][4]
+constexpr uint32_t kPColRows = 2u * kPCols, kPColUnits = kPColRows + kPRowSets * kPRowCols;
+static_assert(kPColUnits + kPUnitSets * kPUnitCols <= 512u, "tensor memory map");
 // barriers
-constexpr uint32_t kPBarFull = 0, kPBarDone = kPRingMax;
-constexpr uint32_t kPBarAccDone = 2 * kPRingMax, kPBarAccFree = kPBarAccDone + 2, kPBarFin = kPBarAccFree + 2, kPBars = kPBarFin + 1;
+constexpr uint32_t kPBarFull = 0, kPBarDone = kPRingMax, kPBarRows = 2 * kPRingMax;
+constexpr uint32_t kPBarAccDone = kPBarRows + kPRowSets, kPBarAccFree = kPBarAccDone + 2, kPBarFin = kPBarAccFree + 2, kPBars = kPBarFin + 1;
 
 struct PairItem {
     unsigned long long page;
@@ -94,6 +102,14 @@ __device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t adesc, uint64
 __device__ __forceinline__ void pair_copy_scales(uint32_t tmem, uint64_t desc) {
     asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
 }
+// Sixteen columns of the warp's 32 lanes of its CTA's own tensor memory; complete behind tmem_st_wait().
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&w)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]), "r"(w[10]), "r"(w[11]),
+                 "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // arrives at the barrier of both CTAs when the tensor operations issued so far are complete
 __device__ __forceinline__ void pair_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
@@ -240,15 +256,19 @@ __device__ __forceinline__ bool digit_sums_quick(const uint32_t (&r)[M], int fir
 template <uint32_t kRows>
 __device__ __forceinline__ uint32_t half_rows(uint32_t nt) { return (((nt + 1u) >> 1) * kRows + 15u) & ~15u; }
 
-// kTok: most tokens of a chunk: twelve, in the official arithmetic 4, 16 or 32.  There the kernel is compiled for each: what 32
+// kTok: most tokens of a chunk: 2, 6 or 12, in the official arithmetic 4, 16 or 32.  The kernel is compiled for each: what 12 or 32
 // tokens need of code in the epilogue, which every launch fetches anew, and of loads for the items' records lay in the way of small blocks (us,
-// one form and three: 8 tokens of 512 x 512 28.4 and 23.2, of 2048 x 1024, 64 experts, 48.6 and 42.2; one token of 4096 x 2048 47.0 and 40.3).
+// official, one form and three: 8 tokens of 512 x 512 28.4 and 23.2, of 2048 x 1024, 64 experts, 48.6 and 42.2; one token of 4096 x 2048 47.0
+// and 40.3).  The forms for small chunks keep to 80 registers (said by a bound of 768 threads): with 96 the CTAs of the launch behind
+// find no room beside this one's, and are set up only when it ends (8 tokens 115 us, 96 registers and one F32 form 115-120, so 109.4; of
+// 2048 x 1024 49.0, 52, 45.0; one token 45.7, 46, 42.3).  Those for 12, 16 and 32 tokens would spill.
 template <bool kDown, bool kOff, uint32_t kTok>
-__global__ void __launch_bounds__(kPThreads, 1)
-k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *status) {
+__global__ void __launch_bounds__(kTok > (kOff ? 4u : 6u) ? kPThreads : 768u, 1)
+k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr uint32_t kRows = kOff ? 6u : 16u, kTileB = kRows * 128u;   // a token's digit rows, and the bytes of its tile
     static_assert(kTok <= kPCols / 2u / kRows * 2u, "the columns of an accumulator");
+    constexpr uint32_t kHalf = (kTok * kRows + 31u) / 32u;       // groups of sixteen rows that a CTA of the pair brings at most
     constexpr uint32_t kMine = kOff ? kTok / 4u : kTok / 2u;      // tokens of an epilogue thread (official: pairs of them)
     constexpr uint32_t kPBatch = kOff ? 56u : 96u;                // items decoded at a time (10 KB of static shared memory are left beside the ring)
     __shared__ __align__(8) uint64_t bars[kPBars];
@@ -263,8 +283,6 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
     const uint32_t K = kDown ? a.inter : a.hidden;
     const uint32_t nu = K >> 8;                                    // units of an item
     const uint32_t ring = a.ring, stage = a.stage;
-    const uint32_t n_atoms = (half_cap * 32u + 127u) >> 7;         // scale atoms of a stage's digit rows, per 128 k
-    const uint32_t off_codes = kStageA + half_cap * 2048u;         // in a stage: the unit, the tiles, the digit rows' scale codes
     const size_t page_off = kDown ? mxfp4_down_offset(a.hidden, a.inter) : 0u;
     const uint32_t bar0 = smem_u32(bars), ring0 = smem_u32(smem);
     auto bar = [&](uint32_t i) { return bar0 + i * 8u; };
@@ -272,8 +290,8 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 
     if (tid < kPBars) {
         uint32_t count = 1u;
-        // the copying thread, the codes' warps; the first CTA's: and the second CTA's stage
-        if (tid < kPRingMax) count = 1u + kPCodes / 32u + (rank == 0u ? 1u : 0u);
+        if (tid < kPRingMax) count = rank == 0u ? 2u : 1u;   // the copying thread; the first CTA's: and the second CTA's stage
+        else if (tid >= kPBarRows && tid < kPBarRows + kPRowSets) count = 2u * kPCodes;   // the codes' warps of both CTAs
         else if (tid >= kPBarAccFree && tid < kPBarAccFree + 2u) count = 2u * kPEpi / 32u;
         mbar_init(bar(tid), count);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -296,7 +314,8 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
     const uint32_t n_local = n_items > me ? (n_items - me + n_pairs - 1u) / n_pairs : 0u;
 
     // what the roles carry from batch to batch
-    uint32_t slot = 0, round = 0, gi = 0, step = 0;
+    uint32_t slot = 0, round = 0, gi = 0, step = 0, set = 0, phase = 0;
+    bool ready = false;   // the issuing warp: the next two stages are there
     bool ok = true;
     auto next_slot = [&]() {
         if (++slot == ring) {
@@ -378,7 +397,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
             if (rank == 0u) {
                 const uint32_t tm = warp_uniform(tmem);
                 const uint64_t a_desc0 = smem_desc(ring0, 1, 64, 2), b_desc0 = smem_desc(ring0 + kStageA, 1, 64, 2);
-                const uint64_t sa_desc0 = smem_desc(ring0 + kUnitBytes, 0, 8, 0), sb_desc0 = smem_desc(ring0 + off_codes, 0, 8, 0);
+                const uint64_t sa_desc0 = smem_desc(ring0 + kUnitBytes, 0, 8, 0);
 #pragma unroll 1
                 for (uint32_t i = 0; i < nb && ok; ++i, ++gi) {
                     const uint32_t buf = gi & 1u, nt = warp_uniform(s_rec[i].nt & 0xFFu);
@@ -387,41 +406,52 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                     if (!ok) break;
                     fence_after();
                     const uint32_t acc = tm + buf * kPCols;
-                    const bool two = n > 128u;   // two scale atoms per 128 k
 #pragma unroll 1
-                    for (uint32_t ku = 0; ku < nu; ++ku) {
-                        ok = stage_wait(bar(kPBarFull + slot), round & 1u, abortp);
-                        if (!ok) break;
+                    for (uint32_t ku = 0; ku < nu; ku += 2u) {
+                        const uint32_t slot1 = slot + 1u == ring ? 0u : slot + 1u, round1 = slot + 1u == ring ? round + 1u : round;
+                        if (!ready) {
+                            ok = __all_sync(0xffffffffu, mbar_wait(bar(kPBarRows + set), phase, abortp) &&
+                                                             mbar_wait(bar(kPBarFull + slot), round & 1u, abortp) &&
+                                                             mbar_wait(bar(kPBarFull + slot1), round1 & 1u, abortp));
+                            if (!ok) break;
+                        }
                         fence_after();
-                        if (elect_one()) {
-                            const uint32_t at = slot * (stage >> 4), sfa = tm + kPColScale + (step & (kPScaleSets - 1u)) * kPScaleCols;
-                            const uint32_t sfb = sfa + 8u;
+                        auto issue = [&](uint32_t at_slot, uint32_t odd) {
+                            const uint32_t at = at_slot * (stage >> 4), sfa = tm + kPColUnits + ((step + odd) & (kPUnitSets - 1u)) * kPUnitCols;
+                            const uint32_t sfb = tm + kPColRows + set * kPRowCols + odd * (kPRowCols / 2u);
                             pair_copy_scales(sfa, sa_desc0 + at);
                             pair_copy_scales(sfa + 4u, sa_desc0 + at + (kAtomBytes >> 4));
-                            pair_copy_scales(sfb, sb_desc0 + at);
-                            pair_copy_scales(sfb + 8u, sb_desc0 + at + n_atoms * (kAtomBytes >> 4));
-                            if (two) {
-                                pair_copy_scales(sfb + 4u, sb_desc0 + at + (kAtomBytes >> 4));
-                                pair_copy_scales(sfb + 12u, sb_desc0 + at + (n_atoms + 1u) * (kAtomBytes >> 4));
-                            }
 #pragma unroll
                             for (uint32_t kk = 0; kk < 4; ++kk) {
                                 const uint32_t atom = kk >> 1, sfid = (kk & 1u) * 2u;
                                 pair_mma(acc, a_desc0 + at + kk * 2u, b_desc0 + at + kk * 2u, idesc | (sfid << 29) | (sfid << 4),
-                                         (sfa + atom * 4u) | (sfid << 30), (sfb + atom * 8u) | (sfid << 30), (ku || kk) ? 1u : 0u);
+                                         (sfa + atom * 4u) | (sfid << 30), (sfb + atom * 8u) | (sfid << 30), (ku || odd || kk) ? 1u : 0u);
                             }
-                            pair_commit(bar(kPBarDone + slot));
-                        }
+                            pair_commit(bar(kPBarDone + at_slot));
+                        };
+                        if (elect_one()) issue(slot, 0u);
                         __syncwarp();
-                        next_slot();
-                        ++step;
+                        // the next two stages are looked at while the operations run
+                        const uint32_t slot2 = slot1 + 1u == ring ? 0u : slot1 + 1u, round2 = slot1 + 1u == ring ? round1 + 1u : round1;
+                        const uint32_t slot3 = slot2 + 1u == ring ? 0u : slot2 + 1u, round3 = slot2 + 1u == ring ? round2 + 1u : round2;
+                        const uint32_t set2 = set + 1u == kPRowSets ? 0u : set + 1u, phase2 = set + 1u == kPRowSets ? phase ^ 1u : phase;
+                        const bool r0 = mbar_test(bar(kPBarRows + set2), phase2), r1 = mbar_test(bar(kPBarFull + slot2), round2 & 1u);
+                        const bool r2 = mbar_test(bar(kPBarFull + slot3), round3 & 1u);
+                        if (elect_one()) issue(slot1, 1u);
+                        __syncwarp();
+                        ready = __all_sync(0xffffffffu, r0 && r1 && r2);
+                        slot = slot2;
+                        round = round2;
+                        set = set2;
+                        phase = phase2;
+                        step += 2u;
                     }
                     if (!ok) break;
                     if (elect_one()) pair_commit(bar(kPBarAccDone + buf));
                     __syncwarp();
                 }
             } else {
-                // ---- the second CTA's stages are complete (every writer has made its bytes visible to the tensor cores) ----
+                // ---- the second CTA's stages are there ----
 #pragma unroll 1
                 for (uint32_t i = 0; i < nb * nu && ok; ++i) {
                     ok = stage_wait(bar(kPBarFull + slot), round & 1u, abortp);
@@ -480,10 +510,10 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                         if (g < nt) {   // uniform in the warpgroup
                             uint32_t r0[16], r1[16];
                             tmem_ld16(lane_base + buf * kPCols + 16u * g, r0);
-                            tmem_ld16(lane_base + buf * kPCols + 16u * (g + 2u), r1);   // (not used beyond nt)
+                            if (m + 1u < kMine) tmem_ld16(lane_base + buf * kPCols + 16u * (g + 2u), r1);   // (not used beyond nt)
                             tmem_ld_wait();
                             v[m] = digit_sum(r0);
-                            v[m + 1u] = digit_sum(r1);
+                            if (m + 1u < kMine) v[m + 1u] = digit_sum(r1);
                         }
                     }
                 }
@@ -537,39 +567,50 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
                     }
                 }
             }
-        } else if (warp >= kPCodeWarp0) {
-            // ---- the scale codes of ALL digit rows of the chunk (both CTAs' tensor cores multiply with every column) as the
-            // atoms tensor memory takes: row n of the operand = 16 * group + digit row, byte (n % 32) * 16 +
-            // (n / 32 % 4) * 4 + block % 4 of the atom of rows n / 128 and four scale blocks.  Digit row j < 8 of a block with
-            // exponent E has the code 127 + E - 23 + 3 j, row 8 + j the code 127 + E - 47 + 3 j; the exponents are stored as
-            // E + 100. ----
-            const uint32_t n = tid - kPCodeWarp0 * 32u;   // this thread's row
-            const uint32_t code_at = off_codes + (n >> 7) * kAtomBytes + (n & 31u) * 16u + ((n >> 5) & 3u) * 4u;
-            const bool has_row = n < half_cap * 32u;
-            // the row's exponents in an item, or nullptr, and (official: where the second half's rows start differs from item to item)
-            // what is added to them
-            uint32_t bias = 0u, bias_then = 0u;
+        } else {
+            // ---- the scale codes of ALL digit rows of the chunk (both CTAs' tensor cores multiply with every column), into tensor
+            // memory as the multiplication wants them: operand row n at lane n % 32 of every quadrant, column n / 32, a word per 128 k.
+            // Digit row j < 8 of a block with exponent E has the code 127 + E - 23 + 3 j, row 8 + j the code 127 + E - 47 + 3 j,
+            // official row j 127 + E - 17 + 3 j; the exponents are stored as E + 100.  Lane t loads token t's, for two stages at a time;
+            // rows that belong to nobody take any. ----
+            const uint32_t rows0 = tmem + kPColRows + (((warp & 3u) * 32u) << 16), full0 = first_cta(bar(kPBarRows));
+            constexpr uint32_t kCols = kHalf;   // tensor memory columns of a stage per 128 k
+            // column c's row of this lane: its token, and (official: where the second half's rows start differs from item to item) what is
+            // added to the exponents, in the lower and the upper half of a word
+            uint32_t row_of[kOff ? kCols : 1u] = {}, bias0 = 0u;
             if constexpr (!kOff) {
-                const uint32_t j = n & 15u;
-                bias = bias_then = 0x01010101u * (uint32_t)(j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20);
+                const uint32_t j = lane & 15u;
+                bias0 = 0x01010101u * (uint32_t)(j < 8u ? 4 + 3 * (int)j : 3 * (int)(j & 7u) - 20);
             }
-            auto exps_of = [&](uint32_t i) -> const uint4 * {
-                if (i >= nb || !has_row) return nullptr;
-                const uint32_t nt = s_rec[i].nt & 0xFFu;
-                uint32_t t = n / kRows;
+            auto rows_of = [&](uint32_t nt) {
                 if constexpr (kOff) {
-                    const uint32_t half = (nt + 1u) >> 1, hr = half_rows<kRows>(nt), m = n < hr ? n : n - hr, in = m / kRows;
-                    t = in < half ? (n < hr ? in : half + in) : nt;   // (rows between the halves belong to nobody)
-                    bias_then = 0x01010101u * (10u + 3u * (m - in * kRows));
+#pragma unroll
+                    for (uint32_t c = 0; c < kCols; ++c) {
+                        const uint32_t n = 32u * c + lane, half = (nt + 1u) >> 1, hr = half_rows<kRows>(nt), m = n < hr ? n : n - hr, in = m / kRows;
+                        row_of[c] = ((n < hr ? in : half + in) & 31u) | ((10u + 3u * (m - in * kRows)) << 16);
+                    }
                 }
-                if (t >= nt) return nullptr;
-                const uint32_t vec = kDown ? s_pair[i][t] : s_pair[i][t] / kPairsPerToken;
+            };
+            // the scale codes of one stage's rows: exponents of its two 128 k in, words out
+            auto words = [&](uint32_t lo, uint32_t hi, uint32_t (&w)[16]) {
+#pragma unroll
+                for (uint32_t c = 0; c < 8u; ++c) {
+                    w[c] = w[8u + c] = 0u;
+                    if (c < kCols) {
+                        const uint32_t at = kOff ? row_of[kOff ? c : 0u] : 2u * c + (lane >> 4), bias = kOff ? (at >> 16) * 0x01010101u : bias0;
+                        w[c] = __shfl_sync(0xffffffffu, lo, at & 31u) + bias;
+                        w[8u + c] = __shfl_sync(0xffffffffu, hi, at & 31u) + bias;
+                    }
+                }
+            };
+            auto exps_of = [&](uint32_t i) -> const uint4 * {
+                if (i >= nb || lane >= (s_rec[i].nt & 0xFFu)) return nullptr;
+                const uint32_t vec = kDown ? s_pair[i][lane] : s_pair[i][lane] / kPairsPerToken;
                 return reinterpret_cast<const uint4 *>(a.exps + (size_t)vec * (K >> 5));
             };
             // two units' exponents per load, four loads in flight, each in registers of its own (a queue that moves them waits
             // for the newest): the units in steps of eight, the last step of an item perhaps short
             const uint4 *now = exps_of(0);
-            bias = bias_then;
             uint4 e[4];
             auto fetch = [&](const uint4 *p, uint32_t u) { return p && u < nu ? __ldcg(p + (u >> 1)) : make_uint4(0u, 0u, 0u, 0u); };
 #pragma unroll
@@ -577,34 +618,40 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t half_cap, uint32_t *st
 #pragma unroll 1
             for (uint32_t i = 0; i < nb && ok; ++i) {
                 const uint4 *const then = exps_of(i + 1u);
-                const bool live = now != nullptr;
+                rows_of(s_rec[i].nt & 0xFFu);
 #pragma unroll 1
                 for (uint32_t u0 = 0; u0 < nu && ok; u0 += 8u) {
                     const bool more = u0 + 8u < nu;
-                    const uint4 *const from = more ? now : then;
+                    const uint4 *const next = more ? now : then;
                     const uint32_t at_u = more ? u0 + 8u : 0u;
 #pragma unroll
-                    for (uint32_t k = 0; k < 8u; ++k) {
-                        if (u0 + k < nu && ok) {
-                            ok = !round || stage_wait(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
-                            if (ok) {
-                                if (has_row) {
-                                    uint8_t *const s = smem + slot * stage + code_at;
-                                    *reinterpret_cast<uint32_t *>(s) = live ? ((k & 1u) ? e[k >> 1].z : e[k >> 1].x) + bias : 0x7F7F7F7Fu;
-                                    *reinterpret_cast<uint32_t *>(s + n_atoms * kAtomBytes) =
-                                        live ? ((k & 1u) ? e[k >> 1].w : e[k >> 1].y) + bias : 0x7F7F7F7Fu;
-                                }
-                                fence_async_smem();   // tcgen05.cp reads them
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive(bar(kPBarFull + slot));
+                    for (uint32_t k = 0; k < 4u; ++k) {
+                        if (u0 + 2u * k < nu && ok) {
+                            if (step >= 2u * kPRowSets) {
+                                // the set's last stage, five before this pair's first, is complete; `slot` follows it
+                                if (step > 2u * kPRowSets) next_slot();
                                 next_slot();
+                                ok = stage_wait(bar(kPBarDone + slot), round & 1u, abortp);
+                            }
+                            if (ok) {
+                                const uint32_t at = rows0 + set * kPRowCols;
+                                uint32_t w[16];
+                                words(e[k].x, e[k].y, w);
+                                tmem_st16(at, w);
+                                words(e[k].z, e[k].w, w);
+                                tmem_st16(at + 16u, w);
+                                tmem_st_wait();
+                                fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive_remote(full0 + set * 8u);
+                                step += 2u;
+                                if (++set == kPRowSets) set = 0;
                             }
                         }
-                        if (k & 1u) e[k >> 1] = fetch(from, at_u + k - 1u);
+                        e[k] = fetch(next, at_u + 2u * k);
                     }
                 }
                 now = then;
-                bias = bias_then;
             }
         }
         __syncwarp();
@@ -671,7 +718,9 @@ size_t pair_dynamic_limit() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     if (limit[dev]) return limit[dev];
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-    const void *const fns[] = {(const void *)k_block_pair<false, false, 12>, (const void *)k_block_pair<true, false, 12>,
+    const void *const fns[] = {(const void *)k_block_pair<false, false, 2>,  (const void *)k_block_pair<true, false, 2>,
+                               (const void *)k_block_pair<false, false, 6>,  (const void *)k_block_pair<true, false, 6>,
+                               (const void *)k_block_pair<false, false, 12>, (const void *)k_block_pair<true, false, 12>,
                                (const void *)k_block_pair<false, true, 4>,   (const void *)k_block_pair<true, true, 4>,
                                (const void *)k_block_pair<false, true, 16>,  (const void *)k_block_pair<true, true, 16>,
                                (const void *)k_block_pair<false, true, 32>,  (const void *)k_block_pair<true, true, 32>};
@@ -691,14 +740,16 @@ size_t pair_dynamic_limit() {
 }
 
 cudaError_t launch_pair_gemm(cudaStream_t st, int sm_count, bool down, bool official, GemmArgs args, uint32_t half, uint32_t *status) {
-    args.stage = kStageA + half * 2048u + 2u * ((half * 32u + 127u) / 128u) * kAtomBytes;
+    args.stage = kStageA + half * 2048u;
     args.ring = std::min<uint32_t>((uint32_t)(pair_dynamic_limit() / args.stage), kPRingMax);
-    if (args.ring < 2u || half == 0u || 2u * half > kPGroups) return cudaErrorInvalidConfiguration;
+    if (args.ring < 2u * kPRowSets || half == 0u || 2u * half > kPGroups) return cudaErrorInvalidConfiguration;
     const size_t smem = (size_t)args.ring * args.stage;
     const dim3 grid((uint32_t)sm_count & ~1u), block(kPThreads);
     auto run = [&](auto up_kernel, auto down_kernel) {
-        return launch_pdl(down ? down_kernel : up_kernel, grid, block, smem, st, 2u, args, half, status);
+        return launch_pdl(down ? down_kernel : up_kernel, grid, block, smem, st, 2u, args, status);
     };
+    if (!official && half == 1u) return run(k_block_pair<false, false, 2>, k_block_pair<true, false, 2>);
+    if (!official && half <= 3u) return run(k_block_pair<false, false, 6>, k_block_pair<true, false, 6>);
     if (!official) return run(k_block_pair<false, false, 12>, k_block_pair<true, false, 12>);
     if (half == 1u) return run(k_block_pair<false, true, 4>, k_block_pair<true, true, 4>);
     if (half <= 3u) return run(k_block_pair<false, true, 16>, k_block_pair<true, true, 16>);

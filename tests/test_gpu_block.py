@@ -108,6 +108,36 @@ def test_block_at_the_other_sizes(ctx, oracle, hidden, inter):
         blk.close()
 
 
+@pytest.mark.parametrize("official", [False, True])
+@pytest.mark.parametrize("hidden,inter", [(512, 1536), (2560, 512), (1536, 3584)])
+def test_block_of_every_chunk_form_and_odd_numbers_of_units(ctx, oracle, hidden, inter, official):
+    """Items of 2, 6, 10 and 14 units of 256 elements (the scale codes are written two units at a time and fetched eight ahead, so
+    items end in the middle of both), in the kernels for each of the three chunk sizes: blocks of 3 and 12 tokens, of 14 over many
+    experts, of 40 over few, whose chunks are full, partly filled and of odd size."""
+    layer = oracle.official_moe_layer if official else oracle.moe_layer_acc64
+    g, pages, shared = make_layer(1700 + hidden, hidden, inter, 8, L.PAGE_MXFP4)
+    pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
+    blk = MoeBlock(ctx, hidden, inter, 40)
+    try:
+        blk.set_semantics(official)
+        for n_tokens, n_experts in ((3, 8), (12, 8), (14, 48), (40, 8)):
+            x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(synth.activations(g, n_tokens, hidden)))
+            wr, bias = dev(synth.router_weight_bf16(g, n_experts, hidden)), dev(synth.router_bias(g, n_experts))
+            table = torch.tensor([pages_dev[e % 8].data_ptr() for e in range(n_experts)], dtype=torch.int64, device="cuda")
+            dx, dy = dev(x), torch.full((n_tokens, hidden), float("nan"), device="cuda")
+            ids = torch.empty((n_tokens, 6), dtype=torch.int32, device="cuda")
+            wts = torch.empty((n_tokens, 6), device="cuda")
+            blk.cmd_routed_moe_block(dx, wr, bias, table, shared_dev.data_ptr(), dy, ids, wts)
+            torch.cuda.synchronize()
+            assert ctx.device_status() == 0
+            y, ids_np, w_np = dy.cpu().numpy(), ids.cpu().numpy(), wts.cpu().numpy()
+            for t in sorted({0, 1, 2, n_tokens // 2, n_tokens - 1}):
+                ref = layer(x[t], [pages[e % 8] for e in ids_np[t]], w_np[t], shared, 0, hidden, inter)
+                assert np.array_equal(y[t].view(np.uint32), ref.view(np.uint32)), (n_tokens, t)
+    finally:
+        blk.close()
+
+
 def test_block_sweep_of_block_sizes_against_the_one_token_kernel(ctx):
     """Block sizes around every boundary of the chunking (1, 2, 6, 7, 12, 13 tokens; 33 and 64 with experts of
     many chunks), ragged routes, few experts so that groups are large: every token equals its own one-token call
