@@ -15,11 +15,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_NAME = "libpolaris_s14_cuda.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
-SOURCES = ["s14_kernels.cu", "s14_moe_umma.cu", "s14_moe_block.cu", "s14_moe_pair.cu", "s14_glue.cu", "s14_head.cu", "s14_fp8_expert.cu", "s14_api.cu", "s14_host.cpp"]
+SOURCES = ["s14_kernels.cu", "s14_router.cu", "s14_moe_umma.cu", "s14_moe_block.cu", "s14_moe_pair.cu", "s14_glue.cu", "s14_head.cu", "s14_fp8_expert.cu", "s14_api.cu", "s14_host.cpp"]
 # the Python mirror's per-token calls, a CPython extension over the library (no CUDA, no torch headers)
 PYCALL_SOURCE = "s14_pycall.cpp"
 PYCALL_PATH = os.path.join(HERE, "_s14call.so")
-HEADERS = ["s14_internal.h", "s14_device.cuh", "s14_umma.cuh", "s14_moe_block.cuh", "s14_host.hpp", os.path.join("..", "..", "include", "polaris_s14_cuda.h")]
+HEADERS = ["s14_internal.h", "s14_device.cuh", "s14_router.cuh", "s14_umma.cuh", "s14_moe_block.cuh", "s14_host.hpp", os.path.join("..", "..", "include", "polaris_s14_cuda.h")]
 
 
 def _nvcc() -> str:

@@ -268,10 +268,10 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
 cudaError_t launch_block_mix(cudaStream_t st, const float *pairs, const int32_t *ids, const float *weights, uint32_t n_tokens,
                              uint32_t top_k, bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts,
                              const BlockEp *ep = nullptr, uint32_t *status = nullptr);
-// Scores and routes of many tokens (s14_kernels.cu): the tokens of a tile share the router rows in
-// shared memory; one warp per token selects.  Same arithmetic as launch_router.  Returns the number
-// of kernels launched.
-int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, cudaError_t *err);
+// Scores and routes of many tokens (s14_router.cu).  Same arithmetic as launch_router.  hidden is a multiple of 512 up to 4096; scores, select:
+// [n_tokens, n_experts] scratch, parts: [8, n_tokens, 256] (for more than 64 tokens; a block's pair outputs, of 7 x 512 values a token
+// at least, have room for it and are written later).  Returns the number of kernels launched.
+int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, cudaError_t *err);
 
 // ---- the steps on either side of the MoE inside one layer (s14_glue.cu) ----
 // scratch: hc_scratch_bytes(the most tokens of a call).  Returns the number of kernels launched.

@@ -12,6 +12,7 @@
 // The elementwise steps (limit-10 SwiGLU, route mix, ordered accumulate) use
 // separate F32 multiplies and adds in both modes, as the reference does.
 #include "s14_device.cuh"
+#include "s14_router.cuh"
 
 namespace s14 {
 
@@ -783,98 +784,6 @@ k_mix_slots(const float *__restrict__ slots, const float *__restrict__ weights, 
 // f32 x bf16 is exact in double), score and score + bias in F32.  The last CTA to finish
 // (a counter in global memory, no waiting) selects the top-k of every token, normalises the
 // weights and, for the one-token decode path, writes the job table of the layer.
-__device__ __forceinline__ void router_select(const float *scores, const float *select,
-                                              uint32_t n_experts, uint32_t top_k, float route_scale,
-                                              int32_t *ids_out, float *weights_out, JobTable *table_out,
-                                              const uint8_t *const *page_table, const uint8_t *shared_page,
-                                              uint32_t shared_kind, uint32_t lane, uint32_t ep_rank,
-                                              uint32_t ep_world, uint32_t shared_owner) {
-    // a round per pick: the largest score + bias (as an ordered integer) of what is left, the lowest expert id on ties.  A loop,
-    // two warp reductions a round (eight rounds of straight code with 64-bit keys through shuffles: a block of 45 tokens 147.6 us, so
-    // 146.8)
-    uint32_t key[8];   // of experts lane, lane + 32, ...; `left` says which are there and not taken
-    uint32_t left = 0u;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t e = i * 32 + lane;
-        key[i] = 0u;
-        if (e < n_experts) {
-            const uint32_t bits = __float_as_uint(__ldcg(select + e));
-            key[i] = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-            left |= 1u << i;
-        }
-    }
-    uint32_t mine = 0u;   // lane j: the expert of route j
-#pragma unroll 1
-    for (uint32_t j = 0; j < top_k; ++j) {
-        uint32_t best = 0u;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) best = max(best, (left >> i & 1u) ? key[i] : 0u);
-        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-        uint32_t id = 0xffffffffu;
-#pragma unroll
-        for (int i = 7; i >= 0; --i)
-            if ((left >> i & 1u) && key[i] == top) id = i * 32u + lane;
-        id = __reduce_min_sync(0xffffffffu, id);
-        if ((id & 31u) == lane) left &= ~(1u << (id >> 5));
-        if (lane == j) mine = id;
-    }
-    const float score = lane < top_k ? __ldcg(scores + mine) : 0.0f;
-    int32_t ids[8];
-    float picked[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        ids[j] = (int32_t)__shfl_sync(0xffffffffu, mine, j);
-        picked[j] = __shfl_sync(0xffffffffu, score, j);
-    }
-    if (lane != 0) return;
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if ((uint32_t)j < top_k) sum = __fadd_rn(sum, picked[j]);
-    // Expert parallel: this rank keeps the jobs of the experts it owns (id mod world == rank) and,
-    // if it is the shared expert's owner, the shared job; every job writes the row of its route
-    // slot so that the ranks' outputs add up to the full set.
-    uint32_t n = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if ((uint32_t)j >= top_k) continue;
-        const float w = __fmul_rn(__fdiv_rn(picked[j], sum), route_scale);
-        if (ids_out) ids_out[j] = ids[j];
-        if (weights_out) weights_out[j] = w;
-        if (table_out && ((uint32_t)ids[j] % ep_world) == ep_rank) {
-            Job jb;
-            jb.page = page_table[ids[j]];
-            jb.kind = S14_PAGE_MXFP4;
-            jb.token = 0;
-            jb.weight = w;
-            jb.is_shared = 0;
-            jb.out_index = (uint32_t)j;
-            table_out->jobs[n] = jb;
-            table_out->token_jobs[n] = (uint8_t)n;
-            ++n;
-        }
-    }
-    if (table_out) {
-        if (shared_page && shared_owner == ep_rank) {
-            Job jb;
-            jb.page = shared_page;
-            jb.kind = shared_kind;
-            jb.token = 0;
-            jb.weight = 1.0f;
-            jb.is_shared = 1;
-            jb.out_index = top_k;
-            table_out->jobs[n] = jb;
-            table_out->token_jobs[n] = (uint8_t)n;
-            ++n;
-        }
-        table_out->n_jobs = n;
-        table_out->n_tokens = 1;
-        table_out->token_job_begin[0] = 0;
-        table_out->token_job_begin[1] = n;
-    }
-}
-
 __global__ void __launch_bounds__(64)
 k_router(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
          float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
@@ -1324,131 +1233,6 @@ k_stack_step(const float *__restrict__ x, const float *__restrict__ y, float *ou
     const float v = y[i];
     if (y_copy) y_copy[i] = v;
     out[i] = residual ? __fadd_rn(x[i], v) : v;
-}
-
-// ---- the router for many tokens ----
-// Scores on the FP64 matrix pipe: a CTA takes 8 * kMt tokens x 8 * kNt experts, its warps the K range in equal parts
-// (their sums meet in shared memory, in warp order).  mma.m8n8k4.f64 wants one element of A (8 tokens x 4 k) and of B
-// (4 k x 8 experts) per lane and step; which k an element stands for is free as long as A and B agree, so a lane
-// takes eight neighbouring elements of its row (32 bytes of x, 16 of the weights) and feeds them to eight steps:
-// operands go from the L2 to registers, four lanes share a cache line, nothing is staged.  Every f32 and bf16 value is
-// exact in double, so is every product, and the sums are double: score and score + bias are those of k_router.
-//
-// A token's row is read once per 8 * kNt experts and a weight row once per 8 * kMt tokens; both come from the L2.
-// 16 x 16 tiles for large blocks (wider ones leave too few CTAs, narrower ones read x more often); a smaller grid than two CTAs
-// per SM takes 16 x 8, up to 64 tokens 8 x 8 with the K range over sixteen warps.  Measured, x 256 experts x 4096:
-// 8 tokens 15 -> 8.3 us, 370 84 -> 40, 1000 166 -> 83 (before: operands staged in shared memory as doubles by 32 x 16
-// tiles with all of K in one warp; up to 32 tokens on the vector pipe); 45 tokens x 192 experts x 2048: 32 -> 10.
-template <uint32_t kMt, uint32_t kNt, uint32_t kWarps>
-__global__ void __launch_bounds__(kWarps * 32u)
-k_router_scores(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
-                float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
-                uint32_t n_tokens, uint32_t score_fn) {
-    __shared__ double s_c[kWarps][kMt * kNt][64];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, row = lane >> 2, col = lane & 3u;
-    const uint32_t e0 = blockIdx.x * (8u * kNt), t0 = blockIdx.y * (8u * kMt);
-    const uint32_t part = hidden / kWarps, first = warp * part + col * 8u;   // a whole number of steps of 32 elements
-    const float *xr[kMt];
-    const uint16_t *wp[kNt];
-    // (a token or expert past the end reads the last one again; its scores are not written)
-#pragma unroll
-    for (uint32_t m = 0; m < kMt; ++m) xr[m] = x + (size_t)min(t0 + m * 8u + row, n_tokens - 1u) * hidden + first;
-#pragma unroll
-    for (uint32_t n = 0; n < kNt; ++n) wp[n] = wr + (size_t)min(e0 + n * 8u + row, n_experts - 1u) * hidden + first;
-    double c[kMt][kNt][2];
-#pragma unroll
-    for (uint32_t m = 0; m < kMt; ++m)
-#pragma unroll
-        for (uint32_t n = 0; n < kNt; ++n) c[m][n][0] = c[m][n][1] = 0.0;
-    float4 xa[kMt], xb[kMt];
-    uint4 q[kNt];
-    auto load = [&](uint32_t k) {
-#pragma unroll
-        for (uint32_t n = 0; n < kNt; ++n) q[n] = __ldcg(reinterpret_cast<const uint4 *>(wp[n] + k));
-#pragma unroll
-        for (uint32_t m = 0; m < kMt; ++m) {
-            xa[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k));
-            xb[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k) + 1);
-        }
-    };
-    dependency_wait();
-    load(0);
-#pragma unroll 1
-    for (uint32_t k = 0; k < part; k += 32u) {
-        float a[kMt][8];
-        uint32_t b[kNt][4];
-#pragma unroll
-        for (uint32_t m = 0; m < kMt; ++m) {
-            a[m][0] = xa[m].x, a[m][1] = xa[m].y, a[m][2] = xa[m].z, a[m][3] = xa[m].w;
-            a[m][4] = xb[m].x, a[m][5] = xb[m].y, a[m][6] = xb[m].z, a[m][7] = xb[m].w;
-        }
-#pragma unroll
-        for (uint32_t n = 0; n < kNt; ++n) b[n][0] = q[n].x, b[n][1] = q[n].y, b[n][2] = q[n].z, b[n][3] = q[n].w;
-        if (k + 32u < part) load(k + 32u);
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            double av[kMt], bv[kNt];
-#pragma unroll
-            for (uint32_t m = 0; m < kMt; ++m) av[m] = (double)a[m][i];
-#pragma unroll
-            for (uint32_t n = 0; n < kNt; ++n)
-                bv[n] = (double)__uint_as_float((i & 1u) ? b[n][i >> 1] & 0xffff0000u : b[n][i >> 1] << 16);
-#pragma unroll
-            for (uint32_t m = 0; m < kMt; ++m)
-#pragma unroll
-                for (uint32_t n = 0; n < kNt; ++n)
-                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                                 : "+d"(c[m][n][0]), "+d"(c[m][n][1])
-                                 : "d"(av[m]), "d"(bv[n]));
-        }
-    }
-    // C (8 x 8): lane holds row lane / 4, columns 2 (lane % 4) and 2 (lane % 4) + 1
-#pragma unroll
-    for (uint32_t m = 0; m < kMt; ++m)
-#pragma unroll
-        for (uint32_t n = 0; n < kNt; ++n)
-            *reinterpret_cast<double2 *>(&s_c[warp][m * kNt + n][row * 8u + col * 2u]) = make_double2(c[m][n][0], c[m][n][1]);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kMt * kNt * 64u; i += kWarps * 32u) {
-        const uint32_t tile = i >> 6, at = i & 63u;
-        double sum = s_c[0][tile][at];
-#pragma unroll
-        for (uint32_t w = 1; w < kWarps; ++w) sum += s_c[w][tile][at];
-        const uint32_t t = t0 + (tile / kNt) * 8u + (at >> 3), e = e0 + (tile % kNt) * 8u + (at & 7u);
-        if (t < n_tokens && e < n_experts) {
-            const float sc = router_score_f32(sum, score_fn);
-            scores[(size_t)t * n_experts + e] = sc;
-            select[(size_t)t * n_experts + e] = __fadd_rn(sc, bias ? __ldcg(bias + e) : 0.0f);
-        }
-    }
-}
-
-// One warp per token picks the routes from the scores.
-__global__ void __launch_bounds__(256)
-k_router_select_batch(const float *__restrict__ scores, const float *__restrict__ select, uint32_t n_experts, uint32_t n_tokens,
-                      uint32_t top_k, float route_scale, int32_t *__restrict__ ids_out, float *__restrict__ weights_out) {
-    const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    dependency_wait();   // (triggers behind the wait: the digits launch behind reads x without waiting for this kernel)
-    if (t >= n_tokens) return;
-    router_select(scores + (size_t)t * n_experts, select + (size_t)t * n_experts, n_experts, top_k, route_scale,
-                  ids_out + (size_t)t * top_k, weights_out + (size_t)t * top_k, nullptr, nullptr, nullptr, 0, threadIdx.x & 31u, 0,
-                  1, 0);
-}
-
-int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, cudaError_t *err) {
-    auto run = [&](auto kernel, uint32_t mt, uint32_t nt, uint32_t warps) {
-        return launch_pdl(kernel, dim3(ceil_div(r.n_experts, 8u * nt), ceil_div(r.n_tokens, 8u * mt)), dim3(warps * 32u), 0, st, 0u, r.x,
-                          r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
-    };
-    if (r.hidden % 512u) *err = cudaErrorInvalidValue;   // (a block object's hidden size)
-    // (up to 64 tokens the 8 x 8 tiles of sixteen warps fill the chip: 32 tokens of 4096, 256 experts 4.3 us, in 16 x 8 tiles 9.6)
-    else if (r.n_tokens <= 64u) *err = run(k_router_scores<1, 1, 16>, 1, 1, 16);
-    else if (ceil_div(r.n_tokens, 16u) * ceil_div(r.n_experts, 16u) < 296u) *err = run(k_router_scores<2, 1, 8>, 2, 1, 8);
-    else *err = run(k_router_scores<2, 2, 8>, 2, 2, 8);
-    if (*err != cudaSuccess) return 0;
-    *err = launch_pdl(k_router_select_batch, dim3(ceil_div(r.n_tokens, 8)), dim3(256), 0, st, 0u, (const float *)scores,
-                      (const float *)select, r.n_experts, r.n_tokens, r.top_k, r.route_scale, r.ids_out, r.weights_out);
-    return 2;
 }
 
 cudaError_t launch_stack_step(cudaStream_t st, const float *x, const float *y, float *out, float *y_copy,
