@@ -323,7 +323,7 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
         __syncthreads();
         if (!s_ok) return;
     }
-    if (n >= hidden || why) return;
+    if (n >= hidden) return;
     const size_t at = (size_t)t * kPairsPerToken * hidden + n;
     // (a caller's buffers may lie on any 4-byte boundary)
     auto load = [&](const float *p, float(&r)[kPer]) {
@@ -363,6 +363,7 @@ k_block_mix(const float *__restrict__ d, const int32_t *__restrict__ ids, const 
     constexpr uint32_t kSh = S14_EXPERTS_PER_TOKEN;
     if (has_shared) load_row(kSh, row[kSh]);
     if (residual) load(x + (size_t)t * hidden + n, in);
+    if (why) return;   // (behind the loads, which need not wait for it)
     float out[kPer];
 #pragma unroll
     for (uint32_t i = 0; i < kPer; ++i) {

@@ -306,7 +306,8 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
     cluster_barrier();   // the other CTA's barriers are there
     fence_after();
     const uint32_t tmem = tmem_slot;
-    dependency_wait();
+    // (the down kernel reads records and pages in front of its wait, see below)
+    if constexpr (!kDown) dependency_wait();
     const uint32_t R = (kDown ? (a.hidden >> 7) : (a.inter >> 6)) / 2u;   // items per chunk
     // The pair's items are q = me, me + n_pairs, ...  The chunks of one expert follow one another and so do their items, a row
     // tile's chunks side by side (so that pairs that run at the same time share the expert's units in the L2).
@@ -356,6 +357,30 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
             }
         }
         __syncthreads();
+        if constexpr (kDown) {
+            if (base == 0u) {
+                // The launch in front (the second digits launch) writes the tiles and exponents of the hidden values, but neither the
+                // records nor the pages; it lets this one start behind its own wait, so what is in front of it is complete.  So the items are
+                // decoded and the ring's units asked for while it runs (us: 4 tokens of 512 x 512 27.9, so 25.7, 8 of 2048 x 1024 45.0 and 44.2,
+                // 8 official ones 105.8 and 103.6; 370 tokens 0.5 %).
+                if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds && lane == 31u) {
+#pragma unroll 1
+                    for (uint32_t s = warp - kPProdWarp0; s < ring; s += kPProds) {
+                        const uint32_t i = s / nu, u = s - i * nu;
+                        if (i >= nb) break;
+                        const uint32_t nt = s_rec[i].nt & 0xFFu, half = (nt + 1u) >> 1, first = rank * half;
+                        const uint32_t mine = nt > first ? min(nt - first, half) : 0u, full = bar(kPBarFull + s);
+                        const uint8_t *const src = reinterpret_cast<const uint8_t *>(s_rec[i].page) + page_off +
+                                                   ((size_t)(s_rec[i].r * 2u + rank) * nu + u) * kUnitStride;
+                        mbar_arrive_expect(full, kStageA + mine * kTileB);
+                        if (s_rec[i].nt >> 8) bulk_copy(ring0 + s * stage, src, kStageA, full);
+                        else bulk_copy_stream(ring0 + s * stage, src, kStageA, full, once);
+                    }
+                }
+                __syncwarp();
+                dependency_wait();
+            }
+        }
 
         if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds) {
             // ---- a stage: the unit of this CTA's row tile, then the digit tiles of its half of the chunk ----
@@ -380,7 +405,9 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
                         ok = !round || stage_wait(bar(kPBarDone + slot), (round - 1u) & 1u, abortp);
                         if (!ok) break;
                         const uint32_t full = bar(kPBarFull + slot), dst = to + slot * stage;
-                        if (is_unit) {
+                        if (is_unit && kDown && !round) {
+                            // (asked for in front of the wait)
+                        } else if (is_unit) {
                             mbar_arrive_expect(full, kStageA + mine * kTileB);
                             // an expert with one chunk is read once; with more, its later chunks want the units in the L2
                             if (multi) bulk_copy(dst, src, kStageA, full);
