@@ -177,7 +177,7 @@ inline cudaError_t launch_status(cudaError_t e) {
 //
 // Four kernels read in front of their wait what the launch directly in front of them does not write, and may only follow a launch that
 // triggers behind its own wait, because then everything in front of that one is complete when they start: the first digits launch of a
-// block call (k_block_digits, early: reads x, writes digits), behind the launch that picks the routes or a copy; k_hc_reduce with kAhead (the streams),
+// block call (k_block_digits or its official form, early: reads x, writes digits), behind the launch that picks the routes or a copy; k_hc_reduce with kAhead (the streams),
 // behind k_hc_dots; k_fp8_expert_up (the token and its page; writes h), behind the layer kernel with a page `ahead`; the blocks' down kernel
 // (k_block_pair: records and pages), behind the second digits launch.  The layer kernel
 // without one copies pages, router rows and tables, which are constant during a step, in front of its wait.  k_hc_reduce, k_router and

@@ -27,8 +27,8 @@
 // other, so that the second and later chunks of an expert find its units in the L2.
 // With the official expert arithmetic
 // (fast16/research/polaris_meridian_v1/s14_first_real_token/executor.py:712-743) the same contractions run on
-// quantised inputs: k_block_digits quantises per 128 elements to E4M3FN values (which the digit rows hold
-// exactly), the up epilogue leaves BF16 gate and up projections, the second k_block_digits makes the hidden values of them
+// quantised inputs: k_block_digits_official quantises per 128 elements to E4M3FN values (which the digit rows hold
+// exactly), the up epilogue leaves BF16 gate and up projections, the second digits launch makes the hidden values of them
 // (SwiGLU, times the route's weight, BF16), the down epilogue
 // and the mix round to BF16.
 #include "s14_moe_block.cuh"
@@ -57,7 +57,7 @@ __device__ __forceinline__ float2 e4m3fn_round2(float a, float b) {
     return __half22float2(*reinterpret_cast<const __half2 *>(&h));
 }
 
-// The digit tiles and block exponents of n vectors of K elements (one CTA per vector).  With `quant` the
+// The digit tiles and block exponents of n vectors of K elements, a CTA per vector.  In the official arithmetic the
 // vector is first quantised as the official linears quantise their input
 // (l42_real_reference/l42_reference.py:389-403): per 128 elements amax = max(|x|, 1e-4), scale =
 // 2^ceil(log2(amax / 448)) (F32 quotient, the logarithm taken in double and rounded to F32), x / scale
@@ -71,10 +71,9 @@ __device__ __forceinline__ float2 e4m3fn_round2(float a, float b) {
 // a chunk 1000 tokens made 408 chunks, so 334.
 // With `slots` the vectors are the pairs' gate and up projections and the hidden values are made of them here, element by element over
 // the whole chip: in the up kernel's epilogue they stood in the way of the next item (see s14_moe_pair.cu).
-template <bool kQuant>
 __global__ void __launch_bounds__(512)
-k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early,
-               const uint8_t *__restrict__ slots, const float *__restrict__ weights, uint32_t top_k) {
+k_block_digits_official(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early,
+                        const uint8_t *__restrict__ slots, const float *__restrict__ weights, uint32_t top_k) {
     const uint32_t v = blockIdx.x, g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
     // early: the launch in front neither writes x nor uses what is written here (it picks the routes), and whatever is in front
     // of it is complete when this kernel starts, because it lets this one start behind its own wait (a launch that triggers in
@@ -82,7 +81,7 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
     if (!early) dependency_wait();
     float xs[8];
     uint32_t place = 0u;   // the form that the pair's digit tile takes
-    if (kQuant && slots) {
+    if (slots) {
         place = __ldcg(slots + v) & 3u;
         // the hidden values of pair v from its gates and up projections (s14_first_real_token/executor.py:712-743): the limited SwiGLU
         // in F32, times the route's weight (not for the shared expert), rounded to BF16
@@ -106,40 +105,58 @@ k_block_digits(const float *__restrict__ x, uint32_t K, uint8_t *__restrict__ di
         const float4 p1 = __ldcg(reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g + 1u);
         xs[0] = p0.x, xs[1] = p0.y, xs[2] = p0.z, xs[3] = p0.w, xs[4] = p1.x, xs[5] = p1.y, xs[6] = p1.z, xs[7] = p1.w;
     }
-    if constexpr (kQuant) {
-        // a group of 128 elements is sixteen neighbouring threads
-        float am = 0.0f;
+    // a group of 128 elements is sixteen neighbouring threads
+    float am = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(xs[i]));
+    for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(xs[i]));
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-        am = fmaxf(am, 1e-4f);
-        // (where the quotient is well above a power of two the logarithm's F32 value lies between the two integers)
-        const float quot = __fdiv_rn(am, 448.0f);
-        const uint32_t bits = __float_as_uint(quot);   // (normal: am is at least 1e-4)
-        int e = (int)(bits >> 23) - 126;
-        if ((bits & 0x7FFFFFu) < 128u) e = (int)ceilf((float)log2((double)quot));
-        e = e < -126 ? -126 : (e > 126 ? 126 : e);
-        const float scale = __uint_as_float((uint32_t)(127 + e) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    for (int o = 8; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    am = fmaxf(am, 1e-4f);
+    // (where the quotient is well above a power of two the logarithm's F32 value lies between the two integers)
+    const float quot = __fdiv_rn(am, 448.0f);
+    const uint32_t bits = __float_as_uint(quot);   // (normal: am is at least 1e-4)
+    int e = (int)(bits >> 23) - 126;
+    if ((bits & 0x7FFFFFu) < 128u) e = (int)ceilf((float)log2((double)quot));
+    e = e < -126 ? -126 : (e > 126 ? 126 : e);
+    const float scale = __uint_as_float((uint32_t)(127 + e) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            const float2 q = e4m3fn_round2(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f), fminf(fmaxf(__fmul_rn(xs[i + 1], inv), -448.0f), 448.0f));
-            xs[i] = __fmul_rn(q.x, scale);
-            xs[i + 1] = __fmul_rn(q.y, scale);
-        }
+    for (int i = 0; i < 8; i += 2) {
+        const float2 q = e4m3fn_round2(fminf(fmaxf(__fmul_rn(xs[i], inv), -448.0f), 448.0f), fminf(fmaxf(__fmul_rn(xs[i + 1], inv), -448.0f), 448.0f));
+        xs[i] = __fmul_rn(q.x, scale);
+        xs[i + 1] = __fmul_rn(q.y, scale);
     }
-    if constexpr (kQuant) {
-        uint32_t words[6];
-        digits6_of8(xs, g, words, exps + (size_t)v * (K >> 5));
-        const uint32_t kb = g >> 2, forms = slots ? 1u : 4u;
-        for (uint32_t i = 0; i < forms; ++i) {
-            const uint32_t form = slots ? place : i;
-            uint8_t *const chunk = dig + ((size_t)(v * forms + i) * (K >> 8) + (kb >> 3)) * 768u + (g & 3u) * 4u;
+    uint32_t words[6];
+    digits6_of8(xs, g, words, exps + (size_t)v * (K >> 5));
+    const uint32_t kb = g >> 2, forms = slots ? 1u : 4u;
+    for (uint32_t i = 0; i < forms; ++i) {
+        const uint32_t form = slots ? place : i;
+        uint8_t *const chunk = dig + ((size_t)(v * forms + i) * (K >> 8) + (kb >> 3)) * 768u + (g & 3u) * 4u;
 #pragma unroll
-            for (uint32_t j = 0; j < 6; ++j)
-                *reinterpret_cast<uint32_t *>(chunk + j * 128u + (((kb & 7u) ^ ((6u * form + j) & 7u)) << 4)) = words[j];
+        for (uint32_t j = 0; j < 6; ++j)
+            *reinterpret_cast<uint32_t *>(chunk + j * 128u + (((kb & 7u) ^ ((6u * form + j) & 7u)) << 4)) = words[j];
+    }
+    if (early) dependency_wait();
+}
+
+// F32 arithmetic.  A CTA takes vectors blockIdx.x, + gridDim.x, ... with the next one's loads in flight: with a CTA per vector, as above, a launch
+// is its CTAs' latency - being started, a trip to the L2, code that is new to the SM, shuffles - times the rounds of what fits beside one
+// another (45 tokens of 2048 x 1536 120.2 us for the call, so 118.8, 100 of 2048 x 1024 89.4 and 87.9).  The official form gains nothing by it:
+// there the instructions count, and the loop's registers cost more (8 tokens 106.0 -> 108.5).  Kept to 40 registers (64 here) this one spills
+// and gains nothing.
+constexpr uint32_t kDigitThreads = 1024;   // of an SM, in CTAs of K / 8 (1536 and 2048 are as fast)
+__global__ void __launch_bounds__(512)
+k_block_digits(const float *__restrict__ x, uint32_t n, uint32_t K, uint8_t *__restrict__ dig, uint8_t *__restrict__ exps, uint32_t early) {
+    const uint32_t g = threadIdx.x;   // K / 8 threads: whole warps, K is a multiple of 256
+    if (!early) dependency_wait();   // (early: as above)
+    auto row = [&](uint32_t v) { return reinterpret_cast<const float4 *>(x + (size_t)v * K) + 2u * g; };
+    float4 p0 = __ldcg(row(blockIdx.x)), p1 = __ldcg(row(blockIdx.x) + 1);
+#pragma unroll 1
+    for (uint32_t v = blockIdx.x; v < n; v += gridDim.x) {
+        const float xs[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+        if (v + gridDim.x < n) {
+            p0 = __ldcg(row(v + gridDim.x));
+            p1 = __ldcg(row(v + gridDim.x) + 1);
         }
-    } else {
         digits_of8(xs, g, dig + (size_t)v * (K >> 8) * 2048u, exps + (size_t)v * (K >> 5));
     }
     if (early) dependency_wait();
@@ -431,8 +448,13 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     // reads or writes anything.
     auto digits = [&](const float *v, uint32_t n, uint32_t K, uint8_t *dig, uint8_t *exps, bool early) {
         if (*err != cudaSuccess) return;
-        *err = launch_pdl(official ? k_block_digits<true> : k_block_digits<false>, dim3(n), dim3(K >> 3), 0, st, 0u, v, K, dig, exps,
-                          early ? 1u : 0u, early ? (const uint8_t *)nullptr : (const uint8_t *)w.slots, weights, top_k);
+        const uint32_t threads = K >> 3;
+        if (official)
+            *err = launch_pdl(k_block_digits_official, dim3(n), dim3(threads), 0, st, 0u, v, K, dig, exps, early ? 1u : 0u,
+                              early ? (const uint8_t *)nullptr : (const uint8_t *)w.slots, weights, top_k);
+        else
+            *err = launch_pdl(k_block_digits, dim3(std::min(n, (uint32_t)sm_count * (kDigitThreads / threads))), dim3(threads), 0, st, 0u, v, n, K, dig,
+                              exps, early ? 1u : 0u);
     };
     *err = cudaSuccess;
     // (in front of it: the router's launch, or the copies of the host's routes)
