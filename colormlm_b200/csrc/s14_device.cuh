@@ -97,6 +97,27 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// The sums of P values (a power of two up to 32) over a warp, each added in warp_sum's order: a lane gives away half of the values it
+// holds at every step, so 16 values take 16 exchanges where warp_sum takes 5 each.  Lane l returns value l / (32 / P)'s.
+template <uint32_t P>
+__device__ __forceinline__ double warp_sums(double (&v)[P], uint32_t lane) {
+    static_assert(P >= 1u && P <= 32u && (P & (P - 1u)) == 0u, "a power of two");
+    uint32_t o = 16u;
+#pragma unroll
+    for (uint32_t half = P / 2u; half > 0u; half >>= 1, o >>= 1) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (uint32_t i = 0; i < half; ++i) {
+            const double give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    double sum = v[0];
+#pragma unroll
+    for (; o > 0u; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
 // The reference's SwiGLU (examples/s14_vulkan_numeric.rs:1543-1556) in F32 with
 // separate operations.  expf is evaluated in double and rounded once, which
 // reproduces a correctly rounded expf.  The F32 quotient g / (1 + e) is taken in double and rounded

@@ -16,7 +16,7 @@
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
-#include "s14_device.cuh"
+#include "s14_umma.cuh"
 
 namespace s14 {
 
@@ -110,14 +110,42 @@ __device__ __forceinline__ void load_coefficients(float *s_coef, const float *sc
     if (tid < (kHead ? kHc : kMixMax)) s_coef[3u + tid] = __ldcg(base + tid);
 }
 
-// hc.py:19-84 by one warp: 24 logits -> pre [4], post [4], comb [4][4], F32 in the reference's order.  Lane
-// l < 16 owns comb[l / 4][l % 4]; a row's or column's four values are fetched with shuffles and added in
-// index order, as the Python sums do; lanes 0-3 also make pre and post.  All 32 lanes call it.
-__device__ __forceinline__ void split_sinkhorn_warp(const float *mixes, const float *scale, const float *base, uint32_t iters,
-                                                    float eps, uint32_t lane, float &pre, float &post, float &comb) {
-    const uint32_t l = lane & 15u, i = l >> 2, j = l & 3u, h = lane & 3u;
-    pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(mixes[h], scale[0]), base[h])), eps);
-    post = __fmul_rn(2.0f, sigmoid_f32(__fadd_rn(__fmul_rn(mixes[kHc + h], scale[1]), base[kHc + h])));
+// a / s rounded to nearest, by Markstein's method (IBM Journal of Research and Development 34, 1990): a reciprocal y with its error taken
+// out once, q = a y, and q corrected by y times the remainder a - q s, which a fused multiply-add gives exactly.  For positive numbers from 2^-60
+// to 2^60 (from_range below kInRange), where nothing on the way leaves the range of normal numbers.  The division operator looks
+// at its operands first and costs a serial chain twice as much.
+__device__ __forceinline__ float quotient(float a, float s) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    y = __fmaf_rn(__fmaf_rn(-s, y, 1.0f), y, y);
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-s, q, a), y, q);
+}
+constexpr uint32_t kInRange = 120u << 23;
+__device__ __forceinline__ uint32_t from_range(float v) { return __float_as_uint(v) - (67u << 23); }
+
+// hc.py:19-84: 24 logits -> pre [4], post [4], comb [4][4], F32 in the reference's order, in two warps, as comb is a chain several
+// times as long as the rest.  Both make the logits of the sums (lane m: row m's; lane n_mix: the sum of squares) and leave them in a row of
+// shared memory of their own.
+template <bool kHead>
+__device__ __forceinline__ void mix_logits(double sum, uint32_t n, float norm_eps, uint32_t lane, float *s_mix) {
+    constexpr uint32_t n_mix = kHead ? kHc : kMixMax;
+    const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, sum, n_mix) / (double)n), norm_eps);
+    if (lane < n_mix) s_mix[lane] = __fmul_rn((float)sum, rs);
+    __syncwarp();
+}
+// lanes 0 .. 3
+__device__ __forceinline__ float pre_of(const float *mixes, const float *scale, const float *base, float eps, uint32_t lane) {
+    return __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(mixes[lane], scale[0]), base[lane])), eps);
+}
+__device__ __forceinline__ float post_of(const float *mixes, const float *scale, const float *base, uint32_t lane) {
+    return __fmul_rn(2.0f, sigmoid_f32(__fadd_rn(__fmul_rn(mixes[kHc + lane], scale[1]), base[kHc + lane])));
+}
+// comb by a warp: lane l < 16 owns comb[l / 4][l % 4]; a row's or column's four values are fetched with shuffles and added in
+// index order, as the Python sums do.  All 32 lanes call it.
+__device__ __forceinline__ float sinkhorn_warp(const float *mixes, const float *scale, const float *base, uint32_t iters, float eps,
+                                               uint32_t lane) {
+    const uint32_t l = lane & 15u, i = l >> 2, j = l & 3u;
     float c = __fadd_rn(__fmul_rn(mixes[2 * kHc + l], scale[2]), base[2 * kHc + l]);
     auto row_sum = [&](float v, bool is_max) {
         const float r0 = __shfl_sync(0xffffffffu, v, i * 4u), r1 = __shfl_sync(0xffffffffu, v, i * 4u + 1u);
@@ -132,13 +160,25 @@ __device__ __forceinline__ void split_sinkhorn_warp(const float *mixes, const fl
     };
     // stable row softmax, + eps
     c = (float)exp((double)__fsub_rn(c, row_sum(c, true)));
-    c = __fadd_rn(__fdiv_rn(c, row_sum(c, false)), eps);
+    const float first = __fadd_rn(__fdiv_rn(c, row_sum(c, false)), eps);   // (may be as small as eps, and the quotient a zero)
+    auto rounds = [&](auto divide) {
+        c = first;
+        if (iters) c = divide(c, __fadd_rn(col_sum(c), eps));
 #pragma unroll 1
-    for (uint32_t it = 0; it < iters; ++it) {
-        if (it) c = __fdiv_rn(c, __fadd_rn(row_sum(c, false), eps));
-        c = __fdiv_rn(c, __fadd_rn(col_sum(c), eps));
-    }
-    comb = c;
+        for (uint32_t it = 1; it < iters; ++it) {
+            c = divide(c, __fadd_rn(row_sum(c, false), eps));
+            c = divide(c, __fadd_rn(col_sum(c), eps));
+        }
+    };
+    // 2 x 20 half rounds one after the other: 142 clocks each with the division operator, 108 so.  A value out of `quotient`'s range on the
+    // way (an eps far below 1e-18, an infinity): once more with the operator.
+    uint32_t out = 0u;
+    rounds([&](float a, float d) {
+        out = max(out, max(from_range(a), from_range(d)));
+        return quotient(a, d);
+    });
+    if (__any_sync(0xffffffffu, out >= kInRange)) rounds([](float a, float d) { return __fdiv_rn(a, d); });
+    return c;
 }
 
 // sum_h pre[h] v[h] in stream order
@@ -161,13 +201,25 @@ __device__ __forceinline__ void reduce_streams(const void *x, size_t x0, uint32_
     sum_streams<N>(v, pre, acc);
 }
 
+// `v` to the same shared-memory variable of CTA `r` of the cluster, counted in bytes on its barrier
+__device__ __forceinline__ void store_counted(uint32_t at, uint32_t bar, uint32_t r, double v) {
+    asm volatile(
+        "{\n.reg .b32 a, b;\n"
+        "mapa.shared::cluster.u32 a, %0, %2;\n"
+        "mapa.shared::cluster.u32 b, %1, %2;\n"
+        "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [a], %3, [b];\n}" ::"r"(at),
+        "r"(bar), "r"(r), "l"(__double_as_longlong(v))
+        : "memory");
+}
+
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
 // only) of few tokens: one cluster of sixteen CTAs per token (the head fewer for more tokens: launch_hc_pre).  The call is all
 // latency: 1.5 MB of fn per token, then a serial chain of 20 Sinkhorn rounds.  Every CTA takes its share of the
 // flattened streams against all rows of fn (98 KB, all loads in flight together), the partial sums cross in
 // shared memory, every CTA makes the coefficients itself and reduces its share of the hidden vector: no scratch, no second
-// launch, no vote.  One token of 4096, calls one after another: 10.9 us in the two launches of then, 8.2 now (as the two launches of
-// today: launch_hc_pre).
+// launch, no vote.  One token of 4096, calls one after another: 10.9 us in the two launches of then, 8.1 with clusters, 5.9 now.  Marks of the 8.1,
+// in clocks: start and cluster barrier 1200, rows and products 3550, the warps' sums 2100, their exchange 1700, logits and pre 1400, comb
+// 6400 (20 Sinkhorn rounds of one warp); now 1200, 3050, 350, 1400, and comb 5700 straight behind its logits, with pre beside it.
 constexpr uint32_t kPreThreads = 512;
 template <bool kBf16, bool kHead, uint32_t kCluster>
 __global__ void __launch_bounds__(kPreThreads)
@@ -177,20 +229,27 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     constexpr uint32_t n_mix = kHead ? kHc : kMixMax, kRows = n_mix / 2u;   // rows per half of the CTA
     __shared__ double s_warp[kPreThreads / 32][kRows + 1];
     __shared__ double s_part[kCluster][n_mix + 1];                      // [n_mix]: the sum of squares
-    __shared__ float s_mix[n_mix], s_pre[kHc], s_coef[3 + n_mix];            // [3 + n_mix]: scale, base
+    __shared__ float s_mix[2][n_mix], s_pre[kHc], s_coef[3 + n_mix];         // [3 + n_mix]: scale, base
+    __shared__ __align__(8) uint64_t s_bar;                                  // all CTAs' sums are in s_part
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), t = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t n = kHc * hidden, share = n / kCluster, k0 = rank * share;   // a multiple of 64
     const uint32_t half = tid >> 8, c = tid & 255u;                          // half of the rows, column of four elements
-    double acc[kRows], ss = 0.0;
+    constexpr uint32_t kSums = kHead ? 4u : 16u;   // the rows of a half and the squares, rounded up
+    double acc[kSums], ss = 0.0;
 #pragma unroll
-    for (uint32_t m = 0; m < kRows; ++m) acc[m] = 0.0;
+    for (uint32_t m = 0; m < kSums; ++m) acc[m] = 0.0;
     float4 f[kRows];
     auto fetch = [&](uint32_t i) {
 #pragma unroll
         for (uint32_t m = 0; m < kRows; ++m) f[m] = __ldcg(reinterpret_cast<const float4 *>(fn + (size_t)(half * kRows + m) * n + k0 + i));
     };
-    cluster.sync();  // every CTA of the cluster runs: its shared memory may be written
+    if (tid == 0u) {
+        mbar_init(smem_u32(&s_bar), 1u);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_arrive_expect(smem_u32(&s_bar), kCluster * (n_mix + 1u) * (uint32_t)sizeof(double));
+    }
+    cluster.barrier_arrive();
     dependency_wait();
     if (c * 4u < share) fetch(c * 4u);
     load_coefficients<kHead>(s_coef, scale, base, tid);
@@ -210,49 +269,58 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
         for (uint32_t m = 0; m < kRows; ++m) acc[m] += (d0 * (double)f[m].x + d1 * (double)f[m].y) + (d2 * (double)f[m].z + d3 * (double)f[m].w);
         if (half == 0u) ss += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
     }
-#pragma unroll
-    for (uint32_t m = 0; m < kRows; ++m) {
-        acc[m] = warp_sum(acc[m]);
-        if (lane == 0u) s_warp[warp][m] = acc[m];
-    }
-    ss = warp_sum(ss);
-    if (lane == 0u) s_warp[warp][kRows] = ss;
+    // (thirteen values by five exchanges each, 130 shuffles a warp and sixteen warps, were a microsecond of the chain)
+    acc[kRows] = ss;
+    const double sum = warp_sums(acc, lane);
+    constexpr uint32_t kLanes = 32u / kSums;
+    if (lane % kLanes == 0u && lane / kLanes <= kRows) s_warp[warp][lane / kLanes] = sum;
     __syncthreads();
+    cluster.barrier_wait();  // every CTA of the cluster runs: its shared memory may be written
     if (tid <= n_mix) {
         const uint32_t w0 = tid < n_mix ? (tid / kRows) * 8u : 0u, m = tid < n_mix ? tid % kRows : kRows;
         double s = 0.0;
 #pragma unroll
         for (uint32_t w = 0; w < 8u; ++w) s += s_warp[w0 + w][m];
+        // counted stores: a barrier of the cluster behind plain ones takes 1200 clocks
 #pragma unroll
-        for (uint32_t r = 0; r < kCluster; ++r) *cluster.map_shared_rank(&s_part[rank][tid], r) = s;
+        for (uint32_t r = 0; r < kCluster; ++r) store_counted(smem_u32(&s_part[rank][tid]), smem_u32(&s_bar), r, s);
     }
-    cluster.sync();
-    if (warp == 0u) {
-        double s = 0.0;
+    const uint32_t part = hidden / kCluster;   // a multiple of 16
+    const bool comb_here = !kHead && rank == 0u;
+    // (a CTA leaves when all sums have come, so none is stored into one that has left; sums that do not come make it a NaN)
+    bool come = true;
+    if (warp == 0u || warp == 1u) {
+        uint32_t tries = 0;
+        while (!(come = mbar_try(smem_u32(&s_bar), 0u)) && ++tries < kSpin) {
+        }
+        come = __all_sync(0xffffffffu, come);
+    }
+    if (warp == 1u || (warp == 0u && comb_here)) {
+        double s = come ? 0.0 : __longlong_as_double(-1ll);
         if (lane <= n_mix) {
 #pragma unroll
             for (uint32_t r = 0; r < kCluster; ++r) s += s_part[r][lane];
         }
-        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, n_mix) / (double)n), norm_eps);
-        if (lane < n_mix) s_mix[lane] = __fmul_rn((float)s, rs);
-        __syncwarp();
-        // pre first: the other warps reduce the streams while this one of the first CTA goes on to post and comb
-        if (lane < kHc) {
-            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
-            s_pre[lane] = pre;
-            if (pre_out && rank == 0u) pre_out[(size_t)t * kHc + lane] = pre;
+        mix_logits<kHead>(s, n, norm_eps, lane, s_mix[warp]);
+    }
+    if (warp == 0u) {
+        // comb, while the others go on; this warp has no part of the streams
+        if (comb_here) {
+            const float comb = sinkhorn_warp(s_mix[0], s_coef, s_coef + 3, iters, hc_eps, lane);
+            if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
         }
+        return;
     }
-    __syncthreads();
-    const uint32_t part = hidden / kCluster;   // a multiple of 16
-    if (!kHead && rank == 0u && warp == 0u) {
-        float pre, post, comb;
-        split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
-        if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
-        if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
+    if (warp == 1u && lane < kHc) {
+        const float pre = pre_of(s_mix[1], s_coef, s_coef + 3, hc_eps, lane);
+        s_pre[lane] = pre;
+        if (pre_out && rank == 0u) pre_out[(size_t)t * kHc + lane] = pre;
     }
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(kPreThreads - 32u) : "memory");
+    if (!kHead && rank == 0u && warp == 1u && lane < kHc) post_out[(size_t)t * kHc + lane] = post_of(s_mix[1], s_coef, s_coef + 3, lane);
     const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
-    // the last threads, so that the warp with the Sinkhorn rounds has none of it
+    // (the last threads: rows of up to 30 K elements times the cluster leave the first warp out)
     for (uint32_t i = (kPreThreads - 1u - tid) * 8u; i < part; i += kPreThreads * 8u) {
         float v[8];
         reduce_streams<kBf16, 8>(x, (size_t)t * n, hidden, rank * part + i, pre, v, vec != 0u);
@@ -337,7 +405,8 @@ k_hc_dots(const void *__restrict__ x, const float *__restrict__ fn, uint32_t n, 
 
 // One CTA per token: the coefficients from the partial sums (one warp), then the reduced vector.  All latency: the slices' sums
 // (added one after the other by one warp, four loads in flight, they were half of a call of 20 tokens: 10.5 us, now 8.1), the
-// coefficients, the streams.  kAhead: a thread reads its first N values of every stream in front of the wait for the sums (the rule
+// coefficients, the streams (a call of 20 tokens of 4096 8.2 us, 7.0 with comb in a warp of its own and its rounds shorter, 370 tokens 20.1 and
+// 19.0).  kAhead: a thread reads its first N values of every stream in front of the wait for the sums (the rule
 // is the launch's).
 template <bool kBf16, bool kHead, int N, bool vec, bool kAhead>
 __global__ void __launch_bounds__(256)
@@ -346,7 +415,7 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
             float *__restrict__ post_out, float *__restrict__ comb_out, float *__restrict__ pre_out) {
     constexpr uint32_t kMix = kHead ? kHc : kMixMax;
     __shared__ double s_sum[8][kMix + 1];
-    __shared__ float s_pre[kHc], s_mix[kMix], s_coef[3 + kMix];
+    __shared__ float s_pre[kHc], s_mix[2][kMix], s_coef[3 + kMix];
     // k_hc_dots in front of this launch has waited, so everything in front of that kernel is complete: the launch behind may be
     // set up at once, and the streams may be read in front of the wait for the sums.
     cudaTriggerProgrammaticLaunchCompletion();
@@ -373,29 +442,28 @@ k_hc_reduce(const void *__restrict__ x, const double *__restrict__ partial, uint
     }
     if (warp == 0u) load_coefficients<kHead>(s_coef, scale, base, lane);
     __syncthreads();
-    if (warp == 0u) {
+    constexpr uint32_t kPreWarp = kHead ? 0u : 1u;
+    if (warp <= kPreWarp) {
         double s = 0.0;
         if (lane <= kMix) {
 #pragma unroll
             for (uint32_t w = 0; w < 8u; ++w) s += s_sum[w][lane];
         }
-        const float rs = rsqrt_of((float)(__shfl_sync(0xffffffffu, s, kMix) / (double)(kHc * hidden)), norm_eps);
-        if (lane < kMix) s_mix[lane] = __fmul_rn((float)s, rs);
-        __syncwarp();
-        if (lane < kHc) {
-            const float pre = __fadd_rn(sigmoid_f32(__fadd_rn(__fmul_rn(s_mix[lane], s_coef[0]), s_coef[3 + lane])), hc_eps);
-            s_pre[lane] = pre;
-            if (kHead) pre_out[(size_t)t * kHc + lane] = pre;
-        }
+        mix_logits<kHead>(s, kHc * hidden, norm_eps, lane, s_mix[warp]);
     }
-    __syncthreads();
     if (!kHead && warp == 0u) {  // the other warps reduce the streams meanwhile
-        float pre, post, comb;
-        split_sinkhorn_warp(s_mix, s_coef, s_coef + 3, iters, hc_eps, lane, pre, post, comb);
-        if (lane < kHc) post_out[(size_t)t * kHc + lane] = post;
+        const float comb = sinkhorn_warp(s_mix[0], s_coef, s_coef + 3, iters, hc_eps, lane);
         if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
         return;
     }
+    if (warp == kPreWarp && lane < kHc) {
+        const float pre = pre_of(s_mix[kPreWarp], s_coef, s_coef + 3, hc_eps, lane);
+        s_pre[lane] = pre;
+        if (kHead) pre_out[(size_t)t * kHc + lane] = pre;
+    }
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(256u - kFirst) : "memory");
+    if (!kHead && warp == kPreWarp && lane < kHc) post_out[(size_t)t * kHc + lane] = post_of(s_mix[kPreWarp], s_coef, s_coef + 3, lane);
     const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
     if constexpr (kAhead) {
         if (d < hidden) {
@@ -653,9 +721,9 @@ int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t 
     using U = uint32_t;
     const uint32_t sms = (uint32_t)sm_count;
     if (!head) {
-        // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together (4096, us: one token 8.2, seven 8.4, the
-        // two launches 8.2 and 8.3, on the host one launch more; 7168 9.1 and 9.4, 9.5 and 9.7).  Fourteen clusters of eight took
-        // 9.7 for fourteen tokens, the two launches 8.3 (7168 11.3 and 9.7).
+        // A CTA with 24 rows fills an SM: on 148 SMs seven clusters of sixteen run together (4096, us: one token 5.9, seven 6.0, the
+        // two launches of eight tokens 6.9).  Fourteen clusters of eight took
+        // 9.7 for fourteen tokens, the two launches 8.3 (7168 11.3 and 9.7; both before what is a microsecond and more faster now).
         if (hc_pre_in_clusters(n_tokens, sms)) return of_size(std::false_type{}, std::integral_constant<U, 16>{});
         return of_size(std::false_type{}, std::integral_constant<U, 0>{});
     }

@@ -23,6 +23,38 @@ extern "C" int greedy(uint32_t cluster, const float *logits, uint32_t vocab, int
     return (int)(e != cudaSuccess ? e : s14::launch_pdl(s14::k_greedy_argmax, dim3(cluster), dim3(s14::kArgmaxThreads), 0, cudaStreamPerThread,
                                                          cluster, logits, vocab, result));
 }
+#elif defined(PART_QUOTIENT)
+#include "s14_glue.cu"
+namespace s14 {
+namespace {
+// Every mantissa of the divisor; dividends at random, next to ties (the product of the divisor and a number half way between two floats) and
+// next to whole quotients.  wrong[0]: quotients that are not the division operator's.
+__global__ void k_quotients(uint32_t rounds, unsigned long long *wrong) {
+    const uint32_t mantissa = blockIdx.x * 256u + threadIdx.x;
+    uint32_t state = mantissa * 2654435761u + 1u;
+    auto next = [&] { return state = state * 1664525u + 1013904223u, (state >> 16 ^ state) * 2654435769u; };
+    unsigned long long n = 0;
+    for (uint32_t k = 0; k < rounds; ++k) {
+        const int scale = (int)(next() % 100u) - 50;
+        const float s = ldexpf(__uint_as_float(0x3F800000u | mantissa), scale);
+        const float m = __uint_as_float(0x3F800000u | (next() & 0x7FFFFFu));
+        const double tie = (double)m + ((k & 1u) ? 0x1p-24 : 0.0);
+        const float near = (float)((double)s * tie);
+        for (int step = -2; step <= 2; ++step) {
+            const float a = __uint_as_float(__float_as_uint(near) + step);
+            n += __float_as_uint(quotient(a, s)) != __float_as_uint(__fdiv_rn(a, s));
+        }
+        const float a = ldexpf(m, (int)(next() % 60u) - 30);
+        n += __float_as_uint(quotient(a, s)) != __float_as_uint(__fdiv_rn(a, s));
+    }
+    if (n) atomicAdd(wrong, n);
+}
+}  // namespace
+}  // namespace s14
+extern "C" int quotients(uint32_t rounds, unsigned long long *wrong) {
+    s14::k_quotients<<<(1 << 23) / 256, 256, 0, cudaStreamPerThread>>>(rounds, wrong);
+    return (int)cudaGetLastError();
+}
 #elif defined(PART_QUICK)
 #include "s14_moe_pair.cu"
 namespace s14 {

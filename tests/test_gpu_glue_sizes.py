@@ -181,3 +181,23 @@ def test_many_tokens_on_any_boundary(ctx, bf16, t, h):
         ctx.cmd_hc_post(_offset(branch, offset), _offset(res, offset), post, comb, got_m)
         ctx.cmd_rms_norm(_offset(branch, offset), _offset(nw, offset), got_n)
         assert torch.equal(got_m, want_m) and torch.equal(got_n, want_n)
+
+
+@pytest.mark.parametrize("n_tokens", [1, 20])
+@pytest.mark.parametrize("eps,spread,iters", [(1e-6, 120.0, 20), (1e-30, 1.0, 20), (1e-30, 50.0, 3), (1e-6, 1.0, 1)])
+def test_sinkhorn_rounds_of_any_values(ctx, oracle, n_tokens, eps, spread, iters):
+    """Logits whose softmax underflows, an epsilon out of the range of the rounds' own division (which then are done over with the operator), few
+    rounds: the oracle's coefficients."""
+    hidden = 512
+    g = synth.rng(91)
+    fn, scale, base = synth.hc_params(g, hidden)
+    base = (g.uniform(-1, 1, size=base.shape) * spread).astype(np.float32)
+    x = dev(synth.hc_streams(g, n_tokens, hidden))
+    red = torch.empty((n_tokens, hidden), device="cuda")
+    post, comb = torch.empty((n_tokens, 4), device="cuda"), torch.empty((n_tokens, 4, 4), device="cuda")
+    ctx.cmd_hc_pre(x, dev(fn), dev(scale), dev(base), red, post, comb, iters=iters, hc_eps=eps)
+    torch.cuda.synchronize()
+    r_ref, p_ref, c_ref = oracle.hc_pre(x.cpu().numpy(), fn, scale, base, iters=iters, hc_eps=eps)
+    close_coeff(post.cpu().numpy(), p_ref)
+    close_coeff(comb.cpu().numpy(), c_ref)
+    close_streams(red.cpu().numpy(), r_ref, False)

@@ -131,3 +131,11 @@ def test_what_the_fast_forms_settle_is_exact(part):
     swiglu, swiglu_wrong, sums, sums_wrong = counts.tolist()
     assert swiglu_wrong == 0 and sums_wrong == 0
     assert swiglu > 0.2 * 65536 * len(ups) * len(weights) and sums > 0.3 * 64 * 1024 * 256
+
+
+def test_the_sinkhorn_rounds_quotient_is_the_division_operators(part):
+    """Every mantissa of the divisor, dividends at random and next to ties: 1.2e9 quotients."""
+    lib, wrong = part("QUOTIENT"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    assert lib.quotients(24, ptr(wrong)) == 0
+    torch.cuda.synchronize()
+    assert int(wrong) == 0
