@@ -39,11 +39,21 @@ namespace {
 
 // A chunk's B operand is made of groups of sixteen digit rows: one token each; in the official arithmetic,
 // whose values need six digit rows, the tokens' rows follow one another.  Most groups of a chunk:
-constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens: most experts have one, and short stages make the ring deep
-constexpr uint32_t kGrpSparse = 6;   // fewer than three pairs (official arithmetic: six) per expert on average
+constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens
+constexpr uint32_t kGrpSparse = 6;
 constexpr uint32_t kGrpDense = 12;
-// (Both bounds, and the one of twelve tokens, were found with one-CTA kernels that had other stages; on the pair kernel, whose
-// rings hold eight, eight and seven stages, the three sizes have not been compared with each other.)
+// F32, us with 2 / 6 / 12 (256 experts of 4096 x 2048 unless said; 4 and 8 lie in between): 1 token 41.6 / 43.7 / 45.2, 4 71.9 / 75.9 / 76.2,
+// 8 109.2 / 108.7 / 110.1, 12 141.5 / 138.6 / 136.4, 13 149.5 / 147.1 / 145.3, 32 248 / 236.6 / 234.8, 64 349 / 293.7 / 288.4, 128 576 / 388 / 362,
+// 370 1425 / 761 / 623, 1000 3619 / 1703 / 1319.  With 6 / 12: 20 over 16 of 1024 x 512 31.1 / 34.8, 20 over 64 of 2048 x 1024 52.5 / 55.2,
+// 100 over 64 of 1024 x 512 56.9 / 58.7, 60 over 128 of 1024 x 512 47.0 / 51.2, 200 over 64 of 512 x 512 68.5 / 68.0, 50 over 128 of 2048 x 1024
+// 81.7 / 79.8, 370 over 256 of 1024 x 512 129.0 / 125.5, 45 over 192 of 2048 x 1536 118.8 / 117.2, 100 over 64 of 2048 x 1024 93.2 / 87.8.  So: the
+// kernels for twelve pass over an expert less often, but need the registers in which the next launch's CTAs would be set up, some three
+// microseconds for the call; they pay from 2^29 pairs x hidden x inter on (a page below 2^19 counted as that: an item's fixed part;
+// 200 over 64 of 512 x 512 by the product alone 69.7, so 67.6), where experts have a pair on average at least.
+constexpr uint64_t kDenseWork = 1ull << 29, kDensePage = 1ull << 19;
+// The official arithmetic's bound, six pairs per expert, was found with one-CTA kernels that had other stages; on the pair kernel its
+// sizes have not been compared.
+constexpr uint32_t kDenseOfficial = 6;
 static_assert(kBlockNt == kGrpDense * 8u / 6u * 2u, "a chunk record holds the tokens of the official arithmetic's chunks");
 
 // The nearest E4M3FN values (ties to even) of two numbers of magnitude 448 at most, as F32 values: the conversion there and back.
@@ -440,7 +450,9 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     const uint32_t tpg = official ? 2u : 1u;   // tokens per group of sixteen digit rows
     const bool small = n_tokens <= 12u;
     // (a group is sixteen operand rows: one token, official arithmetic six rows a token; half of a chunk's groups are one CTA's)
-    const uint32_t groups = small ? kGrpSmall : ((uint64_t)n_tokens * top_k >= (uint64_t)(3u * tpg) * n_experts ? kGrpDense : kGrpSparse);
+    const uint64_t pairs = (uint64_t)n_tokens * top_k;
+    const bool dense = official ? pairs >= (uint64_t)kDenseOfficial * n_experts : pairs >= n_experts && pairs * std::max((uint64_t)hidden * inter, kDensePage) >= kDenseWork;
+    const uint32_t groups = small ? kGrpSmall : (dense ? kGrpDense : kGrpSparse);
     const uint32_t S = inter >> 6, RT = hidden >> 7, counted = small ? 1u : 2u;   // slices, row tiles; as `counts` reports them
     const uint32_t cap = official ? groups * 8u / 6u * 2u : groups;   // tokens of a chunk: 4, 16, 32, or 2, 6, 12
     // The launches are programmatic dependents of one another: a kernel's blocks, barriers and tensor memory are

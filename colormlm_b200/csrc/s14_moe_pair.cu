@@ -325,6 +325,10 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
         }
     };
     const unsigned long long once = l2_policy_evict_first();
+    // (without an item the down kernel would end without having waited, and what is behind it would start beside the digits launch in front)
+    if constexpr (kDown) {
+        if (n_local == 0u) dependency_wait();
+    }
 
 #pragma unroll 1
     for (uint32_t base = 0; base < n_local; base += kPBatch) {
