@@ -261,9 +261,12 @@ __device__ __forceinline__ uint32_t half_rows(uint32_t nt) { return (((nt + 1u) 
 // official, one form and three: 8 tokens of 512 x 512 28.4 and 23.2, of 2048 x 1024, 64 experts, 48.6 and 42.2; one token of 4096 x 2048 47.0
 // and 40.3).  The forms for small chunks keep to 80 registers (said by a bound of 768 threads): with 96 the CTAs of the launch behind
 // find no room beside this one's, and are set up only when it ends (8 tokens 115 us, 96 registers and one F32 form 115-120, so 109.4; of
-// 2048 x 1024 49.0, 52, 45.0; one token 45.7, 46, 42.3).  Those for 12, 16 and 32 tokens would spill.
+// 2048 x 1024 49.0, 52, 45.0; one token 45.7, 46, 42.3).  So do the official up kernels of all sizes, with a few bytes spilled (us, 96 and
+// 80: 60 tokens over 32 of 1024 x 512 38.8 and 37.0, 20 over 64 of 2048 x 1024 55.9 and 54.3, 600 over 64 of 4096 x 2048 398 and 387, 1000 over
+// 256 763 and 750).  The official down kernels for 16 and 32 lose by it (300 over 64 of 2048 x 1024 101.2 and 103.8), and so do the F32 ones
+// for twelve (100 over 64 of 2048 x 1024 87.8: up 91.2, down 88.7).
 template <bool kDown, bool kOff, uint32_t kTok>
-__global__ void __launch_bounds__(kTok > (kOff ? 4u : 6u) ? kPThreads : 768u, 1)
+__global__ void __launch_bounds__(kTok > (kOff ? (kDown ? 4u : 32u) : 6u) ? kPThreads : 768u, 1)
 k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr uint32_t kRows = kOff ? 6u : 16u, kTileB = kRows * 128u;   // a token's digit rows, and the bytes of its tile
