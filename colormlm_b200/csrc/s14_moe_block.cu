@@ -51,9 +51,10 @@ constexpr uint32_t kGrpDense = 12;
 // microseconds for the call; they pay from 2^29 pairs x hidden x inter on (a page below 2^19 counted as that: an item's fixed part;
 // 200 over 64 of 512 x 512 by the product alone 69.7, so 67.6), where experts have a pair on average at least.
 constexpr uint64_t kDenseWork = 1ull << 29, kDensePage = 1ull << 19;
-// The official arithmetic's bound, six pairs per expert, was found with one-CTA kernels that had other stages; on the pair kernel its
-// sizes have not been compared.
-constexpr uint32_t kDenseOfficial = 6;
+// Official arithmetic, 6 / 12 groups (16 / 32 tokens): the same, from 2^30 on.  60 over 16 of 512 x 512 30.2 / 32.6, 20 over 64 of 2048 x 1024 53.8 / 55.5,
+// 40 over 32 of it 47.6 / 48.9, 150 over 128 of 1024 x 512 56.1 / 58.1, 45 over 192 of 2048 x 1536 116.4 / 116.2, 80 over 64 of 2048 x 1024 70.0 / 69.8,
+// 370 over 256 of 1024 x 512 83.1 / 83.6, 200 over 256 of 4096 x 2048 386 / 380, 300 over 64 of 2048 x 1024 108.6 / 99.4.
+constexpr uint64_t kDenseOfficial = 1ull << 30;
 static_assert(kBlockNt == kGrpDense * 8u / 6u * 2u, "a chunk record holds the tokens of the official arithmetic's chunks");
 
 // The nearest E4M3FN values (ties to even) of two numbers of magnitude 448 at most, as F32 values: the conversion there and back.
@@ -451,7 +452,7 @@ int launch_moe_block(cudaStream_t st, int sm_count, const BlockWork &w, const fl
     const bool small = n_tokens <= 12u;
     // (a group is sixteen operand rows: one token, official arithmetic six rows a token; half of a chunk's groups are one CTA's)
     const uint64_t pairs = (uint64_t)n_tokens * top_k;
-    const bool dense = official ? pairs >= (uint64_t)kDenseOfficial * n_experts : pairs >= n_experts && pairs * std::max((uint64_t)hidden * inter, kDensePage) >= kDenseWork;
+    const bool dense = pairs >= n_experts && pairs * std::max((uint64_t)hidden * inter, kDensePage) >= (official ? kDenseOfficial : kDenseWork);
     const uint32_t groups = small ? kGrpSmall : (dense ? kGrpDense : kGrpSparse);
     const uint32_t S = inter >> 6, RT = hidden >> 7, counted = small ? 1u : 2u;   // slices, row tiles; as `counts` reports them
     const uint32_t cap = official ? groups * 8u / 6u * 2u : groups;   // tokens of a chunk: 4, 16, 32, or 2, 6, 12

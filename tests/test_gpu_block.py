@@ -113,14 +113,14 @@ def test_block_at_the_other_sizes(ctx, oracle, hidden, inter):
 def test_block_of_every_chunk_form_and_odd_numbers_of_units(ctx, oracle, hidden, inter, official):
     """Items of 2, 6, 10 and 14 units of 256 elements (the scale codes are written two units at a time and fetched eight ahead, so
     items end in the middle of both), in the kernels for each of the three chunk sizes: blocks of 3 and 12 tokens, of 14 over many
-    experts, of 40 over few and of 200, whose chunks are full, partly filled and of odd size."""
+    experts, of 40 over few and of 240, whose chunks are full, partly filled and of odd size."""
     layer = oracle.official_moe_layer if official else oracle.moe_layer_acc64
     g, pages, shared = make_layer(1700 + hidden, hidden, inter, 8, L.PAGE_MXFP4)
     pages_dev, shared_dev = [dev_page(p, hidden, inter) for p in pages], dev_page(shared, hidden, inter)
-    blk = MoeBlock(ctx, hidden, inter, 200)
+    blk = MoeBlock(ctx, hidden, inter, 240)
     try:
         blk.set_semantics(official)
-        for n_tokens, n_experts in ((3, 8), (12, 8), (14, 48), (40, 8), (200, 48)):
+        for n_tokens, n_experts in ((3, 8), (12, 8), (14, 48), (40, 8), (240, 48)):
             x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(synth.activations(g, n_tokens, hidden)))
             wr, bias = dev(synth.router_weight_bf16(g, n_experts, hidden)), dev(synth.router_bias(g, n_experts))
             table = torch.tensor([pages_dev[e % 8].data_ptr() for e in range(n_experts)], dtype=torch.int64, device="cuda")
