@@ -285,14 +285,20 @@ __device__ __forceinline__ float near_score(float l, float err, uint32_t score_f
     return s;
 }
 
+// What k_router_near's logit may be off by, of |x| |w| (see k_router_pick).
+__host__ __device__ constexpr float near_bound(uint32_t hidden) { return 4.3e-6f + 3.37e-8f * (float)hidden; }
+
 // One CTA per token: the logits' parts are added, a bound on their error is made, and the experts that can be among the top_k are
 // scored in double, each warp an eighth of K; then the first warp picks.
 //
 // The bound.  S = |x| |w| (lengths of the rows) is no less than an expert's sum of |x_k w_k|.  What hi and lo leave of x moves a logit by
 // 2^-18 S at most.  A multiplication adds sixteen exact products to a sum in F32; whatever the order and the roundings in it, with 23 bits
-// kept of the largest of the seventeen terms it is off by 18 x 2^-23 of what the magnitudes so far add up to, of which a chain of n
-// multiplications meets half on average: n / 2 x 18 x 2^-23 S, where n = 2 x hidden / 8 / 16 <= 64 and the eight chains share S.  With the eight
-// sums' additions that is less than 2^-13.7 S; taken is 2^-13.5.  (Gaussian rows of 4096: 0.007 of a logit whose deviation is 1.3.)  Squares
+// kept of the largest of the seventeen terms it is off by 18 x 2^-23 of what the magnitudes so far add up to.  An eighth of K is a chain of
+// n = 2 x hidden / 8 / 16 multiplications, and where the row's magnitude lies in a chain's first elements all n of them meet all of it: n x 18 x
+// 2^-23 of the chain's part of S, so of S for the eight together, whose F32 sum adds 7 x 2^-24; hi and lo together are 1 + 2^-8 of x at most.
+// That is near_bound: 1.42e-4 for 4096, 2.2e-5 for 512.  (Half of the chain's magnitude in place of all of it, the mean for rows whose
+// magnitude is spread evenly, is no bound: with such a row the arithmetic described here is off by 1.2 times what that gives.)  Gaussian rows of
+// 4096: 0.012 of a logit whose deviation is 1.3.  Squares
 // that underflow are made up for by 2^-114; an S that is not finite, or a logit that is not, makes every expert a candidate.
 //
 // What it spends its time on, for a token alone on its SM and with two others beside it, in clocks: the parts and the token 1000 / 2000, scores and
@@ -346,7 +352,7 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
 #pragma unroll
     for (uint32_t w = 0; w < 8; ++w) x2 += s_sq[w];
     // (1.001: the sums' own roundings)
-    const float err = 8.65e-5f * sqrtf(__fmaf_rn(x2, 1.001f, 0x1p-114f)) * sqrtf(__fmaf_rn(w2, 1.001f, 0x1p-114f));
+    const float err = near_bound(hidden) * sqrtf(__fmaf_rn(x2, 1.001f, 0x1p-114f)) * sqrtf(__fmaf_rn(w2, 1.001f, 0x1p-114f));
     float off;
     const float s = near_score(logit, err, score_fn, off), sel = s + b;
     off += 0x1p-18f * (fabsf(s) + fabsf(b) + 0x1p-20f);   // the score's own evaluation and the roundings here

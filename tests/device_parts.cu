@@ -55,6 +55,15 @@ extern "C" int quotients(uint32_t rounds, unsigned long long *wrong) {
     s14::k_quotients<<<(1 << 23) / 256, 256, 0, cudaStreamPerThread>>>(rounds, wrong);
     return (int)cudaGetLastError();
 }
+#elif defined(PART_ROUTER)
+#include "s14_router.cu"
+extern "C" float near_bound(uint32_t hidden) { return s14::near_bound(hidden); }
+// parts: [8][n_tokens][256] sums of the approximate logits; scores, select: [n_tokens, 256]
+extern "C" int routes(const s14_router_desc *r, float *scores, float *select, float *parts) {
+    cudaError_t err;
+    s14::launch_router_batch(cudaStreamPerThread, *r, scores, select, parts, &err);
+    return (int)err;
+}
 #elif defined(PART_QUICK)
 #include "s14_moe_pair.cu"
 namespace s14 {
