@@ -1998,7 +1998,7 @@ static int32_t routed_block_router(s14_ctx *ctx, cudaStream_t st, s14_block *blk
     if (!rd->ids_out) rd->ids_out = blk->ids;
     if (!rd->weights_out) rd->weights_out = blk->weights;
     cudaError_t err;
-    ctx->launches += launch_router_batch(st, *rd, blk->scores, blk->select, blk->w.d, &err);
+    ctx->launches += launch_router_batch(st, *rd, blk->scores, blk->select, blk->w.d, ctx->status, &err);
     if (err != cudaSuccess) return cuda_fail(err, "S14 router launch");
     return S14_OK;
     S14_CATCH

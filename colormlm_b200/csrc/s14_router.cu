@@ -94,6 +94,9 @@ k_router_select_batch(const float *__restrict__ scores, const float *__restrict_
 // memory as they are ([8][token][256]) and meet in k_router_pick.  512 threads bring a stage of 64 k by copies three stages
 // ahead into the 128-byte swizzle of K-major operand tiles, the weights as they are (16 KB), the tokens to be split in place; one of them
 // issues the stage's eight multiplications.  It also leaves the sums of the weights' squares, for the bound.
+// A wait that runs out stops the CTA: the threads agree on it at the next barrier, nothing more is loaded or issued, logits and squares
+// become NaN (which sends their tokens to the scores in double, so the routes are right all the same), the status word is set, and tensor memory
+// goes back when the queued multiplications are complete.
 constexpr uint32_t kNearThreads = 512, kNearStages = 4, kNearSplit = 8, kNearK = 64, kNearTokens = 128, kNearW = 16384;
 
 // kind::f16: A and B BF16 (format 1), both K-major, F32 accumulators, M = 128, N = n (a multiple of 16)
@@ -127,7 +130,7 @@ __device__ __forceinline__ void copy_async_wait() {
 
 __global__ void __launch_bounds__(kNearThreads)
 k_router_near(const float *__restrict__ x, const uint16_t *__restrict__ wr, float *__restrict__ part, float *__restrict__ wsq,
-              uint32_t n_experts, uint32_t hidden, uint32_t n_tokens, uint32_t nt) {
+              uint32_t n_experts, uint32_t hidden, uint32_t n_tokens, uint32_t nt, uint32_t *status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[kNearStages];
     __shared__ uint32_t tmem_slot;
@@ -187,6 +190,7 @@ k_router_near(const float *__restrict__ x, const uint16_t *__restrict__ wr, floa
     float sq[2] = {0.0f, 0.0f};   // the squares of this thread's weights
     const uint32_t idesc = umma_idesc_bf16(nt);
     bool ok = true;
+    uint32_t issued = 0;
 #pragma unroll 1
     for (uint32_t c = 0; c < steps; ++c) {
         copy_async_wait<(int)kNearStages - 2>();   // this step's
@@ -223,7 +227,9 @@ k_router_near(const float *__restrict__ x, const uint16_t *__restrict__ wr, floa
             }
         }
         fence_async_smem();
-        __syncthreads();
+        ok = __syncthreads_and(ok);
+        if (!ok) break;
+        issued = c + 1u;
         if (warp == 0) {
             if (elect_one()) {
                 const uint32_t at0 = smem0 + (c % kNearStages) * stage;
@@ -238,21 +244,28 @@ k_router_near(const float *__restrict__ x, const uint16_t *__restrict__ wr, floa
             __syncwarp();
         }
         // the stage that step c + 3 takes is free when step c - 1 is complete
-        if (c >= 1u && c + kNearStages - 1u < steps) ok = mbar_wait(bar0 + ((c - 1u) % kNearStages) * 8u, ((c - 1u) / kNearStages) & 1u, &abort_flag) && ok;
-        load(c + kNearStages - 1u);
+        if (c >= 1u && c + kNearStages - 1u < steps) ok = mbar_wait(bar0 + ((c - 1u) % kNearStages) * 8u, ((c - 1u) / kNearStages) & 1u, &abort_flag);
+        if (ok) load(c + kNearStages - 1u);   // (a thread whose own wait has not run out: the stage is free)
     }
+    copy_async_wait<0>();
+    // all of the CTA's multiplications are complete, or none of its results count
+    const uint32_t last = issued - 1u;   // (the first step is always issued)
+    if (ok) ok = mbar_wait(bar0 + (last % kNearStages) * 8u, (last / kNearStages) & 1u, &abort_flag);
+    ok = __syncthreads_and(ok);
+    if (!ok) {
+        mbar_drain(bar0 + (last % kNearStages) * 8u, (last / kNearStages) & 1u);
+        if (tid == 0) atomicExch(status, 0x5509u);
+    }
+    fence_after();
     if (first_tile) {
 #pragma unroll
         for (uint32_t i = 0; i < 2; ++i) {
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
-            if (piece == 0u) wsq[ks * 256u + e0 + row + 64u * i] = sq[i];
+            if (piece == 0u) wsq[ks * 256u + e0 + row + 64u * i] = ok ? sq[i] : __uint_as_float(0x7FFFFFFFu);
         }
     }
-    ok = mbar_wait(bar0 + ((steps - 1u) % kNearStages) * 8u, ((steps - 1u) / kNearStages) & 1u, &abort_flag) && ok;
-    fence_after();
-    // a lane's expert, sixteen tokens at a time; logits that are not there (a wait ran out) are NaN, which sends the token to the scores in
-    // double
+    // a lane's expert, sixteen tokens at a time
     const uint32_t quad = warp & 3u, e = e0 + quad * 32u + lane;
     for (uint32_t g = (warp >> 2) * 16u; g < nt; g += 64u) {
         uint32_t r[16];
@@ -505,7 +518,7 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
 }
 
 constexpr uint32_t kNearFrom = 64;   // see above
-static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *part, float *wsq, cudaError_t *err) {
+static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *part, float *wsq, uint32_t *status, cudaError_t *err) {
     const uint32_t nt = std::min(ceil_div(ceil_div(r.n_tokens, 9u), 16u) * 16u, kNearTokens), mt = ceil_div(r.n_experts, 128u);
     const size_t smem = (size_t)kNearStages * (kNearW + nt * 256u);
     static bool allowed[64] = {};
@@ -519,7 +532,7 @@ static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *
     // (two tiles of experts, up to nine of tokens, eight parts of K: as many CTAs as SMs)
     if (*err == cudaSuccess)
         *err = launch_pdl(k_router_near, dim3(mt, ceil_div(r.n_tokens, nt), kNearSplit), dim3(kNearThreads), smem, st, 0u, r.x, r.router_weight_bf16,
-                          part, wsq, r.n_experts, r.hidden, r.n_tokens, nt);
+                          part, wsq, r.n_experts, r.hidden, r.n_tokens, nt, status);
     if (*err == cudaSuccess)
         *err = launch_pdl(k_router_pick, dim3(r.n_tokens), dim3(256), 0, st, 0u, r.x, r.router_weight_bf16, r.bias,
                           (const float *)part, (const float *)wsq, r.n_experts, r.hidden, r.n_tokens, r.score_fn, r.top_k,
@@ -527,10 +540,10 @@ static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *
     return *err == cudaSuccess ? 2 : 0;
 }
 
-int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, cudaError_t *err) {
+int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, uint32_t *status, cudaError_t *err) {
     *err = cudaErrorInvalidValue;
     if (r.hidden % 512u || r.hidden > 4096u) return 0;   // (a block object's hidden size)
-    if (r.n_tokens > kNearFrom) return launch_router_near(st, r, parts, scores, err);
+    if (r.n_tokens > kNearFrom) return launch_router_near(st, r, parts, scores, status, err);
     *err = launch_pdl(k_router_scores, dim3(ceil_div(r.n_experts, 8u), ceil_div(r.n_tokens, 8u)), dim3(kScoreWarps * 32u), 0, st, 0u, r.x,
                       r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
     if (*err != cudaSuccess) return 0;

@@ -59,9 +59,9 @@ extern "C" int quotients(uint32_t rounds, unsigned long long *wrong) {
 #include "s14_router.cu"
 extern "C" float near_bound(uint32_t hidden) { return s14::near_bound(hidden); }
 // parts: [8][n_tokens][256] sums of the approximate logits; scores, select: [n_tokens, 256]
-extern "C" int routes(const s14_router_desc *r, float *scores, float *select, float *parts) {
+extern "C" int routes(const s14_router_desc *r, float *scores, float *select, float *parts, uint32_t *status) {
     cudaError_t err;
-    s14::launch_router_batch(cudaStreamPerThread, *r, scores, select, parts, &err);
+    s14::launch_router_batch(cudaStreamPerThread, *r, scores, select, parts, status, &err);
     return (int)err;
 }
 #elif defined(PART_QUICK)

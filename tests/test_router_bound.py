@@ -107,12 +107,15 @@ class Router:
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
         (n, hidden), n_experts = x.shape, bits.shape[0]
         keep = [dev(x), dev(bits.view(np.int16)), dev(bias), torch.empty((n, top_k), dtype=torch.int32, device="cuda"),
-                torch.empty((n, top_k), device="cuda"), torch.empty((2, n, 256), device="cuda"), torch.empty((8, n, 256), device="cuda")]
+                torch.empty((n, top_k), device="cuda"), torch.empty((2, n, 256), device="cuda"), torch.empty((8, n, 256), device="cuda"),
+                torch.zeros(1, dtype=torch.int32, device="cuda")]
         d = L.RouterDesc(x=keep[0].data_ptr(), router_weight_bf16=keep[1].data_ptr(), bias=keep[2].data_ptr(), ids_out=keep[3].data_ptr(),
                          weights_out=keep[4].data_ptr(), n_tokens=n, hidden=hidden, n_experts=n_experts, top_k=top_k, score_fn=score_fn,
                          route_scale=1.5)
-        assert self.lib.routes(C.byref(d), C.c_void_p(keep[5][0].data_ptr()), C.c_void_p(keep[5][1].data_ptr()), C.c_void_p(keep[6].data_ptr())) == 0
+        assert self.lib.routes(C.byref(d), C.c_void_p(keep[5][0].data_ptr()), C.c_void_p(keep[5][1].data_ptr()), C.c_void_p(keep[6].data_ptr()),
+                               C.c_void_p(keep[7].data_ptr())) == 0
         torch.cuda.synchronize()
+        assert int(keep[7]) == 0
         return keep[3].cpu().numpy(), keep[4].cpu().numpy(), keep[6].cpu().numpy()
 
 
