@@ -2249,7 +2249,7 @@ static int32_t hc_reduce_call(s14_ctx *ctx, void *stream, const s14_hc_params *p
     cudaError_t err;
     ctx->launches += launch_hc_pre(stream_of(ctx, stream), ctx->sm_count, p->dtype == S14_STREAM_BF16, head, p->n_tokens, p->hidden, x, p->hc_fn,
                                    p->hc_scale, p->hc_base, p->norm_eps, p->sinkhorn_iters, p->hc_eps, ctx->glue, reduced,
-                                   post, comb, pre, &err);
+                                   post, comb, pre, ctx->status, &err);
     if (err != cudaSuccess) return cuda_fail(err, what);
     return S14_OK;
     S14_CATCH

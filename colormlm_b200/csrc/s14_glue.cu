@@ -211,6 +211,23 @@ __device__ __forceinline__ void store_counted(uint32_t at, uint32_t bar, uint32_
         "r"(bar), "r"(r), "l"(__double_as_longlong(v))
         : "memory");
 }
+// Whether all that is counted on the barrier's first phase has come, bounded (kSpin); by a whole warp, which then reads it.
+__device__ __forceinline__ bool counted_stores_come(uint32_t bar) {
+    bool come = false;
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpin && !(come = mbar_try(bar, 0u)); ++i) {
+    }
+    // (the stores are other CTAs', and the tries are at this one's scope)
+    uint32_t seen;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+        "selp.b32 %0, 1, 0, p;\n}"
+        : "=r"(seen)
+        : "r"(bar)
+        : "memory");
+    return __all_sync(0xffffffffu, come && seen);
+}
 
 // hc_pre (and, kHead, the head's reduce, final_head.py:43-81: hc logits, pre = sigmoid(mix * scale + base) + eps
 // only) of few tokens: one cluster of sixteen CTAs per token (the head fewer for more tokens: launch_hc_pre).  The call is all
@@ -220,12 +237,12 @@ __device__ __forceinline__ void store_counted(uint32_t at, uint32_t bar, uint32_
 // launch, no vote.  One token of 4096, calls one after another: 10.9 us in the two launches of then, 8.1 with clusters, 5.9 now.  Marks of the 8.1,
 // in clocks: start and cluster barrier 1200, rows and products 3550, the warps' sums 2100, their exchange 1700, logits and pre 1400, comb
 // 6400 (20 Sinkhorn rounds of one warp); now 1200, 3050, 350, 1400, and comb 5700 straight behind its logits, with pre beside it.
-constexpr uint32_t kPreThreads = 512;
+constexpr uint32_t kPreThreads = 512, kPreRow = (kPreThreads - 32u) * 8u;   // most elements of a CTA's share of the hidden vector
 template <bool kBf16, bool kHead, uint32_t kCluster>
 __global__ void __launch_bounds__(kPreThreads)
 k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *__restrict__ scale, const float *__restrict__ base,
          uint32_t hidden, float norm_eps, uint32_t iters, float hc_eps, void *__restrict__ reduced, float *__restrict__ post_out,
-         float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec) {
+         float *__restrict__ comb_out, float *__restrict__ pre_out, uint32_t vec, uint32_t *status) {
     constexpr uint32_t n_mix = kHead ? kHc : kMixMax, kRows = n_mix / 2u;   // rows per half of the CTA
     __shared__ double s_warp[kPreThreads / 32][kRows + 1];
     __shared__ double s_part[kCluster][n_mix + 1];                      // [n_mix]: the sum of squares
@@ -287,14 +304,19 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     }
     const uint32_t part = hidden / kCluster;   // a multiple of 16
     const bool comb_here = !kHead && rank == 0u;
-    // (a CTA leaves when all sums have come, so none is stored into one that has left; sums that do not come make it a NaN)
+    // A CTA leaves when all sums have come, so none is stored into one that has left.  Sums that do not come make the coefficients NaN and set the
+    // status word; the warps that have waited for them then stay until every other CTA of the cluster has left or stays likewise, and
+    // once more a wait's length for what is on its way.
     bool come = true;
-    if (warp == 0u || warp == 1u) {
-        uint32_t tries = 0;
-        while (!(come = mbar_try(smem_u32(&s_bar), 0u)) && ++tries < kSpin) {
-        }
-        come = __all_sync(0xffffffffu, come);
-    }
+    if (warp == 0u || warp == 1u) come = counted_stores_come(smem_u32(&s_bar));
+    auto leave = [&] {
+        if (come) return;
+        if (lane == 0u) atomicExch(status, 0x550Au);
+        __syncwarp();
+        cluster.barrier_arrive();
+        cluster.barrier_wait();
+        mbar_drain(smem_u32(&s_bar), 0u);
+    };
     if (warp == 1u || (warp == 0u && comb_here)) {
         double s = come ? 0.0 : __longlong_as_double(-1ll);
         if (lane <= n_mix) {
@@ -309,6 +331,7 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
             const float comb = sinkhorn_warp(s_mix[0], s_coef, s_coef + 3, iters, hc_eps, lane);
             if (lane < kHc * kHc) comb_out[(size_t)t * kHc * kHc + lane] = comb;
         }
+        leave();
         return;
     }
     if (warp == 1u && lane < kHc) {
@@ -320,12 +343,13 @@ k_hc_pre(const void *__restrict__ x, const float *__restrict__ fn, const float *
     asm volatile("bar.sync 1, %0;" ::"n"(kPreThreads - 32u) : "memory");
     if (!kHead && rank == 0u && warp == 1u && lane < kHc) post_out[(size_t)t * kHc + lane] = post_of(s_mix[1], s_coef, s_coef + 3, lane);
     const float pre[kHc] = {s_pre[0], s_pre[1], s_pre[2], s_pre[3]};
-    // (the last threads: rows of up to 30 K elements times the cluster leave the first warp out)
+    // (from the last thread on: the first warp, which has left, would come in above kPreRow elements)
     for (uint32_t i = (kPreThreads - 1u - tid) * 8u; i < part; i += kPreThreads * 8u) {
         float v[8];
         reduce_streams<kBf16, 8>(x, (size_t)t * n, hidden, rank * part + i, pre, v, vec != 0u);
         stream_stn<kBf16, 8>(reduced, (size_t)t * hidden + rank * part + i, v, vec != 0u);
     }
+    leave();
 }
 
 // The dot products of many tokens with the rows of fn, and the sums of squares, on mma.m8n8k4.f64: a CTA takes
@@ -660,12 +684,13 @@ static uint32_t aligned16(P... p) {
 template <bool kBf16, bool kHead, uint32_t kCluster>
 static cudaError_t launch_hc_pre_cluster(cudaStream_t st, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                                          const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps,
-                                         void *reduced, float *post, float *comb, float *pre) {
+                                         void *reduced, float *post, float *comb, float *pre, uint32_t *status) {
     static bool done[64] = {};
+    if (hidden / kCluster > kPreRow) return cudaErrorInvalidValue;
     const cudaError_t e = allow_wide_clusters(k_hc_pre<kBf16, kHead, kCluster>, done);
     if (e != cudaSuccess) return e;
     return launch_pdl(k_hc_pre<kBf16, kHead, kCluster>, dim3(kCluster, n_tokens), dim3(kPreThreads), 0, st, kCluster, x, fn, scale, base,
-                      hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced));
+                      hidden, norm_eps, iters, hc_eps, reduced, post, comb, pre, aligned16(x, reduced), status);
 }
 
 template <bool kBf16, bool kHead>
@@ -700,16 +725,17 @@ static cudaError_t launch_hc_pre_many(cudaStream_t st, int sm_count, uint32_t n_
 // hc_pre by a cluster of CTAs per token, for as many tokens as leave a fifth of the SMs (launch_hc_pre has the figures).
 static bool hc_pre_in_clusters(uint32_t n_tokens, uint32_t sms) { return 16u * n_tokens * 5u <= sms * 4u; }
 
-// scratch: hc_scratch_bytes of the most tokens.  Returns the number of kernels launched.
+// scratch: hc_scratch_bytes of the most tokens; status: the context's word (0x550A: the sums of a token's other CTAs have not come).  Returns the number of kernels launched.
 int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                   const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
-                  float *post, float *comb, float *pre, cudaError_t *err) {
+                  float *post, float *comb, float *pre, uint32_t *status, cudaError_t *err) {
     // one cluster per token while the clusters fit the GPU side by side, else two launches for all tokens
     auto run = [&](auto is_bf16, auto is_head, auto size) {
         constexpr bool kB = decltype(is_bf16)::value, kH = decltype(is_head)::value;
         constexpr uint32_t kC = decltype(size)::value;
         if constexpr (kC != 0u) {
-            *err = launch_hc_pre_cluster<kB, kH, kC>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre);
+            *err = launch_hc_pre_cluster<kB, kH, kC>(st, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, reduced, post, comb, pre,
+                                                     status);
             return 1;
         } else {
             *err = launch_hc_pre_many<kB, kH>(st, sm_count, n_tokens, hidden, x, fn, scale, base, norm_eps, iters, hc_eps, scratch, reduced,

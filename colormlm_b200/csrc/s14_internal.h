@@ -280,7 +280,7 @@ int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores
 size_t hc_scratch_bytes(uint32_t max_tokens, int sm_count);
 int launch_hc_pre(cudaStream_t st, int sm_count, bool bf16, bool head, uint32_t n_tokens, uint32_t hidden, const void *x, const float *fn,
                   const float *scale, const float *base, float norm_eps, uint32_t iters, float hc_eps, double *scratch, void *reduced,
-                  float *post, float *comb, float *pre, cudaError_t *err);
+                  float *post, float *comb, float *pre, uint32_t *status, cudaError_t *err);
 cudaError_t launch_hc_post(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *branch, const void *residual,
                            const float *post, const float *comb, void *merged);
 cudaError_t launch_rms_norm(cudaStream_t st, int sm_count, bool bf16, uint32_t n_tokens, uint32_t hidden, const void *x, const float *w, float eps,

@@ -596,6 +596,8 @@ S14_API int32_t s14_block_last_counts(s14_block *blk, uint32_t counts_out[4]);
  *   router_hash: ids_out[t] = tid2eid_rows[t] (device int64 [T, top_k], the current token's row of the
  *            layer's tid2eid), weights_out = the router's scores of those experts / their sum * route_scale;
  *            desc->bias is not used.
+ * A wait inside hc_pre or hc_head_reduce that runs out (few tokens: the CTAs of a token exchange their sums) sets the
+ * context's device status word to 0x550A; that token's outputs are then not to be used.
  * hc_pre, hc_head_reduce and hc_head_norm_full_logits (below) take x on a 16-byte boundary (F32) or an 8-byte one
  * (BF16), hc_fn and a head's weight on a 16-byte one; the other buffers lie on their elements' boundary. */
 #define S14_STREAM_F32 0u

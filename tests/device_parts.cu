@@ -55,6 +55,20 @@ extern "C" int quotients(uint32_t rounds, unsigned long long *wrong) {
     s14::k_quotients<<<(1 << 23) / 256, 256, 0, cudaStreamPerThread>>>(rounds, wrong);
     return (int)cudaGetLastError();
 }
+#elif defined(PART_SINKHORN)
+#include "s14_glue.cu"
+namespace s14 {
+namespace {
+__global__ void k_sinkhorn(const float *mixes, const float *scale, const float *base, uint32_t iters, float eps, float *comb) {
+    const float c = sinkhorn_warp(mixes + blockIdx.x * kMixMax, scale, base, iters, eps, threadIdx.x);
+    if (threadIdx.x < kHc * kHc) comb[blockIdx.x * kHc * kHc + threadIdx.x] = c;
+}
+}  // namespace
+}  // namespace s14
+extern "C" int sinkhorn(uint32_t n, const float *mixes, const float *scale, const float *base, uint32_t iters, float eps, float *comb) {
+    s14::k_sinkhorn<<<n, 32, 0, cudaStreamPerThread>>>(mixes, scale, base, iters, eps, comb);
+    return (int)cudaGetLastError();
+}
 #elif defined(PART_ROUTER)
 #include "s14_router.cu"
 extern "C" float near_bound(uint32_t hidden) { return s14::near_bound(hidden); }
