@@ -269,7 +269,7 @@ cudaError_t launch_block_mix(cudaStream_t st, const float *pairs, const int32_t 
                              uint32_t top_k, bool has_shared, const float *x, float *y, uint32_t hidden, const uint32_t *counts,
                              const BlockEp *ep = nullptr, uint32_t *status = nullptr);
 // Scores and routes of many tokens (s14_router.cu).  Same arithmetic as launch_router.  hidden is a multiple of 512 up to 4096; scores, select:
-// [n_tokens, n_experts] scratch, parts: [8, n_tokens, 256] (for more than 64 tokens; a block's pair outputs, of 7 x 512 values a token
+// [n_tokens, n_experts] scratch, parts: [8, n_tokens, 256] (for large blocks; a block's pair outputs, of 7 x 512 values a token
 // at least, have room for it and are written later); status: the context's word (0x5509: a wait inside a kernel ran out, the routes are right).  Returns
 // the number of kernels launched.
 int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, uint32_t *status,

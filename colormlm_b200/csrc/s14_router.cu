@@ -11,56 +11,89 @@ inline uint32_t ceil_div(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-// ---- every score in double: blocks of up to 64 tokens ----
-// Scores on the FP64 matrix pipe: a CTA takes 8 tokens x 8 experts, its sixteen warps the K range in equal parts
+// ---- every score in double ----
+// Scores on the FP64 matrix pipe: a CTA takes 8 * kMt tokens x 8 * kNt experts, its warps the K range in equal parts
 // (their sums meet in shared memory, in warp order).  mma.m8n8k4.f64 wants one element of A (8 tokens x 4 k) and of B
 // (4 k x 8 experts) per lane and step; which k an element stands for is free as long as A and B agree, so a lane
 // takes eight neighbouring elements of its row (32 bytes of x, 16 of the weights) and feeds them to eight steps:
 // operands go from the L2 to registers, four lanes share a cache line, nothing is staged.  Every f32 and bf16 value is
 // exact in double, so is every product, and the sums are double: score and score + bias are those of k_router.
-// Measured, x 256 experts x 4096: 8 tokens 8.3 us, 32 tokens 4.3 from the L2; 45 tokens x 192 experts x 2048 10.
-constexpr uint32_t kScoreWarps = 16;
-__global__ void __launch_bounds__(kScoreWarps * 32u)
+//
+// Up to 64 tokens 8 x 8 tiles of sixteen warps fill the chip (x 256 experts x 4096: 8 tokens 8.3 us, 32 tokens 4.3 from the L2, in 16 x 8 tiles
+// 9.6; 45 tokens x 192 experts x 2048 10); above, tiles of 16 x 16, which read a token's row once per sixteen experts, and of 16 x 8 where
+// they would be fewer than two CTAs per SM.
+template <uint32_t kMt, uint32_t kNt, uint32_t kWarps>
+__global__ void __launch_bounds__(kWarps * 32u)
 k_router_scores(const float *__restrict__ x, const uint16_t *__restrict__ wr, const float *__restrict__ bias,
                 float *__restrict__ scores, float *__restrict__ select, uint32_t n_experts, uint32_t hidden,
                 uint32_t n_tokens, uint32_t score_fn) {
-    __shared__ double s_c[kScoreWarps][64];
+    __shared__ double s_c[kWarps][kMt * kNt][64];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, row = lane >> 2, col = lane & 3u;
-    const uint32_t e0 = blockIdx.x * 8u, t0 = blockIdx.y * 8u;
-    const uint32_t part = hidden / kScoreWarps, first = warp * part + col * 8u;   // a whole number of steps of 32 elements
+    const uint32_t e0 = blockIdx.x * (8u * kNt), t0 = blockIdx.y * (8u * kMt);
+    const uint32_t part = hidden / kWarps, first = warp * part + col * 8u;   // a whole number of steps of 32 elements
+    const float *xr[kMt];
+    const uint16_t *wp[kNt];
     // (a token or expert past the end reads the last one again; its scores are not written)
-    const float *const xr = x + (size_t)min(t0 + row, n_tokens - 1u) * hidden + first;
-    const uint16_t *const wp = wr + (size_t)min(e0 + row, n_experts - 1u) * hidden + first;
-    double c0 = 0.0, c1 = 0.0;
-    float4 xa, xb;
-    uint4 q;
+#pragma unroll
+    for (uint32_t m = 0; m < kMt; ++m) xr[m] = x + (size_t)min(t0 + m * 8u + row, n_tokens - 1u) * hidden + first;
+#pragma unroll
+    for (uint32_t n = 0; n < kNt; ++n) wp[n] = wr + (size_t)min(e0 + n * 8u + row, n_experts - 1u) * hidden + first;
+    double c[kMt][kNt][2] = {};
+    float4 xa[kMt], xb[kMt];
+    uint4 q[kNt];
     auto load = [&](uint32_t k) {
-        q = __ldcg(reinterpret_cast<const uint4 *>(wp + k));
-        xa = __ldcg(reinterpret_cast<const float4 *>(xr + k));
-        xb = __ldcg(reinterpret_cast<const float4 *>(xr + k) + 1);
+#pragma unroll
+        for (uint32_t n = 0; n < kNt; ++n) q[n] = __ldcg(reinterpret_cast<const uint4 *>(wp[n] + k));
+#pragma unroll
+        for (uint32_t m = 0; m < kMt; ++m) {
+            xa[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k));
+            xb[m] = __ldcg(reinterpret_cast<const float4 *>(xr[m] + k) + 1);
+        }
     };
     dependency_wait();
     load(0);
 #pragma unroll 1
     for (uint32_t k = 0; k < part; k += 32u) {
-        const float a[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-        const uint32_t b[4] = {q.x, q.y, q.z, q.w};
+        float a[kMt][8];
+        uint32_t b[kNt][4];
+#pragma unroll
+        for (uint32_t m = 0; m < kMt; ++m) {
+            a[m][0] = xa[m].x, a[m][1] = xa[m].y, a[m][2] = xa[m].z, a[m][3] = xa[m].w;
+            a[m][4] = xb[m].x, a[m][5] = xb[m].y, a[m][6] = xb[m].z, a[m][7] = xb[m].w;
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < kNt; ++n) b[n][0] = q[n].x, b[n][1] = q[n].y, b[n][2] = q[n].z, b[n][3] = q[n].w;
         if (k + 32u < part) load(k + 32u);
 #pragma unroll
-        for (uint32_t i = 0; i < 8; ++i)
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                         : "+d"(c0), "+d"(c1)
-                         : "d"((double)a[i]), "d"((double)__uint_as_float((i & 1u) ? b[i >> 1] & 0xffff0000u : b[i >> 1] << 16)));
+        for (uint32_t i = 0; i < 8; ++i) {
+            double av[kMt], bv[kNt];
+#pragma unroll
+            for (uint32_t m = 0; m < kMt; ++m) av[m] = (double)a[m][i];
+#pragma unroll
+            for (uint32_t n = 0; n < kNt; ++n)
+                bv[n] = (double)__uint_as_float((i & 1u) ? b[n][i >> 1] & 0xffff0000u : b[n][i >> 1] << 16);
+#pragma unroll
+            for (uint32_t m = 0; m < kMt; ++m)
+#pragma unroll
+                for (uint32_t n = 0; n < kNt; ++n)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                                 : "+d"(c[m][n][0]), "+d"(c[m][n][1])
+                                 : "d"(av[m]), "d"(bv[n]));
+        }
     }
     // C (8 x 8): lane holds row lane / 4, columns 2 (lane % 4) and 2 (lane % 4) + 1
-    *reinterpret_cast<double2 *>(&s_c[warp][row * 8u + col * 2u]) = make_double2(c0, c1);
-    __syncthreads();
-    if (threadIdx.x < 64u) {
-        const uint32_t at = threadIdx.x;
-        double sum = s_c[0][at];
 #pragma unroll
-        for (uint32_t w = 1; w < kScoreWarps; ++w) sum += s_c[w][at];
-        const uint32_t t = t0 + (at >> 3), e = e0 + (at & 7u);
+    for (uint32_t m = 0; m < kMt; ++m)
+#pragma unroll
+        for (uint32_t n = 0; n < kNt; ++n)
+            *reinterpret_cast<double2 *>(&s_c[warp][m * kNt + n][row * 8u + col * 2u]) = make_double2(c[m][n][0], c[m][n][1]);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kMt * kNt * 64u; i += kWarps * 32u) {
+        const uint32_t tile = i >> 6, at = i & 63u;
+        double sum = s_c[0][tile][at];
+#pragma unroll
+        for (uint32_t w = 1; w < kWarps; ++w) sum += s_c[w][tile][at];
+        const uint32_t t = t0 + (tile / kNt) * 8u + (at >> 3), e = e0 + (tile % kNt) * 8u + (at & 7u);
         if (t < n_tokens && e < n_experts) {
             const float sc = router_score_f32(sum, score_fn);
             scores[(size_t)t * n_experts + e] = sc;
@@ -81,13 +114,12 @@ k_router_select_batch(const float *__restrict__ scores, const float *__restrict_
                   1, 0);
 }
 
-// ---- scores in double only where they decide: blocks of more than 64 tokens ----
+// ---- scores in double only where they decide: large blocks of many experts ----
 // Of a token's 256 scores the six largest matter, and those that come near the sixth.  So the logits are first taken
 // from BF16 products (k_router_near), each with a bound on its error, and k_router_pick takes in double, for every token, the
 // experts that can be among the picked ones: 6.5 on average for Gaussian rows.  Ids and weights are those of scores that are all taken in double.
-// All of them on the FP64 matrix pipe in tiles of 16 tokens x 16 experts (at half of its rate) took, x 256 experts x 4096, 40 us for
-// 370 tokens and 85 for 1000, and the pick 3; now 9 + 13 and 15 + 24, half of the second beside the digits launch: the call of 370 tokens 615 -> 603 us,
-// of 1000 official ones 790 -> 745 (bursts).  65 and 100 tokens gain 1 %, up to 64 the other kernel is the faster.
+// All of them on the FP64 matrix pipe in tiles of 16 tokens x 16 experts (at half of its rate) take, x 256 experts x 4096, 40 us for
+// 370 tokens and 85 for 1000, and the pick 3; this 9 + 13 and 15 + 24, half of the second beside the digits launch (near_pays has the calls).
 //
 // k_router_near: x = hi + lo + r with BF16 values hi and lo, |r| <= 2^-18 |x|; hi and lo against the weights on tcgen05.mma
 // (kind::f16, M = 128 experts, N tokens, F32 sums).  A CTA takes 128 experts, `nt` tokens and an eighth of K; the eighths' sums go to
@@ -517,7 +549,6 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     }
 }
 
-constexpr uint32_t kNearFrom = 64;   // see above
 static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *part, float *wsq, uint32_t *status, cudaError_t *err) {
     const uint32_t nt = std::min(ceil_div(ceil_div(r.n_tokens, 9u), 16u) * 16u, kNearTokens), mt = ceil_div(r.n_experts, 128u);
     const size_t smem = (size_t)kNearStages * (kNearW + nt * 256u);
@@ -540,17 +571,34 @@ static int launch_router_near(cudaStream_t st, const s14_router_desc &r, float *
     return *err == cudaSuccess ? 2 : 0;
 }
 
+// Which of the two ways.  All scores in double take time by tokens x experts x hidden; k_router_near by tiles of 128 experts, and k_router_pick, a CTA per
+// token, hardly less for few experts than for many.  us of the call (inter 512 or 1024), all in double / by the filter: 256 experts x 4096, 80
+// tokens 116.6 both, 150 156.9 / 152.1, 1000 official 366 / 319; 256 x 2048, 100 tokens 116.2 / 116.4, 370 235 / 224; 256 x 1024, 250 97.1 / 97.3, 370
+// 125.5 / 122.1; 192 x 2048, 250 123.9 / 124.4, 370 161.1 / 158.8; 160 x 2048, 250 121.9 / 124.4, 700 261 / 256; but rows so short that
+// the pick is most of it, 256 x 512, 1000 tokens 208.3 / 208.8, official 118.2 / 119.3.  One tile of experts: 128 x 4096, 370 tokens official 155.1 / 156.6,
+// 700 235 / 221; 128 x 2048, 1000 tokens 501 / 499; 64 x 4096, 1000 tokens 370 / 378; 64 x 512, 250 tokens 46.2 / 50.6; 8 x 1024, 1000 tokens 100 / 114.
+constexpr uint32_t kNearFrom = 64;   // (up to 64 tokens the 8 x 8 tiles are the faster for all sizes)
+static bool near_pays(uint32_t n_tokens, uint32_t n_experts, uint32_t hidden) {
+    const uint64_t row = (uint64_t)n_experts * hidden, work = row * n_tokens;
+    if (n_tokens <= kNearFrom) return false;
+    return n_experts > 128u ? row >= 1ull << 18 && work * n_experts >= 1ull << 34 : work >= 1ull << 28;
+}
+
 int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, uint32_t *status, cudaError_t *err) {
     *err = cudaErrorInvalidValue;
     if (r.hidden % 512u || r.hidden > 4096u) return 0;   // (a block object's hidden size)
-    if (r.n_tokens > kNearFrom) return launch_router_near(st, r, parts, scores, status, err);
-    *err = launch_pdl(k_router_scores, dim3(ceil_div(r.n_experts, 8u), ceil_div(r.n_tokens, 8u)), dim3(kScoreWarps * 32u), 0, st, 0u, r.x,
-                      r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
+    if (near_pays(r.n_tokens, r.n_experts, r.hidden)) return launch_router_near(st, r, parts, scores, status, err);
+    auto run = [&](auto kernel, uint32_t mt, uint32_t nt, uint32_t warps) {
+        return launch_pdl(kernel, dim3(ceil_div(r.n_experts, 8u * nt), ceil_div(r.n_tokens, 8u * mt)), dim3(warps * 32u), 0, st, 0u, r.x,
+                          r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
+    };
+    if (r.n_tokens <= 64u) *err = run(k_router_scores<1, 1, 16>, 1, 1, 16);
+    else if (ceil_div(r.n_tokens, 16u) * ceil_div(r.n_experts, 16u) < 296u) *err = run(k_router_scores<2, 1, 8>, 2, 1, 8);
+    else *err = run(k_router_scores<2, 2, 8>, 2, 2, 8);
     if (*err != cudaSuccess) return 0;
     *err = launch_pdl(k_router_select_batch, dim3(ceil_div(r.n_tokens, 8)), dim3(256), 0, st, 0u, (const float *)scores,
                       (const float *)select, r.n_experts, r.n_tokens, r.top_k, r.route_scale, r.ids_out, r.weights_out);
     return 2;
 }
-
 
 }  // namespace s14

@@ -72,10 +72,11 @@ extern "C" int sinkhorn(uint32_t n, const float *mixes, const float *scale, cons
 #elif defined(PART_ROUTER)
 #include "s14_router.cu"
 extern "C" float near_bound(uint32_t hidden) { return s14::near_bound(hidden); }
-// parts: [8][n_tokens][256] sums of the approximate logits; scores, select: [n_tokens, 256]
-extern "C" int routes(const s14_router_desc *r, float *scores, float *select, float *parts, uint32_t *status) {
+extern "C" int near_pays(uint32_t n_tokens, uint32_t n_experts, uint32_t hidden) { return s14::near_pays(n_tokens, n_experts, hidden); }
+// By the filter whatever the size.  parts: [8][n_tokens][256] sums of the approximate logits; squares: [8][256]
+extern "C" int near_routes(const s14_router_desc *r, float *squares, float *parts, uint32_t *status) {
     cudaError_t err;
-    s14::launch_router_batch(cudaStreamPerThread, *r, scores, select, parts, status, &err);
+    s14::launch_router_near(cudaStreamPerThread, *r, parts, squares, status, &err);
     return (int)err;
 }
 #elif defined(PART_QUICK)

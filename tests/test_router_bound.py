@@ -96,7 +96,7 @@ def test_the_bound_holds_for_random_rows(part):
 
 
 class Router:
-    """launch_router_batch on rows given as arrays."""
+    """launch_router_near, which large blocks take, on rows given as arrays."""
 
     def __init__(self, lib):
         self.lib = lib
@@ -105,18 +105,19 @@ class Router:
         import torch
 
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        ptr = lambda t: C.c_void_p(t.data_ptr())
         (n, hidden), n_experts = x.shape, bits.shape[0]
-        keep = [dev(x), dev(bits.view(np.int16)), dev(bias), torch.empty((n, top_k), dtype=torch.int32, device="cuda"),
-                torch.empty((n, top_k), device="cuda"), torch.empty((2, n, 256), device="cuda"), torch.empty((8, n, 256), device="cuda"),
-                torch.zeros(1, dtype=torch.int32, device="cuda")]
-        d = L.RouterDesc(x=keep[0].data_ptr(), router_weight_bf16=keep[1].data_ptr(), bias=keep[2].data_ptr(), ids_out=keep[3].data_ptr(),
-                         weights_out=keep[4].data_ptr(), n_tokens=n, hidden=hidden, n_experts=n_experts, top_k=top_k, score_fn=score_fn,
+        dx, dw, db = dev(x), dev(bits.view(np.int16)), None if bias is None else dev(bias)
+        ids, wts = torch.empty((n, top_k), dtype=torch.int32, device="cuda"), torch.empty((n, top_k), device="cuda")
+        squares, parts, status = torch.empty((8, 256), device="cuda"), torch.empty((8, n, 256), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        d = L.RouterDesc(x=dx.data_ptr(), router_weight_bf16=dw.data_ptr(), bias=0 if db is None else db.data_ptr(), ids_out=ids.data_ptr(),
+                         weights_out=wts.data_ptr(), n_tokens=n, hidden=hidden, n_experts=n_experts, top_k=top_k, score_fn=score_fn,
                          route_scale=1.5)
-        assert self.lib.routes(C.byref(d), C.c_void_p(keep[5][0].data_ptr()), C.c_void_p(keep[5][1].data_ptr()), C.c_void_p(keep[6].data_ptr()),
-                               C.c_void_p(keep[7].data_ptr())) == 0
         torch.cuda.synchronize()
-        assert int(keep[7]) == 0
-        return keep[3].cpu().numpy(), keep[4].cpu().numpy(), keep[6].cpu().numpy()
+        assert self.lib.near_routes(C.byref(d), ptr(squares), ptr(parts), ptr(status)) == 0
+        torch.cuda.synchronize()
+        assert int(status) == 0
+        return ids.cpu().numpy(), wts.cpu().numpy(), parts.cpu().numpy()
 
 
 @pytest.fixture(scope="module")
@@ -163,3 +164,30 @@ def test_rows_with_their_magnitude_in_front(part, router, oracle, score_fn, hidd
     for t in range(0, n, 3):
         rid, rw, _, _ = oracle.router(x[t], bits, bias, score_fn=score_fn, top_k=top_k, route_scale=1.5)
         assert np.array_equal(ids[t], rid) and np.array_equal(wts[t].view(np.uint32), rw.view(np.uint32)), t
+
+
+# the sizes and kinds of rows that the block's own test has, whichever way a block of that size takes
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,n_tokens,n_experts,hidden,top_k", [
+    ("plain", 1, 256, 512, 6), ("plain", 65, 256, 512, 6), ("plain", 144, 129, 2560, 6), ("plain", 145, 7, 1024, 6), ("plain", 300, 128, 4096, 3),
+    ("plain", 1024, 250, 512, 6), ("ties", 80, 256, 1024, 6), ("near", 80, 256, 1024, 6), ("near", 80, 40, 512, 1), ("small", 70, 200, 1024, 6),
+    ("large", 70, 200, 1024, 6), ("zero", 66, 256, 512, 6), ("outlier", 90, 256, 4096, 6)])
+@pytest.mark.parametrize("score_fn", [L.SCORE_SIGMOID, L.SCORE_SQRT_SOFTPLUS])
+def test_the_filters_routes_have_the_oracles_bits(router, oracle, kind, n_tokens, n_experts, hidden, top_k, score_fn):
+    from .test_gpu_router_near import rows
+
+    x, w, b = rows(synth.rng(40 + n_tokens + n_experts + hidden), kind, n_tokens, n_experts, hidden)
+    bits = synth.f32_to_bf16_bits(w)
+    ids, wts, _ = router(x, bits, b, score_fn, top_k)
+    for t in range(0, n_tokens, max(1, n_tokens // 50)):
+        rid, rw, _, _ = oracle.router(x[t], bits, b, score_fn=score_fn, top_k=top_k, route_scale=1.5)
+        assert np.array_equal(ids[t], rid) and np.array_equal(wts[t].view(np.uint32), rw.view(np.uint32)), t
+
+
+@pytest.mark.parametrize("n_tokens,n_experts,hidden,filtered", [
+    (64, 256, 4096, False), (65, 256, 4096, True), (100, 256, 2048, False), (150, 256, 2048, True), (250, 256, 1024, False), (370, 256, 1024, True),
+    (1000, 256, 512, False), (250, 160, 2048, False), (700, 160, 2048, True), (370, 128, 4096, False), (700, 128, 4096, True), (1000, 64, 4096, False),
+    (250, 64, 512, False), (1000, 8, 1024, False), (1024, 8, 4096, False)])
+def test_which_blocks_take_the_filter(part, n_tokens, n_experts, hidden, filtered):
+    """Sizes at which both ways were measured: with few experts or short rows the filter took up to 15 % longer."""
+    assert bool(part.near_pays(n_tokens, n_experts, hidden)) == filtered
