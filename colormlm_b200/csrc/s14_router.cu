@@ -356,7 +356,8 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     __shared__ float s_sq[8], s_sel[256], s_score[256];
     __shared__ double s_sum[8][8];
     __shared__ __align__(16) uint32_t s_top[32];
-    __shared__ uint32_t s_n, s_least[256], s_most[256], s_has[8];
+    __shared__ __align__(16) uint32_t s_least[256];
+    __shared__ uint32_t s_n, s_most[256], s_has[8], s_bar[8];
     __shared__ uint16_t s_list[256];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, t = blockIdx.x, mine_e = min(tid, n_experts - 1u);
     const uint32_t pieces = hidden >> 6, piece0 = warp * pieces + lane;   // of eight elements, this warp's: 8 .. 64
@@ -400,8 +401,16 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     const float err = near_bound(hidden) * sqrtf(__fmaf_rn(x2, 1.001f, 0x1p-114f)) * sqrtf(__fmaf_rn(w2, 1.001f, 0x1p-114f));
     float off;
     const float s = near_score(logit, err, score_fn, off), sel = s + b;
-    off += 0x1p-18f * (fabsf(s) + fabsf(b) + 0x1p-20f);   // the score's own evaluation and the roundings here
-    const bool all = __syncthreads_or(there && !(fabsf(sel) <= 3e38f && off <= 3e38f));
+    // the score's own evaluation and the roundings here (a bias beyond 3e38 - a mask's, infinite or the type's lowest - is the sum whatever the
+    // score is)
+    off += 0x1p-18f * (fabsf(s) + (fabsf(b) <= 3e38f ? fabsf(b) : 0.0f) + 0x1p-20f);
+    const bool all = __syncthreads_or(there && !(fabsf(s) <= 3e38f && off <= 3e38f && b == b));
+    // a token of zeros (padding): every logit is zero
+    const uint32_t bits = __float_as_uint(xa[0].x) | __float_as_uint(xa[0].y) | __float_as_uint(xa[0].z) | __float_as_uint(xa[0].w) |
+                          __float_as_uint(xb[0].x) | __float_as_uint(xb[0].y) | __float_as_uint(xb[0].z) | __float_as_uint(xb[0].w) |
+                          __float_as_uint(xa[1].x) | __float_as_uint(xa[1].y) | __float_as_uint(xa[1].z) | __float_as_uint(xa[1].w) |
+                          __float_as_uint(xb[1].x) | __float_as_uint(xb[1].y) | __float_as_uint(xb[1].z) | __float_as_uint(xb[1].w);
+    const bool zero = x2 == 0.0f && !__syncthreads_or((bits << 1) != 0u) && !all;
     // No more than the top_k-th largest of what the experts have at least: the largest of every one, two, four or eight experts, of 32 such
     // groups at most, and of those the top_k-th (where two of the largest are in one group it is the next one's: a candidate more).  Every
     // warp finds it.
@@ -428,10 +437,38 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     }
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(mine & ((1u << lane) - 1u));
     if (cand) s_list[at] = (uint16_t)tid;
-    if (cand) s_least[tid] = order_key(sel - off);
+    s_least[tid] = there ? order_key(sel - off) : 0u;
     if (cand) s_most[tid] = order_key(sel + off);
     __syncthreads();
     uint32_t n = s_n;
+    if (n > 32u && !all) {
+        // where masks leave fewer groups than top_k with an expert that counts: by the top_k-th largest of all that the experts have at least
+        const uint32_t low = s_least[tid];
+        above = 0u;
+#pragma unroll 8
+        for (uint32_t i = 0; i < 64u; ++i) {
+            const uint4 k4 = reinterpret_cast<const uint4 *>(s_least)[i];
+            above += (k4.x > low) + (k4.y > low) + (k4.z > low) + (k4.w > low);
+        }
+        const uint32_t bar = __reduce_min_sync(0xffffffffu, above < top_k ? low : 0xffffffffu);
+        if (lane == 0) s_bar[warp] = bar;
+        __syncthreads();
+        uint32_t bars = s_bar[0];
+#pragma unroll
+        for (uint32_t w = 1; w < 8u; ++w) bars = min(bars, s_bar[w]);
+        const uint32_t who = __ballot_sync(0xffffffffu, cand && s_most[tid] >= bars);
+        if (lane == 0) s_has[warp] = who;
+        __syncthreads();
+        at = __popc(who & ((1u << lane) - 1u));
+        n = 0u;
+#pragma unroll
+        for (uint32_t w = 0; w < 8u; ++w) {
+            if (w < warp) at += __popc(s_has[w]);
+            n += __popc(s_has[w]);
+        }
+        if (who >> lane & 1u) s_list[at] = (uint16_t)tid;
+        __syncthreads();
+    }
     if (n > 8u && n <= 32u && !all) {
         // more than the groups below: by the top_k-th largest itself, which is among them
         uint32_t e = lane < n ? s_list[lane] : 0u, low = lane < n ? s_least[e] : 0u, before = 0u;
@@ -449,8 +486,13 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     // three to the right, are the double of 2^-896 times its value, subnormal ones included, so nothing has to be converted (a conversion takes
     // an SM four times as long as a multiplication); with the token times 2^800 no product leaves the range of normal doubles, and the sum has
     // the bits of the plain one times 2^-96.  Weights that are not finite come with `all`, and so does this loop's other form.
+    if (zero) {
+        s_score[tid] = router_score_f32(0.0, score_fn);
+        s_sel[tid] = __fadd_rn(s_score[tid], b);
+        __syncthreads();
+    }
 #pragma unroll 1
-    for (uint32_t c0 = 0; c0 < n; c0 += 8u) {
+    for (uint32_t c0 = zero ? n : 0u; c0 < n; c0 += 8u) {
         double acc[8];
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) acc[k] = 0.0;
@@ -584,10 +626,7 @@ static bool near_pays(uint32_t n_tokens, uint32_t n_experts, uint32_t hidden) {
     return n_experts > 128u ? row >= 1ull << 18 && work * n_experts >= 1ull << 34 : work >= 1ull << 28;
 }
 
-int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, uint32_t *status, cudaError_t *err) {
-    *err = cudaErrorInvalidValue;
-    if (r.hidden % 512u || r.hidden > 4096u) return 0;   // (a block object's hidden size)
-    if (near_pays(r.n_tokens, r.n_experts, r.hidden)) return launch_router_near(st, r, parts, scores, status, err);
+static int launch_router_tiles(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, cudaError_t *err) {
     auto run = [&](auto kernel, uint32_t mt, uint32_t nt, uint32_t warps) {
         return launch_pdl(kernel, dim3(ceil_div(r.n_experts, 8u * nt), ceil_div(r.n_tokens, 8u * mt)), dim3(warps * 32u), 0, st, 0u, r.x,
                           r.router_weight_bf16, r.bias, scores, select, r.n_experts, r.hidden, r.n_tokens, r.score_fn);
@@ -599,6 +638,13 @@ int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores
     *err = launch_pdl(k_router_select_batch, dim3(ceil_div(r.n_tokens, 8)), dim3(256), 0, st, 0u, (const float *)scores,
                       (const float *)select, r.n_experts, r.n_tokens, r.top_k, r.route_scale, r.ids_out, r.weights_out);
     return 2;
+}
+
+int launch_router_batch(cudaStream_t st, const s14_router_desc &r, float *scores, float *select, float *parts, uint32_t *status, cudaError_t *err) {
+    *err = cudaErrorInvalidValue;
+    if (r.hidden % 512u || r.hidden > 4096u) return 0;   // (a block object's hidden size)
+    return near_pays(r.n_tokens, r.n_experts, r.hidden) ? launch_router_near(st, r, parts, scores, status, err)
+                                                        : launch_router_tiles(st, r, scores, select, err);
 }
 
 }  // namespace s14

@@ -79,6 +79,12 @@ extern "C" int near_routes(const s14_router_desc *r, float *squares, float *part
     s14::launch_router_near(cudaStreamPerThread, *r, parts, squares, status, &err);
     return (int)err;
 }
+// All scores in double whatever the size.  scores, select: [n_tokens, 256]
+extern "C" int tile_routes(const s14_router_desc *r, float *scores, float *select) {
+    cudaError_t err;
+    s14::launch_router_tiles(cudaStreamPerThread, *r, scores, select, &err);
+    return (int)err;
+}
 #elif defined(PART_QUICK)
 #include "s14_moe_pair.cu"
 namespace s14 {

@@ -101,7 +101,8 @@ class Router:
     def __init__(self, lib):
         self.lib = lib
 
-    def __call__(self, x, bits, bias, score_fn, top_k):
+    def __call__(self, x, bits, bias, score_fn, top_k, tiles=False, calls=1):
+        """tiles: all scores in double.  calls: that many after a first one are timed, the best of five such rounds in `us`."""
         import torch
 
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
@@ -113,10 +114,21 @@ class Router:
         d = L.RouterDesc(x=dx.data_ptr(), router_weight_bf16=dw.data_ptr(), bias=0 if db is None else db.data_ptr(), ids_out=ids.data_ptr(),
                          weights_out=wts.data_ptr(), n_tokens=n, hidden=hidden, n_experts=n_experts, top_k=top_k, score_fn=score_fn,
                          route_scale=1.5)
+        run = (lambda: self.lib.tile_routes(C.byref(d), ptr(parts[0]), ptr(parts[1]))) if tiles else (
+            lambda: self.lib.near_routes(C.byref(d), ptr(squares), ptr(parts), ptr(status)))
         torch.cuda.synchronize()
-        assert self.lib.near_routes(C.byref(d), ptr(squares), ptr(parts), ptr(status)) == 0
+        assert run() == 0
         torch.cuda.synchronize()
         assert int(status) == 0
+        own, self.us = torch.cuda.ExternalStream(2), float("inf")   # (cudaStreamPerThread)
+        for _ in range(5 if calls > 1 else 0):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record(own)
+            for _ in range(calls):
+                run()
+            end.record(own)
+            torch.cuda.synchronize()
+            self.us = min(self.us, begin.elapsed_time(end) * 1e3 / calls)
         return ids.cpu().numpy(), wts.cpu().numpy(), parts.cpu().numpy()
 
 
@@ -191,3 +203,69 @@ def test_the_filters_routes_have_the_oracles_bits(router, oracle, kind, n_tokens
 def test_which_blocks_take_the_filter(part, n_tokens, n_experts, hidden, filtered):
     """Sizes at which both ways were measured: with few experts or short rows the filter took up to 15 % longer."""
     assert bool(part.near_pays(n_tokens, n_experts, hidden)) == filtered
+
+
+LOWEST = np.finfo(np.float32).min
+
+
+def masked(g, x, w, b, kind):
+    """What real calls have beside plain rows: masks as biases, padding, numbers that are none."""
+    n_experts = len(b)
+    off = g.permutation(n_experts) < n_experts // 2
+    if kind in ("half -inf", "half lowest"):
+        b[off] = -np.inf if kind == "half -inf" else LOWEST
+    elif kind == "one group of 32 left":   # every other expert is masked
+        b[:64], b[96:] = -np.inf, LOWEST
+    elif kind == "eight left":             # neighbours
+        b[:40], b[48:] = LOWEST, LOWEST
+    elif kind == "four left":              # fewer than are picked
+        b[4:] = -np.inf
+    elif kind == "some +inf":
+        b[[3, 200, 77]] = np.inf
+    elif kind == "zero tokens":
+        x[::3], x[1] = 0, -0.0
+        b[:] = 0
+    elif kind == "zero tokens and masks":
+        x[::3] = 0
+        b[:], b[off] = 0, -np.inf
+    elif kind == "almost zero tokens":     # their squares underflow
+        x[::3] = np.float32(1e-30) * g.choice([0.0, 1.0, -1.0], x[::3].shape).astype(np.float32)
+    elif kind == "odd tokens":
+        x[0, 5], x[3, 100], x[4, 0], x[5, :] = np.nan, np.inf, -np.inf, 3e38
+    return x, w, b
+
+
+KINDS = ["half -inf", "half lowest", "one group of 32 left", "eight left", "four left", "some +inf", "zero tokens", "zero tokens and masks",
+         "almost zero tokens", "odd tokens"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("score_fn", [L.SCORE_SIGMOID, L.SCORE_SQRT_SOFTPLUS])
+@pytest.mark.parametrize("n_experts,hidden", [(256, 1024), (211, 4096)])
+def test_masks_padding_and_numbers_that_are_none(router, kind, score_fn, n_experts, hidden):
+    """The filter's routes are those of all scores in double."""
+    g = np.random.default_rng(len(kind) + hidden)
+    x, w = g.standard_normal((80, hidden)).astype(np.float32), bf16(g.standard_normal((n_experts, hidden)) * 0.02)
+    x, w, b = masked(g, x, w, (g.random(n_experts) * 0.2 - 0.1).astype(np.float32), kind)
+    bits = synth.f32_to_bf16_bits(w)
+    ids, wts, _ = router(x, bits, b, score_fn, 6)
+    want_ids, want, _ = router(x, bits, b, score_fn, 6, tiles=True)
+    assert np.array_equal(ids, want_ids)
+    assert (np.isnan(wts) & np.isnan(want) | (wts.view(np.uint32) == want.view(np.uint32))).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["half -inf", "half lowest", "one group of 32 left", "zero tokens", "zero tokens and masks"])
+def test_masks_and_padding_cost_little(router, kind):
+    """Every expert a candidate takes six times as long as plain rows; a mask or a token of zeros is no reason for it."""
+    g = np.random.default_rng(1)
+    n, n_experts, hidden = 300, 256, 4096
+    x, w = g.standard_normal((n, hidden)).astype(np.float32), bf16(g.standard_normal((n_experts, hidden)) * 0.02)
+    b = (g.random(n_experts) * 0.2 - 0.1).astype(np.float32)
+    bits = synth.f32_to_bf16_bits(w)
+    router(x, bits, b, L.SCORE_SIGMOID, 6, calls=50)
+    plain = router.us
+    x, _, b = masked(g, x, w, b, kind)
+    router(x, bits, b, L.SCORE_SIGMOID, 6, calls=50)
+    assert router.us < 2.0 * plain
