@@ -6,9 +6,12 @@
 
 namespace s14 {
 
-// score + bias as an integer of the same order
+// score + bias as an integer of the same order; a NaN, whose sign means nothing, below all numbers from zero up and above the negative ones.  (Said
+// here because the compiler may take `bits | sign` for a float's negative absolute value, which makes a NaN such a key in one kernel and
+// the largest one in another.)
 __device__ __forceinline__ uint32_t order_key(float v) {
     const uint32_t bits = __float_as_uint(v);
+    if (v != v) return 0x7FFFFFFFu;
     return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
 }
 // The picks of a warp whose lane holds the keys of experts lane, lane + 32, ... (`left`: which of them are there): lane j returns

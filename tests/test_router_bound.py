@@ -222,6 +222,8 @@ def masked(g, x, w, b, kind):
         b[4:] = -np.inf
     elif kind == "some +inf":
         b[[3, 200, 77]] = np.inf
+    elif kind == "a NaN bias":
+        b[9] = np.nan
     elif kind == "zero tokens":
         x[::3], x[1] = 0, -0.0
         b[:] = 0
@@ -232,11 +234,13 @@ def masked(g, x, w, b, kind):
         x[::3] = np.float32(1e-30) * g.choice([0.0, 1.0, -1.0], x[::3].shape).astype(np.float32)
     elif kind == "odd tokens":
         x[0, 5], x[3, 100], x[4, 0], x[5, :] = np.nan, np.inf, -np.inf, 3e38
+    elif kind == "odd weights":
+        w[7, 3], w[8, 4], w[9, 5] = np.inf, -np.inf, np.nan
     return x, w, b
 
 
-KINDS = ["half -inf", "half lowest", "one group of 32 left", "eight left", "four left", "some +inf", "zero tokens", "zero tokens and masks",
-         "almost zero tokens", "odd tokens"]
+KINDS = ["half -inf", "half lowest", "one group of 32 left", "eight left", "four left", "some +inf", "a NaN bias", "zero tokens", "zero tokens and masks",
+         "almost zero tokens", "odd tokens", "odd weights"]
 
 
 @pytest.mark.gpu
@@ -248,7 +252,8 @@ def test_masks_padding_and_numbers_that_are_none(router, kind, score_fn, n_exper
     g = np.random.default_rng(len(kind) + hidden)
     x, w = g.standard_normal((80, hidden)).astype(np.float32), bf16(g.standard_normal((n_experts, hidden)) * 0.02)
     x, w, b = masked(g, x, w, (g.random(n_experts) * 0.2 - 0.1).astype(np.float32), kind)
-    bits = synth.f32_to_bf16_bits(w)
+    with np.errstate(invalid="ignore"):
+        bits = synth.f32_to_bf16_bits(w)
     ids, wts, _ = router(x, bits, b, score_fn, 6)
     want_ids, want, _ = router(x, bits, b, score_fn, 6, tiles=True)
     assert np.array_equal(ids, want_ids)
@@ -269,3 +274,20 @@ def test_masks_and_padding_cost_little(router, kind):
     x, _, b = masked(g, x, w, b, kind)
     router(x, bits, b, L.SCORE_SIGMOID, 6, calls=50)
     assert router.us < 2.0 * plain
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tiles", [False, True])
+@pytest.mark.parametrize("kind", ["a NaN bias", "odd weights"])
+def test_a_score_that_is_none_is_not_picked(router, oracle, kind, tiles):
+    """By either way, as by the oracle: an expert without a score comes behind those that have one from zero up."""
+    g = np.random.default_rng(2)
+    x, w = g.standard_normal((70, 1024)).astype(np.float32), bf16(g.standard_normal((256, 1024)) * 0.02)
+    x, w, b = masked(g, x, w, (g.random(256) * 0.2).astype(np.float32), kind)
+    with np.errstate(invalid="ignore"):
+        bits = synth.f32_to_bf16_bits(w)
+    ids, wts, _ = router(x, bits, b, L.SCORE_SIGMOID, 6, tiles=tiles)
+    assert not (ids == 9).any()
+    for t in range(0, 70, 7):
+        rid, rw, _, _ = oracle.router(x[t], bits, b, score_fn=L.SCORE_SIGMOID, top_k=6, route_scale=1.5)
+        assert np.array_equal(ids[t], rid) and np.array_equal(wts[t].view(np.uint32), rw.view(np.uint32)), t
