@@ -39,7 +39,7 @@ namespace {
 
 // A chunk's B operand is made of groups of sixteen digit rows: one token each; in the official arithmetic,
 // whose values need six digit rows, the tokens' rows follow one another.  Most groups of a chunk:
-constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens
+constexpr uint32_t kGrpSmall = 2;    // blocks of up to twelve tokens (of twelve 6 and 12 are 2 and 4 % faster at the size below, and not taken)
 constexpr uint32_t kGrpSparse = 6;
 constexpr uint32_t kGrpDense = 12;
 // F32, us with 2 / 6 / 12 (256 experts of 4096 x 2048 unless said; 4 and 8 lie in between): 1 token 41.6 / 43.7 / 45.2, 4 71.9 / 75.9 / 76.2,
@@ -49,7 +49,8 @@ constexpr uint32_t kGrpDense = 12;
 // 81.7 / 79.8, 370 over 256 of 1024 x 512 129.0 / 125.5, 45 over 192 of 2048 x 1536 118.8 / 117.2, 100 over 64 of 2048 x 1024 93.2 / 87.8.  So: the
 // kernels for twelve pass over an expert less often, but need the registers in which the next launch's CTAs would be set up, some three
 // microseconds for the call; they pay from 2^29 pairs x hidden x inter on (a page below 2^19 counted as that: an item's fixed part;
-// 200 over 64 of 512 x 512 by the product alone 69.7, so 67.6), where experts have a pair on average at least.
+// 200 over 64 of 512 x 512 by the product alone 69.7, so 67.6), where experts have a pair on average at least
+// (13 and 32 tokens over 256 lie below it, for 1 %).
 constexpr uint64_t kDenseWork = 1ull << 29, kDensePage = 1ull << 19;
 // Official arithmetic, 6 / 12 groups (16 / 32 tokens): the same, from 2^30 on.  60 over 16 of 512 x 512 30.2 / 32.6, 20 over 64 of 2048 x 1024 53.8 / 55.5,
 // 40 over 32 of it 47.6 / 48.9, 150 over 128 of 1024 x 512 56.1 / 58.1, 45 over 192 of 2048 x 1536 116.4 / 116.2, 80 over 64 of 2048 x 1024 70.0 / 69.8,
@@ -310,7 +311,7 @@ k_block_group(const int32_t *__restrict__ ids, const uint8_t *const *__restrict_
 // The official arithmetic's rows are BF16 values and are stored as such: 115 MB written and read for 1000 tokens, stored as F32, now 57
 // (the call, with its down kernel, 973 us power limited, now 956).  CTAs of 128 threads: 256 took 0.3 us more for a block of 8 tokens.
 // The launch behind may start when the CTAs here exit, not earlier: all of them are resident at once, and while they are, the
-// CTAs of the next block's router scores, which fill the FP64 pipe of an SM, find room on few SMs only, several on one.  Blocks one
+// CTAs of the next block's router scores, which fill the FP64 pipe of an SM (where it takes all of them in double), find room on few SMs only, several on one.  Blocks one
 // after another, 4096 x 2048, 64 experts, us: 200 tokens 336, so 319, official 221 and 210; 2048 x 1024, 370 tokens 212 and 203;
 // 8 and 45 tokens the same.
 template <bool vec, bool kOff>

@@ -9,7 +9,7 @@
 // item's accumulators are read, added and finished while the next item's MMAs run.  The kernel before this one
 // (two row tiles and twelve tokens per SM, one set of accumulators, stages of 58 KB in a ring of three, N = 96) waited for the
 // epilogue between two items and for a stage's way through the memory.  370 tokens, 4096 x 2048, up / down kernel: 507 / 294
-// us, now 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, then 577 / 311, now 424 / 227 (see below).  Small blocks, which took one row tile
+// us, then 393 / 212; 1000 tokens of the official arithmetic 1200 / 444, then 577 / 311 and 424 / 227 (steps since: see below).  Small blocks, which took one row tile
 // and two tokens per SM with stages of 21 KB in a ring of eight and laid out the hidden values' digit rows in the up epilogue:
 // 8 tokens 117 us for the call, now 109.  (Official blocks of two to eight tokens of smaller layers gained nothing: 4 tokens of
 // 2048 x 1536 49 us for the call, now 52.)
@@ -25,7 +25,7 @@
 // with exact sums and the SwiGLU here, up 950 / 3900 / 5500, down 540 / 4150 / 1550: there the epilogue was what bounded both
 // kernels (1000 tokens 1036 us, without an epilogue 825, without three of four MMAs 1003, without the tiles' copies 1067), and fewer steps
 // (six digit rows for eight) alone gave nothing.  So BF16 sums are settled by plain additions and a bound where that is possible, four
-// pairs of tokens side by side, and the SwiGLU is k_block_digits' work: 1161 us power limited, now 992.  (The like for F32 sums, one part of the
+// pairs of tokens side by side, and the SwiGLU is k_block_digits_official's work: 1161 us power limited, now 992.  (The like for F32 sums, one part of the
 // three exact: 370 tokens nothing, 8 tokens 115 -> 120.)  Sustained, the
 // 1000 W limit lowers the clock to 1.4-1.6 GHz: 0.8 J per block of 370 tokens, 0.28 of them in the MMAs.  A pair with more items
 // than a batch of records drains its pipeline between two batches (1000 official tokens: 73 items, batches of 56).
@@ -608,7 +608,7 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
                     }
                 } else if constexpr (kOff) {
                     // threads 0-63 of the warpgroup hold the gates of the slice's elements, threads 64-127 their up projections: BF16
-                    // values into the pair's two rows (the rest is element by element and k_block_digits')
+                    // values into the pair's two rows (the rest is element by element and k_block_digits_official's)
 #pragma unroll
                     for (uint32_t m = 0; m < kMine; ++m) {
 #pragma unroll
@@ -732,7 +732,8 @@ k_block_pair(const __grid_constant__ GemmArgs a, uint32_t *status) {
         mbar_drain(bar(kPBarFin), 0);
     }
     if (warp >= kPProdWarp0 && warp < kPProdWarp0 + kPProds && lane == 0) {
-        // copies in flight land in this CTA's shared memory, arrivals of the tensor operations at its barriers: wait for them
+        // copies in flight land in this CTA's shared memory, arrivals of the tensor operations at its barriers: wait for them.  (A slot's first
+        // round has no wait that could run out, so every unit asked for in front of the kernel's wait is counted in `used`.)
 #pragma unroll 1
         for (uint32_t s = warp - kPProdWarp0; s < ring; s += kPProds) {
             const uint32_t used = round + (s < slot ? 1u : 0u);   // rounds of this slot
