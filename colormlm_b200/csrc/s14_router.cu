@@ -405,12 +405,12 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     // score is)
     off += 0x1p-18f * (fabsf(s) + (fabsf(b) <= 3e38f ? fabsf(b) : 0.0f) + 0x1p-20f);
     const bool all = __syncthreads_or(there && !(fabsf(s) <= 3e38f && off <= 3e38f && b == b));
-    // a token of zeros (padding): every logit is zero
+    // a token of zeros (padding): every logit is zero; one that holds a NaN (padding that nobody has written): every logit is none
     const uint32_t bits = __float_as_uint(xa[0].x) | __float_as_uint(xa[0].y) | __float_as_uint(xa[0].z) | __float_as_uint(xa[0].w) |
                           __float_as_uint(xb[0].x) | __float_as_uint(xb[0].y) | __float_as_uint(xb[0].z) | __float_as_uint(xb[0].w) |
                           __float_as_uint(xa[1].x) | __float_as_uint(xa[1].y) | __float_as_uint(xa[1].z) | __float_as_uint(xa[1].w) |
                           __float_as_uint(xb[1].x) | __float_as_uint(xb[1].y) | __float_as_uint(xb[1].z) | __float_as_uint(xb[1].w);
-    const bool zero = x2 == 0.0f && !__syncthreads_or((bits << 1) != 0u) && !all;
+    const bool none = x2 != x2, alike = none || (x2 == 0.0f && !__syncthreads_or((bits << 1) != 0u) && !all);
     // No more than the top_k-th largest of what the experts have at least: the largest of every one, two, four or eight experts, of 32 such
     // groups at most, and of those the top_k-th (where two of the largest are in one group it is the next one's: a candidate more).  Every
     // warp finds it.
@@ -486,13 +486,13 @@ k_router_pick(const float *__restrict__ x, const uint16_t *__restrict__ wr, cons
     // three to the right, are the double of 2^-896 times its value, subnormal ones included, so nothing has to be converted (a conversion takes
     // an SM four times as long as a multiplication); with the token times 2^800 no product leaves the range of normal doubles, and the sum has
     // the bits of the plain one times 2^-96.  Weights that are not finite come with `all`, and so does this loop's other form.
-    if (zero) {
-        s_score[tid] = router_score_f32(0.0, score_fn);
+    if (alike) {
+        s_score[tid] = router_score_f32(none ? __longlong_as_double(-1ll) : 0.0, score_fn);
         s_sel[tid] = __fadd_rn(s_score[tid], b);
         __syncthreads();
     }
 #pragma unroll 1
-    for (uint32_t c0 = zero ? n : 0u; c0 < n; c0 += 8u) {
+    for (uint32_t c0 = alike ? n : 0u; c0 < n; c0 += 8u) {
         double acc[8];
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) acc[k] = 0.0;

@@ -232,6 +232,8 @@ def masked(g, x, w, b, kind):
         b[:], b[off] = 0, -np.inf
     elif kind == "almost zero tokens":     # their squares underflow
         x[::3] = np.float32(1e-30) * g.choice([0.0, 1.0, -1.0], x[::3].shape).astype(np.float32)
+    elif kind == "NaN tokens":
+        x[::3, 5], x[1] = np.nan, np.nan
     elif kind == "odd tokens":
         x[0, 5], x[3, 100], x[4, 0], x[5, :] = np.nan, np.inf, -np.inf, 3e38
     elif kind == "odd weights":
@@ -240,7 +242,7 @@ def masked(g, x, w, b, kind):
 
 
 KINDS = ["half -inf", "half lowest", "one group of 32 left", "eight left", "four left", "some +inf", "a NaN bias", "zero tokens", "zero tokens and masks",
-         "almost zero tokens", "odd tokens", "odd weights"]
+         "almost zero tokens", "NaN tokens", "odd tokens", "odd weights"]
 
 
 @pytest.mark.gpu
@@ -261,9 +263,9 @@ def test_masks_padding_and_numbers_that_are_none(router, kind, score_fn, n_exper
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["half -inf", "half lowest", "one group of 32 left", "zero tokens", "zero tokens and masks"])
+@pytest.mark.parametrize("kind", ["half -inf", "half lowest", "one group of 32 left", "zero tokens", "zero tokens and masks", "NaN tokens"])
 def test_masks_and_padding_cost_little(router, kind):
-    """Every expert a candidate takes six times as long as plain rows; a mask or a token of zeros is no reason for it."""
+    """Every expert a candidate takes six times as long as plain rows; a mask or a token of zeros or without a number is no reason for it."""
     g = np.random.default_rng(1)
     n, n_experts, hidden = 300, 256, 4096
     x, w = g.standard_normal((n, hidden)).astype(np.float32), bf16(g.standard_normal((n_experts, hidden)) * 0.02)
